@@ -307,8 +307,8 @@ def matvec_sweep(capi, torch, hbm_peak):
 
 def gemm_sweep(capi, torch, tf_peak):
     """isolated int8-weight GEMM (prefill / batched-step operator) at Gemma-3-1B shapes, device-resident.
-    TFLOP/s counts the algorithmic 2*M*K*N; the tensor cores execute three bf16 products per fp32
-    activation (split into three bf16 terms), so the tensor-pipe work is three times that."""
+    TFLOP/s counts the algorithmic 2*M*K*N; the tensor cores execute four int8 products per fp32
+    activation (four 8-bit digits) at twice the bf16 rate, so the share of the tensor pipe is twice that over the bf16 peak."""
     import ctypes as C
 
     lib = capi.load()
@@ -352,8 +352,8 @@ def gemm_sweep(capi, torch, tf_peak):
             # one uncaptured call afterwards reports an error word a replay may have set
             run(0, C.c_void_p(torch.cuda.current_stream().cuda_stream))
             tf = 2.0 * M * K * N / us / 1e6
-            out.append({"M": M, "K": K, "N": N, "us": us, "TFLOPs": tf, "tensor_TFLOPs": 3 * tf,
-                        "tensor_frac": 3 * tf / tf_peak if tf_peak else None})
+            out.append({"M": M, "K": K, "N": N, "us": us, "TFLOPs": tf, "int8_TOPs": 4 * tf,
+                        "tensor_frac": 2 * tf / tf_peak if tf_peak else None})
     return out
 
 

@@ -1,0 +1,53 @@
+"""The integer tensor-core GEMM (kernels_gemm_i8.cuh) at the edges of its tiles: token groups of 8, tiles of 64 tokens
+and 128 columns, K-splits, the longest K; and rows that a shared exponent could spoil. Compared with float64: the digit
+sums are exact, so what is left is one fp32 rounding per join (relative L2 about 5e-8; bound 2e-7)."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def case(M, K, N, seed=3):
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    w = rng.integers(-128, 128, (K, N), dtype=np.int8)
+    s = (rng.random(N, dtype=np.float32) * 1e-2 + 1e-4).astype(np.float32)
+    return x, w, s
+
+
+def exact(x, w, s):
+    return (x.astype(np.float64) @ w.astype(np.float64)) * s.astype(np.float64)
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 63, 64, 65, 129, 513])
+@pytest.mark.parametrize("K,N", [(256, 256), (640, 1152), (6912, 640)])
+def test_tile_edges(capi, M, K, N):
+    x, w, s = case(M, K, N)
+    assert rel_l2(capi.qgemm(x, w, s), exact(x, w, s)) <= 2e-7
+
+
+def test_many_tiles_per_cta(capi):
+    # 54 column tiles x 33 token tiles: twelve tiles per CTA, both accumulators reused
+    x, w, s = case(2051, 256, 6912)
+    assert rel_l2(capi.qgemm(x, w, s), exact(x, w, s)) <= 2e-7
+
+
+def test_rows_of_any_range(capi):
+    x, w, s = case(12, 1152, 640)
+    x[1] *= 1e-30                    # tiny and huge rows beside ordinary ones: the exponent is per row
+    x[2] *= 1e25
+    x[3] = 0
+    x[4] *= np.exp(3 * np.random.default_rng(1).standard_normal(1152)).astype(np.float32)  # six decades inside a row
+    x[5] = np.float32(2.0) ** np.arange(1152, dtype=np.float32).clip(0, 20)               # powers of two: the top of the range
+    x[6] = 1.0 - 2.0 ** -24
+    x[7, 5] = np.nan
+    x[8, 6] = np.inf
+    c = capi.qgemm(x, w, s)
+    want = exact(np.where(np.isfinite(x), x, 0), w, s)
+    for r in (0, 1, 2, 4, 5, 6, 9, 10, 11):
+        assert rel_l2(c[r], want[r]) <= 2e-7, r
+    assert not c[3].any()
+    assert np.isnan(c[7]).all() and not np.isfinite(c[8]).any()

@@ -8,7 +8,7 @@
 //     S = Q K_j^T                    M128 x N64, contraction over the 256 head dimensions
 //     online softmax on S            (max in use m and sum l per row; a row = one TMEM lane, two threads)
 //     O = corr * O + P V_j           M128 x N256, contraction over the 64 keys
-// fp32 accuracy on bf16 tensor cores as in the GEMM (kernels_gemm_tc.cuh): every fp32 operand is split into
+// fp32 accuracy on bf16 tensor cores as in the GEMM (kernels_tc.cuh): every fp32 operand is split into
 // three bf16 terms x = hi + mid + lo and a product a * b is the six term products whose weight reaches
 // 2^-24 (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi), all accumulated in fp32 in TMEM.
 //
@@ -28,7 +28,7 @@
 // All waits are bounded; a wait that runs out sets *err, and the CTA lets its copies land and frees its
 // TMEM before it returns.
 #pragma once
-#include "kernels_gemm_tc.cuh"
+#include "kernels_tc.cuh"
 
 namespace tg {
 

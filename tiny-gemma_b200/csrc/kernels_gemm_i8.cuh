@@ -1,0 +1,605 @@
+// GEMM with int8 weights on the integer tensor cores (tcgen05 kind::i8 + TMEM):
+//   C[m, n] = scale[n] * sum_k A[m,k] * W[k,n],  A fp32, W int8 [K,N] row-major
+// (gemm::qgemmnn, reference linalg.hpp:210-308, which runs a full-K fp32 FMA chain per output).
+//
+// Arithmetic: a row of A is written as x = 2^(e-30) * (d3 * 2^24 + d2 * 2^16 + d1 * 2^8 + d0), one exponent e per
+// row (2^e > the row's largest |x|), four signed 8-bit digits. An element within a factor 2^7 of the row's largest
+// keeps all 24 bits of its fp32 mantissa; below that the representation is still exact to 2^-31 of the largest. The
+// weights go to the tensor cores as they lie in memory, the digit products are summed EXACTLY in int32 (at most
+// 6912 * 128 * 128 < 2^31), and only the epilogue rounds: it joins the four sums in fp32. Against three bf16 terms with fp32 accumulation
+// (6 bytes per activation, weights converted on the SM, truncating adds): 4 products at twice the bf16 rate instead of
+// 3, no conversion of W, and no accumulation error that grows with K, so K is never split for accuracy.
+//
+// Operand roles are swapped: the MMA's M dimension (128 TMEM lanes) runs over columns of W, its N dimension over
+// (token, digit). So the token count pads to 8, not to 128, one MMA of N = 256 covers all four digits of 64 tokens
+// against one fetched W tile, and in the epilogue the 32 lanes of a warp hold 32 consecutive columns of one token: a
+// store instruction writes 128 contiguous bytes straight from registers.
+//
+// Operand layouts:
+//   W       box of 128 columns x 128 rows by TMA with the 128-byte swizzle = MN-major operand, 8 k-rows per 1 KiB atom
+//   digits  [K / 64][groups of 8 tokens][4 digits][8 tokens][64 k] bytes, 64-byte swizzle (K-major operand, 512 B per
+//           (group, digit)): a CTA's tokens of one K-block are contiguous, one bulk copy each
+// Accumulator column of (group g, digit d, token r): 32 g + 8 d + r.
+//
+// The kernel is persistent, one CTA per SM walking tiles of 128 columns x up to 64 tokens, with two accumulators of 256
+// TMEM columns: the epilogue of a tile (8 warps) and the loads of the next one run under MMAs. One tile per CTA spent
+// more time outside its K loop than in it (K = 1152: ~10K of 20K clk: start ~1.5K, first operands ~2.5K, epilogue ~4K).
+// A completed mbarrier test costs ~180 clk on this part, so a stage is large: 128 k, 48 KB, 512 clk of MMAs.
+// The operands come at 96 B/clk of MMA time, which the L2 delivers (a pure bulk-copy loop measured 80-85 B/clk averaged
+// over all SMs, 19 TB/s); one 256-column tile without the second accumulator needs 64 B/clk and was slower.
+//
+// All waits are bounded; a wait that runs out sets *err and the CTA drains and frees its TMEM before returning.
+#pragma once
+#include <cuda.h>
+
+#include "kernels_tc.cuh"  // tcgen05 / bulk-copy helpers
+#include "tg_common.cuh"
+
+namespace tg {
+
+constexpr int I8_BK = 64;                      // k per block of the packed digits
+constexpr int I8_GROUP_BYTES = 4 * 8 * I8_BK;  // one (K-block, token group): 4 digits x 8 tokens x 64 k
+constexpr int I8_SK = 128;                     // k per stage
+constexpr int I8_TG = 8;                       // token groups of a tile, at most
+constexpr int I8_W_BYTES = 128 * I8_SK, I8_X_BYTES = (I8_SK / I8_BK) * I8_TG * I8_GROUP_BYTES;
+constexpr int I8_STAGE = I8_W_BYTES + I8_X_BYTES;
+constexpr int I8_NST = 4;
+constexpr int I8_SMEM = I8_NST * I8_STAGE + 1024;
+constexpr int I8_THREADS = 320;                // producer, MMA issuer, 8 epilogue warps
+
+// ------------------------------------------------------------------ digits
+// exponent of a row from the bits of its largest |x| (NaN and infinity compare above every finite value)
+__device__ __forceinline__ int i8_row_exp(uint32_t maxbits) { return max(int(maxbits >> 23) - 126, -96); }
+__device__ __forceinline__ float i8_pow2(int e) { return __uint_as_float(uint32_t(e + 127) << 23); }  // -126 <= e <= 127
+// what a digit sum is multiplied with: 2^(e - 30), or NaN for a row that holds a NaN or an infinity
+__device__ __forceinline__ float i8_row_scale(uint32_t maxbits) {
+	return maxbits >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : i8_pow2(i8_row_exp(maxbits) - 30);
+}
+__device__ __forceinline__ float i8_row_mul(uint32_t maxbits) { return i8_pow2(30 - i8_row_exp(maxbits)); }
+__device__ __forceinline__ uint32_t i8_abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+
+// byte i of the result = digit i: q = sum d_i 256^i with d_i in [-128, 127] <=> q + 0x80808080 has bytes d_i + 128
+__device__ __forceinline__ uint32_t i8_digits(float x, float mul) {
+	return (uint32_t(__float2int_rn(x * mul)) + 0x80808080u) ^ 0x80808080u;
+}
+// byte offset of (row, 4 consecutive k starting at k4 * 4, digit 0) in the packed operand; digits are 512 B apart
+__device__ __forceinline__ size_t i8_offset(int row, int k4, int groups) {
+	const int kb = k4 >> 4, chunk = (k4 >> 2) & 3, r = row & 7;
+	return (size_t(kb) * groups + (row >> 3)) * I8_GROUP_BYTES + r * 64 + ((chunk ^ (r >> 1)) << 4) + ((k4 & 3) << 2);
+}
+// four consecutive values of a row -> one 4-byte store per digit
+__device__ __forceinline__ void i8_pack4(uint8_t *out, int groups, int row, int k4, const float4 &v, float mul) {
+	const uint32_t a = i8_digits(v.x, mul), b = i8_digits(v.y, mul), c = i8_digits(v.z, mul), d = i8_digits(v.w, mul);
+	const uint32_t ab01 = __byte_perm(a, b, 0x5140), ab23 = __byte_perm(a, b, 0x7362);
+	const uint32_t cd01 = __byte_perm(c, d, 0x5140), cd23 = __byte_perm(c, d, 0x7362);
+	uint8_t *p = out + i8_offset(row, k4, groups);
+	*reinterpret_cast<uint32_t *>(p) = __byte_perm(ab01, cd01, 0x5410);
+	*reinterpret_cast<uint32_t *>(p + 512) = __byte_perm(ab01, cd01, 0x7632);
+	*reinterpret_cast<uint32_t *>(p + 1024) = __byte_perm(ab23, cd23, 0x5410);
+	*reinterpret_cast<uint32_t *>(p + 1536) = __byte_perm(ab23, cd23, 0x7632);
+}
+__device__ __forceinline__ uint32_t warp_umax(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+template <int NW> __device__ __forceinline__ uint32_t block_umax(uint32_t v, uint32_t *red) {
+	v = warp_umax(v);
+	__syncthreads();
+	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+	__syncthreads();
+	uint32_t t = 0;
+#pragma unroll
+	for (int w = 0; w < NW; w++) t = max(t, red[w]);
+	return t;
+}
+
+// fp32 rows -> digits. One CTA of NT threads per row (rows >= M: zeros), the row in registers: K <= NT * 4 * PER.
+template <int NT, int PER>
+__global__ void __launch_bounds__(NT) i8_pack_kernel(const float *A, uint8_t *out, float *rowscale, int M, int K, int groups) {
+	pdl_trigger();
+	pdl_wait();
+	__shared__ uint32_t red[NT / 32];
+	const int row = blockIdx.x, tid = threadIdx.x;
+	float4 v[PER];
+	uint32_t mx = 0;
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = tid + NT * j;
+		v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (row < M && 4 * k4 < K) v[j] = *reinterpret_cast<const float4 *>(A + size_t(row) * K + 4 * k4);
+		mx = max(max(max(mx, i8_abs_bits(v[j].x)), max(i8_abs_bits(v[j].y), i8_abs_bits(v[j].z))), i8_abs_bits(v[j].w));
+	}
+	mx = block_umax<NT / 32>(mx, red);
+	const float mul = i8_row_mul(mx);
+	if (tid == 0) rowscale[row] = i8_row_scale(mx);
+#pragma unroll
+	for (int j = 0; j < PER; j++)
+		if (4 * (tid + NT * j) < K) i8_pack4(out, groups, row, tid + NT * j, v[j], mul);
+}
+
+// Residual + sandwich norms of one row, fused with the operand packing of the next GEMM:
+//   if t:     h += rmsnorm(t; w_post)        (reference modules.hpp: post-norm, then the residual add)
+//   if w_pre: pack( rmsnorm(h; w_pre) )      (the pre-norm of the following matmuls)
+// t is the partial sums of the GEMM before: t[d] = tscale[d] * sum_sp t[(sp * M + row) * dim + d], added in split order.
+// A row belongs to NT threads, its values stay in their registers (dim <= 4 * NT * PER). A row is a chain of dependent
+// round trips (loads, two reductions), so everything that does not depend on the partial sums is requested before them.
+//   NT = 288 (one CTA per row): a few hundred rows, all resident at once, the chain's length counts
+//   NT = 32  (one warp per row, 8 rows per CTA): thousands of rows; no barriers, shuffles only, more rows in flight
+template <int NT, int PER>
+__global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *h, const float *t, const float *w_post, const float *w_pre, uint8_t *out,
+                                                                         float *rowscale, int M, int dim, int groups, int nsplit,
+                                                                         const float *tscale) {
+	constexpr int NW = NT / 32;
+	__shared__ float2 red[NT == 32 ? 1 : NW];
+	const int lt = NT == 32 ? int(threadIdx.x & 31) : int(threadIdx.x);
+	const int row = NT == 32 ? int(blockIdx.x * 8 + (threadIdx.x >> 5)) : int(blockIdx.x);
+	const int n4 = dim / 4;
+	// sum of a, maximum of the bit patterns b over the row's threads
+	auto reduce = [&](float a, uint32_t b) -> float2 {
+		a = warp_sum(a);
+		b = warp_umax(b);
+		if (NT == 32) return make_float2(a, __uint_as_float(b));
+		__syncthreads();
+		if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(a, __uint_as_float(b));
+		__syncthreads();
+		float s = 0.0f;
+		uint32_t m = 0;
+#pragma unroll
+		for (int w = 0; w < NW; w++) {
+			s += red[w].x;
+			m = max(m, __float_as_uint(red[w].y));
+		}
+		return make_float2(s, __uint_as_float(m));
+	};
+	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 wpost[PER], wpre[PER];  // the weights are nobody's output: requested before the wait for the predecessor
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = lt + NT * j;
+		wpost[j] = wpre[j] = z4;
+		if (NT != 32 && k4 < n4) {
+			if (t) wpost[j] = __ldg(reinterpret_cast<const float4 *>(w_post) + k4);
+			if (w_pre) wpre[j] = __ldg(reinterpret_cast<const float4 *>(w_pre) + k4);
+		}
+	}
+	pdl_trigger();
+	pdl_wait();
+	if (row >= groups * 8) return;  // (whole warps or whole CTAs)
+	if (row >= M) {
+		if (w_pre) {
+#pragma unroll
+			for (int j = 0; j < PER; j++)
+				if (lt + NT * j < n4) i8_pack4(out, groups, row, lt + NT * j, z4, 0.0f);
+			if (lt == 0) rowscale[row] = 0.0f;
+		}
+		return;
+	}
+	float4 *hrow = reinterpret_cast<float4 *>(h + size_t(row) * dim);
+	float4 hv[PER];
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = lt + NT * j;
+		hv[j] = z4;
+		if (k4 < n4) hv[j] = hrow[k4];
+	}
+	if (t) {
+		float4 acc[PER];
+#pragma unroll
+		for (int j = 0; j < PER; j++) acc[j] = z4;
+		const float4 *base = reinterpret_cast<const float4 *>(t + size_t(row) * dim);
+		const size_t stride = size_t(M) * n4;
+		constexpr int QB = NT == 32 ? 1 : 4;  // splits requested together
+		for (int s0 = 0; s0 < nsplit; s0 += QB) {
+			float4 q[QB][PER];
+#pragma unroll
+			for (int i = 0; i < QB; i++)
+#pragma unroll
+				for (int j = 0; j < PER; j++) {
+					const int k4 = lt + NT * j;
+					q[i][j] = z4;
+					if (k4 < n4 && s0 + i < nsplit) q[i][j] = base[size_t(s0 + i) * stride + k4];
+				}
+#pragma unroll
+			for (int i = 0; i < QB; i++)
+#pragma unroll
+				for (int j = 0; j < PER; j++) {
+					acc[j].x += q[i][j].x; acc[j].y += q[i][j].y; acc[j].z += q[i][j].z; acc[j].w += q[i][j].w;
+				}
+		}
+		float ss = 0.0f;
+#pragma unroll
+		for (int j = 0; j < PER; j++) {
+			const int k4 = lt + NT * j;
+			if (k4 < n4) {
+				const float4 s4 = __ldg(reinterpret_cast<const float4 *>(tscale) + k4);
+				acc[j].x *= s4.x; acc[j].y *= s4.y; acc[j].z *= s4.z; acc[j].w *= s4.w;
+				ss = fmaf(acc[j].x, acc[j].x, ss);
+				ss = fmaf(acc[j].y, acc[j].y, ss);
+				ss = fmaf(acc[j].z, acc[j].z, ss);
+				ss = fmaf(acc[j].w, acc[j].w, ss);
+			}
+		}
+		const float r = inv_rms(reduce(ss, 0u).x, dim);
+#pragma unroll
+		for (int j = 0; j < PER; j++) {
+			const int k4 = lt + NT * j;
+			if (k4 < n4) {
+				const float4 w4 = NT == 32 ? __ldg(reinterpret_cast<const float4 *>(w_post) + k4) : wpost[j];
+				hv[j].x += (acc[j].x * r) * (w4.x + 1.0f);
+				hv[j].y += (acc[j].y * r) * (w4.y + 1.0f);
+				hv[j].z += (acc[j].z * r) * (w4.z + 1.0f);
+				hv[j].w += (acc[j].w * r) * (w4.w + 1.0f);
+				hrow[k4] = hv[j];
+			}
+		}
+	}
+	if (!w_pre) return;
+	// sum of squares, and the largest |h * (w + 1)|: times the norm factor it bounds the row that is packed
+	float ss = 0.0f;
+	uint32_t mx = 0;
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = lt + NT * j;
+		if (NT == 32 && k4 < n4) wpre[j] = __ldg(reinterpret_cast<const float4 *>(w_pre) + k4);
+		ss = fmaf(hv[j].x, hv[j].x, ss);
+		ss = fmaf(hv[j].y, hv[j].y, ss);
+		ss = fmaf(hv[j].z, hv[j].z, ss);
+		ss = fmaf(hv[j].w, hv[j].w, ss);
+		mx = max(mx, max(max(i8_abs_bits(hv[j].x * (wpre[j].x + 1.0f)), i8_abs_bits(hv[j].y * (wpre[j].y + 1.0f))),
+		                 max(i8_abs_bits(hv[j].z * (wpre[j].z + 1.0f)), i8_abs_bits(hv[j].w * (wpre[j].w + 1.0f)))));
+	}
+	const float2 sm = reduce(ss, mx);
+	const float r = inv_rms(sm.x, dim);
+	const uint32_t mb = i8_abs_bits(sm.y * r);
+	const float mul = i8_row_mul(mb);
+	if (lt == 0) rowscale[row] = i8_row_scale(mb);
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = lt + NT * j;
+		if (k4 < n4)
+			i8_pack4(out, groups, row, k4,
+			         make_float4((hv[j].x * r) * (wpre[j].x + 1.0f), (hv[j].y * r) * (wpre[j].y + 1.0f), (hv[j].z * r) * (wpre[j].z + 1.0f),
+			                     (hv[j].w * r) * (wpre[j].w + 1.0f)),
+			         mul);
+	}
+}
+
+// GeGLU fused with the packing of the down projection's operand: pack( lut(gate) * up ). ug: partial sums of the grouped
+// up|gate GEMM (rows of 2I: up columns, then gate columns), su / sg their column scales. One CTA of 256 threads per row,
+// the row's products in registers (I <= 1024 * PER): their largest is needed before the first can be packed.
+template <int PER>
+__global__ void __launch_bounds__(256, 2) geglu_i8_kernel(const float *ug, uint8_t *out, float *rowscale, int M, int I, int groups, GeluLut lut,
+                                                       int nsplit, const float *su, const float *sg) {
+	pdl_trigger();
+	pdl_wait();
+	__shared__ uint32_t red[8];
+	const int row = blockIdx.x, tid = threadIdx.x, n4 = I / 4;
+	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 x[PER];
+	uint32_t mx = 0;
+	const float4 *base = reinterpret_cast<const float4 *>(ug + size_t(row) * 2 * I);
+	const size_t stride = size_t(M) * 2 * n4;
+#pragma unroll
+	for (int j = 0; j < PER; j++) {
+		const int k4 = tid + 256 * j;
+		x[j] = z4;
+		if (row < M && k4 < n4) {
+			float4 u = z4, g = z4;
+			for (int s = 0; s < nsplit; s++) {
+				const float4 a = base[size_t(s) * stride + k4], b = base[size_t(s) * stride + n4 + k4];
+				u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w;
+				g.x += b.x; g.y += b.y; g.z += b.z; g.w += b.w;
+			}
+			const float4 s4 = __ldg(reinterpret_cast<const float4 *>(su) + k4), t4 = __ldg(reinterpret_cast<const float4 *>(sg) + k4);
+			x[j].x = lut(g.x * t4.x) * (u.x * s4.x);
+			x[j].y = lut(g.y * t4.y) * (u.y * s4.y);
+			x[j].z = lut(g.z * t4.z) * (u.z * s4.z);
+			x[j].w = lut(g.w * t4.w) * (u.w * s4.w);
+		}
+		mx = max(mx, max(max(i8_abs_bits(x[j].x), i8_abs_bits(x[j].y)), max(i8_abs_bits(x[j].z), i8_abs_bits(x[j].w))));
+	}
+	mx = block_umax<8>(mx, red);
+	const float mul = i8_row_mul(mx);
+	if (tid == 0) rowscale[row] = i8_row_scale(mx);
+#pragma unroll
+	for (int j = 0; j < PER; j++)
+		if (tid + 256 * j < n4) i8_pack4(out, groups, row, tid + 256 * j, x[j], mul);
+}
+
+// ------------------------------------------------------------------ GEMM
+struct GemmI8Args {
+	const uint8_t *x;       // packed digits
+	const float *rowscale;  // [8 * groups]
+	int groups;             // token groups in the packed operand
+	int tg, tok_tiles;      // token groups per tile, token tiles
+	int n_fast;             // 1: consecutive tiles are the column tiles of one token tile; 0: the token tiles of one column tile
+	int tiles;              // col_tiles * tok_tiles * nsplit
+	// Up to three weight matrices with the same K share one launch (q|k|v, up|gate): matrix g owns the column tiles
+	// [tile_end[g-1], tile_end[g]) and columns col0[g].. of a partial-sum row (N = all columns)
+	int col_tiles;
+	int tile_end[3];
+	int col0[3];
+	const float *scales[3];  // [N_g]
+	float *C[3];             // [M] rows of ldc[g] floats (finished result)
+	int ldc[3];
+	float *partial;          // [nsplit][M][N] sums without the column scales (raw, or nsplit > 1)
+	int M, N, K, nsplit;
+	int raw;                 // 1: partial sums even unsplit; the consumer adds the splits and applies the column scales
+	int w_stream;            // 1: W is read by few CTAs: L2 evict-first
+	unsigned long long *top1;  // non-null (nsplit == 1): no C; per token the largest scaled value and its column, as a key
+	int top1_col0;
+	int *err;
+};
+
+// W tile [128 k][128 n], 128-byte swizzle: MN-major operand; 1 KiB from one group of 8 k-rows to the next
+__device__ __forceinline__ uint64_t i8_desc_w(uint32_t addr) {
+	return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t(1) << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61);
+}
+// digits, 64-byte swizzle: K-major operand; 512 B from one group of 8 rows (group, digit) to the next
+__device__ __forceinline__ uint64_t i8_desc_x(uint32_t addr) {
+	return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t(1) << 16) | (uint64_t(512 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(4) << 61);
+}
+// D int32, A and B signed 8 bit, A MN-major (bit 15), B K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t i8_idesc(int n) {
+	return (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (uint32_t(n >> 3) << 17) | (8u << 24);
+}
+__device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+	asm volatile(
+	    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+	    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+	    "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+	    : "memory");
+}
+
+// tile index -> what it covers (every role of a CTA walks the same tiles)
+struct I8Tile {
+	int grp, n0;         // matrix, first column inside it
+	int g0, ng;          // token groups
+	int split, s0, ns;   // K-split, its first stage and number of stages
+};
+__device__ __forceinline__ I8Tile i8_tile(const GemmI8Args &a, int t) {
+	I8Tile r;
+	int ct, tt;
+	const int per = a.col_tiles * a.tok_tiles;
+	r.split = t / per;
+	t -= r.split * per;
+	if (a.n_fast) {
+		tt = t / a.col_tiles;
+		ct = t - tt * a.col_tiles;
+	} else {
+		ct = t / a.tok_tiles;
+		tt = t - ct * a.tok_tiles;
+	}
+	r.grp = (ct >= a.tile_end[0]) + (ct >= a.tile_end[1]);  // tile_end of unused slots = INT_MAX
+	// (selects over constant indices: a run-time index into the parameter arrays would move them to local memory)
+	r.n0 = (ct - (r.grp == 0 ? 0 : (r.grp == 1 ? a.tile_end[0] : a.tile_end[1]))) * 128;
+	r.g0 = tt * a.tg;
+	r.ng = min(a.tg, a.groups - r.g0);
+	const int all = a.K / I8_SK;
+	r.s0 = r.split * all / a.nsplit;
+	r.ns = (r.split + 1) * all / a.nsplit - r.s0;
+	return r;
+}
+
+__global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
+                                                                 const __grid_constant__ CUtensorMap wmap1,
+                                                                 const __grid_constant__ CUtensorMap wmap2, GemmI8Args a) {
+	pdl_trigger();
+	extern __shared__ uint8_t i8_smem_raw[];
+	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(i8_smem_raw) + 1023) & ~uintptr_t(1023));
+	__shared__ uint64_t full_bar[I8_NST];   // W and digits of the stage landed
+	__shared__ uint64_t free_bar[I8_NST];   // the MMAs that read the stage have completed
+	__shared__ uint64_t acc_full[2];        // the accumulator's MMAs have completed
+	__shared__ uint64_t acc_free[2];        // the 8 epilogue warps have read the accumulator
+	__shared__ uint64_t drain_bar;          // every MMA issued has completed
+	__shared__ uint32_t tmem_base_s;
+	__shared__ int s_fail, s_issued;
+
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	if (tid == 0) {
+		for (int s = 0; s < I8_NST; s++) {
+			mbar_init(&full_bar[s], 1);
+			mbar_init(&free_bar[s], 1);
+		}
+		for (int b = 0; b < 2; b++) {
+			mbar_init(&acc_full[b], 1);
+			mbar_init(&acc_free[b], 8);
+		}
+		mbar_init(&drain_bar, 1);
+		s_fail = 0;
+		s_issued = 0;
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	if (warp == 1) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512)
+		             : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	const uint32_t tmem_base = tmem_base_s;
+
+	if (warp == 0) {
+		// ------------------------------------------------------------ producer
+		if (lane == 0) {
+			const uint64_t pol = l2_evict_first_policy();
+			auto load_w = [&](const I8Tile &t, int st, int s) {
+				mbar_expect_tx(&full_bar[s], uint32_t(I8_W_BYTES) + uint32_t(t.ng) * (I8_SK / I8_BK) * I8_GROUP_BYTES);
+				const CUtensorMap *wmap = t.grp == 0 ? &wmap0 : (t.grp == 1 ? &wmap1 : &wmap2);
+				uint8_t *dst = smem + size_t(s) * I8_STAGE;
+				if (a.w_stream)
+					tma_load_2d(dst, wmap, t.n0, (t.s0 + st) * I8_SK, &full_bar[s], pol);
+				else
+					tma_load_2d(dst, wmap, t.n0, (t.s0 + st) * I8_SK, &full_bar[s]);
+			};
+			auto load_x = [&](const I8Tile &t, int st, int s) {
+				const uint32_t bytes = uint32_t(t.ng) * I8_GROUP_BYTES;
+				uint8_t *dst = smem + size_t(s) * I8_STAGE + I8_W_BYTES;
+				const uint8_t *src = a.x + (size_t(t.s0 + st) * (I8_SK / I8_BK) * a.groups + t.g0) * I8_GROUP_BYTES;
+#pragma unroll
+				for (int q = 0; q < I8_SK / I8_BK; q++)
+					bulk_load(dst + q * (I8_TG * I8_GROUP_BYTES), src + size_t(q) * a.groups * I8_GROUP_BYTES, bytes, &full_bar[s]);
+			};
+			// The weights are nobody's output: the first tiles are requested before the wait for the predecessor.
+			int pre = 0;
+			if (int(blockIdx.x) < a.tiles) {
+				const I8Tile t = i8_tile(a, blockIdx.x);
+				pre = min(I8_NST, t.ns);
+				for (int st = 0; st < pre; st++) load_w(t, st, st);
+				pdl_wait();
+				for (int st = 0; st < pre; st++) load_x(t, st, st);
+			}
+			int c = pre, s = pre == I8_NST ? 0 : pre;  // stages issued so far, next slot
+			uint32_t ph = 0;                           // parity of the slot's previous use being over
+			bool go = true;
+			s_issued = c;
+			for (int ti = blockIdx.x; ti < a.tiles && go; ti += gridDim.x) {
+				const I8Tile t = i8_tile(a, ti);
+				for (int st = (ti == int(blockIdx.x) ? pre : 0); st < t.ns; st++) {
+					if (c >= I8_NST && !tc_wait(&free_bar[s], ph, a.err)) { s_fail = 1; go = false; break; }
+					load_w(t, st, s);
+					load_x(t, st, s);
+					s_issued = ++c;
+					if (++s == I8_NST) {
+						s = 0;
+						if (c > I8_NST) ph ^= 1;
+					}
+				}
+			}
+		}
+	} else if (warp == 1) {
+		// ------------------------------------------------------------ MMA issuer
+		if (lane == 0) {
+			int s = 0, it = 0;
+			uint32_t ph = 0;
+			bool ready = false, go = true;
+			for (int ti = blockIdx.x; ti < a.tiles && go; ti += gridDim.x, it++) {
+				const I8Tile t = i8_tile(a, ti);
+				const uint32_t d = tmem_base + uint32_t(it & 1) * 256, id = i8_idesc(32 * t.ng);
+				if (it >= 2 && !tc_wait(&acc_free[it & 1], ((it >> 1) - 1) & 1, a.err)) { s_fail = 1; break; }
+				for (int st = 0; st < t.ns; st++) {
+					if (!ready && !tc_wait(&full_bar[s], ph, a.err)) { s_fail = 1; go = false; break; }
+					tc_fence_after();
+					const uint32_t w = smem_u32(smem) + uint32_t(s) * I8_STAGE, x = w + I8_W_BYTES;
+					const int sn = s + 1 == I8_NST ? 0 : s + 1;
+#pragma unroll
+					for (int j = 0; j < I8_SK / 32; j++) {
+						i8_mma(d, i8_desc_w(w + j * 4096), i8_desc_x(x + (j >> 1) * (I8_TG * I8_GROUP_BYTES) + (j & 1) * 32), id, (st > 0 || j > 0) ? 1u : 0u);
+						// the next stage's barrier is tested between the MMAs of this one: behind them, the test would let
+						// the tensor pipe run dry
+						if (j == 1) ready = mbar_try_wait(&full_bar[sn], sn == 0 ? ph ^ 1 : ph);
+					}
+					tc_commit(&free_bar[s]);
+					if (sn == 0) ph ^= 1;
+					s = sn;
+				}
+				if (go) tc_commit(&acc_full[it & 1]);
+			}
+			tc_commit(&drain_bar);
+		}
+	} else {
+		// ------------------------------------------------------------ epilogue (warps 2..9)
+		pdl_wait();  // the row scales are the predecessor's output, and C may be its input
+		const int quad = warp & 3, sub = (warp - 2) >> 2;  // TMEM lanes 32 * quad ..; two warps share them
+		const bool fin = a.nsplit == 1 && !a.raw;
+		int it = 0;
+		for (int ti = blockIdx.x; ti < a.tiles; ti += gridDim.x, it++) {
+			const I8Tile t = i8_tile(a, ti);
+			const float *const scg = t.grp == 0 ? a.scales[0] : (t.grp == 1 ? a.scales[1] : a.scales[2]);
+			float *const Cg = t.grp == 0 ? a.C[0] : (t.grp == 1 ? a.C[1] : a.C[2]);
+			const size_t ld = fin ? size_t(t.grp == 0 ? a.ldc[0] : (t.grp == 1 ? a.ldc[1] : a.ldc[2])) : size_t(a.N);
+			const int pcol = t.grp == 0 ? a.col0[0] : (t.grp == 1 ? a.col0[1] : a.col0[2]);
+			const int nl = t.n0 + quad * 32 + lane;  // this lane's column
+			float *dst = fin ? Cg + nl : a.partial + size_t(t.split) * a.M * a.N + pcol + nl;
+			const float sc = fin ? scg[nl] : 1.0f;
+			const uint32_t acc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(it & 1) * 256;
+			const float4 *rs = reinterpret_cast<const float4 *>(a.rowscale + t.g0 * 8);
+			// one token group: 32 accumulator columns = 4 digits x 8 tokens, and its row scales
+			auto request = [&](int g, uint32_t (&r)[32], float4 (&q)[2]) {
+				tc_ld32(acc + uint32_t(g * 32), r);
+				q[0] = rs[2 * g];
+				q[1] = rs[2 * g + 1];
+			};
+			auto finish = [&](int g, uint32_t (&r)[32], float4 (&q)[2]) {
+				const int tok = (t.g0 + g) * 8;
+				const float rsv[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
+				float v[8];
+#pragma unroll
+				for (int i = 0; i < 8; i++) {
+					float y = float(int(r[24 + i]));
+					y = fmaf(y, 256.0f, float(int(r[16 + i])));
+					y = fmaf(y, 256.0f, float(int(r[8 + i])));
+					y = fmaf(y, 256.0f, float(int(r[i])));
+					v[i] = (y * rsv[i]) * sc;
+				}
+				if (a.top1) {
+					// Per token the largest value over the warp's 32 columns, the lowest column on equal values; NaN and -inf
+					// never win. Lane i keeps token i's; only a key above the recorded one goes to the atomic.
+					unsigned long long key = 0ull;
+#pragma unroll
+					for (int i = 0; i < 8; i++) {
+						const uint32_t b = __float_as_uint(v[i]);
+						const uint32_t ord = (v[i] > -INFINITY) ? ((b & 0x80000000u) ? ~b : (b | 0x80000000u)) : 0u;
+						const uint32_t m = warp_umax(ord);
+						const int src = __ffs(__ballot_sync(0xffffffffu, ord == m)) - 1;
+						if (lane == i && m)
+							key = (static_cast<unsigned long long>(m) << 32) | (0xFFFFFFFFu - uint32_t(a.top1_col0 + t.n0 + quad * 32 + src));
+					}
+					if (lane < 8 && tok + lane < a.M && key > *reinterpret_cast<volatile unsigned long long *>(a.top1 + tok + lane))
+						atomicMax(a.top1 + tok + lane, key);
+					return;
+				}
+				float *p = dst + size_t(tok) * ld;
+				if (tok + 8 <= a.M) {
+#pragma unroll
+					for (int i = 0; i < 8; i++, p += ld) *p = v[i];
+				} else {
+#pragma unroll
+					for (int i = 0; i < 7; i++, p += ld)
+						if (tok + i < a.M) *p = v[i];
+				}
+			};
+			if (!tc_wait(&acc_full[it & 1], (it >> 1) & 1, a.err)) { s_fail = 1; break; }
+			tc_fence_after();
+			uint32_t ra[32], rb[32];
+			float4 qa[2], qb[2];
+			if (sub < t.ng) request(sub, ra, qa);
+#pragma unroll 1
+			for (int g = sub; g < t.ng; g += 4) {
+				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+				if (g + 2 < t.ng) request(g + 2, rb, qb);
+				finish(g, ra, qa);
+				if (g + 2 < t.ng) {
+					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+					if (g + 4 < t.ng) request(g + 4, ra, qa);
+					finish(g + 2, rb, qb);
+				}
+			}
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) mbar_arrive(&acc_free[it & 1]);
+		}
+	}
+	// ---------------------------------------------------------------- teardown
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 0 && lane == 0 && *(volatile int *)&s_fail) {
+		// a wait ran out: every load that was issued must land before the shared memory is given up
+		const int n = *(volatile int *)&s_issued;
+		for (int c = max(0, n - I8_NST); c < n; c++) {
+			int spins = 0;
+			while (!mbar_try_wait(&full_bar[c % I8_NST], (c / I8_NST) & 1) && ++spins < TC_SPIN_CAP) {
+			}
+		}
+	}
+	if (warp == 1) {
+		if (*(volatile int *)&s_fail && lane == 0) {  // let the MMAs in flight finish before the TMEM goes away
+			int spins = 0;
+			while (!mbar_try_wait(&drain_bar, 0) && ++spins < TC_SPIN_CAP) {
+			}
+		}
+		__syncwarp();
+		tc_fence_after();
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+	}
+}
+
+}  // namespace tg

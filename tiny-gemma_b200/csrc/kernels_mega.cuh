@@ -173,6 +173,11 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 	    "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(pol)
 	    : "memory");
 }
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+	asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+	             "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+	             : "memory");
+}
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {

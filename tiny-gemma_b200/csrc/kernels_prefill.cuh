@@ -138,6 +138,8 @@ struct ReduceGroups {
 	int ldc[3];
 };
 __global__ void qgemm_splitk_reduce_groups_kernel(ReduceGroups g, const float *partial, int M, int N, int nsplit) {
+	pdl_trigger();
+	pdl_wait();
 	size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
 	if (i >= size_t(M) * N) return;
 	float s = 0.0f;

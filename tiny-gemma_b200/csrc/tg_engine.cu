@@ -19,7 +19,7 @@
 #include "kernels_decode.cuh"
 #include "kernels_mega.cuh"
 #include "kernels_persist.cuh"
-#include "kernels_gemm_tc.cuh"
+#include "kernels_gemm_i8.cuh"
 #include "kernels_attn_tc.cuh"
 #include "kernels_prefill.cuh"
 #include "kernels_sampler.cuh"
@@ -105,6 +105,7 @@ struct QW {
 	const float *s = nullptr;
 	int K = 0, N = 0;
 	int ld = 0;  // bytes between rows when the matrix is a column slice of a wider one; 0: N
+	const CUtensorMap *map = nullptr;  // the GEMM's tensor map of the matrix, where its owner keeps one
 };
 
 struct LayerW {
@@ -133,6 +134,7 @@ struct tg_model {
 	const float *wte_s = nullptr, *final_norm = nullptr;
 	std::vector<LayerW> layers;
 	QW lm_head;
+	std::vector<CUtensorMap> maps;  // the GEMM's tensor maps of all matrices (QW::map points in here)
 	float *rope[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [is_local][cos,sin]
 	int rope_npos[2] = {0, 0};
 	float *gelu = nullptr;
@@ -376,19 +378,13 @@ MvcPlan mvc_plan(int K, int N, int dev) {
 }  // namespace
 
 // ------------------------------------------------------------- prefill
-// Tensor-core GEMM (kernels_gemm_tc.cuh): activations are split into three bf16 terms and packed
-// tile by tile once per distinct A (pack_activations), then any number of weight matrices with
-// the same K can be multiplied against that packing (launch_gemm_tc).
+// Tensor-core GEMM (kernels_gemm_i8.cuh): the activations are packed as digits once per distinct A (pack_activations or
+// a kernel that packs its own output), then any number of weight matrices with the same K can be multiplied against them.
 struct TcScratch {
-	__nv_bfloat16 *apack = nullptr;
-	size_t apack_bytes = 0;
-	float *partial = nullptr;  // split-K partial sums
+	uint8_t *x = nullptr;  // digits, and behind them the row scales of the matrix packed last
+	size_t x_bytes = 0;
+	float *partial = nullptr;  // K-split partial sums
 	size_t partial_floats = 0;
-	unsigned *tickets = nullptr;  // [TC_TICKETS] zeros: enables the in-kernel split-K reduction for shallow splits
-	int fused_max_split = 3;      // deeper splits use the reduce kernel: one CTA re-reading a whole tile of every split is
-	                              // latency-bound (measured: 9-way splits reduced in-kernel doubled the batched step time)
-	int max_split = 9;            // cap on the K-split depth: deeper splits (one or two K-blocks per CTA) cost more in partial-sum
-	                              // traffic and per-CTA fixed cost than they gain in parallelism (TG_GEMM_MAX_SPLIT overrides)
 	unsigned long long *top1 = nullptr;  // set for one launch: row-wise (max, column) keys instead of C (unsplit K)
 	int top1_col0 = 0;
 	int *err = nullptr;
@@ -810,8 +806,8 @@ PFN_encodeTiled get_encode_fn() {
 	return fn;
 }
 
-// 2-D uint8 map over a row-major [K, N] int8 matrix; box = TN bytes x box_rows rows, no swizzle
-int make_tmap(CUtensorMap *out, const int8_t *base, int K, int N, int TN, int box_rows, int ld = 0) {
+// 2-D uint8 map over a row-major [K, N] int8 matrix; box = TN bytes x box_rows rows
+int make_tmap(CUtensorMap *out, const int8_t *base, int K, int N, int TN, int box_rows, int ld = 0, bool swizzle128 = false) {
 	PFN_encodeTiled enc = get_encode_fn();
 	if (!enc) return fail(TG_ECUDA, "cuTensorMapEncodeTiled entry point not available");
 	cuuint64_t gdim[2] = {cuuint64_t(N), cuuint64_t(K)};
@@ -819,7 +815,7 @@ int make_tmap(CUtensorMap *out, const int8_t *base, int K, int N, int TN, int bo
 	cuuint32_t box[2] = {cuuint32_t(TN), cuuint32_t(box_rows)};
 	cuuint32_t estr[2] = {1, 1};
 	CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(base), gdim, gstride, box, estr,
-	                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+	                 CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
 	                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 	if (r != CUDA_SUCCESS) return fail(TG_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
 	return TG_OK;
@@ -1517,33 +1513,42 @@ int ensure_log(tg_state *s, int steps) {
 }
 
 
-// K-split of the tensor-core GEMM: enough CTAs to fill the GPU, accumulation chains of at most 24
-// K-blocks (768 rows) for accuracy, as far as the partial-sum buffer allows.
-constexpr size_t TC_TICKETS = 4096;
-// ctas = CTAs of one split (column tiles x row-tile groups of the chosen tile shape)
-int tc_pick_split(int ctas, int M, int K, int N, size_t partial_floats, int max_split) {
-	const int k_blocks = K / TC_BK;
-	// accumulation chains are kept to <= 24 K-blocks; a CTA keeps two accumulators per tile (first / second half of
-	// its K range), so it can take up to 48 K-blocks
-	// split only while every split still fits one wave (ctas * splits <= SMs): a second, partly filled wave
-	// costs as much as the split saves
-	const int fit = std::max(1, env_int("TG_GEMM_SPLIT_CEIL", 0) ? (g_num_sms + ctas - 1) / ctas : g_num_sms / ctas);
-	const int need = (k_blocks + 47) / 48;
-	// the largest divisor of the K-block count that still fits one wave; if the chain limit asks for more,
-	// the smallest divisor that satisfies it
-	int best = 1;
-	for (int ns = 1; ns <= std::min(k_blocks, max_split); ns++) {
-		if (k_blocks % ns) continue;
-		if (ns > 1 && size_t(ns) * M * N > partial_floats) break;
-		if (ns > fit && best >= need) break;
-		best = ns;
+// ------------------------------------------------------------- tensor-core GEMM
+int i8_groups(int M) { return (M + 7) / 8; }
+size_t i8_pack_bytes(int M, int K) { return size_t(i8_groups(M)) * 8 * (size_t(4) * K + 4); }
+float *i8_rowscale(const TcScratch &sc, int M, int K) { return reinterpret_cast<float *>(sc.x + size_t(i8_groups(M)) * 8 * 4 * K); }
+
+// Tokens per tile and K-split of one GEMM launch, by an estimate in clocks of an SM: rounds of tiles per CTA x (stages x
+// the slowest of MMAs, operand bytes and the issuing threads + what a tile change costs) + what the consumer of the
+// partial sums reads. Measured: an MMA of N columns takes max(N / 2, 68) clk (below N = 128 it waits for its 4 KB of W),
+// with all SMs loading an operand byte takes 1/66 clk, and a stage costs its issuing threads ~280 clk.
+struct I8Plan {
+	int tg, tok_tiles, col_tiles, nsplit;
+};
+I8Plan i8_plan(int M, int K, int ntot, size_t partial_floats, int max_split, bool raw) {
+	I8Plan best{1, 1, 1, 1};
+	double best_cost = 1e30;
+	const int groups = i8_groups(M), stages = K / I8_SK, col_tiles = ntot / 128;
+	const int want_split = env_int("TG_GEMM_SPLIT", 0);  // (experiments: fix the split)
+	const int tiles_min = (groups + I8_TG - 1) / I8_TG;
+	for (int n = tiles_min; n <= std::min(groups, tiles_min + 2); n++) {
+		const int tg = (groups + n - 1) / n, tok_tiles = (groups + tg - 1) / tg;
+		const double mma = 4.0 * std::max(16.0 * tg, 68.0), load = (I8_W_BYTES + 2.0 * tg * I8_GROUP_BYTES) / 66.0;
+		const double per_stage = std::max(std::max(mma, load), 280.0);
+		for (int ns = 1; ns <= std::min(max_split, stages); ns++) {
+			if (want_split && ns != std::min(want_split, std::min(max_split, stages))) continue;
+			if ((ns > 1 || raw) && size_t(ns) * M * ntot > partial_floats) break;
+			const long tiles = long(tok_tiles) * col_tiles * ns, rounds = (tiles + g_num_sms - 1) / g_num_sms;
+			double cost = double(rounds) * ((stages + ns - 1) / ns * per_stage + 150.0) + tg * 330.0;
+			cost += double(raw ? ns - 1 : (ns > 1 ? ns + 1 : 0)) * M * ntot * 4.0 / 2500.0;  // partial sums read again, 2.5 KB a clock
+			if (!raw && ns > 1) cost += 4000.0;                                               // a launch more
+			if (cost < best_cost) {
+				best_cost = cost;
+				best = I8Plan{tg, tok_tiles, col_tiles, ns};
+			}
+		}
 	}
 	return best;
-}
-
-size_t tc_pack_bytes(int M, int K) {
-	const size_t m_tiles = (size_t(M) + TC_BM - 1) / TC_BM;
-	return 3 * m_tiles * size_t(K / TC_BK) * TC_TILE_BYTES;
 }
 
 // packed operands of the tensor-core prefill attention for one prompt of S tokens: Q (4 S rows), K (S rows), V
@@ -1564,103 +1569,134 @@ AttnTcPlan attn_tc_plan(int S) {
 }
 
 int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStream_t st) {
-	if (tc_pack_bytes(M, K) > sc.apack_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
-	const int m_tiles = (M + TC_BM - 1) / TC_BM;
-	const size_t chunks = size_t(m_tiles) * TC_BM * (K / 8);
-	const unsigned grid = unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16));
-	launch_k(split_pack_kernel, dim3(grid), dim3(256), 0, st, A, sc.apack, M, K, m_tiles);
+	if (i8_pack_bytes(M, K) > sc.x_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
+	const int groups = i8_groups(M);
+	float *rs = i8_rowscale(sc, M, K);
+	if (K <= 1152)
+		launch_k(i8_pack_kernel<96, 3>, dim3(groups * 8), dim3(96), 0, st, A, sc.x, rs, M, K, groups);
+	else if (K <= 2048)
+		launch_k(i8_pack_kernel<256, 2>, dim3(groups * 8), dim3(256), 0, st, A, sc.x, rs, M, K, groups);
+	else
+		launch_k(i8_pack_kernel<256, 7>, dim3(groups * 8), dim3(256), 0, st, A, sc.x, rs, M, K, groups);
 	count_launch();
-	return check_launch("split_pack");
+	return check_launch("i8_pack");
 }
 
+// h += norm(partial sums), then the packed norm of h for the next GEMM (resnorm_i8_kernel)
+int launch_resnorm(float *h, const float *t, const float *w_post, const float *w_pre, int M, int dim, int nsplit, const float *tscale,
+                   const TcScratch &sc, cudaStream_t st) {
+	const int groups = i8_groups(M);
+	float *rs = i8_rowscale(sc, M, dim);
+	if (M < 1024)
+		launch_k(resnorm_i8_kernel<288, 2>, dim3(groups * 8), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	else if (dim <= 640)
+		launch_k(resnorm_i8_kernel<32, 5>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	else if (dim <= 1152)
+		launch_k(resnorm_i8_kernel<32, 9>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	else
+		launch_k(resnorm_i8_kernel<32, 16>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	count_launch();
+	return check_launch("resnorm");
+}
+
+int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, const float *su, const float *sg, const TcScratch &sc, cudaStream_t st) {
+	const int groups = i8_groups(M);
+	float *rs = i8_rowscale(sc, M, I);
+	if (I <= 2048)
+		launch_k(geglu_i8_kernel<2>, dim3(groups * 8), dim3(256), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
+	else
+		launch_k(geglu_i8_kernel<7>, dim3(groups * 8), dim3(256), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
+	count_launch();
+	return check_launch("geglu");
+}
+
+int make_gemm_map(CUtensorMap *out, const QW &w) { return make_tmap(out, w.q, w.K, w.N, 128, I8_SK, w.ld, true); }
+
 // One launch for up to three weight matrices with the same K that multiply the same packed A
-// (q|k|v, up|gate): more column tiles per launch, one split-K reduce instead of three.
+// (q|k|v, up|gate): more column tiles per launch.
 // raw_nsplit != null: the kernel leaves raw partial sums in sc.partial ([nsplit][M][sum of N]) for a consumer
 // kernel that adds the splits and scales itself; *raw_nsplit receives the split count, no reduce is launched.
 int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const int *ldcs, int M, const TcScratch &sc,
-                         cudaStream_t st, int max_split = 1 << 30, int *raw_nsplit = nullptr) {
+                         cudaStream_t st, int max_split = 16, int *raw_nsplit = nullptr) {
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_tc_kernel<2, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<2, 128>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_tc_kernel<1, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcShape<1, 256>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		configured[dev] = true;
 	}
-	// tile shape: beyond one row tile the wide shape (one row tile x 256 columns) wins: a 256-column MMA
-	// keeps the tensor pipe busier than two of 128 and every fetched A tile is used twice as often
-	const int m_tiles_all = (M + TC_BM - 1) / TC_BM;
-	const bool wide = M >= env_int("TG_GEMM_WIDE_MIN_M", 129);
-	const int bn = wide ? 256 : 128, mt_cta = wide ? 1 : 2;
-	CUtensorMap wmap[3];
-	GemmTcArgs a{};
-	ReduceGroups rg{};
-	int ntot = 0, tiles = 0;
 	const int K = ws[0]->K;
+	int ntot = 0;
+	for (int g = 0; g < ng; g++) {
+		if (ws[g]->K != K) return fail(TG_ESHAPE, "grouped GEMM: the matrices must share K");
+		ntot += ws[g]->N;
+	}
+	const I8Plan pl = i8_plan(M, K, ntot, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
+	CUtensorMap wmap[3];
+	GemmI8Args a{};
+	ReduceGroups rg{};
+	int col0 = 0, tiles = 0;
 	for (int g = 0; g < 3; g++) {
 		const int gg = std::min(g, ng - 1);  // unused slots repeat the last matrix (never selected)
-		if (ws[gg]->K != K) return fail(TG_ESHAPE, "grouped GEMM: the matrices must share K");
-		TG_TRY(make_tmap(&wmap[g], ws[gg]->q, K, ws[gg]->N, bn, TC_BK, ws[gg]->ld));
+		if (ws[gg]->map)
+			wmap[g] = *ws[gg]->map;
+		else if (g < ng)
+			TG_TRY(make_gemm_map(&wmap[g], *ws[gg]));
+		else
+			wmap[g] = wmap[gg];
 		if (g < ng) {
-			a.col0[g] = ntot;
-			a.ncols[g] = ws[g]->N;
-			a.scales[g] = ws[g]->s;
-			a.C[g] = Cs[g];
-			a.ldc[g] = (ldcs && ldcs[g] > 0) ? ldcs[g] : ws[g]->N;
-			ntot += ws[g]->N;
-			tiles += (ws[g]->N + bn - 1) / bn;
+			a.col0[g] = col0;
+			col0 += ws[g]->N;
+			tiles += ws[g]->N / 128;
 			a.tile_end[g] = tiles;
-			rg.col0[g] = a.col0[g];
-			rg.scales[g] = a.scales[g];
-			rg.C[g] = a.C[g];
-			rg.ldc[g] = a.ldc[g];
 		} else {
-			a.col0[g] = ntot;
+			a.col0[g] = col0;
 			a.tile_end[g] = INT_MAX;
-			a.ncols[g] = 0;
-			a.scales[g] = a.scales[ng - 1];
-			a.C[g] = a.C[ng - 1];
-			a.ldc[g] = a.ldc[ng - 1];
 		}
+		a.scales[g] = ws[gg]->s;
+		a.C[g] = Cs ? Cs[gg] : nullptr;
+		a.ldc[g] = (ldcs && ldcs[gg] > 0) ? ldcs[gg] : ws[gg]->N;
+		rg.col0[g] = g < ng ? a.col0[g] : INT_MAX;
+		rg.scales[g] = a.scales[g];
+		rg.C[g] = a.C[g];
+		rg.ldc[g] = a.ldc[g];
 	}
 	rg.ngroups = ng;
-	rg.col0[ng] = ntot;
-	for (int g = ng + 1; g < 4; g++) rg.col0[g] = INT_MAX;
-	a.ngroups = ng;
-	a.apack = sc.apack;
+	rg.col0[3] = INT_MAX;
+	a.x = sc.x;
+	a.rowscale = i8_rowscale(sc, M, K);
+	a.groups = i8_groups(M);
+	a.tg = pl.tg;
+	a.tok_tiles = pl.tok_tiles;
+	a.col_tiles = pl.col_tiles;
+	a.tiles = pl.tok_tiles * pl.col_tiles * pl.nsplit;
+	// matrices that stay in the L2 are swept once per token tile; the vocabulary matrix is read once for all token tiles
+	a.n_fast = size_t(ntot) * K <= (size_t(48) << 20);
+	a.w_stream = pl.tok_tiles <= 4;
 	a.M = M;
 	a.N = ntot;
 	a.K = K;
-	a.m_tiles = m_tiles_all;
-	a.nsplit = tc_pick_split(tiles * ((m_tiles_all + mt_cta - 1) / mt_cta), M, K, ntot, sc.partial_floats, std::min(max_split, env_int("TG_GEMM_MAX_SPLIT", sc.max_split)));
+	a.nsplit = pl.nsplit;
 	a.partial = sc.partial;
+	a.raw = raw_nsplit ? 1 : 0;
 	a.err = sc.err;
 	a.top1 = sc.top1;
 	a.top1_col0 = sc.top1_col0;
-	if (a.top1 && (a.nsplit != 1 || raw_nsplit)) return fail(TG_EINVAL, "top-1 epilogue needs an unsplit K");
-	dim3 grid(tiles, (a.m_tiles + mt_cta - 1) / mt_cta, a.nsplit);
-	const bool fused = !raw_nsplit && sc.tickets && a.nsplit > 1 && a.nsplit <= sc.fused_max_split && size_t(grid.x) * grid.y <= TC_TICKETS;
-	a.tickets = fused ? sc.tickets : nullptr;
-	a.raw = raw_nsplit ? 1 : 0;
-	a.halves = env_int("TG_GEMM_HALVES", 2);
 	if (raw_nsplit) {
 		if (size_t(a.nsplit) * M * ntot > sc.partial_floats) return fail(TG_ENOMEM, "tensor-core GEMM partial-sum scratch too small");
 		*raw_nsplit = a.nsplit;
 	}
-	if (wide)
-		launch_k(qgemm_tc_kernel<1, 256>, grid, dim3(TC_THREADS), TcShape<1, 256>::SMEM, st, wmap[0], wmap[1], wmap[2], a);
-	else
-		launch_k(qgemm_tc_kernel<2, 128>, grid, dim3(TC_THREADS), TcShape<2, 128>::SMEM, st, wmap[0], wmap[1], wmap[2], a);
+	launch_k(qgemm_i8_kernel, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], a);
 	count_launch();
-	TG_TRY(check_launch("qgemm_tc"));
-	if (a.nsplit > 1 && !fused && !raw_nsplit) {
+	TG_TRY(check_launch("qgemm_i8"));
+	if (a.nsplit > 1 && !raw_nsplit) {
 		const size_t n = size_t(M) * ntot;
-		qgemm_splitk_reduce_groups_kernel<<<unsigned((n + 255) / 256), 256, 0, st>>>(rg, sc.partial, M, ntot, a.nsplit);
+		launch_k(qgemm_splitk_reduce_groups_kernel, dim3(unsigned((n + 255) / 256)), dim3(256), 0, st, rg, (const float *)sc.partial, M, ntot, a.nsplit);
 		count_launch();
 		TG_TRY(check_launch("qgemm_reduce"));
 	}
 	return TG_OK;
 }
-int launch_gemm_tc(float *C, const QW &w, int M, const TcScratch &sc, cudaStream_t st, int ldc = 0, int max_split = 1 << 30) {
+int launch_gemm_tc(float *C, const QW &w, int M, const TcScratch &sc, cudaStream_t st, int ldc = 0, int max_split = 16) {
 	float *Cs[1] = {C};
 	const QW *ws[1] = {&w};
 	const int ldcs[1] = {ldc};
@@ -1676,13 +1712,10 @@ int batched_setup(tg_state *s) {
 	const int B = s->B, D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab, qd = c.n_head * c.head_dim;
 	TG_CUDA(cudaMalloc(&s->bx, size_t(B) * D * 4));
 	TG_CUDA(cudaMalloc(&s->bup, size_t(B) * I * 4));
-	s->btc.apack_bytes = tc_pack_bytes(B, std::max(I, std::max(D, qd)));
-	TG_CUDA(cudaMalloc(&s->btc.apack, s->btc.apack_bytes));
+	s->btc.x_bytes = i8_pack_bytes(B, std::max(I, std::max(D, qd)));
+	TG_CUDA(cudaMalloc(&s->btc.x, s->btc.x_bytes));
 	s->btc.partial_floats = std::min(size_t(24) * B * std::max(I, qd), size_t(1) << 28);
 	TG_CUDA(cudaMalloc(&s->btc.partial, s->btc.partial_floats * 4));
-	TG_CUDA(cudaMalloc(&s->btc.tickets, TC_TICKETS * sizeof(unsigned)));
-	TG_CUDA(cudaMemset(s->btc.tickets, 0, TC_TICKETS * sizeof(unsigned)));
-	s->btc.max_split = env_int("TG_BATCH_MAX_SPLIT", 9);
 	s->btc.err = s->err_flag;
 	(void)V;
 	s->batched_ok = true;
@@ -1715,17 +1748,15 @@ int enqueue_decode_batched(tg_state *s, bool with_lm_head) {
 	ea.sqrtD = float(std::sqrt(double(D)));
 	launch_k(embed_decode_kernel, dim3(B), dim3(256), 0, st, ea);
 	count_launch();
-	const int m_tiles = (B + TC_BM - 1) / TC_BM;
-	// t: finished matrix (nsplit 0) or the raw partial sums of the GEMM before (nsplit >= 1, column scales tscale)
-	auto resnorm_pack = [&](const float *t, const float *w_post, const float *w_pre, int nsplit, const float *tscale) {
-		launch_k(resnorm_pack_kernel<256>, dim3(m_tiles * TC_BM), dim3(256), 0, st, h, t, w_post, w_pre, s->btc.apack, B, D, m_tiles, nsplit, D, tscale);
-		count_launch();
+	// t: the raw partial sums of the GEMM before (column scales tscale)
+	auto resnorm_pack = [&](const float *t, const float *w_post, const float *w_pre, int nsplit, const float *tscale) -> int {
+		return launch_resnorm(h, t, w_post, w_pre, B, D, nsplit, tscale, s->btc, st);
 	};
 	auto gemm_raw = [&](int ng, const QW *const *ws, int *ns) -> int {
 		float *Cs[3] = {nullptr, nullptr, nullptr};
-		return launch_gemm_tc_group(ng, Cs, ws, nullptr, B, s->btc, st, 1 << 30, ns);
+		return launch_gemm_tc_group(ng, Cs, ws, nullptr, B, s->btc, st, 16, ns);
 	};
-	resnorm_pack(nullptr, nullptr, m->layers[0].attn_pre, 0, nullptr);
+	TG_TRY(resnorm_pack(nullptr, nullptr, m->layers[0].attn_pre, 0, nullptr));
 	for (int l = 0; l < c.n_layers; l++) {
 		const LayerW &w = m->layers[l];
 		int ns_qkv = 0;
@@ -1766,18 +1797,17 @@ int enqueue_decode_batched(tg_state *s, bool with_lm_head) {
 			const QW *ws[1] = {&w.O};
 			TG_TRY(gemm_raw(1, ws, &ns));
 		}
-		resnorm_pack(s->btc.partial, w.attn_post, w.mlp_pre, ns, w.O.s);
+		TG_TRY(resnorm_pack(s->btc.partial, w.attn_post, w.mlp_pre, ns, w.O.s));
 		{
 			const QW *ws[2] = {&w.U, &w.G};
 			TG_TRY(gemm_raw(2, ws, &ns));
 		}
-		launch_k(geglu_pack_kernel, dim3(unsigned((size_t(m_tiles) * TC_BM * (I / 8) + 255) / 256)), dim3(256), 0, st, (const float *)nullptr, (const float *)s->btc.partial, s->btc.apack, B, I, m_tiles, lut, ns, w.U.s, w.G.s);
-		count_launch();
+		TG_TRY(launch_geglu(s->btc.partial, B, I, lut, ns, w.U.s, w.G.s, s->btc, st));
 		{
 			const QW *ws[1] = {&w.Dn};
 			TG_TRY(gemm_raw(1, ws, &ns));
 		}
-		resnorm_pack(s->btc.partial, w.mlp_post, l + 1 < c.n_layers ? m->layers[l + 1].attn_pre : nullptr, ns, w.Dn.s);
+		TG_TRY(resnorm_pack(s->btc.partial, w.mlp_post, l + 1 < c.n_layers ? m->layers[l + 1].attn_pre : nullptr, ns, w.Dn.s));
 		TG_TRY(check_launch("batched layer"));
 	}
 	launch_k(rmsnorm_rows_kernel, dim3(B), dim3(256), 0, st, s->xnorm, (const float *)h, m->final_norm, (const float *)nullptr, D);
@@ -1842,10 +1872,11 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	const bool use_tc = env_int("TG_GEMM_TC", 1) != 0;
 	TcScratch tc;
 	if (use_tc) {
-		tc.apack = reinterpret_cast<__nv_bfloat16 *>(p);
-		tc.apack_bytes = tc_pack_bytes(S, std::max(I, std::max(D, qd)));
+		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
+		tc.x = reinterpret_cast<uint8_t *>(p);
+		tc.x_bytes = i8_pack_bytes(S, std::max(I, std::max(D, qd)));
 		tc.err = s->err_flag;
-		p += (tc.apack_bytes + 3) / 4;
+		p += (tc.x_bytes + 3) / 4;
 	}
 	// long prompts: attention on the tensor cores, from packed copies of q, k and v, one sequence after the other
 	// (from 640 tokens on: below, the three packing launches cost what the tensor cores save)
@@ -1875,23 +1906,17 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	         float(std::sqrt(double(D))), s->err_flag);
 	count_launch();
 	TG_TRY(check_launch("embed_prefill"));
-	const int m_tiles = (S + TC_BM - 1) / TC_BM;
 	// Tensor-core path: the norms are fused with the operand packing of the GEMM that follows them
-	// (resnorm_pack_kernel, geglu_pack_kernel), so a layer is 7 GEMMs (+ their split-K reduces) and 6 other launches.
-	auto resnorm_pack = [&](const float *t, const float *w_post, const float *w_pre, int nsplit, const float *tscale) {
-		if (S >= env_int("TG_RESNORM_NARROW_MIN", 1024))
-			launch_k(resnorm_pack_kernel<128>, dim3(m_tiles * TC_BM), dim3(128), 0, st, h, t, w_post, w_pre, tc.apack, S, D, m_tiles, nsplit, D, tscale);
-		else
-			launch_k(resnorm_pack_kernel<256>, dim3(m_tiles * TC_BM), dim3(256), 0, st, h, t, w_post, w_pre, tc.apack, S, D, m_tiles, nsplit, D, tscale);
-		count_launch();
+	// (resnorm_i8_kernel, geglu_i8_kernel).
+	auto resnorm_pack = [&](const float *t, const float *w_post, const float *w_pre, int nsplit, const float *tscale) -> int {
+		return launch_resnorm(h, t, w_post, w_pre, S, D, nsplit, tscale, tc, st);
 	};
 	auto gemm_raw = [&](int ng, const QW *const *ws, int *ns) -> int {
 		float *Cs[3] = {nullptr, nullptr, nullptr};
-		return launch_gemm_tc_group(ng, Cs, ws, nullptr, S, tc, st, 1 << 30, ns);
+		return launch_gemm_tc_group(ng, Cs, ws, nullptr, S, tc, st, 16, ns);
 	};
 	if (use_tc) {
-		if (tc_pack_bytes(S, std::max(I, std::max(D, qd))) > tc.apack_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
-		resnorm_pack(nullptr, nullptr, m->layers[0].attn_pre, 0, nullptr);
+		TG_TRY(resnorm_pack(nullptr, nullptr, m->layers[0].attn_pre, 0, nullptr));
 	}
 	for (int l = 0; l < c.n_layers; l++) {
 		const LayerW &w = m->layers[l];
@@ -1969,19 +1994,17 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 				const QW *ws[1] = {&w.O};
 				TG_TRY(gemm_raw(1, ws, &ns));
 			}
-			resnorm_pack(tc.partial, w.attn_post, w.mlp_pre, ns, w.O.s);
+			TG_TRY(resnorm_pack(tc.partial, w.attn_post, w.mlp_pre, ns, w.O.s));
 			{
 				const QW *ws[2] = {&w.U, &w.G};
 				TG_TRY(gemm_raw(2, ws, &ns));
 			}
-			launch_k(geglu_pack_kernel, dim3(unsigned(std::min<size_t>((size_t(m_tiles) * TC_BM * (I / 8) + 255) / 256, 65535 * 16))), dim3(256), 0, st,
-			         (const float *)nullptr, (const float *)tc.partial, tc.apack, S, I, m_tiles, lut, ns, w.U.s, w.G.s);
-			count_launch();
+			TG_TRY(launch_geglu(tc.partial, S, I, lut, ns, w.U.s, w.G.s, tc, st));
 			{
 				const QW *ws[1] = {&w.Dn};
 				TG_TRY(gemm_raw(1, ws, &ns));
 			}
-			resnorm_pack(tc.partial, w.mlp_post, l + 1 < c.n_layers ? m->layers[l + 1].attn_pre : nullptr, ns, w.Dn.s);
+			TG_TRY(resnorm_pack(tc.partial, w.mlp_post, l + 1 < c.n_layers ? m->layers[l + 1].attn_pre : nullptr, ns, w.Dn.s));
 		} else {
 			TG_TRY(gemm(tt, ao, w.O, true));
 			rmsnorm_rows_kernel<<<S, 256, 0, st>>>(h, tt, w.attn_post, h, D);
@@ -2093,6 +2116,14 @@ int tg_model_create(const tg_config *cfg, int device, tg_model **out) {
 	}
 	cudaMemset(m->blob, 0, m->nbytes);
 	bind_model(m);
+	{  // the GEMM's tensor maps: encoded once here instead of at every launch
+		std::vector<QW *> ws{&m->lm_head};
+		for (LayerW &w : m->layers)
+			for (QW *q : {&w.Q, &w.K, &w.V, &w.O, &w.U, &w.G, &w.Dn}) ws.push_back(q);
+		m->maps.resize(ws.size());
+		for (size_t i = 0; i < ws.size(); i++)
+			if (make_gemm_map(&m->maps[i], *ws[i]) == TG_OK) ws[i]->map = &m->maps[i];
+	}
 	*out = m;
 	return TG_OK;
 }
@@ -2304,9 +2335,8 @@ int tg_state_free(tg_state *s) {
 	cudaFree(s->pf_ids);
 	cudaFree(s->bx);
 	cudaFree(s->bup);
-	cudaFree(s->btc.apack);
+	cudaFree(s->btc.x);
 	cudaFree(s->btc.partial);
-	cudaFree(s->btc.tickets);
 	cudaFree(s->d_tmaps);
 	cudaFree(s->d_layers);
 	cudaFree(s->mg_ll);
@@ -2379,7 +2409,7 @@ int tg_prefill(tg_state *s, const int *ids, int S, float *logits_host) {
 	size_t part = std::max(size_t(4) * R * D, size_t(1) << 22);  // split-K scratch
 	part = std::max(part, std::min(size_t(24) * R * std::max(I, qd), size_t(1) << 28));  // tensor-core GEMM partial sums (<= 1 GiB)
 	need += part;
-	need += (tc_pack_bytes(int(R), std::max(I, std::max(D, qd))) + 3) / 4 + 64;
+	need += (i8_pack_bytes(int(R), std::max(I, std::max(D, qd))) + 3) / 4 + 512;
 	need += (attn_tc_plan(S).total() + 3) / 4 + 512;  // packed q, k, v of the tensor-core attention (long prompts)
 	if (need > s->pf_floats) {
 		if (s->pf) cudaFree(s->pf);
@@ -2712,13 +2742,13 @@ int tg_dev_lm_head_top1(tg_model *m, const float *hidden_dev, int M, int col0, i
 	static Top1Scratch scr[TG_MAX_DEVICES];
 	const int slot = current_device_slot();
 	Top1Scratch &t = scr[slot];
-	const size_t need = tc_pack_bytes(M, D);
-	if (need > t.tc.apack_bytes) {
-		if (t.tc.apack) cudaFree(t.tc.apack);
-		t.tc.apack = nullptr;
-		t.tc.apack_bytes = 0;
-		TG_CUDA(cudaMalloc(&t.tc.apack, need));
-		t.tc.apack_bytes = need;
+	const size_t need = i8_pack_bytes(M, D);
+	if (need > t.tc.x_bytes) {
+		if (t.tc.x) cudaFree(t.tc.x);
+		t.tc.x = nullptr;
+		t.tc.x_bytes = 0;
+		TG_CUDA(cudaMalloc(&t.tc.x, need));
+		t.tc.x_bytes = need;
 	}
 	if (M > t.keys_cap) {
 		if (t.keys) cudaFree(t.keys);
@@ -2909,13 +2939,13 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 	if (env_int("TG_GEMM_TC", 1)) {
 		// tensor-core path: packed bf16 activations + an error word, per device, grown on demand
 		static TcScratch tc[64];
-		const size_t need = tc_pack_bytes(M, K);
-		if (need > tc[dev].apack_bytes) {
-			if (tc[dev].apack) cudaFree(tc[dev].apack);
-			tc[dev].apack = nullptr;
-			tc[dev].apack_bytes = 0;
-			TG_CUDA(cudaMalloc(&tc[dev].apack, need));
-			tc[dev].apack_bytes = need;
+		const size_t need = i8_pack_bytes(M, K);
+		if (need > tc[dev].x_bytes) {
+			if (tc[dev].x) cudaFree(tc[dev].x);
+			tc[dev].x = nullptr;
+			tc[dev].x_bytes = 0;
+			TG_CUDA(cudaMalloc(&tc[dev].x, need));
+			tc[dev].x_bytes = need;
 		}
 		const size_t pneed = std::min(size_t(24) * M * N, size_t(1) << 28);
 		if (pneed > tc[dev].partial_floats) {
