@@ -33,42 +33,53 @@ __device__ __forceinline__ void emit_token(const SampleArgs &a, int b, int tok) 
 
 // ops::argmax_logits, reference ops.hpp:744-760: ascending scan with a strict
 // '>' — the lowest index wins ties, NaN never wins, -1 if nothing exceeds -inf.
-__global__ void __launch_bounds__(SM_THREADS) argmax_kernel(SampleArgs a) {
+// grid (V / SR_PART rounded up, rows): a row is 1 MB, which one CTA reads in ~35 us (a chain of dependent round trips)
+// and 32 CTAs in ~3. The CTAs of a row meet in a 64-bit key (larger value first, then the lower index); the one that
+// arrives last emits the token and leaves key and ticket zero for the next launch.
+constexpr int SR_THREADS = 256;
+constexpr int SR_PART = 8192;  // columns per CTA
+__global__ void __launch_bounds__(SR_THREADS) argmax_kernel(SampleArgs a, unsigned long long *keys, unsigned *tickets) {
 	pdl_trigger();
 	pdl_wait();
-	__shared__ float sv[SM_NWARPS];
-	__shared__ int si[SM_NWARPS];
-	const int b = blockIdx.x, tid = threadIdx.x;
+	__shared__ unsigned long long sk[SR_THREADS / 32];
+	const int b = blockIdx.y, tid = threadIdx.x;
 	const float *x = a.logits + size_t(b) * a.V;
+	float4 v[SR_PART / (4 * SR_THREADS)];
+#pragma unroll
+	for (int j = 0; j < SR_PART / (4 * SR_THREADS); j++) {
+		const int i = blockIdx.x * SR_PART + 4 * (tid + SR_THREADS * j);
+		v[j] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+		if (i < a.V) v[j] = __ldcg(reinterpret_cast<const float4 *>(x + i));
+	}
 	float best = -INFINITY;
 	int arg = -1;
-	for (int i = tid * 4; i < a.V; i += SM_THREADS * 4) {
-		float4 v = __ldcg(reinterpret_cast<const float4 *>(x + i));
-		if (v.x > best) { best = v.x; arg = i; }
-		if (v.y > best) { best = v.y; arg = i + 1; }
-		if (v.z > best) { best = v.z; arg = i + 2; }
-		if (v.w > best) { best = v.w; arg = i + 3; }
-	}
-	// (value desc, index asc); arg == -1 loses to any real index at equal value
-	auto better = [](float v1, int i1, float v2, int i2) {
-		if (v1 > v2) return true;
-		if (v1 < v2) return false;
-		if (i2 < 0) return i1 >= 0;
-		if (i1 < 0) return false;
-		return i1 < i2;
-	};
 #pragma unroll
-	for (int o = 16; o > 0; o >>= 1) {
-		float ov = __shfl_xor_sync(0xffffffffu, best, o);
-		int oi = __shfl_xor_sync(0xffffffffu, arg, o);
-		if (better(ov, oi, best, arg)) { best = ov; arg = oi; }
+	for (int j = 0; j < SR_PART / (4 * SR_THREADS); j++) {
+		const int i = blockIdx.x * SR_PART + 4 * (tid + SR_THREADS * j);
+		if (v[j].x > best) { best = v[j].x; arg = i; }
+		if (v[j].y > best) { best = v[j].y; arg = i + 1; }
+		if (v[j].z > best) { best = v[j].z; arg = i + 2; }
+		if (v[j].w > best) { best = v[j].w; arg = i + 3; }
 	}
-	if ((tid & 31) == 0) { sv[tid >> 5] = best; si[tid >> 5] = arg; }
+	unsigned long long key = 0ull;
+	if (arg >= 0) {
+		const uint32_t u = __float_as_uint(best == 0.0f ? 0.0f : best);  // (-0 and +0 are equal)
+		key = (static_cast<unsigned long long>((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32) | (0xFFFFFFFFu - uint32_t(arg));
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
+	if ((tid & 31) == 0) sk[tid >> 5] = key;
 	__syncthreads();
 	if (tid == 0) {
-		for (int w = 1; w < SM_NWARPS; w++)
-			if (better(sv[w], si[w], best, arg)) { best = sv[w]; arg = si[w]; }
-		emit_token(a, b, arg);
+		for (int w = 1; w < SR_THREADS / 32; w++) key = max(key, sk[w]);
+		if (key) atomicMax(keys + b, key);
+		__threadfence();
+		if (atomicAdd(tickets + b, 1u) == gridDim.x - 1) {
+			__threadfence();
+			const unsigned long long k = atomicExch(keys + b, 0ull);
+			tickets[b] = 0u;
+			emit_token(a, b, k ? int(0xFFFFFFFFu - uint32_t(k)) : -1);
+		}
 	}
 }
 
@@ -299,91 +310,212 @@ __device__ int cdf_cross_block(const float *p, int n, float *cum_io, float randf
 // Steps 1-5 are data-parallel. Step 6 must reproduce a *sequential* fp32 sum
 // (fp32 addition is not associative, and the crossing index depends on the
 // rounding): cdf_cross_block evaluates that chain exactly, in parallel, over
-// chunks that the whole CTA stages into shared memory.
+// chunks that a CTA stages into shared memory.
 constexpr int MP_CHUNK = 8192;
 
-__global__ void __launch_bounds__(SM_THREADS) minp_kernel(SampleArgs a) {
-	__shared__ float red[SM_NWARPS];
-	__shared__ float chunk[MP_CHUNK];
-	__shared__ int scratch[2 * SM_NWARPS + 8];
-	__shared__ float s_cum;
-	const int b = blockIdx.x, tid = threadIdx.x;
-	float *x = a.logits + size_t(b) * a.V;
-	float randf = 0.0f;
-	{
-		int rc = a.randf_count[b];
-		if (rc < a.randf_cap) randf = a.randf[size_t(rc) * a.B + b];
-	}
-	// (1)+(2)
+// Any number of rows, each spread over V / SR_PART CTAs: four kernels (row maximum; exponentials and segment sums;
+// scaling and segment maps; the walk). One CTA per row took ~1 ms for a row of 262144: four passes over 1 MB and
+// the whole chain of step 6, all latency. Step 6 here: the row is cut into segments of 1024. The sum at a segment's
+// start is known approximately from the segment sums, so its binade is, and with it the segment's composite map of that
+// binade (see above), which all segments compute at once. The walk then applies whole segments, 32 at a time by a warp
+// scan, and checks every one against the exact state: a segment whose predicted binade is not the actual one, or inside
+// which the sum leaves the binade or reaches randf, is evaluated element by element (about ten of 256).
+constexpr int SR_SEG = 1024;
+struct MinpRows {
+	float *part_max;  // [B][V / SR_PART]
+	float2 *seg_sum;  // [B][V / SR_SEG] masked sum, whole sum
+	int4 *seg_map;    // [B][V / SR_SEG] a0, a1, exponent of the binade
+};
+__global__ void __launch_bounds__(SR_THREADS) minp_max_kernel(SampleArgs a, MinpRows w) {
+	pdl_trigger();
+	pdl_wait();
+	__shared__ float red[SR_THREADS / 32];
+	const int b = blockIdx.y, tid = threadIdx.x;
+	const float *x = a.logits + size_t(b) * a.V + size_t(blockIdx.x) * SR_PART;
 	float mx = -INFINITY;
-	for (int i = tid * 4; i < a.V; i += SM_THREADS * 4) {
-		float4 v = __ldcg(reinterpret_cast<const float4 *>(x + i));
-		v.x = v.x / a.temp; v.y = v.y / a.temp; v.z = v.z / a.temp; v.w = v.w / a.temp;
-		__stcg(reinterpret_cast<float4 *>(x + i), v);
-		mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+#pragma unroll
+	for (int j = 0; j < SR_PART / (4 * SR_THREADS); j++) {
+		const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + tid + SR_THREADS * j);
+		mx = fmaxf(mx, fmaxf(fmaxf(v.x / a.temp, v.y / a.temp), fmaxf(v.z / a.temp, v.w / a.temp)));
 	}
 	mx = warp_max(mx);
 	if ((tid & 31) == 0) red[tid >> 5] = mx;
 	__syncthreads();
-	float rowmax = -INFINITY;
-	for (int w = 0; w < SM_NWARPS; w++) rowmax = fmaxf(rowmax, red[w]);
-	__syncthreads();
-	// (3)
-	float mp = -INFINITY;
-	for (int i = tid * 4; i < a.V; i += SM_THREADS * 4) {
-		float4 v = __ldcg(reinterpret_cast<const float4 *>(x + i));
-		v.x = expf(v.x - rowmax); v.y = expf(v.y - rowmax); v.z = expf(v.z - rowmax); v.w = expf(v.w - rowmax);
-		__stcg(reinterpret_cast<float4 *>(x + i), v);
-		mp = fmaxf(mp, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+	if (tid == 0) {
+		for (int i = 1; i < SR_THREADS / 32; i++) mx = fmaxf(mx, red[i]);
+		w.part_max[size_t(b) * gridDim.x + blockIdx.x] = mx;
 	}
-	mp = warp_max(mp);
-	if ((tid & 31) == 0) red[tid >> 5] = mp;
-	__syncthreads();
-	float maxp = -INFINITY;
-	for (int w = 0; w < SM_NWARPS; w++) maxp = fmaxf(maxp, red[w]);
-	__syncthreads();
-	// (4)
-	const float cut = a.minp * maxp;
-	float ds = 0.0f;
-	for (int i = tid * 4; i < a.V; i += SM_THREADS * 4) {
-		float4 v = __ldcg(reinterpret_cast<const float4 *>(x + i));
-		ds += (v.x < cut) ? 0.0f : v.x;
-		ds += (v.y < cut) ? 0.0f : v.y;
-		ds += (v.z < cut) ? 0.0f : v.z;
-		ds += (v.w < cut) ? 0.0f : v.w;
+}
+// a warp takes one segment
+__global__ void __launch_bounds__(SR_THREADS) minp_exp_kernel(SampleArgs a, MinpRows w) {
+	pdl_trigger();
+	pdl_wait();
+	const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int seg = blockIdx.x * (SR_PART / SR_SEG) + warp;
+	float4 *x = reinterpret_cast<float4 *>(a.logits + size_t(b) * a.V + size_t(seg) * SR_SEG);
+	float4 v[SR_SEG / 128];
+#pragma unroll
+	for (int j = 0; j < SR_SEG / 128; j++) v[j] = __ldcg(x + lane + 32 * j);
+	float rowmax = -INFINITY;
+	for (int c = lane; c < int(gridDim.x); c += 32) rowmax = fmaxf(rowmax, w.part_max[size_t(b) * gridDim.x + c]);
+	rowmax = warp_max(rowmax);
+	const float cut = a.minp * expf(rowmax - rowmax);  // the largest probability is exp(0)
+	float ds = 0.0f, us = 0.0f;
+#pragma unroll
+	for (int j = 0; j < SR_SEG / 128; j++) {
+		v[j].x = expf(v[j].x / a.temp - rowmax);
+		v[j].y = expf(v[j].y / a.temp - rowmax);
+		v[j].z = expf(v[j].z / a.temp - rowmax);
+		v[j].w = expf(v[j].w / a.temp - rowmax);
+		__stcg(x + lane + 32 * j, v[j]);
+		us += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+		ds += (v[j].x < cut) ? 0.0f : v[j].x;
+		ds += (v[j].y < cut) ? 0.0f : v[j].y;
+		ds += (v[j].z < cut) ? 0.0f : v[j].z;
+		ds += (v[j].w < cut) ? 0.0f : v[j].w;
 	}
 	ds = warp_sum(ds);
-	if ((tid & 31) == 0) red[tid >> 5] = ds;
+	us = warp_sum(us);
+	if (lane == 0) w.seg_sum[size_t(b) * (a.V / SR_SEG) + seg] = make_float2(ds, us);
+}
+// compose the maps of a warp's lanes in lane order; every lane gets the whole
+__device__ __forceinline__ CdfFn cdf_warp_compose(CdfFn f) {
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		CdfFn g;
+		g.a0 = __shfl_down_sync(0xffffffffu, f.a0, o);
+		g.a1 = __shfl_down_sync(0xffffffffu, f.a1, o);
+		f = cdf_compose(f, g);  // (right for the lanes whose group of 2 o starts with them: lane 0 in the end)
+	}
+	f.a0 = __shfl_sync(0xffffffffu, f.a0, 0);
+	f.a1 = __shfl_sync(0xffffffffu, f.a1, 0);
+	return f;
+}
+__global__ void __launch_bounds__(SR_THREADS) minp_scale_kernel(SampleArgs a, MinpRows w) {
+	pdl_trigger();
+	pdl_wait();
+	__shared__ float red[SR_THREADS / 32];
+	__shared__ float s_pre[SR_THREADS / 32];
+	const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int nseg = a.V / SR_SEG, seg = blockIdx.x * (SR_PART / SR_SEG) + warp;
+	float4 *x = reinterpret_cast<float4 *>(a.logits + size_t(b) * a.V + size_t(seg) * SR_SEG);
+	// element order inside the segment: blocks of 256, 8 consecutive ones per lane
+	float4 v[2 * (SR_SEG / 256)];
+#pragma unroll
+	for (int q = 0; q < SR_SEG / 256; q++) {
+		v[2 * q] = __ldcg(x + 64 * q + 2 * lane);
+		v[2 * q + 1] = __ldcg(x + 64 * q + 2 * lane + 1);
+	}
+	// the denominator (the same order in every CTA), and what lies before this CTA's first segment
+	const float2 *ss = w.seg_sum + size_t(b) * nseg;
+	const int first = blockIdx.x * (SR_PART / SR_SEG);
+	float ds = 0.0f, us = 0.0f;
+	for (int i = tid; i < nseg; i += SR_THREADS) {
+		const float2 t = ss[i];
+		ds += t.x;
+		us += i < first ? t.y : 0.0f;
+	}
+	ds = warp_sum(ds);
+	us = warp_sum(us);
+	if (lane == 0) {
+		red[warp] = ds;
+		s_pre[warp] = us;
+	}
 	__syncthreads();
-	float denom = 0.0f;
-	for (int w = 0; w < SM_NWARPS; w++) denom += red[w];
+	float denom = 0.0f, before = 0.0f;
+#pragma unroll
+	for (int i = 0; i < SR_THREADS / 32; i++) {
+		denom += red[i];
+		before += s_pre[i];
+	}
+	for (int i = first; i < seg; i++) before += ss[i].y;
 	const float inv = 1.0f / denom;
-	// (5)+(6): every chunk is scaled (the reference scales the whole row); the running sum is
-	// evaluated chunk by chunk until the crossing is known
+	const int e = int((__float_as_uint(before * inv) >> 23) & 0xffu) - 127;
+	const bool usable = before * inv >= 7.888609e-31f && e <= 120;
+	const float inv_u = usable ? __uint_as_float(unsigned(23 - e + 127) << 23) : 1.0f;
+	CdfFn whole{0, 0};
+#pragma unroll
+	for (int q = 0; q < SR_SEG / 256; q++) {
+		CdfFn f{0, 0};
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			float4 &t = v[2 * q + h];
+			t.x *= inv;
+			t.y *= inv;
+			t.z *= inv;
+			t.w *= inv;
+			__stcg(x + 64 * q + 2 * lane + h, t);
+			f = cdf_compose(f, cdf_element(t.x, inv_u));
+			f = cdf_compose(f, cdf_element(t.y, inv_u));
+			f = cdf_compose(f, cdf_element(t.z, inv_u));
+			f = cdf_compose(f, cdf_element(t.w, inv_u));
+		}
+		whole = cdf_compose(whole, cdf_warp_compose(f));
+	}
+	if (lane == 0) w.seg_map[size_t(b) * nseg + seg] = make_int4(whole.a0, whole.a1, usable ? e : -1000, 0);
+}
+// one CTA per row
+__global__ void __launch_bounds__(SR_THREADS) minp_walk_kernel(SampleArgs a, MinpRows w) {
+	pdl_trigger();
+	pdl_wait();
+	__shared__ float chunk[SR_SEG];
+	__shared__ int scratch[2 * (SR_THREADS / 32) + 8];
+	__shared__ float s_cum;
+	__shared__ int s_seg;
+	const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+	const int nseg = a.V / SR_SEG;
+	const float *x = a.logits + size_t(b) * a.V;
+	const int4 *maps = w.seg_map + size_t(b) * nseg;
+	float randf = 0.0f;
+	const int rc = a.randf_count[b];
+	if (rc < a.randf_cap) randf = a.randf[size_t(rc) * a.B + b];
 	if (tid == 0) s_cum = 0.0f;
-	__syncthreads();
 	int found = -1;
-	for (int c0 = 0; c0 < a.V; c0 += MP_CHUNK) {
-		const int n = min(MP_CHUNK, a.V - c0);
-		for (int i = tid * 4; i < n; i += SM_THREADS * 4) {
-			float4 v = __ldcg(reinterpret_cast<const float4 *>(x + c0 + i));
-			v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-			__stcg(reinterpret_cast<float4 *>(x + c0 + i), v);
-			*reinterpret_cast<float4 *>(&chunk[i]) = v;
+	for (int seg = 0; seg < nseg && found < 0; seg++) {
+		__syncthreads();
+		if (tid < 32) {  // whole segments
+			float cum = s_cum;
+			for (; seg < nseg;) {
+				const int4 m = seg + lane < nseg ? __ldcg(maps + seg + lane) : make_int4(0, 0, -2000, 0);
+				const int e = int((__float_as_uint(cum) >> 23) & 0xffu) - 127;
+				if (!(cum >= 7.888609e-31f) || e > 120) break;
+				const float u = __uint_as_float(unsigned(e - 23 + 127) << 23), inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
+				const int S0 = int(cum * inv_u);
+				const float y = randf * inv_u;
+				const int Tmin = min((y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG, 1 << 24);
+				CdfFn inc{m.x, m.y};
+#pragma unroll
+				for (int o = 1; o < 32; o <<= 1) {
+					CdfFn prev;
+					prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
+					prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
+					if (lane >= o) inc = cdf_compose(prev, inc);
+				}
+				const int S = cdf_apply(inc, S0);
+				const unsigned bad = __ballot_sync(0xffffffffu, m.z != e || S >= Tmin);
+				const int n = bad ? __ffs(bad) - 1 : 32;
+				if (n > 0) cum = float(__shfl_sync(0xffffffffu, S, n - 1)) * u;
+				seg += n;
+				if (n < 32) break;
+			}
+			if (lane == 0) {
+				s_cum = cum;
+				s_seg = seg;
+			}
 		}
 		__syncthreads();
-		if (found < 0) {
-			const int r = cdf_cross_block<SM_NWARPS>(chunk, n, &s_cum, randf, scratch, c0 == 0 ? 1024 : 0);
-			if (r >= 0) found = c0 + r;
-		}
+		seg = s_seg;
+		if (seg >= nseg) break;
+		reinterpret_cast<float4 *>(chunk)[tid] = __ldcg(reinterpret_cast<const float4 *>(x + size_t(seg) * SR_SEG) + tid);
 		__syncthreads();
+		const int r = cdf_cross_block<SR_THREADS / 32>(chunk, SR_SEG, &s_cum, randf, scratch, seg == 0 ? SR_SEG : 0);
+		if (r >= 0) found = seg * SR_SEG + r;
 	}
 	if (tid == 0) {
 		emit_token(a, b, found < 0 ? 0 : found);
-		a.randf_count[b] += 1;
+		a.randf_count[b] = rc + 1;
 	}
 }
-
 
 // ------------------------------------------------------------------ grid-wide min-p (one sequence)
 // ops::minp_logits for a single row spread over G CTAs of SG_THREADS threads (cooperative launch: the

@@ -114,7 +114,7 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, int *err
 	int spins = 0;
 	while (!mbar_try_wait(bar, parity)) {
 		if (++spins > TC_SPIN_CAP) {
-			atomicExch(err, 6);
+			*static_cast<volatile int *>(err) = 6;  // (a plain store: the word may lie in host memory)
 			return false;
 		}
 	}

@@ -390,6 +390,22 @@ struct TcScratch {
 	int *err = nullptr;
 };
 
+// Scratch of the row samplers (argmax_kernel, minp_*_kernel) for B rows of V logits, carved out of one block
+struct SampScratch {
+	MinpRows rows{};
+	unsigned long long *keys = nullptr;
+	unsigned *tickets = nullptr;
+	static size_t bytes(int B, size_t V) { return size_t(B) * ((V / SR_SEG + 1) * (16 + 8) + (V / SR_PART + 1) * 4 + 12) + 64; }
+	SampScratch(uint8_t *p, int B, size_t V) {
+		const size_t nseg = size_t(B) * (V / SR_SEG + 1);
+		rows.seg_map = reinterpret_cast<int4 *>(p);
+		rows.seg_sum = reinterpret_cast<float2 *>(p + nseg * 16);
+		keys = reinterpret_cast<unsigned long long *>(p + nseg * 24);
+		tickets = reinterpret_cast<unsigned *>(p + nseg * 24 + size_t(B) * 8);
+		rows.part_max = reinterpret_cast<float *>(p + nseg * 24 + size_t(B) * 12);
+	}
+};
+
 // ===================================================================== state
 struct tg_state {
 	tg_model *m = nullptr;
@@ -413,6 +429,7 @@ struct tg_state {
 	unsigned *attn_tickets = nullptr;
 	float *attn_part = nullptr;        // [B][nsplit_max][1032]
 	int attn_nsplit_local = 16, attn_nsplit_global = 64;
+	uint8_t *samp_ws = nullptr;        // the row samplers' scratch (SampScratch)
 	int *step_pos = nullptr, *next_pos = nullptr, *ring_base = nullptr;  // [B]
 	int *tok = nullptr;                // [B]
 	int *tok_log = nullptr;            // [log_cap][B]
@@ -543,6 +560,8 @@ int state_alloc(tg_state *s) {
 		TG_CUDA(cudaMemsetAsync(*p, 0, n * 4, s->stream));
 		return TG_OK;
 	};
+	TG_CUDA(cudaMalloc(&s->samp_ws, SampScratch::bytes(B, V)));
+	TG_CUDA(cudaMemsetAsync(s->samp_ws, 0, SampScratch::bytes(B, V), s->stream));  // (keys and tickets start at zero)
 	TG_TRY(alloci(&s->step_pos, B));
 	TG_TRY(alloci(&s->next_pos, B));
 	TG_TRY(alloci(&s->ring_base, B));
@@ -1443,6 +1462,21 @@ SampleArgs sample_args(tg_state *s, float minp, float temp, bool log_tokens) {
 	return a;
 }
 
+int launch_argmax_rows(const SampleArgs &a, const SampScratch &ws, cudaStream_t st) {
+	launch_k(argmax_kernel, dim3((a.V + SR_PART - 1) / SR_PART, a.B), dim3(SR_THREADS), 0, st, a, ws.keys, ws.tickets);
+	count_launch();
+	return check_launch("argmax");
+}
+int launch_minp_rows(const SampleArgs &a, const SampScratch &ws, cudaStream_t st) {
+	const dim3 grid(a.V / SR_PART, a.B);
+	launch_k(minp_max_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
+	launch_k(minp_exp_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
+	launch_k(minp_scale_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
+	launch_k(minp_walk_kernel, dim3(a.B), dim3(SR_THREADS), 0, st, a, ws.rows);
+	count_launch(4);
+	return check_launch("minp");
+}
+
 int enqueue_sampler(tg_state *s, float minp, float temp, bool log_tokens) {
 	SampleArgs a = sample_args(s, minp, temp, log_tokens);
 	if (minp < 1.0f && s->mega_ok && s->B == 1 && env_int("TG_MINP_GRID", 1)) {
@@ -1457,14 +1491,9 @@ int enqueue_sampler(tg_state *s, float minp, float temp, bool log_tokens) {
 		count_launch();
 		return check_launch("minp_grid");
 	}
-	if (minp < 1.0f) {  // transformer.hpp:208,229: min-p sampling iff minp < 1
-		minp_kernel<<<s->B, SM_THREADS, 0, s->stream>>>(a);
-		count_launch();
-		return check_launch("minp");
-	}
-	launch_k(argmax_kernel, dim3(s->B), dim3(SM_THREADS), 0, s->stream, a);
-	count_launch();
-	return check_launch("argmax");
+	// transformer.hpp:208,229: min-p sampling iff minp < 1
+	const SampScratch ws(s->samp_ws, s->B, a.V);
+	return minp < 1.0f ? launch_minp_rows(a, ws, s->stream) : launch_argmax_rows(a, ws, s->stream);
 }
 
 // the pinned staging buffer may be overwritten only when no enqueued copy still reads it
@@ -2324,6 +2353,7 @@ int tg_state_free(tg_state *s) {
 	cudaFree(s->tickets);
 	cudaFree(s->attn_tickets);
 	cudaFree(s->attn_part);
+	cudaFree(s->samp_ws);
 	cudaFree(s->step_pos);
 	cudaFree(s->next_pos);
 	cudaFree(s->ring_base);
@@ -2955,9 +2985,11 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 			TG_CUDA(cudaMalloc(&tc[dev].partial, pneed * 4));
 			tc[dev].partial_floats = pneed;
 		}
+		static int *err_host[64] = {nullptr};  // the error word, in host memory that the device writes
 		if (!tc[dev].err) {
-			TG_CUDA(cudaMalloc(&tc[dev].err, 4));
-			TG_CUDA(cudaMemset(tc[dev].err, 0, 4));
+			TG_CUDA(cudaHostAlloc(&err_host[dev], 4, cudaHostAllocMapped | cudaHostAllocPortable));
+			*err_host[dev] = 0;
+			TG_CUDA(cudaHostGetDevicePointer(&tc[dev].err, err_host[dev], 0));
 		}
 		TG_TRY(pack_activations(a, M, K, tc[dev], (cudaStream_t)stream));
 		TG_TRY(launch_gemm_tc(c, q, M, tc[dev], (cudaStream_t)stream));
@@ -2966,11 +2998,9 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
 		TG_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
 		if (cap != cudaStreamCaptureStatusNone) return TG_OK;
-		int flag = 0;
-		TG_CUDA(cudaMemcpyAsync(&flag, tc[dev].err, 4, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
 		TG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-		if (flag) {
-			cudaMemset(tc[dev].err, 0, 4);
+		if (*static_cast<volatile int *>(err_host[dev])) {
+			*err_host[dev] = 0;
 			return fail(TG_ECUDA, "tensor-core GEMM: a pipeline wait ran out");
 		}
 		return TG_OK;
@@ -3039,53 +3069,127 @@ int tg_qgemm(float *c, const float *a, const int8_t *w, const float *scales, int
 	return TG_OK;
 }
 
+namespace {
+// What the samplers on host buffers work in: a stream, device memory and pinned staging, kept by the calling thread (so
+// no two threads share one) and given back when the thread ends. Allocating and freeing these per call took several
+// times the work itself. Kept up to HOST_WS_MAX bytes each; a larger call takes and frees its own.
+constexpr size_t HOST_WS_MAX = size_t(8) << 20;
+constexpr int HOST_WS_CHUNKS = 4;  // copies to and from the caller's pageable memory overlap the transfers in chunks
+struct HostWs {
+	cudaStream_t st = nullptr;
+	cudaEvent_t ev[HOST_WS_CHUNKS] = {};
+	uint8_t *dev = nullptr, *pin = nullptr;
+	size_t dev_bytes = 0, pin_bytes = 0;
+	void release() {
+		if (st) cudaStreamSynchronize(st);
+		for (cudaEvent_t &e : ev)
+			if (e) cudaEventDestroy(e);
+		cudaFree(dev);
+		cudaFreeHost(pin);
+		if (st) cudaStreamDestroy(st);
+		cudaGetLastError();
+		*this = HostWs();
+	}
+	int reserve(size_t d, size_t p) {
+		if (!st) {
+			TG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+			for (cudaEvent_t &e : ev) TG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+		}
+		if (d > dev_bytes) {
+			cudaFree(dev);
+			dev = nullptr;
+			dev_bytes = 0;
+			TG_CUDA(cudaMalloc(&dev, d));
+			dev_bytes = d;
+		}
+		if (p > pin_bytes) {
+			cudaFreeHost(pin);
+			pin = nullptr;
+			pin_bytes = 0;
+			TG_CUDA(cudaMallocHost(&pin, p));
+			pin_bytes = p;
+		}
+		return TG_OK;
+	}
+	// the caller's buffer -> dst (enqueued; the caller's memory has been read on return)
+	int upload(uint8_t *dst, const void *src, size_t bytes) {
+		const size_t ch = (bytes / HOST_WS_CHUNKS + 4095) & ~size_t(4095);
+		for (size_t o = 0; o < bytes; o += ch) {
+			const size_t n = std::min(ch, bytes - o);
+			std::memcpy(pin + o, static_cast<const uint8_t *>(src) + o, n);
+			TG_CUDA(cudaMemcpyAsync(dst + o, pin + o, n, cudaMemcpyHostToDevice, st));
+		}
+		return TG_OK;
+	}
+	// src -> the caller's buffer (complete on return)
+	int download(void *dst, const uint8_t *src, size_t bytes) {
+		const size_t ch = (bytes / HOST_WS_CHUNKS + 4095) & ~size_t(4095);
+		int k = 0;
+		for (size_t o = 0; o < bytes; o += ch, k++) {
+			TG_CUDA(cudaMemcpyAsync(pin + o, src + o, std::min(ch, bytes - o), cudaMemcpyDeviceToHost, st));
+			TG_CUDA(cudaEventRecord(ev[k], st));
+		}
+		k = 0;
+		for (size_t o = 0; o < bytes; o += ch, k++) {
+			TG_CUDA(cudaEventSynchronize(ev[k]));
+			std::memcpy(static_cast<uint8_t *>(dst) + o, pin + o, std::min(ch, bytes - o));
+		}
+		return TG_OK;
+	}
+	~HostWs() {
+		if (st || dev || pin) release();
+	}
+};
+
+// one row of n logits in host memory: arg-max, or min-p with the probabilities written back
+int sample_host_row(const float *in, float *out, int n, bool minp_mode, float minp, float temp, float randf, int *tok) {
+	TG_TRY(ensure_device(0));
+	static thread_local HostWs kept;
+	HostWs own;
+	const size_t row = size_t(n) * 4, row_up = (row + 255) & ~size_t(255), wsb = (SampScratch::bytes(1, n) + 255) & ~size_t(255);
+	const size_t dbytes = 256 + row_up + wsb;  // [token][uniform count][uniform] .. [key][ticket] ..., the row, the scratch
+	HostWs &w = dbytes > HOST_WS_MAX ? own : kept;
+	const bool fresh = dbytes > w.dev_bytes;
+	TG_TRY(w.reserve(dbytes, row_up + 256));
+	if (fresh) TG_CUDA(cudaMemsetAsync(w.dev, 0, 256, w.st));  // (the kernels leave key and ticket zero)
+	struct {
+		int tok, count;
+		float randf;
+	} up = {0, 0, randf};
+	uint8_t *pin_words = w.pin + row_up;
+	std::memcpy(pin_words, &up, sizeof up);
+	TG_CUDA(cudaMemcpyAsync(w.dev, pin_words, sizeof up, cudaMemcpyHostToDevice, w.st));
+	TG_TRY(w.upload(w.dev + 256, in, row));
+	SampleArgs a{};
+	a.logits = reinterpret_cast<float *>(w.dev + 256);
+	a.V = n;
+	a.tok_out = reinterpret_cast<int *>(w.dev);
+	a.B = 1;
+	a.minp = minp;
+	a.temp = temp;
+	a.randf = reinterpret_cast<const float *>(w.dev + 8);
+	a.randf_count = reinterpret_cast<int *>(w.dev + 4);
+	a.randf_cap = 1;
+	SampScratch ws(w.dev + 256 + row_up, 1, n);
+	ws.keys = reinterpret_cast<unsigned long long *>(w.dev + 64);
+	ws.tickets = reinterpret_cast<unsigned *>(w.dev + 72);
+	TG_TRY(minp_mode ? launch_minp_rows(a, ws, w.st) : launch_argmax_rows(a, ws, w.st));
+	TG_CUDA(cudaMemcpyAsync(pin_words, w.dev, 4, cudaMemcpyDeviceToHost, w.st));
+	if (minp_mode) TG_TRY(w.download(out, w.dev + 256, row));
+	TG_CUDA(cudaStreamSynchronize(w.st));
+	std::memcpy(tok, pin_words, 4);
+	return TG_OK;
+}
+}  // namespace
+
 int tg_argmax_logits(const float *logits, int n, int *tok) {
 	if (!logits || !tok || n < 4 || n % 4) return fail(TG_EINVAL, "bad argument (n must be a multiple of 4)");
-	TG_TRY(ensure_device(0));
-	DevBuf dl, dt, dc;
-	TG_TRY(dl.alloc(size_t(n) * 4));
-	TG_TRY(dt.alloc(4));
-	TG_TRY(dc.alloc(4));
-	TG_CUDA(cudaMemcpy(dl.p, logits, size_t(n) * 4, cudaMemcpyHostToDevice));
-	SampleArgs a{};
-	a.logits = (float *)dl.p;
-	a.V = n;
-	a.tok_out = (int *)dt.p;
-	a.B = 1;
-	argmax_kernel<<<1, SM_THREADS>>>(a);
-	count_launch();
-	TG_TRY(check_launch("argmax"));
-	TG_CUDA(cudaMemcpy(tok, dt.p, 4, cudaMemcpyDeviceToHost));
-	return TG_OK;
+	return sample_host_row(logits, nullptr, n, false, 2.0f, 1.0f, 0.0f, tok);
 }
 
 int tg_minp_logits(float *logits, int n, float minp, float temp, float randf, int *tok) {
 	if (!logits || !tok || n < MP_CHUNK || n % MP_CHUNK) return fail(TG_EINVAL, "bad argument (n must be a multiple of 8192)");
-	TG_TRY(ensure_device(0));
-	DevBuf dl, dt, dr, dc;
-	TG_TRY(dl.alloc(size_t(n) * 4));
-	TG_TRY(dt.alloc(4));
-	TG_TRY(dr.alloc(4));
-	TG_TRY(dc.alloc(4));
-	TG_CUDA(cudaMemcpy(dl.p, logits, size_t(n) * 4, cudaMemcpyHostToDevice));
-	TG_CUDA(cudaMemcpy(dr.p, &randf, 4, cudaMemcpyHostToDevice));
-	TG_CUDA(cudaMemset(dc.p, 0, 4));
-	SampleArgs a{};
-	a.logits = (float *)dl.p;
-	a.V = n;
-	a.tok_out = (int *)dt.p;
-	a.B = 1;
-	a.minp = minp;
-	a.temp = temp;
-	a.randf = (const float *)dr.p;
-	a.randf_count = (int *)dc.p;
-	a.randf_cap = 1;
-	minp_kernel<<<1, SM_THREADS>>>(a);
-	count_launch();
-	TG_TRY(check_launch("minp"));
-	TG_CUDA(cudaMemcpy(tok, dt.p, 4, cudaMemcpyDeviceToHost));
-	TG_CUDA(cudaMemcpy(logits, dl.p, size_t(n) * 4, cudaMemcpyDeviceToHost));
-	return TG_OK;
+	return sample_host_row(logits, logits, n, true, minp, temp, randf, tok);
 }
 
 int tg_inverse_cdf(const float *p, int n, float cum0, float randf, int *idx, float *cum_out) {
