@@ -1,0 +1,504 @@
+// Attention over fp32 K / V rows on the CUDA cores, for the shapes whose time is latency and memory traffic, not
+// arithmetic: one decode step per sequence, and short prompts.
+//
+// The rows of a sequence's keys (values) follow each other in memory, so a chunk of 32 keys is ONE bulk copy of 32 KB
+// into shared memory: the whole traffic of a CTA is asynchronous and costs no registers, and three CTAs fit an SM. The
+// copy of the next K chunk starts when the scores of this one are done, that of the next V chunk when its products are.
+// Per chunk: scores (a warp takes a few keys against all query rows; a lane holds 8 of the 256 dimensions, and the
+// lanes' partial sums meet in a reduce-scatter, one shuffle per score), one softmax step per query row with lane = key,
+// then the products with V (a thread holds 4 dimensions of every row for a share of the keys).
+//
+// The result leaves as the digits of the O projection's operand (kernels_gemm_i8.cuh) where the caller wants them: the
+// CTA that finishes a row has all of it.
+#pragma once
+#include "kernels_decode.cuh"  // AT_NH, AT_HD
+#include "kernels_gemm_i8.cuh"
+#include "tg_common.cuh"
+
+namespace tg {
+
+constexpr int AC_KEYS = 32;
+constexpr int AC_BUF = AC_KEYS * 1024;  // bytes of a K or V chunk
+constexpr int AC_SMEM = 2 * AC_BUF;
+
+// N partial sums per lane (N = 16): afterwards lane L holds the warp's total of value L >> 1
+__device__ __forceinline__ float ac_reduce16(float (&t)[16], int lane) {
+#pragma unroll
+	for (int o = 8; o >= 1; o >>= 1) {
+		const bool up = lane & (2 * o);
+#pragma unroll
+		for (int i = 0; i < o; i++) {
+			const float keep = up ? t[i + o] : t[i], send = up ? t[i] : t[i + o];
+			t[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * o);
+		}
+	}
+	return t[0] + __shfl_xor_sync(0xffffffffu, t[0], 1);
+}
+__device__ __forceinline__ float ac_dot8(const float4 &q0, const float4 &q1, const float4 &k0, const float4 &k1) {
+	float t = q0.x * k0.x;
+	t = fmaf(q0.y, k0.y, t);
+	t = fmaf(q0.z, k0.z, t);
+	t = fmaf(q0.w, k0.w, t);
+	t = fmaf(q1.x, k1.x, t);
+	t = fmaf(q1.y, k1.y, t);
+	t = fmaf(q1.z, k1.z, t);
+	return fmaf(q1.w, k1.w, t);
+}
+__device__ __forceinline__ void ac_fma4(float4 &o, float p, const float4 &v) {
+	o.x = fmaf(p, v.x, o.x);
+	o.y = fmaf(p, v.y, o.y);
+	o.z = fmaf(p, v.z, o.z);
+	o.w = fmaf(p, v.w, o.w);
+}
+
+// ------------------------------------------------------------------ decode: one query per sequence
+struct AttnArgs {
+	const float *qkv;   // [B][1536] = q(4x256) | k(256) | v(256)
+	// qkv_nsplit > 0: qkv instead holds the raw K-split partial sums of the grouped q|k|v GEMM,
+	// [qkv_nsplit][B][1536], and sq / sk / sv are the column scales (splits are added in ascending order)
+	int qkv_nsplit, qkv_B;
+	const float *sq, *sk, *sv;
+	const float *rmsq;  // [256]
+	const float *rmsk;  // [256]
+	const float *cosT;  // [n_pos][256]
+	const float *sinT;
+	float *kcache;      // [B][slots][256]
+	float *vcache;
+	int slots;          // 512 on local layers, max_pos_global on global layers
+	int is_local;
+	const int *step_pos;   // [B]
+	const int *ring_base;  // [B] prompt length if it filled the ring, else 0 (decode.hpp:98-103)
+	float *part;        // [B][nsplit][4*256 + 8]
+	unsigned *tickets;  // [B]
+	float *out;         // [B][1024], or null:
+	uint8_t *x;         // the digits of the result (K = 1024) and their row scales
+	float *rowscale;
+	int groups;
+	int nsplit;
+	int *err_flag;
+};
+constexpr int AT_THREADS = 256;
+constexpr int AT_PART = AT_NH * AT_HD + 8;
+
+__global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) {
+	extern __shared__ __align__(128) uint8_t ac_smem[];
+	__shared__ __align__(16) float rowbuf[AT_NH * AT_HD + 2 * AT_HD];  // q | k | v of the new token, normed and rotated in place
+	__shared__ __align__(16) float sc[AC_KEYS][AT_NH], pr[AC_KEYS][AT_NH];
+	__shared__ float corr_s[AT_NH], m_s[AT_NH], l_s[AT_NH];
+	__shared__ uint64_t kbar, vbar;
+	__shared__ uint32_t red[AT_THREADS / 32];
+	__shared__ int s_last;
+	float *K = reinterpret_cast<float *>(ac_smem), *V = reinterpret_cast<float *>(ac_smem + AC_BUF);
+	const int b = blockIdx.y, split = blockIdx.x;
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	if (tid == 0) {
+		mbar_init(&kbar, 1);
+		mbar_init(&vbar, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	pdl_trigger();
+	pdl_wait();
+	int pos = a.step_pos[b];
+	int slot, valid;
+	if (a.is_local) {
+		slot = (pos - a.ring_base[b]) % a.slots;
+		valid = min(pos + 1, a.slots);
+	} else {
+		if (pos >= a.slots) {  // cache full: refuse to write out of bounds
+			if (tid == 0) *a.err_flag = 2;
+			pos = a.slots - 1;
+		}
+		slot = pos;
+		valid = pos + 1;
+	}
+	// whole chunks of keys are dealt out to the splits; splits without any leave at once
+	const int chunks = (valid + AC_KEYS - 1) / AC_KEYS, per = (chunks + a.nsplit - 1) / a.nsplit, nact = (chunks + per - 1) / per;
+	if (split >= nact) return;
+	const int j0 = split * per * AC_KEYS, j1 = min(valid, j0 + per * AC_KEYS);
+	const int nch = (j1 - j0 + AC_KEYS - 1) / AC_KEYS;
+	float *kc = a.kcache + size_t(b) * a.slots * AT_HD, *vc = a.vcache + size_t(b) * a.slots * AT_HD;
+	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
+		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
+		fence_proxy_async();
+		mbar_expect_tx(bar, bytes);
+		bulk_load(dst, src + size_t(j0 + c * AC_KEYS) * AT_HD, bytes, bar);
+	};
+	__syncthreads();
+	if (tid == 0) {
+		issue(K, kc, 0, &kbar);
+		issue(V, vc, 0, &vbar);
+	}
+	// ---- the new token's q, k, v
+	constexpr int NQ = AT_NH * AT_HD + 2 * AT_HD;
+	for (int n = 4 * tid; n < NQ; n += 4 * AT_THREADS) {
+		float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (a.qkv_nsplit > 0) {
+			const float *p = a.qkv + size_t(b) * NQ + n;
+			const size_t sstride = size_t(a.qkv_B) * NQ;
+			for (int s0 = 0; s0 < a.qkv_nsplit; s0 += 4) {
+				float4 v[4];
+#pragma unroll
+				for (int q = 0; q < 4; q++) {
+					v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+					if (s0 + q < a.qkv_nsplit) v[q] = *reinterpret_cast<const float4 *>(p + size_t(s0 + q) * sstride);
+				}
+#pragma unroll
+				for (int q = 0; q < 4; q++) {
+					acc.x += v[q].x;
+					acc.y += v[q].y;
+					acc.z += v[q].z;
+					acc.w += v[q].w;
+				}
+			}
+			const float *scl = n < AT_NH * AT_HD ? a.sq + n : (n < AT_NH * AT_HD + AT_HD ? a.sk + (n - AT_NH * AT_HD) : a.sv + (n - AT_NH * AT_HD - AT_HD));
+			const float4 s4 = *reinterpret_cast<const float4 *>(scl);
+			acc.x *= s4.x;
+			acc.y *= s4.y;
+			acc.z *= s4.z;
+			acc.w *= s4.w;
+		} else {
+			acc = *reinterpret_cast<const float4 *>(a.qkv + size_t(b) * NQ + n);
+		}
+		*reinterpret_cast<float4 *>(&rowbuf[n]) = acc;
+	}
+	__syncthreads();
+	if (warp <= AT_NH) {  // heads 0..3 of q, then k: per-head norm and RoPE; lane owns d = 4 lane .. and the partners 128 + d
+		const float *w = warp < AT_NH ? a.rmsq : a.rmsk;
+		// the reference scales q by 1/sqrt(256) = 2^-4 before the dot products (ops.hpp:262,283)
+		const float qs = warp < AT_NH ? 0.0625f : 1.0f;
+		const float4 *cr = reinterpret_cast<const float4 *>(a.cosT + size_t(pos) * AT_HD), *sr = reinterpret_cast<const float4 *>(a.sinT + size_t(pos) * AT_HD);
+		const float4 c0 = cr[lane], c1 = cr[32 + lane], s0 = sr[lane], s1 = sr[32 + lane];
+		const float4 w0 = reinterpret_cast<const float4 *>(w)[lane], w1 = reinterpret_cast<const float4 *>(w)[32 + lane];
+		float4 *x = reinterpret_cast<float4 *>(&rowbuf[warp * AT_HD]);
+		const float4 lo = x[lane], hi = x[32 + lane];
+		const float lov[4] = {lo.x, lo.y, lo.z, lo.w}, hiv[4] = {hi.x, hi.y, hi.z, hi.w};
+		const float wlo[4] = {w0.x, w0.y, w0.z, w0.w}, whi[4] = {w1.x, w1.y, w1.z, w1.w};
+		const float clo[4] = {c0.x, c0.y, c0.z, c0.w}, chi[4] = {c1.x, c1.y, c1.z, c1.w};
+		const float slo[4] = {s0.x, s0.y, s0.z, s0.w}, shi[4] = {s1.x, s1.y, s1.z, s1.w};
+		float ss = 0.0f;
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			ss = fmaf(lov[i], lov[i], ss);
+			ss = fmaf(hiv[i], hiv[i], ss);
+		}
+		ss = warp_sum(ss);
+		const float r = inv_rms(ss, AT_HD);
+		float yl[4], yh[4];
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			const float u = (lov[i] * r) * (wlo[i] + 1.0f), v = (hiv[i] * r) * (whi[i] + 1.0f);
+			// y = cos*x + rotate_half(x)*sin, rotate_half = [-x_hi, x_lo]
+			yl[i] = fmaf(-1.0f * v, slo[i], clo[i] * u) * qs;
+			yh[i] = fmaf(u, shi[i], chi[i] * v) * qs;
+		}
+		x[lane] = make_float4(yl[0], yl[1], yl[2], yl[3]);
+		x[32 + lane] = make_float4(yh[0], yh[1], yh[2], yh[3]);
+	}
+	__syncthreads();
+	const float4 *knew = reinterpret_cast<const float4 *>(&rowbuf[AT_NH * AT_HD]), *vnew = knew + 64;
+	if (slot >= j0 && slot < j1) {
+		if (tid < 64)
+			reinterpret_cast<float4 *>(kc + size_t(slot) * AT_HD)[tid] = knew[tid];
+		else if (tid < 128)
+			reinterpret_cast<float4 *>(vc + size_t(slot) * AT_HD)[tid - 64] = vnew[tid - 64];
+	}
+	float4 q0[AT_NH], q1[AT_NH];
+#pragma unroll
+	for (int h = 0; h < AT_NH; h++) {
+		q0[h] = *reinterpret_cast<const float4 *>(&rowbuf[h * AT_HD + 4 * lane]);
+		q1[h] = *reinterpret_cast<const float4 *>(&rowbuf[h * AT_HD + 128 + 4 * lane]);
+	}
+	const int d4 = tid & 63, kg = tid >> 6;
+	float4 o[AT_NH];
+#pragma unroll
+	for (int h = 0; h < AT_NH; h++) o[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+	float m = -INFINITY, l = 0.0f;  // of head `warp` (warps 0..3)
+	for (int c = 0; c < nch; c++) {
+		const int n = min(AC_KEYS, j1 - j0 - c * AC_KEYS), at = slot - (j0 + c * AC_KEYS);  // keys of the chunk; the new token's row in it
+		const bool here = at >= 0 && at < n;
+		tc_wait(&kbar, c & 1, a.err_flag);
+		if (here) {  // the cache does not hold the new token's row yet
+			if (tid < 64) reinterpret_cast<float4 *>(K)[at * 64 + tid] = knew[tid];
+			__syncthreads();
+		}
+		{
+			float t[16];
+#pragma unroll
+			for (int kk = 0; kk < 4; kk++) {
+				const float4 k0 = *reinterpret_cast<const float4 *>(K + (4 * warp + kk) * AT_HD + 4 * lane);
+				const float4 k1 = *reinterpret_cast<const float4 *>(K + (4 * warp + kk) * AT_HD + 128 + 4 * lane);
+#pragma unroll
+				for (int h = 0; h < AT_NH; h++) t[kk * 4 + h] = ac_dot8(q0[h], q1[h], k0, k1);
+			}
+			const float z = ac_reduce16(t, lane);
+			if (!(lane & 1)) sc[4 * warp + (lane >> 3)][(lane >> 1) & 3] = z;
+		}
+		__syncthreads();  // scores complete, K consumed
+		if (tid == 0 && c + 1 < nch) issue(K, kc, c + 1, &kbar);
+		if (warp < AT_NH) {
+			const float z = lane < n ? sc[lane][warp] : -INFINITY;
+			const float mn = fmaxf(m, warp_max(z));  // finite: a chunk has at least one key
+			const float p = expf(z - mn), cr = expf(m - mn);
+			l = fmaf(l, cr, warp_sum(p));
+			m = mn;
+			pr[lane][warp] = p;
+			if (lane == 0) corr_s[warp] = cr;
+		}
+		tc_wait(&vbar, c & 1, a.err_flag);
+		if (here && tid >= 128 && tid < 192) reinterpret_cast<float4 *>(V)[at * 64 + tid - 128] = vnew[tid - 128];
+		__syncthreads();  // probabilities complete
+#pragma unroll
+		for (int h = 0; h < AT_NH; h++) {
+			const float cr = corr_s[h];
+			o[h].x *= cr;
+			o[h].y *= cr;
+			o[h].z *= cr;
+			o[h].w *= cr;
+		}
+#pragma unroll
+		for (int kk = 0; kk < AC_KEYS / 4; kk++) {
+			const int key = kg * (AC_KEYS / 4) + kk;
+			if (key < n) {
+				const float4 v = *reinterpret_cast<const float4 *>(V + key * AT_HD + 4 * d4);
+				const float4 p = *reinterpret_cast<const float4 *>(&pr[key][0]);
+				ac_fma4(o[0], p.x, v);
+				ac_fma4(o[1], p.y, v);
+				ac_fma4(o[2], p.z, v);
+				ac_fma4(o[3], p.w, v);
+			}
+		}
+		__syncthreads();  // V consumed
+		if (tid == 0 && c + 1 < nch) issue(V, vc, c + 1, &vbar);
+	}
+	// ---- join the four key groups: thread (h, d4) ends up with four consecutive outputs
+	float4 *jb = reinterpret_cast<float4 *>(K);
+#pragma unroll
+	for (int h = 0; h < AT_NH; h++) jb[(kg * AT_NH + h) * 64 + d4] = o[h];
+	if (warp < AT_NH && lane == 0) {
+		m_s[warp] = m;
+		l_s[warp] = l;
+	}
+	__syncthreads();
+	const int h = kg;
+	float4 r = jb[h * 64 + d4];
+#pragma unroll
+	for (int g = 1; g < 4; g++) {
+		const float4 t = jb[(g * AT_NH + h) * 64 + d4];
+		r.x += t.x;
+		r.y += t.y;
+		r.z += t.z;
+		r.w += t.w;
+	}
+	float L = l_s[h];
+	if (nact > 1) {
+		float *pb = a.part + size_t(b) * a.nsplit * AT_PART;
+		float *prow = pb + size_t(split) * AT_PART;
+		__stcg(reinterpret_cast<float4 *>(prow) + tid, r);
+		if (tid < AT_NH) {
+			__stcg(prow + AT_NH * AT_HD + tid, m_s[tid]);
+			__stcg(prow + AT_NH * AT_HD + 4 + tid, l_s[tid]);
+		}
+		__threadfence();
+		__syncthreads();
+		if (tid == 0) s_last = atomicAdd(&a.tickets[b], 1u) == unsigned(nact - 1);
+		__syncthreads();
+		if (!s_last) return;
+		__threadfence();
+		float M = -INFINITY;
+		for (int sp = 0; sp < nact; sp++) M = fmaxf(M, __ldcg(pb + size_t(sp) * AT_PART + AT_NH * AT_HD + h));
+		r = make_float4(0.f, 0.f, 0.f, 0.f);
+		L = 0.0f;
+		for (int s0 = 0; s0 < nact; s0 += 4) {
+			float4 v[4];
+			float ms[4], ls[4];
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+				ms[q] = -INFINITY;
+				ls[q] = 0.0f;
+				if (s0 + q < nact) {
+					const float *p = pb + size_t(s0 + q) * AT_PART;
+					v[q] = __ldcg(reinterpret_cast<const float4 *>(p) + tid);
+					ms[q] = __ldcg(p + AT_NH * AT_HD + h);
+					ls[q] = __ldcg(p + AT_NH * AT_HD + 4 + h);
+				}
+			}
+#pragma unroll
+			for (int q = 0; q < 4; q++) {
+				const float w = expf(ms[q] - M);
+				L = fmaf(ls[q], w, L);
+				ac_fma4(r, w, v[q]);
+			}
+		}
+		if (tid == 0) a.tickets[b] = 0u;
+	}
+	r.x /= L;
+	r.y /= L;
+	r.z /= L;
+	r.w /= L;
+	if (a.out) {
+		reinterpret_cast<float4 *>(a.out + size_t(b) * (AT_NH * AT_HD))[tid] = r;
+	} else {
+		const uint32_t mb = block_umax<AT_THREADS / 32>(max(max(i8_abs_bits(r.x), i8_abs_bits(r.y)), max(i8_abs_bits(r.z), i8_abs_bits(r.w))), red);
+		if (tid == 0) a.rowscale[b] = i8_row_scale(mb);
+		i8_pack4(a.x, a.groups, b, tid, r, i8_row_mul(mb));
+	}
+}
+
+// ------------------------------------------------------------------ prefill of short prompts
+// Two queries (8 rows of 4 heads) per CTA of 16 warps. q [S][1024], k and v [S][256] per prompt; blockIdx.y is the prompt.
+// Causal; on local layers a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
+constexpr int APS_THREADS = 512;
+__global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
+                                                                            const float *k, const float *v, int S, int is_local, int window,
+                                                                            int *err) {
+	extern __shared__ __align__(128) uint8_t ac_smem[];
+	constexpr int R = 8;  // query rows
+	__shared__ __align__(16) float sc[AC_KEYS][R], pr[AC_KEYS][R];
+	__shared__ float corr_s[R], l_s[R];
+	__shared__ uint64_t kbar, vbar;
+	__shared__ uint32_t red[APS_THREADS / 32];
+	float *K = reinterpret_cast<float *>(ac_smem), *V = reinterpret_cast<float *>(ac_smem + AC_BUF);
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	if (tid == 0) {
+		mbar_init(&kbar, 1);
+		mbar_init(&vbar, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	__syncthreads();
+	pdl_trigger();
+	pdl_wait();
+	const size_t r0 = size_t(blockIdx.y) * S;
+	const int s0 = int(gridDim.x - 1 - blockIdx.x) * 2;  // (the longest walks start first)
+	const int s_last = min(S - 1, s0 + 1);
+	const int j0 = (is_local && s0 >= window) ? s0 - window : 0, j1 = s_last + 1;
+	const int nch = (j1 - j0 + AC_KEYS - 1) / AC_KEYS;
+	k += (r0 + j0) * 256;
+	v += (r0 + j0) * 256;
+	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
+		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
+		fence_proxy_async();
+		mbar_expect_tx(bar, bytes);
+		bulk_load(dst, src + size_t(c) * AC_KEYS * 256, bytes, bar);
+	};
+	if (tid == 0) {
+		issue(K, k, 0, &kbar);
+		issue(V, v, 0, &vbar);
+	}
+	// row = query * 4 + head
+	float4 q0[R], q1[R];
+#pragma unroll
+	for (int r = 0; r < R; r++) {
+		const int s = s0 + (r >> 2);
+		q0[r] = q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (s < S) {
+			const float4 *qr = reinterpret_cast<const float4 *>(q + (r0 + s) * 1024 + (r & 3) * 256);
+			q0[r] = qr[lane];
+			q1[r] = qr[32 + lane];
+		}
+		// exact: the reference scales q by 1/sqrt(256) = 2^-4 before the dot products
+		q0[r].x *= 0.0625f; q0[r].y *= 0.0625f; q0[r].z *= 0.0625f; q0[r].w *= 0.0625f;
+		q1[r].x *= 0.0625f; q1[r].y *= 0.0625f; q1[r].z *= 0.0625f; q1[r].w *= 0.0625f;
+	}
+	const int d4 = tid & 63, kg = tid >> 6;  // 8 groups of 4 keys
+	float4 o[R];
+#pragma unroll
+	for (int r = 0; r < R; r++) o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+	float m = -INFINITY, l = 0.0f;  // of row `warp` (warps 0..7)
+	for (int c = 0; c < nch; c++) {
+		const int base = j0 + c * AC_KEYS, n = min(AC_KEYS, j1 - base);
+		tc_wait(&kbar, c & 1, err);
+		{
+			float t[16];
+#pragma unroll
+			for (int kk = 0; kk < 2; kk++) {
+				const float4 k0 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 4 * lane);
+				const float4 k1 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 128 + 4 * lane);
+#pragma unroll
+				for (int r = 0; r < R; r++) t[kk * 8 + r] = ac_dot8(q0[r], q1[r], k0, k1);
+			}
+			const float z = ac_reduce16(t, lane);
+			if (!(lane & 1)) sc[2 * warp + (lane >> 4)][(lane >> 1) & 7] = z;
+		}
+		__syncthreads();  // scores complete, K consumed
+		if (tid == 0 && c + 1 < nch) issue(K, k, c + 1, &kbar);
+		if (warp < R) {
+			const int s = s0 + (warp >> 2), j = base + lane;
+			const bool vis = lane < n && j <= s && !(is_local && j + window < s);
+			const float z = vis ? sc[lane][warp] : -INFINITY;
+			const float mn = fmaxf(m, warp_max(z));
+			// (a row may have no visible key in its first chunk: the second query's window starts one later)
+			const float p = vis ? expf(z - mn) : 0.0f, cr = m == -INFINITY ? 0.0f : expf(m - mn);
+			l = fmaf(l, cr, warp_sum(p));
+			m = mn;
+			pr[lane][warp] = p;
+			if (lane == 0) corr_s[warp] = cr;
+		}
+		tc_wait(&vbar, c & 1, err);
+		__syncthreads();  // probabilities complete
+#pragma unroll
+		for (int r = 0; r < R; r++) {
+			const float cr = corr_s[r];
+			o[r].x *= cr;
+			o[r].y *= cr;
+			o[r].z *= cr;
+			o[r].w *= cr;
+		}
+#pragma unroll
+		for (int kk = 0; kk < AC_KEYS / 8; kk++) {
+			const int key = kg * (AC_KEYS / 8) + kk;
+			if (key < n) {
+				const float4 vv = *reinterpret_cast<const float4 *>(V + key * 256 + 4 * d4);
+				const float4 pa = *reinterpret_cast<const float4 *>(&pr[key][0]), pb = *reinterpret_cast<const float4 *>(&pr[key][4]);
+				ac_fma4(o[0], pa.x, vv);
+				ac_fma4(o[1], pa.y, vv);
+				ac_fma4(o[2], pa.z, vv);
+				ac_fma4(o[3], pa.w, vv);
+				ac_fma4(o[4], pb.x, vv);
+				ac_fma4(o[5], pb.y, vv);
+				ac_fma4(o[6], pb.z, vv);
+				ac_fma4(o[7], pb.w, vv);
+			}
+		}
+		__syncthreads();  // V consumed
+		if (tid == 0 && c + 1 < nch) issue(V, v, c + 1, &vbar);
+	}
+	// ---- join the eight key groups (64 KB: both buffers); thread (query, k4) ends up with 4 of its query's 1024 outputs
+	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
+#pragma unroll
+	for (int r = 0; r < R; r++) jb[(kg * R + r) * 64 + d4] = o[r];
+	if (warp < R && lane == 0) l_s[warp] = l;
+	__syncthreads();
+	const int qi = tid >> 8, k4 = tid & 255, row = qi * 4 + (k4 >> 6);
+	float4 r = jb[row * 64 + (k4 & 63)];
+#pragma unroll
+	for (int g = 1; g < 8; g++) {
+		const float4 t = jb[(g * R + row) * 64 + (k4 & 63)];
+		r.x += t.x;
+		r.y += t.y;
+		r.z += t.z;
+		r.w += t.w;
+	}
+	const float L = l_s[row];
+	r.x /= L;
+	r.y /= L;
+	r.z /= L;
+	r.w /= L;
+	const int s = s0 + qi;
+	if (!x) {
+		if (s < S) reinterpret_cast<float4 *>(o_out + (r0 + s) * 1024)[k4] = r;
+		return;
+	}
+	const uint32_t mw = warp_umax(max(max(i8_abs_bits(r.x), i8_abs_bits(r.y)), max(i8_abs_bits(r.z), i8_abs_bits(r.w))));
+	if (lane == 0) red[warp] = mw;
+	__syncthreads();
+	uint32_t mb = 0;
+#pragma unroll
+	for (int w = 0; w < 8; w++) mb = max(mb, red[qi * 8 + w]);
+	if (s < S) {
+		if (k4 == 0) rowscale[r0 + s] = i8_row_scale(mb);
+		i8_pack4(x, groups, int(r0) + s, k4, r, i8_row_mul(mb));
+	}
+}
+
+}  // namespace tg

@@ -490,38 +490,9 @@ __global__ void __launch_bounds__(256) final_hidden_kernel(float *x_out, const f
 //  RoPE decode.hpp:136-211; KVCache::update_single decode.hpp:49-70;
 //  ops::attention_decode ops.hpp:224-370.)
 //
-// Grid (nsplit, B). Each CTA repeats the tiny q/k prologue, takes a contiguous
-// chunk of cache slots, and writes an un-normalised partial (m, l, o). The last
-// CTA of a sequence merges the partials in split order. The softmax is the
-// usual running-max form; the reference renormalises its output at every key,
-// which is the same function up to rounding.
-constexpr int AT_THREADS = 256;
-constexpr int AT_NWARPS = 8;
+// (The batched kernel is attn_decode_kernel in kernels_attn_cc.cuh; here is what the persistent kernels share with it.)
 constexpr int AT_HD = 256;
 constexpr int AT_NH = 4;
-
-struct AttnArgs {
-	const float *qkv;   // [B][1536] = q(4x256) | k(256) | v(256)
-	// qkv_nsplit > 0: qkv instead holds the raw K-split partial sums of the grouped q|k|v GEMM,
-	// [qkv_nsplit][B][1536], and sq / sk / sv are the column scales (splits are added in ascending order)
-	int qkv_nsplit, qkv_B;
-	const float *sq, *sk, *sv;
-	const float *rmsq;  // [256]
-	const float *rmsk;  // [256]
-	const float *cosT;  // [n_pos][256]
-	const float *sinT;
-	float *kcache;      // [B][slots][256]
-	float *vcache;
-	int slots;          // 512 on local layers, max_pos_global on global layers
-	int is_local;
-	const int *step_pos;   // [B]
-	const int *ring_base;  // [B] prompt length if it filled the ring, else 0 (decode.hpp:98-103)
-	float *part;        // [B][nsplit][4*256 + 8]
-	unsigned *tickets;  // [B]
-	float *out;         // [B][1024]
-	int nsplit;
-	int *err_flag;
-};
 
 __device__ __forceinline__ void norm_rope_head(const float *x, const float *w, const float *cosr, const float *sinr,
                                                 float scale, float *dst) {
@@ -549,210 +520,6 @@ __device__ __forceinline__ void norm_rope_head(const float *x, const float *w, c
 		dst[d] = ylo * scale;
 		dst[d + 128] = yhi * scale;
 	}
-}
-
-__global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(AttnArgs a) {
-	pdl_trigger();
-	pdl_wait();
-	__shared__ __align__(16) float qs[AT_NH][AT_HD];
-	__shared__ __align__(16) float ks[AT_HD];
-	__shared__ __align__(16) float vs[AT_HD];
-	__shared__ float wm[AT_NWARPS][AT_NH], wl[AT_NWARPS][AT_NH];
-	__shared__ __align__(16) float wo[AT_NWARPS][AT_NH][AT_HD];
-	__shared__ int s_last;
-
-	const int b = blockIdx.y, split = blockIdx.x;
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	int pos = a.step_pos[b];
-	int slot, valid;
-	if (a.is_local) {
-		int rel = pos - a.ring_base[b];
-		slot = rel % a.slots;
-		valid = min(pos + 1, a.slots);
-	} else {
-		if (pos >= a.slots) {  // cache full: refuse to write out of bounds
-			if (tid == 0) *a.err_flag = 2;
-			pos = a.slots - 1;
-		}
-		slot = pos;
-		valid = pos + 1;
-	}
-	const float *row = a.qkv + size_t(b) * (AT_NH * AT_HD + 2 * AT_HD);
-	if (a.qkv_nsplit > 0) {
-		__shared__ __align__(16) float rowbuf[AT_NH * AT_HD + 2 * AT_HD];
-		constexpr int NQ = AT_NH * AT_HD + 2 * AT_HD;
-		// four consecutive columns x up to eight splits are requested together; the splits are added in
-		// ascending order (the order of the reduce kernel)
-		const size_t sstride = size_t(a.qkv_B) * NQ;
-		for (int n = 4 * tid; n < NQ; n += 4 * AT_THREADS) {
-			const float *p = a.qkv + size_t(b) * NQ + n;
-			float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-			for (int s0 = 0; s0 < a.qkv_nsplit; s0 += 8) {
-				float4 v[8];
-#pragma unroll
-				for (int q = 0; q < 8; q++) {
-					v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-					if (s0 + q < a.qkv_nsplit) v[q] = *reinterpret_cast<const float4 *>(p + size_t(s0 + q) * sstride);
-				}
-#pragma unroll
-				for (int q = 0; q < 8; q++) {
-					acc.x += v[q].x;
-					acc.y += v[q].y;
-					acc.z += v[q].z;
-					acc.w += v[q].w;
-				}
-			}
-			const float *sc = n < AT_NH * AT_HD ? a.sq + n : (n < AT_NH * AT_HD + AT_HD ? a.sk + (n - AT_NH * AT_HD) : a.sv + (n - AT_NH * AT_HD - AT_HD));
-			const float4 s4 = *reinterpret_cast<const float4 *>(sc);
-			*reinterpret_cast<float4 *>(&rowbuf[n]) = make_float4(acc.x * s4.x, acc.y * s4.y, acc.z * s4.z, acc.w * s4.w);
-		}
-		__syncthreads();
-		row = rowbuf;
-	}
-	const float *cosr = a.cosT + size_t(pos) * AT_HD, *sinr = a.sinT + size_t(pos) * AT_HD;
-	if (warp < AT_NH) {
-		// the reference scales q by 1/sqrt(256) = 2^-4 before the dot products (ops.hpp:262,283)
-		norm_rope_head(row + warp * AT_HD, a.rmsq, cosr, sinr, 0.0625f, qs[warp]);
-	} else if (warp == AT_NH) {
-		norm_rope_head(row + AT_NH * AT_HD, a.rmsk, cosr, sinr, 1.0f, ks);
-	} else if (warp == AT_NH + 1) {
-		for (int d = lane; d < AT_HD; d += 32) vs[d] = row[AT_NH * AT_HD + AT_HD + d];
-	}
-	__syncthreads();
-
-	// chunk of slots for this CTA
-	const int chunk = (valid + a.nsplit - 1) / a.nsplit;
-	const int j0 = split * chunk, j1 = min(valid, j0 + chunk);
-	float *kc = a.kcache + size_t(b) * a.slots * AT_HD;
-	float *vc = a.vcache + size_t(b) * a.slots * AT_HD;
-	if (slot >= j0 && slot < j1) {
-		for (int d = tid; d < AT_HD; d += AT_THREADS) {
-			kc[size_t(slot) * AT_HD + d] = ks[d];
-			vc[size_t(slot) * AT_HD + d] = vs[d];
-		}
-	}
-
-	// q in registers: lane owns d = 4*lane..+3 and 128+4*lane..+3 of each head
-	float4 q0[AT_NH], q1[AT_NH];
-#pragma unroll
-	for (int h = 0; h < AT_NH; h++) {
-		q0[h] = *reinterpret_cast<const float4 *>(&qs[h][4 * lane]);
-		q1[h] = *reinterpret_cast<const float4 *>(&qs[h][128 + 4 * lane]);
-	}
-	float m[AT_NH], l[AT_NH];
-	float4 o0[AT_NH], o1[AT_NH];
-#pragma unroll
-	for (int h = 0; h < AT_NH; h++) {
-		m[h] = -INFINITY;
-		l[h] = 0.0f;
-		o0[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-		o1[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-	}
-	for (int j = j0 + warp; j < j1; j += AT_NWARPS) {
-		float4 k0v, k1v, v0v, v1v;
-		if (j == slot) {
-			k0v = *reinterpret_cast<const float4 *>(&ks[4 * lane]);
-			k1v = *reinterpret_cast<const float4 *>(&ks[128 + 4 * lane]);
-			v0v = *reinterpret_cast<const float4 *>(&vs[4 * lane]);
-			v1v = *reinterpret_cast<const float4 *>(&vs[128 + 4 * lane]);
-		} else {
-			const float *kr = kc + size_t(j) * AT_HD, *vr = vc + size_t(j) * AT_HD;
-			k0v = __ldcg(reinterpret_cast<const float4 *>(kr + 4 * lane));
-			k1v = __ldcg(reinterpret_cast<const float4 *>(kr + 128 + 4 * lane));
-			v0v = __ldcg(reinterpret_cast<const float4 *>(vr + 4 * lane));
-			v1v = __ldcg(reinterpret_cast<const float4 *>(vr + 128 + 4 * lane));
-		}
-		float s[AT_NH];
-#pragma unroll
-		for (int h = 0; h < AT_NH; h++) {
-			float t = q0[h].x * k0v.x;
-			t = fmaf(q0[h].y, k0v.y, t);
-			t = fmaf(q0[h].z, k0v.z, t);
-			t = fmaf(q0[h].w, k0v.w, t);
-			t = fmaf(q1[h].x, k1v.x, t);
-			t = fmaf(q1[h].y, k1v.y, t);
-			t = fmaf(q1[h].z, k1v.z, t);
-			t = fmaf(q1[h].w, k1v.w, t);
-			s[h] = t;
-		}
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-			for (int h = 0; h < AT_NH; h++) s[h] += __shfl_xor_sync(0xffffffffu, s[h], o);
-		}
-#pragma unroll
-		for (int h = 0; h < AT_NH; h++) {
-			float mn = fmaxf(m[h], s[h]);
-			float corr = expf(m[h] - mn);  // exp(-inf) = 0 on the first key
-			float p = expf(s[h] - mn);
-			l[h] = fmaf(l[h], corr, p);
-			o0[h].x = fmaf(p, v0v.x, o0[h].x * corr);
-			o0[h].y = fmaf(p, v0v.y, o0[h].y * corr);
-			o0[h].z = fmaf(p, v0v.z, o0[h].z * corr);
-			o0[h].w = fmaf(p, v0v.w, o0[h].w * corr);
-			o1[h].x = fmaf(p, v1v.x, o1[h].x * corr);
-			o1[h].y = fmaf(p, v1v.y, o1[h].y * corr);
-			o1[h].z = fmaf(p, v1v.z, o1[h].z * corr);
-			o1[h].w = fmaf(p, v1v.w, o1[h].w * corr);
-			m[h] = mn;
-		}
-	}
-#pragma unroll
-	for (int h = 0; h < AT_NH; h++) {
-		if (lane == 0) {
-			wm[warp][h] = m[h];
-			wl[warp][h] = l[h];
-		}
-		*reinterpret_cast<float4 *>(&wo[warp][h][4 * lane]) = o0[h];
-		*reinterpret_cast<float4 *>(&wo[warp][h][128 + 4 * lane]) = o1[h];
-	}
-	__syncthreads();
-
-	// merge the 8 warps -> CTA partial (thread owns 4 of the 1024 outputs)
-	float *prow = a.part + (size_t(b) * a.nsplit + split) * (AT_NH * AT_HD + 8);
-	for (int e = tid; e < AT_NH * AT_HD; e += AT_THREADS) {
-		const int h = e / AT_HD, d = e % AT_HD;
-		float M = -INFINITY;
-#pragma unroll
-		for (int w = 0; w < AT_NWARPS; w++) M = fmaxf(M, wm[w][h]);
-		float L = 0.0f, O = 0.0f;
-#pragma unroll
-		for (int w = 0; w < AT_NWARPS; w++) {
-			float sc = (wm[w][h] == -INFINITY) ? 0.0f : expf(wm[w][h] - M);
-			L = fmaf(wl[w][h], sc, L);
-			O = fmaf(wo[w][h][d], sc, O);
-		}
-		__stcg(prow + e, O);
-		if (d == 0) {
-			__stcg(prow + AT_NH * AT_HD + h, M);
-			__stcg(prow + AT_NH * AT_HD + 4 + h, L);
-		}
-	}
-	__threadfence();
-	__syncthreads();
-	if (tid == 0) {
-		unsigned tk = atomicAdd(&a.tickets[b], 1u);
-		s_last = (tk == unsigned(a.nsplit - 1));
-	}
-	__syncthreads();
-	if (!s_last) return;
-	__threadfence();
-	const float *pb = a.part + size_t(b) * a.nsplit * (AT_NH * AT_HD + 8);
-	for (int e = tid; e < AT_NH * AT_HD; e += AT_THREADS) {
-		const int h = e / AT_HD;
-		float M = -INFINITY;
-		for (int sp = 0; sp < a.nsplit; sp++) M = fmaxf(M, __ldcg(pb + size_t(sp) * (AT_NH * AT_HD + 8) + AT_NH * AT_HD + h));
-		float L = 0.0f, O = 0.0f;
-		for (int sp = 0; sp < a.nsplit; sp++) {
-			const float *pr = pb + size_t(sp) * (AT_NH * AT_HD + 8);
-			float ms = __ldcg(pr + AT_NH * AT_HD + h);
-			float sc = (ms == -INFINITY) ? 0.0f : expf(ms - M);
-			L = fmaf(__ldcg(pr + AT_NH * AT_HD + 4 + h), sc, L);
-			O = fmaf(__ldcg(pr + e), sc, O);
-		}
-		a.out[size_t(b) * (AT_NH * AT_HD) + e] = O / L;
-	}
-	if (tid == 0) a.tickets[b] = 0u;
 }
 
 }  // namespace tg

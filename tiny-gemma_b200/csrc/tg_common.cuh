@@ -86,13 +86,18 @@ struct GeluLut {
 	float mn;
 	float eps;
 	int size;
-	__device__ __forceinline__ float operator()(float x) const {
-		float q = (x - mn) / eps;
+	// false: the result is 0; else the table entry, from `size` on the value itself
+	__device__ __forceinline__ bool index(float x, int &idx) const {
+		const float q = (x - mn) / eps;
 		// x86 cvttss2si yields INT_MIN for NaN and out-of-range inputs, which the
 		// reference then treats as a negative index
-		if (!(q < 2147483648.0f) || q < -2147483648.0f) return 0.0f;
-		int idx = int(q);
-		if (idx < 0) return 0.0f;
+		if (!(q < 2147483648.0f) || q < -2147483648.0f) return false;
+		idx = int(q);
+		return idx >= 0;
+	}
+	__device__ __forceinline__ float operator()(float x) const {
+		int idx;
+		if (!index(x, idx)) return 0.0f;
 		if (idx >= size) return x;
 		return __ldg(table + idx);
 	}

@@ -20,6 +20,7 @@
 #include "kernels_mega.cuh"
 #include "kernels_persist.cuh"
 #include "kernels_gemm_i8.cuh"
+#include "kernels_attn_cc.cuh"
 #include "kernels_attn_tc.cuh"
 #include "kernels_prefill.cuh"
 #include "kernels_sampler.cuh"
@@ -589,6 +590,18 @@ int check_ready(const tg_model *m) {
 	return TG_OK;
 }
 
+int launch_attn_decode(const AttnArgs &a, int nb, cudaStream_t st) {
+	static bool configured[TG_MAX_DEVICES] = {false};
+	const int dev = current_device_slot();
+	if (!configured[dev]) {
+		TG_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM));
+		configured[dev] = true;
+	}
+	launch_k(attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), AC_SMEM, st, a);
+	count_launch();
+	return check_launch("attn_decode");
+}
+
 // ------------------------------------------------------------- decode step
 // One token for sequences [b0, b0+nb) (nb <= MV_MAX_B). Kernel sequence per
 // layer: QKV matvec (norm prologue) -> attention -> O matvec -> gate/up matvec
@@ -668,9 +681,7 @@ int enqueue_decode_chunk(tg_state *s, int b0, int nb, bool with_lm_head = true) 
 			a.tickets = s->attn_tickets + b0;
 			a.out = s->attn_out + size_t(b0) * qd;
 			a.err_flag = s->err_flag;
-			attn_decode_kernel<<<dim3(a.nsplit, nb), AT_THREADS, 0, st>>>(a);
-			count_launch();
-			TG_TRY(check_launch("attn_decode"));
+			TG_TRY(launch_attn_decode(a, nb, st));
 		}
 		// ---- O projection
 		{
@@ -1602,11 +1613,11 @@ int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStre
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, K);
 	if (K <= 1152)
-		launch_k(i8_pack_kernel<96, 3>, dim3(groups * 8), dim3(96), 0, st, A, sc.x, rs, M, K, groups);
+		launch_k(i8_pack_kernel<96, 3>, dim3(M), dim3(96), 0, st, A, sc.x, rs, K, groups);
 	else if (K <= 2048)
-		launch_k(i8_pack_kernel<256, 2>, dim3(groups * 8), dim3(256), 0, st, A, sc.x, rs, M, K, groups);
+		launch_k(i8_pack_kernel<256, 2>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups);
 	else
-		launch_k(i8_pack_kernel<256, 7>, dim3(groups * 8), dim3(256), 0, st, A, sc.x, rs, M, K, groups);
+		launch_k(i8_pack_kernel<256, 7>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups);
 	count_launch();
 	return check_launch("i8_pack");
 }
@@ -1617,7 +1628,7 @@ int launch_resnorm(float *h, const float *t, const float *w_post, const float *w
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, dim);
 	if (M < 1024)
-		launch_k(resnorm_i8_kernel<288, 2>, dim3(groups * 8), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+		launch_k(resnorm_i8_kernel<288, 2>, dim3(M), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
 	else if (dim <= 640)
 		launch_k(resnorm_i8_kernel<32, 5>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
 	else if (dim <= 1152)
@@ -1631,10 +1642,12 @@ int launch_resnorm(float *h, const float *t, const float *w_post, const float *w
 int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, const float *su, const float *sg, const TcScratch &sc, cudaStream_t st) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, I);
+	// (two rows of 512 or 576 threads fit an SM; beyond that the CTAs loop, so that the table is loaded once per CTA)
+	const unsigned grid = unsigned(std::min(M, 2 * g_num_sms));
 	if (I <= 2048)
-		launch_k(geglu_i8_kernel<2>, dim3(groups * 8), dim3(256), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
+		launch_k(geglu_i8_kernel<512, 1>, dim3(grid), dim3(512), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
 	else
-		launch_k(geglu_i8_kernel<7>, dim3(groups * 8), dim3(256), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
+		launch_k(geglu_i8_kernel<576, 3>, dim3(grid), dim3(576), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
 	count_launch();
 	return check_launch("geglu");
 }
@@ -1814,13 +1827,12 @@ int enqueue_decode_batched(tg_state *s, bool with_lm_head) {
 			a.nsplit = w.is_local ? s->attn_nsplit_local : s->attn_nsplit_global;
 			a.part = s->attn_part;
 			a.tickets = s->attn_tickets;
-			a.out = s->attn_out;
+			a.x = s->btc.x;  // the O projection's operand
+			a.rowscale = i8_rowscale(s->btc, B, qd);
+			a.groups = i8_groups(B);
 			a.err_flag = s->err_flag;
-			launch_k(attn_decode_kernel, dim3(a.nsplit, B), dim3(AT_THREADS), 0, st, a);
-			count_launch();
-			TG_TRY(check_launch("attn_decode"));
+			TG_TRY(launch_attn_decode(a, B, st));
 		}
-		TG_TRY(pack_activations(s->attn_out, B, qd, s->btc, st));
 		int ns = 0;
 		{
 			const QW *ws[1] = {&w.O};
@@ -1965,8 +1977,17 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 		         m->rope[w.is_local ? 1 : 0][1], s->kcache[l] + size_t(b) * slots * AT_HD, s->vcache[l] + size_t(b) * slots * AT_HD, S_seq,
 		         slots, (const float *)tc.partial, ns_qkv, w.Q.s, w.K.s, w.V.s, S, size_t(slots) * AT_HD);
 		count_launch();
-		if (S_seq <= env_int("TG_ATTN_SMALL_MAX", 384))  // short prompts: a (query, head)'s keys split over four warps, S/2 CTAs
-			launch_k(attn_prefill_small_kernel, dim3((S_seq + 1) / 2, nb), dim3(APS_THREADS), 0, st, ao, q, k, v, S_seq, w.is_local ? 1 : 0, c.n_pos_local);
+		const bool attn_small = S_seq <= env_int("TG_ATTN_SMALL_MAX", 384);  // short prompts: two queries per CTA
+		if (attn_small) {
+			static bool as_configured[TG_MAX_DEVICES] = {false};
+			const int dev = current_device_slot();
+			if (!as_configured[dev]) {
+				TG_CUDA(cudaFuncSetAttribute(attn_prefill_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM));
+				as_configured[dev] = true;
+			}
+			launch_k(attn_prefill_small_kernel, dim3((S_seq + 1) / 2, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
+			         use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, k, v, S_seq, w.is_local ? 1 : 0, c.n_pos_local, s->err_flag);
+		}
 		else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
@@ -2018,7 +2039,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 		if (use_tc) {
 			// the O, up|gate and down GEMMs leave raw K-split partial sums; the kernel that consumes them adds the splits
 			int ns = 0;
-			TG_TRY(pack_activations(ao, S, qd, tc, st));
+			if (!attn_small) TG_TRY(pack_activations(ao, S, qd, tc, st));
 			{
 				const QW *ws[1] = {&w.O};
 				TG_TRY(gemm_raw(1, ws, &ns));
