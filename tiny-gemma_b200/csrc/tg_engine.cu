@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -71,14 +72,10 @@ int g_num_sms = 148;
 constexpr int TG_MAX_DEVICES = 64;
 // Launch with the programmatic-serialization attribute (see pdl_wait in tg_common.cuh): only for kernels that
 // call pdl_wait() before their first global access. TG_PDL=0 launches them as ordinary stream-ordered kernels.
-// The batched decode step switches it off for its own launches (g_pdl_scope_off): replayed from a CUDA graph the
-// step gains nothing from it (measured 3.72 ms with ordinary edges, 3.78 ms with programmatic ones at 256
-// sequences), while the eagerly launched prefill does (178 tokens: 4.00 -> 3.80 ms).
-thread_local bool g_pdl_scope_off = false;
+// Captured into the batched step's CUDA graph the edges stay programmatic: 1.28 -> 1.08 ms at 4 sequences, 2.86 -> 2.63 at 256.
 template <typename... KArgs, typename... Args>
 inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
-	static const int use_env = env_int("TG_PDL", 1);
-	const int use = use_env && !g_pdl_scope_off;
+	static const int use = env_int("TG_PDL", 1);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
@@ -275,22 +272,11 @@ int launch_mv_b(const MvArgs &a, int pro, int epi, dim3 grid, size_t smem, cudaS
 	return launch_mv_t<MB, PRO_PLAIN, EPI_SCALE>(a, grid, smem, st);
 }
 
-// a.B may be 1..4 per launch
-int launch_mv(MvArgs a, int pro, int epi, cudaStream_t st) {
+int launch_mv(const MvArgs &a, int pro, int epi, cudaStream_t st) {
 	dim3 grid(std::min(a.ntiles, 65535), a.nsplit);
-	const int MB = a.B <= 1 ? 1 : (a.B == 2 ? 2 : 4);
-	size_t smem = mv_smem_bytes(MB, pro, epi, a.K, a.kc);
-	switch (MB) {
-		case 1:
-			return launch_mv_b<1>(a, pro, epi, grid, smem, st);
-		case 2:
-			return launch_mv_b<2>(a, pro, epi, grid, smem, st);
-		default:
-			return launch_mv_b<4>(a, pro, epi, grid, smem, st);
-	}
+	return launch_mv_b<1>(a, pro, epi, grid, mv_smem_bytes(1, pro, epi, a.K, a.kc), st);
 }
 
-constexpr int MV_MAX_B = 4;
 constexpr int STEP_RANDF = 64;  // uniforms per sequence that fit the state's step block (more: a buffer of their own)
 
 // Single-wave matvec (qmatvec_cluster_kernel): a [K, N] matrix qualifies when a tile width 16 * tpr and a
@@ -307,13 +293,15 @@ int mvc_launch_t(float *y, const float *x, const int8_t *w, const float *scales,
 	cfg.blockDim = dim3(NT);
 	cfg.dynamicSmemBytes = 0;
 	cfg.stream = st;
-	cudaLaunchAttribute attr[1];
+	cudaLaunchAttribute attr[2];
 	attr[0].id = cudaLaunchAttributeClusterDimension;
 	attr[0].val.clusterDim.x = 1;
 	attr[0].val.clusterDim.y = unsigned(ks);
 	attr[0].val.clusterDim.z = 1;
+	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	cfg.numAttrs = max_clusters ? 1 : 2;
 	if (max_clusters) {  // query only
 		TG_CUDA(cudaOccupancyMaxActiveClusters(max_clusters, qmatvec_cluster_kernel<TPR, NT>, &cfg));
 		return TG_OK;
@@ -332,7 +320,7 @@ int mvc_launch(MvcPlan p, float *y, const float *x, const int8_t *w, const float
 	if (p.tpr == 2) return mvc_launch_t<2, 512>(y, x, w, scales, K, N, p.ks, st, max_clusters);
 	return mvc_launch_t<4, 512>(y, x, w, scales, K, N, p.ks, st, max_clusters);
 }
-MvcPlan mvc_plan(int K, int N, int dev) {
+MvcPlan mvc_plan_search(int K, int N, int dev) {
 	// clusters of each (tile width, size) the device holds at once: asked once per device
 	static int max_active[TG_MAX_DEVICES][2][3][4];  // [256 / 512 threads][tile width][cluster size]
 	static bool asked[TG_MAX_DEVICES] = {false};
@@ -374,6 +362,20 @@ MvcPlan mvc_plan(int K, int N, int dev) {
 		if (best.ks) break;
 	}
 	return best;
+}
+// the plan of a shape, searched once per device (a launch takes less time than the search)
+MvcPlan mvc_plan(int K, int N, int dev) {
+	struct Entry {
+		int K, N, dev;
+		MvcPlan plan;
+	};
+	static std::mutex mu;
+	static std::vector<Entry> known;  // (at most one entry per supported shape and device)
+	std::lock_guard<std::mutex> lock(mu);
+	for (const Entry &e : known)
+		if (e.K == K && e.N == N && e.dev == dev) return e.plan;
+	known.push_back(Entry{K, N, dev, mvc_plan_search(K, N, dev)});
+	return known.back().plan;
 }
 
 }  // namespace
@@ -533,7 +535,7 @@ int state_alloc(tg_state *s) {
 	s->plan_gu = plan_matvec(D, I / MV_TN, target);
 	s->plan_dn = plan_matvec(I, D / MV_TN, target);
 	s->plan_lm = plan_matvec(D, V / MV_TN, target);
-	const int mb = std::min(B, MV_MAX_B);
+	const int mb = 1;  // (the per-phase kernels run one sequence; batches take the tensor-core step)
 	size_t pf = 0;
 	pf = std::max(pf, size_t(s->plan_qkv.nsplit) * mb * (qd + 2 * kd));
 	pf = std::max(pf, size_t(s->plan_o.nsplit) * mb * D);
@@ -603,7 +605,7 @@ int launch_attn_decode(const AttnArgs &a, int nb, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------- decode step
-// One token for sequences [b0, b0+nb) (nb <= MV_MAX_B). Kernel sequence per
+// One token of sequence b0 (nb = 1). Kernel sequence per
 // layer: QKV matvec (norm prologue) -> attention -> O matvec -> gate/up matvec
 // (residual+norm prologue, GeGLU epilogue) -> down matvec; then the lm_head
 // matvec with the last residual+norm prologue.
@@ -785,8 +787,7 @@ int enqueue_decode_batched(tg_state *s, bool with_lm_head);
 
 int enqueue_decode_all(tg_state *s) {
 	if (s->batched_ok) return enqueue_decode_batched(s, true);
-	for (int b0 = 0; b0 < s->B; b0 += MV_MAX_B) TG_TRY(enqueue_decode_chunk(s, b0, std::min(MV_MAX_B, s->B - b0)));
-	return TG_OK;
+	return enqueue_decode_chunk(s, 0, 1);
 }
 
 int enqueue_decode_step(tg_state *s) {
@@ -1624,10 +1625,10 @@ int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStre
 
 // h += norm(partial sums), then the packed norm of h for the next GEMM (resnorm_i8_kernel)
 int launch_resnorm(float *h, const float *t, const float *w_post, const float *w_pre, int M, int dim, int nsplit, const float *tscale,
-                   const TcScratch &sc, cudaStream_t st) {
+                   const TcScratch &sc, cudaStream_t st, int plan_rows = 0) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, dim);
-	if (M < 1024)
+	if ((plan_rows ? plan_rows : M) < 1024)
 		launch_k(resnorm_i8_kernel<288, 2>, dim3(M), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
 	else if (dim <= 640)
 		launch_k(resnorm_i8_kernel<32, 5>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
@@ -1656,10 +1657,12 @@ int make_gemm_map(CUtensorMap *out, const QW &w) { return make_tmap(out, w.q, w.
 
 // One launch for up to three weight matrices with the same K that multiply the same packed A
 // (q|k|v, up|gate): more column tiles per launch.
+// plan_rows: rows that tile and K-split are planned for instead of M (a row's sums depend on the K-split alone, so
+// a row of a stacked batch gets the bits that it gets by itself).
 // raw_nsplit != null: the kernel leaves raw partial sums in sc.partial ([nsplit][M][sum of N]) for a consumer
 // kernel that adds the splits and scales itself; *raw_nsplit receives the split count, no reduce is launched.
 int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const int *ldcs, int M, const TcScratch &sc,
-                         cudaStream_t st, int max_split = 16, int *raw_nsplit = nullptr) {
+                         cudaStream_t st, int max_split = 16, int *raw_nsplit = nullptr, int plan_rows = 0) {
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
@@ -1672,7 +1675,8 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		if (ws[g]->K != K) return fail(TG_ESHAPE, "grouped GEMM: the matrices must share K");
 		ntot += ws[g]->N;
 	}
-	const I8Plan pl = i8_plan(M, K, ntot, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
+	I8Plan pl = i8_plan(plan_rows ? plan_rows : M, K, ntot, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
+	if (plan_rows) pl.tok_tiles = (i8_groups(M) + pl.tg - 1) / pl.tg;
 	CUtensorMap wmap[3];
 	GemmI8Args a{};
 	ReduceGroups rg{};
@@ -1765,11 +1769,6 @@ int batched_setup(tg_state *s) {
 }
 
 int enqueue_decode_batched(tg_state *s, bool with_lm_head) {
-	struct PdlOff {
-		bool was = g_pdl_scope_off;
-		PdlOff() { g_pdl_scope_off = true; }
-		~PdlOff() { g_pdl_scope_off = was; }
-	} pdl_off;
 	tg_model *m = s->m;
 	const tg_config &c = m->cfg;
 	const int B = s->B, D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab;
@@ -1893,6 +1892,7 @@ int launch_gemm(float *C, const float *A, const QW &w, int M, float *partial, si
 // per-sequence steps (RoPE positions, cache fill, causal attention) index by sequence (blockIdx.y).
 int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	const int S = S_seq * nb;  // rows
+	const int plan_rows = s->B < 4 ? S_seq : 0;  // small batches: every sequence gets the bits of a single-sequence state
 	tg_model *m = s->m;
 	const tg_config &c = m->cfg;
 	const int D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab;
@@ -1950,11 +1950,11 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	// Tensor-core path: the norms are fused with the operand packing of the GEMM that follows them
 	// (resnorm_i8_kernel, geglu_i8_kernel).
 	auto resnorm_pack = [&](const float *t, const float *w_post, const float *w_pre, int nsplit, const float *tscale) -> int {
-		return launch_resnorm(h, t, w_post, w_pre, S, D, nsplit, tscale, tc, st);
+		return launch_resnorm(h, t, w_post, w_pre, S, D, nsplit, tscale, tc, st, plan_rows);
 	};
 	auto gemm_raw = [&](int ng, const QW *const *ws, int *ns) -> int {
 		float *Cs[3] = {nullptr, nullptr, nullptr};
-		return launch_gemm_tc_group(ng, Cs, ws, nullptr, S, tc, st, 16, ns);
+		return launch_gemm_tc_group(ng, Cs, ws, nullptr, S, tc, st, 16, ns, plan_rows);
 	};
 	if (use_tc) {
 		TG_TRY(resnorm_pack(nullptr, nullptr, m->layers[0].attn_pre, 0, nullptr));
@@ -2073,9 +2073,9 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 		TG_TRY(check_launch("prefill layer"));
 	}
 	// lm_head on the last position of every sequence (modules.hpp:232-240)
-	if (nb >= 4 && use_tc) {
-		// a group: the last rows are gathered (one strided copy), normed, and scored by ONE GEMM over the
-		// vocabulary matrix, as the batched decode step does — not nb matvecs that each stream its 302 MB
+	if (use_tc) {
+		// the last rows are gathered (one strided copy), normed, and scored by ONE GEMM over the vocabulary matrix, as the
+		// batched decode step does (for a single row too: it streams the 302 MB faster than the matvec kernel)
 		float *last = xn;  // [nb][D] (xn is free: the tensor-core path packs its norm outputs directly)
 		TG_CUDA(cudaMemcpy2DAsync(last, size_t(D) * 4, h + size_t(S_seq - 1) * D, size_t(S_seq) * D * 4, size_t(D) * 4, nb, cudaMemcpyDeviceToDevice, st));
 		launch_k(rmsnorm_rows_kernel, dim3(nb), dim3(256), 0, st, s->xnorm + size_t(b) * D, (const float *)last, m->final_norm, (const float *)nullptr, D);
@@ -2329,7 +2329,7 @@ int tg_state_create(tg_model *m, int batch, int max_pos_global, tg_state **out) 
 	s->B = batch;
 	s->max_pos_global = max_pos_global;
 	int rc = state_alloc(s);
-	if (rc == TG_OK && batch >= env_int("TG_BATCH_TC_MIN", 4)) rc = batched_setup(s);
+	if (rc == TG_OK && batch > 1) rc = batched_setup(s);
 	if (rc == TG_OK && batch == 1 && env_int("TG_MEGA", 1)) {
 		int mrc = mega_setup(s);
 		if (mrc != TG_OK) {
@@ -2451,9 +2451,8 @@ int tg_prefill(tg_state *s, const int *ids, int S, float *logits_host) {
 		TG_TRY(tg_decode(s, ids, logits_host));
 		return TG_OK;
 	}
-	// Batches that take the batched decode step prefill their prompts together, up to 16384 rows per pass (the
-	// scratch grows with the rows: 79 KB per row at the 1B shape); smaller batches stay one sequence per pass, so
-	// that a sequence's results do not depend on its neighbours' presence.
+	// The prompts of a batch are prefilled together, up to 16384 rows per pass (the scratch grows with the rows: 79 KB per
+	// row at the 1B shape).
 	const int group = (s->batched_ok && env_int("TG_GEMM_TC", 1) && env_int("TG_PREFILL_GROUP", 1)) ? std::max(1, std::min(s->B, 16384 / S)) : 1;
 	const size_t R = size_t(group) * S;  // rows per pass
 	size_t need = R * (3 * size_t(D) + 2 * qd + 2 * kd + 2 * size_t(I));
@@ -2746,7 +2745,7 @@ int tg_decode_hidden(tg_state *s, const int *ids) {
 	if (s->batched_ok) {
 		TG_TRY(enqueue_decode_batched(s, false));
 	} else {
-		for (int b0 = 0; b0 < s->B; b0 += MV_MAX_B) TG_TRY(enqueue_decode_chunk(s, b0, std::min(MV_MAX_B, s->B - b0), false));
+		TG_TRY(enqueue_decode_chunk(s, 0, 1, false));
 	}
 	if (ids) TG_TRY(check_err_flag(s));  // fed from the device: enqueue only, tg_state_check reports the error word later
 	for (int b = 0; b < s->B; b++) s->host_pos[b] += 1;
@@ -2876,10 +2875,30 @@ int tg_dev_qmatvec(float *y, const float *x, const int8_t *w, const float *scale
 	static unsigned *tickets[64] = {nullptr};
 	int dev = 0;
 	TG_CUDA(cudaGetDevice(&dev));
-	int sms = 0;
-	if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) g_num_sms = sms;
+	static int sms_of[64] = {0};
+	if (!sms_of[dev]) {
+		int sms = 0;
+		if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) sms_of[dev] = sms;
+	}
+	if (sms_of[dev]) g_num_sms = sms_of[dev];
+	// the vocabulary matrix: one CTA per SM, an equal share of the columns each (below 64 groups of 16 columns per SM the
+	// rows a CTA reads get short and too little is in flight without a K-split)
+	const int groups = (N / 16 + g_num_sms - 1) / g_num_sms;
+	if (groups >= 64 && groups <= MVW_MAX_GROUPS && K % (MVW_SETS * MVW_U) == 0) {
+		const size_t smem = size_t(K) * 4 + size_t(MVW_SETS) * groups * 64;
+		static bool configured[64] = {false};
+		if (!configured[dev]) {
+			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6912 * 4 + MVW_SETS * MVW_MAX_GROUPS * 64));
+			configured[dev] = true;
+		}
+		const int nt = (MVW_SETS * groups + 31) / 32 * 32;
+		launch_k(qmatvec_wide_kernel, dim3((N / 16 + groups - 1) / groups), dim3(nt), smem, (cudaStream_t)stream, y, x, w, scales, K, N, groups);
+		count_launch();
+		return check_launch("qmatvec_wide");
+	}
 	// the layer matrices: one wave of CTAs, K split over a thread-block cluster (TG_MV_CLUSTER=0: the split-K kernel below)
-	if (env_int("TG_MV_CLUSTER", 1)) {
+	static const int use_cluster = env_int("TG_MV_CLUSTER", 1);
+	if (use_cluster) {
 		const MvcPlan cp = mvc_plan(K, N, dev);
 		if (cp.ks) return mvc_launch(cp, y, x, w, scales, K, N, (cudaStream_t)stream);
 	}
