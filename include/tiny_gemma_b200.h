@@ -129,8 +129,9 @@ int tg_prefill(tg_state *s, const int *ids_host, int n_tokens, float *logits_hos
 int tg_decode(tg_state *s, const int *ids_host, float *logits_host);
 
 /* Continuation of a non-empty context (a further turn of a conversation): the n tokens of ids_host
- * are fed one after the other through the decode path, each seeing the cache the earlier ones left, so
- * the result equals n calls of forward_decode (transformer.hpp:75-97) on those tokens. The reference
+ * behind what the cache holds, with the result of n calls of forward_decode (transformer.hpp:75-97) on
+ * those tokens: bit for bit up to 31 tokens (they are fed one after the other through the decode path), to
+ * rounding beyond (all at once, as a prefill behind the cached context). The reference
  * cannot do this with its prefill — KVCache::update_prefill asserts an empty cache (decode.hpp:78-79,
  * listed as a limitation in README.md:96). One sequence per state; logits_host may be NULL, otherwise it
  * receives the logits after the last token. */

@@ -346,11 +346,12 @@ __global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) 
 }
 
 // ------------------------------------------------------------------ prefill of short prompts
-// Two queries (8 rows of 4 heads) per CTA of 16 warps. q [S][1024], k and v [S][256] per prompt; blockIdx.y is the prompt.
-// Causal; on local layers a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
+// Two queries (8 rows of 4 heads) per CTA of 16 warps. q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
+// prompt. Query s is the token at key off + s (off > 0: a continuation, its context comes first). Causal; on local layers
+// a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
 constexpr int APS_THREADS = 512;
 __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
-                                                                            const float *k, const float *v, int S, int is_local, int window,
+                                                                            const float *k, const float *v, int S, int off, int is_local, int window,
                                                                             int *err) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
 	constexpr int R = 8;  // query rows
@@ -371,9 +372,9 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	const size_t r0 = size_t(blockIdx.y) * S;
 	const int s0 = int(gridDim.x - 1 - blockIdx.x) * 2;  // (the longest walks start first)
 	const int s_last = min(S - 1, s0 + 1);
-	const int j0 = (is_local && s0 >= window) ? s0 - window : 0, j1 = s_last + 1;
+	const int j0 = (is_local && off + s0 >= window) ? off + s0 - window : 0, j1 = off + s_last + 1;
 	const int nch = (j1 - j0 + AC_KEYS - 1) / AC_KEYS;
-	k += (r0 + j0) * 256;
+	k += (r0 + j0) * 256;  // (a continuation is one sequence: r0 = 0)
 	v += (r0 + j0) * 256;
 	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
 		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
@@ -423,7 +424,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 		__syncthreads();  // scores complete, K consumed
 		if (tid == 0 && c + 1 < nch) issue(K, k, c + 1, &kbar);
 		if (warp < R) {
-			const int s = s0 + (warp >> 2), j = base + lane;
+			const int s = off + s0 + (warp >> 2), j = base + lane;
 			const bool vis = lane < n && j <= s && !(is_local && j + window < s);
 			const float z = vis ? sc[lane][warp] : -INFINITY;
 			const float mn = fmaxf(m, warp_max(z));

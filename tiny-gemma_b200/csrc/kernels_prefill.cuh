@@ -165,115 +165,118 @@ __global__ void geglu_kernel(float *gate, const float *up, size_t n, GeluLut lut
 	if (i < n) gate[i] = lut(gate[i]) * up[i];
 }
 
-// q/k per-head RMSNorm + RoPE at position s (offset 0) in place on
-// q [S][4*256] and k [S][256], and KVCache::update_prefill (reference
-// decode.hpp:72-105): the last min(S, slots) prompt positions go to cache
-// slots 0.. in order. One CTA (5 warps + 1) per prompt position.
+// q/k per-head RMSNorm + RoPE at position pos0 + s, in place on q [rows][4*256] and k [rows][256], and the cache append
+// (KVCache::update_prefill, reference decode.hpp:72-105): positions s >= cache_from go to cache slot
+// (s + slot_off) % slots. One CTA of six warps per position: four query heads, k, v; a lane owns d = 4 lane .. and the
+// partners 128 + d. Tables, norm weights and scales are nobody's output and are requested before the wait for the
+// predecessor; behind it there is one round trip (the projections) and one reduction.
 // With nsplit > 0 the projections arrive as the raw K-split partial sums of the grouped q|k|v GEMM
-// (part[(sp * S + s) * 1536 + n], columns q | k | v) with the column scales sq / sk / sv; the splits are
+// (part[(sp * rows + row) * 1536 + n], columns q | k | v) with the column scales sq / sk / sv; the splits are
 // added in ascending order and scaled here, and v is written out as well.
 // Several prompts of the same length share a launch: blockIdx.y is the prompt, its rows are
 // blockIdx.y * S .. of the `rows` rows of q / k / v / part, and its caches follow each other at
 // cache_stride floats.
-__global__ void __launch_bounds__(192) qk_norm_rope_prefill_kernel(float *q, float *k, float *v, const float *rmsq,
-                                                                    const float *rmsk, const float *cosT,
-                                                                    const float *sinT, float *kcache, float *vcache,
-                                                                    int S, int slots, const float *part, int nsplit,
-                                                                    const float *sq, const float *sk, const float *sv,
-                                                                    int rows, size_t cache_stride) {
+struct RopeArgs {
+	float *q, *k, *v;
+	const float *rmsq, *rmsk, *cosT, *sinT;
+	float *kcache, *vcache;
+	int S, pos0, slots, cache_from, slot_off;
+	const float *part;
+	int nsplit;
+	const float *sq, *sk, *sv;
+	int rows;
+	size_t cache_stride;
+};
+__global__ void __launch_bounds__(192) qk_norm_rope_prefill_kernel(RopeArgs a) {
+	const int s = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+	float4 w0 = one, w1 = one, c0 = one, c1 = one, n0 = one, n1 = one, f0 = one, f1 = one;
+	if (warp < 5) {
+		const float4 *w = reinterpret_cast<const float4 *>(warp < 4 ? a.rmsq : a.rmsk);
+		const float4 *c = reinterpret_cast<const float4 *>(a.cosT + size_t(a.pos0 + s) * 256), *n = reinterpret_cast<const float4 *>(a.sinT + size_t(a.pos0 + s) * 256);
+		w0 = __ldg(w + lane);
+		w1 = __ldg(w + 32 + lane);
+		c0 = __ldg(c + lane);
+		c1 = __ldg(c + 32 + lane);
+		n0 = __ldg(n + lane);
+		n1 = __ldg(n + 32 + lane);
+	}
+	if (a.nsplit > 0) {
+		const float4 *f = reinterpret_cast<const float4 *>(warp < 4 ? a.sq + warp * 256 : (warp == 4 ? a.sk : a.sv));
+		f0 = __ldg(f + lane);
+		f1 = __ldg(f + 32 + lane);
+	}
 	pdl_trigger();
 	pdl_wait();
-	const int s = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	{
-		const size_t r0 = size_t(blockIdx.y) * S;  // first row of this prompt
-		q += r0 * 1024;
-		k += r0 * 256;
-		v += r0 * 256;
-		if (part) part += r0 * 1536;
-		kcache += blockIdx.y * cache_stride;
-		vcache += blockIdx.y * cache_stride;
-	}
-	const float *cosr = cosT + size_t(s) * 256, *sinr = sinT + size_t(s) * 256;
-	const int start = (S >= slots) ? (S - slots) : 0;
-	const int c = s - start;  // cache slot, if >= 0
-	// raw element n of this position's q|k|v row (n = column in the concatenated 1536), scaled by scale[ns]
-	auto raw = [&](int n, const float *scale, int ns) -> float {
-		return sum_splits(part + size_t(s) * 1536 + n, size_t(rows) * 1536, nsplit) * scale[ns];
-	};
-	// x: the head's 256 floats (finished projection if nsplit == 0; always the destination)
-	auto norm_rope = [&](float *x, const float *w, int n0, const float *scale, int ns0) {
-		float lo[4], hi[4];
-		float ss = 0.0f;
-		if (nsplit > 0) {
-			// the lane's eight elements x four splits are requested together; splits are added in ascending order
+	const size_t row = size_t(blockIdx.y) * a.S + s;
+	float4 *x = reinterpret_cast<float4 *>(warp < 4 ? a.q + row * 1024 + warp * 256 : (warp == 4 ? a.k : a.v) + row * 256);
+	float4 lo, hi;
+	if (a.nsplit > 0) {
+		lo = hi = make_float4(0.f, 0.f, 0.f, 0.f);
+		const size_t sstride = size_t(a.rows) * 384;
+		const float4 *base = reinterpret_cast<const float4 *>(a.part) + row * 384 + warp * 64 + lane;
+		for (int s0 = 0; s0 < a.nsplit; s0 += 4) {
+			float4 u[4], v[4];
 #pragma unroll
-			for (int i = 0; i < 4; i++) lo[i] = hi[i] = 0.0f;
-			const size_t sstride = size_t(rows) * 1536;
-			const float *base = part + size_t(s) * 1536 + n0 + 4 * lane;
-			for (int s0 = 0; s0 < nsplit; s0 += 4) {
-				float4 a[4], b[4];
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					a[q] = b[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-					if (s0 + q < nsplit) {
-						a[q] = *reinterpret_cast<const float4 *>(base + size_t(s0 + q) * sstride);
-						b[q] = *reinterpret_cast<const float4 *>(base + size_t(s0 + q) * sstride + 128);
-					}
-				}
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					lo[0] += a[q].x; lo[1] += a[q].y; lo[2] += a[q].z; lo[3] += a[q].w;
-					hi[0] += b[q].x; hi[1] += b[q].y; hi[2] += b[q].z; hi[3] += b[q].w;
+			for (int i = 0; i < 4; i++) {
+				u[i] = v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+				if (s0 + i < a.nsplit) {
+					u[i] = base[size_t(s0 + i) * sstride];
+					v[i] = base[size_t(s0 + i) * sstride + 32];
 				}
 			}
 #pragma unroll
 			for (int i = 0; i < 4; i++) {
-				lo[i] *= scale[ns0 + 4 * lane + i];
-				hi[i] *= scale[ns0 + 128 + 4 * lane + i];
-			}
-		} else {
-#pragma unroll
-			for (int i = 0; i < 4; i++) {
-				lo[i] = x[4 * lane + i];
-				hi[i] = x[128 + 4 * lane + i];
+				lo.x += u[i].x; lo.y += u[i].y; lo.z += u[i].z; lo.w += u[i].w;
+				hi.x += v[i].x; hi.y += v[i].y; hi.z += v[i].z; hi.w += v[i].w;
 			}
 		}
-#pragma unroll
-		for (int i = 0; i < 4; i++) {
-			ss = fmaf(lo[i], lo[i], ss);
-			ss = fmaf(hi[i], hi[i], ss);
-		}
-		ss = warp_sum(ss);
-		const float r = inv_rms(ss, 256);
-#pragma unroll
-		for (int i = 0; i < 4; i++) {
-			const int d = 4 * lane + i;
-			float a = (lo[i] * r) * (w[d] + 1.0f);
-			float b = (hi[i] * r) * (w[d + 128] + 1.0f);
-			x[d] = fmaf(-1.0f * b, sinr[d], cosr[d] * a);
-			x[d + 128] = fmaf(a, sinr[d + 128], cosr[d + 128] * b);
-		}
-	};
-	if (warp < 4) {
-		norm_rope(q + size_t(s) * 1024 + warp * 256, rmsq, warp * 256, sq, warp * 256);
-	} else if (warp == 4) {
-		float *kr = k + size_t(s) * 256;
-		norm_rope(kr, rmsk, 1024, sk, 0);
-		__syncwarp();
-		if (c >= 0)
-			for (int d = lane; d < 256; d += 32) kcache[size_t(c) * 256 + d] = kr[d];
+		lo.x *= f0.x; lo.y *= f0.y; lo.z *= f0.z; lo.w *= f0.w;
+		hi.x *= f1.x; hi.y *= f1.y; hi.z *= f1.z; hi.w *= f1.w;
 	} else {
-		for (int d = lane; d < 256; d += 32) {
-			float val;
-			if (nsplit > 0) {
-				val = raw(1280 + d, sv, d);
-				v[size_t(s) * 256 + d] = val;
-			} else {
-				val = v[size_t(s) * 256 + d];
-			}
-			if (c >= 0) vcache[size_t(c) * 256 + d] = val;
-		}
+		lo = x[lane];
+		hi = x[32 + lane];
 	}
+	if (warp < 5) {
+		float ss = lo.x * lo.x;
+		ss = fmaf(lo.y, lo.y, ss);
+		ss = fmaf(lo.z, lo.z, ss);
+		ss = fmaf(lo.w, lo.w, ss);
+		ss = fmaf(hi.x, hi.x, ss);
+		ss = fmaf(hi.y, hi.y, ss);
+		ss = fmaf(hi.z, hi.z, ss);
+		ss = fmaf(hi.w, hi.w, ss);
+		const float r = inv_rms(warp_sum(ss), 256);
+		auto rot = [&](float &l, float &h, float wl, float wh, float cl, float ch, float nl, float nh) {
+			const float u = (l * r) * (wl + 1.0f), v = (h * r) * (wh + 1.0f);
+			// y = cos*x + rotate_half(x)*sin, rotate_half = [-x_hi, x_lo]
+			l = fmaf(-1.0f * v, nl, cl * u);
+			h = fmaf(u, nh, ch * v);
+		};
+		rot(lo.x, hi.x, w0.x, w1.x, c0.x, c1.x, n0.x, n1.x);
+		rot(lo.y, hi.y, w0.y, w1.y, c0.y, c1.y, n0.y, n1.y);
+		rot(lo.z, hi.z, w0.z, w1.z, c0.z, c1.z, n0.z, n1.z);
+		rot(lo.w, hi.w, w0.w, w1.w, c0.w, c1.w, n0.w, n1.w);
+	}
+	x[lane] = lo;
+	x[32 + lane] = hi;
+	if (warp >= 4 && s >= a.cache_from) {
+		float4 *c = reinterpret_cast<float4 *>((warp == 4 ? a.kcache : a.vcache) + blockIdx.y * a.cache_stride + size_t((s + a.slot_off) % a.slots) * 256);
+		c[lane] = lo;
+		c[32 + lane] = hi;
+	}
+}
+
+// the last `ctx` positions before pos0 of a ring cache -> rows 0 .. ctx of k / v, in order (row i: slot (i + slot_off) % slots)
+__global__ void __launch_bounds__(128) ring_gather_kernel(float *k, float *v, const float *kcache, const float *vcache, int slot_off, int slots) {
+	pdl_trigger();
+	pdl_wait();
+	const int i = blockIdx.x, d = threadIdx.x & 63;
+	const size_t src = size_t((i + slot_off) % slots) * 64 + d, dst = size_t(i) * 64 + d;
+	if (threadIdx.x < 64)
+		reinterpret_cast<float4 *>(k)[dst] = reinterpret_cast<const float4 *>(kcache)[src];
+	else
+		reinterpret_cast<float4 *>(v)[dst] = reinterpret_cast<const float4 *>(vcache)[src];
 }
 
 // ops::attention_prefill, reference ops.hpp:377-526: causal; on sliding-window

@@ -469,6 +469,7 @@ struct tg_state {
 	bool warmed = false;
 	int graph_launches = 0;
 	std::vector<int> host_pos;  // mirror of next_pos for call-order checks
+	int host_ring = 0;          // mirror of ring_base
 	// batched decode step (tensor-core GEMMs with M = batch)
 	bool batched_ok = false;
 	float *bx = nullptr, *bup = nullptr;  // [B][D] normed input, [B][I] up projection
@@ -1886,11 +1887,45 @@ int launch_gemm(float *C, const float *A, const QW &w, int M, float *partial, si
 	return TG_OK;
 }
 
+// scratch of a prefill pass over R rows of prompts of S tokens each, and room for n_ids token ids
+int ensure_prefill_scratch(tg_state *s, size_t R, int S, int n_ids) {
+	const tg_config &c = s->m->cfg;
+	const int D = c.hidden_size, I = c.intermediate_size;
+	const int qd = c.n_head * c.head_dim, kd = c.n_kv * c.head_dim;
+	const bool use_tc = env_int("TG_GEMM_TC", 1) != 0;
+	size_t need = R * (2 * size_t(D) + 2 * qd + 2 * kd) + size_t(2) * 512 * kd;
+	if (!use_tc) need += R * (size_t(D) + 2 * size_t(I));
+	size_t part = std::max(size_t(4) * R * D, size_t(1) << 22);  // split-K scratch
+	part = std::max(part, std::min(size_t(24) * R * std::max(I, qd), size_t(1) << 28));  // tensor-core GEMM partial sums (<= 1 GiB)
+	need += part;
+	need += (i8_pack_bytes(int(R), std::max(I, std::max(D, qd))) + 3) / 4 + 512;
+	need += (attn_tc_plan(S).total() + 3) / 4 + 512;  // packed q, k, v of the tensor-core attention (long prompts)
+	if (need > s->pf_floats) {
+		if (s->pf) cudaFree(s->pf);
+		s->pf = nullptr;
+		s->pf_floats = 0;
+		cudaError_t e = cudaMalloc(&s->pf, need * 4);
+		if (e != cudaSuccess) return fail(TG_ENOMEM, std::string("cudaMalloc(prefill scratch): ") + cudaGetErrorString(e));
+		s->pf_floats = need;
+	}
+	if (n_ids > s->pf_ids_cap) {
+		if (s->pf_ids) cudaFree(s->pf_ids);
+		s->pf_ids = nullptr;
+		TG_CUDA(cudaMalloc(&s->pf_ids, size_t(n_ids) * 4));
+		s->pf_ids_cap = n_ids;
+	}
+	return TG_OK;
+}
+
 // prefill of the nb sequences b .. b + nb - 1, S tokens each, already in s->pf_ids (device). Their rows are
 // stacked (row = sequence * S + position): embedding, norms, GEMMs and GeGLU work on all nb * S rows at once —
 // a GEMM over 178 rows runs at a sixth of the tensor throughput of one over thousands — and only the
 // per-sequence steps (RoPE positions, cache fill, causal attention) index by sequence (blockIdx.y).
-int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
+// pos0 >= 0: a continuation instead of a prompt (one sequence): the S_seq tokens follow pos0 cached positions and see what
+// S_seq decode steps would see (on local layers the 512 positions up to their own; a prompt's rule shows one more).
+// Scratch: the local layers' keys and values are laid out behind up to 511 rows of context.
+constexpr int APPEND_CTX = 512;
+int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1, int id0 = 0) {
 	const int S = S_seq * nb;  // rows
 	const int plan_rows = s->B < 4 ? S_seq : 0;  // small batches: every sequence gets the bits of a single-sequence state
 	tg_model *m = s->m;
@@ -1904,13 +1939,16 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	float *h = p;        p += size_t(S) * D;
 	float *xn = p;       p += size_t(S) * D;
 	float *q = p;        p += size_t(S) * qd;
-	float *k = p;        p += size_t(S) * kd;
-	float *v = p;        p += size_t(S) * kd;
+	float *k = p;        p += size_t(S + (pos0 >= 0 ? APPEND_CTX : 0)) * kd;
+	float *v = p;        p += size_t(S + (pos0 >= 0 ? APPEND_CTX : 0)) * kd;
 	float *ao = p;       p += size_t(S) * qd;
-	float *tt = p;       p += size_t(S) * D;
-	float *up = p;       p += size_t(S) * I;
-	float *gate = p;     p += size_t(S) * I;
 	const bool use_tc = env_int("TG_GEMM_TC", 1) != 0;
+	float *tt = nullptr, *up = nullptr, *gate = nullptr;  // (the tensor-core path keeps these as partial sums)
+	if (!use_tc) {
+		tt = p;          p += size_t(S) * D;
+		up = p;          p += size_t(S) * I;
+		gate = p;        p += size_t(S) * I;
+	}
 	TcScratch tc;
 	if (use_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
@@ -1921,7 +1959,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 	}
 	// long prompts: attention on the tensor cores, from packed copies of q, k and v, one sequence after the other
 	// (from 640 tokens on: below, the three packing launches cost what the tensor cores save)
-	const bool attn_tc = use_tc && S_seq > env_int("TG_ATTN_SMALL_MAX", 384) && env_int("TG_ATTN_TC", 1) &&
+	const bool attn_tc = use_tc && pos0 < 0 && S_seq > env_int("TG_ATTN_SMALL_MAX", 384) && env_int("TG_ATTN_TC", 1) &&
 	                     S_seq >= env_int("TG_ATTN_TC_MIN", 640);
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
@@ -1943,7 +1981,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 		return launch_gemm_tc(C, w, S, tc, st);
 	};
 
-	launch_k(embed_prefill_kernel, dim3(S), dim3(256), 0, st, m->wte, m->wte_s, (const int *)(s->pf_ids + size_t(b) * S_seq), h, S, D, V,
+	launch_k(embed_prefill_kernel, dim3(S), dim3(256), 0, st, m->wte, m->wte_s, (const int *)(s->pf_ids + size_t(b) * S_seq + id0), h, S, D, V,
 	         float(std::sqrt(double(D))), s->err_flag);
 	count_launch();
 	TG_TRY(check_launch("embed_prefill"));
@@ -1973,11 +2011,55 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 			TG_TRY(gemm(k, xn, w.K, false));
 			TG_TRY(gemm(v, xn, w.V, false));
 		}
-		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, q, k, v, w.rmsq, w.rmsk, m->rope[w.is_local ? 1 : 0][0],
-		         m->rope[w.is_local ? 1 : 0][1], s->kcache[l] + size_t(b) * slots * AT_HD, s->vcache[l] + size_t(b) * slots * AT_HD, S_seq,
-		         slots, (const float *)tc.partial, ns_qkv, w.Q.s, w.K.s, w.V.s, S, size_t(slots) * AT_HD);
+		float *kc = s->kcache[l] + size_t(b) * slots * AT_HD, *vc = s->vcache[l] + size_t(b) * slots * AT_HD;
+		// keys and values of the attention: the prompt's own rows; for a continuation the context in front of them, which a
+		// global cache holds in place (the new rows are written behind it) and a ring is unrolled into the scratch
+		float *kb = k, *vb = v;
+		int off = 0, window = c.n_pos_local;
+		RopeArgs ra{};
+		if (pos0 >= 0) {
+			window = c.n_pos_local - 1;
+			if (w.is_local) {
+				off = std::min(pos0, window);
+				const int first = (((pos0 - off - s->host_ring) % slots) + slots) % slots;  // slot of the oldest context row
+				if (off > 0) {
+					launch_k(ring_gather_kernel, dim3(off), dim3(128), 0, st, k, v, (const float *)kc, (const float *)vc, first, slots);
+					count_launch();
+				}
+				ra.cache_from = std::max(0, S_seq - slots);
+				ra.slot_off = (first + off) % slots;
+			} else {
+				kb = kc;
+				vb = vc;
+				off = pos0;
+				ra.cache_from = S_seq;  // (in place already)
+			}
+		} else {
+			ra.cache_from = std::max(0, S_seq - slots);
+			ra.slot_off = -ra.cache_from;
+		}
+		ra.q = q;
+		ra.k = kb + size_t(off) * AT_HD;
+		ra.v = vb + size_t(off) * AT_HD;
+		ra.rmsq = w.rmsq;
+		ra.rmsk = w.rmsk;
+		ra.cosT = m->rope[w.is_local ? 1 : 0][0];
+		ra.sinT = m->rope[w.is_local ? 1 : 0][1];
+		ra.kcache = kc;
+		ra.vcache = vc;
+		ra.S = S_seq;
+		ra.pos0 = std::max(0, pos0);
+		ra.slots = slots;
+		ra.part = tc.partial;
+		ra.nsplit = ns_qkv;
+		ra.sq = w.Q.s;
+		ra.sk = w.K.s;
+		ra.sv = w.V.s;
+		ra.rows = S;
+		ra.cache_stride = size_t(slots) * AT_HD;
+		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
 		count_launch();
-		const bool attn_small = S_seq <= env_int("TG_ATTN_SMALL_MAX", 384);  // short prompts: two queries per CTA
+		const bool attn_small = pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 384);  // short prompts: two queries per CTA
 		if (attn_small) {
 			static bool as_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
@@ -1986,7 +2068,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1) {
 				as_configured[dev] = true;
 			}
 			launch_k(attn_prefill_small_kernel, dim3((S_seq + 1) / 2, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
-			         use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, k, v, S_seq, w.is_local ? 1 : 0, c.n_pos_local, s->err_flag);
+			         use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, s->err_flag);
 		}
 		else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
@@ -2419,6 +2501,7 @@ int tg_state_reset(tg_state *s) {
 	// are never read (valid_pos bounds every loop) so they are left in place
 	TG_CUDA(cudaStreamSynchronize(s->stream));
 	s->host_pos.assign(B, 0);
+	s->host_ring = 0;
 	return TG_OK;
 }
 
@@ -2444,8 +2527,7 @@ int tg_prefill(tg_state *s, const int *ids, int S, float *logits_host) {
 	for (int b = 0; b < s->B; b++)
 		if (s->host_pos[b] != 0) return fail(TG_ESTATE, "prefill needs an empty KV cache (decode.hpp:78-79)");
 	TG_CUDA(cudaSetDevice(m->device));
-	const int D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab;
-	const int qd = c.n_head * c.head_dim, kd = c.n_kv * c.head_dim;
+	const int V = c.n_vocab;
 	if (S == 1) {
 		// a one-token prompt takes the reference's decode branch (modules.hpp:135)
 		TG_TRY(tg_decode(s, ids, logits_host));
@@ -2455,26 +2537,7 @@ int tg_prefill(tg_state *s, const int *ids, int S, float *logits_host) {
 	// row at the 1B shape).
 	const int group = (s->batched_ok && env_int("TG_GEMM_TC", 1) && env_int("TG_PREFILL_GROUP", 1)) ? std::max(1, std::min(s->B, 16384 / S)) : 1;
 	const size_t R = size_t(group) * S;  // rows per pass
-	size_t need = R * (3 * size_t(D) + 2 * qd + 2 * kd + 2 * size_t(I));
-	size_t part = std::max(size_t(4) * R * D, size_t(1) << 22);  // split-K scratch
-	part = std::max(part, std::min(size_t(24) * R * std::max(I, qd), size_t(1) << 28));  // tensor-core GEMM partial sums (<= 1 GiB)
-	need += part;
-	need += (i8_pack_bytes(int(R), std::max(I, std::max(D, qd))) + 3) / 4 + 512;
-	need += (attn_tc_plan(S).total() + 3) / 4 + 512;  // packed q, k, v of the tensor-core attention (long prompts)
-	if (need > s->pf_floats) {
-		if (s->pf) cudaFree(s->pf);
-		s->pf = nullptr;
-		s->pf_floats = 0;
-		cudaError_t e = cudaMalloc(&s->pf, need * 4);
-		if (e != cudaSuccess) return fail(TG_ENOMEM, std::string("cudaMalloc(prefill scratch): ") + cudaGetErrorString(e));
-		s->pf_floats = need;
-	}
-	if (S * s->B > s->pf_ids_cap) {
-		if (s->pf_ids) cudaFree(s->pf_ids);
-		s->pf_ids = nullptr;
-		TG_CUDA(cudaMalloc(&s->pf_ids, size_t(S) * s->B * 4));
-		s->pf_ids_cap = S * s->B;
-	}
+	TG_TRY(ensure_prefill_scratch(s, R, S, S * s->B));
 	TG_CUDA(cudaMemcpyAsync(s->pf_ids, ids, size_t(S) * s->B * 4, cudaMemcpyHostToDevice, s->stream));
 	for (int b = 0; b < s->B; b += group) TG_TRY(enqueue_prefill_seq(s, b, S, std::min(group, s->B - b)));
 	// position_ptr = S; ring base per decode.hpp:98-103
@@ -2489,6 +2552,7 @@ int tg_prefill(tg_state *s, const int *ids, int S, float *logits_host) {
 		TG_CUDA(cudaMemcpyAsync(logits_host, s->logits, size_t(s->B) * V * 4, cudaMemcpyDeviceToHost, s->stream));
 	TG_TRY(check_err_flag(s));
 	s->host_pos.assign(s->B, S);
+	s->host_ring = rb[0];
 	return TG_OK;
 }
 
@@ -2530,7 +2594,21 @@ int tg_append(tg_state *s, const int *ids, int n, float *logits_host) {
 	if (s->host_pos[0] + n > s->max_pos_global) return fail(TG_ESTATE, "global KV cache too small for the appended tokens");
 	for (int i = 0; i < n; i++)
 		if (ids[i] < 0 || ids[i] >= m->cfg.n_vocab) return fail(TG_EINVAL, "token id out of range");
-	if (s->ps_ok) {
+	// Up to APPEND_DECODE tokens go through the decode path, bit for bit what tg_decode gives. A longer turn is a prefill
+	// behind the cached context: all its tokens at once (61 tokens behind 1500: 46 -> 3 ms for 1B), the same results to
+	// rounding.
+	constexpr int APPEND_DECODE = 31, APPEND_ROWS = 4096;
+	if (n > APPEND_DECODE && env_int("TG_GEMM_TC", 1)) {
+		const int p0 = s->host_pos[0];
+		TG_TRY(ensure_prefill_scratch(s, std::min(n, APPEND_ROWS), std::min(n, APPEND_ROWS), n));
+		TG_CUDA(cudaMemcpyAsync(s->pf_ids, ids, size_t(n) * 4, cudaMemcpyHostToDevice, s->stream));
+		for (int o = 0; o < n; o += APPEND_ROWS) TG_TRY(enqueue_prefill_seq(s, 0, std::min(APPEND_ROWS, n - o), 1, p0 + o, o));
+		TG_TRY(staging_acquire(s));
+		s->host_pin[0] = p0 + n;
+		TG_CUDA(cudaMemcpyAsync(s->next_pos, s->host_pin, 4, cudaMemcpyHostToDevice, s->stream));
+		TG_CUDA(cudaMemcpyAsync(s->step_pos, s->host_pin, 4, cudaMemcpyHostToDevice, s->stream));
+		s->host_pos[0] = p0 + n;
+	} else if (s->ps_ok) {
 		// one launch of the persistent kernel: every step takes its token from the list instead of a sampler
 		if (s->force_cap < n) {
 			cudaFree(s->force_ids);
