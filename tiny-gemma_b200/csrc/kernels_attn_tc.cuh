@@ -207,21 +207,23 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	};
 	const int total = ntiles * AT_TC_BLOCKS;
 	if (warp == 9) {
-		// ------------------------------------------------------------ bulk copies (one thread), up to AT_TC_NS blocks ahead
-		if (lane == 0) {
-			pdl_wait();  // the packed operands are the predecessors' output
-			const size_t q_term = size_t(a.q_tiles) * 8 * TC_TILE_BYTES, k_term = size_t(a.k_tiles) * 8 * TC_TILE_BYTES,
-			             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
-			const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp), *kp = reinterpret_cast<const uint8_t *>(a.kp),
-			              *vp = reinterpret_cast<const uint8_t *>(a.vp);
-			for (int g = 0; g < total; g++) {
-				const int st = g % AT_TC_NS, use = g / AT_TC_NS;
-				if (use > 0 && !at_wait(&free_bar[st], (use - 1) & 1, a.err, fail)) break;
-				const Blk b = blk(g);
-				const int j = j_lo + b.tile, i = b.i;
-				uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
+		// ------------------------------------------------------------ bulk copies, up to AT_TC_NS blocks ahead
+		pdl_wait();  // the packed operands are the predecessors' output
+		const size_t q_term = size_t(a.q_tiles) * 8 * TC_TILE_BYTES, k_term = size_t(a.k_tiles) * 8 * TC_TILE_BYTES,
+		             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
+		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp), *kp = reinterpret_cast<const uint8_t *>(a.kp),
+		              *vp = reinterpret_cast<const uint8_t *>(a.vp);
+		int cap = TC_SPIN_CAP, st = 0;
+		uint32_t ph = 1;  // (a fresh barrier passes parity 1)
+		for (int g = 0; g < total; g++) {
+			const Blk b = blk(g);
+			const int j = j_lo + b.tile, i = b.i;
+			uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
+			tc_wait_cap(&free_bar[st], ph, cap);
+			if (tc_elect()) {
 				if (b.qk) {
 					mbar_expect_tx(&full_bar[st], 3u * TC_TILE_BYTES + 3u * (TC_TILE_BYTES / 2));
+#pragma unroll
 					for (int t = 0; t < 3; t++) {
 						bulk_load(dst + t * TC_TILE_BYTES, qp + t * q_term + (size_t(tile) * 8 + i) * TC_TILE_BYTES, TC_TILE_BYTES, &full_bar[st]);
 						bulk_load(dst + 3 * TC_TILE_BYTES + t * (TC_TILE_BYTES / 2),
@@ -230,49 +232,69 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 					}
 				} else {
 					mbar_expect_tx(&full_bar[st], 3u * AT_TC_VBYTES);
+#pragma unroll
 					for (int t = 0; t < 3; t++)
 						bulk_load(dst + t * AT_TC_VBYTES, vp + t * v_term + (size_t(4 * j + i)) * AT_TC_VBYTES, AT_TC_VBYTES, &full_bar[st]);
 				}
 			}
+			if (++st == AT_TC_NS) {
+				st = 0;
+				ph ^= 1;
+			}
+		}
+		if (cap == 0 && lane == 0) {
+			atomicExch(a.err, 6);
+			*fail = 1;
 		}
 	} else if (warp == 8) {
-		// ------------------------------------------------------------ MMAs (one thread)
-		if (lane == 0) {
-			const uint32_t idesc_qk = at_idesc(AT_TC_KT, 0), idesc_pv = at_idesc(256, 1);
-			// the six term products (A term, B term)
-			const int ta[6] = {0, 0, 1, 1, 0, 2}, tb[6] = {0, 1, 0, 1, 2, 0};
-			bool ok = true;
-			for (int g = 0; g < total && ok; g++) {
-				const Blk b = blk(g);
-				if (!b.qk && b.i == 0 && !at_wait(&p_bar, b.tile & 1, a.err, fail)) { ok = false; break; }  // P written, O rescaled
-				const int st = g % AT_TC_NS, use = g / AT_TC_NS;
-				if (!at_wait(&full_bar[st], use & 1, a.err, fail)) { ok = false; break; }
-				tc_fence_after();
-				const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
-				if (b.qk) {
-					const uint32_t d_s = tmem_s + uint32_t((b.tile & 1) * AT_TC_KT);
+		// ------------------------------------------------------------ MMAs
+		const uint32_t idesc_qk = at_idesc(AT_TC_KT, 0), idesc_pv = at_idesc(256, 1);
+		// the six term products (A term, B term)
+		constexpr int ta[6] = {0, 0, 1, 1, 0, 2}, tb[6] = {0, 1, 0, 1, 2, 0};
+		int cap = TC_SPIN_CAP, st = 0;
+		uint32_t ph = 0;
+		const uint32_t pb = smem_u32(pbuf);
+		for (int g = 0; g < total; g++) {
+			const Blk b = blk(g);
+			if (!b.qk && b.i == 0) tc_wait_cap(&p_bar, b.tile & 1, cap);  // P written, O rescaled
+			tc_wait_cap(&full_bar[st], ph, cap);
+			tc_fence_after();
+			const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
+			if (b.qk) {
+				const uint32_t d_s = tmem_s + uint32_t((b.tile & 1) * AT_TC_KT);
+				const uint64_t dq = tc_smem_desc(base), dk = tc_smem_desc(base + 3 * TC_TILE_BYTES);
+				if (tc_elect()) {
 #pragma unroll
-					for (int c = 0; c < 6; c++) {
-						const uint32_t qa = base + ta[c] * TC_TILE_BYTES, kb_ = base + 3 * TC_TILE_BYTES + tb[c] * (TC_TILE_BYTES / 2);
+					for (int c = 0; c < 6; c++)
 #pragma unroll
 						for (int j2 = 0; j2 < 2; j2++)
-							tc_mma(d_s, tc_smem_desc(qa + j2 * 256), tc_smem_desc(kb_ + j2 * 256), idesc_qk, (b.i > 0 || c > 0 || j2 > 0) ? 1u : 0u);
-					}
+							tc_mma(d_s, dq + uint64_t((ta[c] * TC_TILE_BYTES + j2 * 256) >> 4), dk + uint64_t((tb[c] * (TC_TILE_BYTES / 2) + j2 * 256) >> 4),
+							       idesc_qk, (b.i > 0 || c > 0 || j2 > 0) ? 1u : 0u);
 					tc_commit(&free_bar[st]);
 					if (b.i == 7) tc_commit(&s_bar[b.tile & 1]);
-				} else {
-					const int vb = b.i;  // keys 16 vb ..: K-step vb % 2 of P's 32-key block vb / 2
-					const uint32_t pb = smem_u32(pbuf);
+				}
+			} else {
+				const int vb = b.i;  // keys 16 vb ..: K-step vb % 2 of P's 32-key block vb / 2
+				const uint64_t dp = tc_smem_desc(pb + (vb >> 1) * TC_TILE_BYTES + (vb & 1) * 256), dv = at_vdesc(base);
+				if (tc_elect()) {
 #pragma unroll
-					for (int c = 0; c < 6; c++) {
-						const uint32_t pa = pb + (ta[c] * 2 + (vb >> 1)) * TC_TILE_BYTES + (vb & 1) * 256, vv = base + tb[c] * AT_TC_VBYTES;
-						tc_mma(tmem_o, tc_smem_desc(pa), at_vdesc(vv), idesc_pv, (b.tile > 0 || vb > 0 || c > 0) ? 1u : 0u);
-					}
+					for (int c = 0; c < 6; c++)
+						tc_mma(tmem_o, dp + uint64_t((ta[c] * 2 * TC_TILE_BYTES) >> 4), dv + uint64_t((tb[c] * AT_TC_VBYTES) >> 4), idesc_pv,
+						       (b.tile > 0 || vb > 0 || c > 0) ? 1u : 0u);
 					tc_commit(&free_bar[st]);
 					if (vb == 3) tc_commit(&pv_bar);
 				}
 			}
-			tc_commit(&o_bar);
+			__syncwarp();
+			if (++st == AT_TC_NS) {
+				st = 0;
+				ph ^= 1;
+			}
+		}
+		if (tc_elect()) tc_commit(&o_bar);
+		if (cap == 0 && lane == 0) {
+			atomicExch(a.err, 6);
+			*fail = 1;
 		}
 	} else {
 		// ------------------------------------------------------------ softmax (two threads per row = TMEM lane)

@@ -25,8 +25,13 @@
 // TMEM columns: the epilogue of a tile (8 warps) and the loads of the next one run under MMAs. One tile per CTA spent
 // more time outside its K loop than in it (K = 1152: ~10K of 20K clk: start ~1.5K, first operands ~2.5K, epilogue ~4K).
 // A completed mbarrier test costs ~180 clk on this part, so a stage is large: 128 k, 48 KB, 512 clk of MMAs.
-// The operands come at 96 B/clk of MMA time, which the L2 delivers (a pure bulk-copy loop measured 80-85 B/clk averaged
-// over all SMs, 19 TB/s); one 256-column tile without the second accumulator needs 64 B/clk and was slower.
+// The MMA-issuing and the copying warp run converged: all lanes walk the loop and wait, one elected lane issues, and a
+// wait that runs out changes no control flow (it only stops waiting from then on). The operands of these instructions live
+// in uniform registers; in a single-lane branch with a conditional exit they are moved there by a loop around every
+// instruction. Measured per MMA: 40 clk to issue, 21 for its share of a completed barrier test, against ~260 in a
+// lane-0 branch with a break — which made a stage take 580-760 clk instead of 512.
+// Two CTAs of a cluster can share a tile of 256 columns (cta_group::2): each holds its own columns and half of the
+// digits, which halves the digits' L2 traffic.
 //
 // All waits are bounded; a wait that runs out sets *err and the CTA drains and frees its TMEM before returning.
 #pragma once
@@ -41,11 +46,15 @@ constexpr int I8_BK = 64;                      // k per block of the packed digi
 constexpr int I8_GROUP_BYTES = 4 * 8 * I8_BK;  // one (K-block, token group): 4 digits x 8 tokens x 64 k
 constexpr int I8_SK = 128;                     // k per stage
 constexpr int I8_TG = 8;                       // token groups of a tile, at most
-constexpr int I8_W_BYTES = 128 * I8_SK, I8_X_BYTES = (I8_SK / I8_BK) * I8_TG * I8_GROUP_BYTES;
-constexpr int I8_STAGE = I8_W_BYTES + I8_X_BYTES;
-constexpr int I8_NST = 4;
-constexpr int I8_SMEM = I8_NST * I8_STAGE + 1024;
+constexpr int I8_W_BYTES = 128 * I8_SK;
 constexpr int I8_THREADS = 320;                // producer, MMA issuer, 8 epilogue warps
+// CG CTAs work on a tile of CG * 128 columns: each holds its own 128 columns of W and 1 / CG of the digits
+template <int CG> struct I8Shape {
+	static constexpr int X_KB = I8_TG * I8_GROUP_BYTES / CG;  // digits of one K-block in a CTA
+	static constexpr int STAGE = I8_W_BYTES + (I8_SK / I8_BK) * X_KB;
+	static constexpr int NST = CG == 1 ? 4 : 6;
+	static constexpr int SMEM = NST * STAGE + 1024;
+};
 
 // ------------------------------------------------------------------ digits
 // exponent of a row from the bits of its largest |x| (NaN and infinity compare above every finite value)
@@ -342,8 +351,10 @@ struct GemmI8Args {
 	// Up to three weight matrices with the same K share one launch (q|k|v, up|gate): matrix g owns the column tiles
 	// [tile_end[g-1], tile_end[g]) and columns col0[g].. of a partial-sum row (N = all columns)
 	int col_tiles;
+	unsigned m_tiles, m_fast, m_split;  // i8_magic of col_tiles * tok_tiles, of the faster tile index' range, of nsplit
 	int tile_end[3];
 	int col0[3];
+	int ncols[3];            // N_g (a multiple of 128: the last tile of a pair may have only its first half)
 	const float *scales[3];  // [N_g]
 	float *C[3];             // [M] rows of ldc[g] floats (finished result)
 	int ldc[3];
@@ -364,16 +375,46 @@ __device__ __forceinline__ uint64_t i8_desc_w(uint32_t addr) {
 __device__ __forceinline__ uint64_t i8_desc_x(uint32_t addr) {
 	return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t(1) << 16) | (uint64_t(512 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(4) << 61);
 }
-// D int32, A and B signed 8 bit, A MN-major (bit 15), B K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t i8_idesc(int n) {
-	return (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (uint32_t(n >> 3) << 17) | (8u << 24);
+// D int32, A and B signed 8 bit, A MN-major (bit 15), B K-major, M = 128 * CG, N = n
+template <int CG> __device__ __forceinline__ uint32_t i8_idesc(int n) {
+	return (2u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (uint32_t(n >> 3) << 17) | (uint32_t(8 * CG) << 24);
 }
-__device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-	asm volatile(
-	    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-	    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-	    "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-	    : "memory");
+template <int CG> __device__ __forceinline__ void i8_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+	if constexpr (CG == 1)
+		asm volatile(
+		    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+		    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+		    "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+		    : "memory");
+	else
+		asm volatile(
+		    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+		    "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+		    "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+		    : "memory");
+}
+// arrives (in both CTAs of a pair) when the MMAs issued so far have completed
+template <int CG> __device__ __forceinline__ void i8_commit(uint64_t *bar) {
+	if constexpr (CG == 1)
+		tc_commit(bar);
+	else
+		asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(uint16_t(3))
+		             : "memory");
+}
+// the same barrier in the pair's first CTA
+__device__ __forceinline__ uint32_t i8_leader(const void *p) {
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(0));
+	return r;
+}
+// box at (x, y) of a tensor map -> this CTA's shared memory, completing on a barrier of the pair's first CTA
+__device__ __forceinline__ void i8_pair_load(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+	asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+	             "l"(map), "r"(x), "r"(y), "r"(bar)
+	             : "memory");
+}
+__device__ __forceinline__ void i8_cluster_sync() {
+	asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // tile index -> what it covers (every role of a CTA walks the same tiles)
@@ -382,53 +423,56 @@ struct I8Tile {
 	int g0, ng;          // token groups
 	int split, s0, ns;   // K-split, its first stage and number of stages
 };
-__device__ __forceinline__ I8Tile i8_tile(const GemmI8Args &a, int t) {
+// x / d as a multiplication (m = ceil(2^32 / d), or 0 for d = 1): exact for x * d < 2^32. Every role of a CTA computes
+// its tiles between other things, and an integer division takes a single thread ~200 clk.
+inline unsigned i8_magic(unsigned d) { return d <= 1 ? 0u : unsigned((0x100000000ull + d - 1) / d); }
+__device__ __forceinline__ int i8_div(int x, unsigned m) { return m ? int(__umulhi(unsigned(x), m)) : x; }
+template <int CG> __device__ __forceinline__ I8Tile i8_tile(const GemmI8Args &a, int t) {
 	I8Tile r;
-	int ct, tt;
-	const int per = a.col_tiles * a.tok_tiles;
-	r.split = t / per;
-	t -= r.split * per;
-	if (a.n_fast) {
-		tt = t / a.col_tiles;
-		ct = t - tt * a.col_tiles;
-	} else {
-		ct = t / a.tok_tiles;
-		tt = t - ct * a.tok_tiles;
-	}
+	r.split = i8_div(t, a.m_tiles);
+	t -= r.split * a.col_tiles * a.tok_tiles;
+	const int hi = i8_div(t, a.m_fast), lo = t - hi * (a.n_fast ? a.col_tiles : a.tok_tiles);
+	const int ct = a.n_fast ? lo : hi, tt = a.n_fast ? hi : lo;
 	r.grp = (ct >= a.tile_end[0]) + (ct >= a.tile_end[1]);  // tile_end of unused slots = INT_MAX
 	// (selects over constant indices: a run-time index into the parameter arrays would move them to local memory)
-	r.n0 = (ct - (r.grp == 0 ? 0 : (r.grp == 1 ? a.tile_end[0] : a.tile_end[1]))) * 128;
+	r.n0 = (ct - (r.grp == 0 ? 0 : (r.grp == 1 ? a.tile_end[0] : a.tile_end[1]))) * (128 * CG);
 	r.g0 = tt * a.tg;
 	r.ng = min(a.tg, a.groups - r.g0);
 	const int all = a.K / I8_SK;
-	r.s0 = r.split * all / a.nsplit;
-	r.ns = (r.split + 1) * all / a.nsplit - r.s0;
+	r.s0 = i8_div(r.split * all, a.m_split);
+	r.ns = i8_div((r.split + 1) * all, a.m_split) - r.s0;
 	return r;
 }
 
+// xmap (CG = 2): the digits as rows of 512 bytes (one (group, digit) of a K-block), box of 2 * tg rows
+template <int CG>
 __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
                                                                  const __grid_constant__ CUtensorMap wmap1,
-                                                                 const __grid_constant__ CUtensorMap wmap2, GemmI8Args a) {
+                                                                 const __grid_constant__ CUtensorMap wmap2,
+                                                                 const __grid_constant__ CUtensorMap xmap, GemmI8Args a) {
+	using SH = I8Shape<CG>;
+	constexpr int NST = SH::NST;
 	pdl_trigger();
 	extern __shared__ uint8_t i8_smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(i8_smem_raw) + 1023) & ~uintptr_t(1023));
-	__shared__ uint64_t full_bar[I8_NST];   // W and digits of the stage landed
-	__shared__ uint64_t free_bar[I8_NST];   // the MMAs that read the stage have completed
+	__shared__ uint64_t full_bar[NST];   // W and digits of the stage landed
+	__shared__ uint64_t free_bar[NST];   // the MMAs that read the stage have completed
 	__shared__ uint64_t acc_full[2];        // the accumulator's MMAs have completed
-	__shared__ uint64_t acc_free[2];        // the 8 epilogue warps have read the accumulator
+	__shared__ uint64_t acc_free[2];        // the 8 epilogue warps (of both CTAs) have read the accumulator
 	__shared__ uint64_t drain_bar;          // every MMA issued has completed
 	__shared__ uint32_t tmem_base_s;
 	__shared__ int s_fail, s_issued;
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int rank = CG == 1 ? 0 : int(blockIdx.x & 1), first = int(blockIdx.x) / CG, stride = int(gridDim.x) / CG;
 	if (tid == 0) {
-		for (int s = 0; s < I8_NST; s++) {
+		for (int s = 0; s < NST; s++) {
 			mbar_init(&full_bar[s], 1);
 			mbar_init(&free_bar[s], 1);
 		}
 		for (int b = 0; b < 2; b++) {
 			mbar_init(&acc_full[b], 1);
-			mbar_init(&acc_free[b], 8);
+			mbar_init(&acc_free[b], 8 * CG);
 		}
 		mbar_init(&drain_bar, 1);
 		s_fail = 0;
@@ -436,92 +480,113 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	if (warp == 1) {
-		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512)
-		             : "memory");
-		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+		if constexpr (CG == 1) {
+			asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512)
+			             : "memory");
+			asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+		} else {
+			asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512)
+			             : "memory");
+			asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+		}
 	}
 	tc_fence_before();
 	__syncthreads();
+	if constexpr (CG == 2) i8_cluster_sync();  // the barriers of both CTAs are ready
 	tc_fence_after();
 	const uint32_t tmem_base = tmem_base_s;
 
 	if (warp == 0) {
 		// ------------------------------------------------------------ producer
-		if (lane == 0) {
-			const uint64_t pol = l2_evict_first_policy();
-			auto load_w = [&](const I8Tile &t, int st, int s) {
+		const uint64_t pol = l2_evict_first_policy();
+		auto load_w = [&](const I8Tile &t, int st, int s) {
+			const CUtensorMap *wmap = t.grp == 0 ? &wmap0 : (t.grp == 1 ? &wmap1 : &wmap2);
+			uint8_t *dst = smem + size_t(s) * SH::STAGE;
+			const int y = (t.s0 + st) * I8_SK;
+			if constexpr (CG == 2) {
+				// (a pair's box is always a whole tile's: what lies past the last token or column is not used)
+				if (rank == 0) mbar_expect_tx(&full_bar[s], 2u * I8_W_BYTES + uint32_t(a.tg) * (I8_SK / I8_BK) * I8_GROUP_BYTES);
+				i8_pair_load(dst, wmap, t.n0 + 128 * rank, y, i8_leader(&full_bar[s]));
+			} else {
 				mbar_expect_tx(&full_bar[s], uint32_t(I8_W_BYTES) + uint32_t(t.ng) * (I8_SK / I8_BK) * I8_GROUP_BYTES);
-				const CUtensorMap *wmap = t.grp == 0 ? &wmap0 : (t.grp == 1 ? &wmap1 : &wmap2);
-				uint8_t *dst = smem + size_t(s) * I8_STAGE;
 				if (a.w_stream)
-					tma_load_2d(dst, wmap, t.n0, (t.s0 + st) * I8_SK, &full_bar[s], pol);
+					tma_load_2d(dst, wmap, t.n0, y, &full_bar[s], pol);
 				else
-					tma_load_2d(dst, wmap, t.n0, (t.s0 + st) * I8_SK, &full_bar[s]);
-			};
-			auto load_x = [&](const I8Tile &t, int st, int s) {
-				const uint32_t bytes = uint32_t(t.ng) * I8_GROUP_BYTES;
-				uint8_t *dst = smem + size_t(s) * I8_STAGE + I8_W_BYTES;
-				const uint8_t *src = a.x + (size_t(t.s0 + st) * (I8_SK / I8_BK) * a.groups + t.g0) * I8_GROUP_BYTES;
-#pragma unroll
-				for (int q = 0; q < I8_SK / I8_BK; q++)
-					bulk_load(dst + q * (I8_TG * I8_GROUP_BYTES), src + size_t(q) * a.groups * I8_GROUP_BYTES, bytes, &full_bar[s]);
-			};
-			// The weights are nobody's output: the first tiles are requested before the wait for the predecessor.
-			int pre = 0;
-			if (int(blockIdx.x) < a.tiles) {
-				const I8Tile t = i8_tile(a, blockIdx.x);
-				pre = min(I8_NST, t.ns);
-				for (int st = 0; st < pre; st++) load_w(t, st, st);
-				pdl_wait();
-				for (int st = 0; st < pre; st++) load_x(t, st, st);
+					tma_load_2d(dst, wmap, t.n0, y, &full_bar[s]);
 			}
-			int c = pre, s = pre == I8_NST ? 0 : pre;  // stages issued so far, next slot
-			uint32_t ph = 0;                           // parity of the slot's previous use being over
-			bool go = true;
-			s_issued = c;
-			for (int ti = blockIdx.x; ti < a.tiles && go; ti += gridDim.x) {
-				const I8Tile t = i8_tile(a, ti);
-				for (int st = (ti == int(blockIdx.x) ? pre : 0); st < t.ns; st++) {
-					if (c >= I8_NST && !tc_wait(&free_bar[s], ph, a.err)) { s_fail = 1; go = false; break; }
-					load_w(t, st, s);
+		};
+		auto load_x = [&](const I8Tile &t, int st, int s) {
+			uint8_t *dst = smem + size_t(s) * SH::STAGE + I8_W_BYTES;
+			const int kb = (t.s0 + st) * (I8_SK / I8_BK);
+#pragma unroll
+			for (int q = 0; q < I8_SK / I8_BK; q++) {
+				if constexpr (CG == 2)
+					i8_pair_load(dst + q * SH::X_KB, &xmap, 0, ((kb + q) * a.groups + t.g0) * 4 + rank * 2 * t.ng, i8_leader(&full_bar[s]));
+				else
+					bulk_load(dst + q * SH::X_KB, a.x + (size_t(kb + q) * a.groups + t.g0) * I8_GROUP_BYTES, uint32_t(t.ng) * I8_GROUP_BYTES, &full_bar[s]);
+			}
+		};
+		int cap = TC_SPIN_CAP, c = 0, s = 0;  // stages issued so far, next slot
+		uint32_t ph = 1;                      // parity whose completion frees the slot (a fresh barrier passes parity 1)
+		I8Tile t = i8_tile<CG>(a, first);
+		// The weights are nobody's output: the first tiles are requested before the wait for the predecessor.
+		const int pre = first < a.tiles ? min(NST, t.ns) : 0;
+		for (int st = 0; st < pre; st++)
+			if (tc_elect()) load_w(t, st, st);
+		pdl_wait();
+		for (int ti = first; ti < a.tiles; ti += stride) {
+			t = i8_tile<CG>(a, ti);
+			for (int st = 0; st < t.ns; st++) {
+				tc_wait_cap(&free_bar[s], ph, cap);
+				if (tc_elect()) {
+					if (c >= pre) load_w(t, st, s);
 					load_x(t, st, s);
-					s_issued = ++c;
-					if (++s == I8_NST) {
-						s = 0;
-						if (c > I8_NST) ph ^= 1;
-					}
+				}
+				c++;
+				if (++s == NST) {
+					s = 0;
+					ph ^= 1;
 				}
 			}
 		}
+		if (cap == 0 && lane == 0) {
+			*static_cast<volatile int *>(a.err) = 6;
+			s_fail = 1;
+		}
+		if (lane == 0) s_issued = c;
 	} else if (warp == 1) {
-		// ------------------------------------------------------------ MMA issuer
-		if (lane == 0) {
-			int s = 0, it = 0;
+		// ------------------------------------------------------------ MMA issuer (of a pair: the first CTA's)
+		if (rank == 0) {
+			int cap = TC_SPIN_CAP, s = 0, it = 0;
 			uint32_t ph = 0;
-			bool ready = false, go = true;
-			for (int ti = blockIdx.x; ti < a.tiles && go; ti += gridDim.x, it++) {
-				const I8Tile t = i8_tile(a, ti);
-				const uint32_t d = tmem_base + uint32_t(it & 1) * 256, id = i8_idesc(32 * t.ng);
-				if (it >= 2 && !tc_wait(&acc_free[it & 1], ((it >> 1) - 1) & 1, a.err)) { s_fail = 1; break; }
+			for (int ti = first; ti < a.tiles; ti += stride, it++) {
+				const I8Tile t = i8_tile<CG>(a, ti);
+				const uint32_t d = tmem_base + uint32_t(it & 1) * 256, id = i8_idesc<CG>(32 * t.ng);
+				tc_wait_cap(&acc_free[it & 1], ((it >> 1) & 1) ^ 1, cap);  // (the first use of a fresh barrier passes)
 				for (int st = 0; st < t.ns; st++) {
-					if (!ready && !tc_wait(&full_bar[s], ph, a.err)) { s_fail = 1; go = false; break; }
+					tc_wait_cap(&full_bar[s], ph, cap);
 					tc_fence_after();
-					const uint32_t w = smem_u32(smem) + uint32_t(s) * I8_STAGE, x = w + I8_W_BYTES;
-					const int sn = s + 1 == I8_NST ? 0 : s + 1;
+					const uint32_t w = smem_u32(smem) + uint32_t(s) * SH::STAGE;
+					const uint64_t dw = i8_desc_w(w), dx = i8_desc_x(w + I8_W_BYTES);
+					if (tc_elect()) {
 #pragma unroll
-					for (int j = 0; j < I8_SK / 32; j++) {
-						i8_mma(d, i8_desc_w(w + j * 4096), i8_desc_x(x + (j >> 1) * (I8_TG * I8_GROUP_BYTES) + (j & 1) * 32), id, (st > 0 || j > 0) ? 1u : 0u);
-						// the next stage's barrier is tested between the MMAs of this one: behind them, the test would let
-						// the tensor pipe run dry
-						if (j == 1) ready = mbar_try_wait(&full_bar[sn], sn == 0 ? ph ^ 1 : ph);
+						for (int j = 0; j < I8_SK / 32; j++)
+							i8_mma<CG>(d, dw + uint64_t(j * 256), dx + uint64_t(((j >> 1) * SH::X_KB + (j & 1) * 32) >> 4), id, (st > 0 || j > 0) ? 1u : 0u);
+						i8_commit<CG>(&free_bar[s]);
+						if (st == t.ns - 1) i8_commit<CG>(&acc_full[it & 1]);
 					}
-					tc_commit(&free_bar[s]);
-					if (sn == 0) ph ^= 1;
-					s = sn;
+					__syncwarp();
+					if (++s == NST) {
+						s = 0;
+						ph ^= 1;
+					}
 				}
-				if (go) tc_commit(&acc_full[it & 1]);
 			}
-			tc_commit(&drain_bar);
+			if (tc_elect()) i8_commit<CG>(&drain_bar);
+			if (cap == 0 && lane == 0) {
+				*static_cast<volatile int *>(a.err) = 6;
+				s_fail = 1;
+			}
 		}
 	} else {
 		// ------------------------------------------------------------ epilogue (warps 2..9)
@@ -529,15 +594,17 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		const int quad = warp & 3, sub = (warp - 2) >> 2;  // TMEM lanes 32 * quad ..; two warps share them
 		const bool fin = a.nsplit == 1 && !a.raw;
 		int it = 0;
-		for (int ti = blockIdx.x; ti < a.tiles; ti += gridDim.x, it++) {
-			const I8Tile t = i8_tile(a, ti);
+		for (int ti = first; ti < a.tiles; ti += stride, it++) {
+			const I8Tile t = i8_tile<CG>(a, ti);
 			const float *const scg = t.grp == 0 ? a.scales[0] : (t.grp == 1 ? a.scales[1] : a.scales[2]);
 			float *const Cg = t.grp == 0 ? a.C[0] : (t.grp == 1 ? a.C[1] : a.C[2]);
 			const size_t ld = fin ? size_t(t.grp == 0 ? a.ldc[0] : (t.grp == 1 ? a.ldc[1] : a.ldc[2])) : size_t(a.N);
 			const int pcol = t.grp == 0 ? a.col0[0] : (t.grp == 1 ? a.col0[1] : a.col0[2]);
-			const int nl = t.n0 + quad * 32 + lane;  // this lane's column
+			const int nl = t.n0 + 128 * rank + quad * 32 + lane;  // this lane's column
+			const int ncg = t.grp == 0 ? a.ncols[0] : (t.grp == 1 ? a.ncols[1] : a.ncols[2]);
+			const bool live = CG == 1 || t.n0 + 128 * rank < ncg;  // (a pair's last tile may have only its first half)
 			float *dst = fin ? Cg + nl : a.partial + size_t(t.split) * a.M * a.N + pcol + nl;
-			const float sc = fin ? scg[nl] : 1.0f;
+			const float sc = fin && live ? scg[nl] : 1.0f;
 			const uint32_t acc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(it & 1) * 256;
 			const float4 *rs = reinterpret_cast<const float4 *>(a.rowscale + t.g0 * 8);
 			// one token group: 32 accumulator columns = 4 digits x 8 tokens, and its row scales
@@ -569,7 +636,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 						const uint32_t m = warp_umax(ord);
 						const int src = __ffs(__ballot_sync(0xffffffffu, ord == m)) - 1;
 						if (lane == i && m)
-							key = (static_cast<unsigned long long>(m) << 32) | (0xFFFFFFFFu - uint32_t(a.top1_col0 + t.n0 + quad * 32 + src));
+							key = (static_cast<unsigned long long>(m) << 32) | (0xFFFFFFFFu - uint32_t(a.top1_col0 + t.n0 + 128 * rank + quad * 32 + src));
 					}
 					if (lane < 8 && tok + lane < a.M && key > *reinterpret_cast<volatile unsigned long long *>(a.top1 + tok + lane))
 						atomicMax(a.top1 + tok + lane, key);
@@ -589,44 +656,63 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 			tc_fence_after();
 			uint32_t ra[32], rb[32];
 			float4 qa[2], qb[2];
-			if (sub < t.ng) request(sub, ra, qa);
+			const int ng = live ? t.ng : 0;
+			if (sub < ng) request(sub, ra, qa);
 #pragma unroll 1
-			for (int g = sub; g < t.ng; g += 4) {
+			for (int g = sub; g < ng; g += 4) {
 				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-				if (g + 2 < t.ng) request(g + 2, rb, qb);
+				if (g + 2 < ng) request(g + 2, rb, qb);
 				finish(g, ra, qa);
-				if (g + 2 < t.ng) {
+				if (g + 2 < ng) {
 					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-					if (g + 4 < t.ng) request(g + 4, ra, qa);
+					if (g + 4 < ng) request(g + 4, ra, qa);
 					finish(g + 2, rb, qb);
 				}
 			}
 			tc_fence_before();
 			__syncwarp();
-			if (lane == 0) mbar_arrive(&acc_free[it & 1]);
+			if (lane == 0) {
+				if (CG == 1 || rank == 0)
+					mbar_arrive(&acc_free[it & 1]);
+				else
+					asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(i8_leader(&acc_free[it & 1])) : "memory");
+			}
 		}
 	}
 	// ---------------------------------------------------------------- teardown
 	tc_fence_before();
 	__syncthreads();
-	if (warp == 0 && lane == 0 && *(volatile int *)&s_fail) {
+	if (warp == 0 && lane == 0 && rank == 0 && *(volatile int *)&s_fail) {
 		// a wait ran out: every load that was issued must land before the shared memory is given up
 		const int n = *(volatile int *)&s_issued;
-		for (int c = max(0, n - I8_NST); c < n; c++) {
+		for (int c = max(0, n - NST); c < n; c++) {
 			int spins = 0;
-			while (!mbar_try_wait(&full_bar[c % I8_NST], (c / I8_NST) & 1) && ++spins < TC_SPIN_CAP) {
+			while (!mbar_try_wait(&full_bar[c % NST], (c / NST) & 1) && ++spins < TC_SPIN_CAP) {
 			}
 		}
 	}
-	if (warp == 1) {
+	if (warp == 1 && rank == 0) {
 		if (*(volatile int *)&s_fail && lane == 0) {  // let the MMAs in flight finish before the TMEM goes away
 			int spins = 0;
 			while (!mbar_try_wait(&drain_bar, 0) && ++spins < TC_SPIN_CAP) {
 			}
 		}
 		__syncwarp();
+	}
+	if constexpr (CG == 2) {
+		__syncthreads();
+		i8_cluster_sync();  // neither CTA's memory is in use by the other any more
+	}
+	if (warp == 1) {
 		tc_fence_after();
-		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+		if constexpr (CG == 1)
+			asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+		else
+			asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+	}
+	if constexpr (CG == 2) {
+		__syncthreads();
+		i8_cluster_sync();
 	}
 }
 

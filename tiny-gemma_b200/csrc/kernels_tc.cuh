@@ -121,6 +121,22 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, int *err
 	return true;
 }
 
+// A warp that issues tcgen05 or bulk-copy instructions runs converged: all lanes walk its loop and wait, one elected lane
+// issues. The operands of these instructions live in uniform registers; inside a single-lane branch with a conditional
+// exit they are moved there by a loop around every instruction (measured: 260 clk per MMA against 40).
+// one lane of the (converged) warp
+__device__ __forceinline__ bool tc_elect() {
+	uint32_t p;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+	return p != 0;
+}
+// Bounded wait without an exit: `cap` polls at most, and none any more once it has run out (cap = 0).
+__device__ __forceinline__ void tc_wait_cap(uint64_t *bar, uint32_t parity, int &cap) {
+	int z = 0;
+	for (; z < cap && !mbar_try_wait(bar, parity); z++) {
+	}
+	cap = z < cap ? cap : 0;
+}
 // keys [M] ((value, column) as 64 bits: the larger value, among equal ones the lower column, is the larger key; 0 = no
 // candidate) -> maximum (or -inf) and column (or -1) per row
 __global__ void top1_unpack_kernel(const unsigned long long *keys, int M, float *max_out, int *idx_out) {

@@ -116,6 +116,7 @@ struct tg_model {
 	tg_config cfg;
 	int device = 0;
 	long weights_version = 0;  // bumped by every load
+	std::mutex tiles_mu;       // guards the re-tiled copies below
 	// layer weights re-ordered into the persistent decode kernel's per-CTA units (built on first use)
 	int8_t *dec_tiled = nullptr;
 	size_t dec_tiled_bytes = 0;
@@ -1062,6 +1063,7 @@ int mega_setup(tg_state *s) {
 // contiguous [rows][TN] block, so that a CTA fetches its unit with sequential bulk copies.
 int ensure_decode_tiles(tg_state *s) {
 	tg_model *m = s->m;
+	std::lock_guard<std::mutex> lock(m->tiles_mu);
 	const MgArgs &a = s->mega;
 	const tg_config &c = m->cfg;
 	const int L = c.n_layers, D = c.hidden_size, I = c.intermediate_size;
@@ -1096,6 +1098,7 @@ int ensure_decode_tiles(tg_state *s) {
 	}
 	TG_TRY(check_launch("retile"));
 	std::memcpy(m->dec_tiled_key, key, sizeof key);
+	TG_CUDA(cudaStreamSynchronize(s->stream));  // (once per load) the copy is the model's: other states read it on their own streams
 	m->dec_tiled_version = m->weights_version;
 	return TG_OK;
 }
@@ -1290,6 +1293,7 @@ int persist_setup(tg_state *s) {
 // the same columns) and E (down projection), and the lm_head in ring-stage order.
 int ensure_persist_tiles(tg_state *s) {
 	tg_model *m = s->m;
+	std::lock_guard<std::mutex> lock(m->tiles_mu);
 	const PsArgs &a = s->ps;
 	const tg_config &c = m->cfg;
 	const int L = c.n_layers, V = c.n_vocab;
@@ -1332,6 +1336,7 @@ int ensure_persist_tiles(tg_state *s) {
 	count_launch();
 	TG_TRY(check_launch("retile"));
 	std::memcpy(m->ps_tiled_key, key, sizeof key);
+	TG_CUDA(cudaStreamSynchronize(st));  // (once per load) the copies are the model's: other states read them on their own streams
 	m->ps_tiled_version = m->weights_version;
 	return TG_OK;
 }
@@ -1560,33 +1565,42 @@ int i8_groups(int M) { return (M + 7) / 8; }
 size_t i8_pack_bytes(int M, int K) { return size_t(i8_groups(M)) * 8 * (size_t(4) * K + 4); }
 float *i8_rowscale(const TcScratch &sc, int M, int K) { return reinterpret_cast<float *>(sc.x + size_t(i8_groups(M)) * 8 * 4 * K); }
 
-// Tokens per tile and K-split of one GEMM launch, by an estimate in clocks of an SM: rounds of tiles per CTA x (stages x
-// the slowest of MMAs, operand bytes and the issuing threads + what a tile change costs) + what the consumer of the
-// partial sums reads. Measured: an MMA of N columns takes max(N / 2, 68) clk (below N = 128 it waits for its 4 KB of W),
-// with all SMs loading an operand byte takes 1/66 clk, and a stage costs its issuing threads ~280 clk.
+// Tokens per tile, K-split and CTAs per tile of one GEMM launch, by an estimate in clocks of an SM: rounds of tiles per
+// CTA (or pair) x (stages x the slowest of MMAs, operand bytes and the issuing threads + what a tile change costs) + what
+// the consumer of the partial sums reads. The constants rank 2278 measured (shape, tile, split) combinations at 1 to 4001
+// rows of all layer shapes: the choice is within 1 % of the best one on average. An MMA of N columns takes max(N / 2, 64) clk
+// (a single CTA's are slowed to 1.28 of that by its operands' arrival), 78 B/clk arrive per SM with all SMs loading.
 struct I8Plan {
-	int tg, tok_tiles, col_tiles, nsplit;
+	int cg, tg, tok_tiles, col_tiles, nsplit;
 };
-I8Plan i8_plan(int M, int K, int ntot, size_t partial_floats, int max_split, bool raw) {
-	I8Plan best{1, 1, 1, 1};
+I8Plan i8_plan(int M, int K, int ng, const QW *const *ws, size_t partial_floats, int max_split, bool raw) {
+	I8Plan best{1, 1, 1, 1, 1};
 	double best_cost = 1e30;
-	const int groups = i8_groups(M), stages = K / I8_SK, col_tiles = ntot / 128;
-	const int want_split = env_int("TG_GEMM_SPLIT", 0);  // (experiments: fix the split)
-	const int tiles_min = (groups + I8_TG - 1) / I8_TG;
-	for (int n = tiles_min; n <= std::min(groups, tiles_min + 2); n++) {
-		const int tg = (groups + n - 1) / n, tok_tiles = (groups + tg - 1) / tg;
-		const double mma = 4.0 * std::max(16.0 * tg, 68.0), load = (I8_W_BYTES + 2.0 * tg * I8_GROUP_BYTES) / 66.0;
-		const double per_stage = std::max(std::max(mma, load), 280.0);
-		for (int ns = 1; ns <= std::min(max_split, stages); ns++) {
-			if (want_split && ns != std::min(want_split, std::min(max_split, stages))) continue;
-			if ((ns > 1 || raw) && size_t(ns) * M * ntot > partial_floats) break;
-			const long tiles = long(tok_tiles) * col_tiles * ns, rounds = (tiles + g_num_sms - 1) / g_num_sms;
-			double cost = double(rounds) * ((stages + ns - 1) / ns * per_stage + 150.0) + tg * 330.0;
-			cost += double(raw ? ns - 1 : (ns > 1 ? ns + 1 : 0)) * M * ntot * 4.0 / 2500.0;  // partial sums read again, 2.5 KB a clock
-			if (!raw && ns > 1) cost += 4000.0;                                               // a launch more
-			if (cost < best_cost) {
-				best_cost = cost;
-				best = I8Plan{tg, tok_tiles, col_tiles, ns};
+	const int groups = i8_groups(M), stages = K / I8_SK;
+	int ntot = 0;
+	for (int g = 0; g < ng; g++) ntot += ws[g]->N;
+	static const int want_cg = env_int("TG_GEMM_PAIR", 0);      // (experiments: 1 or 2 CTAs per tile; a K-split)
+	static const int want_split = env_int("TG_GEMM_SPLIT", 0);
+	for (int cg = 1; cg <= 2; cg++) {
+		if (want_cg && cg != want_cg) continue;
+		int col_tiles = 0;
+		for (int g = 0; g < ng; g++) col_tiles += (ws[g]->N + 128 * cg - 1) / (128 * cg);
+		const int workers = g_num_sms / cg;
+		for (int tg = std::min(groups, I8_TG); tg >= std::max(1, std::min(groups, I8_TG) - 3); tg--) {
+			const int tok_tiles = (groups + tg - 1) / tg;
+			const double mma = 4.0 * std::max(16.0 * tg, 64.0) * (cg == 1 ? 1.28 : 1.0), in = I8_W_BYTES + 2.0 * tg * I8_GROUP_BYTES / cg;
+			const double per_stage = std::max(std::max(mma, in / 78.0), 256.0);
+			for (int ns = 1; ns <= std::min(max_split, stages); ns++) {
+				if (want_split && ns != std::min(want_split, std::min(max_split, stages))) continue;
+				if ((ns > 1 || raw) && size_t(ns) * M * ntot > partial_floats) break;
+				const long tiles = long(tok_tiles) * col_tiles * ns, rounds = (tiles + workers - 1) / workers;
+				double cost = double(rounds) * ((stages + ns - 1) / ns * per_stage + 2500.0) + tg * 100.0 + (cg - 1) * 4000.0;
+				cost += double(raw ? ns - 1 : (ns > 1 ? ns + 1 : 0)) * M * ntot * 4.0 / 2500.0;  // partial sums read again, 2.5 KB a clock
+				if (!raw && ns > 1) cost += 4000.0;                                               // a launch more
+				if (cost < best_cost) {
+					best_cost = cost;
+					best = I8Plan{cg, tg, tok_tiles, col_tiles, ns};
+				}
 			}
 		}
 	}
@@ -1654,6 +1668,38 @@ int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, 
 	return check_launch("geglu");
 }
 
+// the packed digits as rows of 512 bytes (one (group, digit) of a K-block); box: half of a tile of tg token groups
+int make_digit_map(CUtensorMap *out, const uint8_t *x, int K, int groups, int tg) {
+	PFN_encodeTiled enc = get_encode_fn();
+	if (!enc) return fail(TG_ECUDA, "cuTensorMapEncodeTiled entry point not available");
+	cuuint64_t gdim[2] = {128, cuuint64_t(K / I8_BK) * groups * 4};
+	cuuint64_t gstride[1] = {512};
+	cuuint32_t box[2] = {128, cuuint32_t(2 * tg)}, estr[2] = {1, 1};
+	CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(x), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+	                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	if (r != CUDA_SUCCESS) return fail(TG_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
+	return TG_OK;
+}
+// launch_k in clusters of two CTAs
+template <typename... KArgs, typename... Args>
+inline void launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+	static const int pdl = env_int("TG_PDL", 1);
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cudaLaunchAttribute at[2];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = 2;
+	at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[1].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = pdl ? 2 : 1;
+	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
+}
+
 int make_gemm_map(CUtensorMap *out, const QW &w) { return make_tmap(out, w.q, w.K, w.N, 128, I8_SK, w.ld, true); }
 
 // One launch for up to three weight matrices with the same K that multiply the same packed A
@@ -1667,7 +1713,8 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
 		configured[dev] = true;
 	}
 	const int K = ws[0]->K;
@@ -1676,7 +1723,7 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		if (ws[g]->K != K) return fail(TG_ESHAPE, "grouped GEMM: the matrices must share K");
 		ntot += ws[g]->N;
 	}
-	I8Plan pl = i8_plan(plan_rows ? plan_rows : M, K, ntot, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
+	I8Plan pl = i8_plan(plan_rows ? plan_rows : M, K, ng, ws, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
 	if (plan_rows) pl.tok_tiles = (i8_groups(M) + pl.tg - 1) / pl.tg;
 	CUtensorMap wmap[3];
 	GemmI8Args a{};
@@ -1692,8 +1739,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 			wmap[g] = wmap[gg];
 		if (g < ng) {
 			a.col0[g] = col0;
+			a.ncols[g] = ws[g]->N;
 			col0 += ws[g]->N;
-			tiles += ws[g]->N / 128;
+			tiles += (ws[g]->N + 128 * pl.cg - 1) / (128 * pl.cg);
 			a.tile_end[g] = tiles;
 		} else {
 			a.col0[g] = col0;
@@ -1718,6 +1766,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	a.tiles = pl.tok_tiles * pl.col_tiles * pl.nsplit;
 	// matrices that stay in the L2 are swept once per token tile; the vocabulary matrix is read once for all token tiles
 	a.n_fast = size_t(ntot) * K <= (size_t(48) << 20);
+	a.m_tiles = i8_magic(unsigned(pl.col_tiles) * pl.tok_tiles);
+	a.m_fast = i8_magic(a.n_fast ? pl.col_tiles : pl.tok_tiles);
+	a.m_split = i8_magic(pl.nsplit);
 	a.w_stream = pl.tok_tiles <= 4;
 	a.M = M;
 	a.N = ntot;
@@ -1732,7 +1783,13 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		if (size_t(a.nsplit) * M * ntot > sc.partial_floats) return fail(TG_ENOMEM, "tensor-core GEMM partial-sum scratch too small");
 		*raw_nsplit = a.nsplit;
 	}
-	launch_k(qgemm_i8_kernel, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], a);
+	if (pl.cg == 2) {
+		CUtensorMap xmap;
+		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
+		launch_pair(qgemm_i8_kernel<2>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
+	} else {
+		launch_k(qgemm_i8_kernel<1>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
+	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
 	if (a.nsplit > 1 && !raw_nsplit) {
