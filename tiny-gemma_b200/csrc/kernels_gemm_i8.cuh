@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 		for (int j = 0; j < PER; j++) acc[j] = z4;
 		const float4 *base = reinterpret_cast<const float4 *>(t + size_t(row) * dim);
 		const size_t stride = size_t(M) * n4;
-		constexpr int QB = NT == 32 ? 1 : 4;  // splits requested together
+		constexpr int QB = NT == 32 ? 1 : 8;  // splits requested together
 		for (int s0 = 0; s0 < nsplit; s0 += QB) {
 			float4 q[QB][PER];
 #pragma unroll

@@ -675,7 +675,7 @@ __global__ void retile_lm_kernel(int8_t *dst, const int8_t *src, int V, int ngro
 
 // lut::GeLUTable::lookup (reference ops.hpp:41-51) with the table kept L2-resident
 __device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint64_t keep) {
-	const float q = (x - t.mn) / t.eps;
+	const float q = t.inv != 0.0f ? (x - t.mn) * t.inv : (x - t.mn) / t.eps;
 	if (!(q < 2147483648.0f) || q < -2147483648.0f) return 0.0f;  // (x86 cvttss2si: INT_MIN, a negative index)
 	const int idx = int(q);
 	if (idx < 0) return 0.0f;

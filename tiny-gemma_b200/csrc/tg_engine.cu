@@ -586,7 +586,11 @@ int state_alloc(tg_state *s) {
 	return TG_OK;
 }
 
-GeluLut make_lut(const tg_model *m) { return GeluLut{m->gelu, m->gelu_min, m->gelu_eps, m->gelu_size}; }
+GeluLut make_lut(const tg_model *m) {
+	int e = 0;
+	const bool pow2 = std::frexp(m->gelu_eps, &e) == 0.5f && std::abs(e) < 100;
+	return GeluLut{m->gelu, m->gelu_min, m->gelu_eps, m->gelu_size, pow2 ? 1.0f / m->gelu_eps : 0.0f};
+}
 
 int check_ready(const tg_model *m) {
 	if (!m->rope[0][0] || !m->rope[1][0] || !m->gelu)
@@ -1596,7 +1600,7 @@ I8Plan i8_plan(int M, int K, int ng, const QW *const *ws, size_t partial_floats,
 				const long tiles = long(tok_tiles) * col_tiles * ns, rounds = (tiles + workers - 1) / workers;
 				double cost = double(rounds) * ((stages + ns - 1) / ns * per_stage + 2500.0) + tg * 100.0 + (cg - 1) * 4000.0;
 				cost += double(raw ? ns - 1 : (ns > 1 ? ns + 1 : 0)) * M * ntot * 4.0 / 2500.0;  // partial sums read again, 2.5 KB a clock
-				if (!raw && ns > 1) cost += 4000.0;                                               // a launch more
+				cost += raw ? (ns + 7) / 8 * 600.0 : (ns > 1 ? 4000.0 : 0.0);  // its dependent round trips; a launch more
 				if (cost < best_cost) {
 					best_cost = cost;
 					best = I8Plan{cg, tg, tok_tiles, col_tiles, ns};
