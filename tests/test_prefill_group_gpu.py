@@ -1,0 +1,25 @@
+"""Equal prompts prefilled together against each of them alone, on both sides of the line between the attention kernels
+of short prompts and of many rows, with lengths that end inside a tile of 32 queries and of 64 keys (the GEMMs see other
+row counts, so the logits agree to rounding)."""
+
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,S", [(2, 479), (2, 481), (31, 31), (31, 33), (5, 193), (13, 95), (2, 961), (256, 4)])
+def test_group_is_each_prompt(capi, synth, weights_270m, n, S):
+    m = capi.Model("270m").load_file(weights_270m)
+    m.build_tables(1 << 20)
+    prompts = np.stack([synth.random_prompt(S, 40 + i) for i in range(n)])
+    st, one = m.state(n, S + 8), m.state(1, S + 8)
+    logits = st.prefill(prompts)
+    for i in sorted({0, 1, n // 2, n - 1}):
+        one.reset()
+        assert rel_l2(logits[i], one.prefill(prompts[i])[0]) <= 5e-5, i
+    st.close()
+    one.close()
+    m.close()

@@ -44,6 +44,18 @@ __device__ __forceinline__ float ac_dot8(const float4 &q0, const float4 &q1, con
 	t = fmaf(q1.z, k1.z, t);
 	return fmaf(q1.w, k1.w, t);
 }
+// the same two products per instruction (the two halves are added at the end)
+__device__ __forceinline__ float ac_dot8x2(const float4 &q0, const float4 &q1, const float4 &k0, const float4 &k1) {
+	float2 t = make_float2(q0.x * k0.x, q0.y * k0.y);
+	t = ffma2(make_float2(q0.z, q0.w), make_float2(k0.z, k0.w), t);
+	t = ffma2(make_float2(q1.x, q1.y), make_float2(k1.x, k1.y), t);
+	t = ffma2(make_float2(q1.z, q1.w), make_float2(k1.z, k1.w), t);
+	return t.x + t.y;
+}
+__device__ __forceinline__ void ac_fma4x2(float4 &o, float p, const float4 &v) {
+	const float2 pp = make_float2(p, p), lo = ffma2(pp, make_float2(v.x, v.y), make_float2(o.x, o.y)), hi = ffma2(pp, make_float2(v.z, v.w), make_float2(o.z, o.w));
+	o = make_float4(lo.x, lo.y, hi.x, hi.y);
+}
 __device__ __forceinline__ void ac_fma4(float4 &o, float p, const float4 &v) {
 	o.x = fmaf(p, v.x, o.x);
 	o.y = fmaf(p, v.y, o.y);
@@ -346,7 +358,8 @@ __global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) 
 }
 
 // ------------------------------------------------------------------ prefill of short prompts
-// Two queries (8 rows of 4 heads) per CTA of 16 warps. q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
+// Two queries (8 rows of 4 heads) per CTA of 16 warps; the FMAs and the score reductions bound it (~920 issue slots per 32
+// keys and step), so products are packed two to an instruction. q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
 // prompt. Query s is the token at key off + s (off > 0: a continuation, its context comes first). Causal; on local layers
 // a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
 constexpr int APS_THREADS = 512;
@@ -416,7 +429,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 				const float4 k0 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 4 * lane);
 				const float4 k1 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 128 + 4 * lane);
 #pragma unroll
-				for (int r = 0; r < R; r++) t[kk * 8 + r] = ac_dot8(q0[r], q1[r], k0, k1);
+				for (int r = 0; r < R; r++) t[kk * 8 + r] = ac_dot8x2(q0[r], q1[r], k0, k1);
 			}
 			const float z = ac_reduce16(t, lane);
 			if (!(lane & 1)) sc[2 * warp + (lane >> 4)][(lane >> 1) & 7] = z;
@@ -451,14 +464,14 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 			if (key < n) {
 				const float4 vv = *reinterpret_cast<const float4 *>(V + key * 256 + 4 * d4);
 				const float4 pa = *reinterpret_cast<const float4 *>(&pr[key][0]), pb = *reinterpret_cast<const float4 *>(&pr[key][4]);
-				ac_fma4(o[0], pa.x, vv);
-				ac_fma4(o[1], pa.y, vv);
-				ac_fma4(o[2], pa.z, vv);
-				ac_fma4(o[3], pa.w, vv);
-				ac_fma4(o[4], pb.x, vv);
-				ac_fma4(o[5], pb.y, vv);
-				ac_fma4(o[6], pb.z, vv);
-				ac_fma4(o[7], pb.w, vv);
+				ac_fma4x2(o[0], pa.x, vv);
+				ac_fma4x2(o[1], pa.y, vv);
+				ac_fma4x2(o[2], pa.z, vv);
+				ac_fma4x2(o[3], pa.w, vv);
+				ac_fma4x2(o[4], pb.x, vv);
+				ac_fma4x2(o[5], pb.y, vv);
+				ac_fma4x2(o[6], pb.z, vv);
+				ac_fma4x2(o[7], pb.w, vv);
 			}
 		}
 		__syncthreads();  // V consumed

@@ -46,6 +46,8 @@ constexpr int AT_TC_VBYTES = 8192;                 // one term of a V block: [16
 __global__ void __launch_bounds__(256) attn_pack_v_kernel(const float *v, __nv_bfloat16 *out, int S, int nblocks) {
 	pdl_trigger();
 	pdl_wait();
+	v += size_t(blockIdx.y) * S * 256;  // blockIdx.y: the prompt
+	out += size_t(blockIdx.y) * 3 * nblocks * 4096;
 	const size_t term_stride = size_t(nblocks) * 4096;  // elements
 	const size_t n_items = size_t(nblocks) * 16 * 32;   // (key, 8 consecutive dimensions)
 	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_items; c += size_t(gridDim.x) * blockDim.x) {
@@ -135,6 +137,7 @@ __device__ __forceinline__ bool at_exchange(float *val, int *tag, int me, float 
 }
 
 struct AttnTcArgs {
+	// per prompt (blockIdx.y), one behind the other:
 	const __nv_bfloat16 *qp;  // [3][q_tiles][8][8 KiB]
 	const __nv_bfloat16 *kp;  // [3][k_tiles][8][8 KiB]
 	const __nv_bfloat16 *vp;  // [3][v_blocks][8 KiB]
@@ -211,8 +214,8 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		pdl_wait();  // the packed operands are the predecessors' output
 		const size_t q_term = size_t(a.q_tiles) * 8 * TC_TILE_BYTES, k_term = size_t(a.k_tiles) * 8 * TC_TILE_BYTES,
 		             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
-		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp), *kp = reinterpret_cast<const uint8_t *>(a.kp),
-		              *vp = reinterpret_cast<const uint8_t *>(a.vp);
+		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 3 * q_term, *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 3 * k_term,
+		              *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 3 * v_term;
 		int cap = TC_SPIN_CAP, st = 0;
 		uint32_t ph = 1;  // (a fresh barrier passes parity 1)
 		for (int g = 0; g < total; g++) {
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			const bool got = at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, &l_other, a.err, fail);
 			const float lt = l + l_other;
 			const float inv = (row_ok && got) ? 1.0f / lt : 0.0f;  // (a visible key always exists: the query itself)
-			float *orow = a.o + (size_t(tile) * 128 + r) * 256;
+			float *orow = a.o + (size_t(blockIdx.y) * a.S * 4 + size_t(tile) * 128 + r) * 256;
 #pragma unroll 1
 			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
 				uint32_t ov[32];

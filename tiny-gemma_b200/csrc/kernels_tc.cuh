@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(256) split_pack_kernel(const float *A, __nv_bf
 	pdl_trigger();
 	pdl_wait();
 	const int k_blocks = K / TC_BK;
+	A += size_t(blockIdx.y) * M * K;  // blockIdx.y: one of several matrices behind each other
+	out += size_t(blockIdx.y) * 3 * m_tiles * k_blocks * (TC_TILE_BYTES / 2);
 	const size_t n_chunks = size_t(m_tiles) * TC_BM * (K / 8);  // one thread per (row, 8 consecutive k)
 	const size_t term_stride = size_t(m_tiles) * k_blocks * (TC_TILE_BYTES / 2);
 	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_chunks; c += size_t(gridDim.x) * blockDim.x) {

@@ -1960,7 +1960,7 @@ int ensure_prefill_scratch(tg_state *s, size_t R, int S, int n_ids) {
 	part = std::max(part, std::min(size_t(24) * R * std::max(I, qd), size_t(1) << 28));  // tensor-core GEMM partial sums (<= 1 GiB)
 	need += part;
 	need += (i8_pack_bytes(int(R), std::max(I, std::max(D, qd))) + 3) / 4 + 512;
-	need += (attn_tc_plan(S).total() + 3) / 4 + 512;  // packed q, k, v of the tensor-core attention (long prompts)
+	need += (attn_tc_plan(S).total() * (R / S) + 3) / 4 + 512;  // packed q, k, v of the tensor-core attention (long prompts)
 	if (need > s->pf_floats) {
 		if (s->pf) cudaFree(s->pf);
 		s->pf = nullptr;
@@ -2018,18 +2018,19 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		tc.err = s->err_flag;
 		p += (tc.x_bytes + 3) / 4;
 	}
-	// long prompts: attention on the tensor cores, from packed copies of q, k and v, one sequence after the other
-	// (from 640 tokens on: below, the three packing launches cost what the tensor cores save)
-	const bool attn_tc = use_tc && pos0 < 0 && S_seq > env_int("TG_ATTN_SMALL_MAX", 384) && env_int("TG_ATTN_TC", 1) &&
-	                     S_seq >= env_int("TG_ATTN_TC_MIN", 640);
+	// Attention on the tensor cores, from packed copies of q, k and v: for more than 960 tokens, of one prompt or of a group
+	// of equal prompts. Below, the CUDA-core kernel with two queries per CTA is faster, since its CTAs are more (prefill of
+	// 450 tokens 2.9 against 3.6 ms, 832 tokens 4.93 against 5.04, 16 prompts of 61 tokens 3.98 against 4.29; 8 of 178 tokens
+	// 5.71 against 5.67, 256 of 178 tokens 170 against 150).
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
+	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && nb * S_seq > env_int("TG_ATTN_SMALL_MAX", 960) && S_seq >= env_int("TG_ATTN_TC_MIN", 0);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
 		at_q = reinterpret_cast<__nv_bfloat16 *>(p);
-		at_k = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + atp.q_bytes);
-		at_v = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + atp.q_bytes + atp.k_bytes);
-		p += (atp.total() + 3) / 4;
+		at_k = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + atp.q_bytes * nb);
+		at_v = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + (atp.q_bytes + atp.k_bytes) * nb);
+		p += (atp.total() * nb + 3) / 4;
 	}
 	float *part = p;
 	size_t part_floats = s->pf_floats - size_t(part - s->pf);
@@ -2120,7 +2121,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		ra.cache_stride = size_t(slots) * AT_HD;
 		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
 		count_launch();
-		const bool attn_small = pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 384);  // short prompts: two queries per CTA
+		const bool attn_small = !attn_tc && (pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 960));  // short prompts: two queries per CTA
 		if (attn_small) {
 			static bool as_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
@@ -2130,8 +2131,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			}
 			launch_k(attn_prefill_small_kernel, dim3((S_seq + 1) / 2, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
 			         use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, s->err_flag);
-		}
-		else if (attn_tc) {
+		} else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
 			if (!at_configured[dev]) {
@@ -2140,22 +2140,20 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			}
 			auto pack_rows = [&](const float *src, __nv_bfloat16 *dst, int rows, int tiles) {
 				const size_t chunks = size_t(tiles) * TC_BM * (256 / 8);
-				launch_k(split_pack_kernel, dim3(unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16))), dim3(256), 0, st, src, dst, rows,
+				launch_k(split_pack_kernel, dim3(unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0, st, src, dst, rows,
 				         256, tiles);
 				count_launch();
 			};
-			for (int i = 0; i < nb; i++) {  // (the packed copies are reused from sequence to sequence: stream order)
-			const float *qi = q + size_t(i) * S_seq * qd, *ki = k + size_t(i) * S_seq * kd, *vi = v + size_t(i) * S_seq * kd;
-			pack_rows(qi, at_q, 4 * S_seq, atp.q_tiles);  // rows = (query, head) pairs as they lie in q [S][4][256]
-			pack_rows(ki, at_k, S_seq, atp.k_tiles);
-			launch_k(attn_pack_v_kernel, dim3(unsigned(std::min<size_t>((size_t(atp.v_blocks) * 512 + 255) / 256, size_t(g_num_sms) * 16))), dim3(256), 0,
-			         st, vi, at_v, S_seq, atp.v_blocks);
+			pack_rows(q, at_q, 4 * S_seq, atp.q_tiles);  // rows = (query, head) pairs as they lie in q [S][4][256]
+			pack_rows(k, at_k, S_seq, atp.k_tiles);
+			launch_k(attn_pack_v_kernel, dim3(unsigned(std::min<size_t>((size_t(atp.v_blocks) * 512 + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0,
+			         st, (const float *)v, at_v, S_seq, atp.v_blocks);
 			count_launch();
 			AttnTcArgs aa{};
 			aa.qp = at_q;
 			aa.kp = at_k;
 			aa.vp = at_v;
-			aa.o = ao + size_t(i) * S_seq * qd;
+			aa.o = ao;
 			aa.S = S_seq;
 			aa.q_tiles = atp.q_tiles;
 			aa.k_tiles = atp.k_tiles;
@@ -2163,9 +2161,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			aa.is_local = w.is_local ? 1 : 0;
 			aa.window = c.n_pos_local;
 			aa.err = s->err_flag;
-			launch_k(attn_prefill_tc_kernel, dim3(atp.q_tiles), dim3(AT_TC_THREADS), size_t(AT_TC_SMEM), st, aa);
-			if (i + 1 < nb) count_launch();
-			}
+			launch_k(attn_prefill_tc_kernel, dim3(atp.q_tiles, nb), dim3(AT_TC_THREADS), size_t(AT_TC_SMEM), st, aa);
 		} else
 			if (env_int("TG_ATTN_BLOCK4", 1)) {  // long prompts: four keys per step (TG_ATTN_BLOCK4=0: the per-key kernel)
 				static bool configured[TG_MAX_DEVICES] = {false};
