@@ -2,9 +2,9 @@
 // arithmetic: one decode step per sequence, and short prompts.
 //
 // The rows of a sequence's keys (values) follow each other in memory, so a chunk of 32 keys is ONE bulk copy of 32 KB
-// into shared memory: the whole traffic of a CTA is asynchronous and costs no registers, and three CTAs fit an SM. The
-// copy of the next K chunk starts when the scores of this one are done, that of the next V chunk when its products are.
-// Per chunk: scores (a warp takes a few keys against all query rows; a lane holds 8 of the 256 dimensions, and the
+// into shared memory: the whole traffic of a CTA is asynchronous and costs no registers. A buffer is filled again as soon
+// as its scores (K) or products (V) are done.
+// The prefill kernel's step over a chunk: scores (a warp takes a few keys against all query rows; a lane holds 8 of the 256 dimensions, and the
 // lanes' partial sums meet in a reduce-scatter, one shuffle per score), one softmax step per query row with lane = key,
 // then the products with V (a thread holds 4 dimensions of every row for a share of the keys).
 //
@@ -91,29 +91,86 @@ struct AttnArgs {
 };
 constexpr int AT_THREADS = 256;
 constexpr int AT_PART = AT_NH * AT_HD + 8;
+// A step reads every cached row once: HBM bounds it for many sequences, the chain of dependent round trips for few.
+// A warp takes 4 keys of every 32 against all four heads and runs on its own through a ring of three 4 KB buffers (K, V,
+// K, V, ..), with its own running maximum: nothing in the loop waits for another warp. The ring keeps 64 to 96 KB per CTA
+// in flight, two CTAs per SM (HBM's rate times its latency under load is ~70 KB per SM). 256 sequences of 182 keys, 94 MB:
+// 33.5 us with one K and one V buffer and block-wide steps over 32 keys and two splits, 23 us now.
+constexpr int AD_KEYS = 4, AD_ROUND = AD_KEYS * AT_THREADS / 32;
+constexpr int AD_BUF = AD_KEYS * 1024;
+constexpr int AD_STAGES = 3;
+constexpr int AD_SMEM = AT_THREADS / 32 * AD_STAGES * AD_BUF;
 
-__global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
-	__shared__ __align__(16) float rowbuf[AT_NH * AT_HD + 2 * AT_HD];  // q | k | v of the new token, normed and rotated in place
-	__shared__ __align__(16) float sc[AC_KEYS][AT_NH], pr[AC_KEYS][AT_NH];
-	__shared__ float corr_s[AT_NH], m_s[AT_NH], l_s[AT_NH];
-	__shared__ uint64_t kbar, vbar;
+	__shared__ __align__(16) float rowbuf[AT_NH * AT_HD + 2 * AT_HD];  // q | k | v of the new token, normed and rotated
+	__shared__ float m_s[AT_THREADS / 32][AT_NH], l_s[AT_THREADS / 32][AT_NH];
+	__shared__ uint64_t full[AT_THREADS / 32][AD_STAGES];
 	__shared__ uint32_t red[AT_THREADS / 32];
 	__shared__ int s_last;
-	float *K = reinterpret_cast<float *>(ac_smem), *V = reinterpret_cast<float *>(ac_smem + AC_BUF);
 	const int b = blockIdx.y, split = blockIdx.x;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	if (tid == 0) {
-		mbar_init(&kbar, 1);
-		mbar_init(&vbar, 1);
+	uint8_t *ring = ac_smem + warp * (AD_STAGES * AD_BUF);
+	if (lane == 0) {
+		for (int i = 0; i < AD_STAGES; i++) mbar_init(&full[warp][i], 1);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	__syncwarp();
+	// the weights are nobody's output: requested before the wait for the predecessor. Warps 0..3: a head of q, 4: k, 5: v
+	constexpr int NQ = AT_NH * AT_HD + 2 * AT_HD;
+	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 w0 = z4, w1 = z4, s0 = z4, s1 = z4;
+	if (warp <= AT_NH) {
+		const float4 *w = reinterpret_cast<const float4 *>(warp < AT_NH ? a.rmsq : a.rmsk);
+		w0 = __ldg(w + lane);
+		w1 = __ldg(w + 32 + lane);
+	}
+	if (warp < AT_NH + 2 && a.qkv_nsplit > 0) {
+		const float4 *scl = reinterpret_cast<const float4 *>(warp < AT_NH ? a.sq + warp * AT_HD : (warp == AT_NH ? a.sk : a.sv));
+		s0 = __ldg(scl + lane);
+		s1 = __ldg(scl + 32 + lane);
 	}
 	pdl_trigger();
 	pdl_wait();
 	int pos = a.step_pos[b];
+	const int base = a.is_local ? a.ring_base[b] : 0;
+	float4 lo = z4, hi = z4;
+	if (warp < AT_NH + 2) {  // (in flight together with the position)
+		const float4 *p = reinterpret_cast<const float4 *>(a.qkv + size_t(b) * NQ + warp * AT_HD);
+		if (a.qkv_nsplit > 0) {
+			const size_t sstride = size_t(a.qkv_B) * (NQ / 4);
+			for (int sp = 0; sp < a.qkv_nsplit; sp += 4) {
+				float4 u[4], v[4];
+#pragma unroll
+				for (int q = 0; q < 4; q++) {
+					u[q] = v[q] = z4;
+					if (sp + q < a.qkv_nsplit) {
+						u[q] = p[size_t(sp + q) * sstride + lane];
+						v[q] = p[size_t(sp + q) * sstride + 32 + lane];
+					}
+				}
+#pragma unroll
+				for (int q = 0; q < 4; q++) {
+					lo.x += u[q].x;
+					lo.y += u[q].y;
+					lo.z += u[q].z;
+					lo.w += u[q].w;
+					hi.x += v[q].x;
+					hi.y += v[q].y;
+					hi.z += v[q].z;
+					hi.w += v[q].w;
+				}
+			}
+			lo = make_float4(lo.x * s0.x, lo.y * s0.y, lo.z * s0.z, lo.w * s0.w);
+			hi = make_float4(hi.x * s1.x, hi.y * s1.y, hi.z * s1.z, hi.w * s1.w);
+		} else {
+			lo = p[lane];
+			hi = p[32 + lane];
+		}
+	}
 	int slot, valid;
 	if (a.is_local) {
-		slot = (pos - a.ring_base[b]) % a.slots;
+		slot = (pos - base) % a.slots;
 		valid = min(pos + 1, a.slots);
 	} else {
 		if (pos >= a.slots) {  // cache full: refuse to write out of bounds
@@ -123,70 +180,32 @@ __global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) 
 		slot = pos;
 		valid = pos + 1;
 	}
-	// whole chunks of keys are dealt out to the splits; splits without any leave at once
-	const int chunks = (valid + AC_KEYS - 1) / AC_KEYS, per = (chunks + a.nsplit - 1) / a.nsplit, nact = (chunks + per - 1) / per;
+	// whole rounds of 32 keys are dealt out to the splits; splits without any leave at once
+	const int rounds = (valid + AD_ROUND - 1) / AD_ROUND, per = (rounds + a.nsplit - 1) / a.nsplit, nact = (rounds + per - 1) / per;
 	if (split >= nact) return;
-	const int j0 = split * per * AC_KEYS, j1 = min(valid, j0 + per * AC_KEYS);
-	const int nch = (j1 - j0 + AC_KEYS - 1) / AC_KEYS;
+	const int j0 = split * per * AD_ROUND, j1 = min(valid, j0 + per * AD_ROUND);
+	const int jw = j0 + AD_KEYS * warp, nit = max(0, (j1 - jw + AD_ROUND - 1) / AD_ROUND);  // this warp's first key, its groups of keys
 	float *kc = a.kcache + size_t(b) * a.slots * AT_HD, *vc = a.vcache + size_t(b) * a.slots * AT_HD;
-	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
-		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
-		fence_proxy_async();
-		mbar_expect_tx(bar, bytes);
-		bulk_load(dst, src + size_t(j0 + c * AC_KEYS) * AT_HD, bytes, bar);
-	};
-	__syncthreads();
-	if (tid == 0) {
-		issue(K, kc, 0, &kbar);
-		issue(V, vc, 0, &vbar);
-	}
-	// ---- the new token's q, k, v
-	constexpr int NQ = AT_NH * AT_HD + 2 * AT_HD;
-	for (int n = 4 * tid; n < NQ; n += 4 * AT_THREADS) {
-		float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-		if (a.qkv_nsplit > 0) {
-			const float *p = a.qkv + size_t(b) * NQ + n;
-			const size_t sstride = size_t(a.qkv_B) * NQ;
-			for (int s0 = 0; s0 < a.qkv_nsplit; s0 += 4) {
-				float4 v[4];
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-					if (s0 + q < a.qkv_nsplit) v[q] = *reinterpret_cast<const float4 *>(p + size_t(s0 + q) * sstride);
-				}
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					acc.x += v[q].x;
-					acc.y += v[q].y;
-					acc.z += v[q].z;
-					acc.w += v[q].w;
-				}
-			}
-			const float *scl = n < AT_NH * AT_HD ? a.sq + n : (n < AT_NH * AT_HD + AT_HD ? a.sk + (n - AT_NH * AT_HD) : a.sv + (n - AT_NH * AT_HD - AT_HD));
-			const float4 s4 = *reinterpret_cast<const float4 *>(scl);
-			acc.x *= s4.x;
-			acc.y *= s4.y;
-			acc.z *= s4.z;
-			acc.w *= s4.w;
-		} else {
-			acc = *reinterpret_cast<const float4 *>(a.qkv + size_t(b) * NQ + n);
+	// item i of the warp's ring: the keys (i even) or the values (i odd) of group i / 2; called by the whole warp
+	auto issue = [&](int i) {
+		const int j = jw + (i >> 1) * AD_ROUND, st = i % AD_STAGES;
+		const uint32_t bytes = uint32_t(min(AD_KEYS, j1 - j)) * 1024u;
+		if (i < 2 * nit && tc_elect()) {
+			mbar_expect_tx(&full[warp][st], bytes);
+			bulk_load(ring + st * AD_BUF, (i & 1 ? vc : kc) + size_t(j) * AT_HD, bytes, &full[warp][st]);
 		}
-		*reinterpret_cast<float4 *>(&rowbuf[n]) = acc;
-	}
-	__syncthreads();
-	if (warp <= AT_NH) {  // heads 0..3 of q, then k: per-head norm and RoPE; lane owns d = 4 lane .. and the partners 128 + d
-		const float *w = warp < AT_NH ? a.rmsq : a.rmsk;
+	};
+#pragma unroll
+	for (int i = 0; i < AD_STAGES; i++) issue(i);
+	if (warp <= AT_NH) {  // per-head norm and RoPE; lane owns d = 4 lane .. and the partners 128 + d
 		// the reference scales q by 1/sqrt(256) = 2^-4 before the dot products (ops.hpp:262,283)
 		const float qs = warp < AT_NH ? 0.0625f : 1.0f;
 		const float4 *cr = reinterpret_cast<const float4 *>(a.cosT + size_t(pos) * AT_HD), *sr = reinterpret_cast<const float4 *>(a.sinT + size_t(pos) * AT_HD);
-		const float4 c0 = cr[lane], c1 = cr[32 + lane], s0 = sr[lane], s1 = sr[32 + lane];
-		const float4 w0 = reinterpret_cast<const float4 *>(w)[lane], w1 = reinterpret_cast<const float4 *>(w)[32 + lane];
-		float4 *x = reinterpret_cast<float4 *>(&rowbuf[warp * AT_HD]);
-		const float4 lo = x[lane], hi = x[32 + lane];
+		const float4 c0 = cr[lane], c1 = cr[32 + lane], n0 = sr[lane], n1 = sr[32 + lane];
 		const float lov[4] = {lo.x, lo.y, lo.z, lo.w}, hiv[4] = {hi.x, hi.y, hi.z, hi.w};
 		const float wlo[4] = {w0.x, w0.y, w0.z, w0.w}, whi[4] = {w1.x, w1.y, w1.z, w1.w};
 		const float clo[4] = {c0.x, c0.y, c0.z, c0.w}, chi[4] = {c1.x, c1.y, c1.z, c1.w};
-		const float slo[4] = {s0.x, s0.y, s0.z, s0.w}, shi[4] = {s1.x, s1.y, s1.z, s1.w};
+		const float slo[4] = {n0.x, n0.y, n0.z, n0.w}, shi[4] = {n1.x, n1.y, n1.z, n1.w};
 		float ss = 0.0f;
 #pragma unroll
 		for (int i = 0; i < 4; i++) {
@@ -203,112 +222,123 @@ __global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(AttnArgs a) 
 			yl[i] = fmaf(-1.0f * v, slo[i], clo[i] * u) * qs;
 			yh[i] = fmaf(u, shi[i], chi[i] * v) * qs;
 		}
-		x[lane] = make_float4(yl[0], yl[1], yl[2], yl[3]);
-		x[32 + lane] = make_float4(yh[0], yh[1], yh[2], yh[3]);
+		lo = make_float4(yl[0], yl[1], yl[2], yl[3]);
+		hi = make_float4(yh[0], yh[1], yh[2], yh[3]);
+	}
+	if (warp < AT_NH + 2) {
+		float4 *x = reinterpret_cast<float4 *>(&rowbuf[warp * AT_HD]);
+		x[lane] = lo;
+		x[32 + lane] = hi;
+		if (warp >= AT_NH && slot >= j0 && slot < j1) {
+			float4 *c = reinterpret_cast<float4 *>((warp == AT_NH ? kc : vc) + size_t(slot) * AT_HD);
+			c[lane] = lo;
+			c[32 + lane] = hi;
+		}
 	}
 	__syncthreads();
-	const float4 *knew = reinterpret_cast<const float4 *>(&rowbuf[AT_NH * AT_HD]), *vnew = knew + 64;
-	if (slot >= j0 && slot < j1) {
-		if (tid < 64)
-			reinterpret_cast<float4 *>(kc + size_t(slot) * AT_HD)[tid] = knew[tid];
-		else if (tid < 128)
-			reinterpret_cast<float4 *>(vc + size_t(slot) * AT_HD)[tid - 64] = vnew[tid - 64];
-	}
 	float4 q0[AT_NH], q1[AT_NH];
 #pragma unroll
 	for (int h = 0; h < AT_NH; h++) {
 		q0[h] = *reinterpret_cast<const float4 *>(&rowbuf[h * AT_HD + 4 * lane]);
 		q1[h] = *reinterpret_cast<const float4 *>(&rowbuf[h * AT_HD + 128 + 4 * lane]);
 	}
-	const int d4 = tid & 63, kg = tid >> 6;
-	float4 o[AT_NH];
+	float4 o0[AT_NH], o1[AT_NH];  // lane: dimensions 4 lane .. and 128 + 4 lane ..
 #pragma unroll
-	for (int h = 0; h < AT_NH; h++) o[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-	float m = -INFINITY, l = 0.0f;  // of head `warp` (warps 0..3)
-	for (int c = 0; c < nch; c++) {
-		const int n = min(AC_KEYS, j1 - j0 - c * AC_KEYS), at = slot - (j0 + c * AC_KEYS);  // keys of the chunk; the new token's row in it
-		const bool here = at >= 0 && at < n;
-		tc_wait(&kbar, c & 1, a.err_flag);
-		if (here) {  // the cache does not hold the new token's row yet
-			if (tid < 64) reinterpret_cast<float4 *>(K)[at * 64 + tid] = knew[tid];
-			__syncthreads();
+	for (int h = 0; h < AT_NH; h++) o0[h] = o1[h] = z4;
+	float m = -INFINITY, l = 0.0f;  // of head (lane >> 1) & 3
+	// the cache does not hold the new token's row yet (n: 4 for the key row of rowbuf, 5 for the value row)
+	auto patch = [&](uint8_t *buf, int at, int n) {
+		if (at < 0 || at >= AD_KEYS) return;
+		float4 *d = reinterpret_cast<float4 *>(buf + at * 1024);
+		const float4 *x = reinterpret_cast<const float4 *>(&rowbuf[n * AT_HD]);
+		d[lane] = x[lane];
+		d[32 + lane] = x[32 + lane];
+		fence_proxy_async();  // (the buffer's next content arrives by a bulk copy)
+		__syncwarp();
+	};
+	int cap = TC_SPIN_CAP;
+	for (int it = 0; it < nit; it++) {
+		const int j = jw + it * AD_ROUND, n = min(AD_KEYS, j1 - j);
+		const int ik = 2 * it, iv = 2 * it + 1;
+		uint8_t *K = ring + ik % AD_STAGES * AD_BUF, *V = ring + iv % AD_STAGES * AD_BUF;
+		tc_wait_cap(&full[warp][ik % AD_STAGES], ik / AD_STAGES & 1, cap);
+		patch(K, slot - j, AT_NH);
+		float t[16];
+#pragma unroll
+		for (int kk = 0; kk < AD_KEYS; kk++) {  // (rows past n hold an older group's keys, or nothing yet: their scores are not used)
+			const float4 k0 = *reinterpret_cast<const float4 *>(K + kk * 1024 + 16 * lane), k1 = *reinterpret_cast<const float4 *>(K + kk * 1024 + 512 + 16 * lane);
+#pragma unroll
+			for (int h = 0; h < AT_NH; h++) t[kk * 4 + h] = ac_dot8(q0[h], q1[h], k0, k1);
 		}
-		{
-			float t[16];
+		float z = ac_reduce16(t, lane);  // key lane >> 3, head (lane >> 1) & 3
+		__syncwarp();
+		issue(ik + AD_STAGES);
+		if ((lane >> 3) >= n) z = -INFINITY;
+		float mn = fmaxf(m, z);
+		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 8));
+		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 16));  // finite: a group has at least one key
+		const float p = expf(z - mn), cr = expf(m - mn);
+		float ps = p + __shfl_xor_sync(0xffffffffu, p, 8);
+		ps += __shfl_xor_sync(0xffffffffu, ps, 16);
+		l = fmaf(l, cr, ps);
+		m = mn;
+		if (__any_sync(0xffffffffu, cr != 1.0f)) {
 #pragma unroll
-			for (int kk = 0; kk < 4; kk++) {
-				const float4 k0 = *reinterpret_cast<const float4 *>(K + (4 * warp + kk) * AT_HD + 4 * lane);
-				const float4 k1 = *reinterpret_cast<const float4 *>(K + (4 * warp + kk) * AT_HD + 128 + 4 * lane);
-#pragma unroll
-				for (int h = 0; h < AT_NH; h++) t[kk * 4 + h] = ac_dot8(q0[h], q1[h], k0, k1);
-			}
-			const float z = ac_reduce16(t, lane);
-			if (!(lane & 1)) sc[4 * warp + (lane >> 3)][(lane >> 1) & 3] = z;
-		}
-		__syncthreads();  // scores complete, K consumed
-		if (tid == 0 && c + 1 < nch) issue(K, kc, c + 1, &kbar);
-		if (warp < AT_NH) {
-			const float z = lane < n ? sc[lane][warp] : -INFINITY;
-			const float mn = fmaxf(m, warp_max(z));  // finite: a chunk has at least one key
-			const float p = expf(z - mn), cr = expf(m - mn);
-			l = fmaf(l, cr, warp_sum(p));
-			m = mn;
-			pr[lane][warp] = p;
-			if (lane == 0) corr_s[warp] = cr;
-		}
-		tc_wait(&vbar, c & 1, a.err_flag);
-		if (here && tid >= 128 && tid < 192) reinterpret_cast<float4 *>(V)[at * 64 + tid - 128] = vnew[tid - 128];
-		__syncthreads();  // probabilities complete
-#pragma unroll
-		for (int h = 0; h < AT_NH; h++) {
-			const float cr = corr_s[h];
-			o[h].x *= cr;
-			o[h].y *= cr;
-			o[h].z *= cr;
-			o[h].w *= cr;
-		}
-#pragma unroll
-		for (int kk = 0; kk < AC_KEYS / 4; kk++) {
-			const int key = kg * (AC_KEYS / 4) + kk;
-			if (key < n) {
-				const float4 v = *reinterpret_cast<const float4 *>(V + key * AT_HD + 4 * d4);
-				const float4 p = *reinterpret_cast<const float4 *>(&pr[key][0]);
-				ac_fma4(o[0], p.x, v);
-				ac_fma4(o[1], p.y, v);
-				ac_fma4(o[2], p.z, v);
-				ac_fma4(o[3], p.w, v);
+			for (int h = 0; h < AT_NH; h++) {
+				const float c = __shfl_sync(0xffffffffu, cr, 2 * h);
+				o0[h] = make_float4(o0[h].x * c, o0[h].y * c, o0[h].z * c, o0[h].w * c);
+				o1[h] = make_float4(o1[h].x * c, o1[h].y * c, o1[h].z * c, o1[h].w * c);
 			}
 		}
-		__syncthreads();  // V consumed
-		if (tid == 0 && c + 1 < nch) issue(V, vc, c + 1, &vbar);
+		tc_wait_cap(&full[warp][iv % AD_STAGES], iv / AD_STAGES & 1, cap);
+		patch(V, slot - j, AT_NH + 1);
+#pragma unroll
+		for (int kk = 0; kk < AD_KEYS; kk++) {
+			if (kk < n) {
+				const float4 v0 = *reinterpret_cast<const float4 *>(V + kk * 1024 + 16 * lane), v1 = *reinterpret_cast<const float4 *>(V + kk * 1024 + 512 + 16 * lane);
+#pragma unroll
+				for (int h = 0; h < AT_NH; h++) {
+					const float w = __shfl_sync(0xffffffffu, p, 8 * kk + 2 * h);
+					ac_fma4(o0[h], w, v0);
+					ac_fma4(o1[h], w, v1);
+				}
+			}
+		}
+		__syncwarp();
+		issue(iv + AD_STAGES);
 	}
-	// ---- join the four key groups: thread (h, d4) ends up with four consecutive outputs
-	float4 *jb = reinterpret_cast<float4 *>(K);
+	if (cap == 0) *static_cast<volatile int *>(a.err_flag) = 6;
+	// ---- join the warps: thread (h, d4) ends up with four consecutive outputs
+	__syncthreads();  // (every warp has consumed its ring)
+	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
 #pragma unroll
-	for (int h = 0; h < AT_NH; h++) jb[(kg * AT_NH + h) * 64 + d4] = o[h];
-	if (warp < AT_NH && lane == 0) {
-		m_s[warp] = m;
-		l_s[warp] = l;
+	for (int h = 0; h < AT_NH; h++) {
+		jb[(warp * AT_NH + h) * 64 + lane] = o0[h];
+		jb[(warp * AT_NH + h) * 64 + 32 + lane] = o1[h];
+	}
+	if (lane < 2 * AT_NH && !(lane & 1)) {
+		m_s[warp][lane >> 1] = m;
+		l_s[warp][lane >> 1] = l;
 	}
 	__syncthreads();
-	const int h = kg;
-	float4 r = jb[h * 64 + d4];
+	const int h = tid >> 6, d4 = tid & 63;
+	float Ms = -INFINITY, L = 0.0f;
 #pragma unroll
-	for (int g = 1; g < 4; g++) {
-		const float4 t = jb[(g * AT_NH + h) * 64 + d4];
-		r.x += t.x;
-		r.y += t.y;
-		r.z += t.z;
-		r.w += t.w;
+	for (int g = 0; g < AT_THREADS / 32; g++) Ms = fmaxf(Ms, m_s[g][h]);  // finite: warp 0 has a key
+	float4 r = z4;
+#pragma unroll
+	for (int g = 0; g < AT_THREADS / 32; g++) {
+		const float w = expf(m_s[g][h] - Ms);
+		L = fmaf(l_s[g][h], w, L);
+		ac_fma4(r, w, jb[(g * AT_NH + h) * 64 + d4]);
 	}
-	float L = l_s[h];
 	if (nact > 1) {
 		float *pb = a.part + size_t(b) * a.nsplit * AT_PART;
 		float *prow = pb + size_t(split) * AT_PART;
 		__stcg(reinterpret_cast<float4 *>(prow) + tid, r);
-		if (tid < AT_NH) {
-			__stcg(prow + AT_NH * AT_HD + tid, m_s[tid]);
-			__stcg(prow + AT_NH * AT_HD + 4 + tid, l_s[tid]);
+		if (d4 == 0) {
+			__stcg(prow + AT_NH * AT_HD + h, Ms);
+			__stcg(prow + AT_NH * AT_HD + 4 + h, L);
 		}
 		__threadfence();
 		__syncthreads();
