@@ -89,7 +89,8 @@ struct GeluLut {
 	float inv;  // 1 / eps where eps is a power of two (x * inv is then exactly x / eps, at a tenth of the instructions), else 0
 	// false: the result is 0; else the table entry, from `size` on the value itself
 	__device__ __forceinline__ bool index(float x, int &idx) const {
-		const float q = inv != 0.0f ? (x - mn) * inv : (x - mn) / eps;
+		// (scaling by a power of two commutes with rounding: one FMA is the difference, rounded, divided)
+		const float q = inv != 0.0f ? fmaf(x, inv, -(mn * inv)) : (x - mn) / eps;
 		// x86 cvttss2si yields INT_MIN for NaN and out-of-range inputs, which the
 		// reference then treats as a negative index
 		if (!(q < 2147483648.0f) || q < -2147483648.0f) return false;

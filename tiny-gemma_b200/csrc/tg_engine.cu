@@ -1663,6 +1663,23 @@ int launch_resnorm(float *h, const float *t, const float *w_post, const float *w
 int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, const float *su, const float *sg, const TcScratch &sc, cudaStream_t st) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, I);
+	// several unsplit rows per SM: the CTA's next rows are copied while it works on one (one CTA per SM for the 55 KB rows of
+	// 6912, two for the 16 KB of 2048)
+	if (nsplit == 1 && M >= 4 * g_num_sms && I <= 7168) {
+		static bool configured[TG_MAX_DEVICES] = {false};
+		const int dev = current_device_slot();
+		if (!configured[dev]) {
+			TG_CUDA(cudaFuncSetAttribute(geglu_i8_stream_kernel<896, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 8 * 7168));
+			TG_CUDA(cudaFuncSetAttribute(geglu_i8_stream_kernel<512, 1, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * 8 * 2048));
+			configured[dev] = true;
+		}
+		if (I <= 2048)
+			launch_k(geglu_i8_stream_kernel<512, 1, 5>, dim3(2 * g_num_sms), dim3(512), size_t(5) * 8 * I, st, ug, sc.x, rs, M, I, groups, lut, su, sg, sc.err);
+		else
+			launch_k(geglu_i8_stream_kernel<896, 2, 3>, dim3(g_num_sms), dim3(896), size_t(3) * 8 * I, st, ug, sc.x, rs, M, I, groups, lut, su, sg, sc.err);
+		count_launch();
+		return check_launch("geglu");
+	}
 	// (two rows of 512 or 576 threads fit an SM; beyond that the CTAs loop, so that the table is loaded once per CTA)
 	const unsigned grid = unsigned(std::min(M, 2 * g_num_sms));
 	if (I <= 2048)
