@@ -19,7 +19,7 @@ def rows(kind, n, rng):
     return x
 
 
-@pytest.mark.parametrize("n", [8192, 24576, 262144])
+@pytest.mark.parametrize("n", [8192, 24576, 262144, 655360])
 @pytest.mark.parametrize("kind", ["flat", "noise", "steep", "empty"])
 def test_minp_token_is_the_sequential_crossing(capi, n, kind):
     rng = np.random.default_rng(n)

@@ -105,8 +105,7 @@ struct MgArgs {
 	unsigned seq0;   // layer tags of this launch start above seq0
 	float *logits;                    // [V]
 	float *probs;                     // [V] exp(z - max) of the min-p sampler (before normalisation)
-	int samp_ch;                      // probabilities staged per round of the inverse CDF (multiple of 4, fits the weight ring)
-	float *samp_f;                    // [3][grid] sampler partials
+	float *samp_f;                    // sampler partials (minp_grid_part_bytes)
 	int *samp_i;                      // [grid]
 	float *xnorm_out;                 // [D] final-normed hidden state (parity read-back)
 	unsigned *bar;                    // grid barrier counter, zero at launch
@@ -779,7 +778,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) mega_decode_kernel(const __grid
 	extern __shared__ uint8_t smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(smem_raw) + 1023) & ~uintptr_t(1023));
 	__shared__ uint64_t bar_A, bar_C, bar_D, bar_E, bar_lm[MG_LM_STAGES], emp_lm[MG_LM_STAGES];
-	__shared__ float bred[MG_NWARPS];
+	__shared__ float bred[2 * MG_NWARPS];
 	__shared__ int s_abort;
 	__shared__ float s_f[8];
 	__shared__ int s_i[4];
@@ -1393,72 +1392,15 @@ __global__ void __launch_bounds__(MG_THREADS, 1) mega_decode_kernel(const __grid
 			} else {
 				// ops::minp_logits (reference ops.hpp:762-859). z = logit / temp; rowmax = gmax;
 				// p = exp(z - rowmax); maxp = exp(0) = 1 so cut = minp * 1; denom = sum of p >= cut.
-				const float cut = a.minp * expf(gmax - gmax);
-				float ds = 0.0f;
-				{
-					const int my_tiles = (a.LM.ntiles - cta + G - 1) / G;
-#pragma unroll 1
-					for (int j = tid; j < my_tiles * MG_LM_TN; j += MG_THREADS) {
-						const int v = (cta + (j / MG_LM_TN) * G) * MG_LM_TN + (j % MG_LM_TN);
-						const float pv = expf(__ldcg(a.logits + v) / a.temp - gmax);
-						__stcg(a.probs + v, pv);
-						ds += (pv < cut) ? 0.0f : pv;
-					}
-				}
-				ds = mg_block_sum<MG_NWARPS>(ds, bred);
-				if (tid == 0) __stcg(a.samp_f + G + cta, ds);
-				mg_grid_sync(ctx);
-				if (cta == 0) {
-					// denominator: per-CTA sums added in a fixed tree by warp 0
-					if (warp == 0) {
-						float dv = 0.0f;
-#pragma unroll 1
-						for (int c = lane; c < G; c += 32) dv += __ldcg(a.samp_f + G + c);
-						dv = warp_sum(dv);
-						if (lane == 0) s_f[6] = 1.0f / dv;
-					}
-					float randf = 0.0f;
-					const int rc = __ldcg(a.randf_count);
-					if (rc < a.randf_cap) randf = __ldg(a.randf + rc);
-					__syncthreads();
-					const float inv = s_f[6];
-					// inverse CDF: the first index whose sequential fp32 running sum reaches randf,
-					// evaluated exactly and in parallel (cdf_cross_block) over chunks of probabilities
-					// p = exp(z - max) * inv staged in the idle weight ring
-					float *cbuf = reinterpret_cast<float *>(R_D);
-					const int CH = a.samp_ch;
-					if (tid == 0) {
-						s_i[1] = -1;
-						s_f[5] = 0.0f;
-					}
-					__syncthreads();
-#pragma unroll 1
-					for (int c0 = 0; c0 < a.V; c0 += CH) {
-						const int n = min(CH, a.V - c0);
-#pragma unroll 4
-						for (int i = tid * 4; i < n; i += MG_THREADS * 4) {
-							float4 v = __ldcg(reinterpret_cast<const float4 *>(a.probs + c0 + i));
-							v.x *= inv;
-							v.y *= inv;
-							v.z *= inv;
-							v.w *= inv;
-							*reinterpret_cast<float4 *>(cbuf + i) = v;
-						}
-						__syncthreads();
-						const int r = cdf_cross_block<MG_NWARPS>(cbuf, n, &s_f[5], randf, s_cdf, c0 == 0 ? 1024 : 0);
-						if (r >= 0) {
-							if (tid == 0) s_i[1] = c0 + r;
-							break;
-						}
-					}
-					__syncthreads();
-					if (tid == 0) {
-						__stcg(a.samp_i + G, s_i[1] < 0 ? 0 : s_i[1]);
-						*a.randf_count = rc + 1;
-					}
-				}
-				mg_grid_sync(ctx);
-				next_tok = __ldcg(a.samp_i + G);
+				// The row is worked on in the idle weight ring. (The count is read by every CTA before the barriers
+				// behind which CTA 0 raises it.)
+				const int rc = __ldcg(a.randf_count);
+				const float randf = rc < a.randf_cap ? __ldg(a.randf + rc) : 0.0f;
+				next_tok = minp_grid_row<MG_NWARPS>(a.logits, a.probs, a.V, a.minp, a.temp, gmax, randf, a.samp_f, reinterpret_cast<float *>(R_D), bred, s_cdf,
+				                             [&] { mg_grid_sync(ctx); });
+				if (cta == 0 && tid == 0) *a.randf_count = rc + 1;
+				fence_proxy_async();  // (bulk copies refill the ring)
+				__syncthreads();
 			}
 			if (cta == 0 && tid == 0) {
 				if (a.tok_log && n_logged < a.log_cap) a.tok_log[n_logged] = next_tok;

@@ -58,7 +58,6 @@ constexpr int PS_NW = PS_THREADS / 32;
 constexpr int PS_MAX_LAYERS = 32;
 constexpr int PS_MAX_CH = 32;            // most cache chunks per head
 constexpr int PS_ATT_ROW = AT_HD + 8;    // floats per attention partial: o[256], m, l, padding
-constexpr int PS_SAMP_TILE = 128;        // vocabulary tile of the sampler's passes (same partition as minp_grid_kernel)
 constexpr uint32_t PS_BULK_PIECE = 16384;
 constexpr unsigned PS_EMPTY = 0xFFFFFFFFu;  // "not written yet": a NaN no computation produces
 
@@ -110,7 +109,6 @@ struct PsArgs {
 	int nch_local, nch_mid, nch_long;  // cache chunks per head: sliding-window layers / global up to 2048 keys / beyond
 	float *logits;
 	float *probs;
-	int samp_ch;
 	float *samp_f;
 	int *samp_i;
 	float *xnorm_out;
@@ -675,7 +673,7 @@ __global__ void retile_lm_kernel(int8_t *dst, const int8_t *src, int V, int ngro
 
 // lut::GeLUTable::lookup (reference ops.hpp:41-51) with the table kept L2-resident
 __device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint64_t keep) {
-	const float q = t.inv != 0.0f ? (x - t.mn) * t.inv : (x - t.mn) / t.eps;
+	const float q = (x - t.mn) / t.eps;
 	if (!(q < 2147483648.0f) || q < -2147483648.0f) return 0.0f;  // (x86 cvttss2si: INT_MIN, a negative index)
 	const int idx = int(q);
 	if (idx < 0) return 0.0f;
@@ -1217,13 +1215,21 @@ if (a.sampler == 0) {
 		float gmax = -INFINITY;
 		int gidx = -1;
 #pragma unroll 1
-		for (int c = lane; c < G; c += 32) {
-			float v = __ldcg(a.samp_f + c);
-			int ix = __ldcg(a.samp_i + c);
-			if (better(v, ix, gmax, gidx)) {
-				gmax = v;
-				gidx = ix;
+		for (int cb = lane; cb < G; cb += 32 * 5) {  // (five loads of each in flight)
+			float v[5];
+			int ix[5];
+#pragma unroll
+			for (int q = 0; q < 5; q++) {
+				const int c = cb + 32 * q;
+				v[q] = c < G ? __ldcg(a.samp_f + c) : -INFINITY;
+				ix[q] = c < G ? __ldcg(a.samp_i + c) : -1;
 			}
+#pragma unroll
+			for (int q = 0; q < 5; q++)
+				if (better(v[q], ix[q], gmax, gidx)) {
+					gmax = v[q];
+					gidx = ix[q];
+				}
 		}
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) {
@@ -1247,72 +1253,15 @@ if (a.sampler == 0) {
 	} else {
 		// ops::minp_logits (reference ops.hpp:762-859). z = logit / temp; rowmax = gmax;
 		// p = exp(z - rowmax); maxp = exp(0) = 1 so cut = minp * 1; denom = sum of p >= cut.
-		const float cut = a.minp * expf(gmax - gmax);
-		float ds = 0.0f;
-		{
-			const int ntile = a.V / PS_SAMP_TILE;
-			const int my_tiles = (ntile - cta + G - 1) / G;
-#pragma unroll 1
-			for (int j = tid; j < my_tiles * PS_SAMP_TILE; j += PS_THREADS) {
-				const int v = (cta + (j / PS_SAMP_TILE) * G) * PS_SAMP_TILE + (j % PS_SAMP_TILE);
-				const float pv = expf(__ldcg(a.logits + v) / a.temp - gmax);
-				__stcg(a.probs + v, pv);
-				ds += (pv < cut) ? 0.0f : pv;
-			}
-		}
-		ds = block_sum<PS_NW>(ds, bred);
-		if (tid == 0) __stcg(a.samp_f + G + cta, ds);
-		ps_grid_sync(pw, wh, a.bar, a.bar_base + ++epoch * G);
-		if (cta == 0) {
-			// denominator: per-CTA sums added in a fixed tree by warp 0
-			if (warp == 0) {
-				float dv = 0.0f;
-#pragma unroll 1
-				for (int c = lane; c < G; c += 32) dv += __ldcg(a.samp_f + G + c);
-				dv = warp_sum(dv);
-				if (lane == 0) s_f[6] = 1.0f / dv;
-			}
-			float randf = 0.0f;
-			const int rc = __ldcg(a.randf_count);
-			if (rc < a.randf_cap) randf = __ldg(a.randf + rc);
-			__syncthreads();
-			const float inv = s_f[6];
-			// inverse CDF: the first index whose sequential fp32 running sum reaches randf,
-			// evaluated exactly and in parallel (cdf_cross_block) over chunks of probabilities
-			// p = exp(z - max) * inv staged in the idle weight ring
-			const int CH = a.samp_ch;
-			if (tid == 0) {
-				s_i[1] = -1;
-				s_f[5] = 0.0f;
-			}
-			__syncthreads();
-#pragma unroll 1
-			for (int c0 = 0; c0 < a.V; c0 += CH) {
-				const int n = min(CH, a.V - c0);
-#pragma unroll 4
-				for (int i = tid * 4; i < n; i += PS_THREADS * 4) {
-					float4 v = __ldcg(reinterpret_cast<const float4 *>(a.probs + c0 + i));
-					v.x *= inv;
-					v.y *= inv;
-					v.z *= inv;
-					v.w *= inv;
-					*reinterpret_cast<float4 *>(cbuf + i) = v;
-				}
-				__syncthreads();
-				const int r = cdf_cross_block<PS_NW>(cbuf, n, &s_f[5], randf, s_cdf, c0 == 0 ? 1024 : 0);
-				if (r >= 0) {
-					if (tid == 0) s_i[1] = c0 + r;
-					break;
-				}
-			}
-			__syncthreads();
-			if (tid == 0) {
-				__stcg(a.samp_i + G, s_i[1] < 0 ? 0 : s_i[1]);
-				*a.randf_count = rc + 1;
-			}
-		}
-		ps_grid_sync(pw, wh, a.bar, a.bar_base + ++epoch * G);
-		next_tok = __ldcg(a.samp_i + G);
+		// The row is worked on in the idle weight ring. (The count is read by every CTA before the barriers
+		// behind which CTA 0 raises it.)
+		const int rc = __ldcg(a.randf_count);
+		const float randf = rc < a.randf_cap ? __ldg(a.randf + rc) : 0.0f;
+		next_tok = minp_grid_row<PS_NW>(a.logits, a.probs, a.V, a.minp, a.temp, gmax, randf, a.samp_f, cbuf, bred, s_cdf,
+		                             [&] { ps_grid_sync(pw, wh, a.bar, a.bar_base + ++epoch * G); });
+		if (cta == 0 && tid == 0) *a.randf_count = rc + 1;
+		ps_fence_async();  // (bulk copies refill the ring)
+		__syncthreads();
 	}
 	if (cta == 0 && tid == 0) {
 		if (a.tok_log && n_logged < a.log_cap) a.tok_log[n_logged] = next_tok;

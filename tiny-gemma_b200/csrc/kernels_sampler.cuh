@@ -140,8 +140,12 @@ constexpr int CDF_PER_WARP = 32 * CDF_PER_LANE;
 __device__ __forceinline__ void cdf_cross_seq(const float *p, int end, float randf, float &cum, int &pos, int &res) {
 	float c = cum;
 	int i = pos;
+	float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+	if (i + 8 <= end) {
+		a = *reinterpret_cast<const float4 *>(p + i);
+		b = *reinterpret_cast<const float4 *>(p + i + 4);
+	}
 	for (; i + 8 <= end; i += 8) {
-		const float4 a = *reinterpret_cast<const float4 *>(p + i), b = *reinterpret_cast<const float4 *>(p + i + 4);
 		float cs[8];
 		cs[0] = c + a.x;
 		cs[1] = cs[0] + a.y;
@@ -151,6 +155,10 @@ __device__ __forceinline__ void cdf_cross_seq(const float *p, int end, float ran
 		cs[5] = cs[4] + b.y;
 		cs[6] = cs[5] + b.z;
 		cs[7] = cs[6] + b.w;
+		if (i + 16 <= end) {  // (the next group is on its way while this one's chain of additions runs)
+			a = *reinterpret_cast<const float4 *>(p + i + 8);
+			b = *reinterpret_cast<const float4 *>(p + i + 12);
+		}
 		if (cs[7] >= randf) {
 			int k = 7;
 #pragma unroll
@@ -302,6 +310,95 @@ __device__ int cdf_cross_block(const float *p, int n, float *cum_io, float randf
 	return *s_res;
 }
 
+// The same for a block of at most 256 elements by one warp, without a barrier: p[0..n) in shared memory, 16-byte aligned, n a
+// multiple of 8, all lanes call it with the same arguments. Returns the index inside the block or -1; cum becomes the sum
+// behind the last element consumed. seq: add the elements one by one (the start of a row).
+constexpr int CDF_BLK = 256;
+__device__ __forceinline__ int cdf_cross_warp(const float *p, int n, float &cum, float randf, bool seq) {
+	const int lane = threadIdx.x & 31, base = 8 * lane;
+	if (seq) {
+		int pos = 0, res = -1;
+		float c = cum;
+		if (lane == 0) cdf_cross_seq(p, n, randf, c, pos, res);
+		cum = __shfl_sync(0xffffffffu, c, 0);
+		return __shfl_sync(0xffffffffu, res, 0);
+	}
+	float x[8];
+#pragma unroll
+	for (int k = 0; k < 8; k++) x[k] = base < n ? p[base + k] : 0.0f;
+	int pos = 0;
+#pragma unroll 1
+	for (int guard = 0; pos < n && guard < n + 8; guard++) {  // every round consumes at least one element
+		const int e = int((__float_as_uint(cum) >> 23) & 0xffu) - 127;
+		if (!(cum >= 7.888609e-31f) || e > 120) {
+			// zero, tiny, inf or NaN: plain fp32 steps until the sum is an ordinary number
+			int res = -1;
+			for (; pos < n && res < 0; pos++) {
+				cum += p[pos];
+				if (cum >= randf) res = pos;
+				if (cum >= 7.888609e-31f && cum < 1e36f) {
+					pos++;
+					break;
+				}
+			}
+			if (res >= 0) return res;
+			continue;
+		}
+		const float u = __uint_as_float(unsigned(e - 23 + 127) << 23), inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
+		const int S0 = int(cum * inv_u);
+		const float y = randf * inv_u;
+		const int Tmin = min((y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG, 1 << 24);
+		CdfFn el[8], inc{0, 0};
+#pragma unroll
+		for (int k = 0; k < 8; k++) {
+			el[k] = CdfFn{0, 0};
+			if (base + k >= pos && base + k < n) el[k] = cdf_element(x[k], inv_u);
+			inc = cdf_compose(inc, el[k]);
+		}
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			CdfFn prev;
+			prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
+			prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
+			if (lane >= o) inc = cdf_compose(prev, inc);
+		}
+		const int end = cdf_apply(inc, S0);  // the sum behind this lane's elements
+		int S = __shfl_up_sync(0xffffffffu, end, 1);
+		if (lane == 0) S = S0;
+		const unsigned hit = __ballot_sync(0xffffffffu, end >= Tmin);
+		if (!hit) {
+			cum = float(__shfl_sync(0xffffffffu, end, 31)) * u;  // exact: below 2^24
+			return -1;
+		}
+		int at = -1, before = 0, after = 0;
+		float pe = 0.0f;
+#pragma unroll
+		for (int k = 0; k < 8; k++) {
+			const int nx = cdf_apply(el[k], S);
+			if (at < 0 && nx >= Tmin) {
+				at = base + k;
+				before = S;
+				after = nx;
+				pe = x[k];
+			}
+			S = nx;
+		}
+		const int src = __ffs(hit) - 1;
+		at = __shfl_sync(0xffffffffu, at, src);
+		before = __shfl_sync(0xffffffffu, before, src);
+		after = __shfl_sync(0xffffffffu, after, src);
+		pe = __shfl_sync(0xffffffffu, pe, src);
+		if (after < (1 << 24)) {  // the sum reached randf inside the binade
+			cum = float(after) * u;
+			return at;
+		}
+		cum = float(before) * u + pe;  // the one addition that leaves the binade
+		if (cum >= randf) return at;
+		pos = at + 1;
+	}
+	return -1;
+}
+
 // ops::minp_logits, reference ops.hpp:762-859.
 //  (1) x /= temp  (2) rowmax  (3) p = exp(x - rowmax), maxp  (4) cut = minp*maxp,
 //  denom = sum of p >= cut  (5) every p *= 1/denom — tokens under the cut keep
@@ -317,14 +414,15 @@ constexpr int MP_CHUNK = 8192;
 // scaling and segment maps; the walk). One CTA per row took ~1 ms for a row of 262144: four passes over 1 MB and
 // the whole chain of step 6, all latency. Step 6 here: the row is cut into segments of 1024. The sum at a segment's
 // start is known approximately from the segment sums, so its binade is, and with it the segment's composite map of that
-// binade (see above), which all segments compute at once. The walk then applies whole segments, 32 at a time by a warp
-// scan, and checks every one against the exact state: a segment whose predicted binade is not the actual one, or inside
-// which the sum leaves the binade or reaches randf, is evaluated element by element (about ten of 256).
+// binade (see above), which all segments, and all blocks of 256, compute at once. The walk then applies whole segments, 32 at
+// a time by a warp scan, and checks every one against the exact state: a segment whose predicted binade is not the actual
+// one, or inside which the sum leaves the binade or reaches randf, is walked by its blocks, such a block by its elements.
 constexpr int SR_SEG = 1024;
 struct MinpRows {
 	float *part_max;  // [B][V / SR_PART]
 	float2 *seg_sum;  // [B][V / SR_SEG] masked sum, whole sum
 	int4 *seg_map;    // [B][V / SR_SEG] a0, a1, exponent of the binade
+	int4 *blk_map;    // [B][V / CDF_BLK]
 };
 __global__ void __launch_bounds__(SR_THREADS) minp_max_kernel(SampleArgs a, MinpRows w) {
 	pdl_trigger();
@@ -430,16 +528,20 @@ __global__ void __launch_bounds__(SR_THREADS) minp_scale_kernel(SampleArgs a, Mi
 	}
 	for (int i = first; i < seg; i++) before += ss[i].y;
 	const float inv = 1.0f / denom;
-	const int e = int((__float_as_uint(before * inv) >> 23) & 0xffu) - 127;
-	const bool usable = before * inv >= 7.888609e-31f && e <= 120;
-	const float inv_u = usable ? __uint_as_float(unsigned(23 - e + 127) << 23) : 1.0f;
 	CdfFn whole{0, 0};
+	int es = 0;  // the binade of all blocks so far, or -1000
 #pragma unroll
-	for (int q = 0; q < SR_SEG / 256; q++) {
+	for (int q = 0; q < SR_SEG / CDF_BLK; q++) {
+		const float at = before * inv;
+		const int e = int((__float_as_uint(at) >> 23) & 0xffu) - 127;
+		const bool usable = at >= 7.888609e-31f && e <= 120;
+		const float inv_u = usable ? __uint_as_float(unsigned(23 - e + 127) << 23) : 1.0f;
 		CdfFn f{0, 0};
+		float sum = 0.0f;
 #pragma unroll
 		for (int h = 0; h < 2; h++) {
 			float4 &t = v[2 * q + h];
+			sum += (t.x + t.y) + (t.z + t.w);
 			t.x *= inv;
 			t.y *= inv;
 			t.z *= inv;
@@ -450,84 +552,263 @@ __global__ void __launch_bounds__(SR_THREADS) minp_scale_kernel(SampleArgs a, Mi
 			f = cdf_compose(f, cdf_element(t.z, inv_u));
 			f = cdf_compose(f, cdf_element(t.w, inv_u));
 		}
-		whole = cdf_compose(whole, cdf_warp_compose(f));
+		f = cdf_warp_compose(f);
+		before += warp_sum(sum);
+		whole = cdf_compose(whole, f);
+		const int eq = usable ? e : -1000;
+		es = q == 0 || es == eq ? eq : -1000;
+		if (lane == 0) w.blk_map[(size_t(b) * nseg + seg) * (SR_SEG / CDF_BLK) + q] = make_int4(f.a0, f.a1, eq, 0);
 	}
-	if (lane == 0) w.seg_map[size_t(b) * nseg + seg] = make_int4(whole.a0, whole.a1, usable ? e : -1000, 0);
+	if (lane == 0) w.seg_map[size_t(b) * nseg + seg] = make_int4(whole.a0, whole.a1, es, 0);
 }
-// one CTA per row
-__global__ void __launch_bounds__(SR_THREADS) minp_walk_kernel(SampleArgs a, MinpRows w) {
+// One warp applies the maps get(i) = (a0, a1, binade) of whole segments from `seg` on to the running sum, 32 at a time, up to the first
+// one whose binade is not the actual one or inside which the sum leaves the binade or reaches randf.
+template <class Get> __device__ __forceinline__ float cdf_walk_maps(Get get, int nseg, float randf, float cum, int &seg) {
+	const int lane = threadIdx.x & 31;
+	while (seg < nseg) {
+		const int4 m = seg + lane < nseg ? get(seg + lane) : make_int4(0, 0, -2000, 0);
+		const int e = int((__float_as_uint(cum) >> 23) & 0xffu) - 127;
+		if (!(cum >= 7.888609e-31f) || e > 120) break;
+		const float u = __uint_as_float(unsigned(e - 23 + 127) << 23), inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
+		const int S0 = int(cum * inv_u);
+		const float y = randf * inv_u;
+		const int Tmin = min((y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG, 1 << 24);
+		CdfFn inc{m.x, m.y};
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1) {
+			CdfFn prev;
+			prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
+			prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
+			if (lane >= o) inc = cdf_compose(prev, inc);
+		}
+		const int S = cdf_apply(inc, S0);
+		const unsigned bad = __ballot_sync(0xffffffffu, m.z != e || S >= Tmin);
+		const int n = bad ? __ffs(bad) - 1 : 32;
+		if (n > 0) cum = float(__shfl_sync(0xffffffffu, S, n - 1)) * u;
+		seg += n;
+		if (n < 32) break;
+	}
+	return cum;
+}
+// One warp walks a row p of V elements in segments of seg_len (nb blocks of CDF_BLK, the last segment may end early): segment
+// maps, inside a segment whose map does not hold the maps of its blocks, inside such a block its elements. Returns the crossing
+// index, 0 if there is none. chunk: CDF_BLK floats of shared memory.
+template <class Seg, class Blk>
+__device__ __forceinline__ int cdf_walk_row(Seg seg_map, Blk blk_map, const float *p, int V, int seg_len, int nb, float randf, float *chunk) {
+	const int lane = threadIdx.x & 31, nseg = (V + seg_len - 1) / seg_len;
+	float cum = 0.0f;
+#pragma unroll 1
+	for (int c = 0; c < nseg; c++) {
+		cum = cdf_walk_maps(seg_map, nseg, randf, cum, c);
+		if (c >= nseg) break;
+		const int m = min(seg_len, V - c * seg_len), mb = (m + CDF_BLK - 1) / CDF_BLK;
+#pragma unroll 1
+		for (int b = 0; b < mb; b++) {
+			cum = cdf_walk_maps([&](int i) { return blk_map(c * nb + i); }, mb, randf, cum, b);
+			if (b >= mb) break;
+			const int left = min(CDF_BLK, m - CDF_BLK * b);
+			__syncwarp();
+			if (8 * lane < left) {
+				const float4 *src = reinterpret_cast<const float4 *>(p + size_t(c) * seg_len + CDF_BLK * b + 8 * lane);
+				const float4 v0 = __ldcg(src), v1 = __ldcg(src + 1);
+				reinterpret_cast<float4 *>(chunk + 8 * lane)[0] = v0;
+				reinterpret_cast<float4 *>(chunk + 8 * lane)[1] = v1;
+			}
+			__syncwarp();
+			const int r = cdf_cross_warp(chunk, left, cum, randf, c == 0 && b == 0);
+			if (r >= 0) return c * seg_len + CDF_BLK * b + r;
+		}
+	}
+	return 0;
+}
+// one warp walks a row; the CTA brings the row's maps into shared memory before (minp_walk_smem(V) bytes): the walk is a chain of
+// dependent steps, and a load from the L2 in each would double it. Rows whose maps pass 44 KB (staged = 0) are read there.
+inline size_t minp_walk_smem(int V) { return size_t(V / SR_SEG) * (1 + SR_SEG / CDF_BLK) * 16; }
+__global__ void __launch_bounds__(SR_THREADS) minp_walk_kernel(SampleArgs a, MinpRows w, int staged) {
 	pdl_trigger();
 	pdl_wait();
-	__shared__ float chunk[SR_SEG];
-	__shared__ int scratch[2 * (SR_THREADS / 32) + 8];
-	__shared__ float s_cum;
-	__shared__ int s_seg;
-	const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+	extern __shared__ __align__(16) int4 mw_maps[];  // [nseg] segments, [nseg][NB] blocks
+	__shared__ __align__(16) float chunk[CDF_BLK];
+	constexpr int NB = SR_SEG / CDF_BLK;
+	const int b = blockIdx.x, tid = threadIdx.x;
 	const int nseg = a.V / SR_SEG;
 	const float *x = a.logits + size_t(b) * a.V;
-	const int4 *maps = w.seg_map + size_t(b) * nseg;
+	auto map = [&](int i) { return __ldcg(i < nseg ? w.seg_map + size_t(b) * nseg + i : w.blk_map + size_t(b) * nseg * NB + (i - nseg)); };
+	if (staged) {
+#pragma unroll 4
+		for (int i = tid; i < nseg * (1 + NB); i += SR_THREADS) mw_maps[i] = map(i);
+	}
 	float randf = 0.0f;
 	const int rc = a.randf_count[b];
 	if (rc < a.randf_cap) randf = a.randf[size_t(rc) * a.B + b];
-	if (tid == 0) s_cum = 0.0f;
-	int found = -1;
-	for (int seg = 0; seg < nseg && found < 0; seg++) {
-		__syncthreads();
-		if (tid < 32) {  // whole segments
-			float cum = s_cum;
-			for (; seg < nseg;) {
-				const int4 m = seg + lane < nseg ? __ldcg(maps + seg + lane) : make_int4(0, 0, -2000, 0);
-				const int e = int((__float_as_uint(cum) >> 23) & 0xffu) - 127;
-				if (!(cum >= 7.888609e-31f) || e > 120) break;
-				const float u = __uint_as_float(unsigned(e - 23 + 127) << 23), inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
-				const int S0 = int(cum * inv_u);
-				const float y = randf * inv_u;
-				const int Tmin = min((y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG, 1 << 24);
-				CdfFn inc{m.x, m.y};
-#pragma unroll
-				for (int o = 1; o < 32; o <<= 1) {
-					CdfFn prev;
-					prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
-					prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
-					if (lane >= o) inc = cdf_compose(prev, inc);
-				}
-				const int S = cdf_apply(inc, S0);
-				const unsigned bad = __ballot_sync(0xffffffffu, m.z != e || S >= Tmin);
-				const int n = bad ? __ffs(bad) - 1 : 32;
-				if (n > 0) cum = float(__shfl_sync(0xffffffffu, S, n - 1)) * u;
-				seg += n;
-				if (n < 32) break;
-			}
-			if (lane == 0) {
-				s_cum = cum;
-				s_seg = seg;
-			}
-		}
-		__syncthreads();
-		seg = s_seg;
-		if (seg >= nseg) break;
-		reinterpret_cast<float4 *>(chunk)[tid] = __ldcg(reinterpret_cast<const float4 *>(x + size_t(seg) * SR_SEG) + tid);
-		__syncthreads();
-		const int r = cdf_cross_block<SR_THREADS / 32>(chunk, SR_SEG, &s_cum, randf, scratch, seg == 0 ? SR_SEG : 0);
-		if (r >= 0) found = seg * SR_SEG + r;
-	}
+	__syncthreads();
+	if (tid >= 32) return;
+	const int found = cdf_walk_row([&](int i) { return staged ? mw_maps[i] : map(i); }, [&](int i) { return staged ? mw_maps[nseg + i] : map(nseg + i); }, x, a.V, SR_SEG, NB, randf, chunk);
 	if (tid == 0) {
-		emit_token(a, b, found < 0 ? 0 : found);
+		emit_token(a, b, found);
 		a.randf_count[b] = rc + 1;
 	}
 }
 
+// ------------------------------------------------------------------ min-p of one row by a whole grid
+// Steps (3) to (6) for a kernel of G CTAs that can meet at a grid barrier (`sync`): CTA c owns the columns
+// [c * cols, (c + 1) * cols), a warp of it blocks of 256. The CTA leaves its masked and whole sum, then (the denominator and
+// the approximate sum before every block being known) the composite map of every block in the binade that the running sum
+// is expected in, and the map of all its columns where that is one binade. One warp of every CTA then walks the row: CTA
+// maps, inside a CTA whose map does not hold the block maps, inside such a block its elements (about 20 blocks of 1024: where the
+// sum changes its binade, and the last one). So every CTA knows the token without another exchange. The row was walked
+// element by element by one CTA in rounds of 3072 before: a token of the 1B model 829 us for a crossing index in the middle
+// of the row, now 740 (695 for the arg-max).
+// part: minp_grid_part_bytes(V, G) bytes, of which the first G floats are the caller's; sm: shared memory, minp_grid_floats(V, G)
+// floats, 16-byte aligned; red: 2 * NW floats. V is a multiple of 128.
+__host__ __device__ __forceinline__ int minp_grid_cols(int V, int G) { return (V / 128 + G - 1) / G * 128; }
+__host__ __device__ __forceinline__ int minp_grid_blocks(int V, int G) { return (minp_grid_cols(V, G) + CDF_BLK - 1) / CDF_BLK; }
+__host__ __device__ __forceinline__ int minp_grid_floats(int V, int G) {
+	const int nb = minp_grid_blocks(V, G);
+	return CDF_BLK * nb + 4 * G * (1 + nb) + (nb + 3) / 4 * 4;
+}
+__host__ __device__ __forceinline__ size_t minp_grid_part_bytes(int V, int G) { return size_t((3 * G + 3) / 4 * 4 + 4 * G * (1 + minp_grid_blocks(V, G))) * 4; }
+template <int NW, class Sync>
+__device__ __forceinline__ int minp_grid_row(const float *logits, float *probs, int V, float minp, float temp, float gmax, float randf, float *part,
+                                             float *sm, float *red, int *scratch, Sync sync) {
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, G = gridDim.x;
+	const int cols = minp_grid_cols(V, G), nb = minp_grid_blocks(V, G), c0 = min(V, cta * cols), n = min(V, c0 + cols) - c0;
+	float *pl = sm;                                              // [nb][256]
+	int4 *maps = reinterpret_cast<int4 *>(sm + CDF_BLK * nb);    // [G] per CTA, [G][nb] per block
+	float *blk = reinterpret_cast<float *>(maps + G * (1 + nb));  // [nb] sums of this CTA's blocks
+	int4 *gmaps = reinterpret_cast<int4 *>(part + (3 * G + 3) / 4 * 4);
+	// p = exp(z - max); the largest is exp(0), so the cut is minp * exp(gmax - gmax)
+	const float cut = minp * expf(gmax - gmax);
+	float ds = 0.0f, us = 0.0f;
+#pragma unroll 1
+	for (int b = warp; b < nb; b += NW) {
+		float s = 0.0f;
+		if (CDF_BLK * b + 8 * lane < n) {
+			float4 v[2];
+#pragma unroll
+			for (int h = 0; h < 2; h++) v[h] = __ldcg(reinterpret_cast<const float4 *>(logits + c0 + CDF_BLK * b + 8 * lane) + h);
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				v[h].x = expf(v[h].x / temp - gmax);
+				v[h].y = expf(v[h].y / temp - gmax);
+				v[h].z = expf(v[h].z / temp - gmax);
+				v[h].w = expf(v[h].w / temp - gmax);
+				*(reinterpret_cast<float4 *>(pl + CDF_BLK * b + 8 * lane) + h) = v[h];
+				s += (v[h].x + v[h].y) + (v[h].z + v[h].w);
+				ds += (v[h].x < cut) ? 0.0f : v[h].x;
+				ds += (v[h].y < cut) ? 0.0f : v[h].y;
+				ds += (v[h].z < cut) ? 0.0f : v[h].z;
+				ds += (v[h].w < cut) ? 0.0f : v[h].w;
+			}
+		}
+		s = warp_sum(s);
+		if (lane == 0) blk[b] = s;
+		us += s;
+	}
+	ds = warp_sum(ds);
+	__syncthreads();
+	if (lane == 0) {
+		red[warp] = ds;
+		red[NW + warp] = us;
+	}
+	__syncthreads();
+	if (tid == 0) {
+		ds = us = 0.0f;
+		for (int w = 0; w < NW; w++) {
+			ds += red[w];
+			us += red[NW + w];
+		}
+		__stcg(part + G + cta, ds);
+		__stcg(part + 2 * G + cta, us);
+	}
+	sync();
+	if (warp == 0) {
+		float dv = 0.0f, bv = 0.0f;
+		for (int cb = lane; cb < G; cb += 32 * 5) {  // (five loads of each row in flight)
+			float d[5], u[5];
+#pragma unroll
+			for (int q = 0; q < 5; q++) {
+				const int c = cb + 32 * q;
+				d[q] = c < G ? __ldcg(part + G + c) : 0.0f;
+				u[q] = c < cta ? __ldcg(part + 2 * G + c) : 0.0f;
+			}
+#pragma unroll
+			for (int q = 0; q < 5; q++) {
+				dv += d[q];
+				bv += u[q];
+			}
+		}
+		dv = warp_sum(dv);
+		bv = warp_sum(bv);
+		if (lane == 0) {
+			red[0] = 1.0f / dv;
+			red[1] = bv;
+		}
+	}
+	__syncthreads();
+	const float inv = red[0];
+#pragma unroll 1
+	for (int b = warp; b < nb; b += NW) {
+		float before = red[1];
+		for (int q = 0; q < b; q++) before += blk[q];
+		before *= inv;
+		const int e = int((__float_as_uint(before) >> 23) & 0xffu) - 127;
+		const bool usable = before >= 7.888609e-31f && e <= 120;
+		const float inv_u = usable ? __uint_as_float(unsigned(23 - e + 127) << 23) : 1.0f;
+		CdfFn f{0, 0};
+		if (CDF_BLK * b + 8 * lane < n) {
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				float4 t = *(reinterpret_cast<const float4 *>(pl + CDF_BLK * b + 8 * lane) + h);
+				t.x *= inv;
+				t.y *= inv;
+				t.z *= inv;
+				t.w *= inv;
+				__stcg(reinterpret_cast<float4 *>(probs + c0 + CDF_BLK * b + 8 * lane) + h, t);
+				f = cdf_compose(f, cdf_element(t.x, inv_u));
+				f = cdf_compose(f, cdf_element(t.y, inv_u));
+				f = cdf_compose(f, cdf_element(t.z, inv_u));
+				f = cdf_compose(f, cdf_element(t.w, inv_u));
+			}
+		}
+		f = cdf_warp_compose(f);
+		if (lane == 0) {
+			const int4 m = make_int4(f.a0, f.a1, usable ? e : -1000, 0);
+			maps[b] = m;
+			__stcg(gmaps + G + cta * nb + b, m);
+		}
+	}
+	__syncthreads();
+	if (tid == 0) {
+		CdfFn whole{0, 0};
+		int e = maps[0].z;
+		for (int b = 0; CDF_BLK * b < n; b++) {
+			whole = cdf_compose(whole, CdfFn{maps[b].x, maps[b].y});
+			if (maps[b].z != e) e = -1000;
+		}
+		__stcg(gmaps + cta, make_int4(whole.a0, whole.a1, e, 0));
+	}
+	sync();
+	for (int c = tid; c < G * (1 + nb); c += 32 * NW) maps[c] = __ldcg(gmaps + c);
+	__syncthreads();
+	if (warp == 0) {
+		const int found = cdf_walk_row([&](int i) { return maps[i]; }, [&](int i) { return maps[G + i]; }, probs, V, cols, nb, randf, pl);
+		if (lane == 0) scratch[0] = found;
+	}
+	__syncthreads();
+	const int found = scratch[0];
+	__syncthreads();
+	return found;
+}
+
 // ------------------------------------------------------------------ grid-wide min-p (one sequence)
 // ops::minp_logits for a single row spread over G CTAs of SG_THREADS threads (cooperative launch: the
-// CTAs meet at a bounded grid barrier). It partitions the row and orders every floating-point sum
-// exactly like the sampler inside the persistent decode kernel — CTA c owns the 128-column tiles
-// c, c + G, ...; per-thread strided sums, a 12-warp block sum, the G partial sums added by one warp
-// in lane-strided order — so a token sampled step by step (tg_decode + tg_sample_minp) is the token
-// the device-resident loop samples. The row is overwritten with the probabilities, as the
+// CTAs meet at a bounded grid barrier). It partitions the row and orders every floating-point sum exactly like the
+// sampler inside the persistent decode kernels (minp_grid_row), so a token sampled step by step (tg_decode +
+// tg_sample_minp) is the token the device-resident loop samples. The row is overwritten with the probabilities, as the
 // reference does.
 constexpr int SG_THREADS = 384;
 constexpr int SG_NWARPS = SG_THREADS / 32;
-constexpr int SG_TILE = 128;
 constexpr int SG_SPIN_CAP = 1 << 22;
 
 __device__ __forceinline__ bool sg_grid_sync(unsigned *bar, unsigned &epoch, unsigned G, int *fail) {
@@ -549,38 +830,25 @@ __device__ __forceinline__ bool sg_grid_sync(unsigned *bar, unsigned &epoch, uns
 	return !*(volatile int *)fail;
 }
 
-template <int NW>
-__device__ __forceinline__ float sg_block_sum(float v, float *red) {
-	v = warp_sum(v);
-	__syncthreads();
-	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-	__syncthreads();
-	float t = 0.0f;
-#pragma unroll
-	for (int w = 0; w < NW; w++) t += red[w];
-	return t;
-}
-
-// part: [2 * G] floats of scratch, probs: [V] floats of scratch, bar: one zeroed word, err: error word
-__global__ void __launch_bounds__(SG_THREADS, 1) minp_grid_kernel(SampleArgs a, unsigned *bar, float *part, float *probs, int *err) {
-	__shared__ float red[SG_NWARPS];
-	__shared__ float chunk[MP_CHUNK];
-	__shared__ int scratch[2 * SG_NWARPS + 8];
-	__shared__ float s_cum, s_inv, s_max;
-	__shared__ int s_fail, s_tok;
+// part: minp_grid_part_bytes(V, G) of scratch, bar: one zeroed word, err: error word, minp_grid_floats(V, G) dynamic floats
+__global__ void __launch_bounds__(SG_THREADS, 1) minp_grid_kernel(SampleArgs a, unsigned *bar, float *part, int *err) {
+	extern __shared__ __align__(16) float sm[];
+	__shared__ float red[2 * SG_NWARPS];
+	__shared__ int scratch[1];
+	__shared__ float s_max;
+	__shared__ int s_fail;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int cta = blockIdx.x, G = gridDim.x;
-	const int ntiles = a.V / SG_TILE;
-	const int my_tiles = (ntiles - cta + G - 1) / G;
+	const int cols = minp_grid_cols(a.V, G), c0 = min(a.V, cta * cols), c1 = min(a.V, c0 + cols);
 	unsigned epoch = 0;
 	if (tid == 0) s_fail = 0;
 	__syncthreads();
 	// (1)+(2) row maximum of z = logit / temp
 	float mx = -INFINITY;
-#pragma unroll 1
-	for (int j = tid; j < my_tiles * SG_TILE; j += SG_THREADS) {
-		const int v = (cta + (j / SG_TILE) * G) * SG_TILE + (j % SG_TILE);
-		mx = fmaxf(mx, __ldcg(a.logits + v) / a.temp);
+#pragma unroll 2
+	for (int i = c0 + 4 * tid; i < c1; i += 4 * SG_THREADS) {
+		const float4 v = __ldcg(reinterpret_cast<const float4 *>(a.logits + i));
+		mx = fmaxf(mx, fmaxf(fmaxf(v.x / a.temp, v.y / a.temp), fmaxf(v.z / a.temp, v.w / a.temp)));
 	}
 	mx = warp_max(mx);
 	if (lane == 0) red[warp] = mx;
@@ -600,68 +868,14 @@ __global__ void __launch_bounds__(SG_THREADS, 1) minp_grid_kernel(SampleArgs a, 
 	}
 	__syncthreads();
 	const float gmax = s_max;
-	// (3)+(4) p = exp(z - max); maxp = exp(0), so the cut is minp * exp(gmax - gmax); masked denominator
-	const float cut = a.minp * expf(gmax - gmax);
-	float ds = 0.0f;
-#pragma unroll 1
-	for (int j = tid; j < my_tiles * SG_TILE; j += SG_THREADS) {
-		const int v = (cta + (j / SG_TILE) * G) * SG_TILE + (j % SG_TILE);
-		const float pv = expf(__ldcg(a.logits + v) / a.temp - gmax);
-		__stcg(probs + v, pv);
-		ds += (pv < cut) ? 0.0f : pv;
-	}
-	ds = sg_block_sum<SG_NWARPS>(ds, red);
-	if (tid == 0) __stcg(part + G + cta, ds);
-	sg_grid_sync(bar, epoch, G, &s_fail);
-	if (warp == 0) {
-		float dv = 0.0f;
-#pragma unroll 1
-		for (int c = lane; c < G; c += 32) dv += __ldcg(part + G + c);
-		dv = warp_sum(dv);
-		if (lane == 0) s_inv = 1.0f / dv;
-	}
-	__syncthreads();
-	const float inv = s_inv;
-	// (5) every probability is scaled in place of its logit
-#pragma unroll 1
-	for (int j = tid; j < my_tiles * SG_TILE; j += SG_THREADS) {
-		const int v = (cta + (j / SG_TILE) * G) * SG_TILE + (j % SG_TILE);
-		__stcg(a.logits + v, __ldcg(probs + v) * inv);
-	}
-	// (6) inverse CDF by CTA 0
-	if (cta == 0 && !*(volatile int *)&s_fail) {
-		float randf = 0.0f;
-		const int rc = a.randf_count[0];
-		if (rc < a.randf_cap) randf = a.randf[size_t(rc) * a.B];
-		if (tid == 0) {
-			s_cum = 0.0f;
-			s_tok = -1;
-		}
-		__syncthreads();
-#pragma unroll 1
-		for (int c0 = 0; c0 < a.V; c0 += MP_CHUNK) {
-			const int n = min(MP_CHUNK, a.V - c0);
-#pragma unroll 4
-			for (int i = tid * 4; i < n; i += SG_THREADS * 4) {
-				float4 v = __ldcg(reinterpret_cast<const float4 *>(probs + c0 + i));
-				v.x *= inv;
-				v.y *= inv;
-				v.z *= inv;
-				v.w *= inv;
-				*reinterpret_cast<float4 *>(chunk + i) = v;
-			}
-			__syncthreads();
-			const int r = cdf_cross_block<SG_NWARPS>(chunk, n, &s_cum, randf, scratch, c0 == 0 ? 1024 : 0);
-			if (r >= 0) {
-				if (tid == 0) s_tok = c0 + r;
-				break;
-			}
-		}
-		__syncthreads();
-		if (tid == 0) {
-			emit_token(a, 0, s_tok < 0 ? 0 : s_tok);
-			a.randf_count[0] = rc + 1;
-		}
+	const int rc = a.randf_count[0];  // (read by every CTA before the barriers behind which CTA 0 counts up)
+	const float randf = rc < a.randf_cap ? a.randf[size_t(rc) * a.B] : 0.0f;
+	// (3) to (6); every probability is scaled in place of its logit
+	const int tok = minp_grid_row<SG_NWARPS>(a.logits, a.logits, a.V, a.minp, a.temp, gmax, randf, part, sm, red, scratch,
+	                                         [&] { sg_grid_sync(bar, epoch, G, &s_fail); });
+	if (cta == 0 && tid == 0 && !*(volatile int *)&s_fail) {
+		emit_token(a, 0, tok);
+		a.randf_count[0] = rc + 1;
 	}
 	if (tid == 0 && *(volatile int *)&s_fail) atomicExch(err, 8);
 }

@@ -399,14 +399,16 @@ struct SampScratch {
 	MinpRows rows{};
 	unsigned long long *keys = nullptr;
 	unsigned *tickets = nullptr;
-	static size_t bytes(int B, size_t V) { return size_t(B) * ((V / SR_SEG + 1) * (16 + 8) + (V / SR_PART + 1) * 4 + 12) + 64; }
+	static size_t bytes(int B, size_t V) { return size_t(B) * ((V / SR_SEG + 1) * (16 + SR_SEG / CDF_BLK * 16 + 8) + (V / SR_PART + 1) * 4 + 12) + 64; }
 	SampScratch(uint8_t *p, int B, size_t V) {
 		const size_t nseg = size_t(B) * (V / SR_SEG + 1);
 		rows.seg_map = reinterpret_cast<int4 *>(p);
-		rows.seg_sum = reinterpret_cast<float2 *>(p + nseg * 16);
-		keys = reinterpret_cast<unsigned long long *>(p + nseg * 24);
-		tickets = reinterpret_cast<unsigned *>(p + nseg * 24 + size_t(B) * 8);
-		rows.part_max = reinterpret_cast<float *>(p + nseg * 24 + size_t(B) * 12);
+		rows.blk_map = rows.seg_map + nseg;
+		p += nseg * (16 + SR_SEG / CDF_BLK * 16);
+		rows.seg_sum = reinterpret_cast<float2 *>(p);
+		keys = reinterpret_cast<unsigned long long *>(p + nseg * 8);
+		tickets = reinterpret_cast<unsigned *>(p + nseg * 8 + size_t(B) * 8);
+		rows.part_max = reinterpret_cast<float *>(p + nseg * 8 + size_t(B) * 12);
 	}
 };
 
@@ -1010,7 +1012,7 @@ int mega_setup(tg_state *s) {
 	TG_CUDA(cudaMemset(s->mg_ll, 0xFF, s->mg_ll_bytes));
 	a.pe_stride = a.E.nsplit * D + ((G - a.E.units + 3) & ~3) + 4;
 	TG_TRY(allocz((void **)&s->mg_pe, size_t(2) * a.pe_stride * sizeof(uint2)));
-	TG_TRY(allocz((void **)&s->mg_samp_f, size_t(3) * G * 4));
+	TG_TRY(allocz((void **)&s->mg_samp_f, minp_grid_part_bytes(V, G)));
 	TG_TRY(allocz((void **)&s->mg_samp_i, size_t(G + 8) * 4));
 	TG_TRY(allocz((void **)&s->mg_bar, 64));
 	a.tmaps = s->d_tmaps;
@@ -1033,8 +1035,7 @@ int mega_setup(tg_state *s) {
 	a.probs = s->mg_probs;
 	{
 		const int region_floats = (a.off_h - a.off_D) / 4;
-		a.samp_ch = std::max(3072, std::min(region_floats, 24576) / 3072 * 3072);
-		if (a.samp_ch > region_floats) return fail(TG_ESHAPE, "sampler staging does not fit the weight ring");
+		if (minp_grid_floats(V, G) > region_floats) return fail(TG_ESHAPE, "sampler staging does not fit the weight ring");
 	}
 	a.samp_f = s->mg_samp_f;
 	a.samp_i = s->mg_samp_i;
@@ -1205,8 +1206,7 @@ int persist_setup(tg_state *s) {
 	a.smem_total = off + 128;
 	{
 		const int region_floats = region / 4;
-		a.samp_ch = std::min(region_floats, 24576) / 3072 * 3072;
-		if (a.samp_ch < 3072) return fail(TG_ESHAPE, "persistent kernel: sampler staging does not fit");
+		if (minp_grid_floats(V, G) > region_floats) return fail(TG_ESHAPE, "persistent kernel: sampler staging does not fit");
 	}
 	cudaFuncAttributes fa{};
 	TG_CUDA(cudaFuncGetAttributes(&fa, decode_persist_kernel<true>));
@@ -1495,7 +1495,9 @@ int launch_minp_rows(const SampleArgs &a, const SampScratch &ws, cudaStream_t st
 	launch_k(minp_max_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
 	launch_k(minp_exp_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
 	launch_k(minp_scale_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
-	launch_k(minp_walk_kernel, dim3(a.B), dim3(SR_THREADS), 0, st, a, ws.rows);
+	const size_t maps = minp_walk_smem(a.V);
+	const int staged = maps <= 48 * 1024 - 4096;
+	launch_k(minp_walk_kernel, dim3(a.B), dim3(SR_THREADS), staged ? maps : 0, st, a, ws.rows, staged);
 	count_launch(4);
 	return check_launch("minp");
 }
@@ -1507,10 +1509,10 @@ int enqueue_sampler(tg_state *s, float minp, float temp, bool log_tokens) {
 		TG_CUDA(cudaMemsetAsync(s->mg_bar + 8, 0, 4, s->stream));
 		unsigned *bar = s->mg_bar + 8;
 		float *part = s->mg_samp_f;
-		float *probs = s->mg_probs;
 		int *err = s->err_flag;
-		void *params[] = {&a, &bar, &part, &probs, &err};
-		TG_CUDA(cudaLaunchCooperativeKernel((void *)minp_grid_kernel, dim3(s->mega_grid), dim3(SG_THREADS), params, 0, s->stream));
+		void *params[] = {&a, &bar, &part, &err};
+		TG_CUDA(cudaLaunchCooperativeKernel((void *)minp_grid_kernel, dim3(s->mega_grid), dim3(SG_THREADS), params,
+		                                    size_t(minp_grid_floats(a.V, s->mega_grid)) * 4, s->stream));
 		count_launch();
 		return check_launch("minp_grid");
 	}
