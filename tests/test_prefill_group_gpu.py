@@ -23,3 +23,18 @@ def test_group_is_each_prompt(capi, synth, weights_270m, n, S):
     st.close()
     one.close()
     m.close()
+
+
+def test_small_batch_keeps_the_bits_of_one_prompt(capi, synth, weights_270m):
+    """Two prompts whose rows together, but not alone, pass the line between the attention kernels."""
+    m = capi.Model("270m").load_file(weights_270m)
+    m.build_tables(1024)
+    prompts = np.stack([synth.random_prompt(490, 60 + i) for i in range(2)])
+    st, one = m.state(2, 512), m.state(1, 512)
+    logits = st.prefill(prompts)
+    for i in range(2):
+        one.reset()
+        assert np.array_equal(logits[i], one.prefill(prompts[i])[0]), i
+    st.close()
+    one.close()
+    m.close()

@@ -2043,7 +2043,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 	// 450 tokens 2.9 against 3.6 ms, 832 tokens 4.93 against 5.04, 16 prompts of 61 tokens 3.98 against 4.29; 8 of 178 tokens
 	// 5.71 against 5.67, 256 of 178 tokens 170 against 150).
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
-	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && nb * S_seq > env_int("TG_ATTN_SMALL_MAX", 960) && S_seq >= env_int("TG_ATTN_TC_MIN", 0);
+	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && (plan_rows ? S_seq : nb * S_seq) > env_int("TG_ATTN_SMALL_MAX", 960) && S_seq >= env_int("TG_ATTN_TC_MIN", 0);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
