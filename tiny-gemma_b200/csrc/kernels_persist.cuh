@@ -106,7 +106,8 @@ struct PsArgs {
 	//                                      one presence word for every CTA without a down unit
 	float *ll;
 	int ll_stride, ll_qkv, ll_att, ll_op, ll_act, ll_dn, ll_pres;
-	int nch_local, nch_mid, nch_long;  // cache chunks per head: sliding-window layers / global up to 2048 keys / beyond
+	int nch_max, nch_local, nch_global;  // cache chunks per head: at most; a number given for sliding-window and global layers (0: by rule)
+	int slots_local;
 	float *logits;
 	float *probs;
 	float *samp_f;
@@ -1322,6 +1323,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	__shared__ int s_cdf[2 * PS_NW + 8];
 	__shared__ float wm[3 * PS_NW];  // per-warp (m, l, weight) of the attention merge; also the sampler's per-warp maxima
 	__shared__ PsLayer s_ly[PS_MAX_LAYERS];
+	__shared__ int s_nch[2];
 
 #define R_A (smem + a.off_A)
 #define R_C (smem + a.off_C)
@@ -1438,6 +1440,22 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			if (tid == 0 && cta == 0) atomicExch(a.err, 1);
 			tok = 0;
 		}
+		// Cache chunks per head of this token's attention. A warp holds two rows from before the poll for q|k|v, so a chunk takes
+		// a step for every 24 rows; phase C merges three chunks of a head at a time. The steps of both are dependent round
+		// trips, a merge is the shorter one: the multiple of 3 with the least 3 * steps + merges. (A fixed 8 up to 512
+		// rows, as before, against the rule: 411 / 406 us a token at 23 to 55 positions of the 270m model, 744 / 731 at 1500 of the
+		// 1B model.)
+		if (warp == 0) {
+			const bool loc = lane < 16;
+			const int n = min(3 * ((lane & 15) + 1), a.nch_max), v = loc ? min(pos + 1, a.slots_local) : pos + 1;
+			const int steps = ((v + n - 1) / n + 2 * PS_NW - 1) / (2 * PS_NW);
+			const unsigned key = unsigned(3 * steps + (n + 2) / 3) << 8 | unsigned(n);
+			const unsigned kl = __reduce_min_sync(0xffffffffu, loc ? key : ~0u), kg = __reduce_min_sync(0xffffffffu, loc ? ~0u : key);
+			if (lane == 0) {
+				s_nch[1] = a.nch_local ? a.nch_local : int(kl & 255u);
+				s_nch[0] = a.nch_global ? a.nch_global : int(kg & 255u);
+			}
+		}
 #pragma unroll 1
 		for (int d = tid; d < D; d += PS_THREADS) h[d] = a.wte_s[d] * (a.sqrtD * float(a.wte[size_t(tok) * D + d]));
 		__syncthreads();
@@ -1458,7 +1476,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 				slot = p;
 				valid = p + 1;
 			}
-			const int nch = ly.is_local ? a.nch_local : (valid <= 512 ? a.nch_local : (valid <= 2048 ? a.nch_mid : a.nch_long));
+			const int nch = s_nch[ly.is_local];
 			const int nsA = AT_NH * nch;  // CTAs that take part in attention
 			const int lc = step * L + l;
 			const int nl = (l + 1 < L) ? l + 1 : (more ? 0 : -1);  // the layer whose units are fetched next

@@ -1168,9 +1168,10 @@ int persist_setup(tg_state *s) {
 	a.A.cta0 = G - a.A.units;  // the attention CTAs (low indices) hold no Q|K|V unit where possible
 	// cache chunks per head; at least 8 CTAs must stay out of the attention phase (they wipe the hand-off arena)
 	const int chmax = std::max(1, std::min(PS_MAX_CH, (G - 8) / AT_NH));
-	a.nch_local = std::min(chmax, env_int("TG_PS_NCH_LOCAL", 8));
-	a.nch_mid = std::min(chmax, env_int("TG_PS_NCH_MID", 16));
-	a.nch_long = std::min(chmax, env_int("TG_PS_NCH_LONG", 32));
+	a.nch_max = chmax;
+	a.nch_local = std::min(chmax, std::max(0, env_int("TG_PS_NCH_LOCAL", 0)));
+	a.nch_global = std::min(chmax, std::max(0, env_int("TG_PS_NCH_GLOBAL", 0)));
+	a.slots_local = c.n_pos_local;
 	const int npres = G - a.E.units;
 	if (D / 4 + npres > PS_THREADS || G < 16) return fail(TG_ESHAPE, "persistent kernel: grid too small for the down-projection plan");
 	// lm_head: tiles of 24 column groups (two per warp); ring stages of at most ~40 KB
