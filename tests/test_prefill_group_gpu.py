@@ -38,3 +38,19 @@ def test_small_batch_keeps_the_bits_of_one_prompt(capi, synth, weights_270m):
     st.close()
     one.close()
     m.close()
+
+
+@pytest.mark.parametrize("n,S", [(4, 148), (4, 149), (7, 211)])
+def test_group_of_the_larger_model(capi, synth, weights_1b, n, S):
+    """Rows of 6912 columns on both sides of the line from which the GeGLU streams its rows (4 per SM)."""
+    m = capi.Model("1B").load_file(weights_1b)
+    m.build_tables(1 << 20)
+    prompts = np.stack([synth.random_prompt(S, 80 + i) for i in range(n)])
+    st, one = m.state(n, S + 8), m.state(1, S + 8)
+    logits = st.prefill(prompts)
+    for i in (0, n - 1):
+        one.reset()
+        assert rel_l2(logits[i], one.prefill(prompts[i])[0]) <= 5e-5, i
+    st.close()
+    one.close()
+    m.close()
