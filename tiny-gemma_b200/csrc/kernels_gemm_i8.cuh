@@ -280,6 +280,11 @@ __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_
 	if (in_smem)
 		for (int i = tid; i < lut.size; i += NT) table[i] = lut.table[i];
 	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 fs0 = z4, gs0 = z4;
+	if (PER == 1) {  // (nobody's output: requested before the wait; more of them would not fit the registers)
+		fs0 = __ldg(reinterpret_cast<const float4 *>(su) + min(tid, n4 - 1));
+		gs0 = __ldg(reinterpret_cast<const float4 *>(sg) + min(tid, n4 - 1));
+	}
 	__syncthreads();
 	pdl_trigger();
 	pdl_wait();
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_
 #pragma unroll
 		for (int j = 0; j < PER; j++) {
 			const int k4 = min(tid + NT * j, n4 - 1);
-			const float4 fs = __ldg(reinterpret_cast<const float4 *>(su) + k4), gs = __ldg(reinterpret_cast<const float4 *>(sg) + k4);
+			const float4 fs = PER == 1 ? fs0 : __ldg(reinterpret_cast<const float4 *>(su) + k4), gs = PER == 1 ? gs0 : __ldg(reinterpret_cast<const float4 *>(sg) + k4);
 			u[j].x = gelu(g[j].x * gs.x) * (u[j].x * fs.x);
 			u[j].y = gelu(g[j].y * gs.y) * (u[j].y * fs.y);
 			u[j].z = gelu(g[j].z * gs.z) * (u[j].z * fs.z);
