@@ -35,6 +35,27 @@ def test_many_tiles_per_cta(capi):
     assert rel_l2(capi.qgemm(x, w, s), exact(x, w, s)) <= 2e-7
 
 
+def test_more_tiles_than_a_16_bit_square(capi):
+    # 4360 rows of the vocabulary's columns: the tile index times its divisor passes 2^32 (70656 tiles of one CTA)
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    M, K, N = 4360, 256, 262144
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    w = torch.randint(-128, 128, (K, N), dtype=torch.int8, device="cuda", generator=g)
+    s = torch.rand(N, device="cuda", generator=g) * 1e-2 + 1e-4
+    c = torch.full((M, N), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    args = [C.c_void_p(t.data_ptr()) for t in (c, x, w, s)]
+    assert capi.load().tg_dev_qgemm(*args, M, K, N, None) == 0
+    torch.cuda.synchronize()
+    for n in range(0, N, 32768):
+        want = (x.double() @ w[:, n:n + 32768].double()) * s[n:n + 32768].double()
+        err = (c[:, n:n + 32768].double() - want).norm() / want.norm()
+        assert float(err) <= 2e-7, n
+
+
 def test_rows_of_any_range(capi):
     x, w, s = case(12, 1152, 640)
     x[1] *= 1e-30                    # tiny and huge rows beside ordinary ones: the exponent is per row

@@ -37,16 +37,12 @@
 #pragma once
 #include <cuda.h>
 
-#include "kernels_tc.cuh"  // tcgen05 / bulk-copy helpers
+#include "gemm_i8_tiles.h"  // plan, tile walk
+#include "kernels_tc.cuh"   // tcgen05 / bulk-copy helpers
 #include "tg_common.cuh"
 
 namespace tg {
 
-constexpr int I8_BK = 64;                      // k per block of the packed digits
-constexpr int I8_GROUP_BYTES = 4 * 8 * I8_BK;  // one (K-block, token group): 4 digits x 8 tokens x 64 k
-constexpr int I8_SK = 128;                     // k per stage
-constexpr int I8_TG = 8;                       // token groups of a tile, at most
-constexpr int I8_W_BYTES = 128 * I8_SK;
 constexpr int I8_THREADS = 320;                // producer, MMA issuer, 8 epilogue warps
 // CG CTAs work on a tile of CG * 128 columns: each holds its own 128 columns of W and 1 / CG of the digits
 template <int CG> struct I8Shape {
@@ -422,25 +418,17 @@ __global__ void __launch_bounds__(NT) geglu_i8_stream_kernel(const float *ug, ui
 }
 
 // ------------------------------------------------------------------ GEMM
-struct GemmI8Args {
+struct GemmI8Args : I8Walk {
 	const uint8_t *x;       // packed digits
 	const float *rowscale;  // [8 * groups]
-	int groups;             // token groups in the packed operand
-	int tg, tok_tiles;      // token groups per tile, token tiles
-	int n_fast;             // 1: consecutive tiles are the column tiles of one token tile; 0: the token tiles of one column tile
-	int tiles;              // col_tiles * tok_tiles * nsplit
-	// Up to three weight matrices with the same K share one launch (q|k|v, up|gate): matrix g owns the column tiles
-	// [tile_end[g-1], tile_end[g]) and columns col0[g].. of a partial-sum row (N = all columns)
-	int col_tiles;
-	unsigned m_tiles, m_fast, m_split;  // i8_magic of col_tiles * tok_tiles, of the faster tile index' range, of nsplit
-	int tile_end[3];
+	// matrix g of the walk has the columns col0[g].. of a partial-sum row (N = all columns)
 	int col0[3];
 	int ncols[3];            // N_g (a multiple of 128: the last tile of a pair may have only its first half)
 	const float *scales[3];  // [N_g]
 	float *C[3];             // [M] rows of ldc[g] floats (finished result)
 	int ldc[3];
 	float *partial;          // [nsplit][M][N] sums without the column scales (raw, or nsplit > 1)
-	int M, N, K, nsplit;
+	int M, N;
 	int raw;                 // 1: partial sums even unsplit; the consumer adds the splits and applies the column scales
 	int w_stream;            // 1: W is read by few CTAs: L2 evict-first
 	unsigned long long *top1;  // non-null (nsplit == 1): no C; per token the largest scaled value and its column, as a key
@@ -496,33 +484,6 @@ __device__ __forceinline__ void i8_pair_load(void *dst, const CUtensorMap *map, 
 }
 __device__ __forceinline__ void i8_cluster_sync() {
 	asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
-
-// tile index -> what it covers (every role of a CTA walks the same tiles)
-struct I8Tile {
-	int grp, n0;         // matrix, first column inside it
-	int g0, ng;          // token groups
-	int split, s0, ns;   // K-split, its first stage and number of stages
-};
-// x / d as a multiplication (m = ceil(2^32 / d), or 0 for d = 1): exact for x * d < 2^32. Every role of a CTA computes
-// its tiles between other things, and an integer division takes a single thread ~200 clk.
-inline unsigned i8_magic(unsigned d) { return d <= 1 ? 0u : unsigned((0x100000000ull + d - 1) / d); }
-__device__ __forceinline__ int i8_div(int x, unsigned m) { return m ? int(__umulhi(unsigned(x), m)) : x; }
-template <int CG> __device__ __forceinline__ I8Tile i8_tile(const GemmI8Args &a, int t) {
-	I8Tile r;
-	r.split = i8_div(t, a.m_tiles);
-	t -= r.split * a.col_tiles * a.tok_tiles;
-	const int hi = i8_div(t, a.m_fast), lo = t - hi * (a.n_fast ? a.col_tiles : a.tok_tiles);
-	const int ct = a.n_fast ? lo : hi, tt = a.n_fast ? hi : lo;
-	r.grp = (ct >= a.tile_end[0]) + (ct >= a.tile_end[1]);  // tile_end of unused slots = INT_MAX
-	// (selects over constant indices: a run-time index into the parameter arrays would move them to local memory)
-	r.n0 = (ct - (r.grp == 0 ? 0 : (r.grp == 1 ? a.tile_end[0] : a.tile_end[1]))) * (128 * CG);
-	r.g0 = tt * a.tg;
-	r.ng = min(a.tg, a.groups - r.g0);
-	const int all = a.K / I8_SK;
-	r.s0 = i8_div(r.split * all, a.m_split);
-	r.ns = i8_div((r.split + 1) * all, a.m_split) - r.s0;
-	return r;
 }
 
 // xmap (CG = 2): the digits as rows of 512 bytes (one (group, digit) of a K-block), box of 2 * tg rows
@@ -673,7 +634,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		// ------------------------------------------------------------ epilogue (warps 2..9)
 		pdl_wait();  // the row scales are the predecessor's output, and C may be its input
 		const int quad = warp & 3, sub = (warp - 2) >> 2;  // TMEM lanes 32 * quad ..; two warps share them
-		const bool fin = a.nsplit == 1 && !a.raw;
+		const bool fin = a.nsplit.d == 1 && !a.raw;
 		int it = 0;
 		for (int ti = first; ti < a.tiles; ti += stride, it++) {
 			const I8Tile t = i8_tile<CG>(a, ti);

@@ -1569,51 +1569,8 @@ int ensure_log(tg_state *s, int steps) {
 
 
 // ------------------------------------------------------------- tensor-core GEMM
-int i8_groups(int M) { return (M + 7) / 8; }
 size_t i8_pack_bytes(int M, int K) { return size_t(i8_groups(M)) * 8 * (size_t(4) * K + 4); }
 float *i8_rowscale(const TcScratch &sc, int M, int K) { return reinterpret_cast<float *>(sc.x + size_t(i8_groups(M)) * 8 * 4 * K); }
-
-// Tokens per tile, K-split and CTAs per tile of one GEMM launch, by an estimate in clocks of an SM: rounds of tiles per
-// CTA (or pair) x (stages x the slowest of MMAs, operand bytes and the issuing threads + what a tile change costs) + what
-// the consumer of the partial sums reads. The constants rank 2278 measured (shape, tile, split) combinations at 1 to 4001
-// rows of all layer shapes: the choice is within 1 % of the best one on average. An MMA of N columns takes max(N / 2, 64) clk
-// (a single CTA's are slowed to 1.28 of that by its operands' arrival), 78 B/clk arrive per SM with all SMs loading.
-struct I8Plan {
-	int cg, tg, tok_tiles, col_tiles, nsplit;
-};
-I8Plan i8_plan(int M, int K, int ng, const QW *const *ws, size_t partial_floats, int max_split, bool raw) {
-	I8Plan best{1, 1, 1, 1, 1};
-	double best_cost = 1e30;
-	const int groups = i8_groups(M), stages = K / I8_SK;
-	int ntot = 0;
-	for (int g = 0; g < ng; g++) ntot += ws[g]->N;
-	static const int want_cg = env_int("TG_GEMM_PAIR", 0);      // (experiments: 1 or 2 CTAs per tile; a K-split)
-	static const int want_split = env_int("TG_GEMM_SPLIT", 0);
-	for (int cg = 1; cg <= 2; cg++) {
-		if (want_cg && cg != want_cg) continue;
-		int col_tiles = 0;
-		for (int g = 0; g < ng; g++) col_tiles += (ws[g]->N + 128 * cg - 1) / (128 * cg);
-		const int workers = g_num_sms / cg;
-		for (int tg = std::min(groups, I8_TG); tg >= std::max(1, std::min(groups, I8_TG) - 3); tg--) {
-			const int tok_tiles = (groups + tg - 1) / tg;
-			const double mma = 4.0 * std::max(16.0 * tg, 64.0) * (cg == 1 ? 1.28 : 1.0), in = I8_W_BYTES + 2.0 * tg * I8_GROUP_BYTES / cg;
-			const double per_stage = std::max(std::max(mma, in / 78.0), 256.0);
-			for (int ns = 1; ns <= std::min(max_split, stages); ns++) {
-				if (want_split && ns != std::min(want_split, std::min(max_split, stages))) continue;
-				if ((ns > 1 || raw) && size_t(ns) * M * ntot > partial_floats) break;
-				const long tiles = long(tok_tiles) * col_tiles * ns, rounds = (tiles + workers - 1) / workers;
-				double cost = double(rounds) * ((stages + ns - 1) / ns * per_stage + 2500.0) + tg * 100.0 + (cg - 1) * 4000.0;
-				cost += double(raw ? ns - 1 : (ns > 1 ? ns + 1 : 0)) * M * ntot * 4.0 / 2500.0;  // partial sums read again, 2.5 KB a clock
-				cost += raw ? (ns + 7) / 8 * 600.0 : (ns > 1 ? 4000.0 : 0.0);  // its dependent round trips; a launch more
-				if (cost < best_cost) {
-					best_cost = cost;
-					best = I8Plan{cg, tg, tok_tiles, col_tiles, ns};
-				}
-			}
-		}
-	}
-	return best;
-}
 
 // packed operands of the tensor-core prefill attention for one prompt of S tokens: Q (4 S rows), K (S rows), V
 struct AttnTcPlan {
@@ -1743,17 +1700,21 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		configured[dev] = true;
 	}
 	const int K = ws[0]->K;
-	int ntot = 0;
+	int ntot = 0, cols[3] = {0, 0, 0};
 	for (int g = 0; g < ng; g++) {
 		if (ws[g]->K != K) return fail(TG_ESHAPE, "grouped GEMM: the matrices must share K");
-		ntot += ws[g]->N;
+		cols[g] = ws[g]->N;
+		ntot += cols[g];
 	}
-	I8Plan pl = i8_plan(plan_rows ? plan_rows : M, K, ng, ws, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr);
+	static const int want_cg = env_int("TG_GEMM_PAIR", 0);  // (experiments: 1 or 2 CTAs per tile; a K-split)
+	static const int want_split = env_int("TG_GEMM_SPLIT", 0);
+	I8Plan pl = i8_plan(plan_rows ? plan_rows : M, K, ng, cols, g_num_sms, sc.partial_floats, sc.top1 ? 1 : max_split, raw_nsplit != nullptr, want_cg, want_split);
 	if (plan_rows) pl.tok_tiles = (i8_groups(M) + pl.tg - 1) / pl.tg;
 	CUtensorMap wmap[3];
 	GemmI8Args a{};
+	i8_fill_walk(a, pl, M, K, ng, cols);
 	ReduceGroups rg{};
-	int col0 = 0, tiles = 0;
+	int col0 = 0;
 	for (int g = 0; g < 3; g++) {
 		const int gg = std::min(g, ng - 1);  // unused slots repeat the last matrix (never selected)
 		if (ws[gg]->map)
@@ -1766,11 +1727,8 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 			a.col0[g] = col0;
 			a.ncols[g] = ws[g]->N;
 			col0 += ws[g]->N;
-			tiles += (ws[g]->N + 128 * pl.cg - 1) / (128 * pl.cg);
-			a.tile_end[g] = tiles;
 		} else {
 			a.col0[g] = col0;
-			a.tile_end[g] = INT_MAX;
 		}
 		a.scales[g] = ws[gg]->s;
 		a.C[g] = Cs ? Cs[gg] : nullptr;
@@ -1784,29 +1742,17 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	rg.col0[3] = INT_MAX;
 	a.x = sc.x;
 	a.rowscale = i8_rowscale(sc, M, K);
-	a.groups = i8_groups(M);
-	a.tg = pl.tg;
-	a.tok_tiles = pl.tok_tiles;
-	a.col_tiles = pl.col_tiles;
-	a.tiles = pl.tok_tiles * pl.col_tiles * pl.nsplit;
-	// matrices that stay in the L2 are swept once per token tile; the vocabulary matrix is read once for all token tiles
-	a.n_fast = size_t(ntot) * K <= (size_t(48) << 20);
-	a.m_tiles = i8_magic(unsigned(pl.col_tiles) * pl.tok_tiles);
-	a.m_fast = i8_magic(a.n_fast ? pl.col_tiles : pl.tok_tiles);
-	a.m_split = i8_magic(pl.nsplit);
 	a.w_stream = pl.tok_tiles <= 4;
 	a.M = M;
 	a.N = ntot;
-	a.K = K;
-	a.nsplit = pl.nsplit;
 	a.partial = sc.partial;
 	a.raw = raw_nsplit ? 1 : 0;
 	a.err = sc.err;
 	a.top1 = sc.top1;
 	a.top1_col0 = sc.top1_col0;
 	if (raw_nsplit) {
-		if (size_t(a.nsplit) * M * ntot > sc.partial_floats) return fail(TG_ENOMEM, "tensor-core GEMM partial-sum scratch too small");
-		*raw_nsplit = a.nsplit;
+		if (size_t(pl.nsplit) * M * ntot > sc.partial_floats) return fail(TG_ENOMEM, "tensor-core GEMM partial-sum scratch too small");
+		*raw_nsplit = pl.nsplit;
 	}
 	if (pl.cg == 2) {
 		CUtensorMap xmap;
@@ -1817,9 +1763,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
-	if (a.nsplit > 1 && !raw_nsplit) {
+	if (pl.nsplit > 1 && !raw_nsplit) {
 		const size_t n = size_t(M) * ntot;
-		launch_k(qgemm_splitk_reduce_groups_kernel, dim3(unsigned((n + 255) / 256)), dim3(256), 0, st, rg, (const float *)sc.partial, M, ntot, a.nsplit);
+		launch_k(qgemm_splitk_reduce_groups_kernel, dim3(unsigned((n + 255) / 256)), dim3(256), 0, st, rg, (const float *)sc.partial, M, ntot, pl.nsplit);
 		count_launch();
 		TG_TRY(check_launch("qgemm_reduce"));
 	}
