@@ -249,7 +249,10 @@ def test_sliding_window_ring_270m(capi, model_270m, ref_or_none, golden, weights
     assert rel_l2(cases.subsample(logits[0]), g["sw_last_logits"]) <= tol
     # after 8 decode steps slots 0..7 of a local layer hold the new tokens, 8.. the prompt tail
     k, _ = st.kv_read(0, 0, 10)
-    assert rel_max(k, g["sw_l0_k_first10"]) <= 1e-5
+    # With tables of another build than the golden's (libraries evaluate powf differently) a frequency f <= 1 may differ by an
+    # ulp of 1 / f, 2^-23 relative, and an angle of up to 607 by that and by its own two roundings (ulp 2^-14): at most
+    # 607 * 2^-23 + 2^-14 = 1.34e-4 rad, which moves a component by that times the pair's length, <= sqrt(2) max |k|.
+    assert rel_max(k, g["sw_l0_k_first10"]) <= (1e-5 if exact_tables else 2e-4)
     assert st.position() == int(g["sw_kv_info_l0"][0]) == 608
     st.close()
 
