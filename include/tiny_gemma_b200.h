@@ -171,7 +171,9 @@ int tg_hidden_read(tg_state *s, float *hidden_host);
  * K,N must be in the reference's supported set, else TG_ESHAPE. */
 int tg_qmatvec(float *y_host, const float *x_host, const int8_t *w_host, const float *scales_host, int K, int N);
 /* ops::linear_prefill, ops.hpp:618-632 -> gemm::launch_qgemm, linalg.hpp:298-308:
- * C[M,N] = scale[n] * (A[M,K] . W[K,N]) */
+ * C[M,N] = scale[n] * (A[M,K] . W[K,N]). A row of A is multiplied as 31-bit fixed point relative to its
+ * largest element; rows whose elements range too far for that (more than an eighth of them below 2^-12 of
+ * the largest) are recomputed from the fp32 values with sums in fp64, which takes longer. */
 int tg_qgemm(float *c_host, const float *a_host, const int8_t *w_host, const float *scales_host, int M, int K, int N);
 /* ops::argmax_logits / ops::minp_logits on a host logits buffer of n entries
  * (n = 262144 in the reference); minp mutates logits_host like the reference */
@@ -203,8 +205,9 @@ int tg_dev_qmatvec(float *y_dev, const float *x_dev, const int8_t *w_dev, const 
 int tg_dev_qmatvec_static(float *y_dev, const float *x_dev, const int8_t *w_dev, const float *scales_dev, int K, int N,
                           void *cuda_stream);
 /* tg_dev_qgemm synchronises the stream before it returns (it reads the kernel's error word), except
- * while the stream is being captured into a CUDA graph: then it only records its launches, and an
- * error raised by a replay is reported by the next call made outside a capture. */
+ * while the stream is being captured into a CUDA graph: then it only records its launches (one more than
+ * otherwise: every replay looks for rows of wide range itself), and an error raised by a replay is
+ * reported by the next call made outside a capture. */
 int tg_dev_qgemm(float *c_dev, const float *a_dev, const int8_t *w_dev, const float *scales_dev, int M, int K, int N,
                  void *cuda_stream);
 

@@ -72,3 +72,56 @@ def test_rows_of_any_range(capi):
         assert rel_l2(c[r], want[r]) <= 2e-7, r
     assert not c[3].any()
     assert np.isnan(c[7]).all() and not np.isfinite(c[8]).any()
+
+
+@pytest.mark.parametrize("K,N", [(256, 640), (1152, 256), (2048, 256), (6912, 1152)])
+@pytest.mark.parametrize("M", [1, 9, 130])
+def test_columns_that_do_not_see_the_large_elements(capi, K, N, M):
+    """every third row holds a few elements far above the rest, which half of the columns give the weight 0: these columns
+    are sums of the others alone, and keep fp32's precision however large the few are (the exponent of a row's digits is the
+    largest element's). Bound per row: 24-bit inputs and one rounding, 2^-24 each; rows of ordinary range 2e-7 as above."""
+    x, w, s = case(M, K, N)
+    big = [0, K // 2, K - 1]
+    for i, r in enumerate(range(0, M, 3)):
+        x[r, big] = np.float32(10.0) ** (4 + 2 * (i % 8)) * np.float32([1.0, -0.7, 0.3])
+    w[big, ::2] = 0
+    c = capi.qgemm(x, w, s)
+    want = exact(x, w, s)
+    for r in range(M):
+        assert rel_l2(c[r, ::2], want[r, ::2]) <= 2e-7, r
+        assert rel_l2(c[r, 1::2], want[r, 1::2]) <= 2e-7, r
+    x *= np.float32(2.0 ** -112)  # rows near the end of fp32's range
+    s *= np.float32(2.0 ** 100)
+    c, want = capi.qgemm(x, w, s), exact(x, w, s)
+    for r in range(M):
+        assert rel_l2(c[r], want[r]) <= 2e-7, r
+
+
+def test_wide_rows_in_a_captured_graph(capi):
+    """a replay looks at the rows that it finds: ordinary ones when the graph is captured, wide ones when it is replayed"""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    M, K, N = 40, 1152, 640
+    x, w, s = case(M, K, N)
+    xd, wd, sd = (torch.from_numpy(t).cuda() for t in (x, w, s))
+    c = torch.empty(M, N, device="cuda")
+    stream = torch.cuda.Stream()
+    args = [C.c_void_p(t.data_ptr()) for t in (c, xd, wd, sd)] + [M, K, N, C.c_void_p(stream.cuda_stream)]
+    lib = capi.load()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        assert lib.tg_dev_qgemm(*args) == 0  # (the scratch is there before the capture)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            assert lib.tg_dev_qgemm(*args) == 0
+    x[5, 7] = 1e9
+    w[7, :] = 0
+    xd.copy_(torch.from_numpy(x))
+    wd.copy_(torch.from_numpy(w))
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    got, want = c.cpu().numpy(), exact(x, w, s)
+    for r in range(M):
+        assert rel_l2(got[r], want[r]) <= 2e-7, r

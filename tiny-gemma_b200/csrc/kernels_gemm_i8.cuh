@@ -4,7 +4,8 @@
 //
 // Arithmetic: a row of A is written as x = 2^(e-30) * (d3 * 2^24 + d2 * 2^16 + d1 * 2^8 + d0), one exponent e per
 // row (2^e > the row's largest |x|), four signed 8-bit digits. An element within a factor 2^7 of the row's largest
-// keeps all 24 bits of its fp32 mantissa; below that the representation is still exact to 2^-31 of the largest. The
+// keeps all 24 bits of its fp32 mantissa; below that the representation is still exact to 2^-31 of the largest (the operators
+// recompute rows for which that is not enough, see i8_wide). The
 // weights go to the tensor cores as they lie in memory, the digit products are summed EXACTLY in int32 (at most
 // 6912 * 128 * 128 < 2^31), and only the epilogue rounds: it joins the four sums in fp32. Against three bf16 terms with fp32 accumulation
 // (6 bytes per activation, weights converted on the SM, truncating adds): 4 products at twice the bf16 rate instead of
@@ -98,9 +99,32 @@ template <int NW> __device__ __forceinline__ uint32_t block_umax(uint32_t v, uin
 // (The rows that pad M to whole groups of 8 are never written: a token's sums involve no other token, and the sums of
 // rows >= M are not stored.)
 
+// Rows that the digits do not hold well enough. An element below 2^-7 of its row's largest loses mantissa bits, and a column
+// whose weights on the large elements are zero sees that loss undiluted. Rows in which more than an eighth of the nonzero elements
+// (of some warp's part of the row) lie below 2^-12 of the largest (such an element is kept to 2^-19 of itself), and rows below 2^-96
+// altogether, are marked by the operators' packing and recomputed by qgemm_wide_rows_kernel. A normal row with one element of s sigmas is marked from s ~ 400
+// on; just below, a column that does not see that element is off by 2e-7. (A model's own passes do not: their rows come out of a norm or
+// a GeGLU, and its decode steps hold them to 2^-24 of the largest in any case.)
+// (called by whole warps; the zeros are told apart only where many elements are small)
+template <int PER> __device__ __forceinline__ bool i8_wide(const float4 (&v)[PER], uint32_t maxbits) {
+	const float below = __uint_as_float(uint32_t(max(int(maxbits >> 23) - 11, 0)) << 23);
+	int small = 0, zero = 0;
+#pragma unroll
+	for (int j = 0; j < PER; j++) small += (fabsf(v[j].x) < below) + (fabsf(v[j].y) < below) + (fabsf(v[j].z) < below) + (fabsf(v[j].w) < below);
+	small = __reduce_add_sync(0xffffffffu, small);
+	if (8 * small > 128 * PER) {
+#pragma unroll
+		for (int j = 0; j < PER; j++) zero += (v[j].x == 0.0f) + (v[j].y == 0.0f) + (v[j].z == 0.0f) + (v[j].w == 0.0f);
+		zero = __reduce_add_sync(0xffffffffu, zero);
+	}
+	const bool tiny = maxbits != 0u && int(maxbits >> 23) - 126 < -96;
+	return maxbits < 0x7F800000u && (tiny || 8 * (small - zero) > 128 * PER - zero);
+}
+
 // fp32 rows -> digits. One CTA of NT threads per row, the row in registers: K <= NT * 4 * PER.
-template <int NT, int PER>
-__global__ void __launch_bounds__(NT) i8_pack_kernel(const float *A, uint8_t *out, float *rowscale, int K, int groups) {
+// WIDE: wide[row] = 1 for a row that the digits do not hold, and *any (host memory) is set.
+template <int NT, int PER, bool WIDE>
+__global__ void __launch_bounds__(NT) i8_pack_kernel(const float *A, uint8_t *out, float *rowscale, int K, int groups, int *wide, int *any) {
 	pdl_trigger();
 	pdl_wait();
 	__shared__ uint32_t red[NT / 32];
@@ -120,6 +144,86 @@ __global__ void __launch_bounds__(NT) i8_pack_kernel(const float *A, uint8_t *ou
 #pragma unroll
 	for (int j = 0; j < PER; j++)
 		if (4 * (tid + NT * j) < K) i8_pack4(out, groups, row, tid + NT * j, v[j], mul);
+	if (WIDE) {
+		const int w = __syncthreads_or(i8_wide(v, mx));
+		if (tid == 0) {
+			wide[row] = w;
+			if (w) *static_cast<volatile int *>(any) = 1;
+		}
+	}
+}
+
+// The marked rows of C = A . W * scales, from the fp32 rows, with products and sums in fp64 (both exact or as good as that):
+// 128 columns per CTA, eight warps with every eighth group of four k each (a warp reads 128 contiguous bytes of W per k), eight
+// rows at a time, the warps' sums added in order. An ordinary call never launches it (the marking itself: 142.9 -> 144.3 us for
+// 4001 rows of 6912 x 1152). Up to eight marked rows add 0.17 ms there, one CTA's chain of loads; 4001 marked rows 5.9 ms, bound by
+// the fp64 pipe and the conversions (one k-group of loads in flight: 12.8 ms; four rows at a time: 14.4).
+__device__ __forceinline__ double i8_to_double(uint32_t word, int byte) {  // exact: 2^52 + (b + 128) in the mantissa
+	return __hiloint2double(0x43300000, int(__byte_perm(word ^ 0x80808080u, 0u, 0x4440u + byte))) - 4503599627370624.0;
+}
+__global__ void __launch_bounds__(256) qgemm_wide_rows_kernel(float *C, const float *A, const int8_t *W, const float *scales, const int *wide, int M, int K, int N) {
+	constexpr int R = 8, H = 4;  // rows at a time, rows whose sums meet at a time
+	__shared__ int list[256], count[8];
+	__shared__ double part[8][H][128];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n0 = blockIdx.x * 128;
+	const int chunk = (M + gridDim.y - 1) / gridDim.y, r0 = blockIdx.y * chunk, r1 = min(M, r0 + chunk);
+	for (int base = r0; base < r1; base += 256) {
+		__syncthreads();
+		const bool mine = base + tid < r1 && wide[base + tid] != 0;
+		const unsigned m = __ballot_sync(0xffffffffu, mine);
+		if (lane == 0) count[warp] = __popc(m);
+		__syncthreads();
+		int n = 0, at = __popc(m & ((1u << lane) - 1u));
+		for (int w = 0; w < 8; w++) {
+			if (w < warp) at += count[w];
+			n += count[w];
+		}
+		if (mine) list[at] = base + tid;
+		__syncthreads();
+		for (int first = 0; first < n; first += R) {
+			const float *row[R];
+#pragma unroll
+			for (int i = 0; i < R; i++) row[i] = A + size_t(list[min(first + i, n - 1)]) * K;
+			double acc[R][4] = {};
+#pragma unroll 2
+			for (int k = 4 * warp; k < K; k += 32) {
+				uint32_t w[4];
+#pragma unroll
+				for (int q = 0; q < 4; q++) w[q] = *reinterpret_cast<const uint32_t *>(W + size_t(k + q) * N + n0 + 4 * lane);
+				float4 x[R];
+#pragma unroll
+				for (int i = 0; i < R; i++) x[i] = *reinterpret_cast<const float4 *>(row[i] + k);
+#pragma unroll
+				for (int q = 0; q < 4; q++) {
+					const double w0 = i8_to_double(w[q], 0), w1 = i8_to_double(w[q], 1), w2 = i8_to_double(w[q], 2), w3 = i8_to_double(w[q], 3);
+#pragma unroll
+					for (int i = 0; i < R; i++) {
+						const double xi = q == 0 ? x[i].x : (q == 1 ? x[i].y : (q == 2 ? x[i].z : x[i].w));
+						acc[i][0] = fma(xi, w0, acc[i][0]);
+						acc[i][1] = fma(xi, w1, acc[i][1]);
+						acc[i][2] = fma(xi, w2, acc[i][2]);
+						acc[i][3] = fma(xi, w3, acc[i][3]);
+					}
+				}
+			}
+#pragma unroll
+			for (int h = 0; h < R; h += H) {
+				__syncthreads();  // (the sums before have been read)
+#pragma unroll
+				for (int i = 0; i < H; i++)
+#pragma unroll
+					for (int c = 0; c < 4; c++) part[warp][i][4 * lane + c] = acc[h + i][c];
+				__syncthreads();
+				for (int q = tid; q < min(H, n - first - h) * 128; q += 256) {
+					const int i = q >> 7, c = q & 127;
+					double s = 0.0;
+#pragma unroll
+					for (int w = 0; w < 8; w++) s += part[w][i][c];
+					C[size_t(list[first + h + i]) * N + n0 + c] = float(s * double(scales[n0 + c]));
+				}
+			}
+		}
+	}
 }
 
 // Residual + sandwich norms of one row, fused with the operand packing of the next GEMM:

@@ -1589,16 +1589,23 @@ AttnTcPlan attn_tc_plan(int S) {
 	return p;
 }
 
-int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStream_t st) {
-	if (i8_pack_bytes(M, K) > sc.x_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
+// wide, any: where the packing marks rows that the digits do not hold (see i8_pack_kernel), or null
+template <bool WIDE> void launch_i8_pack(const float *A, int M, int K, const TcScratch &sc, int *wide, int *any, cudaStream_t st) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, K);
 	if (K <= 1152)
-		launch_k(i8_pack_kernel<96, 3>, dim3(M), dim3(96), 0, st, A, sc.x, rs, K, groups);
+		launch_k(i8_pack_kernel<96, 3, WIDE>, dim3(M), dim3(96), 0, st, A, sc.x, rs, K, groups, wide, any);
 	else if (K <= 2048)
-		launch_k(i8_pack_kernel<256, 2>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups);
+		launch_k(i8_pack_kernel<256, 2, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
 	else
-		launch_k(i8_pack_kernel<256, 7>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups);
+		launch_k(i8_pack_kernel<256, 7, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
+}
+int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStream_t st, int *wide = nullptr, int *any = nullptr) {
+	if (i8_pack_bytes(M, K) > sc.x_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
+	if (wide)
+		launch_i8_pack<true>(A, M, K, sc, wide, any, st);
+	else
+		launch_i8_pack<false>(A, M, K, sc, nullptr, nullptr, st);
 	count_launch();
 	return check_launch("i8_pack");
 }
@@ -3109,9 +3116,9 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 	TG_CUDA(cudaGetDevice(&dev));
 	QW q{w, scales, K, N};
 	if (env_int("TG_GEMM_TC", 1)) {
-		// tensor-core path: packed bf16 activations + an error word, per device, grown on demand
+		// tensor-core path: packed digits, a mark per row and the error word, per device, grown on demand
 		static TcScratch tc[64];
-		const size_t need = i8_pack_bytes(M, K);
+		const size_t need = i8_pack_bytes(M, K) + size_t(M) * 4;
 		if (need > tc[dev].x_bytes) {
 			if (tc[dev].x) cudaFree(tc[dev].x);
 			tc[dev].x = nullptr;
@@ -3127,23 +3134,36 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 			TG_CUDA(cudaMalloc(&tc[dev].partial, pneed * 4));
 			tc[dev].partial_floats = pneed;
 		}
-		static int *err_host[64] = {nullptr};  // the error word, in host memory that the device writes
+		static int *host_words[64] = {nullptr};  // error word, "a row is marked": in host memory that the device writes
 		if (!tc[dev].err) {
-			TG_CUDA(cudaHostAlloc(&err_host[dev], 4, cudaHostAllocMapped | cudaHostAllocPortable));
-			*err_host[dev] = 0;
-			TG_CUDA(cudaHostGetDevicePointer(&tc[dev].err, err_host[dev], 0));
+			TG_CUDA(cudaHostAlloc(&host_words[dev], 8, cudaHostAllocMapped | cudaHostAllocPortable));
+			host_words[dev][0] = host_words[dev][1] = 0;
+			TG_CUDA(cudaHostGetDevicePointer(&tc[dev].err, host_words[dev], 0));
 		}
-		TG_TRY(pack_activations(a, M, K, tc[dev], (cudaStream_t)stream));
-		TG_TRY(launch_gemm_tc(c, q, M, tc[dev], (cudaStream_t)stream));
+		const cudaStream_t st = (cudaStream_t)stream;
+		int *wide = reinterpret_cast<int *>(tc[dev].x + i8_pack_bytes(M, K));
+		auto recompute = [&]() -> int {  // rows that the digits do not hold
+			qgemm_wide_rows_kernel<<<dim3(N / 128, std::min((M + 31) / 32, 64)), 256, 0, st>>>(c, a, w, scales, wide, M, K, N);
+			count_launch();
+			return check_launch("qgemm_wide_rows");
+		};
+		TG_TRY(pack_activations(a, M, K, tc[dev], st, wide, tc[dev].err + 1));
+		TG_TRY(launch_gemm_tc(c, q, M, tc[dev], st));
 		// while the stream is being captured into a graph nothing may synchronise: the error word stays
-		// set on the device and the next call outside a capture reports it
+		// set on the device and the next call outside a capture reports it; marked rows are looked for in every replay
 		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-		TG_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
-		if (cap != cudaStreamCaptureStatusNone) return TG_OK;
-		TG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-		if (*static_cast<volatile int *>(err_host[dev])) {
-			*err_host[dev] = 0;
+		TG_CUDA(cudaStreamIsCapturing(st, &cap));
+		if (cap != cudaStreamCaptureStatusNone) return recompute();
+		TG_CUDA(cudaStreamSynchronize(st));
+		volatile int *words = host_words[dev];
+		if (words[0]) {
+			words[0] = 0;
 			return fail(TG_ECUDA, "tensor-core GEMM: a pipeline wait ran out");
+		}
+		if (words[1]) {
+			words[1] = 0;
+			TG_TRY(recompute());
+			TG_CUDA(cudaStreamSynchronize(st));
 		}
 		return TG_OK;
 	}
