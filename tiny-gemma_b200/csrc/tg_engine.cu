@@ -1992,12 +1992,17 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		tc.err = s->err_flag;
 		p += (tc.x_bytes + 3) / 4;
 	}
-	// Attention on the tensor cores, from packed copies of q, k and v: for more than 960 tokens, of one prompt or of a group
-	// of equal prompts. Below, the CUDA-core kernel with two queries per CTA is faster, since its CTAs are more (prefill of
-	// 450 tokens 2.9 against 3.6 ms, 832 tokens 4.93 against 5.04, 16 prompts of 61 tokens 3.98 against 4.29; 8 of 178 tokens
-	// 5.71 against 5.67, 256 of 178 tokens 170 against 150).
+	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 960 tokens, and for a group of
+	// equal prompts of 16 and more tokens each that has more than 960 + 16384 / S of them in all. Otherwise the CUDA-core kernel
+	// with two queries per CTA is faster: its CTAs are more, and a prompt fills no tiles of 32 queries and 64 keys, as which the
+	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill of the 1B model in ms: one prompt of
+	// 450 tokens 2.9 / 3.6, of 832 4.93 / 5.04; groups of 976 rows of 8 tokens 3.77 / 4.20, of 61 3.81 / 3.97 (1464: 5.27 / 5.31), of 178
+	// 890 rows 3.90 / 4.09, 1424 5.51 / 5.24; of 16 tokens 976 rows 3.66 / 3.99, 2192 7.61 / 7.03 to 7.70, 16384 51.9 / 52.0; of 8 tokens
+	// 8192 rows 27.0 / 28.8, of 2 tokens 1500 rows 5.7 / 9.0; of 178 tokens 16376 rows 57.2 / 49.8. 270m: of 30 tokens 2190 rows 2.36 /
+	// 2.40, 4080 3.82 / 3.53; of 61 tokens 1464 rows 1.79 / 1.83, 2196 2.48 / 2.35; of 8 tokens 8192 rows 7.7 / 9.5.
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
-	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && (plan_rows ? S_seq : nb * S_seq) > env_int("TG_ATTN_SMALL_MAX", 960) && S_seq >= env_int("TG_ATTN_TC_MIN", 0);
+	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", 960) + (at_rows > S_seq ? 16384 / S_seq : 0);
+	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
