@@ -73,9 +73,12 @@ constexpr int TG_MAX_DEVICES = 64;
 // Launch with the programmatic-serialization attribute (see pdl_wait in tg_common.cuh): only for kernels that
 // call pdl_wait() before their first global access. TG_PDL=0 launches them as ordinary stream-ordered kernels.
 // Captured into the batched step's CUDA graph the edges stay programmatic: 1.28 -> 1.08 ms at 4 sequences, 2.86 -> 2.63 at 256.
-template <typename... KArgs, typename... Args>
-inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+bool use_pdl() {
 	static const int use = env_int("TG_PDL", 1);
+	return use != 0;
+}
+template <bool PDL, typename... KArgs, typename... Args>
+inline void launch_as(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
@@ -85,8 +88,12 @@ inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
 	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at;
-	cfg.numAttrs = use ? 1 : 0;
+	cfg.numAttrs = PDL && use_pdl() ? 1 : 0;
 	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
+}
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+	launch_as<true>(kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 inline int current_device_slot() {
@@ -302,7 +309,7 @@ int mvc_launch_t(float *y, const float *x, const int8_t *w, const float *scales,
 	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = max_clusters ? 1 : 2;
+	cfg.numAttrs = max_clusters || !use_pdl() ? 1 : 2;
 	if (max_clusters) {  // query only
 		TG_CUDA(cudaOccupancyMaxActiveClusters(max_clusters, qmatvec_cluster_kernel<TPR, NT>, &cfg));
 		return TG_OK;
@@ -1589,16 +1596,18 @@ AttnTcPlan attn_tc_plan(int S) {
 	return p;
 }
 
-// wide, any: where the packing marks rows that the digits do not hold (see i8_pack_kernel), or null
+// wide, any: where the operators' packing marks rows that the digits do not hold (see i8_pack_kernel), or null. The operators'
+// packing is an ordinary launch: the GEMM behind it requests its first weight tiles before it waits for its predecessor, and
+// there the weights are the caller's, whose own kernel may have been writing them just before. (A model's are not written by kernels.)
 template <bool WIDE> void launch_i8_pack(const float *A, int M, int K, const TcScratch &sc, int *wide, int *any, cudaStream_t st) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, K);
 	if (K <= 1152)
-		launch_k(i8_pack_kernel<96, 3, WIDE>, dim3(M), dim3(96), 0, st, A, sc.x, rs, K, groups, wide, any);
+		launch_as<!WIDE>(i8_pack_kernel<96, 3, WIDE>, dim3(M), dim3(96), 0, st, A, sc.x, rs, K, groups, wide, any);
 	else if (K <= 2048)
-		launch_k(i8_pack_kernel<256, 2, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
+		launch_as<!WIDE>(i8_pack_kernel<256, 2, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
 	else
-		launch_k(i8_pack_kernel<256, 7, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
+		launch_as<!WIDE>(i8_pack_kernel<256, 7, WIDE>, dim3(M), dim3(256), 0, st, A, sc.x, rs, K, groups, wide, any);
 }
 int pack_activations(const float *A, int M, int K, const TcScratch &sc, cudaStream_t st, int *wide = nullptr, int *any = nullptr) {
 	if (i8_pack_bytes(M, K) > sc.x_bytes) return fail(TG_ENOMEM, "tensor-core GEMM scratch too small");
@@ -1672,7 +1681,6 @@ int make_digit_map(CUtensorMap *out, const uint8_t *x, int K, int groups, int tg
 // launch_k in clusters of two CTAs
 template <typename... KArgs, typename... Args>
 inline void launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
-	static const int pdl = env_int("TG_PDL", 1);
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
@@ -1685,7 +1693,7 @@ inline void launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
 	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = at;
-	cfg.numAttrs = pdl ? 2 : 1;
+	cfg.numAttrs = use_pdl() ? 2 : 1;
 	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
 }
 
