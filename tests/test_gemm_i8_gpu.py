@@ -125,3 +125,34 @@ def test_wide_rows_in_a_captured_graph(capi):
     got, want = c.cpu().numpy(), exact(x, w, s)
     for r in range(M):
         assert rel_l2(got[r], want[r]) <= 2e-7, r
+
+
+@pytest.mark.parametrize("K,N", [(640, 1024), (2048, 1152), (1152, 6912)])
+def test_captured_matvec_keeps_its_bits(capi, K, N):
+    """small matrices are launched without the programmatic edge inside a graph, larger ones with it; each node follows
+    the kernel that writes its input"""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    x, w, s = case(8, K, N)
+    xd, wd, sd = (torch.from_numpy(t).cuda() for t in (x, w, s))
+    y, xi = torch.empty(8, N, device="cuda"), torch.empty(K, device="cuda")
+    lib, stream = capi.load(), torch.cuda.Stream()
+
+    def call(i):
+        xi.copy_(xd[i])
+        assert lib.tg_dev_qmatvec(*[C.c_void_p(t.data_ptr()) for t in (y[i], xi, wd, sd)], K, N, C.c_void_p(stream.cuda_stream)) == 0
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call(0)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for i in range(8):
+                call(i)
+    y.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    for i in range(8):
+        assert np.array_equal(y[i].cpu().numpy(), capi.qmatvec(x[i], w, s)), i

@@ -309,7 +309,16 @@ int mvc_launch_t(float *y, const float *x, const int8_t *w, const float *scales,
 	attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[1].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = max_clusters || !use_pdl() ? 1 : 2;
+	// Launched into a stream, the programmatic edge hides the launch (640 x 1024: 6.1 -> 5.3 us a call). Between the nodes of a
+	// graph the launch is hidden anyway, and the edge delays a small kernel: 640 x 1024 3.57 -> 4.97 us, 1152 x 1024 3.99 -> 5.55,
+	// 2048 x 640 4.25 -> 5.65, but 1152 x 6912 6.68 -> 6.20 and 6912 x 1152 6.88 -> 6.15.
+	bool pdl = !max_clusters && use_pdl();
+	if (pdl && size_t(K) * N <= (size_t(4) << 20)) {
+		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+		if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();  // (the launch itself reports what is wrong)
+		pdl = cap == cudaStreamCaptureStatusNone;
+	}
+	cfg.numAttrs = pdl ? 2 : 1;
 	if (max_clusters) {  // query only
 		TG_CUDA(cudaOccupancyMaxActiveClusters(max_clusters, qmatvec_cluster_kernel<TPR, NT>, &cfg));
 		return TG_OK;
