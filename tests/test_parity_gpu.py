@@ -264,7 +264,7 @@ def _seq_cross(p, randf, cum0=0.0):
 
 
 def test_inverse_cdf_is_the_sequential_fp32_chain(capi):
-    """The parallel scan must give the crossing index AND the running sum of the sequential fp32 chain, bit for
+    """The samplers' walk (minp_scale_kernel, minp_walk_kernel) must give the crossing index AND the running sum of the sequential fp32 chain, bit for
     bit: random vectors, vectors quantised so that exact ties (round-half-even) are common, wide dynamic range,
     zeros, a start inside a binade, and thresholds that are never reached."""
     rng = np.random.default_rng(17)

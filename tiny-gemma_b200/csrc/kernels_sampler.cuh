@@ -4,9 +4,6 @@
 
 namespace tg {
 
-constexpr int SM_THREADS = 1024;
-constexpr int SM_NWARPS = SM_THREADS / 32;
-
 struct SampleArgs {
 	float *logits;   // [B][V]; min-p overwrites it with the reference's "probabilities"
 	int V;
@@ -126,17 +123,10 @@ __device__ __forceinline__ CdfFn cdf_element(float p, float inv_u) {
 	return f;
 }
 
-constexpr int CDF_PER_LANE = 8;
-constexpr int CDF_PER_WARP = 32 * CDF_PER_LANE;
-
-// Block-cooperative (NW warps, all threads call it with the same arguments). p[0..n) lies in shared
-// memory; *cum_io (shared) holds the running sum before p[0] and receives the sum after the last
-// element consumed. Returns the first index i with fl(cum + p[0] + ... + p[i]) >= randf, or -1.
-// scratch: 2 * NW + 8 ints of shared memory.
 // The first elements of a row are added one by one by a single thread: the running sum starts at
 // zero and changes binade about log2(position) times, and every change would cost a whole scan
 // round (≈ 1 us, the time of ≈ 400 sequential additions). p >= 0, so the sum never decreases and
-// a group of 8 is searched only when its last partial sum has reached randf.
+// a group of 8 is searched only when its last partial sum has reached randf. p is 16-byte aligned.
 __device__ __forceinline__ void cdf_cross_seq(const float *p, int end, float randf, float &cum, int &pos, int &res) {
 	float c = cum;
 	int i = pos;
@@ -184,135 +174,9 @@ __device__ __forceinline__ void cdf_cross_seq(const float *p, int end, float ran
 	pos = i;
 }
 
-// `seq_limit`: leading elements that one thread adds sequentially (see cdf_cross_seq) before the
-// block-wide scan takes over; pass ~1000 for the start of a row, 0 for later chunks. p must be
-// 16-byte aligned.
-template <int NW>
-__device__ int cdf_cross_block(const float *p, int n, float *cum_io, float randf, int *scratch, int seq_limit = 0) {
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	CdfFn *wt = reinterpret_cast<CdfFn *>(scratch);  // per-warp composite
-	int *s_pos = scratch + 2 * NW, *s_res = scratch + 2 * NW + 1;
-	if (tid == 0) {
-		float cum = *cum_io;
-		int pos = 0, res = -1;
-		if (seq_limit > 0) cdf_cross_seq(p, min(n, seq_limit), randf, cum, pos, res);
-		*cum_io = cum;
-		*s_pos = pos;
-		*s_res = res;
-	}
-	__syncthreads();
-	for (int guard = 0; guard < n + 64; guard++) {  // every round consumes at least one element
-		const int pos = *s_pos;
-		if (*s_res >= 0 || pos >= n) break;
-		const float cum = *cum_io;
-		const unsigned bits = __float_as_uint(cum);
-		const int e = int((bits >> 23) & 0xffu) - 127;
-		if (!(cum >= 7.888609e-31f) || e > 120) {
-			// zero, tiny, inf or NaN: plain fp32 steps until the sum is an ordinary number
-			__syncthreads();
-			if (tid == 0) {
-				float c = cum;
-				int i = pos, r = -1;
-				for (; i < n && r < 0; i++) {
-					c += p[i];
-					if (c >= randf) r = i;
-					if (c >= 7.888609e-31f && c < 1e36f) {
-						i++;
-						break;
-					}
-				}
-				*cum_io = c;
-				*s_pos = i;
-				*s_res = r;
-			}
-			__syncthreads();
-			continue;
-		}
-		const float u = __uint_as_float(unsigned(e - 23 + 127) << 23);
-		const float inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
-		const int S0 = int(cum * inv_u);
-		const float y = randf * inv_u;
-		const int T = (y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG;
-		const int Tmin = min(T, 1 << 24);
-		// this lane's elements
-		const int base = pos + warp * CDF_PER_WARP + lane * CDF_PER_LANE;
-		CdfFn el[CDF_PER_LANE];
-		CdfFn mine{0, 0};
-#pragma unroll
-		for (int k = 0; k < CDF_PER_LANE; k++) {
-			el[k] = CdfFn{0, 0};
-			if (base + k < n) el[k] = cdf_element(p[base + k], inv_u);
-			mine = cdf_compose(mine, el[k]);
-		}
-		// inclusive scan over the lanes
-		CdfFn inc = mine;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			CdfFn prev;
-			prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
-			prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
-			if (lane >= o) inc = cdf_compose(prev, inc);
-		}
-		if (lane == 31) wt[warp] = inc;
-		CdfFn exc;
-		exc.a0 = __shfl_up_sync(0xffffffffu, inc.a0, 1);
-		exc.a1 = __shfl_up_sync(0xffffffffu, inc.a1, 1);
-		if (lane == 0) exc = CdfFn{0, 0};
-		__syncthreads();
-		// state at the start of every warp; first warp in which the sum reaches the threshold
-		int Sw = S0, hit = -1, Shit = 0;
-#pragma unroll 1
-		for (int w = 0; w < NW; w++) {
-			const int nx = cdf_apply(wt[w], Sw);
-			if (hit < 0 && nx >= Tmin) {
-				hit = w;
-				Shit = Sw;
-			}
-			Sw = nx;
-		}
-		__syncthreads();  // wt is rewritten next round
-		if (hit < 0) {
-			if (tid == 0) {
-				*cum_io = float(Sw) * u;  // exact: Sw < 2^24
-				*s_pos = pos + NW * CDF_PER_WARP;
-			}
-		} else if (warp == hit) {
-			int S = cdf_apply(exc, Shit);
-			int jfirst = -1, Sbefore = 0, Safter = 0;
-#pragma unroll
-			for (int k = 0; k < CDF_PER_LANE; k++) {
-				const int nx = cdf_apply(el[k], S);
-				if (jfirst < 0 && nx >= Tmin) {
-					jfirst = base + k;
-					Sbefore = S;
-					Safter = nx;
-				}
-				S = nx;
-			}
-			const unsigned m = __ballot_sync(0xffffffffu, jfirst >= 0);
-			const int src = __ffs(m) - 1;  // m != 0: this warp's total reaches the threshold
-			if (lane == src) {
-				if (Safter < (1 << 24)) {
-					*s_res = jfirst;  // the sum reached randf inside the binade
-					*cum_io = float(Safter) * u;
-					*s_pos = jfirst + 1;
-				} else {
-					const float c = float(Sbefore) * u + p[jfirst];  // the one addition that leaves the binade
-					*cum_io = c;
-					*s_pos = jfirst + 1;
-					if (c >= randf) *s_res = jfirst;
-				}
-			}
-		}
-		__syncthreads();
-	}
-	__syncthreads();
-	return *s_res;
-}
-
-// The same for a block of at most 256 elements by one warp, without a barrier: p[0..n) in shared memory, 16-byte aligned, n a
-// multiple of 8, all lanes call it with the same arguments. Returns the index inside the block or -1; cum becomes the sum
-// behind the last element consumed. seq: add the elements one by one (the start of a row).
+// A block of at most 256 elements by one warp: p[0..n) in shared memory, 16-byte aligned, n a multiple of 8, cum the running sum
+// before p[0]; all lanes call it with the same arguments. Returns the first index with fl(cum + p[0] + ... + p[i]) >= randf inside
+// the block or -1; cum becomes the sum behind the last element consumed. seq: add the elements one by one (the start of a row).
 constexpr int CDF_BLK = 256;
 __device__ __forceinline__ int cdf_cross_warp(const float *p, int n, float &cum, float randf, bool seq) {
 	const int lane = threadIdx.x & 31, base = 8 * lane;
@@ -406,9 +270,8 @@ __device__ __forceinline__ int cdf_cross_warp(const float *p, int n, float &cum,
 //  fp32 sum reaches randf, else 0.
 // Steps 1-5 are data-parallel. Step 6 must reproduce a *sequential* fp32 sum
 // (fp32 addition is not associative, and the crossing index depends on the
-// rounding): cdf_cross_block evaluates that chain exactly, in parallel, over
-// chunks that a CTA stages into shared memory.
-constexpr int MP_CHUNK = 8192;
+// rounding): the maps above evaluate that chain exactly, in parallel
+// (cdf_walk_maps, cdf_cross_warp, cdf_walk_row).
 
 // Any number of rows, each spread over V / SR_PART CTAs: four kernels (row maximum; exponentials and segment sums;
 // scaling and segment maps; the walk). One CTA per row took ~1 ms for a row of 262144: four passes over 1 MB and
@@ -423,6 +286,9 @@ struct MinpRows {
 	float2 *seg_sum;  // [B][V / SR_SEG] masked sum, whole sum
 	int4 *seg_map;    // [B][V / SR_SEG] a0, a1, exponent of the binade
 	int4 *blk_map;    // [B][V / CDF_BLK]
+	// step 6 by itself (tg_inverse_cdf): the running sum before the row, and where the sum at its end goes; a sampler has 0 and null
+	float cum0;
+	float *cum_out;
 };
 __global__ void __launch_bounds__(SR_THREADS) minp_max_kernel(SampleArgs a, MinpRows w) {
 	pdl_trigger();
@@ -520,7 +386,7 @@ __global__ void __launch_bounds__(SR_THREADS) minp_scale_kernel(SampleArgs a, Mi
 		s_pre[warp] = us;
 	}
 	__syncthreads();
-	float denom = 0.0f, before = 0.0f;
+	float denom = 0.0f, before = w.cum0;
 #pragma unroll
 	for (int i = 0; i < SR_THREADS / 32; i++) {
 		denom += red[i];
@@ -591,12 +457,11 @@ template <class Get> __device__ __forceinline__ float cdf_walk_maps(Get get, int
 	return cum;
 }
 // One warp walks a row p of V elements in segments of seg_len (nb blocks of CDF_BLK, the last segment may end early): segment
-// maps, inside a segment whose map does not hold the maps of its blocks, inside such a block its elements. Returns the crossing
-// index, 0 if there is none. chunk: CDF_BLK floats of shared memory.
+// maps, inside a segment whose map does not hold the maps of its blocks, inside such a block its elements. cum: the running sum
+// before the row, then at the end of the walk. Returns the crossing index, 0 if there is none. chunk: CDF_BLK floats of shared memory.
 template <class Seg, class Blk>
-__device__ __forceinline__ int cdf_walk_row(Seg seg_map, Blk blk_map, const float *p, int V, int seg_len, int nb, float randf, float *chunk) {
+__device__ __forceinline__ int cdf_walk_row(Seg seg_map, Blk blk_map, const float *p, int V, int seg_len, int nb, float randf, float &cum, float *chunk) {
 	const int lane = threadIdx.x & 31, nseg = (V + seg_len - 1) / seg_len;
-	float cum = 0.0f;
 #pragma unroll 1
 	for (int c = 0; c < nseg; c++) {
 		cum = cdf_walk_maps(seg_map, nseg, randf, cum, c);
@@ -643,8 +508,10 @@ __global__ void __launch_bounds__(SR_THREADS) minp_walk_kernel(SampleArgs a, Min
 	if (rc < a.randf_cap) randf = a.randf[size_t(rc) * a.B + b];
 	__syncthreads();
 	if (tid >= 32) return;
-	const int found = cdf_walk_row([&](int i) { return staged ? mw_maps[i] : map(i); }, [&](int i) { return staged ? mw_maps[nseg + i] : map(nseg + i); }, x, a.V, SR_SEG, NB, randf, chunk);
+	float cum = w.cum0;
+	const int found = cdf_walk_row([&](int i) { return staged ? mw_maps[i] : map(i); }, [&](int i) { return staged ? mw_maps[nseg + i] : map(nseg + i); }, x, a.V, SR_SEG, NB, randf, cum, chunk);
 	if (tid == 0) {
+		if (w.cum_out) w.cum_out[b] = cum;
 		emit_token(a, b, found);
 		a.randf_count[b] = rc + 1;
 	}
@@ -792,7 +659,8 @@ __device__ __forceinline__ int minp_grid_row(const float *logits, float *probs, 
 	for (int c = tid; c < G * (1 + nb); c += 32 * NW) maps[c] = __ldcg(gmaps + c);
 	__syncthreads();
 	if (warp == 0) {
-		const int found = cdf_walk_row([&](int i) { return maps[i]; }, [&](int i) { return maps[G + i]; }, probs, V, cols, nb, randf, pl);
+		float cum = 0.0f;
+		const int found = cdf_walk_row([&](int i) { return maps[i]; }, [&](int i) { return maps[G + i]; }, probs, V, cols, nb, randf, cum, pl);
 		if (lane == 0) scratch[0] = found;
 	}
 	__syncthreads();
@@ -878,32 +746,6 @@ __global__ void __launch_bounds__(SG_THREADS, 1) minp_grid_kernel(SampleArgs a, 
 		a.randf_count[0] = rc + 1;
 	}
 	if (tid == 0 && *(volatile int *)&s_fail) atomicExch(err, 8);
-}
-
-// The inverse-CDF step in isolation over an explicit vector p[0..n) in global memory, starting
-// from the running sum cum0: *idx = first i with fl(cum0 + p[0] + ... + p[i]) >= randf, else -1.
-// One CTA; *cum_out receives the sum after the last element consumed.
-__global__ void __launch_bounds__(SM_THREADS) inverse_cdf_kernel(const float *p, int n, float cum0, float randf, int *idx,
-                                                                 float *cum_out) {
-	__shared__ float chunk[MP_CHUNK];
-	__shared__ int scratch[2 * SM_NWARPS + 8];
-	__shared__ float s_cum;
-	const int tid = threadIdx.x;
-	if (tid == 0) s_cum = cum0;
-	__syncthreads();
-	int found = -1;
-	for (int c0 = 0; c0 < n && found < 0; c0 += MP_CHUNK) {
-		const int m = min(MP_CHUNK, n - c0);
-		for (int i = tid; i < m; i += SM_THREADS) chunk[i] = p[c0 + i];
-		__syncthreads();
-		const int r = cdf_cross_block<SM_NWARPS>(chunk, m, &s_cum, randf, scratch, c0 == 0 ? 1024 : 0);
-		if (r >= 0) found = c0 + r;
-		__syncthreads();
-	}
-	if (tid == 0) {
-		*idx = found;
-		*cum_out = s_cum;
-	}
 }
 
 }  // namespace tg

@@ -491,7 +491,6 @@ struct tg_state {
 	int host_ring = 0;          // mirror of ring_base
 	// batched decode step (tensor-core GEMMs with M = batch)
 	bool batched_ok = false;
-	float *bx = nullptr, *bup = nullptr;  // [B][D] normed input, [B][I] up projection
 	TcScratch btc;
 	// persistent decode kernel (batch 1)
 	bool mega_ok = false;
@@ -1507,16 +1506,21 @@ int launch_argmax_rows(const SampleArgs &a, const SampScratch &ws, cudaStream_t 
 	count_launch();
 	return check_launch("argmax");
 }
+// the last two steps: probabilities and maps from the exponentials and segment sums, and the walk
+int launch_minp_tail(const SampleArgs &a, const MinpRows &rows, cudaStream_t st) {
+	launch_k(minp_scale_kernel, dim3(a.V / SR_PART, a.B), dim3(SR_THREADS), 0, st, a, rows);
+	const size_t maps = minp_walk_smem(a.V);
+	const int staged = maps <= 48 * 1024 - 4096;
+	launch_k(minp_walk_kernel, dim3(a.B), dim3(SR_THREADS), staged ? maps : 0, st, a, rows, staged);
+	count_launch(2);
+	return check_launch("minp");
+}
 int launch_minp_rows(const SampleArgs &a, const SampScratch &ws, cudaStream_t st) {
 	const dim3 grid(a.V / SR_PART, a.B);
 	launch_k(minp_max_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
 	launch_k(minp_exp_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
-	launch_k(minp_scale_kernel, grid, dim3(SR_THREADS), 0, st, a, ws.rows);
-	const size_t maps = minp_walk_smem(a.V);
-	const int staged = maps <= 48 * 1024 - 4096;
-	launch_k(minp_walk_kernel, dim3(a.B), dim3(SR_THREADS), staged ? maps : 0, st, a, ws.rows, staged);
-	count_launch(4);
-	return check_launch("minp");
+	count_launch(2);
+	return launch_minp_tail(a, ws.rows, st);
 }
 
 int enqueue_sampler(tg_state *s, float minp, float temp, bool log_tokens) {
@@ -1808,15 +1812,12 @@ int launch_gemm_tc(float *C, const QW &w, int M, const TcScratch &sc, cudaStream
 // the attention is per sequence (each against its own cache, positions read on the device).
 int batched_setup(tg_state *s) {
 	const tg_config &c = s->m->cfg;
-	const int B = s->B, D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab, qd = c.n_head * c.head_dim;
-	TG_CUDA(cudaMalloc(&s->bx, size_t(B) * D * 4));
-	TG_CUDA(cudaMalloc(&s->bup, size_t(B) * I * 4));
+	const int B = s->B, D = c.hidden_size, I = c.intermediate_size, qd = c.n_head * c.head_dim;
 	s->btc.x_bytes = i8_pack_bytes(B, std::max(I, std::max(D, qd)));
 	TG_CUDA(cudaMalloc(&s->btc.x, s->btc.x_bytes));
 	s->btc.partial_floats = std::min(size_t(24) * B * std::max(I, qd), size_t(1) << 28);
 	TG_CUDA(cudaMalloc(&s->btc.partial, s->btc.partial_floats * 4));
 	s->btc.err = s->err_flag;
-	(void)V;
 	s->batched_ok = true;
 	return TG_OK;
 }
@@ -2519,8 +2520,6 @@ int tg_state_free(tg_state *s) {
 	cudaFree(s->step_blk);  // err_flag, tok, randf_count, log_count (and the first randf)
 	cudaFree(s->pf);
 	cudaFree(s->pf_ids);
-	cudaFree(s->bx);
-	cudaFree(s->bup);
 	cudaFree(s->btc.x);
 	cudaFree(s->btc.partial);
 	cudaFree(s->d_tmaps);
@@ -3372,23 +3371,46 @@ int tg_argmax_logits(const float *logits, int n, int *tok) {
 }
 
 int tg_minp_logits(float *logits, int n, float minp, float temp, float randf, int *tok) {
-	if (!logits || !tok || n < MP_CHUNK || n % MP_CHUNK) return fail(TG_EINVAL, "bad argument (n must be a multiple of 8192)");
+	if (!logits || !tok || n < SR_PART || n % SR_PART) return fail(TG_EINVAL, "bad argument (n must be a multiple of 8192)");
 	return sample_host_row(logits, logits, n, true, minp, temp, randf, tok);
 }
 
+// The samplers' own kernels on a given vector: it is padded to whole parts with zeros, which add nothing, and its segment sums
+// come from the host, the masked ones such that the scale is 1.
 int tg_inverse_cdf(const float *p, int n, float cum0, float randf, int *idx, float *cum_out) {
-	if (!p || !idx || n < 1) return fail(TG_EINVAL, "bad argument");
+	if (!p || !idx || n < 1 || n > INT_MAX - SR_PART) return fail(TG_EINVAL, "bad argument");
 	TG_TRY(ensure_device(0));
-	DevBuf dp, di, dc;
-	TG_TRY(dp.alloc(size_t(n) * 4));
-	TG_TRY(di.alloc(4));
-	TG_TRY(dc.alloc(4));
+	const int V = (n + SR_PART - 1) / SR_PART * SR_PART;
+	std::vector<float2> sums(V / SR_SEG, make_float2(0.0f, 0.0f));
+	for (int i = 0; i < n; i++) sums[i / SR_SEG].y += p[i];
+	sums[0].x = 1.0f;
+	struct {
+		int tok, count;
+		float randf, cum;
+	} io = {0, 0, randf, 0.0f};
+	DevBuf dp, dws, dio;
+	TG_TRY(dp.alloc(size_t(V) * 4));
+	TG_TRY(dws.alloc(SampScratch::bytes(1, V)));
+	TG_TRY(dio.alloc(sizeof io));
+	SampScratch ws(static_cast<uint8_t *>(dws.p), 1, V);
+	ws.rows.cum0 = cum0;
+	ws.rows.cum_out = reinterpret_cast<float *>(static_cast<uint8_t *>(dio.p) + 12);
+	TG_CUDA(cudaMemset(static_cast<uint8_t *>(dp.p) + size_t(n) * 4, 0, size_t(V - n) * 4));
 	TG_CUDA(cudaMemcpy(dp.p, p, size_t(n) * 4, cudaMemcpyHostToDevice));
-	inverse_cdf_kernel<<<1, SM_THREADS>>>((const float *)dp.p, n, cum0, randf, (int *)di.p, (float *)dc.p);
-	count_launch();
-	TG_TRY(check_launch("inverse_cdf"));
-	TG_CUDA(cudaMemcpy(idx, di.p, 4, cudaMemcpyDeviceToHost));
-	if (cum_out) TG_CUDA(cudaMemcpy(cum_out, dc.p, 4, cudaMemcpyDeviceToHost));
+	TG_CUDA(cudaMemcpy(ws.rows.seg_sum, sums.data(), sums.size() * sizeof(float2), cudaMemcpyHostToDevice));
+	TG_CUDA(cudaMemcpy(dio.p, &io, sizeof io, cudaMemcpyHostToDevice));
+	SampleArgs a{};
+	a.logits = static_cast<float *>(dp.p);
+	a.V = V;
+	a.tok_out = static_cast<int *>(dio.p);
+	a.B = 1;
+	a.randf = reinterpret_cast<const float *>(static_cast<uint8_t *>(dio.p) + 8);
+	a.randf_count = static_cast<int *>(dio.p) + 1;
+	a.randf_cap = 1;
+	TG_TRY(launch_minp_tail(a, ws.rows, nullptr));
+	TG_CUDA(cudaMemcpy(&io, dio.p, sizeof io, cudaMemcpyDeviceToHost));
+	*idx = io.cum >= randf ? io.tok : -1;
+	if (cum_out) *cum_out = io.cum;
 	return TG_OK;
 }
 
