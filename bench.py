@@ -680,7 +680,7 @@ def run_ours(args):
             n = int(min(len(ref_seq), len(dev_seq)))
             diff = np.nonzero(ref_seq[:n] != dev_seq[:n])[0]
             line["parity"] = {"compared": n, "match_len": int(diff[0]) if diff.size else n,
-                              "what": "tokens of the device-resident loop against the reference's CPU run: same weights, "
+                              "what": "tokens of the device-resident loop against the CPU baseline's run (its kind: cpu_baseline): same weights, "
                                       "prompt and std::mt19937 uniforms; the reference's token 0 is drawn from its own "
                                       "prefill logits. With the 1024-entry GeLU table on random-init weights a draw flips "
                                       "on logit noise of 1e-3 (tests/test_e2e_1b_gpu.py holds the teacher-forced bar)"}

@@ -120,7 +120,9 @@ int tg_state_position(tg_state *s, int b, int *position);
  * From 4 sequences on, a sequence's logits agree with those of a
  * single-sequence state to rounding (the GEMMs split other row counts
  * differently), not bit for bit; batches below 4 keep the single sequence's
- * splits and are bit-identical to it. */
+ * splits and are bit-identical to it. A pass keeps at most 2^28 partial sums
+ * of its GEMMs: a prompt of the 1B configuration beyond about 19400 tokens is
+ * TG_ENOMEM (270m: any prompt up to n_pos fits). */
 int tg_prefill(tg_state *s, const int *ids_host, int n_tokens, float *logits_host);
 
 /* gemma::forward_decode, transformer.hpp:75-97: one token per sequence.
@@ -130,7 +132,8 @@ int tg_decode(tg_state *s, const int *ids_host, float *logits_host);
 
 /* Continuation of a non-empty context (a further turn of a conversation): the n tokens of ids_host
  * behind what the cache holds, with the result of n calls of forward_decode (transformer.hpp:75-97) on
- * those tokens: bit for bit up to 31 tokens (they are fed one after the other through the decode path), to
+ * those tokens: bit for bit up to 31 tokens (they are fed one after the other through the decode path, at a
+ * decoded token's time each: 31 tokens of the 1B model 21 to 24 ms, where 32 take 1.4 to 3.1), to
  * rounding beyond (all at once, as a prefill behind the cached context). The reference
  * cannot do this with its prefill — KVCache::update_prefill asserts an empty cache (decode.hpp:78-79,
  * listed as a limitation in README.md:96). One sequence per state; logits_host may be NULL, otherwise it

@@ -1,6 +1,5 @@
 """Writes tests/golden/*.npz from the reference itself. Needs the reference
-checkout (default /root/reference) and oracle/_ref/libtgref.so; run it in the
-build container, commit the outputs:
+checkout (TINY_GEMMA_REFERENCE) and oracle/_ref/libtgref.so; commit the outputs:
 
     python tests/golden/make_golden.py
 

@@ -156,9 +156,6 @@ __global__ void qgemm_splitk_reduce_groups_kernel(ReduceGroups g, const float *p
 	Cp[m * ld + nl] = s * sp_[nl];
 }
 
-// out[b, :] = table lookup per element: gate = lut(gate) * up over [rows][n] with row strides
-// (the batched decode step keeps up and gate in separate buffers)
-
 // ops::gelu (LUT) + ops::mul, reference ops.hpp:62-123: gate = lut(gate) * up
 __global__ void geglu_kernel(float *gate, const float *up, size_t n, GeluLut lut) {
 	size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;

@@ -2647,8 +2647,11 @@ int tg_append(tg_state *s, const int *ids, int n, float *logits_host) {
 	for (int i = 0; i < n; i++)
 		if (ids[i] < 0 || ids[i] >= m->cfg.n_vocab) return fail(TG_EINVAL, "token id out of range");
 	// Up to APPEND_DECODE tokens go through the decode path, bit for bit what tg_decode gives. A longer turn is a prefill
-	// behind the cached context: all its tokens at once (61 tokens behind 1500: 46 -> 3 ms for 1B), the same results to
-	// rounding.
+	// behind the cached context: all its tokens at once, the same results to rounding. The line is one of results, not of time:
+	// short turns keep the decode path's bits (the reference's own way to continue a context), and the prefill would be faster from
+	// 2 to 5 tokens on. Measured, decode path / prefill in ms: 1B behind 64 positions 2 tokens 1.48 / 1.32, 31 tokens 21.5 / 1.36;
+	// behind 1500 3 tokens 2.38 / 2.29, 31 tokens 23.4 / 2.32; behind 4096 4 tokens 3.3 / 3.1, 31 tokens 24.2 / 3.1. 270m behind 64 2
+	// tokens 0.89 / 0.79, behind 1500 4 tokens 1.89 / 1.47, behind 4096 5 tokens 2.36 / 1.95, 31 tokens 14.0 / 1.97.
 	constexpr int APPEND_DECODE = 31, APPEND_ROWS = 4096;
 	if (n > APPEND_DECODE && env_int("TG_GEMM_TC", 1)) {
 		const int p0 = s->host_pos[0];
