@@ -162,6 +162,8 @@ __device__ __forceinline__ double i8_to_double(uint32_t word, int byte) {  // ex
 	return __hiloint2double(0x43300000, int(__byte_perm(word ^ 0x80808080u, 0u, 0x4440u + byte))) - 4503599627370624.0;
 }
 __global__ void __launch_bounds__(256) qgemm_wide_rows_kernel(float *C, const float *A, const int8_t *W, const float *scales, const int *wide, int M, int K, int N) {
+	pdl_trigger();
+	pdl_wait();
 	constexpr int R = 8, H = 4;  // rows at a time, rows whose sums meet at a time
 	__shared__ int list[256], count[8];
 	__shared__ double part[8][H][128];

@@ -3167,7 +3167,10 @@ int tg_dev_qgemm(float *c, const float *a, const int8_t *w, const float *scales,
 		const cudaStream_t st = (cudaStream_t)stream;
 		int *wide = reinterpret_cast<int *>(tc[dev].x + i8_pack_bytes(M, K));
 		auto recompute = [&]() -> int {  // rows that the digits do not hold
-			qgemm_wide_rows_kernel<<<dim3(N / 128, std::min((M + 31) / 32, 64)), 256, 0, st>>>(c, a, w, scales, wide, M, K, N);
+			// Inside a graph it mostly finds nothing to do and costs 1.2 to 2 us (16 x 1152 x 6912 6.3 -> 7.6, 4096 x 1152 x 1024 21.6 ->
+			// 23.6): about one CTA per SM, which is what fits (64 parts of the rows: 25.1), launched programmatically (ordinary: +0.5)
+			const int parts = std::max(1, std::min((M + 7) / 8, g_num_sms / (N / 128)));
+			launch_k(qgemm_wide_rows_kernel, dim3(N / 128, parts), dim3(256), 0, st, c, a, w, scales, (const int *)wide, M, K, N);
 			count_launch();
 			return check_launch("qgemm_wide_rows");
 		};
