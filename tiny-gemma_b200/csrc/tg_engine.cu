@@ -313,7 +313,7 @@ int mvc_launch_t(float *y, const float *x, const int8_t *w, const float *scales,
 	// graph the launch is hidden anyway, and the edge delays a small kernel: 640 x 1024 3.57 -> 4.97 us, 1152 x 1024 3.99 -> 5.55,
 	// 2048 x 640 4.25 -> 5.65, but 1152 x 6912 6.68 -> 6.20 and 6912 x 1152 6.88 -> 6.15.
 	bool pdl = !max_clusters && use_pdl();
-	if (pdl && size_t(K) * N <= (size_t(4) << 20)) {
+	if (pdl && st && st != cudaStreamLegacy && size_t(K) * N <= (size_t(4) << 20)) {  // (the legacy stream is never captured; the question takes 0.1 us)
 		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
 		if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();  // (the launch itself reports what is wrong)
 		pdl = cap == cudaStreamCaptureStatusNone;
