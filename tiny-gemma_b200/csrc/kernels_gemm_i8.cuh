@@ -102,10 +102,10 @@ template <int NW> __device__ __forceinline__ uint32_t block_umax(uint32_t v, uin
 // Rows that the digits do not hold well enough. An element below 2^-7 of its row's largest loses mantissa bits, and a column
 // whose weights on the large elements are zero sees that loss undiluted. Rows in which more than an eighth of the nonzero elements
 // (of some warp's part of the row) lie below 2^-12 of the largest (such an element is kept to 2^-19 of itself), and rows below 2^-96
-// altogether, are marked by the operators' packing and recomputed by qgemm_wide_rows_kernel. A normal row with one element of s sigmas is marked from s ~ 400
-// on; just below, a column that does not see that element is off by 2e-7. (A model's own passes do not: their rows come out of a norm or
-// a GeGLU, and its decode steps hold them to 2^-24 of the largest in any case.)
-// (called by whole warps; the zeros are told apart only where many elements are small)
+// altogether, are marked by the operators' packing and recomputed by qgemm_wide_rows_kernel. A normal row with one element of s
+// sigmas is marked from s = 512 on, from 256 on now and then; below, a column that does not see that element is off by 1.4e-7 at
+// most. (A model's own passes mark nothing: their rows come out of a norm or a GeGLU, and its decode steps hold them to 2^-24 of the
+// largest in any case.) Called by whole warps; the zeros are told apart only where many elements are small.
 template <int PER> __device__ __forceinline__ bool i8_wide(const float4 (&v)[PER], uint32_t maxbits) {
 	const float below = __uint_as_float(uint32_t(max(int(maxbits >> 23) - 11, 0)) << 23);
 	int small = 0, zero = 0;
