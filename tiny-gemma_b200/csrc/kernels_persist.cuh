@@ -10,14 +10,12 @@
 //     region reserved for that phase. A region is refilled for the NEXT layer
 //     as soon as its last reader is done, so about one layer of weights per SM
 //     is always in flight and HBM never waits for the chain;
-//   * makes the tile products warp-autonomous. The activation vector is
-//     quantised once per phase to 24-bit block fixed point (three 8-bit digit
-//     planes, one power-of-two exponent per vector), the weight unit is stored
-//     as 16-byte pieces of 4 rows x 4 columns (a 32-bit word = 4 consecutive
-//     rows of one column), and a lane accumulates dp4a(word, digit plane) for
-//     its 4 columns: the products and sums are exact integers, there is no
-//     int8 -> fp32 conversion in the loop, and a warp finishes its own columns
-//     with six shuffles — no block-wide barrier in any product;
+//   * multiplies on the tensor cores (tcgen05.mma kind::i8), from the shared memory the weights land in. The
+//     activation vector is quantised once per phase to 31-bit block fixed point (four signed 8-bit digits, one
+//     power-of-two exponent per vector); weight columns are the M rows of the operation and the digits its N
+//     columns, so the integer sums are exact. One vector would use 4 of 16 columns and a unit of 16 weight columns
+//     16 of 64 rows: the K range of a unit is cut into segments that sit side by side as further rows (weights) and
+//     columns (digits); the products of equal segments are the ones that are read back, and added as integers;
 //   * hands results over through small L2-resident vectors that validate
 //     themselves (a sentinel marks words not yet written). Polled bytes are the
 //     cost of a hand-off (about 40 ns per KB and CTA), so producers publish
@@ -38,9 +36,9 @@
 // of reference ops.hpp:848-858 evaluated by an exact scan).
 //
 // Arithmetic: y[n] = scale[n] * sum_k x[k] W[k,n] (reference linalg.hpp:41-204)
-// with x rounded to 24 significant bits relative to the largest |x| of the
-// vector (fp32 itself keeps 24 bits relative to each element); products and
-// sums are exact, one rounding when the integer sum becomes a float.
+// with x rounded to a multiple of 2^-30 of the power of two above the largest
+// |x| of the vector (fp32 itself keeps 24 bits relative to each element); products
+// and sums are exact, one rounding when the integer sum becomes a float.
 //
 // Every wait is bounded: a spin that runs out sets *err and a shared abort
 // flag, after which all waits fall through and the kernel returns.
@@ -48,30 +46,21 @@
 #include <cuda.h>
 
 #include "kernels_decode.cuh"
+#include "kernels_gemm_i8.cuh"  // digits, tcgen05 helpers
 #include "kernels_sampler.cuh"
+#include "persist_plan.h"  // units and their tiles
 #include "tg_common.cuh"
 
 namespace tg {
 
-constexpr int PS_THREADS = 384;
-constexpr int PS_NW = PS_THREADS / 32;
 constexpr int PS_MAX_LAYERS = 32;
 constexpr int PS_MAX_CH = 32;            // most cache chunks per head
 constexpr int PS_ATT_ROW = AT_HD + 8;    // floats per attention partial: o[256], m, l, padding
 constexpr uint32_t PS_BULK_PIECE = 16384;
 constexpr unsigned PS_EMPTY = 0xFFFFFFFFu;  // "not written yet": a NaN no computation produces
 
-struct PsPhase {
-	int ngroups;  // column groups (4 columns each) of a unit, per matrix
-	int nq;       // quads (4 rows each) of a unit
-	int nsplit;   // K-splits across CTAs
-	int ntiles;   // column tiles
-	int units;    // ntiles * nsplit
-	int kp;       // warps that share one column group (they split its quads)
-	int wq;       // quads per warp
-	int bytes;    // bytes of a unit
-	int cta0;     // CTA of unit 0
-};
+constexpr int PS_TMEM = 64;              // TMEM columns: 16 per tile of a unit, or two accumulators of the lm_head
+constexpr int PS_LUT = 1024;             // largest GeLU table that is kept in shared memory
 
 struct PsLayer {
 	const float *sq, *sk, *sv, *so, *su, *sg, *sd;  // per-column scales
@@ -87,16 +76,16 @@ struct PsArgs {
 	const PsLayer *layers;
 	int L, D, I, V, QD, KD;
 	PsPhase A, C, Dp, E;
-	// lm_head: column tiles of lm_groups * 4 columns; a tile's rows arrive as lm_nchunk ring stages of lm_cq quads
-	int lm_groups, lm_cq, lm_nchunk, lm_ntiles, lm_stages, lm_stage_bytes;
+	// lm_head: column tiles of 128 columns; a tile's rows arrive as lm_nchunk ring stages of lm_steps * 32 rows
+	int lm_steps, lm_nchunk, lm_ntiles, lm_stages, lm_stage_bytes;
+	PsPhase lm;  // (the digits' layout: one segment)
 	const float *lm_scale, *final_norm;
 	const int8_t *wte;
 	const float *wte_s;
 	float sqrtD;
 	const float *rope[2][2];  // [is_local][cos, sin]
 	GeluLut lut;
-	int off_A, off_C, off_D, off_E, off_h, off_xd, off_att, smem_total;
-	int xd_words;  // words per digit plane buffer
+	int off_A, off_C, off_D, off_E, off_h, off_att, off_lut, smem_total;
 	// Hand-off arena, three copies used by consecutive layers; every float is PS_EMPTY or a value.
 	//   ll_qkv [QD + 2 KD]                 q|k|v, scaled                      (A -> B)
 	//   ll_att [4][PS_MAX_CH][PS_ATT_ROW]  attention partials per head, chunk (B -> C)
@@ -130,8 +119,6 @@ struct PsArgs {
 	int sched;              // 0: up/gate and down units of layer l+1 requested in phase E of layer l; 1: units of layer l requested after the Q|K|V product of layer l
 	long long *gt;  // optional: [CTA][12] global-timer marks of one layer (DBG instantiation)
 	int *beacon;    // optional (mapped host memory): [CTA][16] progress marks of every warp, for diagnosing a stall
-	int e_rows;     // 1: the down projection runs by K-parts per warp (ps_product_rows), e_wq quads per warp
-	int e_wq;
 	int fault_cta;  // test hook: this CTA withholds its down-projection hand-off (-1: none); the waits then run out
 };
 
@@ -213,17 +200,6 @@ __device__ __forceinline__ float ps_ld1(const float *p) {
 __device__ __forceinline__ bool ps_ok(float v) { return __float_as_uint(v) != PS_EMPTY; }
 __device__ __forceinline__ bool ps_ok(const float2 &v) { return ps_ok(v.x) && ps_ok(v.y); }
 __device__ __forceinline__ bool ps_ok(const float4 &v) { return ps_ok(v.x) && ps_ok(v.y) && ps_ok(v.z) && ps_ok(v.w); }
-__device__ __forceinline__ int ps_dp4a_su(uint32_t a, uint32_t b, int c) {  // signed bytes of a times unsigned bytes of b
-	int d;
-	asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-	return d;
-}
-__device__ __forceinline__ int ps_dp4a_ss(uint32_t a, uint32_t b, int c) {
-	int d;
-	asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-	return d;
-}
-
 // What a wait needs to know to give up: the CTA's abort flag, the global error word, the time limit.
 struct PsW {
 	int *s_abort;
@@ -302,101 +278,11 @@ __device__ __noinline__ void ps_grid_sync(const PsW w, int where, unsigned *bar,
 	__syncthreads();
 }
 
-// ------------------------------------------------------------------ quantised activations
-// A vector x[0..4 nq) becomes three word planes xd[p * stride + q], p = 0, 1, 2: byte j of word q of plane p is
-// digit p of round(x[4q + j] * 2^(23 - e)), digits 0 and 1 unsigned, digit 2 signed, where 2^e > max |x|.
-// ps_exponent returns e for a bound on max |x| (clamped so that both scale factors are normal floats).
-__device__ __forceinline__ int ps_exponent(float bound) {
-	const int eb = int(__float_as_uint(bound) >> 23) & 0xFF;  // bound in [2^(eb-127), 2^(eb-126))
-	return max(-100, min(100, eb - 126));
-}
-__device__ __forceinline__ float ps_pow2(int e) { return __uint_as_float(uint32_t(e + 127) << 23); }
-__device__ __forceinline__ void ps_quantise(float4 y, float qs, uint32_t *xd, int stride, int q) {
-	__builtin_assume(__isShared(xd));
-	int v[4];
-	v[0] = __float2int_rn(y.x * qs);
-	v[1] = __float2int_rn(y.y * qs);
-	v[2] = __float2int_rn(y.z * qs);
-	v[3] = __float2int_rn(y.w * qs);
-#pragma unroll
-	for (int i = 0; i < 4; i++) v[i] = max(-8388607, min(8388607, v[i]));
-	const uint32_t p01 = __byte_perm(v[0], v[1], 0x5140), p23 = __byte_perm(v[2], v[3], 0x5140);
-	const uint32_t h01 = __byte_perm(v[0], v[1], 0x0062), h23 = __byte_perm(v[2], v[3], 0x0062);
-	xd[q] = __byte_perm(p01, p23, 0x5410);
-	xd[stride + q] = __byte_perm(p01, p23, 0x7632);
-	xd[2 * stride + q] = __byte_perm(h01, h23, 0x5410);
-}
-// max over the CTA of a non-negative value through `red` (12 floats; one barrier), then the exponent for it
-__device__ __forceinline__ int ps_block_exponent(float mx, float *red) {
-	mx = warp_max(mx);
-	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-	__syncthreads();
-	float M = 0.0f;
-#pragma unroll
-	for (int w = 0; w < PS_NW; w++) M = fmaxf(M, red[w]);
-	return ps_exponent(M * 1.000001f);
-}
-
-// ------------------------------------------------------------------ tile products
-// piece (group g, quad q) of a unit sits at tile[g * nq + q]; word c of a piece = column 4g + c, its
-// bytes = rows 4q .. 4q+3. acc[3c + p] += dp4a(word c, digit plane p).
-struct PsAcc {
-	int v[12];
-};
-__device__ __forceinline__ void ps_mac(PsAcc &a, const uint4 &w, uint32_t x0, uint32_t x1, uint32_t x2) {
-	const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		a.v[3 * c] = ps_dp4a_su(ww[c], x0, a.v[3 * c]);
-		a.v[3 * c + 1] = ps_dp4a_su(ww[c], x1, a.v[3 * c + 1]);
-		a.v[3 * c + 2] = ps_dp4a_ss(ww[c], x2, a.v[3 * c + 2]);
-	}
-}
-// Lane sums of one group -> warp sums. The three digit sums of a column combine to
-// S = a2 * 65536 + a1 * 256 + a0 in fp32 (each below 2^22 per lane: exact conversions, one rounding
-// per fma), then the four columns are reduced over the lanes by halving (2 + 1 + 1 + 1 + 1
-// shuffles). Lanes 0..3 return the sum of column `lane`. Called by whole warps.
-__device__ __noinline__ float ps_finish(const PsAcc a) {
-	const int lane = threadIdx.x & 31;
-	float v[4];
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		// |digit sum| < 2^22 (at most 32 quads per lane: 32 * 4 * 127 * 255): exact int -> float through the
-		// mantissa of 1.5 * 2^23, one add and one subtract instead of a conversion instruction
-		const float f0 = __int_as_float(0x4B400000 + a.v[3 * c]) - 12582912.0f;
-		const float f1 = __int_as_float(0x4B400000 + a.v[3 * c + 1]) - 12582912.0f;
-		const float f2 = __int_as_float(0x4B400000 + a.v[3 * c + 2]) - 12582912.0f;
-		v[c] = fmaf(f2, 65536.0f, fmaf(f1, 256.0f, f0));
-	}
-	{
-		const bool up = lane & 16;
-		const float s0 = up ? v[0] : v[2], s1 = up ? v[1] : v[3];
-		const float k0 = up ? v[2] : v[0], k1 = up ? v[3] : v[1];
-		v[0] = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
-		v[1] = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-	}
-	{
-		const bool up = lane & 8;
-		const float s = up ? v[0] : v[1], k = up ? v[1] : v[0];
-		v[0] = k + __shfl_xor_sync(0xffffffffu, s, 8);
-	}
-	v[0] += __shfl_xor_sync(0xffffffffu, v[0], 4);
-	v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-	v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-	// lane 8 * (2 b4 + b3) holds column 2 b4 + b3
-	return __shfl_sync(0xffffffffu, v[0], (lane & 3) * 8);
-}
-// Shared-memory accesses by 32-bit shared-window address. The helpers below are not inlined (code
-// size), so a pointer argument would be a generic pointer and every access a generic load, which
-// runs at about half the rate of ld.shared in the product loop.
+// ------------------------------------------------------------------ shared memory by 32-bit shared-window address
+// (The helpers below are not inlined, so a pointer argument would be a generic pointer and every access a generic one.)
 __device__ __forceinline__ uint4 ps_lds128(uint32_t addr) {
 	uint4 v;
-	asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-	return v;
-}
-__device__ __forceinline__ uint32_t ps_lds32(uint32_t addr) {
-	uint32_t v;
-	asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+	asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
 	return v;
 }
 __device__ __forceinline__ float ps_ldsf(uint32_t addr) {
@@ -405,223 +291,159 @@ __device__ __forceinline__ float ps_ldsf(uint32_t addr) {
 	return v;
 }
 __device__ __forceinline__ void ps_stsf(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-// Two groups at once: the two reductions' shuffles overlap. Lanes 0..3: (r0, r1) of column `lane`.
-__device__ __noinline__ float2 ps_finish2(const PsAcc a, const PsAcc b) {
-	const int lane = threadIdx.x & 31;
-	float v[4], u[4];
-#pragma unroll
-	for (int c = 0; c < 4; c++) {
-		const float f0 = __int_as_float(0x4B400000 + a.v[3 * c]) - 12582912.0f;
-		const float f1 = __int_as_float(0x4B400000 + a.v[3 * c + 1]) - 12582912.0f;
-		const float f2 = __int_as_float(0x4B400000 + a.v[3 * c + 2]) - 12582912.0f;
-		v[c] = fmaf(f2, 65536.0f, fmaf(f1, 256.0f, f0));
-		const float g0 = __int_as_float(0x4B400000 + b.v[3 * c]) - 12582912.0f;
-		const float g1 = __int_as_float(0x4B400000 + b.v[3 * c + 1]) - 12582912.0f;
-		const float g2 = __int_as_float(0x4B400000 + b.v[3 * c + 2]) - 12582912.0f;
-		u[c] = fmaf(g2, 65536.0f, fmaf(g1, 256.0f, g0));
-	}
-	{
-		const bool up = lane & 16;
-		const float s0 = up ? v[0] : v[2], s1 = up ? v[1] : v[3], t0 = up ? u[0] : u[2], t1 = up ? u[1] : u[3];
-		const float k0 = up ? v[2] : v[0], k1 = up ? v[3] : v[1], m0 = up ? u[2] : u[0], m1 = up ? u[3] : u[1];
-		v[0] = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
-		v[1] = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-		u[0] = m0 + __shfl_xor_sync(0xffffffffu, t0, 16);
-		u[1] = m1 + __shfl_xor_sync(0xffffffffu, t1, 16);
-	}
-	{
-		const bool up = lane & 8;
-		const float s = up ? v[0] : v[1], k = up ? v[1] : v[0], t = up ? u[0] : u[1], m = up ? u[1] : u[0];
-		v[0] = k + __shfl_xor_sync(0xffffffffu, s, 8);
-		u[0] = m + __shfl_xor_sync(0xffffffffu, t, 8);
-	}
-#pragma unroll
-	for (int o = 4; o > 0; o >>= 1) {
-		v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-		u[0] += __shfl_xor_sync(0xffffffffu, u[0], o);
-	}
-	return make_float2(__shfl_sync(0xffffffffu, v[0], (lane & 3) * 8), __shfl_sync(0xffffffffu, u[0], (lane & 3) * 8));
-}
-// The warp that completes a count: every warp calls this once per round after its work; the one
-// that makes the count reach `total` gets true (and resets the counter for the next round).
-__device__ __forceinline__ bool ps_last(uint32_t cnt_s, int total) {
-	const int lane = threadIdx.x & 31;
-	__syncwarp();
-	int old = 0;
-	if (lane == 0) {
-		__threadfence_block();
-		asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(cnt_s) : "memory");
-		if (old == total - 1) asm volatile("st.shared.u32 [%0], %1;" ::"r"(cnt_s), "r"(0) : "memory");
-	}
-	old = __shfl_sync(0xffffffffu, old, 0);
-	if (old == total - 1) __threadfence_block();  // the other warps' shared-memory writes are visible to every lane
-	return old == total - 1;
-}
-// Column sums of one unit: warp -> (group = warp / kp, part = warp % kp) takes quads part * wq .. of
-// its group, of one matrix or of two matrices of the same shape that share the activations (up, then
-// gate: `two`). tile_s, xd_s, part_s (PS_NW * 8 floats), cnt_s (PS_NW + 1 ints) are shared-window
-// addresses. flags bit 0: this warp publishes its group (it is the only warp of the group, or the last
-// of its kp warps to finish, and has added the parts in part order): lanes 0..3 hold the raw sums of
-// columns 4 * group + lane in r0 (and r1). Bit 1: nobody reads the tile any more after this warp.
-struct PsOut {
-	float r0, r1;
-	int flags;
+
+// ------------------------------------------------------------------ quantised activations
+// A vector x[0..4 nq) becomes the digits of round(x * 2^(30 - e)), 2^e > max |x|: q = d0 + 256 d1 + 65536 d2 + 2^24 d3 with
+// d_i in [-128, 127] (the digits of the prefill's GEMM). PsX: where a phase keeps them.
+struct PsX {
+	uint32_t base;  // shared-window address
+	unsigned seg_mul;
+	int seg_q, sbo;
 };
+__device__ __forceinline__ PsX ps_x(const PsPhase &ph, uint32_t smem_s) { return PsX{smem_s + uint32_t(ph.off_x), ph.seg_mul, ph.seg_q, ph.x_sbo}; }
+// exponent for a bound on max |x| (clamped so that both scale factors are normal floats); a vector with an infinity gives NaN
+__device__ __forceinline__ int ps_exponent(float bound) { return max(-96, min(100, (int(__float_as_uint(bound) >> 23) & 0xFF) - 126)); }
+__device__ __forceinline__ float ps_pow2(int e) { return __uint_as_float(uint32_t(e + 127) << 23); }
+__device__ __forceinline__ float ps_qmul(float M) { return ps_pow2(30 - ps_exponent(M * 1.000001f)); }
+__device__ __forceinline__ float ps_qscale(float M) { return M < INFINITY ? ps_pow2(ps_exponent(M * 1.000001f) - 30) : __uint_as_float(0x7FC00000u); }
+__device__ __forceinline__ void ps_sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+// quad q of the vector. (Lanes of a warp hold consecutive quads: four words of a 16-byte chunk, chunks 36 words apart: no bank conflict.)
+__device__ __forceinline__ void ps_quantise(float4 y, float mul, const PsX &x, int q) {
+	const uint32_t a = i8_digits(y.x, mul), b = i8_digits(y.y, mul), c = i8_digits(y.z, mul), d = i8_digits(y.w, mul);
+	const uint32_t ab01 = __byte_perm(a, b, 0x5140), ab23 = __byte_perm(a, b, 0x7362);
+	const uint32_t cd01 = __byte_perm(c, d, 0x5140), cd23 = __byte_perm(c, d, 0x7362);
+	const uint32_t p = x.base + uint32_t(ps_digit_offset(x.seg_mul, x.seg_q, x.sbo, q));
+	ps_sts32(p, __byte_perm(ab01, cd01, 0x5410));
+	ps_sts32(p + 16, __byte_perm(ab01, cd01, 0x7632));
+	ps_sts32(p + 32, __byte_perm(ab23, cd23, 0x5410));
+	ps_sts32(p + 48, __byte_perm(ab23, cd23, 0x7632));
+}
+// maximum of non-negative floats over a warp: their bit patterns order like the values
+__device__ __forceinline__ float ps_warp_max(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); }
+// the PS_NW floats at p (16-byte aligned): sum in index order, maximum
+__device__ __forceinline__ void ps_lds12(uint32_t p, float (&v)[PS_NW]) {
+#pragma unroll
+	for (int i = 0; i < PS_NW; i += 4)
+		asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[i]), "=f"(v[i + 1]), "=f"(v[i + 2]), "=f"(v[i + 3]) : "r"(p + 4u * i) : "memory");
+}
+__device__ __forceinline__ float ps_sum12(uint32_t p) {
+	float v[PS_NW];
+	ps_lds12(p, v);
+	float t = v[0];
+#pragma unroll
+	for (int i = 1; i < PS_NW; i++) t += v[i];
+	return t;
+}
+__device__ __forceinline__ float ps_max12(uint32_t p) {
+	float v[PS_NW];
+	ps_lds12(p, v);
+	float t = v[0];
+#pragma unroll
+	for (int i = 1; i < PS_NW; i++) t = fmaxf(t, v[i]);
+	return t;
+}
+// max over the CTA of a non-negative value through `red` (PS_NW floats; one barrier)
+__device__ __forceinline__ float ps_block_max(float mx, float *red) {
+	mx = ps_warp_max(mx);
+	if ((threadIdx.x & 31) == 0) ps_stsf(ps_smem(red + (threadIdx.x >> 5)), mx);
+	__syncthreads();
+	return ps_max12(ps_smem(red));
+}
+
+// ------------------------------------------------------------------ unit products
+__device__ __forceinline__ uint64_t ps_desc(uint32_t addr, int lbo, int sbo) {  // K-major operand without swizzle
+	return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t(lbo >> 4) << 16) | (uint64_t(sbo >> 4) << 32) | (uint64_t(1) << 46);
+}
+__device__ __forceinline__ uint32_t ps_idesc(int mt) {  // D int32, A and B signed 8 bit, both K-major, M = mt, N = 16
+	return (2u << 4) | (1u << 7) | (1u << 10) | (2u << 17) | (uint32_t(mt >> 4) << 24);
+}
+__device__ __forceinline__ int4 ps_tmem_ld4(uint32_t taddr) {  // 32 lanes x 4 columns
+	int4 v;
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(taddr) : "memory");
+	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+	return v;
+}
+// sum of digit sum i * 256^i, exact (at most 2^30 * 127 * 6912 < 2^50), rounded once
+__device__ __forceinline__ float ps_join(const int4 &s) {
+	return __ll2float_rn((((((long long)s.w << 8) + s.z) << 8) + s.y) * 256ll + s.x);
+}
 // what a CTA's place in the grid fixes for the whole launch (kept in shared memory, read where it is used)
 struct PsCta {
 	const int8_t *srcA, *srcC, *srcD, *srcE;
 	int tileA, tileC, splitC, tileE, splitE, presE, uD, has;
+	// per phase and warp: accumulator column | (first entry of the column sums) << 8; per phase and tile: byte offset of its digits
+	int ep[4][PS_NW], xo[4][PS_TILES];
 };
-__device__ __noinline__ PsOut ps_product(uint32_t tile_s, int ngroups, int nq, int kp, int wq, bool two, uint32_t xd_s, int xs,
-                                         uint32_t part_s, uint32_t cnt_s, long long *trace = nullptr) {
-	PsOut o{0.0f, 0.0f, 0};
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	if (trace && lane == 0) trace[warp * 4] = clock64();
-	const int group = warp / kp;
-	if (group >= ngroups) return o;
-	const int part = warp - group * kp;
-	const int q1 = min(nq, (part + 1) * wq);
-	PsAcc a0, a1;
-#pragma unroll
-	for (int i = 0; i < 12; i++) a0.v[i] = a1.v[i] = 0;
-	const uint32_t t0 = tile_s + uint32_t(group * nq) * 16u, t1 = tile_s + uint32_t((ngroups + group) * nq) * 16u;
-	int q = part * wq + lane;
-	// two quads per round: the second quad's loads are in flight while the first one's products issue
-	// (requesting the next round's operands a round ahead was measured slower: more registers, no gain)
-#pragma unroll 1
-	for (; q + 32 < q1; q += 64) {
-		const uint32_t xa = xd_s + 4u * q;
-		const uint32_t x0 = ps_lds32(xa), x1 = ps_lds32(xa + 4u * xs), x2 = ps_lds32(xa + 8u * xs);
-		const uint32_t y0 = ps_lds32(xa + 128u), y1 = ps_lds32(xa + 4u * xs + 128u), y2 = ps_lds32(xa + 8u * xs + 128u);
-		const uint4 w0 = ps_lds128(t0 + 16u * q), w1 = ps_lds128(t0 + 16u * q + 512u);
-		if (two) {
-			const uint4 v0 = ps_lds128(t1 + 16u * q), v1 = ps_lds128(t1 + 16u * q + 512u);
-			ps_mac(a1, v0, x0, x1, x2);
-			ps_mac(a1, v1, y0, y1, y2);
-		}
-		ps_mac(a0, w0, x0, x1, x2);
-		ps_mac(a0, w1, y0, y1, y2);
-	}
-#pragma unroll 1
-	for (; q < q1; q += 32) {
-		const uint32_t xa = xd_s + 4u * q;
-		const uint32_t x0 = ps_lds32(xa), x1 = ps_lds32(xa + 4u * xs), x2 = ps_lds32(xa + 8u * xs);
-		ps_mac(a0, ps_lds128(t0 + 16u * q), x0, x1, x2);
-		if (two) ps_mac(a1, ps_lds128(t1 + 16u * q), x0, x1, x2);
-	}
-	if (trace && lane == 0) trace[warp * 4 + 1] = clock64();
-	if (two) {
-		const float2 r = ps_finish2(a0, a1);
-		o.r0 = r.x;
-		o.r1 = r.y;
-	} else {
-		o.r0 = ps_finish(a0);
-	}
-	if (trace && lane == 0) trace[warp * 4 + 2] = clock64();
-	bool pub = true;
-	if (kp > 1) {
-		if (lane < 4) {
-			ps_stsf(part_s + 4u * (warp * 8 + lane), o.r0);
-			ps_stsf(part_s + 4u * (warp * 8 + 4 + lane), o.r1);
-		}
-		pub = ps_last(cnt_s + 4u * (1 + group), kp);
-		if (pub) {
-			o.r0 = o.r1 = 0.0f;
-			if (lane < 4)
-				for (int p = 0; p < kp; p++) {
-					o.r0 += ps_ldsf(part_s + 4u * ((group * kp + p) * 8 + lane));
-					o.r1 += ps_ldsf(part_s + 4u * ((group * kp + p) * 8 + 4 + lane));
-				}
-		}
-	}
-	if (pub) o.flags = 1 | (ps_last(cnt_s, ngroups) ? 2 : 0);
-	if (trace && lane == 0) trace[warp * 4 + 3] = clock64();
-	return o;
+__device__ __forceinline__ void ps_fill_map(const PsPhase &ph, int warp, int *ep, int *xo) {
+	const int t = warp >> 2;
+	if (t >= ph.tiles) return;
+	int r0, col;
+	ps_warp_rows(ph, warp, r0, col);
+	ep[warp] = (16 * t + col) | (r0 << 8);
+	xo[t] = (ps_tile_segment(ph.rows, ph.mt, t) / 2) * ph.x_sbo;
 }
-
-// Down projection without a CTA-wide prologue. Warp w takes K-part w of the unit (quads w * wq .. of every
-// group; lane -> quads lane, lane + 32, lane + 64 of the part, wq <= 96): it polls ITS rows of the activation
-// vector, quantises them with a warp-local exponent into registers, multiplies them with all ngroups <= 4
-// groups of the tile and leaves scaled fp32 partial sums in part_s[w][16]. The warp that finishes last adds
-// the PS_NW parts in part order: its lanes 0 .. 4 * ngroups - 1 return the raw sums of columns
-// 4 * group + (lane & 3), group = lane / 4, in r0, with flags = 3. No warp waits for another warp's rows, so
-// a late producer delays only the part that needs it. part_s: PS_NW * 16 floats; cnt_s: one counter.
-__device__ __noinline__ PsOut ps_product_rows(const PsW w, int where, uint32_t tile_s, int ngroups, int nq, int wq, const float *act,
-                                              uint32_t part_s, uint32_t cnt_s, long long *trace = nullptr) {
-	PsOut o{0.0f, 0.0f, 0};
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	if (trace && lane == 0) trace[warp * 4] = clock64();
-	const int qb = warp * wq, qe = min(nq, qb + wq);  // this warp's quads
-	float4 v[3];
-	{
-		int spins = 0;
-		long long t0 = 0;
-		bool ok;
-		do {
-			ok = true;
-#pragma unroll
-			for (int i = 0; i < 3; i++) {
-				const int q = qb + lane + 32 * i;
-				v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-				if (q < qe) v[i] = ps_ld4(act + 4 * q);
-				ok = ok && ps_ok(v[i]);
-			}
-		} while (!ok && ps_retry(w, where, spins, t0));
-	}
-	float mx = 0.0f;
-#pragma unroll
-	for (int i = 0; i < 3; i++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-	mx = warp_max(mx);
-	if (trace && lane == 0) trace[warp * 4 + 1] = clock64();
-	const int e = ps_exponent(mx * 1.000001f);
-	const float qs = ps_pow2(23 - e), back = ps_pow2(e - 23);
-	uint32_t x0[3], x1[3], x2[3];
-#pragma unroll
-	for (int i = 0; i < 3; i++) {
-		int d[4];
-		d[0] = __float2int_rn(v[i].x * qs);
-		d[1] = __float2int_rn(v[i].y * qs);
-		d[2] = __float2int_rn(v[i].z * qs);
-		d[3] = __float2int_rn(v[i].w * qs);
-#pragma unroll
-		for (int j = 0; j < 4; j++) d[j] = max(-8388607, min(8388607, d[j]));
-		const uint32_t p01 = __byte_perm(d[0], d[1], 0x5140), p23 = __byte_perm(d[2], d[3], 0x5140);
-		const uint32_t h01 = __byte_perm(d[0], d[1], 0x0062), h23 = __byte_perm(d[2], d[3], 0x0062);
-		x0[i] = __byte_perm(p01, p23, 0x5410);
-		x1[i] = __byte_perm(p01, p23, 0x7632);
-		x2[i] = __byte_perm(h01, h23, 0x5410);
-	}
-	// quads past the part multiply zeros; their tile address is clamped into the part
-	uint32_t ta[3];
-#pragma unroll
-	for (int i = 0; i < 3; i++) ta[i] = tile_s + 16u * uint32_t(min(qb + lane + 32 * i, qe - 1));
+// Integer sums of a unit's columns: entry s * rows + c of the int4 array at ph.off_acc = digit sums of column c over segment s.
+// Called by the whole CTA behind the barrier that ends the prologue (the digits' writers have fenced). Warp 4 t issues tile
+// t's MMAs into its own 16 TMEM columns (one accumulator per issuing warp), warps 4 t .. 4 t + 3 read them back. bar_w, pw,
+// rdy: barrier of the unit's bulk copy; pm: parity of bar_m[t]. Behind the closing barrier nobody reads the unit or the digits
+// any more. Measured from the prologue's barrier to the values in registers (1B: 27 MMAs of up and gate, 27 of down, 4 of O, 9
+// of q|k|v): about 430 clk + 38 per MMA of 128 rows, 23 per one of 64; the dp4a loops over the same tiles took 2400, 1450,
+// 850 and 1000 clk and 400 to 600 more to reduce over the lanes.
+struct PsMm {  // what a product needs of its phase (by value: a reference to the kernel's arguments would be a generic pointer)
+	int tiles, mt, steps, x_sbo;
+	uint32_t x_s, acc_s, tile_s;
+};
+__device__ __forceinline__ PsMm ps_mm(const PsPhase &ph, uint32_t smem_s, uint32_t tile_s) {
+	return PsMm{ph.tiles, ph.mt, ph.steps, ph.x_sbo, smem_s + uint32_t(ph.off_x), smem_s + uint32_t(ph.off_acc), tile_s};
+}
+__device__ __noinline__ uint32_t ps_product(const PsW w, int where, const PsMm ph, uint32_t tmem, uint64_t *bar_w, uint32_t pw, bool rdy, uint64_t *bar_m,
+                                            uint32_t pm, const int *ep, const int *xo) {
+	__builtin_assume(__isShared(ep));
+	__builtin_assume(__isShared(xo));
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = warp >> 2;
+	if (t < ph.tiles) {
+		if ((warp & 3) == 0) {
+			if (!rdy) ps_wait_bulk(w, where, bar_w, pw);
+			__syncwarp();
+			tc_fence_after();
+			const int mt = ph.mt, steps = ph.steps;
+			const uint64_t da = ps_desc(ph.tile_s + uint32_t(t * steps * mt) * 32u, mt * 16, 128), db = ps_desc(ph.x_s + uint32_t(xo[t]), PS_XCH, ph.x_sbo);
+			const uint32_t id = ps_idesc(mt), d = tmem + 16u * t;
+			if (tc_elect()) {
 #pragma unroll 1
-	for (int g = 0; g < ngroups; g += 2) {
-		PsAcc a0, a1;
-#pragma unroll
-		for (int i = 0; i < 12; i++) a0.v[i] = a1.v[i] = 0;
-		const uint32_t g0 = 16u * uint32_t(g * nq), g1 = 16u * uint32_t(min(g + 1, ngroups - 1) * nq);
-#pragma unroll
-		for (int i = 0; i < 3; i++) {
-			ps_mac(a0, ps_lds128(ta[i] + g0), x0[i], x1[i], x2[i]);
-			ps_mac(a1, ps_lds128(ta[i] + g1), x0[i], x1[i], x2[i]);
+				for (int i = 0; i < steps; i++) i8_mma<1>(d, da + uint64_t(i * mt * 2), db + uint64_t(i * (2 * PS_XCH / 16)), id, i > 0 ? 1u : 0u);
+				i8_commit<1>(&bar_m[t]);
+			}
+			__syncwarp();
 		}
-		const float2 r = ps_finish2(a0, a1);
-		if (lane < 4) {
-			ps_stsf(part_s + 4u * (warp * 16 + 4 * g + lane), r.x * back);
-			if (g + 1 < ngroups) ps_stsf(part_s + 4u * (warp * 16 + 4 * g + 4 + lane), r.y * back);
-		}
+		const int m = ep[warp];
+		ps_wait_bulk(w, where, &bar_m[t], pm);
+		pm ^= 1u;
+		__syncwarp();
+		tc_fence_after();
+		const int4 v = ps_tmem_ld4(tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m & 0xFF));
+		if (4 * lane < ph.mt)
+			asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(ph.acc_s + 16u * uint32_t((m >> 8) + lane)), "r"(v.x), "r"(v.y),
+			             "r"(v.z), "r"(v.w)
+			             : "memory");
+		tc_fence_before();
 	}
-	if (trace && lane == 0) trace[warp * 4 + 2] = clock64();
-	if (ps_last(cnt_s, PS_NW)) {
-		o.flags = 3;
-		if (lane < 4 * ngroups) {
-#pragma unroll
-			for (int p = 0; p < PS_NW; p++) o.r0 += ps_ldsf(part_s + 4u * (p * 16 + lane));
-		}
+	__syncthreads();
+	return pm;
+}
+// column c of a unit: the segments' digit sums added (exact) and joined
+__device__ __forceinline__ float ps_column(const PsPhase &ph, uint32_t smem_s, int c) {
+	uint32_t p = smem_s + uint32_t(ph.off_acc) + 16u * uint32_t(c);
+	int4 s = make_int4(0, 0, 0, 0);
+#pragma unroll 4
+	for (int i = 0; i < ph.segs; i++, p += 16u * uint32_t(ph.rows)) {
+		const uint4 v = ps_lds128(p);
+		s.x += int(v.x);
+		s.y += int(v.y);
+		s.z += int(v.z);
+		s.w += int(v.w);
 	}
-	if (trace && lane == 0) trace[warp * 4 + 3] = clock64();
-	return o;
+	return ps_join(s);
 }
 
 // A CTA's unit is one contiguous block of the re-tiled copy: one bulk copy. Called by one lane.
@@ -633,10 +455,10 @@ __device__ __noinline__ void ps_issue(uint8_t *dst, const int8_t *src, uint32_t 
 	ps_bulk(dst, src, bytes, bar, pol);
 }
 
-// Re-tile `ntiles_mat` column tiles x `nsplit` K-splits of a row-major int8 matrix [K][N] into unit order:
-// unit (split, tile0 + t) is a block at dst + (split * ntiles_total + tile0 + t) * unit_stride + dst_off
-// holding the pieces [group][quad] of 16 bytes described at ps_dot. One thread per piece.
-__device__ __forceinline__ uint4 ps_piece(const int8_t *src, size_t N, size_t row0, size_t col0) {
+// Re-tile `ntiles_mat` column tiles x ph.nsplit K-splits of a row-major int8 matrix [K][N] into unit order: unit (split,
+// tile0 + t) is a block at dst + (split * ntiles + tile0 + t) * bytes in the layout described at PsPhase, whose rows row0.. hold this
+// matrix. One thread per 4 columns x 16 k.
+__device__ __forceinline__ uint4 ps_piece(const int8_t *src, size_t N, size_t row0, size_t col0) {  // 4 x 4: word c = column col0 + c
 	const uint32_t r0 = *reinterpret_cast<const uint32_t *>(src + row0 * N + col0);
 	const uint32_t r1 = *reinterpret_cast<const uint32_t *>(src + (row0 + 1) * N + col0);
 	const uint32_t r2 = *reinterpret_cast<const uint32_t *>(src + (row0 + 2) * N + col0);
@@ -645,41 +467,29 @@ __device__ __forceinline__ uint4 ps_piece(const int8_t *src, size_t N, size_t ro
 	const uint32_t t2 = __byte_perm(r0, r1, 0x7362), t3 = __byte_perm(r2, r3, 0x7362);
 	return make_uint4(__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632));
 }
-__global__ void retile_quads_kernel(int8_t *dst, const int8_t *src, int N, int ngroups, int nq, int nsplit, int ntiles_total,
-                                    int tile0, int ntiles_mat, size_t unit_stride, size_t dst_off) {
-	const size_t total = size_t(nsplit) * ntiles_mat * ngroups * nq;
+__global__ void retile_units_kernel(int8_t *dst, const int8_t *src, int N, PsPhase ph, int tile0, int ntiles_mat, int row0) {
+	const int gcols = ntiles_mat * ph.ncol / 4, uch = ph.nq / 4, sch = ph.seg_q / 4;  // column groups; 16-k chunks of a unit, of a segment
+	const size_t total = size_t(gcols) * uch * ph.nsplit;
 	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-		const int g = int(i % ngroups);
-		const int t = int((i / ngroups) % ntiles_mat);
-		const int q = int((i / (size_t(ngroups) * ntiles_mat)) % nq);
-		const int split = int(i / (size_t(ngroups) * ntiles_mat * nq));
-		const uint4 v = ps_piece(src, size_t(N), (size_t(split) * nq + q) * 4, (size_t(t) * ngroups + g) * 4);
-		*reinterpret_cast<uint4 *>(dst + size_t(split * ntiles_total + tile0 + t) * unit_stride + dst_off + (size_t(g) * nq + q) * 16) = v;
-	}
-}
-// lm_head [K][V] -> [tile][chunk][group][quad] pieces; columns past V (the last tile) are zero.
-__global__ void retile_lm_kernel(int8_t *dst, const int8_t *src, int V, int ngroups, int cq, int nchunk, int ntiles) {
-	const size_t gcols = size_t(ntiles) * ngroups;  // column groups in all
-	const size_t total = gcols * cq * nchunk;
-	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-		const size_t gc = i % gcols;
-		const int row_q = int(i / gcols);  // quad row of the whole matrix
-		const int t = int(gc / ngroups), g = int(gc % ngroups);
-		const int ch = row_q / cq, q = row_q % cq;
-		uint4 v = make_uint4(0u, 0u, 0u, 0u);
-		if (gc * 4 < size_t(V)) v = ps_piece(src, size_t(V), size_t(row_q) * 4, gc * 4);
-		*reinterpret_cast<uint4 *>(dst + ((size_t(t) * nchunk + ch) * ngroups * cq + size_t(g) * cq + q) * 16) = v;
+		const int g = int(i % gcols), kc = int(i / gcols);
+		const int t = g * 4 / ph.ncol, c = g * 4 - t * ph.ncol, split = kc / uch, ku = kc - split * uch, seg = ku / sch, ch = ku - seg * sch;
+		uint4 p[4];
+#pragma unroll
+		for (int j = 0; j < 4; j++) p[j] = ps_piece(src, size_t(N), size_t(kc) * 16 + 4 * j, size_t(g) * 4);
+		uint4 *o = reinterpret_cast<uint4 *>(dst + size_t(split * ph.ntiles + tile0 + t) * ph.bytes + ps_unit_offset(ph, row0 + c, seg, ch));
+		o[0] = make_uint4(p[0].x, p[1].x, p[2].x, p[3].x);
+		o[1] = make_uint4(p[0].y, p[1].y, p[2].y, p[3].y);
+		o[2] = make_uint4(p[0].z, p[1].z, p[2].z, p[3].z);
+		o[3] = make_uint4(p[0].w, p[1].w, p[2].w, p[3].w);
 	}
 }
 
-// lut::GeLUTable::lookup (reference ops.hpp:41-51) with the table kept L2-resident
-__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint64_t keep) {
-	const float q = (x - t.mn) / t.eps;
-	if (!(q < 2147483648.0f) || q < -2147483648.0f) return 0.0f;  // (x86 cvttss2si: INT_MIN, a negative index)
-	const int idx = int(q);
-	if (idx < 0) return 0.0f;
+// lut::GeLUTable::lookup (reference ops.hpp:41-51); tab_s: the table in shared memory where it fits there
+__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint32_t tab_s, uint64_t keep) {
+	int idx;
+	if (!t.index(x, idx)) return 0.0f;
 	if (idx >= t.size) return x;
-	return ps_ldk(t.table + idx, keep);
+	return t.size <= PS_LUT ? ps_ldsf(tab_s + 4u * idx) : ps_ldk(t.table + idx, keep);
 }
 
 // ------------------------------------------------------------------ prologues
@@ -691,15 +501,14 @@ __device__ __forceinline__ float ps_inv_rms(float sumsq, float inv_dim) {
 	return r * fmaf(-0.5f * v, r * r, 1.5f);
 }
 // If part: t[d] = sum_s part[s][d] (scaled partial sums, polled until complete; threads past D/4 poll
-// the presence words);  h += rmsnorm(t; w_post). Then y = rmsnorm(h; w_pre), quantised into xd (stride
-// D/4) with *s_xscale = 2^(e - 23). Every CTA computes the same bits. D <= 4 * PS_THREADS. Thread t
-// owns elements 4t..4t+3, which are quad t. bred: 3 * PS_NW floats.
-__device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h, uint32_t *xd, float *bred, float *s_xscale,
+// the presence words);  h += rmsnorm(t; w_post). Then y = rmsnorm(h; w_pre), quantised with *s_xscale = 2^(e - 30).
+// Every CTA computes the same bits. D <= 4 * PS_THREADS. Thread t owns elements 4t..4t+3, which are quad t. bred: 3 * PS_NW
+// floats, 16-byte aligned.
+__device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h, const PsX x, float *bred, float *s_xscale,
                                         const float *part, int nsplit, const float *pres, int npres, const float *w_post,
-                                        const float *w_pre, uint64_t keep, float *x_out, long long *trace = nullptr) {
+                                        const float *w_pre, uint64_t keep, float *x_out) {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	__builtin_assume(__isShared(h));
-	__builtin_assume(__isShared(xd));
 	__builtin_assume(__isShared(s_xscale));
 	// the norm weights are L2-resident (evict-last): requested together with the first poll loads
 	float4 wpost = make_float4(0.f, 0.f, 0.f, 0.f), wpre = wpost;
@@ -709,7 +518,6 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 	}
 	const uint32_t bred_s = ps_smem(bred);
 	const float invD = 1.0f / float(D);
-	if (trace && lane == 0) trace[warp * 5] = clock64();
 	const bool in = 4 * tid < D;
 	float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
 	if (in) hv = *reinterpret_cast<const float4 *>(h + 4 * tid);
@@ -735,16 +543,11 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 			tv.z += p0.z + p1.z;
 			tv.w += p0.w + p1.w;
 		}
-		if (trace && lane == 0) trace[warp * 5 + 1] = clock64();
 		float ss = fmaf(tv.x, tv.x, fmaf(tv.y, tv.y, fmaf(tv.z, tv.z, tv.w * tv.w)));
 		ss = warp_sum(ss);
 		if (lane == 0) ps_stsf(bred_s + 4u * warp, ss);
 		__syncthreads();
-		if (trace && lane == 0) trace[warp * 5 + 2] = clock64();
-		float t = 0.0f;
-#pragma unroll
-		for (int i = 0; i < PS_NW; i++) t += ps_ldsf(bred_s + 4u * i);
-		const float r1 = ps_inv_rms(t, invD);
+		const float r1 = ps_inv_rms(ps_sum12(bred_s), invD);
 		hv.x = hv.x + (tv.x * r1) * (wpost.x + 1.0f);
 		hv.y = hv.y + (tv.y * r1) * (wpost.y + 1.0f);
 		hv.z = hv.z + (tv.z * r1) * (wpost.z + 1.0f);
@@ -754,34 +557,26 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 	const float4 g = make_float4(wpre.x + 1.0f, wpre.y + 1.0f, wpre.z + 1.0f, wpre.w + 1.0f);
 	float ss2 = fmaf(hv.x, hv.x, fmaf(hv.y, hv.y, fmaf(hv.z, hv.z, hv.w * hv.w)));
 	float mx = fmaxf(fmaxf(fabsf(hv.x * g.x), fabsf(hv.y * g.y)), fmaxf(fabsf(hv.z * g.z), fabsf(hv.w * g.w)));
+	mx = ps_warp_max(mx);
 	ss2 = warp_sum(ss2);
-	mx = warp_max(mx);
 	if (lane == 0) {
 		ps_stsf(bred_s + 4u * (PS_NW + warp), ss2);
 		ps_stsf(bred_s + 4u * (2 * PS_NW + warp), mx);
 	}
 	__syncthreads();
-	if (trace && lane == 0) trace[warp * 5 + 3] = clock64();
-	float t2 = 0.0f, m2 = 0.0f;
-#pragma unroll
-	for (int i = 0; i < PS_NW; i++) {
-		t2 += ps_ldsf(bred_s + 4u * (PS_NW + i));
-		m2 = fmaxf(m2, ps_ldsf(bred_s + 4u * (2 * PS_NW + i)));
-	}
-	const float r2 = ps_inv_rms(t2, invD);
-	const int e = ps_exponent(r2 * m2 * 1.000001f);
+	const float r2 = ps_inv_rms(ps_sum12(bred_s + 4u * PS_NW), invD), M = r2 * ps_max12(bred_s + 8u * PS_NW);
 	if (in) {
 		float4 y;
 		y.x = (hv.x * r2) * g.x;
 		y.y = (hv.y * r2) * g.y;
 		y.z = (hv.z * r2) * g.z;
 		y.w = (hv.w * r2) * g.w;
-		ps_quantise(y, ps_pow2(23 - e), xd, D / 4, tid);
+		ps_quantise(y, ps_qmul(M), x, tid);
 		if (x_out) *reinterpret_cast<float4 *>(x_out + 4 * tid) = y;
 	}
-	if (tid == 0) *s_xscale = ps_pow2(e - 23);
+	if (tid == 0) *s_xscale = ps_qscale(M);
+	ps_fence_async();
 	__syncthreads();
-	if (trace && lane == 0) trace[warp * 5 + 4] = clock64();
 }
 
 // one warp: x[0..256) (dims 4 lane.. and 128 + 4 lane..) -> rmsnorm, RoPE, * scale -> dst (may alias x)
@@ -828,12 +623,11 @@ __device__ __forceinline__ void ps_norm_rope(const float *x, const PsRope &r, fl
 
 // Phase C prologue: merge the attention partials of `hp` heads starting at head h0 over `nch` chunks
 // into the normalised output (reference ops.hpp:316-357 keeps it normalised per step; the split form
-// divides once), quantise it into xd (stride hp * 64).
-__device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, uint32_t *xd,
+// divides once), quantise it.
+__device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, const PsX x,
                                            float *bred, float *s_xscale) {
 	const int tid = threadIdx.x;
 	__builtin_assume(__isShared(scr));
-	__builtin_assume(__isShared(xd));
 	__builtin_assume(__isShared(bred));
 	__builtin_assume(__isShared(s_xscale));
 	const int items = hp * (AT_HD / 4);  // float4 columns
@@ -898,17 +692,17 @@ __device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *
 		y.w *= inv;
 		mx = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
 	}
-	const int e = ps_block_exponent(mx, bred);
-	if (tid < items) ps_quantise(y, ps_pow2(23 - e), xd, items, tid);
-	if (tid == 0) *s_xscale = ps_pow2(e - 23);
+	const float M = ps_block_max(mx, bred);
+	if (tid < items) ps_quantise(y, ps_qmul(M), x, tid);
+	if (tid == 0) *s_xscale = ps_qscale(M);
+	ps_fence_async();
 	__syncthreads();
 }
 
 // Phase E prologue: this CTA's rows of the activation vector (nq quads from act), polled until
-// complete, quantised into xd (stride nq). nq <= 5 * PS_THREADS.
-__device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, uint32_t *xd, float *bred, float *s_xscale) {
+// complete, quantised. nq <= 5 * PS_THREADS.
+__device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, const PsX x, float *bred, float *s_xscale) {
 	const int tid = threadIdx.x;
-	__builtin_assume(__isShared(xd));
 	__builtin_assume(__isShared(bred));
 	__builtin_assume(__isShared(s_xscale));
 	float4 v[5];
@@ -928,14 +722,15 @@ __device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *a
 	float mx = 0.0f;
 #pragma unroll
 	for (int q = 0; q < 5; q++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[q].x), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w))));
-	const int e = ps_block_exponent(mx, bred + PS_NW);
-	const float qs = ps_pow2(23 - e);
+	const float M = ps_block_max(mx, bred);
+	const float qs = ps_qmul(M);
 #pragma unroll
 	for (int q = 0; q < 5; q++) {
 		const int i = q * PS_THREADS + tid;
-		if (i < nq) ps_quantise(v[q], qs, xd, nq, i);
+		if (i < nq) ps_quantise(v[q], qs, x, i);
 	}
-	if (tid == 0) *s_xscale = ps_pow2(e - 23);
+	if (tid == 0) *s_xscale = ps_qscale(M);
+	ps_fence_async();
 	__syncthreads();
 }
 
@@ -1059,102 +854,105 @@ __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache,
 	__syncthreads();  // the scratch is reused by phase C
 }
 
-// lm_head of one token: logits[v] = lm_scale[v] * sum_k x[k] W[k,v]; this CTA takes column tiles cta, cta + G, ...;
-// a tile arrives as lm_nchunk ring stages in `ring`; warp w owns column groups 2w and 2w + 1 of every tile over
-// all of its rows. Returns this lane's best (temperature-scaled) logit and the ring's barrier parities.
+// lm_head of one token: logits[v] = lm_scale[v] * sum_k x[k] W[k,v]; this CTA takes tiles cta, cta + G, ... of 128 columns; a
+// tile arrives as lm_nchunk ring stages in `ring`. Warp PS_NW - 1 copies, warp 8 multiplies into one of two accumulators, warps
+// 0 to 3 take 32 columns each. Returns this lane's best (temperature-scaled) logit and the ring's barrier parities.
 // pre: ring stages the caller has already requested (those that lie inside the up/gate region, which is
-// idle from the last layer's up/gate product on).
+// idle from the last layer's up/gate product on). acc_n: tiles of this CTA so far.
+// HBM bounds it. With dp4a products on all 12 warps a stage took about as long to multiply as to arrive, and 302 MB took 57.6 us;
+// a copy into the same rings that multiplies nothing takes 49.
 struct PsLmOut {
 	float best;
 	int best_i;
 	uint32_t plm, pemp;
 };
-__device__ __noinline__ PsLmOut ps_lm_head(const PsArgs &a, const PsW pw, uint8_t *ring, const uint32_t *xd, float xs, uint64_t *bar_lm,
-                                           uint64_t *emp_lm, uint32_t plm, uint32_t pemp, uint64_t pol, uint64_t keep, int pre) {
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int cta = blockIdx.x, G = gridDim.x, D = a.D, L = a.L;
+__device__ __noinline__ PsLmOut ps_lm_head(const PsArgs &a, const PsW pw, uint8_t *ring, uint32_t smem_s, float xs, uint32_t tmem, uint64_t *bar_lm,
+                                           uint64_t *emp_lm, uint64_t *acc_full, uint64_t *acc_free, uint32_t plm, uint32_t pemp, uint32_t acc_n,
+                                           uint64_t pol, uint64_t keep, int pre) {
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int cta = blockIdx.x, G = gridDim.x, where = (a.L << 4) | 6;
 	__builtin_assume(__isShared(ring));
-	__builtin_assume(__isShared(xd));
-	__builtin_assume(__isShared(bar_lm));
-	__builtin_assume(__isShared(emp_lm));
-float best = -INFINITY;  // running max of this lane's (temperature-scaled) logits, lanes 0..7
-int best_i = -1;
-{
-	const int nst = a.lm_stages, nchunk = a.lm_nchunk, cq = a.lm_cq;
-	const int my_tiles = (a.lm_ntiles - cta + G - 1) / G;
-	const int total = my_tiles * nchunk;
+	const int nst = a.lm_stages, nchunk = a.lm_nchunk, my_tiles = (a.lm_ntiles - cta + G - 1) / G, total = my_tiles * nchunk;
 	const uint32_t sbytes = uint32_t(a.lm_stage_bytes);
-			auto issue_stage = [&](int q, int stg) {  // one lane
-		const int t = cta + (q / nchunk) * G, c = q % nchunk;
-		ps_issue(ring + size_t(stg) * sbytes, a.lm_tiled + (size_t(t) * nchunk + c) * sbytes, sbytes, &bar_lm[stg], pol, pw.s_abort);
-	};
-	if (tid == PS_THREADS - 32) {
-#pragma unroll 1
-		for (int s = pre; s < nst && s < total; s++) issue_stage(s, s);  // (the first `pre` stages were requested during the last layer)
-	}
-	PsAcc a0, a1;
-	float sc = 0.0f;
-	int stg = 0, c = 0, tile = cta;
-	bool lm_rdy = false;
-	const bool wact = 2 * warp < a.lm_groups;
-#pragma unroll 1
-	for (int q = 0; q < total; q++) {
-		if (c == 0) {
-#pragma unroll
-			for (int i = 0; i < 12; i++) a0.v[i] = a1.v[i] = 0;
-			const int v0 = tile * a.lm_groups * 4 + 8 * warp + lane;  // lanes 0..3: group 2w, lanes 4..7: group 2w+1
-			sc = (wact && lane < 8 && v0 < a.V) ? ps_ldk(a.lm_scale + v0, keep) : 0.0f;
-		}
-		if (!lm_rdy) ps_wait_bulk(pw, (L << 4) | 6, &bar_lm[stg], (plm >> stg) & 1u);
-		plm ^= (1u << stg);
-		{  // the next stage's barrier is tested now; its result is needed only after this stage's products
-			const int ns = (stg + 1 == nst) ? 0 : stg + 1;
-			lm_rdy = (q + 1 < total) && ps_mbar_test(&bar_lm[ns], (plm >> ns) & 1u);
-		}
-		if (wact) {
-			const uint4 *t0 = reinterpret_cast<const uint4 *>(ring + size_t(stg) * sbytes) + 2 * warp * cq;
-			const uint32_t *x = xd + c * cq;
-#pragma unroll 1
-			for (int qq = lane; qq < cq; qq += 32) {
-				const uint32_t x0 = x[qq], x1 = x[D / 4 + qq], x2 = x[2 * (D / 4) + qq];
-				ps_mac(a0, t0[qq], x0, x1, x2);
-				ps_mac(a1, t0[cq + qq], x0, x1, x2);
-			}
-		}
-		__syncwarp();
-		if (lane == 0) ps_mbar_arrive(&emp_lm[stg]);
-		if (tid == PS_THREADS - 32) {
-			const int nq = q + nst;
-			if (nq < total) {
-				ps_wait_bulk(pw, (L << 4) | 6, &emp_lm[stg], (pemp >> stg) & 1u);  // all 12 warps have left the stage
-				issue_stage(nq, stg);
-			}
-		}
-		__syncwarp();
-		pemp ^= (1u << stg);
-		if (c == nchunk - 1 && wact) {
-			const float2 r01 = ps_finish2(a0, a1);  // lanes 0..3
-			const float r1s = __shfl_sync(0xffffffffu, r01.y, lane & 3);  // every lane takes part in the shuffle
-			const float r = (lane < 4) ? r01.x : r1s;
-			const int v = tile * a.lm_groups * 4 + 8 * warp + lane;
-			if (lane < 8 && v < a.V) {
-				const float lg = (r * xs) * sc;
-				__stcg(a.logits + v, lg);
-				const float z = (a.sampler == 2) ? lg / a.temp : lg;
-				if (z > best) {  // tiles ascend, so the first maximum keeps the lowest index
-					best = z;
-					best_i = v;
-				}
-			}
-		}
-		if (++stg == nst) stg = 0;
-		if (++c == nchunk) {
+	PsLmOut o{-INFINITY, -1, plm, pemp};
+	if (warp == PS_NW - 1) {
+		int t = cta, c = pre, stg = pre;  // (pre <= nchunk)
+		if (c == nchunk) {
 			c = 0;
-			tile += G;
+			t += G;
+		}
+		if (stg == nst) stg = 0;
+#pragma unroll 1
+		for (int q = pre; q < total; q++) {
+			if (q >= nst) {
+				ps_wait_bulk(pw, where, &emp_lm[stg], (pemp >> stg) & 1u);
+				pemp ^= 1u << stg;
+			}
+			__syncwarp();
+			if (tc_elect()) ps_issue(ring + size_t(stg) * sbytes, a.lm_tiled + (size_t(t) * nchunk + c) * sbytes, sbytes, &bar_lm[stg], pol, pw.s_abort);
+			__syncwarp();
+			if (++stg == nst) stg = 0;
+			if (++c == nchunk) {
+				c = 0;
+				t += G;
+			}
+		}
+	} else if (warp == 8) {
+		const uint32_t id = ps_idesc(128);
+		const uint64_t db0 = ps_desc(smem_s + uint32_t(a.lm.off_x), PS_XCH, a.lm.x_sbo);
+		int stg = 0, c = 0;
+#pragma unroll 1
+		for (int q = 0; q < total; q++) {
+			const uint32_t b = acc_n & 1u;
+			if (c == 0) ps_wait_bulk(pw, where, &acc_free[b], ((acc_n >> 1) & 1u) ^ 1u);  // (the first use of a fresh barrier passes)
+			ps_wait_bulk(pw, where, &bar_lm[stg], (plm >> stg) & 1u);
+			plm ^= 1u << stg;
+			__syncwarp();
+			tc_fence_after();
+			const uint64_t da = ps_desc(ps_smem(ring) + uint32_t(stg) * sbytes, 128 * 16, 128), db = db0 + uint64_t(c * a.lm_steps * (2 * PS_XCH / 16));
+			if (tc_elect()) {
+#pragma unroll 1
+				for (int i = 0; i < a.lm_steps; i++) i8_mma<1>(tmem + 16u * b, da + uint64_t(i * 256), db + uint64_t(i * (2 * PS_XCH / 16)), id, (c | i) ? 1u : 0u);
+				i8_commit<1>(&emp_lm[stg]);
+				if (c == nchunk - 1) i8_commit<1>(&acc_full[b]);
+			}
+			__syncwarp();
+			if (++stg == nst) stg = 0;
+			if (++c == nchunk) {
+				c = 0;
+				acc_n++;
+			}
+		}
+	} else if (warp < 4) {
+#pragma unroll 1
+		for (int t = cta; t < a.lm_ntiles; t += G, acc_n++) {
+			const int v = t * 128 + warp * 32 + lane;
+			const float sc = ps_ldk(a.lm_scale + v, keep);
+			const uint32_t b = acc_n & 1u;
+			ps_wait_bulk(pw, where, &acc_full[b], (acc_n >> 1) & 1u);
+			__syncwarp();
+			tc_fence_after();
+			const int4 s = ps_tmem_ld4(tmem + (uint32_t(warp * 32) << 16) + 16u * b);
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) ps_mbar_arrive(&acc_free[b]);
+			const float lg = (ps_join(s) * xs) * sc;
+			__stcg(a.logits + v, lg);
+			const float z = (a.sampler == 2) ? lg / a.temp : lg;
+			if (z > o.best) {  // tiles ascend, so the first maximum keeps the lowest index
+				o.best = z;
+				o.best_i = v;
+			}
 		}
 	}
-}
-	return PsLmOut{best, best_i, plm, pemp};
+	// every slot's barriers have completed once per use
+#pragma unroll 1
+	for (int s = 0; s < nst && s < total; s++)
+		if ((((total - s + nst - 1) / nst) & 1) != 0) {
+			o.plm ^= 1u << s;
+			o.pemp ^= 1u << s;
+		}
+	return o;
 }
 
 // Sampler of one token (0: none, 1: argmax, 2: min-p) over the logits row; `best`, `best_i` are this lane's
@@ -1313,9 +1111,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	extern __shared__ uint8_t smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(smem_raw) + 127) & ~uintptr_t(127));  // the host adds 128 bytes of slack
 	__shared__ uint64_t bar_A, bar_C, bar_D, bar_E, bar_lm[8], emp_lm[8];
-	__shared__ float bred[3 * PS_NW];
-	__shared__ float s_part[PS_NW * 16];
-	__shared__ int s_cnt[PS_NW + 4];
+	__shared__ uint64_t bar_m[PS_TILES], acc_full[2], acc_free[2];  // MMAs of a unit's tile; the lm_head's two accumulators
+	__shared__ __align__(16) float bred[3 * PS_NW];
+	__shared__ uint32_t s_tmem;
 	__shared__ float s_xscale;
 	__shared__ int s_abort;
 	__shared__ float s_f[8];
@@ -1333,11 +1131,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	// registers this kernel cannot have are spilled to local memory, which the small L1 left beside 224 KB of
 	// shared memory does not hold)
 #define h (reinterpret_cast<float *>(smem + a.off_h))
-#define xd (reinterpret_cast<uint32_t *>(smem + a.off_xd))
 #define att (reinterpret_cast<float *>(smem + a.off_att))  /* wo[12][256] | qraw[768] (q_h, k, v) | qs[256] */
-#define xd_s (ps_smem(smem + a.off_xd))
-#define part_s (ps_smem(s_part))
-#define cnt_s (ps_smem(s_cnt))
+#define smem_s (ps_smem(smem))
+#define tmem (s_tmem)
 #define pol (ps_evict_first())
 #define keep (ps_evict_last())
 
@@ -1353,22 +1149,37 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #pragma unroll 1
 		for (int i = 0; i < 8; i++) {
 			ps_mbar_init(&bar_lm[i], 1);
-			ps_mbar_init(&emp_lm[i], PS_NW);
+			ps_mbar_init(&emp_lm[i], 1);
+		}
+#pragma unroll 1
+		for (int i = 0; i < PS_TILES; i++) ps_mbar_init(&bar_m[i], 1);
+#pragma unroll 1
+		for (int i = 0; i < 2; i++) {
+			ps_mbar_init(&acc_full[i], 1);
+			ps_mbar_init(&acc_free[i], 4);
 		}
 		s_abort = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
-	if (tid < PS_NW + 4) s_cnt[tid] = 0;
+	if (warp == 1) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ps_smem(&s_tmem)), "r"(PS_TMEM) : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
+	if (a.lut.size <= PS_LUT)
+#pragma unroll 1
+		for (int i = tid; i < a.lut.size; i += PS_THREADS) reinterpret_cast<float *>(smem + a.off_lut)[i] = a.lut.table[i];
 	{
 		const int *src = reinterpret_cast<const int *>(a.layers);
 		int *dst = reinterpret_cast<int *>(s_ly);
 #pragma unroll 1
 		for (int i = tid; i < L * int(sizeof(PsLayer) / 4); i += PS_THREADS) dst[i] = src[i];
 	}
+	tc_fence_before();
 	__syncthreads();
+	tc_fence_after();
 	const PsW pw{&s_abort, a.err, a.wait_clocks, unsigned(a.poll_ns)};
 	unsigned epoch = 0;  // grid barriers passed
-	uint32_t pA = 0, pC = 0, pD = 0, pE = 0, plm = 0, pemp = 0;
+	uint32_t pA = 0, pC = 0, pD = 0, pE = 0, plm = 0, pemp = 0, pm = 0, acc_n = 0;
 
 	__shared__ PsCta s_c;
 	{
@@ -1388,6 +1199,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			s_c.srcD = a.tiled + a.tl_D + size_t(hD ? uD : 0) * a.Dp.bytes;
 			s_c.srcE = a.tiled + a.tl_E + size_t(hE ? uE : 0) * a.E.bytes;
 			s_c.has = (hA ? 1 : 0) | (hC ? 2 : 0) | (hD ? 4 : 0) | (hE ? 8 : 0);
+		}
+		if (lane == 0) {
+			ps_fill_map(a.A, warp, s_c.ep[0], s_c.xo[0]);
+			ps_fill_map(a.C, warp, s_c.ep[1], s_c.xo[1]);
+			ps_fill_map(a.Dp, warp, s_c.ep[2], s_c.xo[2]);
+			ps_fill_map(a.E, warp, s_c.ep[3], s_c.xo[3]);
 		}
 		__syncthreads();
 	}
@@ -1419,13 +1236,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	const int rbase = __ldcg(a.ring_base);
 	int n_logged = 0;
 	int dbg_n = 0;
-	// this lane's column in a product: group = warp / kp, column 4 * group + lane (lanes 0..3); active = the warp has a group
-	const bool actA = hasA && warp / a.A.kp < a.A.ngroups, actC = hasC && warp / a.C.kp < a.C.ngroups;
-	const bool actD = hasD && warp / a.Dp.kp < a.Dp.ngroups, actE = hasE && warp / a.E.kp < a.E.ngroups;
-	const int colA = tileA * a.A.ngroups * 4 + (warp / a.A.kp) * 4 + (lane & 3);
-	const int colC = tileC * a.C.ngroups * 4 + (warp / a.C.kp) * 4 + (lane & 3);
-	const int colD = uD * a.Dp.ngroups * 4 + (warp / a.Dp.kp) * 4 + (lane & 3);
-	const int colE = tileE * a.E.ngroups * 4 + (warp / a.E.kp) * 4 + (lane & 3);
+	// thread c publishes column c of the CTA's unit: one store instruction per 32 columns. (Scattered over the warps, 16 bytes each,
+	// the words of a line that 148 CTAs poll take 450 clk longer to arrive.)
+	const bool actA = hasA && tid < a.A.ncol, actC = hasC && tid < a.C.ncol, actD = hasD && tid < a.Dp.ncol, actE = hasE && tid < a.E.ncol;
+	const bool iss = (warp & 3) == 0;  // this warp may issue MMAs
+	const int colA = tileA * a.A.ncol + tid, colC = tileC * a.C.ncol + tid, colD = uD * a.Dp.ncol + tid, colE = tileE * a.E.ncol + tid;
 
 	// ring stages of the lm_head that fit the up/gate region and belong to this CTA's first tile (chunks 0 .. lm_pre - 1)
 	const int lm_pre = (cta < a.lm_ntiles && a.sched == 0) ? min(min(a.lm_stages, a.lm_nchunk), a.Dp.bytes / a.lm_stage_bytes) : 0;
@@ -1489,35 +1304,31 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			// here, a phase or more before its use: a DRAM or L2 access issued while a burst of weight copies
 			// lands can take microseconds, and a publishing warp that waits for its scale delays every consumer.
 			float scA = 0.0f, scC = 0.0f, su_r = 0.0f, sg_r = 0.0f, scE = 0.0f;
-			if (lane < 4) {
-				if (actA) {
-					const int n = colA;
-					scA = ps_ldk(n < a.QD ? ly.sq + n : (n < a.QD + a.KD ? ly.sk + (n - a.QD) : ly.sv + (n - a.QD - a.KD)), keep);
-				}
-				if (actC) scC = ps_ldk(ly.so + colC, keep);
-				if (actD) {
-					su_r = ps_ldk(ly.su + colD, keep);
-					sg_r = ps_ldk(ly.sg + colD, keep);
-				}
-				if (actE) scE = ps_ldk(ly.sd + colE, keep);
+			if (actA) {
+				const int n = colA;
+				scA = ps_ldk(n < a.QD ? ly.sq + n : (n < a.QD + a.KD ? ly.sk + (n - a.QD) : ly.sv + (n - a.QD - a.KD)), keep);
 			}
-			if (a.e_rows && hasE && lane < 4 * a.E.ngroups) scE = ps_ldk(ly.sd + tileE * a.E.ngroups * 4 + lane, keep);
+			if (actC) scC = ps_ldk(ly.so + colC, keep);
+			if (actD) {
+				su_r = ps_ldk(ly.su + colD, keep);
+				sg_r = ps_ldk(ly.sg + colD, keep);
+			}
+			if (actE) scE = ps_ldk(ly.sd + colE, keep);
 			// The units were requested a layer ago: test their barriers early, so that the (long) latency of the
 			// test hides behind the hand-off polls instead of following them.
-			const bool rdyA = actA && ps_mbar_test(&bar_A, pA), rdyC = actC && ps_mbar_test(&bar_C, pC);
+			const bool rdyA = iss && hasA && ps_mbar_test(&bar_A, pA), rdyC = iss && hasC && ps_mbar_test(&bar_C, pC);
 			{
-				ps_resnorm(pw, (l << 4) | 1, D, h, xd, bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
+				ps_resnorm(pw, (l << 4) | 1, D, h, ps_x(a.A, smem_s), bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
 				           G - a.E.units, l > 0 ? s_ly[l - 1].mlp_post : nullptr, ly.attn_pre, keep, nullptr);
 				PS_STAMP();
 				PS_GT(1);
 				PS_BEACON(0x11);
-				if (actA) {
-					if (!rdyA) ps_wait_bulk(pw, (l << 4) | 1, &bar_A, pA);
+				if (hasA) {
 					PS_STAMP();
-					const PsOut o = ps_product(ps_smem(R_A), a.A.ngroups, a.A.nq, a.A.kp, a.A.wq, false, xd_s, D / 4, part_s, cnt_s);
-					if ((o.flags & 1) && lane < 4) ps_st(llb + a.ll_qkv + colA, (o.r0 * s_xscale) * scA);
+					pm = ps_product(pw, (l << 4) | 1, ps_mm(a.A, smem_s, ps_smem(R_A)), tmem, &bar_A, pA, rdyA, bar_m, pm, s_c.ep[0], s_c.xo[0]);
+					if (actA) ps_st(llb + a.ll_qkv + colA, (ps_column(a.A, smem_s, tid) * s_xscale) * scA);
 					PS_STAMP();
-					if ((o.flags & 2) && nl >= 0 && lane == 0) ps_issue(R_A, srcA + size_t(nl) * a.tl_layer, a.A.bytes, &bar_A, pol, &s_abort);
+					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_A, srcA + size_t(nl) * a.tl_layer, a.A.bytes, &bar_A, pol, &s_abort);
 				} else {
 					PS_STAMP();
 					PS_STAMP();
@@ -1563,17 +1374,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			{
 				if (hasC) {
 					const int hp = AT_NH / a.C.nsplit;
-					ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, splitC * hp, hp, nch, att, xd, bred, &s_xscale);
+					ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, splitC * hp, hp, nch, att, ps_x(a.C, smem_s), bred, &s_xscale);
 					PS_STAMP();
 					PS_GT(4);
 					PS_BEACON(0x31);
-					if (actC && !rdyC) ps_wait_bulk(pw, (l << 4) | 3, &bar_C, pC);
 					PS_STAMP();
-					const PsOut o = ps_product(ps_smem(R_C), a.C.ngroups, a.C.nq, a.C.kp, a.C.wq, false, xd_s, hp * (AT_HD / 4), part_s, cnt_s);
-					if ((o.flags & 1) && lane < 4) ps_st(llb + a.ll_op + size_t(splitC) * D + colC, (o.r0 * s_xscale) * scC);
-					if (o.flags & 2) PS_GT_WARP(10);
+					pm = ps_product(pw, (l << 4) | 3, ps_mm(a.C, smem_s, ps_smem(R_C)), tmem, &bar_C, pC, rdyC, bar_m, pm, s_c.ep[1], s_c.xo[1]);
+					if (actC) ps_st(llb + a.ll_op + size_t(splitC) * D + colC, (ps_column(a.C, smem_s, tid) * s_xscale) * scC);
 					PS_STAMP();
-					if ((o.flags & 2) && nl >= 0 && lane == 0) ps_issue(R_C, srcC + size_t(nl) * a.tl_layer, a.C.bytes, &bar_C, pol, &s_abort);
+					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_C, srcC + size_t(nl) * a.tl_layer, a.C.bytes, &bar_C, pol, &s_abort);
 				} else {
 					PS_STAMP();
 					PS_STAMP();
@@ -1586,19 +1395,17 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			}
 			// ============================================================ D: up & gate + GeGLU
 			{
-				const bool rdyD = actD && ps_mbar_test(&bar_D, pD);
-				ps_resnorm(pw, (l << 4) | 4, D, h, xd, bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr,
-				           (DBG && a.dbg && cta == a.dbg_cta && !more && l == L / 2) ? a.dbg + 3930 : nullptr);
+				const bool rdyD = iss && hasD && ps_mbar_test(&bar_D, pD);
+				ps_resnorm(pw, (l << 4) | 4, D, h, ps_x(a.Dp, smem_s), bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr);
 				PS_STAMP();
 				PS_GT(6);
 				PS_BEACON(0x41);
-				if (actD && !rdyD) ps_wait_bulk(pw, (l << 4) | 4, &bar_D, pD);
 				PS_STAMP();
 				if (hasD) {
-					const PsOut o = ps_product(ps_smem(R_D), a.Dp.ngroups, a.Dp.nq, a.Dp.kp, a.Dp.wq, true, xd_s, D / 4, part_s, cnt_s);
-					if ((o.flags & 1) && lane < 4) {
-						const float xs = s_xscale;
-						ps_st(llb + a.ll_act + colD, ps_gelu(a.lut, (o.r1 * xs) * sg_r, keep) * ((o.r0 * xs) * su_r));
+					pm = ps_product(pw, (l << 4) | 4, ps_mm(a.Dp, smem_s, ps_smem(R_D)), tmem, &bar_D, pD, rdyD, bar_m, pm, s_c.ep[2], s_c.xo[2]);
+					if (actD) {
+						const float xs = s_xscale, u = ps_column(a.Dp, smem_s, tid), g = ps_column(a.Dp, smem_s, a.Dp.ncol + tid);
+						ps_st(llb + a.ll_act + colD, ps_gelu(a.lut, (g * xs) * sg_r, smem_s + uint32_t(a.off_lut), keep) * ((u * xs) * su_r));
 					}
 				}
 				pD ^= 1;
@@ -1608,35 +1415,13 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			}
 			// ============================================================ E: down projection
 			{
-				const bool rdyE = hasE && ps_mbar_test(&bar_E, pE);
-				if (a.e_rows && hasE) {
-					// no prologue: every warp polls and quantises its own rows inside the product
-					PS_STAMP();
-					PS_GT(8);
-					PS_BEACON(0x51);
-					if (!rdyE) ps_wait_bulk(pw, (l << 4) | 5, &bar_E, pE);
-					PS_STAMP();
-					const PsOut o = ps_product_rows(pw, (l << 4) | 5, ps_smem(R_E), a.E.ngroups, a.E.nq, a.e_wq, llb + a.ll_act + size_t(splitE) * a.E.nq * 4,
-					                                part_s, cnt_s + 4u * (PS_NW + 2),
-					                                (DBG && a.dbg && cta == a.dbg_cta && !more && l == L / 2) ? a.dbg + 3800 : nullptr);
-					if ((o.flags & 1) && lane < 4 * a.E.ngroups && cta != a.fault_cta)
-						ps_st(llb + a.ll_dn + size_t(splitE) * D + tileE * a.E.ngroups * 4 + lane, o.r0 * scE);
-					if (o.flags & 2) PS_GT_WARP(11);
-					PS_STAMP();
-					// every warp has left the up/gate product and this one: both regions are free
-					if (a.sched == 0 && (o.flags & 2) && l + 1 < L && lane == 0) {
-						ps_issue(R_E, srcE + size_t(l + 1) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
-						if (hasD) ps_issue(R_D, srcD + size_t(l + 1) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
-					}
-				} else {
+				const bool rdyE = iss && hasE && ps_mbar_test(&bar_E, pE);
 				if (hasE) {
-					ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(splitE) * a.E.nq * 4, a.E.nq, xd, bred, &s_xscale);
-				} else {
-					__syncthreads();  // every warp has left the up/gate product
+					ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(splitE) * a.E.nq * 4, a.E.nq, ps_x(a.E, smem_s), bred, &s_xscale);
 				}
 				// the up/gate region is free: request the next layer's unit now that the hand-off loads are done
-				if (a.sched == 0 && tid == 32 && hasD && l + 1 < L) ps_issue(R_D, srcD + size_t(l + 1) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
-				if (tid == 32 && l + 1 == L) {
+				if (a.sched == 0 && tid == PS_THREADS - 32 && hasD && l + 1 < L) ps_issue(R_D, srcD + size_t(l + 1) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
+				if (tid == PS_THREADS - 32 && l + 1 == L) {
 					// last layer: the up/gate region is idle until the lm_head, whose ring starts there. Its first stages
 					// are requested now, so that they land under the down projection and the final norm.
 #pragma unroll 1
@@ -1648,18 +1433,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 				PS_GT(8);
 				PS_BEACON(0x51);
 				if (hasE) {
-					if (actE && !rdyE) ps_wait_bulk(pw, (l << 4) | 5, &bar_E, pE);
 					PS_STAMP();
-					const PsOut o = ps_product(ps_smem(R_E), a.E.ngroups, a.E.nq, a.E.kp, a.E.wq, false, xd_s, a.E.nq, part_s, cnt_s);
-					if ((o.flags & 1) && lane < 4 && cta != a.fault_cta) ps_st(llb + a.ll_dn + size_t(splitE) * D + colE, (o.r0 * s_xscale) * scE);
-					if (o.flags & 2) PS_GT_WARP(11);
+					pm = ps_product(pw, (l << 4) | 5, ps_mm(a.E, smem_s, ps_smem(R_E)), tmem, &bar_E, pE, rdyE, bar_m, pm, s_c.ep[3], s_c.xo[3]);
+					if (actE && cta != a.fault_cta) ps_st(llb + a.ll_dn + size_t(splitE) * D + colE, (ps_column(a.E, smem_s, tid) * s_xscale) * scE);
 					PS_STAMP();
-					if (a.sched == 0 && (o.flags & 2) && l + 1 < L && lane == 0) ps_issue(R_E, srcE + size_t(l + 1) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
+					if (a.sched == 0 && l + 1 < L && tid == PS_THREADS - 64) ps_issue(R_E, srcE + size_t(l + 1) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
 				} else {
 					if (tid == 0) ps_st(llb + a.ll_pres + presE, 0.0f);
 					PS_STAMP();
 					PS_STAMP();
-				}
 				}
 				pE ^= 1;
 				PS_STAMP();
@@ -1669,18 +1451,17 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		}
 
 		// ================================================================ lm_head
-		// logits[v] = lm_scale[v] * sum_k x[k] W[k,v]; this CTA takes column tiles cta, cta + G, ...;
-		// a tile arrives as lm_nchunk ring stages laid over the (now idle) up/gate and down regions;
-		// warp w owns column groups 2w and 2w + 1 of every tile over all of its rows.
+		// (its ring lies over the now idle up/gate and down regions)
 		const int lc = step * L + L;
 		{
 			float *const lllast = a.ll + size_t((lc + 2) % 3) * a.ll_stride;
-			ps_resnorm(pw, (L << 4) | 6, D, h, xd, bred, &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
+			ps_resnorm(pw, (L << 4) | 6, D, h, ps_x(a.lm, smem_s), bred, &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
 			           s_ly[L - 1].mlp_post, a.final_norm, keep, cta == 0 ? a.xnorm_out : nullptr);
 		}
 		PS_STAMP();
 		PS_BEACON(0x61);
-		const PsLmOut lo = ps_lm_head(a, pw, R_D, xd, s_xscale, bar_lm, emp_lm, plm, pemp, pol, keep, lm_pre);
+		const PsLmOut lo = ps_lm_head(a, pw, R_D, smem_s, s_xscale, tmem, bar_lm, emp_lm, acc_full, acc_free, plm, pemp, acc_n, pol, keep, lm_pre);
+		acc_n += (a.lm_ntiles - cta + G - 1) / G;
 		plm = lo.plm;
 		pemp = lo.pemp;
 		__syncthreads();
@@ -1711,6 +1492,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		}
 		__syncthreads();
 	}
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 1) {
+		tc_fence_after();
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PS_TMEM) : "memory");
+	}
 	if (cta == 0 && tid == 0 && a.log_count) *a.log_count = n_logged;
 	// Leave the hand-off arena as the next launch expects it: copy 0 empty (copies 1 and 2 are wiped during
 	// its layers 0 and 1, like every copy a layer before its use). Every CTA is past the last token's grid
@@ -1723,11 +1510,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		for (int i = cta * per + tid; i < min(n4, (cta + 1) * per); i += PS_THREADS) __stcg(c0 + i, make_float4(e, e, e, e));
 	}
 #undef h
-#undef xd
 #undef att
-#undef xd_s
-#undef part_s
-#undef cnt_s
+#undef smem_s
+#undef tmem
 #undef pol
 #undef keep
 #undef R_A

@@ -1125,38 +1125,7 @@ int ensure_decode_tiles(tg_state *s) {
 }
 
 
-// ---------------------------------------------------------------- dp4a persistent decode kernel
-// Plan of one phase: column groups per unit, K-splits across CTAs and warps per group, chosen by an
-// estimate of the phase's time in clocks: the tile product (measured: about 650 clk fixed + 1 clk per
-// 55 bytes, 65 with two matrices that share the activations) plus the bytes the phase makes CTAs poll
-// (measured: about 76 clk per KB and CTA). `poll_kb(nsplit)` gives those KB for a split.
-template <class F>
-bool ps_plan(PsPhase *out, int K, int N, int nmat, int G, int max_bytes, const std::vector<int> &splits,
-             const std::vector<int> &col_blocks, int max_nq, F poll_kb) {
-	double best = 1e30;
-	for (int ns : splits) {
-		if ((K / 4) % ns) continue;
-		const int nq = K / 4 / ns;
-		if (nq > max_nq) continue;
-		for (int ng = 1; ng <= PS_NW; ng++) {
-			bool ok = (N / 4) % ng == 0;
-			for (int cb : col_blocks) ok = ok && (cb / 4) % ng == 0;  // a tile never straddles two matrices
-			if (!ok) continue;
-			const int ntiles = N / 4 / ng, units = ntiles * ns;
-			if (units > G) continue;
-			const int bytes = nmat * ng * nq * 16;
-			if (bytes > max_bytes) continue;
-			const int kp = std::max(1, std::min(PS_NW / ng, (nq + 31) / 32));
-			const double cost = 650.0 + double(bytes) / (nmat == 2 ? 65.0 : 55.0) + 76.0 * poll_kb(ns);
-			if (cost < best) {
-				best = cost;
-				*out = PsPhase{ng, nq, ns, ntiles, units, kp, (nq + kp - 1) / kp, bytes, 0};
-			}
-		}
-	}
-	return best < 1e30;
-}
-
+// ---------------------------------------------------------------- persistent decode kernel
 int persist_setup(tg_state *s) {
 	tg_model *m = s->m;
 	const tg_config &c = m->cfg;
@@ -1167,7 +1136,7 @@ int persist_setup(tg_state *s) {
 	const int G = s->mega_grid;
 	PsArgs &a = s->ps;
 	a = PsArgs{};
-	if (c.n_head != AT_NH || c.head_dim != AT_HD || c.n_kv != 1 || D % 4 || I % 4 || D > 4 * PS_THREADS || L > PS_MAX_LAYERS)
+	if (c.n_head != AT_NH || c.head_dim != AT_HD || c.n_kv != 1 || D % 32 || I % 32 || V % 128 || D > 4 * PS_THREADS || L > PS_MAX_LAYERS)
 		return fail(TG_ESHAPE, "persistent kernel: unsupported shape");
 	const int budget = smem_max - 48 * 1024;
 	const double dkb = D * 4 / 1024.0;
@@ -1189,43 +1158,65 @@ int persist_setup(tg_state *s) {
 	a.slots_local = c.n_pos_local;
 	const int npres = G - a.E.units;
 	if (D / 4 + npres > PS_THREADS || G < 16) return fail(TG_ESHAPE, "persistent kernel: grid too small for the down-projection plan");
-	// lm_head: tiles of 24 column groups (two per warp); ring stages of at most ~40 KB
-	a.lm_groups = 2 * PS_NW;
-	a.lm_cq = D / 4;
-	for (int n = 1; n <= 16; n++)
-		if ((D / 4) % n == 0 && a.lm_groups * (D / 4 / n) * 16 <= 40 * 1024) {
-			a.lm_cq = D / 4 / n;
-			break;
-		}
-	a.lm_nchunk = D / 4 / a.lm_cq;
-	a.lm_ntiles = (V + a.lm_groups * 4 - 1) / (a.lm_groups * 4);
-	a.lm_stage_bytes = a.lm_groups * a.lm_cq * 16;
+	// lm_head: tiles of 128 columns; ring stages of at most 40 KB
+	a.lm = PsPhase{};
+	a.lm.ncol = a.lm.rows = a.lm.mt = 128;
+	a.lm.nmat = a.lm.nsplit = a.lm.segs = a.lm.tiles = 1;
+	a.lm.ntiles = a.lm.units = a.lm_ntiles = V / 128;
+	a.lm.nq = a.lm.seg_q = D / 4;
+	a.lm.steps = D / 32;
+	a.lm.bytes = 128 * D;
+	a.lm.seg_mul = 0;  // (one segment)
+	a.lm.x_sbo = 0;    // (digit rows 8 to 15 of an MMA repeat 0 to 7; only 0 to 3 count)
+	a.lm.x_bytes = D / 16 * PS_XCH;
+	a.lm_nchunk = 1;
+	while (a.lm_nchunk < D / 32 && ((D / 32) % a.lm_nchunk || 128 * D / a.lm_nchunk > 40 * 1024)) a.lm_nchunk++;
+	a.lm_steps = D / 32 / a.lm_nchunk;
+	a.lm_stage_bytes = 128 * 32 * a.lm_steps;
 	auto up = [](int v) { return (v + 127) & ~127; };
 	int off = 0;
+	a.off_h = off;
+	off = up(off + D * 4);
+	// Scratch of the phases, one region: the attention's (16 KB), digits and column sums of the products. A phase's digits may take
+	// the place of what the phase before last left; its column sums, which are read behind the product's last barrier, lie
+	// apart from what the next phase writes before its first one (the attention's q|k|v, the merge's rows).
+	constexpr int ATT = (PS_NW * AT_HD + 4 * AT_HD) * 4, QKV_AT = PS_NW * AT_HD * 4;
+	a.off_att = off;
+	auto acc_bytes = [](const PsPhase &ph) { return ph.rows * ph.segs * 16; };
+	auto behind = [&](PsPhase &ph, int x_at) {  // digits at x_at, column sums behind them
+		ph.off_x = a.off_att + x_at;
+		ph.off_acc = up(ph.off_x + ph.x_bytes);
+		return ph.off_acc + acc_bytes(ph);
+	};
+	int end = off + ATT;
+	if (behind(a.A, 0) > a.off_att + QKV_AT) return fail(TG_ESHAPE, "persistent kernel: q|k|v plan does not fit the scratch");
+	end = std::max(end, behind(a.Dp, 0));
+	end = std::max(end, behind(a.E, 0));
+	end = std::max(end, behind(a.C, ATT));
+	a.lm.off_x = a.off_att;
+	end = std::max(end, a.off_att + a.lm.x_bytes);
+	off = up(end);
+	a.off_lut = off;
+	off = up(off + PS_LUT * 4);
 	a.off_A = off;
 	off = up(off + a.A.bytes);
 	a.off_C = off;
 	off = up(off + a.C.bytes);
 	a.off_D = off;
 	a.off_E = off + a.Dp.bytes;  // contiguous with the up/gate region: the lm_head ring and the sampler staging overlay both
-	const int region = std::max(std::max(a.Dp.bytes + a.E.bytes, 3072 * 4), std::min(3 * a.lm_stage_bytes, smem_max / 2));
+	cudaFuncAttributes fa{};
+	TG_CUDA(cudaFuncGetAttributes(&fa, decode_persist_kernel<true>));
+	// the ring takes five stages where the shared memory has room for them (4 at 1B: its units fill the memory)
+	const int room = smem_max - int(fa.sharedSizeBytes) - 128 - off;
+	const int region = std::max(std::max(a.Dp.bytes + a.E.bytes, 3072 * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
 	off = up(off + region);
 	a.lm_stages = std::min(8, region / a.lm_stage_bytes);
 	if (a.lm_stages < 2) return fail(TG_ESHAPE, "persistent kernel: lm_head ring does not fit");
-	a.off_h = off;
-	off = up(off + D * 4);
-	a.xd_words = std::max(std::max(D / 4, a.E.nq), qd / 4);
-	a.off_xd = off;
-	off = up(off + 3 * a.xd_words * 4);
-	a.off_att = off;
-	off = up(off + (PS_NW * AT_HD + 4 * AT_HD) * 4);
 	a.smem_total = off + 128;
 	{
 		const int region_floats = region / 4;
 		if (minp_grid_floats(V, G) > region_floats) return fail(TG_ESHAPE, "persistent kernel: sampler staging does not fit");
 	}
-	cudaFuncAttributes fa{};
-	TG_CUDA(cudaFuncGetAttributes(&fa, decode_persist_kernel<true>));
 	if (a.smem_total + int(fa.sharedSizeBytes) > smem_max) return fail(TG_ESHAPE, "persistent kernel does not fit in shared memory");
 
 	std::vector<PsLayer> lys(L);
@@ -1301,11 +1292,11 @@ int persist_setup(tg_state *s) {
 	s->ps_ok = true;
 	if (env_int("TG_MEGA_VERBOSE", 0))
 		fprintf(stderr,
-		        "[tg] persist plan: A %dg x%d nq%d kp%d (%d units)  C %dg x%d nq%d kp%d (%d)  D %dg nq%d kp%d (%d)  E %dg x%d nq%d kp%d (%d)  "
-		        "lm cq %d x%d stages %d  smem %d + %d B  grid %d\n",
-		        a.A.ngroups, a.A.nsplit, a.A.nq, a.A.kp, a.A.units, a.C.ngroups, a.C.nsplit, a.C.nq, a.C.kp, a.C.units, a.Dp.ngroups,
-		        a.Dp.nq, a.Dp.kp, a.Dp.units, a.E.ngroups, a.E.nsplit, a.E.nq, a.E.kp, a.E.units, a.lm_cq, a.lm_nchunk, a.lm_stages,
-		        a.smem_total, int(fa.sharedSizeBytes), G);
+		        "[tg] persist plan (columns x splits, segments, tiles of rows x MMAs, units): A %dx%d %d %dx%dx%d (%d)  C %dx%d %d %dx%dx%d (%d)  D %d %d %dx%dx%d (%d)  "
+		        "E %dx%d %d %dx%dx%d (%d)  lm steps %d x%d stages %d  smem %d + %d B  grid %d\n",
+		        a.A.ncol, a.A.nsplit, a.A.segs, a.A.tiles, a.A.mt, a.A.steps, a.A.units, a.C.ncol, a.C.nsplit, a.C.segs, a.C.tiles, a.C.mt, a.C.steps, a.C.units,
+		        a.Dp.ncol, a.Dp.segs, a.Dp.tiles, a.Dp.mt, a.Dp.steps, a.Dp.units, a.E.ncol, a.E.nsplit, a.E.segs, a.E.tiles, a.E.mt, a.E.steps, a.E.units,
+		        a.lm_steps, a.lm_nchunk, a.lm_stages, a.smem_total, int(fa.sharedSizeBytes), G);
 	return TG_OK;
 }
 
@@ -1319,11 +1310,11 @@ int ensure_persist_tiles(tg_state *s) {
 	const tg_config &c = m->cfg;
 	const int L = c.n_layers, V = c.n_vocab;
 	const int qd = c.n_head * c.head_dim, kd = c.n_kv * c.head_dim;
-	const int key[20] = {a.A.ngroups, a.A.nsplit, a.A.nq, a.C.ngroups, a.C.nsplit, a.C.nq, a.Dp.ngroups, a.Dp.nq, a.E.ngroups, a.E.nsplit,
-	                     a.E.nq,      a.lm_groups, a.lm_cq, a.lm_ntiles, L, a.D, a.I, V, 0, 0};
+	const int key[20] = {a.A.ncol, a.A.nsplit, a.A.segs, a.A.mt, a.C.ncol, a.C.nsplit, a.C.segs, a.C.mt, a.Dp.ncol, a.Dp.segs,
+	                     a.Dp.mt,  a.E.ncol,   a.E.nsplit, a.E.segs, a.E.mt, L,      a.D,        a.I,      V,       a.lm_stage_bytes};
 	if (m->ps_tiled && m->ps_tiled_version == m->weights_version && std::memcmp(key, m->ps_tiled_key, sizeof key) == 0) return TG_OK;
 	const size_t bytes = a.tl_layer * L;
-	const size_t lm_bytes = size_t(a.lm_ntiles) * a.lm_nchunk * a.lm_stage_bytes;
+	const size_t lm_bytes = size_t(V) * a.D;
 	if (m->ps_tiled_bytes != bytes) {
 		cudaFree(m->ps_tiled);
 		m->ps_tiled = nullptr;
@@ -1337,24 +1328,22 @@ int ensure_persist_tiles(tg_state *s) {
 		m->ps_lm_bytes = lm_bytes;
 	}
 	cudaStream_t st = s->stream;
-	auto run = [&](int8_t *dst, const QW &w, const PsPhase &ph, int tile0, size_t dst_off) {
-		retile_quads_kernel<<<4 * g_num_sms, 256, 0, st>>>(dst, w.q, w.N, ph.ngroups, ph.nq, ph.nsplit, ph.ntiles, tile0,
-		                                                   w.N / 4 / ph.ngroups, size_t(ph.bytes), dst_off);
+	auto run = [&](int8_t *dst, const QW &w, const PsPhase &ph, int tile0, int row0) {
+		retile_units_kernel<<<8 * g_num_sms, 256, 0, st>>>(dst, w.q, w.N, ph, tile0, w.N / ph.ncol, row0);
 		count_launch();
 	};
 	for (int l = 0; l < L; l++) {
 		const LayerW &w = m->layers[l];
 		int8_t *base = m->ps_tiled + size_t(l) * a.tl_layer;
 		run(base + a.tl_A, w.Q, a.A, 0, 0);
-		run(base + a.tl_A, w.K, a.A, qd / 4 / a.A.ngroups, 0);
-		run(base + a.tl_A, w.V, a.A, (qd + kd) / 4 / a.A.ngroups, 0);
+		run(base + a.tl_A, w.K, a.A, qd / a.A.ncol, 0);
+		run(base + a.tl_A, w.V, a.A, (qd + kd) / a.A.ncol, 0);
 		run(base + a.tl_C, w.O, a.C, 0, 0);
 		run(base + a.tl_D, w.U, a.Dp, 0, 0);
-		run(base + a.tl_D, w.G, a.Dp, 0, size_t(a.Dp.ngroups) * a.Dp.nq * 16);
+		run(base + a.tl_D, w.G, a.Dp, 0, a.Dp.ncol);
 		run(base + a.tl_E, w.Dn, a.E, 0, 0);
 	}
-	retile_lm_kernel<<<8 * g_num_sms, 256, 0, st>>>(m->ps_lm, m->lm_head.q, V, a.lm_groups, a.lm_cq, a.lm_nchunk, a.lm_ntiles);
-	count_launch();
+	run(m->ps_lm, m->lm_head, a.lm, 0, 0);
 	TG_TRY(check_launch("retile"));
 	std::memcpy(m->ps_tiled_key, key, sizeof key);
 	TG_CUDA(cudaStreamSynchronize(st));  // (once per load) the copies are the model's: other states read them on their own streams
@@ -1388,8 +1377,6 @@ int persist_launch(tg_state *s, int n_steps, int sampler, float minp, float temp
 	a.dbg_cta = std::min(std::max(env_int("TG_MEGA_DBG_CTA", 0), 0), s->mega_grid - 1);
 	a.wait_clocks = (long long)(std::max(1, env_int("TG_PS_WAIT_MS", 100))) * 2000000ll;  // ~2 GHz
 	a.fault_cta = env_int("TG_PS_WITHHOLD_CTA", -1);
-	a.e_wq = (a.E.nq + PS_NW - 1) / PS_NW;
-	a.e_rows = (env_int("TG_PS_E_ROWS", 0) && a.E.ngroups <= 4 && a.e_wq <= 96) ? 1 : 0;
 	a.poll_ns = std::max(0, env_int("TG_PS_POLL_NS", 20));
 	a.sched = env_int("TG_PS_SCHED", 0);
 	a.gt = (s->mg_dbg && env_int("TG_PS_GT", 0)) ? s->mg_dbg + 2048 : nullptr;  // (the stamp recorder uses < 600 entries)
