@@ -16,8 +16,10 @@ static uint32_t rnd() { return g_seed = g_seed * 1664525u + 1013904223u, g_seed 
 
 static bool unit_ok(const PsPhase &ph) {
 	const int K = 4 * ph.nq, ks = K / ph.segs;
-	std::vector<int8_t> W(size_t(K) * ph.rows), unit(size_t(ph.bytes)), x(size_t(ph.x_bytes));
-	std::vector<char> seen(size_t(ph.bytes), 0);
+	const size_t weights = size_t(ph.rows) * K;
+	if (size_t(ph.bytes) != weights + 4 * ph.rows || ph.bytes % 16) return false;  // (the columns' scales follow)
+	std::vector<int8_t> W(weights), unit(weights), x(size_t(ph.x_bytes));
+	std::vector<char> seen(weights, 0);
 	std::vector<int32_t> v(K);
 	for (auto &w : W) w = int8_t(int(rnd() % 255) - 127);
 	for (auto &b : x) b = int8_t(rnd());  // (what no digit is written to must not count)
@@ -27,7 +29,7 @@ static bool unit_ok(const PsPhase &ph) {
 	for (int c = 0; c < ph.rows; c++)
 		for (int k = 0; k < K; k++) {
 			const int seg = k / ks, o = ps_unit_offset(ph, c, seg, k % ks / 16) + k % 16;
-			if (o < 0 || o >= ph.bytes || seen[o]) return false;
+			if (o < 0 || size_t(o) >= weights || seen[o]) return false;
 			if (c % 4 == 0 && ps_unit_offset(ph, c + 3, seg, k % ks / 16) != o - k % 16 + 48) return false;  // (4 columns are stored together)
 			seen[o] = 1;
 			unit[o] = W[size_t(k) * ph.rows + c];
@@ -52,7 +54,7 @@ static bool unit_ok(const PsPhase &ph) {
 					for (int k = 0; k < 32; k++) {
 						const int ao = a0 + i * ph.mt * 32 + (k / 16) * ph.mt * 16 + (m / 8) * 128 + (m % 8) * 16 + k % 16;
 						const int xo = x0 + i * 2 * PS_XCH + (k / 16) * PS_XCH + (n / 8) * ph.x_sbo + (n % 8) * 16 + k % 16;
-						if (ao >= ph.bytes || xo >= ph.x_bytes) return false;
+						if (size_t(ao) >= weights || xo >= ph.x_bytes) return false;
 						D[m * 16 + n] += int(unit[ao]) * int(x[xo]);
 					}
 		for (int w = 4 * t; w < 4 * t + 4; w++) {
@@ -98,7 +100,7 @@ int main(int argc, char **argv) {
 				ph.nmat = nmat;
 				ph.rows = nmat * ncol;
 				ph.nq = nq;
-				ph.bytes = ph.rows * nq * 4;
+				ph.bytes = ph.rows * nq * 4 + ph.rows * 4;
 				if (ps_mma_plan(&ph) >= 0) run(ph, "shape");
 			}
 	for (int i = 1; i + 1 < argc; i += 2)

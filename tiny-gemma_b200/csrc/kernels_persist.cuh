@@ -69,6 +69,11 @@ struct PsLayer {
 	int slots, is_local;
 };
 
+// where a token stands in the caches of the sliding-window or of the global layers
+struct PsSpan {
+	int p, slot, valid;  // position, slot of its row, rows to attend to
+	int nch, chunk;      // cache chunks per head, rows of a chunk
+};
 struct PsArgs {
 	const int8_t *tiled;  // re-tiled layer weights: per layer [A units | C units | D units (up, gate) | E units]
 	size_t tl_layer, tl_A, tl_C, tl_D, tl_E;
@@ -95,8 +100,9 @@ struct PsArgs {
 	//                                      one presence word for every CTA without a down unit
 	float *ll;
 	int ll_stride, ll_qkv, ll_att, ll_op, ll_act, ll_dn, ll_pres;
+	int merge_heads;  // heads whose attention output an O unit multiplies (4 / C.nsplit)
 	int nch_max, nch_local, nch_global;  // cache chunks per head: at most; a number given for sliding-window and global layers (0: by rule)
-	int slots_local;
+	int slots_local, slots_global;
 	float *logits;
 	float *probs;
 	float *samp_f;
@@ -293,26 +299,35 @@ __device__ __forceinline__ float ps_ldsf(uint32_t addr) {
 __device__ __forceinline__ void ps_stsf(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
 // ------------------------------------------------------------------ quantised activations
-// A vector x[0..4 nq) becomes the digits of round(x * 2^(30 - e)), 2^e > max |x|: q = d0 + 256 d1 + 65536 d2 + 2^24 d3 with
-// d_i in [-128, 127] (the digits of the prefill's GEMM). PsX: where a phase keeps them.
-struct PsX {
-	uint32_t base;  // shared-window address
-	unsigned seg_mul;
-	int seg_q, sbo;
+// What a phase's unit fixes for the whole launch, in shared memory: a field read from the kernel's arguments costs a
+// constant-cache miss where a layer's code has passed through the caches since, and a value kept in a register across the calls
+// of a layer is spilled.
+struct PsUnit {
+	uint64_t da[PS_TILES], db[PS_TILES];  // descriptors of a tile's first MMA: weights, digits
+	uint32_t id;
+	int tiles, steps, mt;
+	uint32_t x_s, seg_mul;  // digits: shared-window address and layout
+	int seg_q, x_sbo;
+	uint32_t acc_s, scale_s;  // column sums, column scales (behind the unit's weights)
+	int rows, segs, ncol, two;
+	int dst;           // where the unit's columns go in a copy of the hand-off arena
+	int ep[PS_NW];     // per warp: accumulator column | (first entry of the column sums) << 8
 };
-__device__ __forceinline__ PsX ps_x(const PsPhase &ph, uint32_t smem_s) { return PsX{smem_s + uint32_t(ph.off_x), ph.seg_mul, ph.seg_q, ph.x_sbo}; }
+// A vector x[0..4 nq) becomes the digits of round(x * 2^(30 - e)), 2^e > max |x|: q = d0 + 256 d1 + 65536 d2 + 2^24 d3 with
+// d_i in [-128, 127] (the digits of the prefill's GEMM).
+__device__ __forceinline__ uint32_t ps_xaddr(const PsUnit *u, int q) { return u->x_s + uint32_t(ps_digit_offset(u->seg_mul, u->seg_q, u->x_sbo, q)); }
 // exponent for a bound on max |x| (clamped so that both scale factors are normal floats); a vector with an infinity gives NaN
 __device__ __forceinline__ int ps_exponent(float bound) { return max(-96, min(100, (int(__float_as_uint(bound) >> 23) & 0xFF) - 126)); }
 __device__ __forceinline__ float ps_pow2(int e) { return __uint_as_float(uint32_t(e + 127) << 23); }
 __device__ __forceinline__ float ps_qmul(float M) { return ps_pow2(30 - ps_exponent(M * 1.000001f)); }
 __device__ __forceinline__ float ps_qscale(float M) { return M < INFINITY ? ps_pow2(ps_exponent(M * 1.000001f) - 30) : __uint_as_float(0x7FC00000u); }
 __device__ __forceinline__ void ps_sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
-// quad q of the vector. (Lanes of a warp hold consecutive quads: four words of a 16-byte chunk, chunks 36 words apart: no bank conflict.)
-__device__ __forceinline__ void ps_quantise(float4 y, float mul, const PsX &x, int q) {
+// four elements at p = ps_xaddr(u, quad). (Lanes of a warp hold consecutive quads: four words of a 16-byte chunk, chunks 36 words
+// apart: no bank conflict.)
+__device__ __forceinline__ void ps_quantise(float4 y, float mul, uint32_t p) {
 	const uint32_t a = i8_digits(y.x, mul), b = i8_digits(y.y, mul), c = i8_digits(y.z, mul), d = i8_digits(y.w, mul);
 	const uint32_t ab01 = __byte_perm(a, b, 0x5140), ab23 = __byte_perm(a, b, 0x7362);
 	const uint32_t cd01 = __byte_perm(c, d, 0x5140), cd23 = __byte_perm(c, d, 0x7362);
-	const uint32_t p = x.base + uint32_t(ps_digit_offset(x.seg_mul, x.seg_q, x.sbo, q));
 	ps_sts32(p, __byte_perm(ab01, cd01, 0x5410));
 	ps_sts32(p + 16, __byte_perm(ab01, cd01, 0x7632));
 	ps_sts32(p + 32, __byte_perm(ab23, cd23, 0x5410));
@@ -370,73 +385,48 @@ __device__ __forceinline__ float ps_join(const int4 &s) {
 // what a CTA's place in the grid fixes for the whole launch (kept in shared memory, read where it is used)
 struct PsCta {
 	const int8_t *srcA, *srcC, *srcD, *srcE;
-	int tileA, tileC, splitC, tileE, splitE, presE, uD, has;
-	// per phase and warp: accumulator column | (first entry of the column sums) << 8; per phase and tile: byte offset of its digits
-	int ep[4][PS_NW], xo[4][PS_TILES];
+	int splitC, splitE, presE, has;
+	uint32_t tm;  // TMEM base (the word that tcgen05.alloc wrote, which the compiler does not see written: read once, volatile)
 };
-__device__ __forceinline__ void ps_fill_map(const PsPhase &ph, int warp, int *ep, int *xo) {
+// fields of a phase's entry; `warp` fills its own
+__device__ __forceinline__ void ps_fill_unit(const PsPhase &ph, PsUnit *u, int warp, uint32_t smem_s, int off_tile, int dst) {
 	const int t = warp >> 2;
-	if (t >= ph.tiles) return;
-	int r0, col;
-	ps_warp_rows(ph, warp, r0, col);
-	ep[warp] = (16 * t + col) | (r0 << 8);
-	xo[t] = (ps_tile_segment(ph.rows, ph.mt, t) / 2) * ph.x_sbo;
-}
-// Integer sums of a unit's columns: entry s * rows + c of the int4 array at ph.off_acc = digit sums of column c over segment s.
-// Called by the whole CTA behind the barrier that ends the prologue (the digits' writers have fenced). Warp 4 t issues tile
-// t's MMAs into its own 16 TMEM columns (one accumulator per issuing warp), warps 4 t .. 4 t + 3 read them back. bar_w, pw,
-// rdy: barrier of the unit's bulk copy; pm: parity of bar_m[t]. Behind the closing barrier nobody reads the unit or the digits
-// any more. Measured from the prologue's barrier to the values in registers (1B: 27 MMAs of up and gate, 27 of down, 4 of O, 9
-// of q|k|v): about 430 clk + 38 per MMA of 128 rows, 23 per one of 64; the dp4a loops over the same tiles took 2400, 1450,
-// 850 and 1000 clk and 400 to 600 more to reduce over the lanes.
-struct PsMm {  // what a product needs of its phase (by value: a reference to the kernel's arguments would be a generic pointer)
-	int tiles, mt, steps, x_sbo;
-	uint32_t x_s, acc_s, tile_s;
-};
-__device__ __forceinline__ PsMm ps_mm(const PsPhase &ph, uint32_t smem_s, uint32_t tile_s) {
-	return PsMm{ph.tiles, ph.mt, ph.steps, ph.x_sbo, smem_s + uint32_t(ph.off_x), smem_s + uint32_t(ph.off_acc), tile_s};
-}
-__device__ __noinline__ uint32_t ps_product(const PsW w, int where, const PsMm ph, uint32_t tmem, uint64_t *bar_w, uint32_t pw, bool rdy, uint64_t *bar_m,
-                                            uint32_t pm, const int *ep, const int *xo) {
-	__builtin_assume(__isShared(ep));
-	__builtin_assume(__isShared(xo));
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = warp >> 2;
 	if (t < ph.tiles) {
-		if ((warp & 3) == 0) {
-			if (!rdy) ps_wait_bulk(w, where, bar_w, pw);
-			__syncwarp();
-			tc_fence_after();
-			const int mt = ph.mt, steps = ph.steps;
-			const uint64_t da = ps_desc(ph.tile_s + uint32_t(t * steps * mt) * 32u, mt * 16, 128), db = ps_desc(ph.x_s + uint32_t(xo[t]), PS_XCH, ph.x_sbo);
-			const uint32_t id = ps_idesc(mt), d = tmem + 16u * t;
-			if (tc_elect()) {
-#pragma unroll 1
-				for (int i = 0; i < steps; i++) i8_mma<1>(d, da + uint64_t(i * mt * 2), db + uint64_t(i * (2 * PS_XCH / 16)), id, i > 0 ? 1u : 0u);
-				i8_commit<1>(&bar_m[t]);
-			}
-			__syncwarp();
-		}
-		const int m = ep[warp];
-		ps_wait_bulk(w, where, &bar_m[t], pm);
-		pm ^= 1u;
-		__syncwarp();
-		tc_fence_after();
-		const int4 v = ps_tmem_ld4(tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m & 0xFF));
-		if (4 * lane < ph.mt)
-			asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(ph.acc_s + 16u * uint32_t((m >> 8) + lane)), "r"(v.x), "r"(v.y),
-			             "r"(v.z), "r"(v.w)
-			             : "memory");
-		tc_fence_before();
+		int r0, col;
+		ps_warp_rows(ph, warp, r0, col);
+		u->ep[warp] = (16 * t + col) | (r0 << 8);
 	}
-	__syncthreads();
-	return pm;
+	if (warp == 0) {
+#pragma unroll
+		for (int i = 0; i < PS_TILES; i++) {
+			u->da[i] = ps_desc(smem_s + uint32_t(off_tile + i * ph.steps * ph.mt * 32), ph.mt * 16, 128);
+			u->db[i] = ps_desc(smem_s + uint32_t(ph.off_x + (ps_tile_segment(ph.rows, ph.mt, i) / 2) * ph.x_sbo), PS_XCH, ph.x_sbo);
+		}
+		u->id = ps_idesc(ph.mt);
+		u->tiles = ph.tiles;
+		u->steps = ph.steps;
+		u->mt = ph.mt;
+		u->x_s = smem_s + uint32_t(ph.off_x);
+		u->seg_mul = ph.seg_mul;
+		u->seg_q = ph.seg_q;
+		u->x_sbo = ph.x_sbo;
+		u->acc_s = smem_s + uint32_t(ph.off_acc);
+		u->scale_s = smem_s + uint32_t(off_tile + ph.rows * ph.nq * 4);
+		u->rows = ph.rows;
+		u->segs = ph.segs;
+		u->ncol = ph.ncol;
+		u->two = ph.nmat == 2;
+		u->dst = dst;
+	}
 }
 // column c of a unit: the segments' digit sums added (exact) and joined
-__device__ __forceinline__ float ps_column(const PsPhase &ph, uint32_t smem_s, int c) {
-	uint32_t p = smem_s + uint32_t(ph.off_acc) + 16u * uint32_t(c);
+__device__ __forceinline__ float ps_column(const PsUnit *u, int c) {
+	uint32_t p = u->acc_s + 16u * uint32_t(c);
+	const uint32_t step = 16u * uint32_t(u->rows);
+	const int segs = u->segs;
 	int4 s = make_int4(0, 0, 0, 0);
 #pragma unroll 4
-	for (int i = 0; i < ph.segs; i++, p += 16u * uint32_t(ph.rows)) {
+	for (int i = 0; i < segs; i++, p += step) {
 		const uint4 v = ps_lds128(p);
 		s.x += int(v.x);
 		s.y += int(v.y);
@@ -444,6 +434,66 @@ __device__ __forceinline__ float ps_column(const PsPhase &ph, uint32_t smem_s, i
 		s.w += int(v.w);
 	}
 	return ps_join(s);
+}
+// lut::GeLUTable::lookup (reference ops.hpp:41-51); tab_s: the table in shared memory where it fits there
+__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint32_t tab_s, uint64_t keep) {
+	int idx;
+	if (!t.index(x, idx)) return 0.0f;
+	if (idx >= t.size) return x;
+	return t.size <= PS_LUT ? ps_ldsf(tab_s + 4u * idx) : ps_ldk(t.table + idx, keep);
+}
+// One unit's product: dst[c] = column sum * scale, or (up and gate) GeLU(gate) * up. Called by the whole CTA behind the
+// barrier that ends the prologue (the digits' writers have fenced, the issuing warps have waited for the unit). Warp 4 t issues tile
+// t's MMAs into its own 16 TMEM columns (one accumulator per issuing warp), warps 4 t .. 4 t + 3 read them back, thread c
+// publishes column c. One store instruction per 32 columns: scattered over the warps, 16 bytes each, the words of a line that 148
+// CTAs poll take 450 clk longer to arrive. pm: parity of bar_m[t], returned. Behind its barrier nobody reads the unit or the digits any
+// more. Measured from the prologue's barrier to the values in registers (1B: 27 MMAs of up and gate, 27 of down, 4 of
+// O, 9 of q|k|v): about 430 clk + 38 per MMA of 128 rows, 23 per one of 64; dp4a loops over the same tiles took 2400, 1450,
+// 850 and 1000 clk and 400 to 600 more to reduce over the lanes.
+__device__ __noinline__ uint32_t ps_unit(const PsW w, int where, const PsUnit *u, uint32_t tmem, uint64_t *bar_w, uint32_t pw, uint64_t *bar_m, uint32_t pm,
+                                         const float *s_xscale, float *dst, const GeluLut lut, uint32_t lut_s, uint64_t keep) {
+	__builtin_assume(__isShared(u));
+	__builtin_assume(__isShared(s_xscale));
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = warp >> 2;
+	float s0 = 0.0f, s1 = 0.0f;
+	if (32 * warp < u->ncol && (warp & 3) != 0) ps_wait_bulk(w, where, bar_w, pw);  // (the issuing warps have waited)
+	if (tid < u->ncol) {  // column scales: read before the barrier behind which the unit may be refilled
+		s0 = ps_ldsf(u->scale_s + 4u * tid);
+		if (u->two) s1 = ps_ldsf(u->scale_s + 4u * (u->ncol + tid));
+	}
+	if (t < u->tiles) {
+		if ((warp & 3) == 0) {
+			tc_fence_after();
+			const uint64_t da = u->da[t], db = u->db[t];
+			const uint32_t id = u->id, d = tmem + 16u * t;
+			const int steps = u->steps;
+			const uint64_t step = uint64_t(u->mt * 2);
+			if (tc_elect()) {
+#pragma unroll 1
+				for (int i = 0; i < steps; i++) i8_mma<1>(d, da + uint64_t(i) * step, db + uint64_t(i * (2 * PS_XCH / 16)), id, i > 0 ? 1u : 0u);
+				i8_commit<1>(&bar_m[t]);
+			}
+			__syncwarp();
+		}
+		const int m = u->ep[warp];
+		const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m & 0xFF), acc = u->acc_s + 16u * uint32_t((m >> 8) + lane);
+		const bool mine = 4 * lane < u->mt;
+		ps_wait_bulk(w, where, &bar_m[t], pm);
+		pm ^= 1u;
+		__syncwarp();
+		tc_fence_after();
+		const int4 v = ps_tmem_ld4(taddr);
+		if (mine) asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(acc), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+		tc_fence_before();
+	}
+	__syncthreads();
+	if (tid < u->ncol) {
+		const float xs = *s_xscale;
+		float y = (ps_column(u, tid) * xs) * s0;
+		if (u->two) y = ps_gelu(lut, (ps_column(u, u->ncol + tid) * xs) * s1, lut_s, keep) * y;
+		if (dst) ps_st(dst + tid, y);
+	}
+	return pm;
 }
 
 // A CTA's unit is one contiguous block of the re-tiled copy: one bulk copy. Called by one lane.
@@ -457,7 +507,7 @@ __device__ __noinline__ void ps_issue(uint8_t *dst, const int8_t *src, uint32_t 
 
 // Re-tile `ntiles_mat` column tiles x ph.nsplit K-splits of a row-major int8 matrix [K][N] into unit order: unit (split,
 // tile0 + t) is a block at dst + (split * ntiles + tile0 + t) * bytes in the layout described at PsPhase, whose rows row0.. hold this
-// matrix. One thread per 4 columns x 16 k.
+// matrix; the columns' scales follow the weights. One thread per 4 columns x 16 k.
 __device__ __forceinline__ uint4 ps_piece(const int8_t *src, size_t N, size_t row0, size_t col0) {  // 4 x 4: word c = column col0 + c
 	const uint32_t r0 = *reinterpret_cast<const uint32_t *>(src + row0 * N + col0);
 	const uint32_t r1 = *reinterpret_cast<const uint32_t *>(src + (row0 + 1) * N + col0);
@@ -467,7 +517,7 @@ __device__ __forceinline__ uint4 ps_piece(const int8_t *src, size_t N, size_t ro
 	const uint32_t t2 = __byte_perm(r0, r1, 0x7362), t3 = __byte_perm(r2, r3, 0x7362);
 	return make_uint4(__byte_perm(t0, t1, 0x5410), __byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x5410), __byte_perm(t2, t3, 0x7632));
 }
-__global__ void retile_units_kernel(int8_t *dst, const int8_t *src, int N, PsPhase ph, int tile0, int ntiles_mat, int row0) {
+__global__ void retile_units_kernel(int8_t *dst, const int8_t *src, const float *scales, int N, PsPhase ph, int tile0, int ntiles_mat, int row0) {
 	const int gcols = ntiles_mat * ph.ncol / 4, uch = ph.nq / 4, sch = ph.seg_q / 4;  // column groups; 16-k chunks of a unit, of a segment
 	const size_t total = size_t(gcols) * uch * ph.nsplit;
 	for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -482,14 +532,11 @@ __global__ void retile_units_kernel(int8_t *dst, const int8_t *src, int N, PsPha
 		o[2] = make_uint4(p[0].z, p[1].z, p[2].z, p[3].z);
 		o[3] = make_uint4(p[0].w, p[1].w, p[2].w, p[3].w);
 	}
-}
-
-// lut::GeLUTable::lookup (reference ops.hpp:41-51); tab_s: the table in shared memory where it fits there
-__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint32_t tab_s, uint64_t keep) {
-	int idx;
-	if (!t.index(x, idx)) return 0.0f;
-	if (idx >= t.size) return x;
-	return t.size <= PS_LUT ? ps_ldsf(tab_s + 4u * idx) : ps_ldk(t.table + idx, keep);
+	if (!scales) return;
+	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N * ph.nsplit; i += gridDim.x * blockDim.x) {
+		const int split = i / N, n = i - split * N, t = n / ph.ncol, c = n - t * ph.ncol;
+		reinterpret_cast<float *>(dst + size_t(split * ph.ntiles + tile0 + t) * ph.bytes + size_t(ph.rows) * ph.nq * 4)[row0 + c] = scales[n];
+	}
 }
 
 // ------------------------------------------------------------------ prologues
@@ -503,12 +550,14 @@ __device__ __forceinline__ float ps_inv_rms(float sumsq, float inv_dim) {
 // If part: t[d] = sum_s part[s][d] (scaled partial sums, polled until complete; threads past D/4 poll
 // the presence words);  h += rmsnorm(t; w_post). Then y = rmsnorm(h; w_pre), quantised with *s_xscale = 2^(e - 30).
 // Every CTA computes the same bits. D <= 4 * PS_THREADS. Thread t owns elements 4t..4t+3, which are quad t. bred: 3 * PS_NW
-// floats, 16-byte aligned.
-__device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h, const PsX x, float *bred, float *s_xscale,
+// floats, 16-byte aligned. bar_w, pw: barrier of the unit that comes next (null: none); its issuing warps wait for it here, under the
+// hand-off (a completed test takes ~200 clk).
+__device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h, const PsUnit *u, uint64_t *bar_w, uint32_t pw, float *bred, float *s_xscale,
                                         const float *part, int nsplit, const float *pres, int npres, const float *w_post,
                                         const float *w_pre, uint64_t keep, float *x_out) {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	__builtin_assume(__isShared(h));
+	__builtin_assume(__isShared(u));
 	__builtin_assume(__isShared(s_xscale));
 	// the norm weights are L2-resident (evict-last): requested together with the first poll loads
 	float4 wpost = make_float4(0.f, 0.f, 0.f, 0.f), wpre = wpost;
@@ -519,6 +568,8 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 	const uint32_t bred_s = ps_smem(bred);
 	const float invD = 1.0f / float(D);
 	const bool in = 4 * tid < D;
+	const uint32_t xaddr = ps_xaddr(u, tid);
+	if (bar_w && (warp & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
 	float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
 	if (in) hv = *reinterpret_cast<const float4 *>(h + 4 * tid);
 	if (part) {
@@ -571,32 +622,21 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 		y.y = (hv.y * r2) * g.y;
 		y.z = (hv.z * r2) * g.z;
 		y.w = (hv.w * r2) * g.w;
-		ps_quantise(y, ps_qmul(M), x, tid);
+		ps_quantise(y, ps_qmul(M), xaddr);
+		ps_fence_async();
 		if (x_out) *reinterpret_cast<float4 *>(x_out + 4 * tid) = y;
 	}
 	if (tid == 0) *s_xscale = ps_qscale(M);
-	ps_fence_async();
 	__syncthreads();
 }
 
-// one warp: x[0..256) (dims 4 lane.. and 128 + 4 lane..) -> rmsnorm, RoPE, * scale -> dst (may alias x)
+// one warp: x[0..256) (dims 4 lane.. and 128 + 4 lane..) -> rmsnorm, RoPE, * scale
 struct PsRope {
-	float4 w0, w1, c0, c1, s0, s1;
+	float4 c0, c1, s0, s1;
 };
-__device__ __forceinline__ void ps_load_rope(PsRope &r, const float *w, const float *cosr, const float *sinr, uint64_t keep) {
-	const int lane = threadIdx.x & 31;
-	r.w0 = ps_ldk4(w + 4 * lane, keep);
-	r.w1 = ps_ldk4(w + 128 + 4 * lane, keep);
-	r.c0 = ps_ldk4(cosr + 4 * lane, keep);
-	r.c1 = ps_ldk4(cosr + 128 + 4 * lane, keep);
-	r.s0 = ps_ldk4(sinr + 4 * lane, keep);
-	r.s1 = ps_ldk4(sinr + 128 + 4 * lane, keep);
-}
-__device__ __forceinline__ void ps_norm_rope(const float *x, const PsRope &r, float scale, float *dst) {
-	const int lane = threadIdx.x & 31;
-	const float4 lo4 = *reinterpret_cast<const float4 *>(x + 4 * lane), hi4 = *reinterpret_cast<const float4 *>(x + 128 + 4 * lane);
+__device__ __forceinline__ void ps_norm_rope(const float4 &lo4, const float4 &hi4, const float4 &w0_, const float4 &w1_, const PsRope &r, float scale, float4 &ylo4, float4 &yhi4) {
 	const float lo[4] = {lo4.x, lo4.y, lo4.z, lo4.w}, hi[4] = {hi4.x, hi4.y, hi4.z, hi4.w};
-	const float w0[4] = {r.w0.x, r.w0.y, r.w0.z, r.w0.w}, w1[4] = {r.w1.x, r.w1.y, r.w1.z, r.w1.w};
+	const float w0[4] = {w0_.x, w0_.y, w0_.z, w0_.w}, w1[4] = {w1_.x, w1_.y, w1_.z, w1_.w};
 	const float c0[4] = {r.c0.x, r.c0.y, r.c0.z, r.c0.w}, c1[4] = {r.c1.x, r.c1.y, r.c1.z, r.c1.w};
 	const float s0[4] = {r.s0.x, r.s0.y, r.s0.z, r.s0.w}, s1[4] = {r.s1.x, r.s1.y, r.s1.z, r.s1.w};
 	float ss = 0.0f;
@@ -616,50 +656,79 @@ __device__ __forceinline__ void ps_norm_rope(const float *x, const PsRope &r, fl
 		ylo[i] = fmaf(-1.0f * q, s0[i], c0[i] * p) * scale;
 		yhi[i] = fmaf(p, s1[i], c1[i] * q) * scale;
 	}
-	__syncwarp();
-	*reinterpret_cast<float4 *>(dst + 4 * lane) = make_float4(ylo[0], ylo[1], ylo[2], ylo[3]);
-	*reinterpret_cast<float4 *>(dst + 128 + 4 * lane) = make_float4(yhi[0], yhi[1], yhi[2], yhi[3]);
+	ylo4 = make_float4(ylo[0], ylo[1], ylo[2], ylo[3]);
+	yhi4 = make_float4(yhi[0], yhi[1], yhi[2], yhi[3]);
 }
 
 // Phase C prologue: merge the attention partials of `hp` heads starting at head h0 over `nch` chunks
 // into the normalised output (reference ops.hpp:316-357 keeps it normalised per step; the split form
 // divides once), quantise it.
-__device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, const PsX x,
-                                           float *bred, float *s_xscale) {
+__device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, const PsUnit *u, uint64_t *bar_w,
+                                           uint32_t pw, float *bred, float *s_xscale) {
 	const int tid = threadIdx.x;
 	__builtin_assume(__isShared(scr));
+	__builtin_assume(__isShared(u));
 	__builtin_assume(__isShared(bred));
 	__builtin_assume(__isShared(s_xscale));
-	const int items = hp * (AT_HD / 4);  // float4 columns
-	const int ncg = PS_THREADS / items;  // chunk groups
-	const int cg = tid / items, it = tid - cg * items;
-	const int hl = it / (AT_HD / 4), j = it - hl * (AT_HD / 4);
+	// thread = (chunk group cg, float4 column it of the hp * 64); hp is 1, 2 or 4
+	const int sh = 6 + (hp >> 1), items = 1 << sh;
+	const int ncg = hp == 1 ? PS_THREADS / 64 : (hp == 2 ? PS_THREADS / 128 : PS_THREADS / 256);
+	const int cg = tid >> sh, it = tid & (items - 1);
+	const int hl = it >> 6, j = it & 63;
+	const uint32_t xaddr = ps_xaddr(u, it);
+	if (((tid >> 5) & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
 	float m = -INFINITY, l = 0.0f;
 	float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 	if (cg < ncg) {
+		// PB chunks are requested together: one after the other a hand-off of nine chunks took three dependent round trips
+		constexpr int PB = 4;
 #pragma unroll 1
-		for (int ch = cg; ch < nch; ch += ncg) {
-			const float *r0 = att_ll + (size_t(h0 + hl) * PS_MAX_CH + ch) * PS_ATT_ROW;
-			float4 ov;
-			float2 ml;
+		for (int cb = cg; cb < nch; cb += PB * ncg) {
+			float4 ov[PB];
+			float2 ml[PB];
 			int spins = 0;
 			long long t0 = 0;
 			bool ok;
 			do {
-				ov = ps_ld4(r0 + 4 * j);
-				ml = ps_ld2(r0 + AT_HD);
-				ok = ps_ok(ov) && ps_ok(ml);
+				ok = true;
+#pragma unroll
+				for (int i = 0; i < PB; i++) {
+					const int ch = cb + i * ncg;
+					ml[i] = make_float2(-INFINITY, 0.0f);
+					ov[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+					if (ch < nch) {
+						const float *r0 = att_ll + (size_t(h0 + hl) * PS_MAX_CH + ch) * PS_ATT_ROW;
+						ov[i] = ps_ld4(r0 + 4 * j);
+						ml[i] = ps_ld2(r0 + AT_HD);
+					}
+				}
+#pragma unroll
+				for (int i = 0; i < PB; i++) ok = ok && ps_ok(ov[i]) && ps_ok(ml[i]);
 			} while (!ok && ps_retry(w, where, spins, t0));
-			if (ml.x == -INFINITY) continue;  // empty chunk
-			const float mn = fmaxf(m, ml.x);
-			const float ea = expf(m - mn), eb = expf(ml.x - mn);
-			l = fmaf(l, ea, ml.y * eb);
-			o.x = fmaf(o.x, ea, ov.x * eb);
-			o.y = fmaf(o.y, ea, ov.y * eb);
-			o.z = fmaf(o.z, ea, ov.z * eb);
-			o.w = fmaf(o.w, ea, ov.w * eb);
+			float mn = m;
+#pragma unroll
+			for (int i = 0; i < PB; i++) mn = fmaxf(mn, ml[i].x);
+			if (mn == -INFINITY) continue;  // nothing but empty chunks so far
+			const float ea = expf(m - mn);
+			l *= ea;
+			o.x *= ea;
+			o.y *= ea;
+			o.z *= ea;
+			o.w *= ea;
+#pragma unroll
+			for (int i = 0; i < PB; i++) {
+				const float eb = expf(ml[i].x - mn);
+				l = fmaf(ml[i].y, eb, l);
+				o.x = fmaf(ov[i].x, eb, o.x);
+				o.y = fmaf(ov[i].y, eb, o.y);
+				o.z = fmaf(ov[i].z, eb, o.z);
+				o.w = fmaf(ov[i].w, eb, o.w);
+			}
 			m = mn;
 		}
+	}
+	__syncthreads();  // (the attention of this CTA has left the scratch)
+	if (cg < ncg) {
 		float *s = scr + (size_t(cg) * items + it) * 8;
 		*reinterpret_cast<float4 *>(s) = o;
 		*reinterpret_cast<float2 *>(s + 4) = make_float2(m, l);
@@ -668,16 +737,18 @@ __device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *
 	float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 	float mx = 0.0f;
 	if (tid < items) {
-		float M = -INFINITY;
-#pragma unroll 1
-		for (int g = 0; g < ncg; g++) M = fmaxf(M, scr[(size_t(g) * items + tid) * 8 + 4]);
-		float L = 0.0f;
-#pragma unroll 1
-		for (int g = 0; g < ncg; g++) {
+		constexpr int NG = PS_THREADS / 64;
+		float mg[NG], M = -INFINITY, L = 0.0f;
+#pragma unroll
+		for (int g = 0; g < NG; g++) {
+			mg[g] = g < ncg ? scr[(size_t(g) * items + tid) * 8 + 4] : -INFINITY;
+			M = fmaxf(M, mg[g]);
+		}
+#pragma unroll
+		for (int g = 0; g < NG; g++) {
+			if (g >= ncg) break;
 			const float *s = scr + (size_t(g) * items + tid) * 8;
-			const float mg = s[4];
-			if (mg == -INFINITY) continue;
-			const float e = expf(mg - M);
+			const float e = expf(mg[g] - M);
 			const float4 ov = *reinterpret_cast<const float4 *>(s);
 			L = fmaf(s[5], e, L);
 			y.x = fmaf(ov.x, e, y.x);
@@ -693,18 +764,22 @@ __device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *
 		mx = fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)));
 	}
 	const float M = ps_block_max(mx, bred);
-	if (tid < items) ps_quantise(y, ps_qmul(M), x, tid);
+	if (tid < items) {
+		ps_quantise(y, ps_qmul(M), xaddr);
+		ps_fence_async();
+	}
 	if (tid == 0) *s_xscale = ps_qscale(M);
-	ps_fence_async();
 	__syncthreads();
 }
 
 // Phase E prologue: this CTA's rows of the activation vector (nq quads from act), polled until
 // complete, quantised. nq <= 5 * PS_THREADS.
-__device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, const PsX x, float *bred, float *s_xscale) {
+__device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, const PsUnit *u, uint64_t *bar_w, uint32_t pw, float *bred, float *s_xscale) {
 	const int tid = threadIdx.x;
+	__builtin_assume(__isShared(u));
 	__builtin_assume(__isShared(bred));
 	__builtin_assume(__isShared(s_xscale));
+	if (((tid >> 5) & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
 	float4 v[5];
 	int spins = 0;
 	long long t0 = 0;
@@ -727,7 +802,7 @@ __device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *a
 #pragma unroll
 	for (int q = 0; q < 5; q++) {
 		const int i = q * PS_THREADS + tid;
-		if (i < nq) ps_quantise(v[q], qs, x, i);
+		if (i < nq) ps_quantise(v[q], qs, ps_xaddr(u, i));
 	}
 	if (tid == 0) *s_xscale = ps_qscale(M);
 	ps_fence_async();
@@ -738,17 +813,16 @@ __device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *a
 // vector (polled), q/k norm + RoPE, append of the new row (head 0's CTA of the chunk that holds `slot`),
 // running-max softmax over the chunk (warp -> slots j0 + warp, + 12, ...; lane owns dims 4 lane.. and
 // 128 + 4 lane..), merge of the 12 warps, (o[256], m, l) published to prow. att: 16 KB of scratch,
-// wml: 3 * PS_NW floats. Reference: ops.hpp:224-370 (attention_decode), decode.hpp:203-211 (RoPE).
+// wml: 2 * PS_NW floats. Every warp norms and rotates q itself, the one that owns the new row k too: one barrier less, and
+// no values through shared memory. Reference: ops.hpp:224-370 (attention_decode), decode.hpp:203-211 (RoPE).
 __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache, float *vcache, const float *rmsq, const float *rmsk,
                                           const float *cosr, const float *sinr, const float *qkv_ll, int QD, int hh, float *prow, int j0,
                                           int j1, int slot, float *att, float *wml, uint64_t keep) {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	__builtin_assume(__isShared(att));
 	__builtin_assume(__isShared(wml));
-	float *wo = att, *qraw = att + PS_NW * AT_HD, *qs = qraw + 3 * AT_HD;
-	float *wm = wml, *wl = wml + PS_NW, *we = wml + 2 * PS_NW;
-	PsRope rr;
-	if (warp < 2) ps_load_rope(rr, warp == 0 ? rmsq : rmsk, cosr, sinr, keep);
+	float *wo = att, *qraw = att + PS_NW * AT_HD;
+	float *wm = wml, *wl = wml + PS_NW;
 	// The cache rows do not depend on this token's q|k|v: a warp's first two rows are requested before
 	// the poll (the new token's own row comes from shared memory later).
 	float4 kv[2][4];
@@ -756,6 +830,8 @@ __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache,
 #pragma unroll
 		for (int u = 0; u < 2; u++) {
 			const int j = jb + PS_NW * u;
+#pragma unroll
+			for (int i = 0; i < 4; i++) kv[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
 			if (j < j1 && j != slot) {
 				const float *kr = kcache + size_t(j) * AT_HD, *vr = vcache + size_t(j) * AT_HD;
 				kv[u][0] = __ldcg(reinterpret_cast<const float4 *>(kr + 4 * lane));
@@ -766,6 +842,18 @@ __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache,
 		}
 	};
 	load_keys(j0 + warp);
+	const bool own = slot >= j0 && slot < j1 && (slot - j0) % PS_NW == warp;
+	PsRope rr;
+	rr.c0 = ps_ldk4(cosr + 4 * lane, keep);
+	rr.c1 = ps_ldk4(cosr + 128 + 4 * lane, keep);
+	rr.s0 = ps_ldk4(sinr + 4 * lane, keep);
+	rr.s1 = ps_ldk4(sinr + 128 + 4 * lane, keep);
+	const float4 wq0 = ps_ldk4(rmsq + 4 * lane, keep), wq1 = ps_ldk4(rmsq + 128 + 4 * lane, keep);
+	float4 wk0 = wq0, wk1 = wq1;
+	if (own) {
+		wk0 = ps_ldk4(rmsk + 4 * lane, keep);
+		wk1 = ps_ldk4(rmsk + 128 + 4 * lane, keep);
+	}
 	if (tid < 3 * (AT_HD / 4)) {
 		const float *src = qkv_ll + (tid < AT_HD / 4 ? hh * AT_HD + 4 * tid : QD + 4 * (tid - AT_HD / 4));
 		float4 v;
@@ -777,55 +865,62 @@ __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache,
 		*reinterpret_cast<float4 *>(qraw + 4 * tid) = v;
 	}
 	__syncthreads();
-	float *ks = qraw + AT_HD, *vs = qraw + 2 * AT_HD;
+	const float4 *q4 = reinterpret_cast<const float4 *>(qraw);
+	float4 q0, q1, k0, k1;
 	// the reference scales q by 1/sqrt(256) before the dot products (ops.hpp:262,283); k is normed in place
-	if (warp < 2) ps_norm_rope(qraw + warp * AT_HD, rr, warp == 0 ? 0.0625f : 1.0f, warp == 0 ? qs : ks);
-	__syncthreads();
-	if (hh == 0 && slot >= j0 && slot < j1 && tid < 2 * (AT_HD / 4)) {
-		float *dst = (tid < AT_HD / 4 ? kcache : vcache) + size_t(slot) * AT_HD;
-		const int j = tid & (AT_HD / 4 - 1);
-		*reinterpret_cast<float4 *>(dst + 4 * j) = *reinterpret_cast<const float4 *>((tid < AT_HD / 4 ? ks : vs) + 4 * j);
-	}
-	const float4 q0 = *reinterpret_cast<const float4 *>(qs + 4 * lane);
-	const float4 q1 = *reinterpret_cast<const float4 *>(qs + 128 + 4 * lane);
+	ps_norm_rope(q4[lane], q4[32 + lane], wq0, wq1, rr, 0.0625f, q0, q1);
+	if (own) ps_norm_rope(q4[64 + lane], q4[96 + lane], wk0, wk1, rr, 1.0f, k0, k1);
 	float4 o0 = make_float4(0.f, 0.f, 0.f, 0.f), o1 = make_float4(0.f, 0.f, 0.f, 0.f);
 	float m = -INFINITY, lsum = 0.0f;
 #pragma unroll 1
 	for (int jb = j0 + warp; jb < j1; jb += 2 * PS_NW) {
 #pragma unroll
-		for (int u = 0; u < 2; u++) {
-			const int j = jb + PS_NW * u;
-			if (j >= j1) continue;
-			if (j == slot) {  // the new row: not in the cache yet for the other heads' CTAs
-				kv[u][0] = *reinterpret_cast<const float4 *>(ks + 4 * lane);
-				kv[u][1] = *reinterpret_cast<const float4 *>(ks + 128 + 4 * lane);
-				kv[u][2] = *reinterpret_cast<const float4 *>(vs + 4 * lane);
-				kv[u][3] = *reinterpret_cast<const float4 *>(vs + 128 + 4 * lane);
+		for (int u = 0; u < 2; u++)
+			if (own && jb + PS_NW * u == slot) {  // the new row: not in the cache yet for the other heads' CTAs
+				kv[u][0] = k0;
+				kv[u][1] = k1;
+				kv[u][2] = q4[128 + lane];
+				kv[u][3] = q4[160 + lane];
+				if (hh == 0) {
+					float4 *kr = reinterpret_cast<float4 *>(kcache + size_t(slot) * AT_HD), *vr = reinterpret_cast<float4 *>(vcache + size_t(slot) * AT_HD);
+					kr[lane] = k0;
+					kr[32 + lane] = k1;
+					vr[lane] = kv[u][2];
+					vr[32 + lane] = kv[u][3];
+				}
 			}
-			float t = q0.x * kv[u][0].x;
-			t = fmaf(q0.y, kv[u][0].y, t);
-			t = fmaf(q0.z, kv[u][0].z, t);
-			t = fmaf(q0.w, kv[u][0].w, t);
-			t = fmaf(q1.x, kv[u][1].x, t);
-			t = fmaf(q1.y, kv[u][1].y, t);
-			t = fmaf(q1.z, kv[u][1].z, t);
-			t = fmaf(q1.w, kv[u][1].w, t);
-			t = warp_sum(t);
-			const float mn = fmaxf(m, t);
-			const float corr = expf(m - mn);
-			const float pp = expf(t - mn);
-			lsum = fmaf(lsum, corr, pp);
-			o0.x = fmaf(pp, kv[u][2].x, o0.x * corr);
-			o0.y = fmaf(pp, kv[u][2].y, o0.y * corr);
-			o0.z = fmaf(pp, kv[u][2].z, o0.z * corr);
-			o0.w = fmaf(pp, kv[u][2].w, o0.w * corr);
-			o1.x = fmaf(pp, kv[u][3].x, o1.x * corr);
-			o1.y = fmaf(pp, kv[u][3].y, o1.y * corr);
-			o1.z = fmaf(pp, kv[u][3].z, o1.z * corr);
-			o1.w = fmaf(pp, kv[u][3].w, o1.w * corr);
-			m = mn;
+		// two rows at a time: their sums over the lanes overlap
+		float t[2];
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			t[u] = q0.x * kv[u][0].x;
+			t[u] = fmaf(q0.y, kv[u][0].y, t[u]);
+			t[u] = fmaf(q0.z, kv[u][0].z, t[u]);
+			t[u] = fmaf(q0.w, kv[u][0].w, t[u]);
+			t[u] = fmaf(q1.x, kv[u][1].x, t[u]);
+			t[u] = fmaf(q1.y, kv[u][1].y, t[u]);
+			t[u] = fmaf(q1.z, kv[u][1].z, t[u]);
+			t[u] = fmaf(q1.w, kv[u][1].w, t[u]);
 		}
-		load_keys(jb + 2 * PS_NW);
+#pragma unroll
+		for (int of = 16; of > 0; of >>= 1) {
+			t[0] += __shfl_xor_sync(0xffffffffu, t[0], of);
+			t[1] += __shfl_xor_sync(0xffffffffu, t[1], of);
+		}
+		if (jb + PS_NW >= j1) t[1] = -INFINITY;  // (its values are zeros)
+		const float mn = fmaxf(m, fmaxf(t[0], t[1]));
+		const float corr = expf(m - mn), p0 = expf(t[0] - mn), p1 = expf(t[1] - mn);
+		lsum = fmaf(lsum, corr, p0) + p1;
+		o0.x = fmaf(p1, kv[1][2].x, fmaf(p0, kv[0][2].x, o0.x * corr));
+		o0.y = fmaf(p1, kv[1][2].y, fmaf(p0, kv[0][2].y, o0.y * corr));
+		o0.z = fmaf(p1, kv[1][2].z, fmaf(p0, kv[0][2].z, o0.z * corr));
+		o0.w = fmaf(p1, kv[1][2].w, fmaf(p0, kv[0][2].w, o0.w * corr));
+		o1.x = fmaf(p1, kv[1][3].x, fmaf(p0, kv[0][3].x, o1.x * corr));
+		o1.y = fmaf(p1, kv[1][3].y, fmaf(p0, kv[0][3].y, o1.y * corr));
+		o1.z = fmaf(p1, kv[1][3].z, fmaf(p0, kv[0][3].z, o1.z * corr));
+		o1.w = fmaf(p1, kv[1][3].w, fmaf(p0, kv[0][3].w, o1.w * corr));
+		m = mn;
+		if (jb + 2 * PS_NW < j1) load_keys(jb + 2 * PS_NW);
 	}
 	if (lane == 0) {
 		wm[warp] = m;
@@ -834,24 +929,24 @@ __device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache,
 	*reinterpret_cast<float4 *>(wo + warp * AT_HD + 4 * lane) = o0;
 	*reinterpret_cast<float4 *>(wo + warp * AT_HD + 128 + 4 * lane) = o1;
 	__syncthreads();
-	float M = -INFINITY;
+	// merge: lane i of every warp holds warp i's maximum and weight (the caller's next use of the scratch is behind a barrier)
+	if (warp <= AT_HD / 32) {
+		const float mi = lane < PS_NW ? wm[lane] : -INFINITY;
+		const float M = warp_max(mi);
+		const float e = mi == -INFINITY ? 0.0f : expf(mi - M);
+		if (warp < AT_HD / 32) {
+			float O = 0.0f;
 #pragma unroll
-	for (int i = 0; i < PS_NW; i++) M = fmaxf(M, wm[i]);
-	if (tid < PS_NW) we[tid] = (wm[tid] == -INFINITY) ? 0.0f : expf(wm[tid] - M);
-	__syncthreads();
-	if (tid < AT_HD) {
-		float O = 0.0f;
+			for (int i = 0; i < PS_NW; i++) O = fmaf(wo[i * AT_HD + tid], __shfl_sync(0xffffffffu, e, i), O);
+			ps_st(prow + tid, O);
+		} else {
+			const float li = lane < PS_NW ? wl[lane] : 0.0f;
+			float Ls = 0.0f;
 #pragma unroll
-		for (int i = 0; i < PS_NW; i++) O = fmaf(wo[i * AT_HD + tid], we[i], O);
-		ps_st(prow + tid, O);
-	} else if (tid == AT_HD) {
-		float Ls = 0.0f;
-#pragma unroll
-		for (int i = 0; i < PS_NW; i++) Ls = fmaf(wl[i], we[i], Ls);
-		ps_st(prow + AT_HD, M);
-		ps_st(prow + AT_HD + 1, Ls);
+			for (int i = 0; i < PS_NW; i++) Ls = fmaf(__shfl_sync(0xffffffffu, li, i), __shfl_sync(0xffffffffu, e, i), Ls);
+			if (lane < 2) ps_st(prow + AT_HD + lane, lane == 0 ? M : Ls);
+		}
 	}
-	__syncthreads();  // the scratch is reused by phase C
 }
 
 // lm_head of one token: logits[v] = lm_scale[v] * sum_k x[k] W[k,v]; this CTA takes tiles cta, cta + G, ... of 128 columns; a
@@ -1119,9 +1214,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	__shared__ float s_f[8];
 	__shared__ int s_i[4];
 	__shared__ int s_cdf[2 * PS_NW + 8];
-	__shared__ float wm[3 * PS_NW];  // per-warp (m, l, weight) of the attention merge; also the sampler's per-warp maxima
+	__shared__ float wm[2 * PS_NW];  // per-warp (m, l) of the attention merge; also the sampler's per-warp maxima
 	__shared__ PsLayer s_ly[PS_MAX_LAYERS];
-	__shared__ int s_nch[2];
+	__shared__ PsUnit s_u[5];  // A, C, D, E, lm_head
+	__shared__ PsSpan s_at[2];  // [is_local]
 
 #define R_A (smem + a.off_A)
 #define R_C (smem + a.off_C)
@@ -1133,7 +1229,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #define h (reinterpret_cast<float *>(smem + a.off_h))
 #define att (reinterpret_cast<float *>(smem + a.off_att))  /* wo[12][256] | qraw[768] (q_h, k, v) | qs[256] */
 #define smem_s (ps_smem(smem))
-#define tmem (s_tmem)
+#define tmem (s_c.tm)
+#define lut_s (smem_s + uint32_t(a.off_lut))
 #define pol (ps_evict_first())
 #define keep (ps_evict_last())
 
@@ -1162,6 +1259,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	if (warp == 1) {
+		__syncwarp();
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ps_smem(&s_tmem)), "r"(PS_TMEM) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
@@ -1186,13 +1284,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		const int uA = cta - a.A.cta0, uC = cta - a.C.cta0, uD = cta - a.Dp.cta0, uE = cta - a.E.cta0;
 		const bool hA = uA >= 0 && uA < a.A.units, hC = uC >= 0 && uC < a.C.units, hD = uD >= 0 && uD < a.Dp.units, hE = uE >= 0 && uE < a.E.units;
 		if (tid == 0) {
-			s_c.tileA = hA ? uA % a.A.ntiles : 0;
-			s_c.tileC = hC ? uC % a.C.ntiles : 0;
+			s_c.tm = *(volatile uint32_t *)&s_tmem;
 			s_c.splitC = hC ? uC / a.C.ntiles : 0;
-			s_c.tileE = hE ? uE % a.E.ntiles : 0;
 			s_c.splitE = hE ? uE / a.E.ntiles : 0;
 			s_c.presE = uE < 0 ? cta : cta - a.E.units;  // index of this CTA's presence word (if !hasE)
-			s_c.uD = uD;
 			// the unit this CTA fetches for a phase of layer l (one lane issues the copy)
 			s_c.srcA = a.tiled + a.tl_A + size_t(hA ? uA : 0) * a.A.bytes;
 			s_c.srcC = a.tiled + a.tl_C + size_t(hC ? uC : 0) * a.C.bytes;
@@ -1201,10 +1296,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			s_c.has = (hA ? 1 : 0) | (hC ? 2 : 0) | (hD ? 4 : 0) | (hE ? 8 : 0);
 		}
 		if (lane == 0) {
-			ps_fill_map(a.A, warp, s_c.ep[0], s_c.xo[0]);
-			ps_fill_map(a.C, warp, s_c.ep[1], s_c.xo[1]);
-			ps_fill_map(a.Dp, warp, s_c.ep[2], s_c.xo[2]);
-			ps_fill_map(a.E, warp, s_c.ep[3], s_c.xo[3]);
+			ps_fill_unit(a.A, &s_u[0], warp, smem_s, a.off_A, a.ll_qkv + (hA ? uA % a.A.ntiles : 0) * a.A.ncol);
+			ps_fill_unit(a.C, &s_u[1], warp, smem_s, a.off_C, a.ll_op + (hC ? (uC / a.C.ntiles) * D + (uC % a.C.ntiles) * a.C.ncol : 0));
+			ps_fill_unit(a.Dp, &s_u[2], warp, smem_s, a.off_D, a.ll_act + (hD ? uD : 0) * a.Dp.ncol);
+			ps_fill_unit(a.E, &s_u[3], warp, smem_s, a.off_E, a.ll_dn + (hE ? (uE / a.E.ntiles) * D + (uE % a.E.ntiles) * a.E.ncol : 0));
+			ps_fill_unit(a.lm, &s_u[4], warp, smem_s, a.off_D, 0);
 		}
 		__syncthreads();
 	}
@@ -1212,13 +1308,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #define hasC ((s_c.has & 2) != 0)
 #define hasD ((s_c.has & 4) != 0)
 #define hasE ((s_c.has & 8) != 0)
-#define tileA (s_c.tileA)
-#define tileC (s_c.tileC)
 #define splitC (s_c.splitC)
-#define tileE (s_c.tileE)
 #define splitE (s_c.splitE)
 #define presE (s_c.presE)
-#define uD (s_c.uD)
 #define srcA (s_c.srcA)
 #define srcC (s_c.srcC)
 #define srcD (s_c.srcD)
@@ -1236,12 +1328,6 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	const int rbase = __ldcg(a.ring_base);
 	int n_logged = 0;
 	int dbg_n = 0;
-	// thread c publishes column c of the CTA's unit: one store instruction per 32 columns. (Scattered over the warps, 16 bytes each,
-	// the words of a line that 148 CTAs poll take 450 clk longer to arrive.)
-	const bool actA = hasA && tid < a.A.ncol, actC = hasC && tid < a.C.ncol, actD = hasD && tid < a.Dp.ncol, actE = hasE && tid < a.E.ncol;
-	const bool iss = (warp & 3) == 0;  // this warp may issue MMAs
-	const int colA = tileA * a.A.ncol + tid, colC = tileC * a.C.ncol + tid, colD = uD * a.Dp.ncol + tid, colE = tileE * a.E.ncol + tid;
-
 	// ring stages of the lm_head that fit the up/gate region and belong to this CTA's first tile (chunks 0 .. lm_pre - 1)
 	const int lm_pre = (cta < a.lm_ntiles && a.sched == 0) ? min(min(a.lm_stages, a.lm_nchunk), a.Dp.bytes / a.lm_stage_bytes) : 0;
 #pragma unroll 1
@@ -1262,13 +1348,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		// 1B model.)
 		if (warp == 0) {
 			const bool loc = lane < 16;
-			const int n = min(3 * ((lane & 15) + 1), a.nch_max), v = loc ? min(pos + 1, a.slots_local) : pos + 1;
+			const int n = min(3 * ((lane & 15) + 1), a.nch_max), v = loc ? min(pos + 1, a.slots_local) : min(pos + 1, a.slots_global);
 			const int steps = ((v + n - 1) / n + 2 * PS_NW - 1) / (2 * PS_NW);
 			const unsigned key = unsigned(3 * steps + (n + 2) / 3) << 8 | unsigned(n);
 			const unsigned kl = __reduce_min_sync(0xffffffffu, loc ? key : ~0u), kg = __reduce_min_sync(0xffffffffu, loc ? ~0u : key);
-			if (lane == 0) {
-				s_nch[1] = a.nch_local ? a.nch_local : int(kl & 255u);
-				s_nch[0] = a.nch_global ? a.nch_global : int(kg & 255u);
+			if ((lane & 15) == 0) {  // position bookkeeping (KVCache, reference decode.hpp:45-70)
+				const int given = loc ? a.nch_local : a.nch_global, nch = given ? given : int((loc ? kl : kg) & 255u);
+				const int p = loc ? pos : min(pos, a.slots_global - 1);
+				if (!loc && pos >= a.slots_global && cta == 0) atomicExch(a.err, 2);
+				s_at[loc] = PsSpan{p, loc ? (p - rbase) % a.slots_local : p, v, nch, (v + nch - 1) / nch};
 			}
 		}
 #pragma unroll 1
@@ -1278,21 +1366,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #pragma unroll 1
 		for (int l = 0; l < L; l++) {
 			const PsLayer &ly = s_ly[l];
-			// position bookkeeping of this layer's cache (KVCache, reference decode.hpp:45-70)
-			int p = pos, slot, valid;
-			if (ly.is_local) {
-				slot = (p - rbase) % ly.slots;
-				valid = min(p + 1, ly.slots);
-			} else {
-				if (p >= ly.slots) {
-					if (tid == 0 && cta == 0) atomicExch(a.err, 2);
-					p = ly.slots - 1;
-				}
-				slot = p;
-				valid = p + 1;
-			}
-			const int nch = s_nch[ly.is_local];
-			const int nsA = AT_NH * nch;  // CTAs that take part in attention
+			const PsSpan &at = s_at[ly.is_local];
+			const int nsA = AT_NH * at.nch;  // CTAs that take part in attention
 			const int lc = step * L + l;
 			const int nl = (l + 1 < L) ? l + 1 : (more ? 0 : -1);  // the layer whose units are fetched next
 			float *const llb = a.ll + size_t(lc % 3) * a.ll_stride;
@@ -1300,33 +1375,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			PS_BEACON(0x10);
 			PS_GT(0);
 			// ============================================================ A: QKV
-			// Cold data of the whole layer (this lane's column scales, the norm weights of phase D) is requested
-			// here, a phase or more before its use: a DRAM or L2 access issued while a burst of weight copies
-			// lands can take microseconds, and a publishing warp that waits for its scale delays every consumer.
-			float scA = 0.0f, scC = 0.0f, su_r = 0.0f, sg_r = 0.0f, scE = 0.0f;
-			if (actA) {
-				const int n = colA;
-				scA = ps_ldk(n < a.QD ? ly.sq + n : (n < a.QD + a.KD ? ly.sk + (n - a.QD) : ly.sv + (n - a.QD - a.KD)), keep);
-			}
-			if (actC) scC = ps_ldk(ly.so + colC, keep);
-			if (actD) {
-				su_r = ps_ldk(ly.su + colD, keep);
-				sg_r = ps_ldk(ly.sg + colD, keep);
-			}
-			if (actE) scE = ps_ldk(ly.sd + colE, keep);
-			// The units were requested a layer ago: test their barriers early, so that the (long) latency of the
-			// test hides behind the hand-off polls instead of following them.
-			const bool rdyA = iss && hasA && ps_mbar_test(&bar_A, pA), rdyC = iss && hasC && ps_mbar_test(&bar_C, pC);
 			{
-				ps_resnorm(pw, (l << 4) | 1, D, h, ps_x(a.A, smem_s), bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
+				ps_resnorm(pw, (l << 4) | 1, D, h, &s_u[0], hasA ? &bar_A : nullptr, pA, bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
 				           G - a.E.units, l > 0 ? s_ly[l - 1].mlp_post : nullptr, ly.attn_pre, keep, nullptr);
 				PS_STAMP();
 				PS_GT(1);
 				PS_BEACON(0x11);
 				if (hasA) {
 					PS_STAMP();
-					pm = ps_product(pw, (l << 4) | 1, ps_mm(a.A, smem_s, ps_smem(R_A)), tmem, &bar_A, pA, rdyA, bar_m, pm, s_c.ep[0], s_c.xo[0]);
-					if (actA) ps_st(llb + a.ll_qkv + colA, (ps_column(a.A, smem_s, tid) * s_xscale) * scA);
+					pm = ps_unit(pw, (l << 4) | 1, &s_u[0], tmem, &bar_A, pA, bar_m, pm, &s_xscale, llb + s_u[0].dst, a.lut, lut_s, keep);
 					PS_STAMP();
 					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_A, srcA + size_t(nl) * a.tl_layer, a.A.bytes, &bar_A, pol, &s_abort);
 				} else {
@@ -1360,11 +1417,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			}
 			// ============================================================ B: attention
 			if (cta < nsA) {
-				const int chunk = (valid + nch - 1) / nch;
-				const int j0 = (cta >> 2) * chunk;
-				ps_attention(pw, (l << 4) | 2, ly.kcache, ly.vcache, ly.rmsq, ly.rmsk, a.rope[ly.is_local][0] + size_t(p) * AT_HD,
-				             a.rope[ly.is_local][1] + size_t(p) * AT_HD, llb + a.ll_qkv, a.QD, cta & 3,
-				             llb + a.ll_att + (size_t(cta & 3) * PS_MAX_CH + (cta >> 2)) * PS_ATT_ROW, j0, min(valid, j0 + chunk), slot, att, wm,
+				const int j0 = (cta >> 2) * at.chunk;
+				ps_attention(pw, (l << 4) | 2, ly.kcache, ly.vcache, ly.rmsq, ly.rmsk, a.rope[ly.is_local][0] + size_t(at.p) * AT_HD,
+				             a.rope[ly.is_local][1] + size_t(at.p) * AT_HD, llb + a.ll_qkv, a.QD, cta & 3,
+				             llb + a.ll_att + (size_t(cta & 3) * PS_MAX_CH + (cta >> 2)) * PS_ATT_ROW, j0, min(at.valid, j0 + at.chunk), at.slot, att, wm,
 				             keep);
 			}
 			PS_BEACON(0x24);
@@ -1373,14 +1429,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			// ============================================================ C: O projection
 			{
 				if (hasC) {
-					const int hp = AT_NH / a.C.nsplit;
-					ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, splitC * hp, hp, nch, att, ps_x(a.C, smem_s), bred, &s_xscale);
+					ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, splitC * a.merge_heads, a.merge_heads, at.nch, att, &s_u[1], &bar_C, pC, bred, &s_xscale);
 					PS_STAMP();
 					PS_GT(4);
 					PS_BEACON(0x31);
 					PS_STAMP();
-					pm = ps_product(pw, (l << 4) | 3, ps_mm(a.C, smem_s, ps_smem(R_C)), tmem, &bar_C, pC, rdyC, bar_m, pm, s_c.ep[1], s_c.xo[1]);
-					if (actC) ps_st(llb + a.ll_op + size_t(splitC) * D + colC, (ps_column(a.C, smem_s, tid) * s_xscale) * scC);
+					pm = ps_unit(pw, (l << 4) | 3, &s_u[1], tmem, &bar_C, pC, bar_m, pm, &s_xscale, llb + s_u[1].dst, a.lut, lut_s, keep);
 					PS_STAMP();
 					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_C, srcC + size_t(nl) * a.tl_layer, a.C.bytes, &bar_C, pol, &s_abort);
 				} else {
@@ -1395,19 +1449,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			}
 			// ============================================================ D: up & gate + GeGLU
 			{
-				const bool rdyD = iss && hasD && ps_mbar_test(&bar_D, pD);
-				ps_resnorm(pw, (l << 4) | 4, D, h, ps_x(a.Dp, smem_s), bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr);
+				ps_resnorm(pw, (l << 4) | 4, D, h, &s_u[2], hasD ? &bar_D : nullptr, pD, bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr);
 				PS_STAMP();
 				PS_GT(6);
 				PS_BEACON(0x41);
 				PS_STAMP();
-				if (hasD) {
-					pm = ps_product(pw, (l << 4) | 4, ps_mm(a.Dp, smem_s, ps_smem(R_D)), tmem, &bar_D, pD, rdyD, bar_m, pm, s_c.ep[2], s_c.xo[2]);
-					if (actD) {
-						const float xs = s_xscale, u = ps_column(a.Dp, smem_s, tid), g = ps_column(a.Dp, smem_s, a.Dp.ncol + tid);
-						ps_st(llb + a.ll_act + colD, ps_gelu(a.lut, (g * xs) * sg_r, smem_s + uint32_t(a.off_lut), keep) * ((u * xs) * su_r));
-					}
-				}
+				if (hasD) pm = ps_unit(pw, (l << 4) | 4, &s_u[2], tmem, &bar_D, pD, bar_m, pm, &s_xscale, llb + s_u[2].dst, a.lut, lut_s, keep);
 				pD ^= 1;
 				PS_STAMP();
 				PS_GT(7);
@@ -1415,9 +1462,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			}
 			// ============================================================ E: down projection
 			{
-				const bool rdyE = iss && hasE && ps_mbar_test(&bar_E, pE);
 				if (hasE) {
-					ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(splitE) * a.E.nq * 4, a.E.nq, ps_x(a.E, smem_s), bred, &s_xscale);
+					ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(splitE) * a.E.nq * 4, a.E.nq, &s_u[3], &bar_E, pE, bred, &s_xscale);
 				}
 				// the up/gate region is free: request the next layer's unit now that the hand-off loads are done
 				if (a.sched == 0 && tid == PS_THREADS - 32 && hasD && l + 1 < L) ps_issue(R_D, srcD + size_t(l + 1) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
@@ -1434,8 +1480,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 				PS_BEACON(0x51);
 				if (hasE) {
 					PS_STAMP();
-					pm = ps_product(pw, (l << 4) | 5, ps_mm(a.E, smem_s, ps_smem(R_E)), tmem, &bar_E, pE, rdyE, bar_m, pm, s_c.ep[3], s_c.xo[3]);
-					if (actE && cta != a.fault_cta) ps_st(llb + a.ll_dn + size_t(splitE) * D + colE, (ps_column(a.E, smem_s, tid) * s_xscale) * scE);
+					pm = ps_unit(pw, (l << 4) | 5, &s_u[3], tmem, &bar_E, pE, bar_m, pm, &s_xscale, cta != a.fault_cta ? llb + s_u[3].dst : nullptr, a.lut, lut_s, keep);
 					PS_STAMP();
 					if (a.sched == 0 && l + 1 < L && tid == PS_THREADS - 64) ps_issue(R_E, srcE + size_t(l + 1) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
 				} else {
@@ -1455,7 +1500,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		const int lc = step * L + L;
 		{
 			float *const lllast = a.ll + size_t((lc + 2) % 3) * a.ll_stride;
-			ps_resnorm(pw, (L << 4) | 6, D, h, ps_x(a.lm, smem_s), bred, &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
+			ps_resnorm(pw, (L << 4) | 6, D, h, &s_u[4], nullptr, 0, bred, &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
 			           s_ly[L - 1].mlp_post, a.final_norm, keep, cta == 0 ? a.xnorm_out : nullptr);
 		}
 		PS_STAMP();
@@ -1495,6 +1540,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 	tc_fence_before();
 	__syncthreads();
 	if (warp == 1) {
+		__syncwarp();
 		tc_fence_after();
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PS_TMEM) : "memory");
 	}
@@ -1512,6 +1558,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #undef h
 #undef att
 #undef smem_s
+#undef lut_s
 #undef tmem
 #undef pol
 #undef keep
@@ -1523,13 +1570,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #undef hasC
 #undef hasD
 #undef hasE
-#undef tileA
-#undef tileC
 #undef splitC
-#undef tileE
 #undef splitE
 #undef presE
-#undef uD
 #undef srcA
 #undef srcC
 #undef srcD

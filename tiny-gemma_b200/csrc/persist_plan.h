@@ -21,7 +21,7 @@ struct PsPhase {
 	int nsplit;  // K-splits across CTAs
 	int ntiles;  // column tiles
 	int units;   // ntiles * nsplit
-	int bytes;   // bytes of a unit
+	int bytes;   // bytes of a unit: weights, then the scales of its columns
 	int cta0;    // CTA of unit 0
 	int rows;    // nmat * ncol
 	int segs, mt, tiles;
@@ -117,7 +117,7 @@ bool ps_plan(PsPhase *out, int K, int N, int nmat, int G, int max_bytes, const s
 			ph.nsplit = ns;
 			ph.ntiles = N / ncol;
 			ph.units = ph.ntiles * ns;
-			ph.bytes = ph.rows * nq * 4;
+			ph.bytes = ph.rows * nq * 4 + ph.rows * 4;
 			if (ph.units > G || ph.bytes > max_bytes) continue;
 			const double clk = ps_mma_plan(&ph);
 			if (clk < 0) continue;

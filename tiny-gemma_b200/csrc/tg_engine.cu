@@ -1156,6 +1156,8 @@ int persist_setup(tg_state *s) {
 	a.nch_local = std::min(chmax, std::max(0, env_int("TG_PS_NCH_LOCAL", 0)));
 	a.nch_global = std::min(chmax, std::max(0, env_int("TG_PS_NCH_GLOBAL", 0)));
 	a.slots_local = c.n_pos_local;
+	a.slots_global = s->max_pos_global;
+	a.merge_heads = AT_NH / a.C.nsplit;
 	const int npres = G - a.E.units;
 	if (D / 4 + npres > PS_THREADS || G < 16) return fail(TG_ESHAPE, "persistent kernel: grid too small for the down-projection plan");
 	// lm_head: tiles of 128 columns; ring stages of at most 40 KB
@@ -1203,12 +1205,12 @@ int persist_setup(tg_state *s) {
 	a.off_C = off;
 	off = up(off + a.C.bytes);
 	a.off_D = off;
-	a.off_E = off + a.Dp.bytes;  // contiguous with the up/gate region: the lm_head ring and the sampler staging overlay both
+	a.off_E = up(off + a.Dp.bytes);  // behind the up/gate region: the lm_head ring and the sampler staging overlay both
 	cudaFuncAttributes fa{};
 	TG_CUDA(cudaFuncGetAttributes(&fa, decode_persist_kernel<true>));
 	// the ring takes five stages where the shared memory has room for them (4 at 1B: its units fill the memory)
 	const int room = smem_max - int(fa.sharedSizeBytes) - 128 - off;
-	const int region = std::max(std::max(a.Dp.bytes + a.E.bytes, 3072 * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
+	const int region = std::max(std::max(a.off_E + a.E.bytes - a.off_D, 3072 * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
 	off = up(off + region);
 	a.lm_stages = std::min(8, region / a.lm_stage_bytes);
 	if (a.lm_stages < 2) return fail(TG_ESHAPE, "persistent kernel: lm_head ring does not fit");
@@ -1329,7 +1331,7 @@ int ensure_persist_tiles(tg_state *s) {
 	}
 	cudaStream_t st = s->stream;
 	auto run = [&](int8_t *dst, const QW &w, const PsPhase &ph, int tile0, int row0) {
-		retile_units_kernel<<<8 * g_num_sms, 256, 0, st>>>(dst, w.q, w.N, ph, tile0, w.N / ph.ncol, row0);
+		retile_units_kernel<<<8 * g_num_sms, 256, 0, st>>>(dst, w.q, &ph == &a.lm ? nullptr : w.s, w.N, ph, tile0, w.N / ph.ncol, row0);
 		count_launch();
 	};
 	for (int l = 0; l < L; l++) {
