@@ -1,4 +1,4 @@
-"""Host-side model of the GPU's exact parallel inverse CDF (cdf_walk_maps and cdf_cross_warp in
+"""Host-side model of the GPU's exact parallel inverse CDF (cdf_walk_maps in
 tiny-gemma_b200/csrc/kernels_sampler.cuh), checked against the sequential fp32 chain of
 ops::minp_logits (reference ops.hpp:849-857).
 

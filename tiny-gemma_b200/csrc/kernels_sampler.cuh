@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(SR_THREADS) argmax_kernel(SampleArgs a, unsign
 // with a0 = a1 = round(p/u) except on an exact tie, where the pair encodes round-half-even. Such
 // maps compose into maps of the same form (the parity of the result follows from the parity of the
 // input), so a prefix scan of (a0, a1) pairs gives every partial sum of the chain, bit for bit.
-// When a sum would leave the binade, that one addition is done in fp32 and the scan restarts behind
+// A block in which the sum leaves the binade is added up element by element, and the maps go on behind
 // it with the new u. Sums saturate far above every threshold, so they stay monotone.
 struct CdfFn {
 	int a0, a1;
@@ -123,143 +123,56 @@ __device__ __forceinline__ CdfFn cdf_element(float p, float inv_u) {
 	return f;
 }
 
-// The first elements of a row are added one by one by a single thread: the running sum starts at
-// zero and changes binade about log2(position) times, and every change would cost a whole scan
-// round (≈ 1 us, the time of ≈ 400 sequential additions). p >= 0, so the sum never decreases and
-// a group of 8 is searched only when its last partial sum has reached randf. p is 16-byte aligned.
-__device__ __forceinline__ void cdf_cross_seq(const float *p, int end, float randf, float &cum, int &pos, int &res) {
-	float c = cum;
-	int i = pos;
-	float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-	if (i + 8 <= end) {
-		a = *reinterpret_cast<const float4 *>(p + i);
-		b = *reinterpret_cast<const float4 *>(p + i + 4);
-	}
-	for (; i + 8 <= end; i += 8) {
-		float cs[8];
-		cs[0] = c + a.x;
-		cs[1] = cs[0] + a.y;
-		cs[2] = cs[1] + a.z;
-		cs[3] = cs[2] + a.w;
-		cs[4] = cs[3] + b.x;
-		cs[5] = cs[4] + b.y;
-		cs[6] = cs[5] + b.z;
-		cs[7] = cs[6] + b.w;
-		if (i + 16 <= end) {  // (the next group is on its way while this one's chain of additions runs)
-			a = *reinterpret_cast<const float4 *>(p + i + 8);
-			b = *reinterpret_cast<const float4 *>(p + i + 12);
-		}
-		if (cs[7] >= randf) {
-			int k = 7;
+// A block of 256 elements in shared memory (16-byte aligned, zeros behind the row's end), cum the running sum before it. The
+// elements are added one by one, by every lane of the warp alike. Returns the first index with fl(cum + p[0] + ... + p[i]) >= randf
+// inside the block or -1; cum becomes the sum behind the last element consumed. p >= 0: the sum never decreases, so a group of 32
+// is searched only when its last partial sum has reached randf (or is NaN: then maybe none has). The chain of additions is
+// what bounds it: 1200 clk with the next 32 elements on their way, 3200 with the next 8. (A scan of the elements' maps per binade
+// takes 1900 clk, twice for one change of the binade.)
+constexpr int CDF_BLK = 256;
+__device__ __forceinline__ int cdf_cross_block(const float *p, float &cum, float randf) {
+	const uint32_t s = uint32_t(__cvta_generic_to_shared(p));
+	auto load = [&](float4 (&v)[8], int i) {
 #pragma unroll
-			for (int t = 6; t >= 0; t--)
-				if (cs[t] >= randf) k = t;
-			res = i + k;
-			cum = cs[k];
-			pos = i + k + 1;
-			return;
+		for (int k = 0; k < 8; k++)
+			asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[k].x), "=f"(v[k].y), "=f"(v[k].z), "=f"(v[k].w) : "r"(s + 4u * i + 16u * k) : "memory");
+	};
+	auto add = [&](const float4 (&v)[8], float c) {
+#pragma unroll
+		for (int k = 0; k < 8; k++) c = (((c + v[k].x) + v[k].y) + v[k].z) + v[k].w;
+		return c;
+	};
+	float4 a[8], b[8];
+	load(a, 0);
+	float c = cum;
+#pragma unroll 1
+	for (int i = 0; i < CDF_BLK; i += 64) {
+		float before = c;
+		load(b, i + 32);
+		c = add(a, c);
+		int at = i;
+		if (c < randf) {
+			before = c;
+			if (i + 64 < CDF_BLK) load(a, i + 64);
+			c = add(b, c);
+			at = i + 32;
 		}
-		c = cs[7];
-	}
-	for (; i < end; i++) {
-		c += p[i];
-		if (c >= randf) {
-			res = i;
-			cum = c;
-			pos = i + 1;
-			return;
+		if (!(c < randf)) {  // in the 32 elements from `at` on
+#pragma unroll 1
+			for (int k = at; k < at + 32; k++) {
+				before += p[k];
+				if (before >= randf) {
+					cum = before;
+					return k;
+				}
+			}
+			if (at == i) {  // (a NaN: nothing is reached any more, but the chain goes on)
+				if (i + 64 < CDF_BLK) load(a, i + 64);
+				c = add(b, c);
+			}
 		}
 	}
 	cum = c;
-	pos = i;
-}
-
-// A block of at most 256 elements by one warp: p[0..n) in shared memory, 16-byte aligned, n a multiple of 8, cum the running sum
-// before p[0]; all lanes call it with the same arguments. Returns the first index with fl(cum + p[0] + ... + p[i]) >= randf inside
-// the block or -1; cum becomes the sum behind the last element consumed. seq: add the elements one by one (the start of a row).
-constexpr int CDF_BLK = 256;
-__device__ __forceinline__ int cdf_cross_warp(const float *p, int n, float &cum, float randf, bool seq) {
-	const int lane = threadIdx.x & 31, base = 8 * lane;
-	if (seq) {
-		int pos = 0, res = -1;
-		float c = cum;
-		if (lane == 0) cdf_cross_seq(p, n, randf, c, pos, res);
-		cum = __shfl_sync(0xffffffffu, c, 0);
-		return __shfl_sync(0xffffffffu, res, 0);
-	}
-	float x[8];
-#pragma unroll
-	for (int k = 0; k < 8; k++) x[k] = base < n ? p[base + k] : 0.0f;
-	int pos = 0;
-#pragma unroll 1
-	for (int guard = 0; pos < n && guard < n + 8; guard++) {  // every round consumes at least one element
-		const int e = int((__float_as_uint(cum) >> 23) & 0xffu) - 127;
-		if (!(cum >= 7.888609e-31f) || e > 120) {
-			// zero, tiny, inf or NaN: plain fp32 steps until the sum is an ordinary number
-			int res = -1;
-			for (; pos < n && res < 0; pos++) {
-				cum += p[pos];
-				if (cum >= randf) res = pos;
-				if (cum >= 7.888609e-31f && cum < 1e36f) {
-					pos++;
-					break;
-				}
-			}
-			if (res >= 0) return res;
-			continue;
-		}
-		const float u = __uint_as_float(unsigned(e - 23 + 127) << 23), inv_u = __uint_as_float(unsigned(23 - e + 127) << 23);
-		const int S0 = int(cum * inv_u);
-		const float y = randf * inv_u;
-		const int Tmin = min((y < 33554432.0f) ? int(ceilf(y)) : CDF_BIG, 1 << 24);
-		CdfFn el[8], inc{0, 0};
-#pragma unroll
-		for (int k = 0; k < 8; k++) {
-			el[k] = CdfFn{0, 0};
-			if (base + k >= pos && base + k < n) el[k] = cdf_element(x[k], inv_u);
-			inc = cdf_compose(inc, el[k]);
-		}
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			CdfFn prev;
-			prev.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
-			prev.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
-			if (lane >= o) inc = cdf_compose(prev, inc);
-		}
-		const int end = cdf_apply(inc, S0);  // the sum behind this lane's elements
-		int S = __shfl_up_sync(0xffffffffu, end, 1);
-		if (lane == 0) S = S0;
-		const unsigned hit = __ballot_sync(0xffffffffu, end >= Tmin);
-		if (!hit) {
-			cum = float(__shfl_sync(0xffffffffu, end, 31)) * u;  // exact: below 2^24
-			return -1;
-		}
-		int at = -1, before = 0, after = 0;
-		float pe = 0.0f;
-#pragma unroll
-		for (int k = 0; k < 8; k++) {
-			const int nx = cdf_apply(el[k], S);
-			if (at < 0 && nx >= Tmin) {
-				at = base + k;
-				before = S;
-				after = nx;
-				pe = x[k];
-			}
-			S = nx;
-		}
-		const int src = __ffs(hit) - 1;
-		at = __shfl_sync(0xffffffffu, at, src);
-		before = __shfl_sync(0xffffffffu, before, src);
-		after = __shfl_sync(0xffffffffu, after, src);
-		pe = __shfl_sync(0xffffffffu, pe, src);
-		if (after < (1 << 24)) {  // the sum reached randf inside the binade
-			cum = float(after) * u;
-			return at;
-		}
-		cum = float(before) * u + pe;  // the one addition that leaves the binade
-		if (cum >= randf) return at;
-		pos = at + 1;
-	}
 	return -1;
 }
 
@@ -271,7 +184,7 @@ __device__ __forceinline__ int cdf_cross_warp(const float *p, int n, float &cum,
 // Steps 1-5 are data-parallel. Step 6 must reproduce a *sequential* fp32 sum
 // (fp32 addition is not associative, and the crossing index depends on the
 // rounding): the maps above evaluate that chain exactly, in parallel
-// (cdf_walk_maps, cdf_cross_warp, cdf_walk_row).
+// (cdf_walk_maps, cdf_walk_row).
 
 // Any number of rows, each spread over V / SR_PART CTAs: four kernels (row maximum; exponentials and segment sums;
 // scaling and segment maps; the walk). One CTA per row took ~1 ms for a row of 262144: four passes over 1 MB and
@@ -473,14 +386,14 @@ __device__ __forceinline__ int cdf_walk_row(Seg seg_map, Blk blk_map, const floa
 			if (b >= mb) break;
 			const int left = min(CDF_BLK, m - CDF_BLK * b);
 			__syncwarp();
-			if (8 * lane < left) {
+			{
 				const float4 *src = reinterpret_cast<const float4 *>(p + size_t(c) * seg_len + CDF_BLK * b + 8 * lane);
-				const float4 v0 = __ldcg(src), v1 = __ldcg(src + 1);
+				const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), v0 = 8 * lane < left ? __ldcg(src) : z, v1 = 8 * lane < left ? __ldcg(src + 1) : z;
 				reinterpret_cast<float4 *>(chunk + 8 * lane)[0] = v0;
 				reinterpret_cast<float4 *>(chunk + 8 * lane)[1] = v1;
 			}
 			__syncwarp();
-			const int r = cdf_cross_warp(chunk, left, cum, randf, c == 0 && b == 0);
+			const int r = cdf_cross_block(chunk, cum, randf);
 			if (r >= 0) return c * seg_len + CDF_BLK * b + r;
 		}
 	}

@@ -960,7 +960,7 @@ int mega_setup(tg_state *s) {
 	off = up(off + a.C.bytes);
 	a.off_D = off;
 	a.off_E = off + a.Dp.bytes;  // contiguous with D: the lm_head ring overlays both
-	off = up(off + std::max(a.Dp.bytes + a.E.bytes, std::max(ring, 8192 * 4)));
+	off = up(off + std::max(a.Dp.bytes + a.E.bytes, std::max(ring, minp_grid_floats(V, G) * 4)));
 	a.off_h = off;
 	off = up(off + D * 4);
 	a.off_xs = off;
@@ -1210,7 +1210,7 @@ int persist_setup(tg_state *s) {
 	TG_CUDA(cudaFuncGetAttributes(&fa, decode_persist_kernel<true>));
 	// the ring takes five stages where the shared memory has room for them (4 at 1B: its units fill the memory)
 	const int room = smem_max - int(fa.sharedSizeBytes) - 128 - off;
-	const int region = std::max(std::max(a.off_E + a.E.bytes - a.off_D, 3072 * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
+	const int region = std::max(std::max(a.off_E + a.E.bytes - a.off_D, minp_grid_floats(V, G) * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
 	off = up(off + region);
 	a.lm_stages = std::min(8, region / a.lm_stage_bytes);
 	if (a.lm_stages < 2) return fail(TG_ESHAPE, "persistent kernel: lm_head ring does not fit");
