@@ -60,10 +60,10 @@ constexpr uint32_t PS_BULK_PIECE = 16384;
 constexpr unsigned PS_EMPTY = 0xFFFFFFFFu;  // "not written yet": a NaN no computation produces
 
 constexpr int PS_TMEM = 64;              // TMEM columns: 16 per tile of a unit, or two accumulators of the lm_head
+constexpr int PS_ACT = 3;                // quads of a thread in the down projection's prologue, at most
 constexpr int PS_LUT = 1024;             // largest GeLU table that is kept in shared memory
 
 struct PsLayer {
-	const float *sq, *sk, *sv, *so, *su, *sg, *sd;  // per-column scales
 	const float *rmsq, *rmsk, *attn_pre, *attn_post, *mlp_pre, *mlp_post;
 	float *kcache, *vcache;
 	int slots, is_local;
@@ -82,7 +82,7 @@ struct PsArgs {
 	int L, D, I, V, QD, KD;
 	PsPhase A, C, Dp, E;
 	// lm_head: column tiles of 128 columns; a tile's rows arrive as lm_nchunk ring stages of lm_steps * 32 rows
-	int lm_steps, lm_nchunk, lm_ntiles, lm_stages, lm_stage_bytes;
+	int lm_steps, lm_nchunk, lm_ntiles, lm_stages, lm_stage_bytes, lm_pre;
 	PsPhase lm;  // (the digits' layout: one segment)
 	const float *lm_scale, *final_norm;
 	const int8_t *wte;
@@ -100,6 +100,7 @@ struct PsArgs {
 	//                                      one presence word for every CTA without a down unit
 	float *ll;
 	int ll_stride, ll_qkv, ll_att, ll_op, ll_act, ll_dn, ll_pres;
+	uint32_t piece_D, piece_E;  // bytes of a quarter of an up/gate and of a down unit
 	int merge_heads;  // heads whose attention output an O unit multiplies (4 / C.nsplit)
 	int nch_max, nch_local, nch_global;  // cache chunks per head: at most; a number given for sliding-window and global layers (0: by rule)
 	int slots_local, slots_global;
@@ -122,7 +123,6 @@ struct PsArgs {
 	int dbg_cta, dbg_cap;
 	long long wait_clocks;  // SM clocks before a wait gives up
 	int poll_ns;            // sleep between two rounds of a hand-off poll
-	int sched;              // 0: up/gate and down units of layer l+1 requested in phase E of layer l; 1: units of layer l requested after the Q|K|V product of layer l
 	long long *gt;  // optional: [CTA][12] global-timer marks of one layer (DBG instantiation)
 	int *beacon;    // optional (mapped host memory): [CTA][16] progress marks of every warp, for diagnosing a stall
 	int fault_cta;  // test hook: this CTA withholds its down-projection hand-off (-1: none); the waits then run out
@@ -304,7 +304,6 @@ __device__ __forceinline__ void ps_stsf(uint32_t addr, float v) { asm volatile("
 // of a layer is spilled.
 struct PsUnit {
 	uint64_t da[PS_TILES], db[PS_TILES];  // descriptors of a tile's first MMA: weights, digits
-	uint32_t id;
 	int tiles, steps, mt;
 	uint32_t x_s, seg_mul;  // digits: shared-window address and layout
 	int seg_q, x_sbo;
@@ -385,11 +384,19 @@ __device__ __forceinline__ float ps_join(const int4 &s) {
 // what a CTA's place in the grid fixes for the whole launch (kept in shared memory, read where it is used)
 struct PsCta {
 	const int8_t *srcA, *srcC, *srcD, *srcE;
+	uint64_t policy_first, policy_last;  // L2 evict-first (weights) and evict-last (what every token reads again)
 	int splitC, splitE, presE, has;
 	uint32_t tm;  // TMEM base (the word that tcgen05.alloc wrote, which the compiler does not see written: read once, volatile)
 };
+// what one token leaves to the next (in shared memory, written by thread 0 between barriers: a register that lives across the
+// calls of a layer is spilled, and the L1 beside 224 KB of shared memory does not hold the spills)
+struct PsLive {
+	uint32_t plm, pemp, acc_n;  // lm_head: parities of the ring's barriers, tiles so far
+	unsigned epoch;             // grid barriers passed
+	int n_logged, tok, pos;
+};
 // fields of a phase's entry; `warp` fills its own
-__device__ __forceinline__ void ps_fill_unit(const PsPhase &ph, PsUnit *u, int warp, uint32_t smem_s, int off_tile, int dst) {
+__device__ __noinline__ void ps_fill_unit(const PsPhase &ph, PsUnit *u, int warp, uint32_t smem_s, int off_tile, int dst) {
 	const int t = warp >> 2;
 	if (t < ph.tiles) {
 		int r0, col;
@@ -402,7 +409,6 @@ __device__ __forceinline__ void ps_fill_unit(const PsPhase &ph, PsUnit *u, int w
 			u->da[i] = ps_desc(smem_s + uint32_t(off_tile + i * ph.steps * ph.mt * 32), ph.mt * 16, 128);
 			u->db[i] = ps_desc(smem_s + uint32_t(ph.off_x + (ps_tile_segment(ph.rows, ph.mt, i) / 2) * ph.x_sbo), PS_XCH, ph.x_sbo);
 		}
-		u->id = ps_idesc(ph.mt);
 		u->tiles = ph.tiles;
 		u->steps = ph.steps;
 		u->mt = ph.mt;
@@ -419,14 +425,53 @@ __device__ __forceinline__ void ps_fill_unit(const PsPhase &ph, PsUnit *u, int w
 		u->dst = dst;
 	}
 }
-// column c of a unit: the segments' digit sums added (exact) and joined
-__device__ __forceinline__ float ps_column(const PsUnit *u, int c) {
-	uint32_t p = u->acc_s + 16u * uint32_t(c);
-	const uint32_t step = 16u * uint32_t(u->rows);
-	const int segs = u->segs;
+// lut::GeLUTable::lookup (reference ops.hpp:41-51); tab_s: the table in shared memory where it fits there
+__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint32_t tab_s, uint64_t keep) {
+	int idx;
+	if (!t.index(x, idx)) return 0.0f;
+	if (idx >= t.size) return x;
+	return t.size <= PS_LUT ? ps_ldsf(tab_s + 4u * idx) : ps_ldk(t.table + idx, keep);
+}
+// What a thread needs for its part of a unit's product, fetched before the phase's prologue polls: behind the prologue every
+// shared-memory access counts (~30 clk, five of them in a row before the first MMA).
+struct PsRun {
+	uint64_t da, db;          // issuing warps: descriptors of the first MMA
+	uint32_t d, taddr, acc;   // accumulator; where this warp's sums are and go
+	int steps, mt;            // steps: 0 where this warp's tile does not exist
+	uint32_t col;             // this thread's column: sums of its first segment
+	int cstep, segs, ncol, two;
+	float s0, s1;             // its scales
+};
+// The issuing warps, and the ones that read column scales, wait for the unit here (a completed test takes ~200 clk).
+__device__ __forceinline__ PsRun ps_prepare(const PsW &w, int where, const PsUnit *u, uint32_t tmem, uint64_t *bar_w, uint32_t pw) {
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = warp >> 2;
+	PsRun r;
+	r.ncol = u->ncol;
+	if ((warp & 3) == 0 || 32 * warp < r.ncol) ps_wait_bulk(w, where, bar_w, pw);
+	r.da = u->da[t];
+	r.db = u->db[t];
+	r.d = tmem + 16u * t;
+	r.mt = u->mt;
+	r.steps = t < u->tiles ? u->steps : 0;
+	const int m = u->ep[warp];
+	r.taddr = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m & 0xFF);
+	r.acc = u->acc_s + 16u * uint32_t((m >> 8) + lane);
+	r.col = u->acc_s + 16u * uint32_t(tid);
+	r.cstep = 16 * u->rows;
+	r.segs = u->segs;
+	r.two = u->two;
+	r.s0 = r.s1 = 0.0f;
+	if (tid < r.ncol) {  // (before the barrier behind which the unit may be refilled)
+		r.s0 = ps_ldsf(u->scale_s + 4u * tid);
+		if (r.two) r.s1 = ps_ldsf(u->scale_s + 4u * (r.ncol + tid));
+	}
+	return r;
+}
+// the segments' digit sums of a column added (exact) and joined
+__device__ __forceinline__ float ps_column(const PsRun &r, uint32_t p) {
 	int4 s = make_int4(0, 0, 0, 0);
 #pragma unroll 4
-	for (int i = 0; i < segs; i++, p += step) {
+	for (int i = 0; i < r.segs; i++, p += r.cstep) {
 		const uint4 v = ps_lds128(p);
 		s.x += int(v.x);
 		s.y += int(v.y);
@@ -435,68 +480,54 @@ __device__ __forceinline__ float ps_column(const PsUnit *u, int c) {
 	}
 	return ps_join(s);
 }
-// lut::GeLUTable::lookup (reference ops.hpp:41-51); tab_s: the table in shared memory where it fits there
-__device__ __forceinline__ float ps_gelu(const GeluLut &t, float x, uint32_t tab_s, uint64_t keep) {
-	int idx;
-	if (!t.index(x, idx)) return 0.0f;
-	if (idx >= t.size) return x;
-	return t.size <= PS_LUT ? ps_ldsf(tab_s + 4u * idx) : ps_ldk(t.table + idx, keep);
-}
 // One unit's product: dst[c] = column sum * scale, or (up and gate) GeLU(gate) * up. Called by the whole CTA behind the
-// barrier that ends the prologue (the digits' writers have fenced, the issuing warps have waited for the unit). Warp 4 t issues tile
+// barrier that ends the prologue (the digits' writers have fenced). Warp 4 t issues tile
 // t's MMAs into its own 16 TMEM columns (one accumulator per issuing warp), warps 4 t .. 4 t + 3 read them back, thread c
 // publishes column c. One store instruction per 32 columns: scattered over the warps, 16 bytes each, the words of a line that 148
 // CTAs poll take 450 clk longer to arrive. pm: parity of bar_m[t], returned. Behind its barrier nobody reads the unit or the digits any
 // more. Measured from the prologue's barrier to the values in registers (1B: 27 MMAs of up and gate, 27 of down, 4 of
 // O, 9 of q|k|v): about 430 clk + 38 per MMA of 128 rows, 23 per one of 64; dp4a loops over the same tiles took 2400, 1450,
 // 850 and 1000 clk and 400 to 600 more to reduce over the lanes.
-__device__ __noinline__ uint32_t ps_unit(const PsW w, int where, const PsUnit *u, uint32_t tmem, uint64_t *bar_w, uint32_t pw, uint64_t *bar_m, uint32_t pm,
-                                         const float *s_xscale, float *dst, const GeluLut lut, uint32_t lut_s, uint64_t keep) {
-	__builtin_assume(__isShared(u));
-	__builtin_assume(__isShared(s_xscale));
+__device__ __forceinline__ uint32_t ps_unit(const PsW &w, int where, const PsRun &r, uint64_t *bar_m, uint32_t pm, const float *xscale, float *dst, const GeluLut &lut, uint32_t tab_s, uint64_t hint) {
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = warp >> 2;
-	float s0 = 0.0f, s1 = 0.0f;
-	if (32 * warp < u->ncol && (warp & 3) != 0) ps_wait_bulk(w, where, bar_w, pw);  // (the issuing warps have waited)
-	if (tid < u->ncol) {  // column scales: read before the barrier behind which the unit may be refilled
-		s0 = ps_ldsf(u->scale_s + 4u * tid);
-		if (u->two) s1 = ps_ldsf(u->scale_s + 4u * (u->ncol + tid));
-	}
-	if (t < u->tiles) {
+	if (r.steps) {
 		if ((warp & 3) == 0) {
 			tc_fence_after();
-			const uint64_t da = u->da[t], db = u->db[t];
-			const uint32_t id = u->id, d = tmem + 16u * t;
-			const int steps = u->steps;
-			const uint64_t step = uint64_t(u->mt * 2);
+			const uint64_t step = uint64_t(r.mt * 2);
+			const uint32_t id = ps_idesc(r.mt);
 			if (tc_elect()) {
 #pragma unroll 1
-				for (int i = 0; i < steps; i++) i8_mma<1>(d, da + uint64_t(i) * step, db + uint64_t(i * (2 * PS_XCH / 16)), id, i > 0 ? 1u : 0u);
+				for (int i = 0; i < r.steps; i++) i8_mma<1>(r.d, r.da + uint64_t(i) * step, r.db + uint64_t(i * (2 * PS_XCH / 16)), id, i > 0 ? 1u : 0u);
 				i8_commit<1>(&bar_m[t]);
 			}
 			__syncwarp();
 		}
-		const int m = u->ep[warp];
-		const uint32_t taddr = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(m & 0xFF), acc = u->acc_s + 16u * uint32_t((m >> 8) + lane);
-		const bool mine = 4 * lane < u->mt;
 		ps_wait_bulk(w, where, &bar_m[t], pm);
 		pm ^= 1u;
 		__syncwarp();
 		tc_fence_after();
-		const int4 v = ps_tmem_ld4(taddr);
-		if (mine) asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(acc), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+		const int4 v = ps_tmem_ld4(r.taddr);
+		if (4 * lane < r.mt) asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(r.acc), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 		tc_fence_before();
 	}
 	__syncthreads();
-	if (tid < u->ncol) {
-		const float xs = *s_xscale;
-		float y = (ps_column(u, tid) * xs) * s0;
-		if (u->two) y = ps_gelu(lut, (ps_column(u, u->ncol + tid) * xs) * s1, lut_s, keep) * y;
+	if (tid < r.ncol) {
+		const float xs = *xscale;
+		float y = (ps_column(r, r.col) * xs) * r.s0;
+		if (r.two) y = ps_gelu(lut, (ps_column(r, r.col + 16u * r.ncol) * xs) * r.s1, tab_s, hint) * y;
 		if (dst) ps_st(dst + tid, y);
 	}
 	return pm;
 }
 
 // A CTA's unit is one contiguous block of the re-tiled copy: one bulk copy. Called by one lane.
+// Piece `i` of a unit, `size` bytes each; the first one announces all of the unit's bytes to its barrier. Called by one lane.
+__device__ __forceinline__ void ps_issue_piece(uint8_t *dst, const int8_t *src, uint32_t bytes, uint32_t size, int i, uint64_t *bar, uint64_t hint, const int *abort_flag) {
+	if (*(volatile const int *)abort_flag) return;
+	const uint32_t at = uint32_t(i) * size;
+	if (i == 0) ps_mbar_expect(bar, bytes);
+	if (at < bytes) ps_bulk(dst + at, src + at, min(size, bytes - at), bar, hint);
+}
 __device__ __noinline__ void ps_issue(uint8_t *dst, const int8_t *src, uint32_t bytes, uint64_t *bar, uint64_t pol, const int *abort_flag) {
 	if (*(volatile const int *)abort_flag) return;  // a CTA that gave up starts no new copies
 	// (no proxy fence: the region was only READ through the generic proxy, and those loads have completed —
@@ -550,15 +581,11 @@ __device__ __forceinline__ float ps_inv_rms(float sumsq, float inv_dim) {
 // If part: t[d] = sum_s part[s][d] (scaled partial sums, polled until complete; threads past D/4 poll
 // the presence words);  h += rmsnorm(t; w_post). Then y = rmsnorm(h; w_pre), quantised with *s_xscale = 2^(e - 30).
 // Every CTA computes the same bits. D <= 4 * PS_THREADS. Thread t owns elements 4t..4t+3, which are quad t. bred: 3 * PS_NW
-// floats, 16-byte aligned. bar_w, pw: barrier of the unit that comes next (null: none); its issuing warps wait for it here, under the
-// hand-off (a completed test takes ~200 clk).
-__device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h, const PsUnit *u, uint64_t *bar_w, uint32_t pw, float *bred, float *s_xscale,
+// floats, 16-byte aligned.
+__device__ __forceinline__ void ps_resnorm(const PsW w, int where, int D, float *h, const PsUnit *u, float *bred, float *s_xscale,
                                         const float *part, int nsplit, const float *pres, int npres, const float *w_post,
                                         const float *w_pre, uint64_t keep, float *x_out) {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	__builtin_assume(__isShared(h));
-	__builtin_assume(__isShared(u));
-	__builtin_assume(__isShared(s_xscale));
 	// the norm weights are L2-resident (evict-last): requested together with the first poll loads
 	float4 wpost = make_float4(0.f, 0.f, 0.f, 0.f), wpre = wpost;
 	if (4 * tid < D) {
@@ -569,7 +596,6 @@ __device__ __noinline__ void ps_resnorm(const PsW w, int where, int D, float *h,
 	const float invD = 1.0f / float(D);
 	const bool in = 4 * tid < D;
 	const uint32_t xaddr = ps_xaddr(u, tid);
-	if (bar_w && (warp & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
 	float4 hv = make_float4(0.f, 0.f, 0.f, 0.f);
 	if (in) hv = *reinterpret_cast<const float4 *>(h + 4 * tid);
 	if (part) {
@@ -663,20 +689,15 @@ __device__ __forceinline__ void ps_norm_rope(const float4 &lo4, const float4 &hi
 // Phase C prologue: merge the attention partials of `hp` heads starting at head h0 over `nch` chunks
 // into the normalised output (reference ops.hpp:316-357 keeps it normalised per step; the split form
 // divides once), quantise it.
-__device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, const PsUnit *u, uint64_t *bar_w,
-                                           uint32_t pw, float *bred, float *s_xscale) {
+__device__ __forceinline__ void ps_attn_merge(const PsW w, int where, const float *att_ll, int h0, int hp, int nch, float *scr, const PsUnit *u, float *bred,
+                                              float *s_xscale) {
 	const int tid = threadIdx.x;
-	__builtin_assume(__isShared(scr));
-	__builtin_assume(__isShared(u));
-	__builtin_assume(__isShared(bred));
-	__builtin_assume(__isShared(s_xscale));
 	// thread = (chunk group cg, float4 column it of the hp * 64); hp is 1, 2 or 4
 	const int sh = 6 + (hp >> 1), items = 1 << sh;
 	const int ncg = hp == 1 ? PS_THREADS / 64 : (hp == 2 ? PS_THREADS / 128 : PS_THREADS / 256);
 	const int cg = tid >> sh, it = tid & (items - 1);
 	const int hl = it >> 6, j = it & 63;
 	const uint32_t xaddr = ps_xaddr(u, it);
-	if (((tid >> 5) & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
 	float m = -INFINITY, l = 0.0f;
 	float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 	if (cg < ncg) {
@@ -773,21 +794,17 @@ __device__ __noinline__ void ps_attn_merge(const PsW w, int where, const float *
 }
 
 // Phase E prologue: this CTA's rows of the activation vector (nq quads from act), polled until
-// complete, quantised. nq <= 5 * PS_THREADS.
-__device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, const PsUnit *u, uint64_t *bar_w, uint32_t pw, float *bred, float *s_xscale) {
+// complete, quantised. nq <= PS_ACT * PS_THREADS.
+__device__ __forceinline__ void ps_act_quant(const PsW w, int where, const float *act, int nq, const PsUnit *u, float *bred, float *s_xscale) {
 	const int tid = threadIdx.x;
-	__builtin_assume(__isShared(u));
-	__builtin_assume(__isShared(bred));
-	__builtin_assume(__isShared(s_xscale));
-	if (((tid >> 5) & 3) == 0) ps_wait_bulk(w, where, bar_w, pw);
-	float4 v[5];
+	float4 v[PS_ACT];
 	int spins = 0;
 	long long t0 = 0;
 	bool ok;
 	do {
 		ok = true;
 #pragma unroll
-		for (int q = 0; q < 5; q++) {
+		for (int q = 0; q < PS_ACT; q++) {
 			const int i = q * PS_THREADS + tid;
 			v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 			if (i < nq) v[q] = ps_ld4(act + 4 * i);
@@ -796,11 +813,11 @@ __device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *a
 	} while (!ok && ps_retry(w, where, spins, t0));
 	float mx = 0.0f;
 #pragma unroll
-	for (int q = 0; q < 5; q++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[q].x), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w))));
+	for (int q = 0; q < PS_ACT; q++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[q].x), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w))));
 	const float M = ps_block_max(mx, bred);
 	const float qs = ps_qmul(M);
 #pragma unroll
-	for (int q = 0; q < 5; q++) {
+	for (int q = 0; q < PS_ACT; q++) {
 		const int i = q * PS_THREADS + tid;
 		if (i < nq) ps_quantise(v[q], qs, ps_xaddr(u, i));
 	}
@@ -815,12 +832,10 @@ __device__ __noinline__ void ps_act_quant(const PsW w, int where, const float *a
 // 128 + 4 lane..), merge of the 12 warps, (o[256], m, l) published to prow. att: 16 KB of scratch,
 // wml: 2 * PS_NW floats. Every warp norms and rotates q itself, the one that owns the new row k too: one barrier less, and
 // no values through shared memory. Reference: ops.hpp:224-370 (attention_decode), decode.hpp:203-211 (RoPE).
-__device__ __noinline__ void ps_attention(const PsW w, int where, float *kcache, float *vcache, const float *rmsq, const float *rmsk,
+__device__ __forceinline__ void ps_attention(const PsW w, int where, float *kcache, float *vcache, const float *rmsq, const float *rmsk,
                                           const float *cosr, const float *sinr, const float *qkv_ll, int QD, int hh, float *prow, int j0,
                                           int j1, int slot, float *att, float *wml, uint64_t keep) {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	__builtin_assume(__isShared(att));
-	__builtin_assume(__isShared(wml));
 	float *wo = att, *qraw = att + PS_NW * AT_HD;
 	float *wm = wml, *wl = wml + PS_NW;
 	// The cache rows do not depend on this token's q|k|v: a warp's first two rows are requested before
@@ -1197,43 +1212,223 @@ if (a.sampler == 0) {
 #define PS_STAMP()                                                       \
 	do {                                                                 \
 		if constexpr (DBG) {                                             \
-			if (dbg_on && dbg_n < a.dbg_cap) a.dbg[dbg_n++] = clock64(); \
+			if (dbg_on && s_dbg_n < a.dbg_cap) a.dbg[s_dbg_n++] = clock64(); \
 		}                                                                \
 	} while (0)
 
-template <bool DBG>
-__global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __grid_constant__ PsArgs a) {
-	extern __shared__ uint8_t smem_raw[];
-	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(smem_raw) + 127) & ~uintptr_t(127));  // the host adds 128 bytes of slack
-	__shared__ uint64_t bar_A, bar_C, bar_D, bar_E, bar_lm[8], emp_lm[8];
-	__shared__ uint64_t bar_m[PS_TILES], acc_full[2], acc_free[2];  // MMAs of a unit's tile; the lm_head's two accumulators
-	__shared__ __align__(16) float bred[3 * PS_NW];
-	__shared__ uint32_t s_tmem;
-	__shared__ float s_xscale;
-	__shared__ int s_abort;
-	__shared__ float s_f[8];
-	__shared__ int s_i[4];
-	__shared__ int s_cdf[2 * PS_NW + 8];
-	__shared__ float wm[2 * PS_NW];  // per-warp (m, l) of the attention merge; also the sampler's per-warp maxima
-	__shared__ PsLayer s_ly[PS_MAX_LAYERS];
-	__shared__ PsUnit s_u[5];  // A, C, D, E, lm_head
-	__shared__ PsSpan s_at[2];  // [is_local]
+// ------------------------------------------------------------------ the kernel's shared memory
+// (at namespace scope: a layer's code, which is a function of its own, addresses it without pointers)
+extern __shared__ uint8_t ps_dyn[];
+__shared__ PsArgs s_args;  // (the arguments, for the functions)
+__shared__ uint64_t bar_A, bar_C, bar_D, bar_E, bar_lm[8], emp_lm[8];
+__shared__ uint64_t bar_m[PS_TILES], acc_full[2], acc_free[2];  // MMAs of a unit's tile; the lm_head's two accumulators
+__shared__ __align__(16) float bred[3 * PS_NW];
+__shared__ uint32_t s_tmem;
+__shared__ float s_xscale;
+__shared__ int s_abort;
+__shared__ float s_f[8];
+__shared__ int s_i[4];
+__shared__ int s_cdf[2 * PS_NW + 8];
+__shared__ float wm[2 * PS_NW];  // per-warp (m, l) of the attention merge; also the sampler's per-warp maxima
+__shared__ PsLayer s_ly[PS_MAX_LAYERS];
+__shared__ PsUnit s_u[5];  // A, C, D, E, lm_head
+__shared__ PsSpan s_at[2];  // [is_local]
+__shared__ PsCta s_c;
+__shared__ PsLive s_t;
+__shared__ int s_dbg_n;
 
 #define R_A (smem + a.off_A)
 #define R_C (smem + a.off_C)
 #define R_D (smem + a.off_D)
 #define R_E (smem + a.off_E)
-	// (recomputed where they are used: a value that lives across the whole token loop costs a register, and the
-	// registers this kernel cannot have are spilled to local memory, which the small L1 left beside 224 KB of
-	// shared memory does not hold)
+// (recomputed where they are used: a value that lives across the whole token loop costs a register, and the
+// registers this kernel cannot have are spilled to local memory, which the small L1 left beside 224 KB of
+// shared memory does not hold)
 #define h (reinterpret_cast<float *>(smem + a.off_h))
 #define att (reinterpret_cast<float *>(smem + a.off_att))  /* wo[12][256] | qraw[768] (q_h, k, v) | qs[256] */
 #define smem_s (ps_smem(smem))
 #define tmem (s_c.tm)
 #define lut_s (smem_s + uint32_t(a.off_lut))
-#define pol (ps_evict_first())
-#define keep (ps_evict_last())
+#define pol (s_c.policy_first)
+#define keep (s_c.policy_last)
 
+#define hasA ((s_c.has & 1) != 0)
+#define hasC ((s_c.has & 2) != 0)
+#define hasD ((s_c.has & 4) != 0)
+#define hasE ((s_c.has & 8) != 0)
+
+#define lm_pre (cta < a.lm_ntiles ? a.lm_pre : 0)
+
+__device__ __noinline__ void ps_final_norm(const PsW w, int where, int D, float *h_, const PsUnit *u, float *s_x, const float *part, int nsplit,
+                                           const float *pres, int npres, const float *w_post, const float *w_pre, uint64_t hint, float *x_out) {
+	ps_resnorm(w, where, D, h_, u, bred, s_x, part, nsplit, pres, npres, w_post, w_pre, hint, x_out);
+}
+
+// The up/gate and the down unit of a layer are requested in four pieces each, from the layer before on: at the start of phase E
+// (the up/gate region is free), A (the down region is free), B, C and D, under the poll that begins there. Requested at once, the
+// 24 MB of all CTAs held up the hand-off that they met by 1 to 1.5 us, wherever that was.
+#define PS_REFILL_D(layer, i) \
+	if (tid == PS_THREADS - 32 && (layer) < L && hasD) ps_issue_piece(R_D, s_c.srcD + size_t(layer) * a.tl_layer, a.Dp.bytes, a.piece_D, i, &bar_D, pol, &s_abort)
+#define PS_REFILL_E(layer, i) \
+	if (tid == PS_THREADS - 64 && (layer) < L && hasE) ps_issue_piece(R_E, s_c.srcE + size_t(layer) * a.tl_layer, a.E.bytes, a.piece_E, i, &bar_E, pol, &s_abort)
+// (No __builtin_assume(__isShared(p)) in what is inlined here: on the address of a shared variable the compiler folds it to
+// false and drops the code behind it.)
+// One layer. A function of its own, with its phases inlined: a call and its return cost 250 to 350 clk each here (in-kernel
+// clocks), and nine calls a layer were a fifth of its time. pm: parity of bar_m, returned.
+template <bool DBG> __device__ __noinline__ uint32_t ps_layer(const int l, const int lc, const bool more, uint32_t pm) {
+	const PsArgs &a = s_args;
+	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(ps_dyn) + 127) & ~uintptr_t(127));
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int cta = blockIdx.x, G = gridDim.x;
+	const int D = a.D, L = a.L;
+	const PsW pw{&s_abort, a.err, a.wait_clocks, unsigned(a.poll_ns)};
+	const bool dbg_on = DBG && (a.dbg != nullptr) && cta == a.dbg_cta && tid == 0 && !more;
+	const PsLayer &ly = s_ly[l];
+	const PsSpan &at = s_at[ly.is_local];
+	const int nsA = AT_NH * at.nch;  // CTAs that take part in attention
+	const uint32_t par = lc & 1;  // parity of the units' barriers: one completion per layer
+	const int nl = (l + 1 < L) ? l + 1 : (more ? 0 : -1);  // the layer whose units are fetched next
+	float *const llb = a.ll + size_t(lc % 3) * a.ll_stride;
+	float *const llprev = a.ll + size_t((lc + 2) % 3) * a.ll_stride;
+	PS_BEACON(0x10);
+	PS_GT(0);
+	// ============================================================ A: QKV
+	if (l > 0) {
+		PS_REFILL_D(l, 1);
+		PS_REFILL_E(l, 0);
+	}
+	{
+		PsRun run;
+		if (hasA) run = ps_prepare(pw, (l << 4) | 1, &s_u[0], tmem, &bar_A, par);
+		ps_resnorm(pw, (l << 4) | 1, D, h, &s_u[0], bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
+		           G - a.E.units, l > 0 ? s_ly[l - 1].mlp_post : nullptr, ly.attn_pre, keep, nullptr);
+		PS_STAMP();
+		PS_GT(1);
+		PS_BEACON(0x11);
+		if (hasA) {
+			PS_STAMP();
+			pm = ps_unit(pw, (l << 4) | 1, run, bar_m, pm, &s_xscale, llb + s_u[0].dst, a.lut, lut_s, keep);
+			PS_STAMP();
+			if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_A, s_c.srcA + size_t(nl) * a.tl_layer, a.A.bytes, &bar_A, pol, &s_abort);
+		} else {
+			PS_STAMP();
+			PS_STAMP();
+		}
+		PS_STAMP();
+		PS_GT(2);
+		PS_BEACON(0x12);
+		// Wipe the arena copy of the NEXT layer. It was last used two layers ago; every CTA has
+		// finished with it: this CTA got past the prologue above, which needs the down-projection
+		// (or presence) words of ALL CTAs for the previous layer, and a CTA stores those after its
+		// last read of anything older. The CTAs that idle through the attention phase wipe; the
+		// fence orders the wipe before their own next down-projection / presence store.
+		if (cta >= nsA) {
+			float4 *other = reinterpret_cast<float4 *>(a.ll + size_t((lc + 1) % 3) * a.ll_stride);
+			const int nw = G - nsA, n4 = a.ll_stride / 4, per = (n4 + nw - 1) / nw;
+			const float e = __uint_as_float(PS_EMPTY);
+#pragma unroll 1
+			for (int i = (cta - nsA) * per + tid; i < min(n4, (cta - nsA + 1) * per); i += PS_THREADS)
+				__stcg(other + i, make_float4(e, e, e, e));
+			__syncthreads();
+			if (tid == 0) __threadfence();
+		}
+		PS_STAMP();
+	}
+	// ============================================================ B: attention
+	if (l > 0) {
+		PS_REFILL_D(l, 2);
+		PS_REFILL_E(l, 1);
+	}
+	if (cta < nsA) {
+		const int j0 = (cta >> 2) * at.chunk;
+		ps_attention(pw, (l << 4) | 2, ly.kcache, ly.vcache, ly.rmsq, ly.rmsk, a.rope[ly.is_local][0] + size_t(at.p) * AT_HD,
+		             a.rope[ly.is_local][1] + size_t(at.p) * AT_HD, llb + a.ll_qkv, a.QD, cta & 3,
+		             llb + a.ll_att + (size_t(cta & 3) * PS_MAX_CH + (cta >> 2)) * PS_ATT_ROW, j0, min(at.valid, j0 + at.chunk), at.slot, att, wm,
+		             keep);
+	}
+	PS_BEACON(0x24);
+	PS_GT(3);
+	PS_STAMP();
+	// ============================================================ C: O projection
+	if (l > 0) {
+		PS_REFILL_D(l, 3);
+		PS_REFILL_E(l, 2);
+	}
+	{
+		if (hasC) {
+			const PsRun run = ps_prepare(pw, (l << 4) | 3, &s_u[1], tmem, &bar_C, par);
+			ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, s_c.splitC * a.merge_heads, a.merge_heads, at.nch, att, &s_u[1], bred, &s_xscale);
+			PS_STAMP();
+			PS_GT(4);
+			PS_BEACON(0x31);
+			PS_STAMP();
+			pm = ps_unit(pw, (l << 4) | 3, run, bar_m, pm, &s_xscale, llb + s_u[1].dst, a.lut, lut_s, keep);
+			PS_STAMP();
+			if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_C, s_c.srcC + size_t(nl) * a.tl_layer, a.C.bytes, &bar_C, pol, &s_abort);
+		} else {
+			PS_STAMP();
+			PS_STAMP();
+			PS_STAMP();
+		}
+		PS_STAMP();
+		PS_GT(5);
+		PS_BEACON(0x32);
+	}
+	// ============================================================ D: up & gate + GeGLU
+	if (l > 0) PS_REFILL_E(l, 3);
+	{
+		PsRun run;
+		if (hasD) run = ps_prepare(pw, (l << 4) | 4, &s_u[2], tmem, &bar_D, par);
+		ps_resnorm(pw, (l << 4) | 4, D, h, &s_u[2], bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr);
+		PS_STAMP();
+		PS_GT(6);
+		PS_BEACON(0x41);
+		PS_STAMP();
+		if (hasD) pm = ps_unit(pw, (l << 4) | 4, run, bar_m, pm, &s_xscale, llb + s_u[2].dst, a.lut, lut_s, keep);
+		PS_STAMP();
+		PS_GT(7);
+		PS_BEACON(0x42);
+	}
+	// ============================================================ E: down projection
+	PS_REFILL_D(l + 1, 0);
+	{
+		PsRun run;
+		if (hasE) {
+			run = ps_prepare(pw, (l << 4) | 5, &s_u[3], tmem, &bar_E, par);
+			ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(s_c.splitE) * a.E.nq * 4, a.E.nq, &s_u[3], bred, &s_xscale);
+		}
+		if (tid == PS_THREADS - 32 && l + 1 == L) {
+			// last layer: the up/gate region is idle until the lm_head, whose ring starts there. Its first stages
+			// are requested now, so that they land under the down projection and the final norm.
+#pragma unroll 1
+			for (int sg = 0; sg < lm_pre; sg++)
+				ps_issue(R_D + size_t(sg) * a.lm_stage_bytes, a.lm_tiled + (size_t(cta) * a.lm_nchunk + sg) * a.lm_stage_bytes, uint32_t(a.lm_stage_bytes),
+				         &bar_lm[sg], pol, &s_abort);
+		}
+		PS_STAMP();
+		PS_GT(8);
+		PS_BEACON(0x51);
+		if (hasE) {
+			PS_STAMP();
+			pm = ps_unit(pw, (l << 4) | 5, run, bar_m, pm, &s_xscale, cta != a.fault_cta ? llb + s_u[3].dst : nullptr, a.lut, lut_s, keep);
+			PS_STAMP();
+		} else {
+			if (tid == 0) ps_st(llb + a.ll_pres + s_c.presE, 0.0f);
+			PS_STAMP();
+			PS_STAMP();
+		}
+		PS_STAMP();
+		PS_GT(9);
+		PS_BEACON(0x52);
+	}
+	return pm;
+}
+
+template <bool DBG>
+__global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __grid_constant__ PsArgs a) {
+	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(ps_dyn) + 127) & ~uintptr_t(127));  // the host adds 128 bytes of slack
+#pragma unroll 1
+	for (int i = threadIdx.x; i < int(sizeof(PsArgs) / 4); i += PS_THREADS) memcpy(reinterpret_cast<char *>(&s_args) + 4 * i, reinterpret_cast<const char *>(&a) + 4 * i, 4);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int cta = blockIdx.x, G = gridDim.x;
 	const int D = a.D, L = a.L;
@@ -1267,24 +1462,23 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #pragma unroll 1
 		for (int i = tid; i < a.lut.size; i += PS_THREADS) reinterpret_cast<float *>(smem + a.off_lut)[i] = a.lut.table[i];
 	{
-		const int *src = reinterpret_cast<const int *>(a.layers);
-		int *dst = reinterpret_cast<int *>(s_ly);
+		// (bytes: an int store to a struct of pointers would be one that the compiler need not see)
 #pragma unroll 1
-		for (int i = tid; i < L * int(sizeof(PsLayer) / 4); i += PS_THREADS) dst[i] = src[i];
+		for (int i = tid; i < L * int(sizeof(PsLayer) / 4); i += PS_THREADS) memcpy(reinterpret_cast<char *>(s_ly) + 4 * i, reinterpret_cast<const char *>(a.layers) + 4 * i, 4);
 	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
 	const PsW pw{&s_abort, a.err, a.wait_clocks, unsigned(a.poll_ns)};
-	unsigned epoch = 0;  // grid barriers passed
-	uint32_t pA = 0, pC = 0, pD = 0, pE = 0, plm = 0, pemp = 0, pm = 0, acc_n = 0;
+	uint32_t pm = 0;
 
-	__shared__ PsCta s_c;
 	{
 		const int uA = cta - a.A.cta0, uC = cta - a.C.cta0, uD = cta - a.Dp.cta0, uE = cta - a.E.cta0;
 		const bool hA = uA >= 0 && uA < a.A.units, hC = uC >= 0 && uC < a.C.units, hD = uD >= 0 && uD < a.Dp.units, hE = uE >= 0 && uE < a.E.units;
 		if (tid == 0) {
 			s_c.tm = *(volatile uint32_t *)&s_tmem;
+			s_c.policy_first = ps_evict_first();
+			s_c.policy_last = ps_evict_last();
 			s_c.splitC = hC ? uC / a.C.ntiles : 0;
 			s_c.splitE = hE ? uE / a.E.ntiles : 0;
 			s_c.presE = uE < 0 ? cta : cta - a.E.units;  // index of this CTA's presence word (if !hasE)
@@ -1304,38 +1498,26 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		}
 		__syncthreads();
 	}
-#define hasA ((s_c.has & 1) != 0)
-#define hasC ((s_c.has & 2) != 0)
-#define hasD ((s_c.has & 4) != 0)
-#define hasE ((s_c.has & 8) != 0)
-#define splitC (s_c.splitC)
-#define splitE (s_c.splitE)
-#define presE (s_c.presE)
-#define srcA (s_c.srcA)
-#define srcC (s_c.srcC)
-#define srcD (s_c.srcD)
-#define srcE (s_c.srcE)
-
 	if (tid == 0) {
-		if (hasA) ps_issue(R_A, srcA, a.A.bytes, &bar_A, pol, &s_abort);
-		if (hasC) ps_issue(R_C, srcC, a.C.bytes, &bar_C, pol, &s_abort);
-		if (hasD && a.sched == 0) ps_issue(R_D, srcD, a.Dp.bytes, &bar_D, pol, &s_abort);
-		if (hasE && a.sched == 0) ps_issue(R_E, srcE, a.E.bytes, &bar_E, pol, &s_abort);
+		if (hasA) ps_issue(R_A, s_c.srcA, a.A.bytes, &bar_A, pol, &s_abort);
+		if (hasC) ps_issue(R_C, s_c.srcC, a.C.bytes, &bar_C, pol, &s_abort);
+		if (hasD) ps_issue(R_D, s_c.srcD, a.Dp.bytes, &bar_D, pol, &s_abort);
+		if (hasE) ps_issue(R_E, s_c.srcE, a.E.bytes, &bar_E, pol, &s_abort);
 	}
 
-	int tok = __ldcg(a.tok);
-	int pos = __ldcg(a.next_pos);
-	const int rbase = __ldcg(a.ring_base);
-	int n_logged = 0;
-	int dbg_n = 0;
+	if (tid == 0) s_t = PsLive{0, 0, 0, 0, 0, __ldcg(a.tok), __ldcg(a.next_pos)};
+	__syncthreads();
+	if (tid == 0) s_dbg_n = 0;
 	// ring stages of the lm_head that fit the up/gate region and belong to this CTA's first tile (chunks 0 .. lm_pre - 1)
-	const int lm_pre = (cta < a.lm_ntiles && a.sched == 0) ? min(min(a.lm_stages, a.lm_nchunk), a.Dp.bytes / a.lm_stage_bytes) : 0;
+	int lc = 0;  // layers so far
 #pragma unroll 1
 	for (int step = 0; step < a.n_steps; step++) {
 		const bool more = (step + 1 < a.n_steps);
 		const bool dbg_on = DBG && (a.dbg != nullptr) && cta == a.dbg_cta && tid == 0 && !more;
 		PS_STAMP();
 		// ---------------------------------------------------------------- embedding
+		int tok = s_t.tok;
+		const int pos = s_t.pos;
 		if (a.force_ids) tok = __ldg(a.force_ids + step);
 		if (tok < 0 || tok >= a.V) {
 			if (tid == 0 && cta == 0) atomicExch(a.err, 1);
@@ -1356,7 +1538,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 				const int given = loc ? a.nch_local : a.nch_global, nch = given ? given : int((loc ? kl : kg) & 255u);
 				const int p = loc ? pos : min(pos, a.slots_global - 1);
 				if (!loc && pos >= a.slots_global && cta == 0) atomicExch(a.err, 2);
-				s_at[loc] = PsSpan{p, loc ? (p - rbase) % a.slots_local : p, v, nch, (v + nch - 1) / nch};
+				s_at[loc] = PsSpan{p, loc ? (p - __ldcg(a.ring_base)) % a.slots_local : p, v, nch, (v + nch - 1) / nch};
 			}
 		}
 #pragma unroll 1
@@ -1364,170 +1546,43 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		__syncthreads();
 
 #pragma unroll 1
-		for (int l = 0; l < L; l++) {
-			const PsLayer &ly = s_ly[l];
-			const PsSpan &at = s_at[ly.is_local];
-			const int nsA = AT_NH * at.nch;  // CTAs that take part in attention
-			const int lc = step * L + l;
-			const int nl = (l + 1 < L) ? l + 1 : (more ? 0 : -1);  // the layer whose units are fetched next
-			float *const llb = a.ll + size_t(lc % 3) * a.ll_stride;
-			float *const llprev = a.ll + size_t((lc + 2) % 3) * a.ll_stride;
-			PS_BEACON(0x10);
-			PS_GT(0);
-			// ============================================================ A: QKV
-			{
-				ps_resnorm(pw, (l << 4) | 1, D, h, &s_u[0], hasA ? &bar_A : nullptr, pA, bred, &s_xscale, l > 0 ? llprev + a.ll_dn : nullptr, a.E.nsplit, llprev + a.ll_pres,
-				           G - a.E.units, l > 0 ? s_ly[l - 1].mlp_post : nullptr, ly.attn_pre, keep, nullptr);
-				PS_STAMP();
-				PS_GT(1);
-				PS_BEACON(0x11);
-				if (hasA) {
-					PS_STAMP();
-					pm = ps_unit(pw, (l << 4) | 1, &s_u[0], tmem, &bar_A, pA, bar_m, pm, &s_xscale, llb + s_u[0].dst, a.lut, lut_s, keep);
-					PS_STAMP();
-					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_A, srcA + size_t(nl) * a.tl_layer, a.A.bytes, &bar_A, pol, &s_abort);
-				} else {
-					PS_STAMP();
-					PS_STAMP();
-				}
-				pA ^= 1;
-				if (a.sched == 1 && tid == 64) {  // (every warp passed the barrier that ended the prologue: the regions' last readers are long done)
-					if (hasD) ps_issue(R_D, srcD + size_t(l) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
-					if (hasE) ps_issue(R_E, srcE + size_t(l) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
-				}
-				PS_STAMP();
-				PS_GT(2);
-				PS_BEACON(0x12);
-				// Wipe the arena copy of the NEXT layer. It was last used two layers ago; every CTA has
-				// finished with it: this CTA got past the prologue above, which needs the down-projection
-				// (or presence) words of ALL CTAs for the previous layer, and a CTA stores those after its
-				// last read of anything older. The CTAs that idle through the attention phase wipe; the
-				// fence orders the wipe before their own next down-projection / presence store.
-				if (cta >= nsA) {
-					float4 *other = reinterpret_cast<float4 *>(a.ll + size_t((lc + 1) % 3) * a.ll_stride);
-					const int nw = G - nsA, n4 = a.ll_stride / 4, per = (n4 + nw - 1) / nw;
-					const float e = __uint_as_float(PS_EMPTY);
-#pragma unroll 1
-					for (int i = (cta - nsA) * per + tid; i < min(n4, (cta - nsA + 1) * per); i += PS_THREADS)
-						__stcg(other + i, make_float4(e, e, e, e));
-					__syncthreads();
-					if (tid == 0) __threadfence();
-				}
-				PS_STAMP();
-			}
-			// ============================================================ B: attention
-			if (cta < nsA) {
-				const int j0 = (cta >> 2) * at.chunk;
-				ps_attention(pw, (l << 4) | 2, ly.kcache, ly.vcache, ly.rmsq, ly.rmsk, a.rope[ly.is_local][0] + size_t(at.p) * AT_HD,
-				             a.rope[ly.is_local][1] + size_t(at.p) * AT_HD, llb + a.ll_qkv, a.QD, cta & 3,
-				             llb + a.ll_att + (size_t(cta & 3) * PS_MAX_CH + (cta >> 2)) * PS_ATT_ROW, j0, min(at.valid, j0 + at.chunk), at.slot, att, wm,
-				             keep);
-			}
-			PS_BEACON(0x24);
-			PS_GT(3);
-			PS_STAMP();
-			// ============================================================ C: O projection
-			{
-				if (hasC) {
-					ps_attn_merge(pw, (l << 4) | 3, llb + a.ll_att, splitC * a.merge_heads, a.merge_heads, at.nch, att, &s_u[1], &bar_C, pC, bred, &s_xscale);
-					PS_STAMP();
-					PS_GT(4);
-					PS_BEACON(0x31);
-					PS_STAMP();
-					pm = ps_unit(pw, (l << 4) | 3, &s_u[1], tmem, &bar_C, pC, bar_m, pm, &s_xscale, llb + s_u[1].dst, a.lut, lut_s, keep);
-					PS_STAMP();
-					if (nl >= 0 && tid == PS_THREADS - 32) ps_issue(R_C, srcC + size_t(nl) * a.tl_layer, a.C.bytes, &bar_C, pol, &s_abort);
-				} else {
-					PS_STAMP();
-					PS_STAMP();
-					PS_STAMP();
-				}
-				pC ^= 1;
-				PS_STAMP();
-				PS_GT(5);
-				PS_BEACON(0x32);
-			}
-			// ============================================================ D: up & gate + GeGLU
-			{
-				ps_resnorm(pw, (l << 4) | 4, D, h, &s_u[2], hasD ? &bar_D : nullptr, pD, bred, &s_xscale, llb + a.ll_op, a.C.nsplit, nullptr, 0, ly.attn_post, ly.mlp_pre, keep, nullptr);
-				PS_STAMP();
-				PS_GT(6);
-				PS_BEACON(0x41);
-				PS_STAMP();
-				if (hasD) pm = ps_unit(pw, (l << 4) | 4, &s_u[2], tmem, &bar_D, pD, bar_m, pm, &s_xscale, llb + s_u[2].dst, a.lut, lut_s, keep);
-				pD ^= 1;
-				PS_STAMP();
-				PS_GT(7);
-				PS_BEACON(0x42);
-			}
-			// ============================================================ E: down projection
-			{
-				if (hasE) {
-					ps_act_quant(pw, (l << 4) | 5, llb + a.ll_act + size_t(splitE) * a.E.nq * 4, a.E.nq, &s_u[3], &bar_E, pE, bred, &s_xscale);
-				}
-				// the up/gate region is free: request the next layer's unit now that the hand-off loads are done
-				if (a.sched == 0 && tid == PS_THREADS - 32 && hasD && l + 1 < L) ps_issue(R_D, srcD + size_t(l + 1) * a.tl_layer, a.Dp.bytes, &bar_D, pol, &s_abort);
-				if (tid == PS_THREADS - 32 && l + 1 == L) {
-					// last layer: the up/gate region is idle until the lm_head, whose ring starts there. Its first stages
-					// are requested now, so that they land under the down projection and the final norm.
-#pragma unroll 1
-					for (int sg = 0; sg < lm_pre; sg++)
-						ps_issue(R_D + size_t(sg) * a.lm_stage_bytes, a.lm_tiled + (size_t(cta) * a.lm_nchunk + sg) * a.lm_stage_bytes, uint32_t(a.lm_stage_bytes),
-						         &bar_lm[sg], pol, &s_abort);
-				}
-				PS_STAMP();
-				PS_GT(8);
-				PS_BEACON(0x51);
-				if (hasE) {
-					PS_STAMP();
-					pm = ps_unit(pw, (l << 4) | 5, &s_u[3], tmem, &bar_E, pE, bar_m, pm, &s_xscale, cta != a.fault_cta ? llb + s_u[3].dst : nullptr, a.lut, lut_s, keep);
-					PS_STAMP();
-					if (a.sched == 0 && l + 1 < L && tid == PS_THREADS - 64) ps_issue(R_E, srcE + size_t(l + 1) * a.tl_layer, a.E.bytes, &bar_E, pol, &s_abort);
-				} else {
-					if (tid == 0) ps_st(llb + a.ll_pres + presE, 0.0f);
-					PS_STAMP();
-					PS_STAMP();
-				}
-				pE ^= 1;
-				PS_STAMP();
-				PS_GT(9);
-				PS_BEACON(0x52);
-			}
-		}
+		for (int l = 0; l < L; l++, lc++) pm = ps_layer<DBG>(l, lc, more, pm);
 
 		// ================================================================ lm_head
 		// (its ring lies over the now idle up/gate and down regions)
-		const int lc = step * L + L;
 		{
 			float *const lllast = a.ll + size_t((lc + 2) % 3) * a.ll_stride;
-			ps_resnorm(pw, (L << 4) | 6, D, h, &s_u[4], nullptr, 0, bred, &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
+			ps_final_norm(pw, (L << 4) | 6, D, h, &s_u[4], &s_xscale, lllast + a.ll_dn, a.E.nsplit, lllast + a.ll_pres, G - a.E.units,
 			           s_ly[L - 1].mlp_post, a.final_norm, keep, cta == 0 ? a.xnorm_out : nullptr);
 		}
 		PS_STAMP();
 		PS_BEACON(0x61);
-		const PsLmOut lo = ps_lm_head(a, pw, R_D, smem_s, s_xscale, tmem, bar_lm, emp_lm, acc_full, acc_free, plm, pemp, acc_n, pol, keep, lm_pre);
-		acc_n += (a.lm_ntiles - cta + G - 1) / G;
-		plm = lo.plm;
-		pemp = lo.pemp;
+		const PsLmOut lo = ps_lm_head(a, pw, R_D, smem_s, s_xscale, tmem, bar_lm, emp_lm, acc_full, acc_free, s_t.plm, s_t.pemp, s_t.acc_n, pol, keep, lm_pre);
 		__syncthreads();
+		if (tid == 0) {
+			s_t.acc_n += (a.lm_ntiles - cta + G - 1) / G;
+			s_t.plm = lo.plm;
+			s_t.pemp = lo.pemp;
+		}
 
 		// ================================================================ sampler
 		PS_STAMP();
 		PS_BEACON(0x70);
-		const PsSampOut so = ps_sampler(a, pw, lo.best, lo.best_i, epoch, n_logged, wm, s_cdf, s_f, s_i, bred, reinterpret_cast<float *>(R_D));
-		const int next_tok = so.tok;
-		epoch = so.epoch;
-		if (a.sampler != 0) n_logged++;
+		const PsSampOut so = ps_sampler(a, pw, lo.best, lo.best_i, s_t.epoch, s_t.n_logged, wm, s_cdf, s_f, s_i, bred, reinterpret_cast<float *>(R_D));
 		PS_STAMP();
 		PS_BEACON(0x7F);
-		pos += 1;
-		if (cta == 0 && tid == 0) *a.next_pos = pos;
-		// the ring is idle again: fetch the next token's layer-0 up/gate and down units
-		if (tid == 0 && more && a.sched == 0) {
-			if (hasD) ps_issue(R_D, srcD, a.Dp.bytes, &bar_D, pol, &s_abort);
-			if (hasE) ps_issue(R_E, srcE, a.E.bytes, &bar_E, pol, &s_abort);
+		if (tid == 0) {
+			s_t.epoch = so.epoch;
+			if (a.sampler != 0) s_t.n_logged++;
+			s_t.tok = so.tok;
+			s_t.pos++;
+			if (cta == 0) *a.next_pos = s_t.pos;
 		}
-		tok = next_tok;
+		// the ring is idle again: fetch the next token's layer-0 up/gate and down units
+		if (tid == 0 && more) {
+			if (hasD) ps_issue(R_D, s_c.srcD, a.Dp.bytes, &bar_D, pol, &s_abort);
+			if (hasE) ps_issue(R_E, s_c.srcE, a.E.bytes, &bar_E, pol, &s_abort);
+		}
 		if (__syncthreads_or(*(volatile int *)&s_abort)) break;  // the whole CTA leaves together
 	}
 	if (*(volatile int *)&s_abort) {
@@ -1544,7 +1599,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 		tc_fence_after();
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PS_TMEM) : "memory");
 	}
-	if (cta == 0 && tid == 0 && a.log_count) *a.log_count = n_logged;
+	if (cta == 0 && tid == 0 && a.log_count) *a.log_count = s_t.n_logged;
 	// Leave the hand-off arena as the next launch expects it: copy 0 empty (copies 1 and 2 are wiped during
 	// its layers 0 and 1, like every copy a layer before its use). Every CTA is past the last token's grid
 	// barriers, which all CTAs reach only after their last read of the arena.
@@ -1555,6 +1610,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #pragma unroll 1
 		for (int i = cta * per + tid; i < min(n4, (cta + 1) * per); i += PS_THREADS) __stcg(c0 + i, make_float4(e, e, e, e));
 	}
+}
 #undef h
 #undef att
 #undef smem_s
@@ -1566,17 +1622,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 #undef R_C
 #undef R_D
 #undef R_E
+#undef PS_REFILL_D
+#undef PS_REFILL_E
 #undef hasA
 #undef hasC
 #undef hasD
 #undef hasE
-#undef splitC
-#undef splitE
-#undef presE
-#undef srcA
-#undef srcC
-#undef srcD
-#undef srcE
-}
+#undef lm_pre
 
 }  // namespace tg

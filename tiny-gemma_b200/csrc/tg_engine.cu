@@ -1147,7 +1147,7 @@ int persist_setup(tg_state *s) {
 	             [&](int ns) { return 8.0 * (AT_NH / ns) + dkb * ns; }) ||
 	    !ps_plan(&a.Dp, D, I, 2, G, budget, {1}, {}, 1 << 20, [&](int) { return 0.0; }) ||
 	    !ps_plan(&a.E, I, D, 1, G, budget / 2, esplit ? std::vector<int>{esplit} : std::vector<int>{1, 2, 3, 4, 6, 8}, {},
-	             5 * PS_THREADS, [&](int ns) { return I * 4 / 1024.0 / ns + dkb * ns; }))
+	             PS_ACT * PS_THREADS, [&](int ns) { return I * 4 / 1024.0 / ns + dkb * ns; }))
 		return fail(TG_ESHAPE, "persistent kernel: no phase plan fits");
 	a.A.cta0 = G - a.A.units;  // the attention CTAs (low indices) hold no Q|K|V unit where possible
 	// cache chunks per head; at least 8 CTAs must stay out of the attention phase (they wipe the hand-off arena)
@@ -1158,6 +1158,8 @@ int persist_setup(tg_state *s) {
 	a.slots_local = c.n_pos_local;
 	a.slots_global = s->max_pos_global;
 	a.merge_heads = AT_NH / a.C.nsplit;
+	a.piece_D = uint32_t(a.Dp.bytes / 4 + 127) & ~127u;
+	a.piece_E = uint32_t(a.E.bytes / 4 + 127) & ~127u;
 	const int npres = G - a.E.units;
 	if (D / 4 + npres > PS_THREADS || G < 16) return fail(TG_ESHAPE, "persistent kernel: grid too small for the down-projection plan");
 	// lm_head: tiles of 128 columns; ring stages of at most 40 KB
@@ -1213,6 +1215,7 @@ int persist_setup(tg_state *s) {
 	const int region = std::max(std::max(a.off_E + a.E.bytes - a.off_D, minp_grid_floats(V, G) * 4), std::min(5 * a.lm_stage_bytes, room / a.lm_stage_bytes * a.lm_stage_bytes));
 	off = up(off + region);
 	a.lm_stages = std::min(8, region / a.lm_stage_bytes);
+	a.lm_pre = std::min(std::min(a.lm_stages, a.lm_nchunk), a.Dp.bytes / a.lm_stage_bytes);
 	if (a.lm_stages < 2) return fail(TG_ESHAPE, "persistent kernel: lm_head ring does not fit");
 	a.smem_total = off + 128;
 	{
@@ -1225,13 +1228,6 @@ int persist_setup(tg_state *s) {
 	for (int l = 0; l < L; l++) {
 		const LayerW &w = m->layers[l];
 		PsLayer &ly = lys[l];
-		ly.sq = w.Q.s;
-		ly.sk = w.K.s;
-		ly.sv = w.V.s;
-		ly.so = w.O.s;
-		ly.su = w.U.s;
-		ly.sg = w.G.s;
-		ly.sd = w.Dn.s;
 		ly.rmsq = w.rmsq;
 		ly.rmsk = w.rmsk;
 		ly.attn_pre = w.attn_pre;
@@ -1380,7 +1376,6 @@ int persist_launch(tg_state *s, int n_steps, int sampler, float minp, float temp
 	a.wait_clocks = (long long)(std::max(1, env_int("TG_PS_WAIT_MS", 100))) * 2000000ll;  // ~2 GHz
 	a.fault_cta = env_int("TG_PS_WITHHOLD_CTA", -1);
 	a.poll_ns = std::max(0, env_int("TG_PS_POLL_NS", 20));
-	a.sched = env_int("TG_PS_SCHED", 0);
 	a.gt = (s->mg_dbg && env_int("TG_PS_GT", 0)) ? s->mg_dbg + 2048 : nullptr;  // (the stamp recorder uses < 600 entries)
 	// Every word of the hand-off arena copy 0 starts as "empty" (all ones) and the barrier counter at
 	// bar_base: a launch that ran through leaves both that way. After an error (or before the first
