@@ -392,14 +392,38 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 // keys and step), so products are packed two to an instruction. q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
 // prompt. Query s is the token at key off + s (off > 0: a continuation, its context comes first). Causal; on local layers
 // a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
+// A cluster of ks CTAs shares two queries, each with a part of their keys (a chunk of 32 keys is a chain of three barriers, ~2 us): the
+// first one joins the parts, in key order. attn_small_split: how many.
 constexpr int APS_THREADS = 512;
+// CTAs per two queries of a prompt of S tokens behind `off` others. By the prompt alone: a prompt of a group gets the bits that it
+// gets by itself. Two chunks of keys per CTA at least, and not many more CTAs than are resident (one per SM): 178 tokens 2,
+// 61 behind 1500 cached ones 6. (prefill of 178 tokens 1862 -> 1804 us)
+inline int attn_small_split(int S, int off, int is_local, int window) {
+	const int keys = is_local ? std::min(off + S, window + 2) : off + S;
+	return std::max(1, std::min(std::min(8, (keys + AC_KEYS - 1) / AC_KEYS / 2), 192 / ((S + 1) / 2)));
+}
+__device__ __forceinline__ uint32_t ac_mapa(const void *p, int rank) {
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+	return r;
+}
+__device__ __forceinline__ float ac_remote(const float *p, int rank) {
+	float v;
+	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ac_mapa(p, rank)) : "memory");
+	return v;
+}
+__device__ __forceinline__ float4 ac_remote4(const float4 *p, int rank) {
+	float4 v;
+	asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ac_mapa(p, rank)) : "memory");
+	return v;
+}
 __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
                                                                             const float *k, const float *v, int S, int off, int is_local, int window,
-                                                                            int *err) {
+                                                                            int ks, int *err) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
 	constexpr int R = 8;  // query rows
 	__shared__ __align__(16) float sc[AC_KEYS][R], pr[AC_KEYS][R];
-	__shared__ float corr_s[R], l_s[R];
+	__shared__ float corr_s[R], l_s[R], m_s[R];
 	__shared__ uint64_t kbar, vbar;
 	__shared__ uint32_t red[APS_THREADS / 32];
 	float *K = reinterpret_cast<float *>(ac_smem), *V = reinterpret_cast<float *>(ac_smem + AC_BUF);
@@ -413,19 +437,22 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	pdl_trigger();
 	pdl_wait();
 	const size_t r0 = size_t(blockIdx.y) * S;
-	const int s0 = int(gridDim.x - 1 - blockIdx.x) * 2;  // (the longest walks start first)
+	const int rank = ks > 1 ? int(blockIdx.x) % ks : 0;  // of the cluster's CTAs
+	const int s0 = (int(gridDim.x) / ks - 1 - int(blockIdx.x) / ks) * 2;  // (the longest walks start first)
 	const int s_last = min(S - 1, s0 + 1);
 	const int j0 = (is_local && off + s0 >= window) ? off + s0 - window : 0, j1 = off + s_last + 1;
-	const int nch = (j1 - j0 + AC_KEYS - 1) / AC_KEYS;
+	// this CTA's chunks: c_lo .. c_lo + nch - 1 of all
+	const int all = (j1 - j0 + AC_KEYS - 1) / AC_KEYS, c_lo = all * rank / ks, nch = all * (rank + 1) / ks - c_lo;
 	k += (r0 + j0) * 256;  // (a continuation is one sequence: r0 = 0)
 	v += (r0 + j0) * 256;
 	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
+		c += c_lo;
 		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
 		fence_proxy_async();
 		mbar_expect_tx(bar, bytes);
 		bulk_load(dst, src + size_t(c) * AC_KEYS * 256, bytes, bar);
 	};
-	if (tid == 0) {
+	if (tid == 0 && nch > 0) {
 		issue(K, k, 0, &kbar);
 		issue(V, v, 0, &vbar);
 	}
@@ -450,7 +477,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	for (int r = 0; r < R; r++) o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
 	float m = -INFINITY, l = 0.0f;  // of row `warp` (warps 0..7)
 	for (int c = 0; c < nch; c++) {
-		const int base = j0 + c * AC_KEYS, n = min(AC_KEYS, j1 - base);
+		const int base = j0 + (c_lo + c) * AC_KEYS, n = min(AC_KEYS, j1 - base);
 		tc_wait(&kbar, c & 1, err);
 		{
 			float t[16];
@@ -511,7 +538,10 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
 #pragma unroll
 	for (int r = 0; r < R; r++) jb[(kg * R + r) * 64 + d4] = o[r];
-	if (warp < R && lane == 0) l_s[warp] = l;
+	if (warp < R && lane == 0) {
+		l_s[warp] = l;
+		m_s[warp] = m;
+	}
 	__syncthreads();
 	const int qi = tid >> 8, k4 = tid & 255, row = qi * 4 + (k4 >> 6);
 	float4 r = jb[row * 64 + (k4 & 63)];
@@ -523,7 +553,31 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 		r.z += t.z;
 		r.w += t.w;
 	}
-	const float L = l_s[row];
+	float L = l_s[row];
+	if (ks > 1) {  // the other CTAs' parts, through the cluster's shared memory, in key order
+		float4 *mine = jb;
+		__syncthreads();  // (the key groups have been read)
+		mine[tid] = r;
+		i8_cluster_sync();
+		if (rank == 0) {
+			float M = m_s[row];
+#pragma unroll 1
+			for (int p = 1; p < ks; p++) {
+				const float pm = ac_remote(&m_s[row], p), pl = ac_remote(&l_s[row], p);
+				if (pm == -INFINITY) continue;  // (no key of its chunks is visible)
+				const float4 o4 = ac_remote4(&mine[tid], p);
+				const float mn = fmaxf(M, pm), ea = M == -INFINITY ? 0.0f : expf(M - mn), eb = expf(pm - mn);
+				L = fmaf(L, ea, pl * eb);
+				r.x = fmaf(r.x, ea, o4.x * eb);
+				r.y = fmaf(r.y, ea, o4.y * eb);
+				r.z = fmaf(r.z, ea, o4.z * eb);
+				r.w = fmaf(r.w, ea, o4.w * eb);
+				M = mn;
+			}
+		}
+		i8_cluster_sync();  // (nobody leaves while its memory is read)
+		if (rank != 0) return;
+	}
 	r.x /= L;
 	r.y /= L;
 	r.z /= L;

@@ -1683,9 +1683,9 @@ int make_digit_map(CUtensorMap *out, const uint8_t *x, int K, int groups, int tg
 	if (r != CUDA_SUCCESS) return fail(TG_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
 	return TG_OK;
 }
-// launch_k in clusters of two CTAs
+// launch_k in clusters of `size` CTAs
 template <typename... KArgs, typename... Args>
-inline void launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+inline void launch_clusters(int size, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = grid;
 	cfg.blockDim = block;
@@ -1693,7 +1693,7 @@ inline void launch_pair(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
 	cfg.stream = st;
 	cudaLaunchAttribute at[2];
 	at[0].id = cudaLaunchAttributeClusterDimension;
-	at[0].val.clusterDim.x = 2;
+	at[0].val.clusterDim.x = size;
 	at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
 	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	at[1].val.programmaticStreamSerializationAllowed = 1;
@@ -1777,7 +1777,7 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	if (pl.cg == 2) {
 		CUtensorMap xmap;
 		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
-		launch_pair(qgemm_i8_kernel<2>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
+		launch_clusters(2, qgemm_i8_kernel<2>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
 	} else {
 		launch_k(qgemm_i8_kernel<1>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
 	}
@@ -2118,8 +2118,9 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 				TG_CUDA(cudaFuncSetAttribute(attn_prefill_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM));
 				as_configured[dev] = true;
 			}
-			launch_k(attn_prefill_small_kernel, dim3((S_seq + 1) / 2, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
-			         use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, s->err_flag);
+			const int ks = attn_small_split(S_seq, off, w.is_local ? 1 : 0, window);
+			launch_clusters(ks, attn_prefill_small_kernel, dim3((S_seq + 1) / 2 * ks, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
+			                use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, ks, s->err_flag);
 		} else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
