@@ -35,3 +35,20 @@ def test_shared_keys(capi, synth, weights_270m, monkeypatch, ctx, S):
     # fp32 softmax sums in another order, 18 layers: the bound of the other comparisons of attention kernels
     assert rel_l2(got[0], got[1]) <= 1e-4, (ctx, S)
     assert np.all(np.isfinite(got[0]))
+
+
+@pytest.mark.parametrize("n,S", [(1, 672), (1, 673), (4, 170), (5, 150), (5, 151), (20, 61), (21, 61)])  # rows 672; 420 + 50000 / S
+def test_line_between_the_kernels(capi, synth, weights_270m, monkeypatch, n, S):
+    """Prompts and groups on both sides of the line between the attention kernels, against the short-prompt kernel."""
+    m = capi.Model("270m").load_file(weights_270m)
+    m.build_tables(1 << 20)
+    prompts = np.stack([synth.random_prompt(S, 20 + i) for i in range(n)])
+    st = m.state(n, S + 8)
+    a = st.prefill(prompts)
+    st.reset()
+    monkeypatch.setenv("TG_ATTN_SMALL_MAX", "100000")
+    b = st.prefill(prompts)
+    st.close()
+    m.close()
+    for i in range(n):
+        assert rel_l2(a[i], b[i]) <= 5e-5, i
