@@ -459,14 +459,25 @@ __global__ void __launch_bounds__(MVC_THREADS, 1) qmatvec_cluster_kernel(float *
 
 // =========================================================== wide matvec (one sequence, the vocabulary matrix)
 // y[n] = scale[n] * sum_k x[k] W[k,n] for a matrix of hundreds of MB: HBM bound. One CTA per SM owns `groups` groups of
-// 16 consecutive columns (262144 columns over 148 SMs: 112 groups, 1792 contiguous bytes of every row, no last wave) in
-// four row sets; a thread keeps eight 16-byte loads in flight behind the eight it is working on (57 + 57 KB per SM).
-// 128-column tiles with eight loads and a pause between the batches took 83 us for 1152 x 262144 (56 % of the measured
-// copy bandwidth).
-constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8;
+// 16 consecutive columns (262144 columns over 148 SMs: 112 groups, 1792 contiguous bytes of every row, whole lines) in
+// four row sets. A thread copies its own 16-byte pieces into a ring of three stages of eight rows in shared memory (cp.async, no
+// barrier: it reads nobody else's) and works on one stage with the next two on their way, 114 KB per SM. 1152 x 262144: 59.5 us with
+// the next eight loads in registers (57 KB) and 111 groups, whose pieces of a row began anywhere in a line; 58.9 with whole lines alone, 59.9 with
+// the ring alone, 54.9 with both (5.5 TB/s; a copy into rings of 147 KB that multiplies nothing: 49).
+constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8, MVW_STAGES = 3;
+__device__ __forceinline__ void mvw_copy(uint32_t dst, const int8_t *src) {
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// a += (b - (2^23 + 128)) * c, both halves: b holds the bits of 2^23 + 128 + a weight (exact, see i8_lane_to_f32)
+__device__ __forceinline__ void mvw_fma2(float2 &a, uint32_t b0, uint32_t b1, float c) {
+	asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmov.b64 z, {%5, %5};\n\t"
+	    "add.rn.f32x2 y, y, z;\n\tmov.b64 z, {%4, %4};\n\tfma.rn.f32x2 x, y, z, x;\n\tmov.b64 {%0, %1}, x;\n\t}"
+	    : "+f"(a.x), "+f"(a.y)
+	    : "r"(b0), "r"(b1), "f"(c), "f"(-8388736.0f));
+}
 __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kernel(float *y, const float *x, const int8_t *w, const float *scales,
                                                                                    int K, int N, int groups) {
-	extern __shared__ float mvw_smem[];  // x [K], then the row sets' sums [4][groups * 16]
+	extern __shared__ __align__(16) float mvw_smem[];  // x [K], the ring [3][8][threads] of 16 bytes; the row sets' sums [4][groups * 16] in its place
 	pdl_trigger();
 	pdl_wait();
 	float *xs = mvw_smem;
@@ -477,43 +488,53 @@ __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kern
 	const int8_t *p = w + size_t(on ? set : 0) * N + (on ? col : 0);
 	const size_t step = size_t(MVW_SETS) * N;
 	const int n = on ? K / MVW_SETS : 0;  // K is a multiple of 4 * MVW_U
-	int4 cur[MVW_U], nxt[MVW_U];
+	const uint32_t ring = uint32_t(__cvta_generic_to_shared(xs + K)) + 16u * tid;
+	int next = 0;  // rows requested so far
+	auto request = [&](int st) {
+		if (next < n) {
 #pragma unroll
-	for (int u = 0; u < MVW_U; u++) {
-		cur[u] = make_int4(0, 0, 0, 0);
-		if (n) cur[u] = ld_stream_int4(p + u * step);
-	}
+			for (int u = 0; u < MVW_U; u++) mvw_copy(ring + uint32_t((st * MVW_U + u) * nt) * 16u, p + u * step);
+			p += MVW_U * step;
+			next += MVW_U;
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+#pragma unroll
+	for (int st = 0; st < MVW_STAGES; st++) request(st);
 	for (int k = tid; k < K; k += nt) xs[k] = x[k];
 	__syncthreads();
-	float acc[16];
+	float2 acc[8];
 #pragma unroll
-	for (int i = 0; i < 16; i++) acc[i] = 0.0f;
+	for (int i = 0; i < 8; i++) acc[i] = make_float2(0.0f, 0.0f);
+	int st = 0;
 #pragma unroll 1
 	for (int it = 0; it < n; it += MVW_U) {
-		p += MVW_U * step;
-#pragma unroll
-		for (int u = 0; u < MVW_U; u++)
-			if (it + MVW_U < n) nxt[u] = ld_stream_int4(p + u * step);
+		asm volatile("cp.async.wait_group %0;" ::"n"(MVW_STAGES - 1) : "memory");
 #pragma unroll
 		for (int u = 0; u < MVW_U; u++) {
+			uint32_t words[4];
+			asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+			             : "=r"(words[0]), "=r"(words[1]), "=r"(words[2]), "=r"(words[3])
+			             : "r"(ring + uint32_t((st * MVW_U + u) * nt) * 16u)
+			             : "memory");
 			const float xv = xs[(it + u) * MVW_SETS + set];
-			const uint32_t words[4] = {uint32_t(cur[u].x), uint32_t(cur[u].y), uint32_t(cur[u].z), uint32_t(cur[u].w)};
 #pragma unroll
 			for (int j = 0; j < 4; j++) {
-				float f[4];
-				i8x4_to_f32(words[j], f);
-#pragma unroll
-				for (int i = 0; i < 4; i++) acc[4 * j + i] = fmaf(xv, f[i], acc[4 * j + i]);
+				const uint32_t b = words[j] ^ 0x80808080u;  // (as i8x4_to_f32)
+				mvw_fma2(acc[2 * j], __byte_perm(b, 0x4B000000u, 0x7650u), __byte_perm(b, 0x4B000000u, 0x7651u), xv);
+				mvw_fma2(acc[2 * j + 1], __byte_perm(b, 0x4B000000u, 0x7652u), __byte_perm(b, 0x4B000000u, 0x7653u), xv);
 			}
 		}
-#pragma unroll
-		for (int u = 0; u < MVW_U; u++) cur[u] = nxt[u];
+		request(st);
+		if (++st == MVW_STAGES) st = 0;
 	}
+	asm volatile("cp.async.wait_group 0;" ::: "memory");
+	__syncthreads();  // (the ring is done with everywhere)
 	float *sums = xs + K;
 	if (set < MVW_SETS) {
 #pragma unroll
-		for (int i = 0; i < 16; i += 4)
-			*reinterpret_cast<float4 *>(sums + (set * groups + g) * 16 + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+		for (int i = 0; i < 8; i += 2)
+			*reinterpret_cast<float4 *>(sums + (set * groups + g) * 16 + 2 * i) = make_float4(acc[i].x, acc[i].y, acc[i + 1].x, acc[i + 1].y);
 	}
 	__syncthreads();
 	for (int c = tid; c < groups * 16; c += nt) {

@@ -3016,15 +3016,15 @@ int tg_dev_qmatvec(float *y, const float *x, const int8_t *w, const float *scale
 	if (sms_of[dev]) g_num_sms = sms_of[dev];
 	// the vocabulary matrix: one CTA per SM, an equal share of the columns each (below 64 groups of 16 columns per SM the
 	// rows a CTA reads get short and too little is in flight without a K-split)
-	const int groups = (N / 16 + g_num_sms - 1) / g_num_sms;
+	const int groups = ((N / 16 + g_num_sms - 1) / g_num_sms + 7) / 8 * 8;  // (whole 128-byte lines)
 	if (groups >= 64 && groups <= MVW_MAX_GROUPS && K % (MVW_SETS * MVW_U) == 0) {
-		const size_t smem = size_t(K) * 4 + size_t(MVW_SETS) * groups * 64;
+		const int nt = (MVW_SETS * groups + 31) / 32 * 32;
+		const size_t smem = size_t(K) * 4 + size_t(MVW_STAGES) * MVW_U * nt * 16;  // (the sums take less than the ring)
 		static bool configured[64] = {false};
 		if (!configured[dev]) {
-			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6912 * 4 + MVW_SETS * MVW_MAX_GROUPS * 64));
+			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6912 * 4 + MVW_STAGES * MVW_U * MVW_SETS * MVW_MAX_GROUPS * 16));
 			configured[dev] = true;
 		}
-		const int nt = (MVW_SETS * groups + 31) / 32 * 32;
 		launch_k(qmatvec_wide_kernel, dim3((N / 16 + groups - 1) / groups), dim3(nt), smem, (cudaStream_t)stream, y, x, w, scales, K, N, groups);
 		count_launch();
 		return check_launch("qmatvec_wide");
