@@ -80,6 +80,17 @@ __global__ void __launch_bounds__(SR_THREADS) argmax_kernel(SampleArgs a, unsign
 	}
 }
 
+// the tokens of the rows' keys that the vocabulary GEMM left (the same keys); they go back to zero for the next launch
+__global__ void top1_emit_kernel(SampleArgs a, unsigned long long *keys) {
+	pdl_trigger();
+	pdl_wait();
+	const int b = blockIdx.x * blockDim.x + threadIdx.x;
+	if (b >= a.B) return;
+	const unsigned long long k = keys[b];
+	keys[b] = 0ull;
+	emit_token(a, b, k ? int(0xFFFFFFFFu - uint32_t(k)) : -1);
+}
+
 // ------------------------------------------------------------------ exact parallel inverse CDF
 // Step (6) of min-p sampling is "the first index whose running fp32 sum reaches randf", where the
 // running sum is the sequential chain cum = fl(cum + p[i]). fp32 addition is not associative, so a
