@@ -43,7 +43,7 @@ def test_small_batch_keeps_the_bits_of_one_prompt(capi, synth, weights_270m):
 
 @pytest.mark.parametrize("n,S", [(4, 148), (4, 149), (7, 211)])
 def test_group_of_the_larger_model(capi, synth, weights_1b, n, S):
-    """Rows of 6912 columns on both sides of the line from which the GeGLU streams its rows (4 per SM)."""
+    """Rows of 6912 columns on both sides of the line from which the GEMM multiplies up and gate itself (4 per SM)."""
     m = capi.Model("1B").load_file(weights_1b)
     m.build_tables(1 << 20)
     prompts = np.stack([synth.random_prompt(S, 80 + i) for i in range(n)])

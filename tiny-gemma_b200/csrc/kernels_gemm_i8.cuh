@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_
 	}
 }
 
-// The same for many rows whose sums are not split: HBM bounds it (16384 x 6912: 0.91 GB in, 0.45 GB out, 0.21 ms at the copy
-// rate). The rows of a CTA arrive by bulk copies in a ring of STAGES rows, so that loads are in flight while a row waits
-// at its barriers and is packed; with the row's loads in registers alone the launch took 0.315 ms, with the ring 0.247.
+// The same for a thousand rows or so of few columns (a 2048-column model's) whose sums are not split, where the GEMM's epilogue does not
+// multiply them (launch_gemm_geglu): the rows of a CTA arrive by bulk copies in a ring of STAGES rows, so that loads are in
+// flight while a row waits at its barriers and is packed. HBM bounds it.
 template <int NT, int PER, int STAGES>
 __global__ void __launch_bounds__(NT) geglu_i8_stream_kernel(const float *ug, uint8_t *out, float *rowscale, int M, int I, int groups, GeluLut lut,
                                                              const float *su, const float *sg, int *err) {
@@ -540,6 +540,7 @@ struct GemmI8Args : I8Walk {
 	unsigned long long *top1;  // non-null (nsplit == 1): no C; per token the largest scaled value and its column, as a key
 	int top1_col0;
 	int *err;
+	GeluLut lut;  // GLU
 };
 
 // W tile [128 k][128 n], 128-byte swizzle: MN-major operand; 1 KiB from one group of 8 k-rows to the next
@@ -593,7 +594,12 @@ __device__ __forceinline__ void i8_cluster_sync() {
 }
 
 // xmap (CG = 2): the digits as rows of 512 bytes (one (group, digit) of a K-block), box of 2 * tg rows
-template <int CG>
+//
+// GLU: matrix 0 is up, matrix 1 gate, of the same size; the walk is one matrix's and every tile of it is done twice in a row, up and
+// then gate. A thread keeps its 32 up values in registers and leaves lut(gate) * up: one column of products goes through memory instead
+// of two of sums, and the launch behind it is a plain packing. 4096 x 1152 x (6912 | 6912): 164 us + 68 for the GeGLU -> 184 + 32. The
+// epilogue bounds it: with a branch per look-up it took 215 us, and with the table index in a loop of its own as well (GeluLut::index) 250.
+template <int CG, bool GLU>
 __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
                                                                  const __grid_constant__ CUtensorMap wmap1,
                                                                  const __grid_constant__ CUtensorMap wmap2,
@@ -610,9 +616,19 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 	__shared__ uint64_t drain_bar;          // every MMA issued has completed
 	__shared__ uint32_t tmem_base_s;
 	__shared__ int s_fail, s_issued;
+	__shared__ float table[GLU ? GE_LUT : 1];
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int rank = CG == 1 ? 0 : int(blockIdx.x & 1), first = int(blockIdx.x) / CG, stride = int(gridDim.x) / CG;
+	// the n-th tile of this CTA or pair
+	auto has_tile = [&](int n) { return first + (GLU ? n >> 1 : n) * stride < a.tiles; };
+	auto tile = [&](int n) {
+		I8Tile t = i8_tile<CG>(a, first + (GLU ? n >> 1 : n) * stride);
+		if (GLU) t.grp = n & 1;
+		return t;
+	};
+	if (GLU && a.lut.size <= GE_LUT)
+		for (int i = tid; i < a.lut.size; i += I8_THREADS) table[i] = a.lut.table[i];
 	if (tid == 0) {
 		for (int s = 0; s < NST; s++) {
 			mbar_init(&full_bar[s], 1);
@@ -676,14 +692,14 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		};
 		int cap = TC_SPIN_CAP, c = 0, s = 0;  // stages issued so far, next slot
 		uint32_t ph = 1;                      // parity whose completion frees the slot (a fresh barrier passes parity 1)
-		I8Tile t = i8_tile<CG>(a, first);
+		I8Tile t = tile(0);
 		// The weights are nobody's output: the first tiles are requested before the wait for the predecessor.
 		const int pre = first < a.tiles ? min(NST, t.ns) : 0;
 		for (int st = 0; st < pre; st++)
 			if (tc_elect()) load_w(t, st, st);
 		pdl_wait();
-		for (int ti = first; ti < a.tiles; ti += stride) {
-			t = i8_tile<CG>(a, ti);
+		for (int it = 0; has_tile(it); it++) {
+			t = tile(it);
 			for (int st = 0; st < t.ns; st++) {
 				tc_wait_cap(&free_bar[s], ph, cap);
 				if (tc_elect()) {
@@ -705,10 +721,10 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 	} else if (warp == 1) {
 		// ------------------------------------------------------------ MMA issuer (of a pair: the first CTA's)
 		if (rank == 0) {
-			int cap = TC_SPIN_CAP, s = 0, it = 0;
+			int cap = TC_SPIN_CAP, s = 0;
 			uint32_t ph = 0;
-			for (int ti = first; ti < a.tiles; ti += stride, it++) {
-				const I8Tile t = i8_tile<CG>(a, ti);
+			for (int it = 0; has_tile(it); it++) {
+				const I8Tile t = tile(it);
 				const uint32_t d = tmem_base + uint32_t(it & 1) * 256, id = i8_idesc<CG>(32 * t.ng);
 				tc_wait_cap(&acc_free[it & 1], ((it >> 1) & 1) ^ 1, cap);  // (the first use of a fresh barrier passes)
 				for (int st = 0; st < t.ns; st++) {
@@ -741,9 +757,11 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		pdl_wait();  // the row scales are the predecessor's output, and C may be its input
 		const int quad = warp & 3, sub = (warp - 2) >> 2;  // TMEM lanes 32 * quad ..; two warps share them
 		const bool fin = a.nsplit.d == 1 && !a.raw;
-		int it = 0;
-		for (int ti = first; ti < a.tiles; ti += stride, it++) {
-			const I8Tile t = i8_tile<CG>(a, ti);
+		const float *const lut_values = GLU && a.lut.size <= GE_LUT ? table : a.lut.table;
+		const float lut_base = -(a.lut.mn * a.lut.inv);
+		float kept[GLU ? 32 : 1];  // GLU: the up values of the tile before
+		for (int it = 0; has_tile(it); it++) {
+			const I8Tile t = tile(it);
 			const float *const scg = t.grp == 0 ? a.scales[0] : (t.grp == 1 ? a.scales[1] : a.scales[2]);
 			float *const Cg = t.grp == 0 ? a.C[0] : (t.grp == 1 ? a.C[1] : a.C[2]);
 			const size_t ld = fin ? size_t(t.grp == 0 ? a.ldc[0] : (t.grp == 1 ? a.ldc[1] : a.ldc[2])) : size_t(a.N);
@@ -752,18 +770,18 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 			const int ncg = t.grp == 0 ? a.ncols[0] : (t.grp == 1 ? a.ncols[1] : a.ncols[2]);
 			const bool live = CG == 1 || t.n0 + 128 * rank < ncg;  // (a pair's last tile may have only its first half)
 			float *dst = fin ? Cg + nl : a.partial + size_t(t.split) * a.M * a.N + pcol + nl;
-			const float sc = fin && live ? scg[nl] : 1.0f;
+			const float sc = (GLU || fin) && live ? scg[nl] : 1.0f;
 			const uint32_t acc = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(it & 1) * 256;
 			const float4 *rs = reinterpret_cast<const float4 *>(a.rowscale + t.g0 * 8);
 			// one token group: 32 accumulator columns = 4 digits x 8 tokens, and its row scales; lane i of the first eight: the largest
 			// value recorded for token i so far (top1)
 			auto request = [&](int g, uint32_t (&r)[32], float4 (&q)[2], uint32_t &seen) {
 				tc_ld32(acc + uint32_t(g * 32), r);
-				if (a.top1) seen = reinterpret_cast<const volatile uint32_t *>(a.top1)[2 * min((t.g0 + g) * 8 + (lane & 7), a.M - 1) + 1];
+				if (!GLU && a.top1) seen = reinterpret_cast<const volatile uint32_t *>(a.top1)[2 * min((t.g0 + g) * 8 + (lane & 7), a.M - 1) + 1];
 				q[0] = rs[2 * g];
 				q[1] = rs[2 * g + 1];
 			};
-			auto finish = [&](int g, uint32_t (&r)[32], float4 (&q)[2], uint32_t seen) {
+			auto finish = [&](int g, uint32_t (&r)[32], float4 (&q)[2], uint32_t seen, auto keep) {
 				const int tok = (t.g0 + g) * 8;
 				const float rsv[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
 				float v[8];
@@ -775,7 +793,29 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 					y = fmaf(y, 256.0f, float(int(r[i])));
 					v[i] = (y * rsv[i]) * sc;
 				}
-				if (a.top1) {
+				if constexpr (GLU) {
+					if (t.grp == 0) {
+#pragma unroll
+						for (int i = 0; i < 8; i++) kept[keep() + i] = v[i];
+						return;
+					}
+					// GeluLut::index, eight at a time and selected instead of branched on (int(x) >= 0 is x > -1)
+					float x[8], y[8];
+					if (a.lut.inv != 0.0f) {
+#pragma unroll
+						for (int i = 0; i < 8; i++) x[i] = fmaf(v[i], a.lut.inv, lut_base);
+					} else {
+#pragma unroll
+						for (int i = 0; i < 8; i++) x[i] = (v[i] - a.lut.mn) / a.lut.eps;
+					}
+#pragma unroll
+					for (int i = 0; i < 8; i++) y[i] = lut_values[min(max(int(x[i]), 0), a.lut.size - 1)];
+#pragma unroll
+					for (int i = 0; i < 8; i++) {
+						const float in = int(x[i]) < a.lut.size ? y[i] : v[i];
+						v[i] = (x[i] > -1.0f && x[i] < 2147483648.0f ? in : 0.0f) * kept[keep() + i];
+					}
+				} else if (a.top1) {
 					// Per token the largest value over the warp's 32 columns, the lowest column on equal values; NaN and -inf
 					// never win. Lane i keeps token i's; only a key above the recorded one goes to the atomic. After a row's first
 					// tiles hardly any value reaches what is recorded, and one vote says so (eight maxima over the lanes and a round
@@ -818,16 +858,23 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 			float4 qa[2], qb[2];
 			const int ng = live ? t.ng : 0;
 			if (sub < ng) request(sub, ra, qa, sa);
-#pragma unroll 1
-			for (int g = sub; g < ng; g += 4) {
+			auto pair_of_groups = [&](int g, auto keep_a, auto keep_b) {
 				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 				if (g + 2 < ng) request(g + 2, rb, qb, sb);
-				finish(g, ra, qa, sa);
+				finish(g, ra, qa, sa, keep_a);
 				if (g + 2 < ng) {
 					asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 					if (g + 4 < ng) request(g + 4, ra, qa, sa);
-					finish(g + 2, rb, qb, sb);
+					finish(g + 2, rb, qb, sb, keep_b);
 				}
+			};
+			if constexpr (GLU) {  // (written out: what is kept has to stay in registers)
+				static_assert(I8_TG == 8, "two pairs of token groups per warp");
+				if (sub < ng) pair_of_groups(sub, [] { return 0; }, [] { return 8; });
+				if (sub + 4 < ng) pair_of_groups(sub + 4, [] { return 16; }, [] { return 24; });
+			} else {
+#pragma unroll 1
+				for (int g = sub; g < ng; g += 4) pair_of_groups(g, [] { return 0; }, [] { return 0; });
 			}
 			tc_fence_before();
 			__syncwarp();

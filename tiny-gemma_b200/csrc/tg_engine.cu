@@ -1646,20 +1646,15 @@ int launch_resnorm(float *h, const float *t, const float *w_post, const float *w
 int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, const float *su, const float *sg, const TcScratch &sc, cudaStream_t st) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, I);
-	// several unsplit rows per SM: the CTA's next rows are copied while it works on one (one CTA per SM for the 55 KB rows of
-	// 6912, two for the 16 KB of 2048)
-	if (nsplit == 1 && M >= 4 * g_num_sms && I <= 7168) {
+	// several unsplit rows per SM: the CTA's next rows are copied while it works on one, two CTAs per SM for the 16 KB of 2048 columns
+	if (nsplit == 1 && M >= 4 * g_num_sms && I <= 2048) {
 		static bool configured[TG_MAX_DEVICES] = {false};
 		const int dev = current_device_slot();
 		if (!configured[dev]) {
-			TG_CUDA(cudaFuncSetAttribute(geglu_i8_stream_kernel<896, 2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 8 * 7168));
 			TG_CUDA(cudaFuncSetAttribute(geglu_i8_stream_kernel<512, 1, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * 8 * 2048));
 			configured[dev] = true;
 		}
-		if (I <= 2048)
-			launch_k(geglu_i8_stream_kernel<512, 1, 5>, dim3(2 * g_num_sms), dim3(512), size_t(5) * 8 * I, st, ug, sc.x, rs, M, I, groups, lut, su, sg, sc.err);
-		else
-			launch_k(geglu_i8_stream_kernel<896, 2, 3>, dim3(g_num_sms), dim3(896), size_t(3) * 8 * I, st, ug, sc.x, rs, M, I, groups, lut, su, sg, sc.err);
+		launch_k(geglu_i8_stream_kernel<512, 1, 5>, dim3(2 * g_num_sms), dim3(512), size_t(5) * 8 * I, st, ug, sc.x, rs, M, I, groups, lut, su, sg, sc.err);
 		count_launch();
 		return check_launch("geglu");
 	}
@@ -1717,8 +1712,8 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
 		configured[dev] = true;
 	}
 	const int K = ws[0]->K;
@@ -1779,9 +1774,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	if (pl.cg == 2) {
 		CUtensorMap xmap;
 		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
-		launch_clusters(2, qgemm_i8_kernel<2>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
+		launch_clusters(2, qgemm_i8_kernel<2, false>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
 	} else {
-		launch_k(qgemm_i8_kernel<1>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
+		launch_k(qgemm_i8_kernel<1, false>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
 	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
@@ -1792,6 +1787,59 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		TG_TRY(check_launch("qgemm_reduce"));
 	}
 	return TG_OK;
+}
+
+// up | gate, GeGLU and the packing of the down projection's operand. Many rows whose sums are not split: the GEMM's epilogue
+// multiplies (qgemm_i8_kernel<2, true>) and a plain packing follows; else raw sums and a GeGLU kernel. The epilogue's tiles come in
+// twos, so the line is where a pair of CTAs has three of them and more: below, the last round is emptier than that of single tiles.
+// Prompt passes, fused against not: 2048 columns, 592 rows (1.1 tiles) 1.84 ms against 1.76, 900 and 1500 (2.6) the same, 2048 (3.5)
+// 2.98 against 3.02, 4096 4.34 against 4.53; 6912 columns, 592 rows (3.6) the same, 1024 4.69 against 4.86, 2048 7.27 against 7.5.
+int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const TcScratch &sc, cudaStream_t st, int plan_rows = 0) {
+	const int K = U.K, I = U.N, cols[2] = {I, I};
+	const int rows = plan_rows ? plan_rows : M;
+	// (a row's sums follow the K-split of the rows planned for, whichever kernel multiplies)
+	static const bool asked = env_int("TG_GEMM_PAIR", 0) || env_int("TG_GEMM_SPLIT", 0);
+	const I8Plan pl = i8_plan(M, K, 1, cols, g_num_sms, sc.partial_floats, 1, true, 2, 1);
+	const bool many = !asked && M >= 4 * g_num_sms && long(pl.tok_tiles) * pl.col_tiles >= 3 * (g_num_sms / 2);
+	const bool fits = I <= 7168 && G.K == K && G.N == I && size_t(2) * M * I <= sc.partial_floats;
+	if (!many || !fits || i8_plan(rows, K, 2, cols, g_num_sms, sc.partial_floats, 16, true).nsplit != 1) {
+		float *Cs[2] = {nullptr, nullptr};
+		const QW *ws[2] = {&U, &G};
+		int ns = 0;
+		TG_TRY(launch_gemm_tc_group(2, Cs, ws, nullptr, M, sc, st, 16, &ns, plan_rows));
+		return launch_geglu(sc.partial, M, I, lut, ns, U.s, G.s, sc, st);
+	}
+	static bool configured[TG_MAX_DEVICES] = {false};
+	const int dev = current_device_slot();
+	if (!configured[dev]) {
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		configured[dev] = true;
+	}
+	GemmI8Args a{};
+	i8_fill_walk(a, pl, M, K, 1, cols);
+	CUtensorMap wmap[2], xmap;
+	const QW *ws[2] = {&U, &G};
+	for (int g = 0; g < 2; g++) {
+		if (ws[g]->map)
+			wmap[g] = *ws[g]->map;
+		else
+			TG_TRY(make_gemm_map(&wmap[g], *ws[g]));
+		a.ncols[g] = I;
+		a.scales[g] = ws[g]->s;
+	}
+	TG_TRY(make_digit_map(&xmap, sc.x, K, a.groups, a.tg));
+	a.x = sc.x;
+	a.rowscale = i8_rowscale(sc, M, K);
+	a.M = M;
+	a.N = I;
+	a.partial = sc.partial;
+	a.raw = 1;
+	a.err = sc.err;
+	a.lut = lut;
+	launch_clusters(2, qgemm_i8_kernel<2, true>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[1], xmap, a);
+	count_launch();
+	TG_TRY(check_launch("qgemm_i8"));
+	return pack_activations(sc.partial, M, I, sc, st);
 }
 int launch_gemm_tc(float *C, const QW &w, int M, const TcScratch &sc, cudaStream_t st, int ldc = 0, int max_split = 16) {
 	float *Cs[1] = {C};
@@ -1886,11 +1934,7 @@ int enqueue_decode_batched(tg_state *s, StepHead head) {
 			TG_TRY(gemm_raw(1, ws, &ns));
 		}
 		TG_TRY(resnorm_pack(s->btc.partial, w.attn_post, w.mlp_pre, ns, w.O.s));
-		{
-			const QW *ws[2] = {&w.U, &w.G};
-			TG_TRY(gemm_raw(2, ws, &ns));
-		}
-		TG_TRY(launch_geglu(s->btc.partial, B, I, lut, ns, w.U.s, w.G.s, s->btc, st));
+		TG_TRY(launch_gemm_geglu(w.U, w.G, B, lut, s->btc, st));
 		{
 			const QW *ws[1] = {&w.Dn};
 			TG_TRY(gemm_raw(1, ws, &ns));
@@ -2184,11 +2228,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 				TG_TRY(gemm_raw(1, ws, &ns));
 			}
 			TG_TRY(resnorm_pack(tc.partial, w.attn_post, w.mlp_pre, ns, w.O.s));
-			{
-				const QW *ws[2] = {&w.U, &w.G};
-				TG_TRY(gemm_raw(2, ws, &ns));
-			}
-			TG_TRY(launch_geglu(tc.partial, S, I, lut, ns, w.U.s, w.G.s, tc, st));
+			TG_TRY(launch_gemm_geglu(w.U, w.G, S, lut, tc, st, plan_rows));
 			{
 				const QW *ws[1] = {&w.Dn};
 				TG_TRY(gemm_raw(1, ws, &ns));
