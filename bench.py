@@ -708,7 +708,7 @@ def run_batched(args):
     line = {
         "metric": "decode_tok_s", "value": rec["tok_s"], "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": W,
         "ms_per_step": rec["ms_per_step"], "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "int8w/f32 (bf16x3 tensor-core GEMM)", "data": "synthetic",
+        "dtype": "int8w/f32 (int8-digit tensor-core GEMM)", "data": "synthetic",
         "config": {"workload": "gemma3-%s int8 weight-only, %d independent sequences in total, %d-token random "
                                "prompts, greedy decode" % (MODEL, rec["sequences"], PROMPT_LEN), "model_size": MODEL,
                    "prompt_len": PROMPT_LEN, "batch_per_gpu": rec["sequences_per_gpu"],

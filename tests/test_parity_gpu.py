@@ -354,8 +354,8 @@ def test_batch_rows_are_independent(capi, model_270m, synth):
 
 
 def test_batched_decode_tensor_core_step(capi, model_270m, synth):
-    """Batches of 16 and more take the batched step (tensor-core GEMMs with M = batch, bf16x3
-    activations). Teacher-forced against batch-1 states (CUDA-core matvecs) on a smooth GeLU table:
+    """Batches of 16 and more take the batched step (tensor-core GEMMs with M = batch, activations
+    in 8-bit digits). Teacher-forced against batch-1 states (CUDA-core matvecs) on a smooth GeLU table:
     the two differ only by the GEMM's split-activation rounding, <= 1e-4 relative L2 on the logits."""
     model_270m.build_tables(1 << 20)
     B, S, steps = 20, 24, 5
@@ -381,7 +381,7 @@ def test_batched_decode_tensor_core_step(capi, model_270m, synth):
 
 @pytest.mark.parametrize("size", ["270m", "1B"])
 def test_both_persistent_decode_kernels_agree(capi, synth, weights_270m, weights_1b, size, monkeypatch):
-    """The batch-1 decode path is the dp4a kernel (24-bit block fixed-point activations, exact integer products);
+    """The batch-1 decode path is the tensor-core kernel (31-bit block fixed-point activations, exact integer products);
     TG_PERSIST=0 selects the fp32-FMA kernel it replaced, which stays as the fall-back for shapes without a plan.
     Same prompt, smooth GeLU table: logits of the last of 24 steps within 2e-5, greedy tokens equal where the top-2
     gap is above that noise."""
@@ -410,7 +410,7 @@ def test_both_persistent_decode_kernels_agree(capi, synth, weights_270m, weights
 
 
 def test_small_grid_decodes_the_same_tokens(capi, synth, weights_270m, monkeypatch):
-    """TG_MEGA_GRID=48 leaves the persistent decode a third of the SMs. The dp4a kernel has no plan for so few
+    """TG_MEGA_GRID=48 leaves the persistent decode a third of the SMs. The tensor-core kernel has no plan for so few
     CTAs, so the fp32-FMA kernel runs, with another unit-to-CTA plan than on the full grid (O-projection K-slices
     of two heads, 16 instead of 116 CTAs left to wipe the hand-off arena during the attention phase).
     Teacher-forced on the full grid's greedy tokens: the logits of every one of 16 steps within 2e-5, the arg-max

@@ -104,7 +104,7 @@ template <int NW> __device__ __forceinline__ uint32_t block_umax(uint32_t v, uin
 // (of some warp's part of the row) lie below 2^-12 of the largest (such an element is kept to 2^-19 of itself), and rows below 2^-96
 // altogether, are marked by the operators' packing and recomputed by qgemm_wide_rows_kernel. A normal row with one element of s
 // sigmas is marked from s = 512 on, from 256 on now and then; below, a column that does not see that element is off by 1.4e-7 at
-// most. (A model's own passes mark nothing: their rows come out of a norm or a GeGLU, and its decode steps hold them to 2^-24 of the
+// most. (A model's own passes mark nothing: their rows come out of a norm or a GeGLU, and its decode steps hold them to 2^-31 of the
 // largest in any case.) Called by whole warps; the zeros are told apart only where many elements are small.
 template <int PER> __device__ __forceinline__ bool i8_wide(const float4 (&v)[PER], uint32_t maxbits) {
 	const float below = __uint_as_float(uint32_t(max(int(maxbits >> 23) - 11, 0)) << 23);
@@ -599,13 +599,17 @@ __device__ __forceinline__ void i8_cluster_sync() {
 // then gate. A thread keeps its 32 up values in registers and leaves lut(gate) * up: one column of products goes through memory instead
 // of two of sums, and the launch behind it is a plain packing. 4096 x 1152 x (6912 | 6912): 164 us + 68 for the GeGLU -> 184 + 32. The
 // epilogue bounds it: with a branch per look-up it took 215 us, and with the table index in a loop of its own as well (GeluLut::index) 250.
-template <int CG, bool GLU>
+// What the epilogue does is a parameter of the kernel, not of the launch: with the code of the others beside it
+// a prompt of 178 tokens took 1.79 ms instead of 1.76 (156 registers instead of 140, and more code to fetch).
+enum I8Epilogue { I8_SUMS, I8_GLU, I8_TOP1 };  // finished values or raw sums; the product of up and gate; a key per token
+template <int CG, I8Epilogue EPI>
 __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
                                                                  const __grid_constant__ CUtensorMap wmap1,
                                                                  const __grid_constant__ CUtensorMap wmap2,
                                                                  const __grid_constant__ CUtensorMap xmap, GemmI8Args a) {
 	using SH = I8Shape<CG>;
 	constexpr int NST = SH::NST;
+	constexpr bool GLU = EPI == I8_GLU, TOP1 = EPI == I8_TOP1;
 	pdl_trigger();
 	extern __shared__ uint8_t i8_smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(i8_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -777,7 +781,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 			// value recorded for token i so far (top1)
 			auto request = [&](int g, uint32_t (&r)[32], float4 (&q)[2], uint32_t &seen) {
 				tc_ld32(acc + uint32_t(g * 32), r);
-				if (!GLU && a.top1) seen = reinterpret_cast<const volatile uint32_t *>(a.top1)[2 * min((t.g0 + g) * 8 + (lane & 7), a.M - 1) + 1];
+				if (TOP1) seen = reinterpret_cast<const volatile uint32_t *>(a.top1)[2 * min((t.g0 + g) * 8 + (lane & 7), a.M - 1) + 1];
 				q[0] = rs[2 * g];
 				q[1] = rs[2 * g + 1];
 			};
@@ -815,7 +819,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 						const float in = int(x[i]) < a.lut.size ? y[i] : v[i];
 						v[i] = (x[i] > -1.0f && x[i] < 2147483648.0f ? in : 0.0f) * kept[keep() + i];
 					}
-				} else if (a.top1) {
+				} else if constexpr (TOP1) {
 					// Per token the largest value over the warp's 32 columns, the lowest column on equal values; NaN and -inf
 					// never win. Lane i keeps token i's; only a key above the recorded one goes to the atomic. After a row's first
 					// tiles hardly any value reaches what is recorded, and one vote says so (eight maxima over the lanes and a round

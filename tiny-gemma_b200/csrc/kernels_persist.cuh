@@ -77,7 +77,7 @@ struct PsSpan {
 struct PsArgs {
 	const int8_t *tiled;  // re-tiled layer weights: per layer [A units | C units | D units (up, gate) | E units]
 	size_t tl_layer, tl_A, tl_C, tl_D, tl_E;
-	const int8_t *lm_tiled;  // re-tiled lm_head: [tile][chunk][group][quad] pieces
+	const int8_t *lm_tiled;  // re-tiled lm_head: [tile][chunk] ring stages of core matrices
 	const PsLayer *layers;
 	int L, D, I, V, QD, KD;
 	PsPhase A, C, Dp, E;

@@ -129,7 +129,7 @@ struct tg_model {
 	size_t dec_tiled_bytes = 0;
 	long dec_tiled_version = -1;
 	int dec_tiled_key[12] = {0};
-	// the same for the dp4a decode kernel: layer units as 4 x 4 pieces, and the lm_head in ring-stage order
+	// the same for the tensor-core decode kernel: layer units as core matrices with their scales, and the lm_head in ring-stage order
 	int8_t *ps_tiled = nullptr, *ps_lm = nullptr;
 	size_t ps_tiled_bytes = 0, ps_lm_bytes = 0;
 	long ps_tiled_version = -1;
@@ -505,7 +505,7 @@ struct tg_state {
 	unsigned *mg_bar = nullptr;
 	int mega_grid = 0;
 	long long *mg_dbg = nullptr;
-	// dp4a persistent decode kernel
+	// tensor-core persistent decode kernel
 	bool ps_ok = false;
 	PsArgs ps{};
 	PsLayer *d_pslayers = nullptr;
@@ -1712,8 +1712,10 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
 		configured[dev] = true;
 	}
 	const int K = ws[0]->K;
@@ -1774,9 +1776,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	if (pl.cg == 2) {
 		CUtensorMap xmap;
 		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
-		launch_clusters(2, qgemm_i8_kernel<2, false>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
+		launch_clusters(2, sc.top1 ? qgemm_i8_kernel<2, I8_TOP1> : qgemm_i8_kernel<2, I8_SUMS>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
 	} else {
-		launch_k(qgemm_i8_kernel<1, false>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
+		launch_k(sc.top1 ? qgemm_i8_kernel<1, I8_TOP1> : qgemm_i8_kernel<1, I8_SUMS>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
 	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
@@ -1790,7 +1792,7 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 }
 
 // up | gate, GeGLU and the packing of the down projection's operand. Many rows whose sums are not split: the GEMM's epilogue
-// multiplies (qgemm_i8_kernel<2, true>) and a plain packing follows; else raw sums and a GeGLU kernel. The epilogue's tiles come in
+// multiplies (qgemm_i8_kernel<2, I8_GLU>) and a plain packing follows; else raw sums and a GeGLU kernel. The epilogue's tiles come in
 // twos, so the line is where a pair of CTAs has three of them and more: below, the last round is emptier than that of single tiles.
 // Prompt passes, fused against not: 2048 columns, 592 rows (1.1 tiles) 1.84 ms against 1.76, 900 and 1500 (2.6) the same, 2048 (3.5)
 // 2.98 against 3.02, 4096 4.34 against 4.53; 6912 columns, 592 rows (3.6) the same, 1024 4.69 against 4.86, 2048 7.27 against 7.5.
@@ -1812,7 +1814,7 @@ int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
 		configured[dev] = true;
 	}
 	GemmI8Args a{};
@@ -1836,7 +1838,7 @@ int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const
 	a.raw = 1;
 	a.err = sc.err;
 	a.lut = lut;
-	launch_clusters(2, qgemm_i8_kernel<2, true>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[1], xmap, a);
+	launch_clusters(2, qgemm_i8_kernel<2, I8_GLU>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[1], xmap, a);
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
 	return pack_activations(sc.partial, M, I, sc, st);
@@ -2515,7 +2517,7 @@ int tg_state_create(tg_model *m, int batch, int max_pos_global, tg_state **out) 
 			if (env_int("TG_MEGA", 1) == 2) rc = mrc;  // 2 = required
 			s->mega_ok = false;
 		} else if (env_int("TG_PERSIST", 1)) {
-			// the dp4a kernel (kernels_persist.cuh) is the batch-1 decode path; a shape it has no plan for falls back
+			// the tensor-core kernel (kernels_persist.cuh) is the batch-1 decode path; a shape it has no plan for falls back
 			// to the fp32-FMA kernel (kernels_mega.cuh), which TG_PERSIST=0 also selects
 			int prc = persist_setup(s);
 			if (prc != TG_OK) {
