@@ -2052,15 +2052,16 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		tc.err = s->err_flag;
 		p += (tc.x_bytes + 3) / 4;
 	}
-	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 672 tokens, and for a group of
-	// equal prompts of 16 and more tokens each that has more than 420 + 50000 / S of them in all. Otherwise the CUDA-core kernel
+	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 960 tokens, and for a group of
+	// equal prompts of 16 and more tokens each that has more than 960 + 16384 / S of them in all. Otherwise the CUDA-core kernel
 	// with two queries per CTA is faster: its CTAs are more, and a prompt fills no tiles of 32 queries and 64 keys, as which the
-	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill in ms, 1B and 270m: one prompt of 450 tokens
-	// 2.93 / 3.27 and 1.41 / 1.64, of 600 3.56 / 3.80 and 1.74 / 1.88, of 832 4.85 / 4.36 and 2.39 / 2.05; groups of 178 tokens: 712 rows 3.67 / 3.46
-	// and 1.72 / 1.54, 1424 6.24 / 5.04 and 2.66 / 1.86; of 61: 976 rows 3.81 / 3.91 and 1.60 / 1.67, 1464 5.02 / 4.94 and 1.82 / 1.77; of 30: 2100 rows
-	// 6.70 / 7.00 and 2.38 / 2.32; of 16: 2048 rows 6.48 / 6.73 and 2.28 / 2.31. (Before the two fp16 terms the lines were 960 and 960 + 16384 / S.)
+	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill of the 1B model in ms: one prompt of
+	// 450 tokens 2.9 / 3.6, of 832 4.93 / 5.04; groups of 976 rows of 8 tokens 3.77 / 4.20, of 61 3.81 / 3.97 (1464: 5.27 / 5.31), of 178
+	// 890 rows 3.90 / 4.09, 1424 5.51 / 5.24; of 16 tokens 976 rows 3.66 / 3.99, 2192 7.61 / 7.03 to 7.70, 16384 51.9 / 52.0; of 8 tokens
+	// 8192 rows 27.0 / 28.8, of 2 tokens 1500 rows 5.7 / 9.0; of 178 tokens 16376 rows 57.2 / 49.8. 270m: of 30 tokens 2190 rows 2.36 /
+	// 2.40, 4080 3.82 / 3.53; of 61 tokens 1464 rows 1.79 / 1.83, 2196 2.48 / 2.35; of 8 tokens 8192 rows 7.7 / 9.5.
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
-	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", at_rows > S_seq ? 420 + 50000 / S_seq : 672);
+	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", 960) + (at_rows > S_seq ? 16384 / S_seq : 0);
 	const bool attn_tc = use_tc && pos0 < 0 && c.n_layers <= AttnTcPlan::MAX_WORDS && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
 	__half *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	unsigned *at_vmax = nullptr;  // [layer][prompt]
