@@ -8,28 +8,26 @@
 //     S = Q K_j^T                    M128 x N64, contraction over the 256 head dimensions
 //     online softmax on S            (max in use m and sum l per row; a row = one TMEM lane, two threads)
 //     O = corr * O + P V_j           M128 x N256, contraction over the 64 keys
-// fp32 accuracy on 16-bit tensor cores: every fp32 operand is split into two fp16 terms x = hi + lo, each rounded to
-// nearest (11 + 11 significant bits: off by at most 2^-23 of x), and a product a * b is the three term products hi hi, hi lo,
-// lo hi, accumulated in fp32 in TMEM. (Three bf16 terms and six products kept 2^-27 of an operand, but every further product is
-// a further rounding of the fp32 accumulator, which outweighs both: see the errors at attn_tc_scale.) fp16 has a range of 2^15 to 2^-24: the operands are
-// scaled by powers of two that the packing kernels and the attention take from the same place: q and k by the bound that their norm
-// weights give, v by the prompt's largest |v| (an atomic maximum in the norm + RoPE kernel), p by 16.
+// fp32 accuracy on bf16 tensor cores: every fp32 operand is split into three bf16 terms x = hi + mid + lo (kernels_tc.cuh:
+// all 24 bits, fp32's range) and a product a * b is the six term products whose weight reaches
+// 2^-24 (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi), all accumulated in fp32 in TMEM.
+// Two fp16 terms and three products take less time (16384 tokens of the 1B model 59 ms instead of 66), but they hold 22 to 23 bits of an
+// operand inside fp16's range only, so v would need a scale from keys that a row may not see: its bits, and whether it is finite,
+// would hang on later tokens.
 //
 // Operands are packed once per layer in the tensor core's shared-memory layouts (no swizzle, 8 x 8 core
 // matrices), so that the CTA fetches them with plain bulk copies:
-//     Q, K: attn_pack_rows_kernel ([2 terms][128-row tiles][8 blocks of 32 dimensions][8 KiB], K-major; a 64-key
+//     Q, K: split_pack_kernel ([3 terms][128-row tiles][8 blocks of 32 dimensions][8 KiB], K-major; a 64-key
 //           tile is one half of a 128-row tile)
-//     V:    attn_pack_v_kernel ([2 terms][16-key blocks][8 KiB], N-major like the GEMM's weight operand)
-// Two terms of Q (128 KiB) stay in shared memory for the whole walk; with three they were fetched again for every key tile,
-// 288 of 384 KB.
+//     V:    attn_pack_v_kernel ([3 terms][16-key blocks][8 KiB], N-major like the GEMM's weight operand)
 // Warps 0-7: softmax and epilogue (two threads per row: warps w and w + 4 share the TMEM lanes 32 (w % 4) ..
 // and take half of a tile's keys each); warp 8: one thread issues the MMAs; warp 9: one thread issues the bulk
-// copies, up to three ring blocks ahead of the MMAs.
-// Per key tile the ring carries four K blocks (64 dimensions each) and four V blocks (16 keys each).
+// copies, up to four ring blocks ahead of the MMAs.
+// Per key tile the ring carries eight Q|K blocks (one per 32 dimensions) and four V blocks (16 keys each).
 // S is double-buffered in TMEM and the MMAs are issued as Q K_0^T, Q K_1^T, P V_0, Q K_2^T, P V_1, ...: while the
 // softmax warps work on tile t the tensor core runs Q K_{t+1}^T and P V_{t-1}. The running max is only moved (and
 // O rescaled, a TMEM round trip) when a row's new max exceeds the one in use by more than 8: the probabilities
-// are then at most e^8, times 16 inside fp16's range, and the final division by the row sum removes the common factor.
+// are then at most e^8, far inside fp32, and the final division by the row sum removes the common factor.
 // All waits are bounded; a wait that runs out sets *err, and the CTA lets its copies land and frees its
 // TMEM before it returns.
 #pragma once
@@ -38,101 +36,53 @@
 namespace tg {
 
 constexpr int AT_TC_KT = 64;                       // keys per tile
-constexpr int AT_TC_STAGE = 16 * 1024;             // ring stage: K (2 terms x 2 blocks of 32 dimensions x 4 KiB), or V (2 x 8 KiB)
-constexpr int AT_TC_NS = 3;                        // ring stages
-constexpr int AT_TC_QBYTES = 2 * 8 * TC_TILE_BYTES;  // Q: 2 terms x 8 blocks of 32 dimensions
-constexpr int AT_TC_PBYTES = 2 * 2 * TC_TILE_BYTES;  // P: 2 terms x 2 blocks of 32 keys x [128][32] fp16
-constexpr int AT_TC_SMEM = AT_TC_QBYTES + AT_TC_NS * AT_TC_STAGE + AT_TC_PBYTES + 1024;
+constexpr int AT_TC_STAGE = 36 * 1024;             // ring stage: Q (3 x 8 KiB) + K (3 x 4 KiB), or V (3 x 8 KiB)
+constexpr int AT_TC_NS = 4;                        // ring stages
+constexpr int AT_TC_PBYTES = 3 * 2 * TC_TILE_BYTES;  // P: 3 terms x 2 blocks of 32 keys x [128][32] bf16
+constexpr int AT_TC_SMEM = AT_TC_NS * AT_TC_STAGE + AT_TC_PBYTES + 1024;
 constexpr int AT_TC_THREADS = 320;                 // 8 softmax warps, the MMA-issuing warp, the copy-issuing warp
-constexpr int AT_TC_BLOCKS = 8;                    // ring blocks per key tile: 4 of K (64 dimensions each), 4 of V (16 keys each)
-constexpr int AT_TC_VBYTES = 8192;                 // one term of a V block: [16 keys][256 dimensions] fp16
-constexpr float AT_TC_PSCALE = 16.0f;
+constexpr int AT_TC_BLOCKS = 12;                   // ring blocks per key tile: 8 of Q|K (32 dimensions each), 4 of V (16 keys each)
+constexpr int AT_TC_VBYTES = 8192;                 // one term of a V block: [16 keys][256 dimensions] bf16
 
-// ------------------------------------------------------------------ scales
-// Against the fp32 kernels (attn_prefill_blk_kernel), keys and values of the layers 1, 5 and the last and logits behind 4001 tokens:
-// 270m 3.0e-6, 4.8e-6, 7.0e-6, 8.6e-6 relative, with three bf16 terms and six products 4.2e-6, 5.6e-6, 7.6e-6, 1.09e-5; 1B 2.5e-6, 4.0e-6, 7.6e-6,
-// 6.9e-6 against 3.6e-6, 4.8e-6, 9.4e-6, 8.9e-6. Prefill of 16384 tokens 66.1 -> 59.1 ms.
-// the power of two that brings a magnitude of at most `bound` to at most 2^13 (RoPE tables of up to 2.8 times the unit circle
-// stay inside fp16's 2^16; an element 2^-22 of the bound keeps its 22 bits)
-__device__ __forceinline__ float attn_tc_scale(float bound) {
-	const int e = int(__float_as_uint(bound) >> 23) - 126;  // bound < 2^e
-	return __uint_as_float(uint32_t(max(1, min(253, 127 + 13 - e))) << 23);
-}
-// Scale of normed and rotated rows of 256: |x| / rms <= 16, the norm's gain 1 + w, sqrt(2) from the rotation. Called by whole warps.
-__device__ __forceinline__ float attn_tc_row_scale(const float *w) {
-	float m = 0.0f;
-#pragma unroll
-	for (int i = 0; i < 8; i++) m = fmaxf(m, fabsf(__ldg(w + 32 * i + (threadIdx.x & 31)) + 1.0f));
-	return attn_tc_scale(22.7f * warp_max(m));
-}
-// x * scale as two fp16 terms, pairs of consecutive elements
-__device__ __forceinline__ void attn_tc_split(float a, float b, uint32_t &hi, uint32_t &lo) {
-	const __half2 h = __floats2half2_rn(a, b);
-	const float2 f = __half22float2(h);
-	const __half2 l = __floats2half2_rn(a - f.x, b - f.y);  // (the differences are exact)
-	hi = *reinterpret_cast<const uint32_t *>(&h);
-	lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-// rows [M][256] (normed by gain 1 + w, rotated) -> [2 terms][m_tiles][8 blocks][8 KiB]; rows >= M are zero. blockIdx.y: the prompt
-__global__ void __launch_bounds__(256) attn_pack_rows_kernel(const float *A, const float *w, __half *out, int M, int m_tiles) {
-	const float sc = attn_tc_row_scale(w);  // (the weights are nobody's output)
-	pdl_trigger();
-	pdl_wait();
-	A += size_t(blockIdx.y) * M * 256;
-	const size_t term_stride = size_t(m_tiles) * 8 * (TC_TILE_BYTES / 2);  // elements
-	out += size_t(blockIdx.y) * 2 * term_stride;
-	const size_t n_chunks = size_t(m_tiles) * TC_BM * 32;  // one thread per (row, 8 consecutive dimensions)
-	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_chunks; c += size_t(gridDim.x) * blockDim.x) {
-		int row, k8;
-		tc_chunk_to_row_k8(c, 32, row, k8);
-		float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-		if (row < M) {
-			a = *reinterpret_cast<const float4 *>(A + size_t(row) * 256 + 8 * k8);
-			b = *reinterpret_cast<const float4 *>(A + size_t(row) * 256 + 8 * k8 + 4);
-		}
-		uint4 hi, lo;
-		attn_tc_split(a.x * sc, a.y * sc, hi.x, lo.x);
-		attn_tc_split(a.z * sc, a.w * sc, hi.y, lo.y);
-		attn_tc_split(b.x * sc, b.y * sc, hi.z, lo.z);
-		attn_tc_split(b.z * sc, b.w * sc, hi.w, lo.w);
-		const size_t off = (size_t(row / TC_BM) * 8 + (k8 >> 2)) * (TC_TILE_BYTES / 2) + ((row % TC_BM) / 8) * 256 + (k8 & 3) * 64 + (row % 8) * 8;
-		*reinterpret_cast<uint4 *>(out + off) = hi;
-		*reinterpret_cast<uint4 *>(out + term_stride + off) = lo;
-	}
-}
-
-// v fp32 [S][256] -> two fp16 terms (scaled by the prompt's largest |v|, vmax) in the N-major operand layout, one 8 KiB tile per 16 keys (one MMA K-step):
+// v fp32 [S][256] -> three bf16 terms in the N-major operand layout, one 8 KiB tile per 16 keys (one MMA K-step):
 // byte offset of (key k, dimension n) = (n / 8) * 256 + (k / 8) * 128 + (k % 8) * 16 + (n % 8) * 2. Keys >= S are zero.
-__global__ void __launch_bounds__(256) attn_pack_v_kernel(const float *v, const unsigned *vmax, __half *out, int S, int nblocks) {
+__global__ void __launch_bounds__(256) attn_pack_v_kernel(const float *v, __nv_bfloat16 *out, int S, int nblocks) {
 	pdl_trigger();
 	pdl_wait();
-	const float sc = attn_tc_scale(__uint_as_float(vmax[blockIdx.y]));
 	v += size_t(blockIdx.y) * S * 256;  // blockIdx.y: the prompt
-	out += size_t(blockIdx.y) * 2 * nblocks * 4096;
+	out += size_t(blockIdx.y) * 3 * nblocks * 4096;
 	const size_t term_stride = size_t(nblocks) * 4096;  // elements
 	const size_t n_items = size_t(nblocks) * 16 * 32;   // (key, 8 consecutive dimensions)
 	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_items; c += size_t(gridDim.x) * blockDim.x) {
 		const int key = int(c >> 5), n8 = int(c & 31);
-		float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+		float x[8];
 		if (key < S) {
-			a = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8);
-			b = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8 + 4);
+			const float4 a = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8);
+			const float4 b = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8 + 4);
+			x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+		} else {
+#pragma unroll
+			for (int i = 0; i < 8; i++) x[i] = 0.0f;
 		}
-		uint4 hi, lo;
-		attn_tc_split(a.x * sc, a.y * sc, hi.x, lo.x);
-		attn_tc_split(a.z * sc, a.w * sc, hi.y, lo.y);
-		attn_tc_split(b.x * sc, b.y * sc, hi.z, lo.z);
-		attn_tc_split(b.z * sc, b.w * sc, hi.w, lo.w);
+		__align__(16) __nv_bfloat16 hi[8], mid[8], lo[8];
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			hi[i] = __float2bfloat16_rn(x[i]);
+			const float r1 = x[i] - __bfloat162float(hi[i]);
+			mid[i] = __float2bfloat16_rn(r1);
+			lo[i] = __float2bfloat16_rn(r1 - __bfloat162float(mid[i]));
+		}
 		const int kb = key >> 4, k = key & 15;
 		const size_t off = size_t(kb) * 4096 + n8 * 128 + (k >> 3) * 64 + (k & 7) * 8;  // elements
-		*reinterpret_cast<uint4 *>(out + off) = hi;
-		*reinterpret_cast<uint4 *>(out + term_stride + off) = lo;
+		*reinterpret_cast<uint4 *>(out + off) = *reinterpret_cast<const uint4 *>(hi);
+		*reinterpret_cast<uint4 *>(out + term_stride + off) = *reinterpret_cast<const uint4 *>(mid);
+		*reinterpret_cast<uint4 *>(out + 2 * term_stride + off) = *reinterpret_cast<const uint4 *>(lo);
 	}
 }
 
-// instruction descriptor: D fp32, A and B fp16, A K-major, B K-major (b_mn = 0) or N-major (1), M = 128, N = n
+// instruction descriptor: D fp32, A and B bf16, A K-major, B K-major (b_mn = 0) or N-major (1), M = 128, N = n
 __device__ __forceinline__ uint32_t at_idesc(int n, int b_mn) {
-	return (1u << 4) | (uint32_t(b_mn) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
+	return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(b_mn) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
 }
 // shared-memory matrix descriptor of a V block: no swizzle, 128 B between the two 8-key groups, 256 B between
 // groups of 8 dimensions
@@ -191,11 +141,9 @@ __device__ __forceinline__ bool at_exchange(float *val, int *tag, int me, float 
 
 struct AttnTcArgs {
 	// per prompt (blockIdx.y), one behind the other:
-	const __half *qp;         // [2][q_tiles][8][8 KiB]
-	const __half *kp;         // [2][k_tiles][8][8 KiB]
-	const __half *vp;         // [2][v_blocks][8 KiB]
-	const unsigned *vmax;     // largest |v|, as bits
-	const float *rmsq, *rmsk;  // norm weights: the scales of q and k
+	const __nv_bfloat16 *qp;  // [3][q_tiles][8][8 KiB]
+	const __nv_bfloat16 *kp;  // [3][k_tiles][8][8 KiB]
+	const __nv_bfloat16 *vp;  // [3][v_blocks][8 KiB]
 	float *o;                 // [S][4][256]
 	int S, q_tiles, k_tiles, v_blocks;
 	int is_local, window;
@@ -206,8 +154,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	pdl_trigger();
 	extern __shared__ uint8_t at_smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(at_smem_raw) + 1023) & ~uintptr_t(1023));
-	uint8_t *qbuf = smem, *ring = smem + AT_TC_QBYTES, *pbuf = ring + AT_TC_NS * AT_TC_STAGE;
-	__shared__ uint64_t q_bar;               // Q landed
+	uint8_t *pbuf = smem + AT_TC_NS * AT_TC_STAGE;
 	__shared__ uint64_t full_bar[AT_TC_NS];  // the stage's copies landed
 	__shared__ uint64_t free_bar[AT_TC_NS];  // the MMAs that read the stage have completed
 	__shared__ uint64_t s_bar[2];            // S = Q K^T of a key tile is complete (two S buffers, tiles alternate)
@@ -238,7 +185,6 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		mbar_init(&p_bar, 8);
 		mbar_init(&pv_bar, 1);
 		mbar_init(&o_bar, 1);
-		mbar_init(&q_bar, 1);
 		s_fail = 0;
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -254,16 +200,16 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	volatile int *fail = &s_fail;
 
 	// MMA order: QK(0), then for t = 1 .. n: QK(t) (if t < n), PV(t - 1). Ring block g in that order:
-	// g < 4: QK(0) block g; else g' = g - 4, t = 1 + g' / 8, r = g' % 8: QK(t) block r (r < 4, t < n) or PV(t - 1)
-	// block r - 4 (t < n), and the last four blocks are PV(n - 1).
+	// g < 8: QK(0) block g; else g' = g - 8, t = 1 + g' / 12, r = g' % 12: QK(t) block r (r < 8, t < n) or PV(t - 1)
+	// block r - 8 (t < n), and the last four blocks are PV(n - 1).
 	struct Blk {
-		int qk, tile, i;  // qk: 1 = K block i (dimensions 64 i ..) of key tile `tile`, 0 = V block i (keys 16 i ..) of it
+		int qk, tile, i;  // qk: 1 = Q|K block i (dimensions 32 i ..) of key tile `tile`, 0 = V block i (keys 16 i ..) of it
 	};
 	auto blk = [&](int g) -> Blk {
-		if (g < 4) return Blk{1, 0, g};
-		const int gp = g - 4, t = 1 + gp / AT_TC_BLOCKS, r = gp % AT_TC_BLOCKS;
+		if (g < 8) return Blk{1, 0, g};
+		const int gp = g - 8, t = 1 + gp / AT_TC_BLOCKS, r = gp % AT_TC_BLOCKS;
 		if (t >= ntiles) return Blk{0, ntiles - 1, r};
-		return r < 4 ? Blk{1, t, r} : Blk{0, t - 1, r - 4};
+		return r < 8 ? Blk{1, t, r} : Blk{0, t - 1, r - 8};
 	};
 	const int total = ntiles * AT_TC_BLOCKS;
 	if (warp == 9) {
@@ -271,35 +217,29 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		pdl_wait();  // the packed operands are the predecessors' output
 		const size_t q_term = size_t(a.q_tiles) * 8 * TC_TILE_BYTES, k_term = size_t(a.k_tiles) * 8 * TC_TILE_BYTES,
 		             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
-		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 2 * q_term, *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 2 * k_term,
-		              *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 2 * v_term;
-		if (tc_elect()) {
-			mbar_expect_tx(&q_bar, uint32_t(AT_TC_QBYTES));
-#pragma unroll
-			for (int t = 0; t < 2; t++)
-				bulk_load(qbuf + t * 8 * TC_TILE_BYTES, qp + t * q_term + size_t(tile) * 8 * TC_TILE_BYTES, 8 * TC_TILE_BYTES, &q_bar);
-		}
-		__syncwarp();
+		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 3 * q_term, *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 3 * k_term,
+		              *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 3 * v_term;
 		int cap = TC_SPIN_CAP, st = 0;
 		uint32_t ph = 1;  // (a fresh barrier passes parity 1)
 		for (int g = 0; g < total; g++) {
 			const Blk b = blk(g);
 			const int j = j_lo + b.tile, i = b.i;
-			uint8_t *dst = ring + size_t(st) * AT_TC_STAGE;
+			uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
 			tc_wait_cap(&free_bar[st], ph, cap);
 			if (tc_elect()) {
 				if (b.qk) {
-					mbar_expect_tx(&full_bar[st], uint32_t(AT_TC_STAGE));
+					mbar_expect_tx(&full_bar[st], 3u * TC_TILE_BYTES + 3u * (TC_TILE_BYTES / 2));
 #pragma unroll
-					for (int t = 0; t < 2; t++)
-#pragma unroll
-						for (int h = 0; h < 2; h++)
-							bulk_load(dst + (2 * t + h) * (TC_TILE_BYTES / 2), kp + t * k_term + (size_t(j >> 1) * 8 + 2 * i + h) * TC_TILE_BYTES + (j & 1) * (TC_TILE_BYTES / 2),
-							          TC_TILE_BYTES / 2, &full_bar[st]);
+					for (int t = 0; t < 3; t++) {
+						bulk_load(dst + t * TC_TILE_BYTES, qp + t * q_term + (size_t(tile) * 8 + i) * TC_TILE_BYTES, TC_TILE_BYTES, &full_bar[st]);
+						bulk_load(dst + 3 * TC_TILE_BYTES + t * (TC_TILE_BYTES / 2),
+						          kp + t * k_term + (size_t(j >> 1) * 8 + i) * TC_TILE_BYTES + (j & 1) * (TC_TILE_BYTES / 2), TC_TILE_BYTES / 2,
+						          &full_bar[st]);
+					}
 				} else {
-					mbar_expect_tx(&full_bar[st], 2u * AT_TC_VBYTES);
+					mbar_expect_tx(&full_bar[st], 3u * AT_TC_VBYTES);
 #pragma unroll
-					for (int t = 0; t < 2; t++)
+					for (int t = 0; t < 3; t++)
 						bulk_load(dst + t * AT_TC_VBYTES, vp + t * v_term + (size_t(4 * j + i)) * AT_TC_VBYTES, AT_TC_VBYTES, &full_bar[st]);
 				}
 			}
@@ -315,39 +255,36 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	} else if (warp == 8) {
 		// ------------------------------------------------------------ MMAs
 		const uint32_t idesc_qk = at_idesc(AT_TC_KT, 0), idesc_pv = at_idesc(256, 1);
-		// the three term products (A term, B term)
-		constexpr int ta[3] = {0, 0, 1}, tb[3] = {0, 1, 0};
+		// the six term products (A term, B term)
+		constexpr int ta[6] = {0, 0, 1, 1, 0, 2}, tb[6] = {0, 1, 0, 1, 2, 0};
 		int cap = TC_SPIN_CAP, st = 0;
 		uint32_t ph = 0;
 		const uint32_t pb = smem_u32(pbuf);
-		tc_wait_cap(&q_bar, 0, cap);
 		for (int g = 0; g < total; g++) {
 			const Blk b = blk(g);
 			if (!b.qk && b.i == 0) tc_wait_cap(&p_bar, b.tile & 1, cap);  // P written, O rescaled
 			tc_wait_cap(&full_bar[st], ph, cap);
 			tc_fence_after();
-			const uint32_t base = smem_u32(ring + size_t(st) * AT_TC_STAGE);
+			const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
 			if (b.qk) {
 				const uint32_t d_s = tmem_s + uint32_t((b.tile & 1) * AT_TC_KT);
-				const uint64_t dq = tc_smem_desc(smem_u32(qbuf) + 2 * b.i * TC_TILE_BYTES), dk = tc_smem_desc(base);
+				const uint64_t dq = tc_smem_desc(base), dk = tc_smem_desc(base + 3 * TC_TILE_BYTES);
 				if (tc_elect()) {
 #pragma unroll
-					for (int h = 0; h < 2; h++)
+					for (int c = 0; c < 6; c++)
 #pragma unroll
-						for (int c = 0; c < 3; c++)
-#pragma unroll
-							for (int j2 = 0; j2 < 2; j2++)
-								tc_mma(d_s, dq + uint64_t(((8 * ta[c] + h) * TC_TILE_BYTES + j2 * 256) >> 4),
-								       dk + uint64_t(((2 * tb[c] + h) * (TC_TILE_BYTES / 2) + j2 * 256) >> 4), idesc_qk, (b.i > 0 || h > 0 || c > 0 || j2 > 0) ? 1u : 0u);
+						for (int j2 = 0; j2 < 2; j2++)
+							tc_mma(d_s, dq + uint64_t((ta[c] * TC_TILE_BYTES + j2 * 256) >> 4), dk + uint64_t((tb[c] * (TC_TILE_BYTES / 2) + j2 * 256) >> 4),
+							       idesc_qk, (b.i > 0 || c > 0 || j2 > 0) ? 1u : 0u);
 					tc_commit(&free_bar[st]);
-					if (b.i == 3) tc_commit(&s_bar[b.tile & 1]);
+					if (b.i == 7) tc_commit(&s_bar[b.tile & 1]);
 				}
 			} else {
 				const int vb = b.i;  // keys 16 vb ..: K-step vb % 2 of P's 32-key block vb / 2
 				const uint64_t dp = tc_smem_desc(pb + (vb >> 1) * TC_TILE_BYTES + (vb & 1) * 256), dv = at_vdesc(base);
 				if (tc_elect()) {
 #pragma unroll
-					for (int c = 0; c < 3; c++)
+					for (int c = 0; c < 6; c++)
 						tc_mma(tmem_o, dp + uint64_t((ta[c] * 2 * TC_TILE_BYTES) >> 4), dv + uint64_t((tb[c] * AT_TC_VBYTES) >> 4), idesc_pv,
 						       (b.tile > 0 || vb > 0 || c > 0) ? 1u : 0u);
 					tc_commit(&free_bar[st]);
@@ -375,8 +312,6 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		const bool row_ok = qi < a.S;
 		const int k_min = a.is_local ? max(0, qi - a.window) : 0;
 		const uint32_t lane_base = uint32_t(qd * 32) << 16;
-		// S is scaled back (and by 1 / sqrt(256)): powers of two
-		const float s_back = 0.0625f / (attn_tc_row_scale(a.rmsq) * attn_tc_row_scale(a.rmsk));
 		float m = -INFINITY, l = 0.0f;             // max in use (the same in both threads of a row), sum over this thread's keys
 		bool ok = true;
 		for (int jt = 0; jt < ntiles && ok; jt++) {
@@ -392,7 +327,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			if (all_vis) {
 #pragma unroll
 				for (int c = 0; c < 32; c++) {
-					const float x = __uint_as_float(sv[c]) * s_back;
+					const float x = __uint_as_float(sv[c]) * 0.0625f;  // 1 / sqrt(256), exact
 					sv[c] = __float_as_uint(x);
 					mt = fmaxf(mt, x);
 				}
@@ -401,7 +336,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 				for (int c = 0; c < 32; c++) {
 					const int key = kbase + c;
 					const bool vis = row_ok && key <= qi && key >= k_min;
-					const float x = vis ? __uint_as_float(sv[c]) * s_back : -INFINITY;
+					const float x = vis ? __uint_as_float(sv[c]) * 0.0625f : -INFINITY;
 					sv[c] = __float_as_uint(x);
 					mt = fmaxf(mt, x);
 				}
@@ -416,15 +351,24 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			const float mn = (mt > m + 8.0f || m == -INFINITY) ? fmaxf(m, mt) : m;
 			const bool none = mn == -INFINITY;            // no visible key so far
 			const float corr = none ? 1.0f : expf(m - mn);  // exp(-inf) = 0 at the row's first visible tile; 1 when the max stays
-			// probabilities and their two fp16 terms
+			// probabilities and their three bf16 terms by truncation (p >= 0; hi + mid + lo = p exactly: 8 + 8 + 8 bits)
 			float sum = 0.0f;
-			uint32_t ph[16], pl[16];  // fp16 pairs
+			uint32_t ph[16], pm[16], pl[16];  // bf16 pairs
 #pragma unroll
 			for (int c = 0; c < 32; c += 2) {
-				const float p0 = none ? 0.0f : expf(__uint_as_float(sv[c]) - mn), p1 = none ? 0.0f : expf(__uint_as_float(sv[c + 1]) - mn);  // exp(-inf) = 0 for masked keys
-				sum += p0;
-				sum += p1;
-				attn_tc_split(p0 * AT_TC_PSCALE, p1 * AT_TC_PSCALE, ph[c / 2], pl[c / 2]);
+				uint32_t hb[2], mb[2], lb[2];
+#pragma unroll
+				for (int u = 0; u < 2; u++) {
+					const float pv = none ? 0.0f : expf(__uint_as_float(sv[c + u]) - mn);  // exp(-inf) = 0 for masked keys
+					sum += pv;
+					hb[u] = __float_as_uint(pv) & 0xFFFF0000u;
+					const float r1 = pv - __uint_as_float(hb[u]);
+					mb[u] = __float_as_uint(r1) & 0xFFFF0000u;
+					lb[u] = __float_as_uint(r1 - __uint_as_float(mb[u]));  // at most 8 significant bits: exact in bf16
+				}
+				ph[c / 2] = __byte_perm(hb[0], hb[1], 0x7632);
+				pm[c / 2] = __byte_perm(mb[0], mb[1], 0x7632);
+				pl[c / 2] = __byte_perm(lb[0], lb[1], 0x7632);
 			}
 			l = fmaf(l, corr, sum);
 			m = mn;
@@ -436,7 +380,8 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			for (int k8 = 0; k8 < 4; k8++) {
 				uint8_t *dst = pbuf + hf * TC_TILE_BYTES + (r >> 3) * 512 + k8 * 128 + (r & 7) * 16;
 				*reinterpret_cast<uint4 *>(dst) = make_uint4(ph[4 * k8], ph[4 * k8 + 1], ph[4 * k8 + 2], ph[4 * k8 + 3]);
-				*reinterpret_cast<uint4 *>(dst + 2 * TC_TILE_BYTES) = make_uint4(pl[4 * k8], pl[4 * k8 + 1], pl[4 * k8 + 2], pl[4 * k8 + 3]);
+				*reinterpret_cast<uint4 *>(dst + 2 * TC_TILE_BYTES) = make_uint4(pm[4 * k8], pm[4 * k8 + 1], pm[4 * k8 + 2], pm[4 * k8 + 3]);
+				*reinterpret_cast<uint4 *>(dst + 4 * TC_TILE_BYTES) = make_uint4(pl[4 * k8], pl[4 * k8 + 1], pl[4 * k8 + 2], pl[4 * k8 + 3]);
 			}
 			// O = corr * O: this thread's half of the row's 256 columns
 			if (jt > 0 && !__all_sync(0xffffffffu, corr == 1.0f)) {
@@ -459,11 +404,10 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		// ------------------------------------------------------------ epilogue: o = O / l
 		if (ok && at_wait(&o_bar, 0, a.err, fail)) {
 			tc_fence_after();
-			pdl_wait();  // (vmax; long satisfied)
 			float l_other = 0.0f;  // (the partner is past its last read of slot 0: it arrived at p_bar, which o_bar follows)
 			const bool got = at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, &l_other, a.err, fail);
 			const float lt = l + l_other;
-			const float inv = (row_ok && got) ? 1.0f / (lt * (AT_TC_PSCALE * attn_tc_scale(__uint_as_float(a.vmax[blockIdx.y])))) : 0.0f;  // (a visible key always exists: the query itself)
+			const float inv = (row_ok && got) ? 1.0f / lt : 0.0f;  // (a visible key always exists: the query itself)
 			float *orow = a.o + (size_t(blockIdx.y) * a.S * 4 + size_t(tile) * 128 + r) * 256;
 #pragma unroll 1
 			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {

@@ -183,7 +183,6 @@ struct RopeArgs {
 	const float *sq, *sk, *sv;
 	int rows;
 	size_t cache_stride;
-	unsigned *vmax;  // per prompt the largest |v|, as bits (null: nobody asks)
 };
 __global__ void __launch_bounds__(192) qk_norm_rope_prefill_kernel(RopeArgs a) {
 	const int s = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -258,11 +257,6 @@ __global__ void __launch_bounds__(192) qk_norm_rope_prefill_kernel(RopeArgs a) {
 	}
 	x[lane] = lo;
 	x[32 + lane] = hi;
-	if (warp == 5 && a.vmax) {
-		const unsigned m = warp_umax(max(max(max(i8_abs_bits(lo.x), i8_abs_bits(lo.y)), max(i8_abs_bits(lo.z), i8_abs_bits(lo.w))),
-		                                 max(max(i8_abs_bits(hi.x), i8_abs_bits(hi.y)), max(i8_abs_bits(hi.z), i8_abs_bits(hi.w)))));
-		if (lane == 0 && m > *static_cast<volatile unsigned *>(a.vmax + blockIdx.y)) atomicMax(a.vmax + blockIdx.y, m);
-	}
 	if (warp >= 4 && s >= a.cache_from) {
 		float4 *c = reinterpret_cast<float4 *>((warp == 4 ? a.kcache : a.vcache) + blockIdx.y * a.cache_stride + size_t((s + a.slot_off) % a.slots) * 256);
 		c[lane] = lo;

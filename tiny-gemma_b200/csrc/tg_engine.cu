@@ -1589,17 +1589,16 @@ float *i8_rowscale(const TcScratch &sc, int M, int K) { return reinterpret_cast<
 struct AttnTcPlan {
 	int q_tiles, k_tiles, v_blocks;
 	size_t q_bytes, k_bytes, v_bytes;
-	static constexpr int MAX_WORDS = 64;  // a prompt's largest |v| per layer
-	size_t total() const { return q_bytes + k_bytes + v_bytes + MAX_WORDS * 4; }
+	size_t total() const { return q_bytes + k_bytes + v_bytes; }
 };
 AttnTcPlan attn_tc_plan(int S) {
 	AttnTcPlan p;
 	p.q_tiles = (4 * S + TC_BM - 1) / TC_BM;
 	p.k_tiles = (S + TC_BM - 1) / TC_BM;
 	p.v_blocks = 4 * ((S + AT_TC_KT - 1) / AT_TC_KT);  // 16 keys each
-	p.q_bytes = size_t(2) * p.q_tiles * 8 * TC_TILE_BYTES;
-	p.k_bytes = size_t(2) * p.k_tiles * 8 * TC_TILE_BYTES;
-	p.v_bytes = size_t(2) * p.v_blocks * AT_TC_VBYTES;
+	p.q_bytes = size_t(3) * p.q_tiles * 8 * TC_TILE_BYTES;
+	p.k_bytes = size_t(3) * p.k_tiles * 8 * TC_TILE_BYTES;
+	p.v_bytes = size_t(3) * p.v_blocks * AT_TC_VBYTES;
 	return p;
 }
 
@@ -2062,17 +2061,14 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 	// 2.40, 4080 3.82 / 3.53; of 61 tokens 1464 rows 1.79 / 1.83, 2196 2.48 / 2.35; of 8 tokens 8192 rows 7.7 / 9.5.
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
 	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", 960) + (at_rows > S_seq ? 16384 / S_seq : 0);
-	const bool attn_tc = use_tc && pos0 < 0 && c.n_layers <= AttnTcPlan::MAX_WORDS && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
-	__half *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
-	unsigned *at_vmax = nullptr;  // [layer][prompt]
+	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
+	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
-		at_q = reinterpret_cast<__half *>(p);
-		at_k = reinterpret_cast<__half *>(reinterpret_cast<uint8_t *>(p) + atp.q_bytes * nb);
-		at_v = reinterpret_cast<__half *>(reinterpret_cast<uint8_t *>(p) + (atp.q_bytes + atp.k_bytes) * nb);
-		at_vmax = reinterpret_cast<unsigned *>(reinterpret_cast<uint8_t *>(p) + (atp.q_bytes + atp.k_bytes + atp.v_bytes) * nb);
+		at_q = reinterpret_cast<__nv_bfloat16 *>(p);
+		at_k = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + atp.q_bytes * nb);
+		at_v = reinterpret_cast<__nv_bfloat16 *>(reinterpret_cast<uint8_t *>(p) + (atp.q_bytes + atp.k_bytes) * nb);
 		p += (atp.total() * nb + 3) / 4;
-		TG_CUDA(cudaMemsetAsync(at_vmax, 0, size_t(c.n_layers) * nb * 4, st));
 	}
 	float *part = p;
 	size_t part_floats = s->pf_floats - size_t(part - s->pf);
@@ -2161,7 +2157,6 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		ra.sv = w.V.s;
 		ra.rows = S;
 		ra.cache_stride = size_t(slots) * AT_HD;
-		ra.vmax = attn_tc ? at_vmax + size_t(l) * nb : nullptr;
 		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
 		count_launch();
 		const bool attn_small = !attn_tc && (pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 960));  // short prompts: two queries per CTA
@@ -2182,24 +2177,21 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 				TG_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_TC_SMEM));
 				at_configured[dev] = true;
 			}
-			auto pack_rows = [&](const float *src, const float *norm, __half *dst, int rows, int tiles) {
+			auto pack_rows = [&](const float *src, __nv_bfloat16 *dst, int rows, int tiles) {
 				const size_t chunks = size_t(tiles) * TC_BM * (256 / 8);
-				launch_k(attn_pack_rows_kernel, dim3(unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0, st, src, norm, dst,
-				         rows, tiles);
+				launch_k(split_pack_kernel, dim3(unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0, st, src, dst, rows,
+				         256, tiles);
 				count_launch();
 			};
-			pack_rows(q, w.rmsq, at_q, 4 * S_seq, atp.q_tiles);  // rows = (query, head) pairs as they lie in q [S][4][256]
-			pack_rows(k, w.rmsk, at_k, S_seq, atp.k_tiles);
+			pack_rows(q, at_q, 4 * S_seq, atp.q_tiles);  // rows = (query, head) pairs as they lie in q [S][4][256]
+			pack_rows(k, at_k, S_seq, atp.k_tiles);
 			launch_k(attn_pack_v_kernel, dim3(unsigned(std::min<size_t>((size_t(atp.v_blocks) * 512 + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0,
-			         st, (const float *)v, (const unsigned *)ra.vmax, at_v, S_seq, atp.v_blocks);
+			         st, (const float *)v, at_v, S_seq, atp.v_blocks);
 			count_launch();
 			AttnTcArgs aa{};
 			aa.qp = at_q;
 			aa.kp = at_k;
 			aa.vp = at_v;
-			aa.vmax = ra.vmax;
-			aa.rmsq = w.rmsq;
-			aa.rmsk = w.rmsk;
 			aa.o = ao;
 			aa.S = S_seq;
 			aa.q_tiles = atp.q_tiles;
