@@ -37,7 +37,8 @@ def test_shared_keys(capi, synth, weights_270m, monkeypatch, ctx, S):
     assert np.all(np.isfinite(got[0]))
 
 
-@pytest.mark.parametrize("n,S", [(1, 672), (1, 673), (4, 170), (5, 150), (5, 151), (20, 61), (21, 61)])  # rows 672; 420 + 50000 / S
+@pytest.mark.parametrize("n,S", [(1, 672), (1, 673), (4, 170), (5, 150), (5, 151), (20, 61), (21, 61),
+                                 (1, 832), (1, 833), (4, 177), (4, 178), (22, 61)])  # rows 832; 400 + 55000 / S
 def test_line_between_the_kernels(capi, synth, weights_270m, monkeypatch, n, S):
     """Prompts and groups on both sides of the line between the attention kernels, against the short-prompt kernel."""
     m = capi.Model("270m").load_file(weights_270m)

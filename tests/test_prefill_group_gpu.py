@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,S", [(2, 479), (2, 481), (31, 31), (31, 33), (5, 193), (13, 95), (2, 961), (256, 4),
-                                 (123, 16), (128, 16), (300, 15), (45, 33), (47, 33), (970, 1)])  # a group's line: 960 + 16384 / S rows, S >= 16
+                                 (123, 16), (128, 16), (300, 15), (45, 33), (47, 33), (970, 1),
+                                 (239, 16), (240, 16), (62, 33), (63, 33)])  # a group's line: 400 + 55000 / S rows, S >= 16
 def test_group_is_each_prompt(capi, synth, weights_270m, n, S):
     m = capi.Model("270m").load_file(weights_270m)
     m.build_tables(1 << 20)

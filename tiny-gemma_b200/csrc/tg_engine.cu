@@ -2051,16 +2051,15 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		tc.err = s->err_flag;
 		p += (tc.x_bytes + 3) / 4;
 	}
-	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 960 tokens, and for a group of
-	// equal prompts of 16 and more tokens each that has more than 960 + 16384 / S of them in all. Otherwise the CUDA-core kernel
+	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 832 tokens, and for a group of
+	// equal prompts of 16 and more tokens each that has more than 400 + 55000 / S of them in all. Otherwise the CUDA-core kernel
 	// with two queries per CTA is faster: its CTAs are more, and a prompt fills no tiles of 32 queries and 64 keys, as which the
-	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill of the 1B model in ms: one prompt of
-	// 450 tokens 2.9 / 3.6, of 832 4.93 / 5.04; groups of 976 rows of 8 tokens 3.77 / 4.20, of 61 3.81 / 3.97 (1464: 5.27 / 5.31), of 178
-	// 890 rows 3.90 / 4.09, 1424 5.51 / 5.24; of 16 tokens 976 rows 3.66 / 3.99, 2192 7.61 / 7.03 to 7.70, 16384 51.9 / 52.0; of 8 tokens
-	// 8192 rows 27.0 / 28.8, of 2 tokens 1500 rows 5.7 / 9.0; of 178 tokens 16376 rows 57.2 / 49.8. 270m: of 30 tokens 2190 rows 2.36 /
-	// 2.40, 4080 3.82 / 3.53; of 61 tokens 1464 rows 1.79 / 1.83, 2196 2.48 / 2.35; of 8 tokens 8192 rows 7.7 / 9.5.
+	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill in ms, 1B and 270m: one prompt of 700 tokens
+	// 4.03 / 4.45 and 1.99 / 2.28, of 832 4.73 / 4.76 and 2.37 / 2.38, of 960 5.46 / 5.14 and 2.81 / 2.58; groups of 178 tokens: 712 rows 3.59 / 3.51
+	// and 1.69 / 1.64, 1424 6.09 / 5.00 and 2.65 / 1.96; of 61: 976 rows 3.70 / 3.83 and 1.59 / 1.70, 1464 4.86 / 4.79 and 1.80 / 1.79; of 30: 2100 rows
+	// 6.58 / 6.90 and 2.29 / 2.30, 3600 10.4 / 10.7 and 3.35 / 3.04; of 16: 2048 rows 6.17 / 6.37 and 2.23 / 2.32, 2880 9.01 / 9.81 and 2.79 / 2.97.
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
-	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", 960) + (at_rows > S_seq ? 16384 / S_seq : 0);
+	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", at_rows > S_seq ? 400 + 55000 / S_seq : 832);
 	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
@@ -2159,7 +2158,9 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		ra.cache_stride = size_t(slots) * AT_HD;
 		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
 		count_launch();
-		const bool attn_small = !attn_tc && (pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 960));  // short prompts: two queries per CTA
+		// Two queries per CTA: what the tensor cores do not take. The 960 decides between the CUDA-core kernels where the tensor cores are
+		// switched off (prefill of 1400 tokens, two queries per CTA / long-prompt kernel, 1B and 270m: 7.9 / 9.0 and 4.0 / 4.8 ms, 2000: 11.6 / 11.2 and 6.0 / 5.8).
+		const bool attn_small = !attn_tc && (pos0 >= 0 || S_seq <= env_int("TG_ATTN_SMALL_MAX", 960));
 		if (attn_small) {
 			static bool as_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
