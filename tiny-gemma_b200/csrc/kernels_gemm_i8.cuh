@@ -38,6 +38,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "gemm_i8_tiles.h"  // plan, tile walk
 #include "kernels_tc.cuh"   // tcgen05 / bulk-copy helpers
 #include "tg_common.cuh"
@@ -540,8 +542,16 @@ struct GemmI8Args : I8Walk {
 	unsigned long long *top1;  // non-null (nsplit == 1): no C; per token the largest scaled value and its column, as a key
 	int top1_col0;
 	int *err;
-	GeluLut lut;  // GLU
 };
+// The table's 24 bytes are arguments of the kernel alone that looks up: with 760 bytes of arguments (four tensor maps in front) instead of
+// 736 a launch outside a graph took 0.5 to 0.9 us longer (as a call, 77 x 1152 x 6912 19.9 us instead of 19.0, 1500 x 1152 x 1024 23.4
+// instead of 22.7; with 888 bytes as with 760).
+struct GemmI8GluArgs : GemmI8Args {
+	GeluLut lut;
+};
+enum I8Epilogue { I8_SUMS, I8_GLU, I8_TOP1 };  // finished values or raw sums; the product of up and gate; a key per token
+template <I8Epilogue EPI> using I8KernelArgs = std::conditional_t<EPI == I8_GLU, GemmI8GluArgs, GemmI8Args>;
+static_assert(4 * sizeof(CUtensorMap) + sizeof(GemmI8Args) <= 736, "see GemmI8GluArgs");
 
 // W tile [128 k][128 n], 128-byte swizzle: MN-major operand; 1 KiB from one group of 8 k-rows to the next
 __device__ __forceinline__ uint64_t i8_desc_w(uint32_t addr) {
@@ -601,15 +611,16 @@ __device__ __forceinline__ void i8_cluster_sync() {
 // epilogue bounds it: with a branch per look-up it took 215 us, and with the table index in a loop of its own as well (GeluLut::index) 250.
 // What the epilogue does is a parameter of the kernel, not of the launch: with the code of the others beside it
 // a prompt of 178 tokens took 1.79 ms instead of 1.76 (156 registers instead of 140, and more code to fetch).
-enum I8Epilogue { I8_SUMS, I8_GLU, I8_TOP1 };  // finished values or raw sums; the product of up and gate; a key per token
 template <int CG, I8Epilogue EPI>
 __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
                                                                  const __grid_constant__ CUtensorMap wmap1,
                                                                  const __grid_constant__ CUtensorMap wmap2,
-                                                                 const __grid_constant__ CUtensorMap xmap, GemmI8Args a) {
+                                                                 const __grid_constant__ CUtensorMap xmap, I8KernelArgs<EPI> a) {
 	using SH = I8Shape<CG>;
 	constexpr int NST = SH::NST;
 	constexpr bool GLU = EPI == I8_GLU, TOP1 = EPI == I8_TOP1;
+	GeluLut lut{};
+	if constexpr (GLU) lut = a.lut;
 	pdl_trigger();
 	extern __shared__ uint8_t i8_smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(i8_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -631,8 +642,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		if (GLU) t.grp = n & 1;
 		return t;
 	};
-	if (GLU && a.lut.size <= GE_LUT)
-		for (int i = tid; i < a.lut.size; i += I8_THREADS) table[i] = a.lut.table[i];
+	if (GLU && lut.size <= GE_LUT)
+		for (int i = tid; i < lut.size; i += I8_THREADS) table[i] = lut.table[i];
 	if (tid == 0) {
 		for (int s = 0; s < NST; s++) {
 			mbar_init(&full_bar[s], 1);
@@ -761,8 +772,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		pdl_wait();  // the row scales are the predecessor's output, and C may be its input
 		const int quad = warp & 3, sub = (warp - 2) >> 2;  // TMEM lanes 32 * quad ..; two warps share them
 		const bool fin = a.nsplit.d == 1 && !a.raw;
-		const float *const lut_values = GLU && a.lut.size <= GE_LUT ? table : a.lut.table;
-		const float lut_base = -(a.lut.mn * a.lut.inv);
+		const float *const lut_values = GLU && lut.size <= GE_LUT ? table : lut.table;
+		const float lut_base = -(lut.mn * lut.inv);
 		float kept[GLU ? 32 : 1];  // GLU: the up values of the tile before
 		for (int it = 0; has_tile(it); it++) {
 			const I8Tile t = tile(it);
@@ -805,18 +816,18 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 					}
 					// GeluLut::index, eight at a time and selected instead of branched on (int(x) >= 0 is x > -1)
 					float x[8], y[8];
-					if (a.lut.inv != 0.0f) {
+					if (lut.inv != 0.0f) {
 #pragma unroll
-						for (int i = 0; i < 8; i++) x[i] = fmaf(v[i], a.lut.inv, lut_base);
+						for (int i = 0; i < 8; i++) x[i] = fmaf(v[i], lut.inv, lut_base);
 					} else {
 #pragma unroll
-						for (int i = 0; i < 8; i++) x[i] = (v[i] - a.lut.mn) / a.lut.eps;
+						for (int i = 0; i < 8; i++) x[i] = (v[i] - lut.mn) / lut.eps;
 					}
 #pragma unroll
-					for (int i = 0; i < 8; i++) y[i] = lut_values[min(max(int(x[i]), 0), a.lut.size - 1)];
+					for (int i = 0; i < 8; i++) y[i] = lut_values[min(max(int(x[i]), 0), lut.size - 1)];
 #pragma unroll
 					for (int i = 0; i < 8; i++) {
-						const float in = int(x[i]) < a.lut.size ? y[i] : v[i];
+						const float in = int(x[i]) < lut.size ? y[i] : v[i];
 						v[i] = (x[i] > -1.0f && x[i] < 2147483648.0f ? in : 0.0f) * kept[keep() + i];
 					}
 				} else if constexpr (TOP1) {

@@ -1816,7 +1816,7 @@ int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const
 		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
 		configured[dev] = true;
 	}
-	GemmI8Args a{};
+	GemmI8GluArgs a{};
 	i8_fill_walk(a, pl, M, K, 1, cols);
 	CUtensorMap wmap[2], xmap;
 	const QW *ws[2] = {&U, &G};
