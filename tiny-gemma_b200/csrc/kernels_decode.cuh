@@ -460,13 +460,17 @@ __global__ void __launch_bounds__(MVC_THREADS, 1) qmatvec_cluster_kernel(float *
 // =========================================================== wide matvec (one sequence, the vocabulary matrix)
 // y[n] = scale[n] * sum_k x[k] W[k,n] for a matrix of hundreds of MB: HBM bound. One CTA per SM owns `groups` groups of
 // 16 consecutive columns (262144 columns over 148 SMs: 112 groups, 1792 contiguous bytes of every row, whole lines) in
-// four row sets. A thread copies its own 16-byte pieces into a ring of three stages of eight rows in shared memory (cp.async, no
-// barrier: it reads nobody else's) and works on one stage with the next two on their way, 114 KB per SM. 1152 x 262144: 59.5 us with
-// the next eight loads in registers (57 KB) and 111 groups, whose pieces of a row began anywhere in a line; 58.9 with whole lines alone, 59.9 with
-// the ring alone, 54.9 with both (5.5 TB/s; a copy into rings of 147 KB that multiplies nothing: 49).
-constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8, MVW_STAGES = 3;
-__device__ __forceinline__ void mvw_copy(uint32_t dst, const int8_t *src) {
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// four row sets. A thread copies its own 16-byte pieces into a ring of two stages of eight rows in shared memory (cp.async, no
+// barrier: it reads nobody else's) and works on one stage with the next on its way, 57 KB per SM. The copies are marked evict-first in
+// the L2: nothing is read twice, and at normal priority they push out the dirty lines that earlier kernels left there, whose way to
+// DRAM then goes with the reads (126 MB behind a kernel that wrote as much: a third of the launch).
+// 1152 x 262144 in us (twelve matrices in turn / one matrix again after a pause / the same after 400 MB were written / operands just made):
+// loads into registers 56.3 / 64 / 69 / 67; three stages at normal priority 54.6 / 62 / 76 / 77; three stages evict-first - / 60 / 67 / 63; two
+// stages evict-first 50.4 / 56 / 63 / 60 (6.0 TB/s; 48.7 for one matrix back to back, of which the L2 keeps a part). Groups of 111, whose pieces of a
+// row begin anywhere in a line, took 59.9 where 112 took 54.9; single FMAs instead of paired ones take 52.0 instead of 50.4.
+constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8, MVW_STAGES = 2;
+__device__ __forceinline__ void mvw_copy(uint32_t dst, const int8_t *src, uint64_t policy) {
+	asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
 }
 // a += (b - (2^23 + 128)) * c, both halves: b holds the bits of 2^23 + 128 + a weight (exact, see i8_lane_to_f32)
 __device__ __forceinline__ void mvw_fma2(float2 &a, uint32_t b0, uint32_t b1, float c) {
@@ -477,7 +481,7 @@ __device__ __forceinline__ void mvw_fma2(float2 &a, uint32_t b0, uint32_t b1, fl
 }
 __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kernel(float *y, const float *x, const int8_t *w, const float *scales,
                                                                                    int K, int N, int groups) {
-	extern __shared__ __align__(16) float mvw_smem[];  // x [K], the ring [3][8][threads] of 16 bytes; the row sets' sums [4][groups * 16] in its place
+	extern __shared__ __align__(16) float mvw_smem[];  // x [K], the ring [2][8][threads] of 16 bytes; the row sets' sums [4][groups * 16] in its place
 	pdl_trigger();
 	pdl_wait();
 	float *xs = mvw_smem;
@@ -489,11 +493,13 @@ __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kern
 	const size_t step = size_t(MVW_SETS) * N;
 	const int n = on ? K / MVW_SETS : 0;  // K is a multiple of 4 * MVW_U
 	const uint32_t ring = uint32_t(__cvta_generic_to_shared(xs + K)) + 16u * tid;
+	uint64_t policy;
+	asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
 	int next = 0;  // rows requested so far
 	auto request = [&](int st) {
 		if (next < n) {
 #pragma unroll
-			for (int u = 0; u < MVW_U; u++) mvw_copy(ring + uint32_t((st * MVW_U + u) * nt) * 16u, p + u * step);
+			for (int u = 0; u < MVW_U; u++) mvw_copy(ring + uint32_t((st * MVW_U + u) * nt) * 16u, p + u * step, policy);
 			p += MVW_U * step;
 			next += MVW_U;
 		}
