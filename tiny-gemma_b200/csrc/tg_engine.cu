@@ -16,7 +16,8 @@
 #include <string>
 #include <vector>
 
-#include "../../include/tiny_gemma_b200.h"
+#include "tg_status.h"
+#include "host_ws.h"
 #include "kernels_decode.cuh"
 #include "kernels_mega.cuh"
 #include "kernels_persist.cuh"
@@ -38,19 +39,6 @@ int fail(int code, const std::string &msg) {
 	g_err = msg;
 	return code;
 }
-
-#define TG_CUDA(call)                                                                                   \
-	do {                                                                                                \
-		cudaError_t e__ = (call);                                                                       \
-		if (e__ != cudaSuccess)                                                                         \
-			return fail(TG_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e__));                 \
-	} while (0)
-
-#define TG_TRY(call)                \
-	do {                            \
-		int rc__ = (call);          \
-		if (rc__ != TG_OK) return rc__; \
-	} while (0)
 
 inline void count_launch(int n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
@@ -3311,127 +3299,36 @@ int tg_qgemm(float *c, const float *a, const int8_t *w, const float *scales, int
 }
 
 namespace {
-// What the samplers on host buffers work in: a stream, device memory and pinned staging, kept by the calling thread (so
-// no two threads share one) and given back when the thread ends. Allocating and freeing these per call took several
-// times the work itself. Kept up to HOST_WS_MAX bytes each; a larger call takes and frees its own.
-constexpr size_t HOST_WS_MAX = size_t(8) << 20;
-constexpr int HOST_WS_CHUNKS = 4;  // copies to and from the caller's pageable memory overlap the transfers in chunks
-struct HostWs {
-	cudaStream_t st = nullptr;
-	cudaEvent_t ev[HOST_WS_CHUNKS] = {};
-	uint8_t *dev = nullptr, *pin = nullptr;
-	size_t dev_bytes = 0, pin_bytes = 0;
-	void release() {
-		if (st) cudaStreamSynchronize(st);
-		for (cudaEvent_t &e : ev)
-			if (e) cudaEventDestroy(e);
-		cudaFree(dev);
-		cudaFreeHost(pin);
-		if (st) cudaStreamDestroy(st);
-		cudaGetLastError();
-		*this = HostWs();
-	}
-	int reserve(size_t d, size_t p) {
-		if (!st) {
-			TG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-			for (cudaEvent_t &e : ev) TG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-		}
-		if (d > dev_bytes) {
-			cudaFree(dev);
-			dev = nullptr;
-			dev_bytes = 0;
-			TG_CUDA(cudaMalloc(&dev, d));
-			dev_bytes = d;
-		}
-		if (p > pin_bytes) {
-			cudaFreeHost(pin);
-			pin = nullptr;
-			pin_bytes = 0;
-			TG_CUDA(cudaMallocHost(&pin, p));
-			pin_bytes = p;
-		}
-		return TG_OK;
-	}
-	// the caller's buffer -> dst (enqueued; the caller's memory has been read on return)
-	int upload(uint8_t *dst, const void *src, size_t bytes) {
-		const size_t ch = (bytes / HOST_WS_CHUNKS + 4095) & ~size_t(4095);
-		for (size_t o = 0; o < bytes; o += ch) {
-			const size_t n = std::min(ch, bytes - o);
-			std::memcpy(pin + o, static_cast<const uint8_t *>(src) + o, n);
-			TG_CUDA(cudaMemcpyAsync(dst + o, pin + o, n, cudaMemcpyHostToDevice, st));
-		}
-		return TG_OK;
-	}
-	// src -> the pinned buffer (enqueued), and from there into the caller's (complete on return)
-	int download(const uint8_t *src, size_t bytes) {
-		const size_t ch = (bytes / HOST_WS_CHUNKS + 4095) & ~size_t(4095);
-		int k = 0;
-		for (size_t o = 0; o < bytes; o += ch, k++) {
-			TG_CUDA(cudaMemcpyAsync(pin + o, src + o, std::min(ch, bytes - o), cudaMemcpyDeviceToHost, st));
-			TG_CUDA(cudaEventRecord(ev[k], st));
-		}
-		return TG_OK;
-	}
-	int deliver(void *dst, size_t bytes) {
-		const size_t ch = (bytes / HOST_WS_CHUNKS + 4095) & ~size_t(4095);
-		int k = 0;
-		for (size_t o = 0; o < bytes; o += ch, k++) {
-			TG_CUDA(cudaEventSynchronize(ev[k]));
-			std::memcpy(static_cast<uint8_t *>(dst) + o, pin + o, std::min(ch, bytes - o));
-		}
-		return TG_OK;
-	}
-	~HostWs() {
-		if (st || dev || pin) release();
-	}
-};
-
 // one row of n logits in host memory: arg-max, or min-p with the probabilities written back
 int sample_host_row(const float *in, float *out, int n, bool minp_mode, float minp, float temp, float randf, int *tok) {
 	TG_TRY(ensure_device(0));
 	static thread_local HostWs kept;
 	HostWs own;
-	const size_t row = size_t(n) * 4, row_up = (row + 255) & ~size_t(255), wsb = (SampScratch::bytes(1, n) + 255) & ~size_t(255);
-	const size_t dbytes = 256 + row_up + wsb;  // [token][uniform count][uniform] .. [key][ticket] ..., the row, the scratch
-	HostWs &w = dbytes > HOST_WS_MAX ? own : kept;
-	const bool fresh = dbytes > w.dev_bytes;
-	TG_TRY(w.reserve(dbytes, row_up + 256));
-	if (fresh) TG_CUDA(cudaMemsetAsync(w.dev, 0, 256, w.st));  // (the kernels leave key and ticket zero)
-	struct {
-		int tok, count;
-		float randf;
-	} up = {0, 0, randf};
-	uint8_t *pin_words = w.pin + row_up;
-	std::memcpy(pin_words, &up, sizeof up);
-	TG_CUDA(cudaMemcpyAsync(w.dev, pin_words, sizeof up, cudaMemcpyHostToDevice, w.st));
-	TG_TRY(w.upload(w.dev + 256, in, row));
+	const size_t row_up = (size_t(n) * 4 + 255) & ~size_t(255), scratch = (SampScratch::bytes(1, n) + 255) & ~size_t(255);
+	HostWs &ws = 256 + row_up + scratch > HOST_WS_MAX ? own : kept;
 	SampleArgs a{};
-	a.logits = reinterpret_cast<float *>(w.dev + 256);
-	a.V = n;
-	a.tok_out = reinterpret_cast<int *>(w.dev);
-	a.B = 1;
-	a.minp = minp;
-	a.temp = temp;
-	a.randf = reinterpret_cast<const float *>(w.dev + 8);
-	a.randf_count = reinterpret_cast<int *>(w.dev + 4);
-	a.randf_cap = 1;
-	SampScratch ws(w.dev + 256 + row_up, 1, n);
-	ws.keys = reinterpret_cast<unsigned long long *>(w.dev + 64);
-	ws.tickets = reinterpret_cast<unsigned *>(w.dev + 72);
-	if (minp_mode) {
-		// the probabilities are copied back before the walk for the token: it runs (28 us) while the host takes them out of the
-		// pinned buffer (~18 us less of 270 a call)
-		TG_TRY(launch_minp_head(a, ws, w.st));
-		TG_TRY(w.download(w.dev + 256, row));
-		TG_TRY(launch_minp_walk(a, ws.rows, w.st));
-	} else {
-		TG_TRY(launch_argmax_rows(a, ws, w.st));
-	}
-	TG_CUDA(cudaMemcpyAsync(pin_words, w.dev, 4, cudaMemcpyDeviceToHost, w.st));
-	if (minp_mode) TG_TRY(w.deliver(out, row));
-	TG_CUDA(cudaStreamSynchronize(w.st));
-	std::memcpy(tok, pin_words, 4);
-	return TG_OK;
+	auto place = [&](const HostWs &w, uint8_t *row) {
+		a.logits = reinterpret_cast<float *>(row);
+		a.V = n;
+		a.tok_out = reinterpret_cast<int *>(w.dev);
+		a.B = 1;
+		a.minp = minp;
+		a.temp = temp;
+		a.randf = reinterpret_cast<const float *>(w.dev + 8);
+		a.randf_count = reinterpret_cast<int *>(w.dev + 4);
+		a.randf_cap = 1;
+		SampScratch sc(row + row_up, 1, n);
+		sc.keys = reinterpret_cast<unsigned long long *>(w.dev + 64);
+		sc.tickets = reinterpret_cast<unsigned *>(w.dev + 72);
+		return sc;
+	};
+	return host_row(
+	    ws, in, minp_mode ? out : nullptr, n, scratch, randf, tok,
+	    [&](HostWs &w, uint8_t *row) { return launch_minp_head(a, place(w, row), w.st); },
+	    [&](HostWs &w, uint8_t *row) {
+		    const SampScratch sc = place(w, row);
+		    return minp_mode ? launch_minp_walk(a, sc.rows, w.st) : launch_argmax_rows(a, sc, w.st);
+	    });
 }
 }  // namespace
 
