@@ -883,7 +883,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 					finish(g + 2, rb, qb, sb, keep_b);
 				}
 			};
-			if constexpr (GLU) {  // (written out: what is kept has to stay in registers)
+			if constexpr (GLU) {  // (written out: what is kept is indexed by constants and stays in registers but for 24 bytes, at the limit of 168)
 				static_assert(I8_TG == 8, "two pairs of token groups per warp");
 				if (sub < ng) pair_of_groups(sub, [] { return 0; }, [] { return 8; });
 				if (sub + 4 < ng) pair_of_groups(sub + 4, [] { return 16; }, [] { return 24; });

@@ -1523,11 +1523,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) decode_persist_kernel(const __g
 			if (tid == 0 && cta == 0) atomicExch(a.err, 1);
 			tok = 0;
 		}
-		// Cache chunks per head of this token's attention. A warp holds two rows from before the poll for q|k|v, so a chunk takes
-		// a step for every 24 rows; phase C merges three chunks of a head at a time. The steps of both are dependent round
-		// trips, a merge is the shorter one: the multiple of 3 with the least 3 * steps + merges. (A fixed 8 up to 512
-		// rows, as before, against the rule: 411 / 406 us a token at 23 to 55 positions of the 270m model, 744 / 731 at 1500 of the
-		// 1B model.)
+		// Cache chunks per head of this token's attention: the multiple of 3 with the least 3 * steps + a third of the chunks. A warp holds two
+		// rows from before the poll for q|k|v, so a chunk takes a dependent step for every 24 rows; the merge in phase C requests four chunks per
+		// group of threads at once (12 a round trip with the 1B plan's three groups, 24 with the 270m plan's six), but every further chunk's CTA
+		// also publishes a row, so more chunks than rows ask for cost time: with 24 cached rows 3 chunks take 434 us a token and 24 take 459 (1B; 270m 267 and
+		// 273), with 210 12 take 441 and 24 455 (290 and 293). Behind 400 rows the price of a merge in the rule is too high: 24 chunks take 453 us
+		// where its 12 take 457 at 400 rows, 455 / 460 at 520 and 470 / 476 at 4096 positions (270m 277 / 281, 282 / 288, 301 / 307).
 		if (warp == 0) {
 			const bool loc = lane < 16;
 			const int n = min(3 * ((lane & 15) + 1), a.nch_max), v = loc ? min(pos + 1, a.slots_local) : min(pos + 1, a.slots_global);

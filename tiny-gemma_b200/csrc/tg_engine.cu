@@ -1856,7 +1856,7 @@ int batched_setup(tg_state *s) {
 int enqueue_decode_batched(tg_state *s, StepHead head) {
 	tg_model *m = s->m;
 	const tg_config &c = m->cfg;
-	const int B = s->B, D = c.hidden_size, I = c.intermediate_size, V = c.n_vocab;
+	const int B = s->B, D = c.hidden_size, V = c.n_vocab;
 	const int qd = c.n_head * c.head_dim;
 	cudaStream_t st = s->stream;
 	const GeluLut lut = make_lut(m);
