@@ -460,17 +460,29 @@ __global__ void __launch_bounds__(MVC_THREADS, 1) qmatvec_cluster_kernel(float *
 // =========================================================== wide matvec (one sequence, the vocabulary matrix)
 // y[n] = scale[n] * sum_k x[k] W[k,n] for a matrix of hundreds of MB: HBM bound. One CTA per SM owns `groups` groups of
 // 16 consecutive columns (262144 columns over 148 SMs: 112 groups, 1792 contiguous bytes of every row, whole lines) in
-// four row sets. A thread copies its own 16-byte pieces into a ring of two stages of eight rows in shared memory (cp.async, no
-// barrier: it reads nobody else's) and works on one stage with the next on its way, 57 KB per SM. The copies are marked evict-first in
-// the L2: nothing is read twice, and at normal priority they push out the dirty lines that earlier kernels left there, whose way to
-// DRAM then goes with the reads (126 MB behind a kernel that wrote as much: a third of the launch).
-// 1152 x 262144 in us (twelve matrices in turn / one matrix again after a pause / the same after 400 MB were written / operands just made):
-// loads into registers 56.3 / 64 / 69 / 67; three stages at normal priority 54.6 / 62 / 76 / 77; three stages evict-first - / 60 / 67 / 63; two
-// stages evict-first 50.4 / 56 / 63 / 60 (6.0 TB/s; 48.7 for one matrix back to back, of which the L2 keeps a part). Groups of 111, whose pieces of a
-// row begin anywhere in a line, took 59.9 where 112 took 54.9; single FMAs instead of paired ones take 52.0 instead of 50.4.
-constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8, MVW_STAGES = 2;
+// four row sets. A thread copies its own 16-byte pieces into a ring of stages of eight rows in shared memory (cp.async, no
+// barrier: it reads nobody else's) and works on one stage with the next on their way, 57 KB each per SM.
+// KEPT, a matrix that the L2 holds (of the accepted depths 256, 67 MB): three stages; such a launch is mostly its own start, and the next call finds
+// lines of it. Otherwise two stages, evict-first in the L2: nothing is read twice, and at normal priority the reads push out the dirty lines that
+// earlier kernels left there, whose way to DRAM then goes with them (126 MB behind a kernel that wrote as much: a third of the launch).
+// In us, several matrices in turn / one again after a pause / the same after 400 MB were written:
+//                                  256 x 262144            640 x 262144            1152 x 262144           2048 x 262144
+//     loads into registers         17.3 / 22.4 / 29.1      34.4 / 41.8 / 44.5      56.2 / 62.9 / 67.6      95.1 / 104 / 112
+//     3 stages, normal priority    17.1 / 20.6 / 29.2 (*)  33.5 / 39.8 / 49.0      54.8 / 60.3 / 75.4      92.7 / 99.7 / 117
+//     3 stages, evict-first        15.7 / 21.0 / 28.0      32.9 / 37.2 / 42.7      54.3 / 59.2 / 66.1      92.1 / 96.2 / 107
+//     2 stages, normal priority    20.4 / 20.7 / 29.0      31.6 / 38.0 / 46.2      50.7 / 56.8 / 71.9      83.5 / 90.6 / 112
+//     2 stages, evict-first        18.8 / 20.5 / 27.0      30.7 / 37.8 / 42.8      50.0 / 55.2 / 61.6      83.5 / 89.1 / 99.5
+// (*) 13.1 for one matrix back to back (evict-first 15.2). 50.0 us are 6.0 TB/s. First pass over 302 MB that were just made: 67, 77, 63 and, with two stages
+// evict-first, 60. Groups of 111, whose pieces of a row begin anywhere in a line, took 59.9 where 112 took 54.9; single FMAs instead of paired ones
+// 52.0 instead of 50.4.
+constexpr int MVW_SETS = 4, MVW_MAX_GROUPS = 128, MVW_U = 8;
+__host__ __device__ constexpr int mvw_stages(bool kept) { return kept ? 3 : 2; }
+template <bool KEPT>
 __device__ __forceinline__ void mvw_copy(uint32_t dst, const int8_t *src, uint64_t policy) {
-	asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
+	if constexpr (KEPT)
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+	else
+		asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy) : "memory");
 }
 // a += (b - (2^23 + 128)) * c, both halves: b holds the bits of 2^23 + 128 + a weight (exact, see i8_lane_to_f32)
 __device__ __forceinline__ void mvw_fma2(float2 &a, uint32_t b0, uint32_t b1, float c) {
@@ -479,9 +491,10 @@ __device__ __forceinline__ void mvw_fma2(float2 &a, uint32_t b0, uint32_t b1, fl
 	    : "+f"(a.x), "+f"(a.y)
 	    : "r"(b0), "r"(b1), "f"(c), "f"(-8388736.0f));
 }
+template <bool KEPT>
 __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kernel(float *y, const float *x, const int8_t *w, const float *scales,
                                                                                    int K, int N, int groups) {
-	extern __shared__ __align__(16) float mvw_smem[];  // x [K], the ring [2][8][threads] of 16 bytes; the row sets' sums [4][groups * 16] in its place
+	extern __shared__ __align__(16) float mvw_smem[];  // x [K], the ring [stages][8][threads] of 16 bytes; the row sets' sums [4][groups * 16] in its place
 	pdl_trigger();
 	pdl_wait();
 	float *xs = mvw_smem;
@@ -493,20 +506,21 @@ __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kern
 	const size_t step = size_t(MVW_SETS) * N;
 	const int n = on ? K / MVW_SETS : 0;  // K is a multiple of 4 * MVW_U
 	const uint32_t ring = uint32_t(__cvta_generic_to_shared(xs + K)) + 16u * tid;
-	uint64_t policy;
-	asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+	constexpr int STAGES = mvw_stages(KEPT);
+	uint64_t policy = 0;
+	if constexpr (!KEPT) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
 	int next = 0;  // rows requested so far
 	auto request = [&](int st) {
 		if (next < n) {
 #pragma unroll
-			for (int u = 0; u < MVW_U; u++) mvw_copy(ring + uint32_t((st * MVW_U + u) * nt) * 16u, p + u * step, policy);
+			for (int u = 0; u < MVW_U; u++) mvw_copy<KEPT>(ring + uint32_t((st * MVW_U + u) * nt) * 16u, p + u * step, policy);
 			p += MVW_U * step;
 			next += MVW_U;
 		}
 		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
 #pragma unroll
-	for (int st = 0; st < MVW_STAGES; st++) request(st);
+	for (int st = 0; st < STAGES; st++) request(st);
 	for (int k = tid; k < K; k += nt) xs[k] = x[k];
 	__syncthreads();
 	float2 acc[8];
@@ -515,7 +529,7 @@ __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kern
 	int st = 0;
 #pragma unroll 1
 	for (int it = 0; it < n; it += MVW_U) {
-		asm volatile("cp.async.wait_group %0;" ::"n"(MVW_STAGES - 1) : "memory");
+		asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
 #pragma unroll
 		for (int u = 0; u < MVW_U; u++) {
 			uint32_t words[4];
@@ -532,7 +546,7 @@ __global__ void __launch_bounds__(MVW_SETS *MVW_MAX_GROUPS, 1) qmatvec_wide_kern
 			}
 		}
 		request(st);
-		if (++st == MVW_STAGES) st = 0;
+		if (++st == STAGES) st = 0;
 	}
 	asm volatile("cp.async.wait_group 0;" ::: "memory");
 	__syncthreads();  // (the ring is done with everywhere)

@@ -3048,9 +3048,10 @@ int tg_dev_qmatvec(float *y, const float *x, const int8_t *w, const float *scale
 	static unsigned *tickets[64] = {nullptr};
 	int dev = 0;
 	TG_CUDA(cudaGetDevice(&dev));
-	static int sms_of[64] = {0};
+	static int sms_of[64] = {0}, l2_of[64] = {0};
 	if (!sms_of[dev]) {
 		int sms = 0;
+		if (cudaDeviceGetAttribute(&l2_of[dev], cudaDevAttrL2CacheSize, dev) != cudaSuccess) l2_of[dev] = 0;
 		if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) sms_of[dev] = sms;
 	}
 	if (sms_of[dev]) g_num_sms = sms_of[dev];
@@ -3059,13 +3060,17 @@ int tg_dev_qmatvec(float *y, const float *x, const int8_t *w, const float *scale
 	const int groups = ((N / 16 + g_num_sms - 1) / g_num_sms + 7) / 8 * 8;  // (whole 128-byte lines)
 	if (groups >= 64 && groups <= MVW_MAX_GROUPS && K % (MVW_SETS * MVW_U) == 0) {
 		const int nt = (MVW_SETS * groups + 31) / 32 * 32;
-		const size_t smem = size_t(K) * 4 + size_t(MVW_STAGES) * MVW_U * nt * 16;  // (the sums take less than the ring)
+		const bool kept = size_t(K) * N <= size_t(l2_of[dev]);
+		auto kernel = kept ? qmatvec_wide_kernel<true> : qmatvec_wide_kernel<false>;
+		const size_t smem = size_t(K) * 4 + size_t(mvw_stages(kept)) * MVW_U * nt * 16;  // (the sums take less than the ring)
 		static bool configured[64] = {false};
 		if (!configured[dev]) {
-			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6912 * 4 + MVW_STAGES * MVW_U * MVW_SETS * MVW_MAX_GROUPS * 16));
+			constexpr int stage = MVW_U * MVW_SETS * MVW_MAX_GROUPS * 16;
+			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2048 * 4 + mvw_stages(true) * stage));
+			TG_CUDA(cudaFuncSetAttribute(qmatvec_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6912 * 4 + mvw_stages(false) * stage));
 			configured[dev] = true;
 		}
-		launch_k(qmatvec_wide_kernel, dim3((N / 16 + groups - 1) / groups), dim3(nt), smem, (cudaStream_t)stream, y, x, w, scales, K, N, groups);
+		launch_k(kernel, dim3((N / 16 + groups - 1) / groups), dim3(nt), smem, (cudaStream_t)stream, y, x, w, scales, K, N, groups);
 		count_launch();
 		return check_launch("qmatvec_wide");
 	}
