@@ -4,85 +4,172 @@
 //
 // The four heads share one KV head, so the (query, head) pairs of 32 consecutive queries form a 128-row
 // operand: row r of tile t is query 32 t + r / 4, head r % 4 — the rows of q [S][4][256] as they lie.
-// One CTA owns a row tile and walks its keys in tiles of 64:
-//     S = Q K_j^T                    M128 x N64, contraction over the 256 head dimensions
+// One CTA owns a row tile and walks its keys in tiles of 128:
+//     S = Q K_j^T                    M128 x N128, contraction over the 256 head dimensions
 //     online softmax on S            (max in use m and sum l per row; a row = one TMEM lane, two threads)
-//     O = corr * O + P V_j           M128 x N256, contraction over the 64 keys
-// fp32 accuracy on bf16 tensor cores: every fp32 operand is split into three bf16 terms x = hi + mid + lo (kernels_tc.cuh:
-// all 24 bits, fp32's range) and a product a * b is the six term products whose weight reaches
+//     O = corr * O + P V_j           M128 x N256, contraction over the tile's keys
+// Only the keys that some row of the tile sees are worked on, in units of 16: the first tile of a window and the last one of
+// a row tile have a smaller N and fewer V blocks.
+// fp32 accuracy on bf16 tensor cores: every fp32 operand is split into three bf16 terms x = hi + mid + lo (all 24 bits, fp32's
+// range) and a product a * b is the six term products whose weight reaches
 // 2^-24 (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi), all accumulated in fp32 in TMEM.
-// Two fp16 terms and three products take less time (16384 tokens of the 1B model 59 ms instead of 66), but they hold 22 to 23 bits of an
+// Two fp16 terms and three products take less time, but they hold 22 to 23 bits of an
 // operand inside fp16's range only, so v would need a scale from keys that a row may not see: its bits, and whether it is finite,
 // would hang on later tokens.
 //
 // Operands are packed once per layer in the tensor core's shared-memory layouts (no swizzle, 8 x 8 core
-// matrices), so that the CTA fetches them with plain bulk copies:
-//     Q, K: split_pack_kernel ([3 terms][128-row tiles][8 blocks of 32 dimensions][8 KiB], K-major; a 64-key
-//           tile is one half of a 128-row tile)
-//     V:    attn_pack_v_kernel ([3 terms][16-key blocks][8 KiB], N-major like the GEMM's weight operand)
+// matrices), by the kernel that finishes the projections (attn_qkv_pack_kernel), so that the CTA fetches them with plain bulk copies:
+//     Q, K: [3 terms][128-row tiles][16 blocks of 16 dimensions][4 KiB], K-major
+//     V:    [3 terms][16-key blocks][8 KiB], N-major
 // Warps 0-7: softmax and epilogue (two threads per row: warps w and w + 4 share the TMEM lanes 32 (w % 4) ..
 // and take half of a tile's keys each); warp 8: one thread issues the MMAs; warp 9: one thread issues the bulk
-// copies, up to four ring blocks ahead of the MMAs.
-// Per key tile the ring carries eight Q|K blocks (one per 32 dimensions) and four V blocks (16 keys each).
+// copies, up to five ring blocks ahead of the MMAs.
+// Per key tile the ring carries 16 Q|K blocks (16 dimensions each) and up to eight V blocks (16 keys each), 24 KiB apiece: Q does
+// not fit beside P and the ring and is fetched again for every key tile.
+// The tensor pipe bounds it. An MMA of N = 64 takes 48 clk for 32 clk of products, because its 128 rows of A are
+// read from shared memory all the same; of N = 128 it takes 64 for 64.
 // S is double-buffered in TMEM and the MMAs are issued as Q K_0^T, Q K_1^T, P V_0, Q K_2^T, P V_1, ...: while the
 // softmax warps work on tile t the tensor core runs Q K_{t+1}^T and P V_{t-1}. The running max is only moved (and
 // O rescaled, a TMEM round trip) when a row's new max exceeds the one in use by more than 8: the probabilities
 // are then at most e^8, far inside fp32, and the final division by the row sum removes the common factor.
+// The epilogue leaves the digits of the O projection's operand (a row of it is the four heads of a query).
 // All waits are bounded; a wait that runs out sets *err, and the CTA lets its copies land and frees its
 // TMEM before it returns.
 #pragma once
+#include "kernels_gemm_i8.cuh"  // digits of the O projection's operand
+#include "kernels_prefill.cuh"  // RopeArgs
 #include "kernels_tc.cuh"
 
 namespace tg {
 
-constexpr int AT_TC_KT = 64;                       // keys per tile
-constexpr int AT_TC_STAGE = 36 * 1024;             // ring stage: Q (3 x 8 KiB) + K (3 x 4 KiB), or V (3 x 8 KiB)
-constexpr int AT_TC_NS = 4;                        // ring stages
-constexpr int AT_TC_PBYTES = 3 * 2 * TC_TILE_BYTES;  // P: 3 terms x 2 blocks of 32 keys x [128][32] bf16
-constexpr int AT_TC_SMEM = AT_TC_NS * AT_TC_STAGE + AT_TC_PBYTES + 1024;
+constexpr int AT_TC_BM = 128;                      // rows of a tile: 32 queries x 4 heads
+constexpr int AT_TC_KT = 128;                      // keys per tile
+constexpr int AT_TC_QBYTES = AT_TC_BM * 16 * 2;    // one term of a Q or K block: [128 rows][16 dimensions] bf16
+constexpr int AT_TC_VBYTES = 16 * 256 * 2;         // one term of a V block: [16 keys][256 dimensions] bf16
+constexpr int AT_TC_STAGE = 6 * AT_TC_QBYTES;      // ring stage: Q and K blocks (3 x 4 KiB each), or a V block (3 x 8 KiB)
+static_assert(AT_TC_STAGE == 3 * AT_TC_VBYTES, "");
+constexpr int AT_TC_NS = 5;                        // ring stages
+constexpr int AT_TC_PTERM = AT_TC_BM * AT_TC_KT * 2;  // P: one term of [8 blocks of 16 keys][128 rows][16 keys] bf16
+constexpr int AT_TC_SMEM = AT_TC_NS * AT_TC_STAGE + 3 * AT_TC_PTERM + 1024;
 constexpr int AT_TC_THREADS = 320;                 // 8 softmax warps, the MMA-issuing warp, the copy-issuing warp
-constexpr int AT_TC_BLOCKS = 12;                   // ring blocks per key tile: 8 of Q|K (32 dimensions each), 4 of V (16 keys each)
-constexpr int AT_TC_VBYTES = 8192;                 // one term of a V block: [16 keys][256 dimensions] bf16
 
-// v fp32 [S][256] -> three bf16 terms in the N-major operand layout, one 8 KiB tile per 16 keys (one MMA K-step):
-// byte offset of (key k, dimension n) = (n / 8) * 256 + (k / 8) * 128 + (k % 8) * 16 + (n % 8) * 2. Keys >= S are zero.
-__global__ void __launch_bounds__(256) attn_pack_v_kernel(const float *v, __nv_bfloat16 *out, int S, int nblocks) {
-	pdl_trigger();
-	pdl_wait();
-	v += size_t(blockIdx.y) * S * 256;  // blockIdx.y: the prompt
-	out += size_t(blockIdx.y) * 3 * nblocks * 4096;
-	const size_t term_stride = size_t(nblocks) * 4096;  // elements
-	const size_t n_items = size_t(nblocks) * 16 * 32;   // (key, 8 consecutive dimensions)
-	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_items; c += size_t(gridDim.x) * blockDim.x) {
-		const int key = int(c >> 5), n8 = int(c & 31);
-		float x[8];
-		if (key < S) {
-			const float4 a = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8);
-			const float4 b = *reinterpret_cast<const float4 *>(v + size_t(key) * 256 + 8 * n8 + 4);
-			x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-		} else {
+// eight fp32 values -> three bf16 terms, one 16-byte store each; every residual is exact
+__device__ __forceinline__ void at_split8(__nv_bfloat16 *out, size_t term_stride, const float (&x)[8]) {
+	__align__(16) __nv_bfloat16 hi[8], mid[8], lo[8];
 #pragma unroll
-			for (int i = 0; i < 8; i++) x[i] = 0.0f;
-		}
-		__align__(16) __nv_bfloat16 hi[8], mid[8], lo[8];
+	for (int i = 0; i < 8; i++) {
+		hi[i] = __float2bfloat16_rn(x[i]);
+		const float r1 = x[i] - __bfloat162float(hi[i]);
+		mid[i] = __float2bfloat16_rn(r1);
+		lo[i] = __float2bfloat16_rn(r1 - __bfloat162float(mid[i]));
+	}
+	*reinterpret_cast<uint4 *>(out) = *reinterpret_cast<const uint4 *>(hi);
+	*reinterpret_cast<uint4 *>(out + term_stride) = *reinterpret_cast<const uint4 *>(mid);
+	*reinterpret_cast<uint4 *>(out + 2 * term_stride) = *reinterpret_cast<const uint4 *>(lo);
+}
+__device__ __forceinline__ void at_load8(float (&x)[8], const float *p) {
+	const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+	x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+
+// The raw sums of the grouped q|k|v GEMM (RopeArgs::part) -> splits added, scaled, q/k norm, RoPE, cache append (as
+// qk_norm_rope_prefill_kernel) and the packed operands of the attention, in one pass over memory. 16384 x 1536: 61 us,
+// where that kernel, two packing passes over q and k and one over v took 210.
+// A CTA is 8 positions. A warp does eight rows of the packed operands: warps 0-3 two positions of q with four heads
+// each, 4 the keys, 5 the values. Lane (row, quarter) = (lane % 8, lane / 8) holds the dimensions 32 i + 8 * quarter .. + 8, i < 8: a row's sum of squares is two
+// shuffles away, RoPE's partner dimension is in the same lane, and a store of the warp fills four core matrices, 512 contiguous bytes (v: whole 128-byte lines).
+// Positions >= S are packed as zeros (the tiles of the operands are whole).
+__global__ void __launch_bounds__(192) attn_qkv_pack_kernel(RopeArgs a, __nv_bfloat16 *qp, __nv_bfloat16 *kp, __nv_bfloat16 *vp, int q_tiles, int k_tiles,
+                                                            int v_blocks) {
+	pdl_trigger();
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 7, d0 = 8 * (lane >> 3);
+	const int p0 = int(blockIdx.x) * 8, s = warp < 4 ? p0 + 2 * warp + (r >> 2) : p0 + r, head = warp < 4 ? r & 3 : 0;
+	const int col = warp < 4 ? head * 256 : (warp == 4 ? 1024 : 1280);  // of a row of q | k | v
+	const bool in = s < a.S;
+	pdl_wait();
+	float x[8][8];
+	const float *src = a.part + (size_t(blockIdx.y) * a.S + min(s, a.S - 1)) * 1536 + col + d0;
+#pragma unroll
+	for (int i = 0; i < 8; i++) at_load8(x[i], src + 32 * i);
+	for (int sp = 1; sp < a.nsplit; sp++) {
+		src += size_t(a.rows) * 1536;
 #pragma unroll
 		for (int i = 0; i < 8; i++) {
-			hi[i] = __float2bfloat16_rn(x[i]);
-			const float r1 = x[i] - __bfloat162float(hi[i]);
-			mid[i] = __float2bfloat16_rn(r1);
-			lo[i] = __float2bfloat16_rn(r1 - __bfloat162float(mid[i]));
+			float y[8];
+			at_load8(y, src + 32 * i);
+#pragma unroll
+			for (int e = 0; e < 8; e++) x[i][e] += y[e];
 		}
-		const int kb = key >> 4, k = key & 15;
-		const size_t off = size_t(kb) * 4096 + n8 * 128 + (k >> 3) * 64 + (k & 7) * 8;  // elements
-		*reinterpret_cast<uint4 *>(out + off) = *reinterpret_cast<const uint4 *>(hi);
-		*reinterpret_cast<uint4 *>(out + term_stride + off) = *reinterpret_cast<const uint4 *>(mid);
-		*reinterpret_cast<uint4 *>(out + 2 * term_stride + off) = *reinterpret_cast<const uint4 *>(lo);
+	}
+	const float *sc = (warp < 4 ? a.sq + head * 256 : (warp == 4 ? a.sk : a.sv)) + d0;
+#pragma unroll
+	for (int i = 0; i < 8; i++) {
+		float f[8];
+		at_load8(f, sc + 32 * i);
+#pragma unroll
+		for (int e = 0; e < 8; e++) x[i][e] = in ? x[i][e] * f[e] : 0.0f;
+	}
+	if (warp < 5) {
+		float ss = 0.0f;
+#pragma unroll
+		for (int i = 0; i < 8; i++)
+#pragma unroll
+			for (int e = 0; e < 8; e++) ss = fmaf(x[i][e], x[i][e], ss);
+		ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+		ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+		const float rn = inv_rms(ss, 256);
+		const float *w = (warp < 4 ? a.rmsq : a.rmsk) + d0;
+		const size_t pos = size_t(a.pos0 + min(s, a.S - 1)) * 256 + d0;
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+			float wl[8], wh[8], cl[8], ch[8], nl[8], nh[8];
+			at_load8(wl, w + 32 * i);
+			at_load8(wh, w + 128 + 32 * i);
+			at_load8(cl, a.cosT + pos + 32 * i);
+			at_load8(ch, a.cosT + pos + 128 + 32 * i);
+			at_load8(nl, a.sinT + pos + 32 * i);
+			at_load8(nh, a.sinT + pos + 128 + 32 * i);
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				// y = cos*x + rotate_half(x)*sin, rotate_half = [-x_hi, x_lo]
+				const float u = (x[i][e] * rn) * (wl[e] + 1.0f), v = (x[i + 4][e] * rn) * (wh[e] + 1.0f);
+				x[i][e] = fmaf(-1.0f * v, nl[e], cl[e] * u);
+				x[i + 4][e] = fmaf(u, nh[e], ch[e] * v);
+			}
+		}
+	}
+	if (warp >= 4 && in && s >= a.cache_from) {
+		float *c = (warp == 4 ? a.kcache : a.vcache) + blockIdx.y * a.cache_stride + size_t((s + a.slot_off) % a.slots) * 256 + d0;
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			*reinterpret_cast<float4 *>(c + 32 * i) = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
+			*reinterpret_cast<float4 *>(c + 32 * i + 4) = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
+		}
+	}
+	if (warp < 5) {
+		const int tiles = warp < 4 ? q_tiles : k_tiles, row = warp < 4 ? 4 * s + head : s;
+		const size_t term = size_t(tiles) * AT_TC_BM * 256;  // elements
+		__nv_bfloat16 *out = (warp < 4 ? qp : kp) + blockIdx.y * 3 * term + size_t(row / AT_TC_BM) * (AT_TC_BM * 256) + (row % AT_TC_BM / 8) * 128 + r * 8;
+		// dimension 32 i + d0: block 2 i + d0 / 16, 8-wide half (d0 / 8) % 2 of its rows
+		const int off = (d0 >> 4) * (AT_TC_QBYTES / 2) + ((d0 >> 3) & 1) * 64;
+#pragma unroll
+		for (int i = 0; i < 8; i++) at_split8(out + off + i * AT_TC_QBYTES, term, x[i]);
+	} else if (s < 16 * v_blocks) {
+		const size_t term = size_t(v_blocks) * (AT_TC_VBYTES / 2);
+		// (key, dimension n) of a block: (n / 8) * 256 + (key / 8) * 128 + (key % 8) * 16 + (n % 8) * 2 bytes
+		__nv_bfloat16 *out = vp + blockIdx.y * 3 * term + size_t(s >> 4) * (AT_TC_VBYTES / 2) + ((s >> 3) & 1) * 64 + r * 8 + (d0 >> 3) * 128;
+#pragma unroll
+		for (int i = 0; i < 8; i++) at_split8(out + i * 512, term, x[i]);
 	}
 }
 
 // instruction descriptor: D fp32, A and B bf16, A K-major, B K-major (b_mn = 0) or N-major (1), M = 128, N = n
 __device__ __forceinline__ uint32_t at_idesc(int n, int b_mn) {
-	return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(b_mn) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
+	return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(b_mn) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(AT_TC_BM >> 4) << 24);
+}
+// shared-memory matrix descriptor of a Q, K or P block: K-major, no swizzle, 128 B to the next 8 k, 256 B to the next 8 rows
+__device__ __forceinline__ uint64_t at_qdesc(uint32_t smem_addr) {
+	return uint64_t((smem_addr & 0x3FFFF) >> 4) | (uint64_t(128 >> 4) << 16) | (uint64_t(256 >> 4) << 32) | (uint64_t(1) << 46);
 }
 // shared-memory matrix descriptor of a V block: no swizzle, 128 B between the two 8-key groups, 256 B between
 // groups of 8 dimensions
@@ -141,10 +228,12 @@ __device__ __forceinline__ bool at_exchange(float *val, int *tag, int me, float 
 
 struct AttnTcArgs {
 	// per prompt (blockIdx.y), one behind the other:
-	const __nv_bfloat16 *qp;  // [3][q_tiles][8][8 KiB]
-	const __nv_bfloat16 *kp;  // [3][k_tiles][8][8 KiB]
+	const __nv_bfloat16 *qp;  // [3][q_tiles][16][4 KiB]
+	const __nv_bfloat16 *kp;  // [3][k_tiles][16][4 KiB]
 	const __nv_bfloat16 *vp;  // [3][v_blocks][8 KiB]
-	float *o;                 // [S][4][256]
+	uint8_t *x;               // digits of the rows [prompts * S][4 * 256] (i8_offset), and their scales
+	float *rowscale;
+	int groups;
 	int S, q_tiles, k_tiles, v_blocks;
 	int is_local, window;
 	int *err;
@@ -170,10 +259,13 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	const int tile = int(gridDim.x) - 1 - int(blockIdx.x);  // the tiles with the most keys start first
 	const int q0 = tile * 32;                                // first query of the tile
 	const int q_hi = min(a.S - 1, q0 + 31);
-	// key tiles this row tile needs
-	const int j_lo = a.is_local ? max(0, q0 - a.window) / AT_TC_KT : 0;
-	const int j_hi = q_hi / AT_TC_KT;
+	// key tiles this row tile needs, and the blocks of 16 keys of them: u_lo .. 8 of the first, 0 .. u_hi of the last
+	const int key_lo = a.is_local ? max(0, q0 - a.window) : 0;
+	const int j_lo = key_lo / AT_TC_KT, j_hi = q_hi / AT_TC_KT;
 	const int ntiles = j_hi - j_lo + 1;
+	const int u_lo = key_lo % AT_TC_KT / 16, u_hi = q_hi % AT_TC_KT / 16 + 1;
+	auto first_block = [&](int t) { return t == 0 ? u_lo : 0; };
+	auto end_block = [&](int t) { return t == ntiles - 1 ? u_hi : AT_TC_KT / 16; };
 
 	if (tid == 0) {
 		for (int s = 0; s < AT_TC_NS; s++) {
@@ -189,114 +281,124 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	for (int i = tid; i < 2 * 128 * 2; i += AT_TC_THREADS) (&xt[0][0][0])[i] = 0;
-	if (warp == 8) {  // TMEM: S in columns 0..63 and 64..127 (alternating tiles), O in columns 128..383
+	if (warp == 8) {  // TMEM: S in columns 0..127 and 128..255 (alternating tiles), O in columns 256..511
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
-	const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 128u;
+	const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 2u * AT_TC_KT;
 	volatile int *fail = &s_fail;
 
-	// MMA order: QK(0), then for t = 1 .. n: QK(t) (if t < n), PV(t - 1). Ring block g in that order:
-	// g < 8: QK(0) block g; else g' = g - 8, t = 1 + g' / 12, r = g' % 12: QK(t) block r (r < 8, t < n) or PV(t - 1)
-	// block r - 8 (t < n), and the last four blocks are PV(n - 1).
-	struct Blk {
-		int qk, tile, i;  // qk: 1 = Q|K block i (dimensions 32 i ..) of key tile `tile`, 0 = V block i (keys 16 i ..) of it
+	// Order of the ring blocks and of the MMAs: QK(0), then for t = 1 .. n: QK(t) (if t < n), PV(t - 1)
+	auto walk = [&](auto &&qk, auto &&pv) {
+		for (int t = 0; t <= ntiles; t++) {
+			if (t < ntiles)
+				for (int i = 0; i < 16; i++) qk(t, i);  // dimensions 16 i ..
+			if (t > 0)
+				for (int u = first_block(t - 1); u < end_block(t - 1); u++) pv(t - 1, u);  // keys 16 u ..
+		}
 	};
-	auto blk = [&](int g) -> Blk {
-		if (g < 8) return Blk{1, 0, g};
-		const int gp = g - 8, t = 1 + gp / AT_TC_BLOCKS, r = gp % AT_TC_BLOCKS;
-		if (t >= ntiles) return Blk{0, ntiles - 1, r};
-		return r < 8 ? Blk{1, t, r} : Blk{0, t - 1, r - 8};
-	};
-	const int total = ntiles * AT_TC_BLOCKS;
 	if (warp == 9) {
 		// ------------------------------------------------------------ bulk copies, up to AT_TC_NS blocks ahead
-		pdl_wait();  // the packed operands are the predecessors' output
-		const size_t q_term = size_t(a.q_tiles) * 8 * TC_TILE_BYTES, k_term = size_t(a.k_tiles) * 8 * TC_TILE_BYTES,
+		pdl_wait();  // the packed operands are the predecessor's output
+		const size_t q_term = size_t(a.q_tiles) * 16 * AT_TC_QBYTES, k_term = size_t(a.k_tiles) * 16 * AT_TC_QBYTES,
 		             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
-		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 3 * q_term, *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 3 * k_term,
-		              *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 3 * v_term;
+		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 3 * q_term + size_t(tile) * 16 * AT_TC_QBYTES,
+		              *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 3 * k_term, *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 3 * v_term;
 		int cap = TC_SPIN_CAP, st = 0;
 		uint32_t ph = 1;  // (a fresh barrier passes parity 1)
-		for (int g = 0; g < total; g++) {
-			const Blk b = blk(g);
-			const int j = j_lo + b.tile, i = b.i;
-			uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
-			tc_wait_cap(&free_bar[st], ph, cap);
-			if (tc_elect()) {
-				if (b.qk) {
-					mbar_expect_tx(&full_bar[st], 3u * TC_TILE_BYTES + 3u * (TC_TILE_BYTES / 2));
-#pragma unroll
-					for (int t = 0; t < 3; t++) {
-						bulk_load(dst + t * TC_TILE_BYTES, qp + t * q_term + (size_t(tile) * 8 + i) * TC_TILE_BYTES, TC_TILE_BYTES, &full_bar[st]);
-						bulk_load(dst + 3 * TC_TILE_BYTES + t * (TC_TILE_BYTES / 2),
-						          kp + t * k_term + (size_t(j >> 1) * 8 + i) * TC_TILE_BYTES + (j & 1) * (TC_TILE_BYTES / 2), TC_TILE_BYTES / 2,
-						          &full_bar[st]);
-					}
-				} else {
-					mbar_expect_tx(&full_bar[st], 3u * AT_TC_VBYTES);
-#pragma unroll
-					for (int t = 0; t < 3; t++)
-						bulk_load(dst + t * AT_TC_VBYTES, vp + t * v_term + (size_t(4 * j + i)) * AT_TC_VBYTES, AT_TC_VBYTES, &full_bar[st]);
-				}
-			}
+		auto next = [&] {
 			if (++st == AT_TC_NS) {
 				st = 0;
 				ph ^= 1;
 			}
-		}
+		};
+		walk(
+		    [&](int t, int i) {
+			    const uint32_t lo = uint32_t(first_block(t)) * 512u, bytes = uint32_t(end_block(t)) * 512u - lo;  // the block's rows of K: 32 bytes each
+			    uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
+			    const uint8_t *q = qp + size_t(i) * AT_TC_QBYTES, *k = kp + (size_t(j_lo + t) * 16 + i) * AT_TC_QBYTES + lo;
+			    tc_wait_cap(&free_bar[st], ph, cap);
+			    if (tc_elect()) {
+				    mbar_expect_tx(&full_bar[st], 3u * (AT_TC_QBYTES + bytes));
+#pragma unroll
+				    for (int c = 0; c < 3; c++) {
+					    bulk_load(dst + c * AT_TC_QBYTES, q + c * q_term, AT_TC_QBYTES, &full_bar[st]);
+					    bulk_load(dst + (3 + c) * AT_TC_QBYTES, k + c * k_term, bytes, &full_bar[st]);
+				    }
+			    }
+			    next();
+		    },
+		    [&](int t, int u) {
+			    uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
+			    const uint8_t *v = vp + (size_t(j_lo + t) * (AT_TC_KT / 16) + u) * AT_TC_VBYTES;
+			    tc_wait_cap(&free_bar[st], ph, cap);
+			    if (tc_elect()) {
+				    mbar_expect_tx(&full_bar[st], 3u * AT_TC_VBYTES);
+#pragma unroll
+				    for (int c = 0; c < 3; c++) bulk_load(dst + c * AT_TC_VBYTES, v + c * v_term, AT_TC_VBYTES, &full_bar[st]);
+			    }
+			    next();
+		    });
 		if (cap == 0 && lane == 0) {
 			atomicExch(a.err, 6);
 			*fail = 1;
 		}
 	} else if (warp == 8) {
 		// ------------------------------------------------------------ MMAs
-		const uint32_t idesc_qk = at_idesc(AT_TC_KT, 0), idesc_pv = at_idesc(256, 1);
+		const uint32_t idesc_pv = at_idesc(256, 1);
 		// the six term products (A term, B term)
 		constexpr int ta[6] = {0, 0, 1, 1, 0, 2}, tb[6] = {0, 1, 0, 1, 2, 0};
 		int cap = TC_SPIN_CAP, st = 0;
 		uint32_t ph = 0;
 		const uint32_t pb = smem_u32(pbuf);
-		for (int g = 0; g < total; g++) {
-			const Blk b = blk(g);
-			if (!b.qk && b.i == 0) tc_wait_cap(&p_bar, b.tile & 1, cap);  // P written, O rescaled
-			tc_wait_cap(&full_bar[st], ph, cap);
+		bool ready = false;  // the next block has landed: asked before the MMAs of the one before it are issued (an answer takes 180 clk)
+		auto landed = [&] {
+			if (!ready) tc_wait_cap(&full_bar[st], ph, cap);
 			tc_fence_after();
-			const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
-			if (b.qk) {
-				const uint32_t d_s = tmem_s + uint32_t((b.tile & 1) * AT_TC_KT);
-				const uint64_t dq = tc_smem_desc(base), dk = tc_smem_desc(base + 3 * TC_TILE_BYTES);
-				if (tc_elect()) {
-#pragma unroll
-					for (int c = 0; c < 6; c++)
-#pragma unroll
-						for (int j2 = 0; j2 < 2; j2++)
-							tc_mma(d_s, dq + uint64_t((ta[c] * TC_TILE_BYTES + j2 * 256) >> 4), dk + uint64_t((tb[c] * (TC_TILE_BYTES / 2) + j2 * 256) >> 4),
-							       idesc_qk, (b.i > 0 || c > 0 || j2 > 0) ? 1u : 0u);
-					tc_commit(&free_bar[st]);
-					if (b.i == 7) tc_commit(&s_bar[b.tile & 1]);
-				}
-			} else {
-				const int vb = b.i;  // keys 16 vb ..: K-step vb % 2 of P's 32-key block vb / 2
-				const uint64_t dp = tc_smem_desc(pb + (vb >> 1) * TC_TILE_BYTES + (vb & 1) * 256), dv = at_vdesc(base);
-				if (tc_elect()) {
-#pragma unroll
-					for (int c = 0; c < 6; c++)
-						tc_mma(tmem_o, dp + uint64_t((ta[c] * 2 * TC_TILE_BYTES) >> 4), dv + uint64_t((tb[c] * AT_TC_VBYTES) >> 4), idesc_pv,
-						       (b.tile > 0 || vb > 0 || c > 0) ? 1u : 0u);
-					tc_commit(&free_bar[st]);
-					if (vb == 3) tc_commit(&pv_bar);
-				}
-			}
+			const int n = st + 1 == AT_TC_NS ? 0 : st + 1;
+			ready = mbar_test_wait(&full_bar[n], n ? ph : ph ^ 1u);
+			ready = __all_sync(0xffffffffu, ready);
+		};
+		auto next = [&] {
 			__syncwarp();
 			if (++st == AT_TC_NS) {
 				st = 0;
 				ph ^= 1;
 			}
-		}
+		};
+		walk(
+		    [&](int t, int i) {
+			    landed();
+			    const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE), lo = uint32_t(first_block(t)) * 16u, n = uint32_t(end_block(t)) * 16u - lo;
+			    const uint32_t d_s = tmem_s + uint32_t(t & 1) * AT_TC_KT + lo, idesc = at_idesc(int(n), 0);
+			    const uint64_t dq = at_qdesc(base), dk = at_qdesc(base + 3 * AT_TC_QBYTES);
+			    if (tc_elect()) {
+#pragma unroll
+				    for (int c = 0; c < 6; c++)
+					    tc_mma(d_s, dq + uint64_t((ta[c] * AT_TC_QBYTES) >> 4), dk + uint64_t((tb[c] * AT_TC_QBYTES) >> 4), idesc, (i > 0 || c > 0) ? 1u : 0u);
+				    tc_commit(&free_bar[st]);
+				    if (i == 15) tc_commit(&s_bar[t & 1]);
+			    }
+			    next();
+		    },
+		    [&](int t, int u) {
+			    if (u == first_block(t)) tc_wait_cap(&p_bar, t & 1, cap);  // P written, O rescaled
+			    landed();
+			    const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
+			    const uint64_t dp = at_qdesc(pb + uint32_t(u) * AT_TC_QBYTES), dv = at_vdesc(base);
+			    if (tc_elect()) {
+#pragma unroll
+				    for (int c = 0; c < 6; c++)
+					    tc_mma(tmem_o, dp + uint64_t((ta[c] * AT_TC_PTERM) >> 4), dv + uint64_t((tb[c] * AT_TC_VBYTES) >> 4), idesc_pv,
+					           (t > 0 || u > u_lo || c > 0) ? 1u : 0u);
+				    tc_commit(&free_bar[st]);
+				    if (u == end_block(t) - 1) tc_commit(&pv_bar);
+			    }
+			    next();
+		    });
 		if (tc_elect()) tc_commit(&o_bar);
 		if (cap == 0 && lane == 0) {
 			atomicExch(a.err, 6);
@@ -305,7 +407,8 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 	} else {
 		// ------------------------------------------------------------ softmax (two threads per row = TMEM lane)
 		// warps w and w + 4 share the TMEM lanes 32 (w % 4) ..: thread (w, lane) owns row 32 (w % 4) + lane and the
-		// 32 keys 32 (w / 4) .. of every tile (= one of P's two 32-key blocks), and half of O's columns
+		// 64 keys 64 (w / 4) .. of every tile, and half of O's columns
+		constexpr int HK = AT_TC_KT / 2;
 		const int qd = warp & 3, hf = warp >> 2;
 		const int r = qd * 32 + lane;              // row of the tile
 		const int qi = q0 + (r >> 2);              // this row's query
@@ -317,27 +420,28 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		for (int jt = 0; jt < ntiles && ok; jt++) {
 			if (!at_wait(&s_bar[jt & 1], (jt >> 1) & 1, a.err, fail)) { ok = false; break; }
 			tc_fence_after();
-			uint32_t sv[32];
-			tc_ld32(tmem_s + lane_base + uint32_t((jt & 1) * AT_TC_KT + 32 * hf), sv);
+			uint32_t sv[2][32];
+			tc_ld32(tmem_s + lane_base + uint32_t((jt & 1) * AT_TC_KT + HK * hf), sv[0]);
+			tc_ld32(tmem_s + lane_base + uint32_t((jt & 1) * AT_TC_KT + HK * hf + 32), sv[1]);
 			asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-			const int kbase = (j_lo + jt) * AT_TC_KT + 32 * hf;
+			const int tbase = (j_lo + jt) * AT_TC_KT, kbase = tbase + HK * hf;
 			// (most tiles lie wholly inside every row's key range: no per-key test there)
-			const bool all_vis = (j_lo + jt) * AT_TC_KT + AT_TC_KT - 1 <= q0 && (!a.is_local || (j_lo + jt) * AT_TC_KT >= q0 + 31 - a.window);
+			const bool all_vis = tbase + AT_TC_KT - 1 <= q0 && (!a.is_local || tbase >= q0 + 31 - a.window);
 			float mt = -INFINITY;
 			if (all_vis) {
 #pragma unroll
-				for (int c = 0; c < 32; c++) {
-					const float x = __uint_as_float(sv[c]) * 0.0625f;  // 1 / sqrt(256), exact
-					sv[c] = __float_as_uint(x);
+				for (int c = 0; c < HK; c++) {
+					const float x = __uint_as_float(sv[c >> 5][c & 31]) * 0.0625f;  // 1 / sqrt(256), exact
+					sv[c >> 5][c & 31] = __float_as_uint(x);
 					mt = fmaxf(mt, x);
 				}
-			} else {
+			} else {  // (columns of keys that no row sees hold nothing: selected away)
 #pragma unroll
-				for (int c = 0; c < 32; c++) {
+				for (int c = 0; c < HK; c++) {
 					const int key = kbase + c;
 					const bool vis = row_ok && key <= qi && key >= k_min;
-					const float x = vis ? __uint_as_float(sv[c]) * 0.0625f : -INFINITY;
-					sv[c] = __float_as_uint(x);
+					const float x = vis ? __uint_as_float(sv[c >> 5][c & 31]) * 0.0625f : -INFINITY;
+					sv[c >> 5][c & 31] = __float_as_uint(x);
 					mt = fmaxf(mt, x);
 				}
 			}
@@ -351,37 +455,42 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			const float mn = (mt > m + 8.0f || m == -INFINITY) ? fmaxf(m, mt) : m;
 			const bool none = mn == -INFINITY;            // no visible key so far
 			const float corr = none ? 1.0f : expf(m - mn);  // exp(-inf) = 0 at the row's first visible tile; 1 when the max stays
-			// probabilities and their three bf16 terms by truncation (p >= 0; hi + mid + lo = p exactly: 8 + 8 + 8 bits)
 			float sum = 0.0f;
-			uint32_t ph[16], pm[16], pl[16];  // bf16 pairs
 #pragma unroll
-			for (int c = 0; c < 32; c += 2) {
-				uint32_t hb[2], mb[2], lb[2];
-#pragma unroll
-				for (int u = 0; u < 2; u++) {
-					const float pv = none ? 0.0f : expf(__uint_as_float(sv[c + u]) - mn);  // exp(-inf) = 0 for masked keys
-					sum += pv;
-					hb[u] = __float_as_uint(pv) & 0xFFFF0000u;
-					const float r1 = pv - __uint_as_float(hb[u]);
-					mb[u] = __float_as_uint(r1) & 0xFFFF0000u;
-					lb[u] = __float_as_uint(r1 - __uint_as_float(mb[u]));  // at most 8 significant bits: exact in bf16
-				}
-				ph[c / 2] = __byte_perm(hb[0], hb[1], 0x7632);
-				pm[c / 2] = __byte_perm(mb[0], mb[1], 0x7632);
-				pl[c / 2] = __byte_perm(lb[0], lb[1], 0x7632);
+			for (int c = 0; c < HK; c++) {
+				const float p = none ? 0.0f : expf(__uint_as_float(sv[c >> 5][c & 31]) - mn);  // exp(-inf) = 0 for masked keys
+				sum += p;
+				sv[c >> 5][c & 31] = __float_as_uint(p);
 			}
 			l = fmaf(l, corr, sum);
 			m = mn;
 			// the previous tile's P V reads P (and accumulates into O) until pv_bar: wait for it before touching either
 			if (jt > 0 && !at_wait(&pv_bar, (jt - 1) & 1, a.err, fail)) { ok = false; break; }
 			tc_fence_after();
-			// P[term][block hf] tiles of [128][32] in the A-operand layout
+			// the probabilities' three bf16 terms by truncation (p >= 0; hi + mid + lo = p exactly: 8 + 8 + 8 bits), eight keys of the row at a time
 #pragma unroll
-			for (int k8 = 0; k8 < 4; k8++) {
-				uint8_t *dst = pbuf + hf * TC_TILE_BYTES + (r >> 3) * 512 + k8 * 128 + (r & 7) * 16;
-				*reinterpret_cast<uint4 *>(dst) = make_uint4(ph[4 * k8], ph[4 * k8 + 1], ph[4 * k8 + 2], ph[4 * k8 + 3]);
-				*reinterpret_cast<uint4 *>(dst + 2 * TC_TILE_BYTES) = make_uint4(pm[4 * k8], pm[4 * k8 + 1], pm[4 * k8 + 2], pm[4 * k8 + 3]);
-				*reinterpret_cast<uint4 *>(dst + 4 * TC_TILE_BYTES) = make_uint4(pl[4 * k8], pl[4 * k8 + 1], pl[4 * k8 + 2], pl[4 * k8 + 3]);
+			for (int k8 = 0; k8 < HK / 8; k8++) {
+				uint32_t ph[4], pm[4], pl[4];  // bf16 pairs
+#pragma unroll
+				for (int c = 0; c < 4; c++) {
+					uint32_t hb[2], mb[2], lb[2];
+#pragma unroll
+					for (int u = 0; u < 2; u++) {
+						const int e = 8 * k8 + 2 * c + u;
+						const float pv = __uint_as_float(sv[e >> 5][e & 31]);
+						hb[u] = __float_as_uint(pv) & 0xFFFF0000u;
+						const float r1 = pv - __uint_as_float(hb[u]);
+						mb[u] = __float_as_uint(r1) & 0xFFFF0000u;
+						lb[u] = __float_as_uint(r1 - __uint_as_float(mb[u]));  // at most 8 significant bits: exact in bf16
+					}
+					ph[c] = __byte_perm(hb[0], hb[1], 0x7632);
+					pm[c] = __byte_perm(mb[0], mb[1], 0x7632);
+					pl[c] = __byte_perm(lb[0], lb[1], 0x7632);
+				}
+				uint8_t *dst = pbuf + (HK / 16 * hf + (k8 >> 1)) * AT_TC_QBYTES + (r >> 3) * 256 + (k8 & 1) * 128 + (r & 7) * 16;
+				*reinterpret_cast<uint4 *>(dst) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+				*reinterpret_cast<uint4 *>(dst + AT_TC_PTERM) = make_uint4(pm[0], pm[1], pm[2], pm[3]);
+				*reinterpret_cast<uint4 *>(dst + 2 * AT_TC_PTERM) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
 			}
 			// O = corr * O: this thread's half of the row's 256 columns
 			if (jt > 0 && !__all_sync(0xffffffffu, corr == 1.0f)) {
@@ -401,25 +510,51 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			__syncwarp();
 			if (lane == 0) mbar_arrive(&p_bar);
 		}
-		// ------------------------------------------------------------ epilogue: o = O / l
+		// ------------------------------------------------------------ epilogue: the digits of o = O / l
+		// A row of the O projection's operand is the four heads of a query: four neighbouring lanes, in both halves. Its largest value
+		// first, then O once more. (The partner is past its last read of a slot: it arrived at p_bar, which o_bar follows.)
 		if (ok && at_wait(&o_bar, 0, a.err, fail)) {
 			tc_fence_after();
-			float l_other = 0.0f;  // (the partner is past its last read of slot 0: it arrived at p_bar, which o_bar follows)
-			const bool got = at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, &l_other, a.err, fail);
-			const float lt = l + l_other;
-			const float inv = (row_ok && got) ? 1.0f / lt : 0.0f;  // (a visible key always exists: the query itself)
-			float *orow = a.o + (size_t(blockIdx.y) * a.S * 4 + size_t(tile) * 128 + r) * 256;
+			float other = 0.0f;
+			bool got = at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, &other, a.err, fail);
+			const float inv = 1.0f / (l + other);  // (a visible key always exists: the query itself)
+			uint32_t mx = 0;
 #pragma unroll 1
 			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
 				uint32_t ov[32];
 				tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
 				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-				if (row_ok) {
 #pragma unroll
-					for (int i = 0; i < 32; i += 4)
-						*reinterpret_cast<float4 *>(orow + 32 * c8 + i) =
-						    make_float4(__uint_as_float(ov[i]) * inv, __uint_as_float(ov[i + 1]) * inv, __uint_as_float(ov[i + 2]) * inv,
-						                __uint_as_float(ov[i + 3]) * inv);
+				for (int i = 0; i < 32; i++) mx = max(mx, i8_abs_bits(__uint_as_float(ov[i]) * inv));
+			}
+			mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+			mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+			got = got && at_exchange(xm[1][r], xt[1][r], hf, __uint_as_float(mx), 0x40000001, &other, a.err, fail);
+			mx = max(mx, __float_as_uint(other));
+			const float mul = i8_row_mul(mx);
+			const int row = int(blockIdx.y) * a.S + qi, head = r & 3;
+			const bool store = row_ok && got;
+			if (store && hf == 0 && head == 0) a.rowscale[row] = i8_row_scale(mx);
+#pragma unroll 1
+			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
+				uint32_t ov[32];
+				tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
+				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+				if (store) {
+#pragma unroll
+					for (int h = 0; h < 2; h++) {  // 16 dimensions: one chunk of 16 bytes per digit
+						uint32_t d[4][4];
+#pragma unroll
+						for (int q = 0; q < 4; q++) {
+							uint32_t b[4];
+#pragma unroll
+							for (int i = 0; i < 4; i++) b[i] = i8_digits(__uint_as_float(ov[16 * h + 4 * q + i]) * inv, mul);
+							i8_transpose4(b, d[0][q], d[1][q], d[2][q], d[3][q]);
+						}
+						uint8_t *p = a.x + i8_offset(row, (head * 256 + 32 * c8 + 16 * h) >> 2, a.groups);
+#pragma unroll
+						for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(p + 512 * i) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
+					}
 				}
 			}
 		}

@@ -75,16 +75,23 @@ __device__ __forceinline__ size_t i8_offset(int row, int k4, int groups) {
 	const int kb = k4 >> 4, chunk = (k4 >> 2) & 3, r = row & 7;
 	return (size_t(kb) * groups + (row >> 3)) * I8_GROUP_BYTES + r * 64 + ((chunk ^ (r >> 1)) << 4) + ((k4 & 3) << 2);
 }
+// the digits of four values -> four words of one digit each
+__device__ __forceinline__ void i8_transpose4(const uint32_t (&q)[4], uint32_t &d0, uint32_t &d1, uint32_t &d2, uint32_t &d3) {
+	const uint32_t ab01 = __byte_perm(q[0], q[1], 0x5140), ab23 = __byte_perm(q[0], q[1], 0x7362);
+	const uint32_t cd01 = __byte_perm(q[2], q[3], 0x5140), cd23 = __byte_perm(q[2], q[3], 0x7362);
+	d0 = __byte_perm(ab01, cd01, 0x5410);
+	d1 = __byte_perm(ab01, cd01, 0x7632);
+	d2 = __byte_perm(ab23, cd23, 0x5410);
+	d3 = __byte_perm(ab23, cd23, 0x7632);
+}
 // four consecutive values of a row -> one 4-byte store per digit
 __device__ __forceinline__ void i8_pack4(uint8_t *out, int groups, int row, int k4, const float4 &v, float mul) {
-	const uint32_t a = i8_digits(v.x, mul), b = i8_digits(v.y, mul), c = i8_digits(v.z, mul), d = i8_digits(v.w, mul);
-	const uint32_t ab01 = __byte_perm(a, b, 0x5140), ab23 = __byte_perm(a, b, 0x7362);
-	const uint32_t cd01 = __byte_perm(c, d, 0x5140), cd23 = __byte_perm(c, d, 0x7362);
+	const uint32_t q[4] = {i8_digits(v.x, mul), i8_digits(v.y, mul), i8_digits(v.z, mul), i8_digits(v.w, mul)};
+	uint32_t d[4];
+	i8_transpose4(q, d[0], d[1], d[2], d[3]);
 	uint8_t *p = out + i8_offset(row, k4, groups);
-	*reinterpret_cast<uint32_t *>(p) = __byte_perm(ab01, cd01, 0x5410);
-	*reinterpret_cast<uint32_t *>(p + 512) = __byte_perm(ab01, cd01, 0x7632);
-	*reinterpret_cast<uint32_t *>(p + 1024) = __byte_perm(ab23, cd23, 0x5410);
-	*reinterpret_cast<uint32_t *>(p + 1536) = __byte_perm(ab23, cd23, 0x7632);
+#pragma unroll
+	for (int i = 0; i < 4; i++) *reinterpret_cast<uint32_t *>(p + 512 * i) = d[i];
 }
 __device__ __forceinline__ uint32_t warp_umax(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 template <int NW> __device__ __forceinline__ uint32_t block_umax(uint32_t v, uint32_t *red) {

@@ -1,10 +1,4 @@
-// Helpers of the tcgen05 / TMEM kernels: fp32 operands as three bf16 terms (x = hi + mid + lo, 8 + 8 + 8 mantissa bits,
-// each residual computed exactly in fp32), packed in the tensor core's shared-memory layout so that a kernel fetches an
-// operand tile with one bulk copy; MMA, commit, fence, TMEM-load and bounded-wait wrappers.
-//
-// Operand layout (K-major, no swizzle): 8 x 8 bf16 "core matrices" of 128 contiguous bytes (8 rows of 16 bytes); byte
-// offset of (r, k) in a [128][32] tile = (r/8)*512 + (k/8)*128 + (r%8)*16 + (k%8)*2, i.e. 128 B between the 8-wide K
-// groups of an MMA (leading offset), 512 B between groups of 8 rows (stride offset).
+// Helpers of the tcgen05 / TMEM kernels: MMA, commit, fence, TMEM-load and bounded-wait wrappers.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -14,75 +8,9 @@
 
 namespace tg {
 
-constexpr int TC_BM = 128, TC_BK = 32;
-constexpr int TC_TILE_BYTES = TC_BM * TC_BK * 2;  // 8 KiB: one [128][32] bf16 operand tile
 constexpr int TC_SPIN_CAP = 1 << 24;
 
-// ------------------------------------------------------------------ split + pack
-// out: [3 terms][m_tiles][k_blocks][TC_TILE_BYTES]; rows >= M are zero.
-// fp32 x[8] (8 consecutive k of one row) -> the three bf16 terms, stored at the operand-layout offset
-__device__ __forceinline__ void tc_pack8(__nv_bfloat16 *out, size_t term_stride, int k_blocks, int row, int k8, const float (&x)[8]) {
-	__align__(16) __nv_bfloat16 hi[8], mid[8], lo[8];
-#pragma unroll
-	for (int i = 0; i < 8; i++) {
-		hi[i] = __float2bfloat16_rn(x[i]);
-		const float r1 = x[i] - __bfloat162float(hi[i]);  // exact
-		mid[i] = __float2bfloat16_rn(r1);
-		const float r2 = r1 - __bfloat162float(mid[i]);   // exact
-		lo[i] = __float2bfloat16_rn(r2);
-	}
-	const int mt = row / TC_BM, r = row % TC_BM, kb = (8 * k8) / TC_BK, kc = ((8 * k8) % TC_BK) / 8;
-	const size_t off = (size_t(mt) * k_blocks + kb) * (TC_TILE_BYTES / 2) + (r / 8) * 256 + kc * 64 + (r % 8) * 8;
-	*reinterpret_cast<uint4 *>(out + off) = *reinterpret_cast<const uint4 *>(hi);
-	*reinterpret_cast<uint4 *>(out + term_stride + off) = *reinterpret_cast<const uint4 *>(mid);
-	*reinterpret_cast<uint4 *>(out + 2 * term_stride + off) = *reinterpret_cast<const uint4 *>(lo);
-}
-
-// Work item c of a packing kernel -> (row, group of 8 consecutive k). Eight consecutive items are the eight rows
-// of a core matrix at the same k group, so that a warp's 16-byte stores fill whole 128-byte lines of the packed
-// tile (items in row-major order wrote every other 16 bytes of a line); each thread still reads 32 contiguous
-// bytes of its row (one sector).
-__device__ __forceinline__ void tc_chunk_to_row_k8(size_t c, int k8s, int &row, int &k8) {
-	const size_t g = c / (size_t(8) * k8s);          // group of 8 rows
-	const int w = int(c - g * (size_t(8) * k8s));    // item inside the group
-	row = int(g) * 8 + (w & 7);
-	k8 = w >> 3;
-}
-
-__global__ void __launch_bounds__(256) split_pack_kernel(const float *A, __nv_bfloat16 *out, int M, int K, int m_tiles) {
-	pdl_trigger();
-	pdl_wait();
-	const int k_blocks = K / TC_BK;
-	A += size_t(blockIdx.y) * M * K;  // blockIdx.y: one of several matrices behind each other
-	out += size_t(blockIdx.y) * 3 * m_tiles * k_blocks * (TC_TILE_BYTES / 2);
-	const size_t n_chunks = size_t(m_tiles) * TC_BM * (K / 8);  // one thread per (row, 8 consecutive k)
-	const size_t term_stride = size_t(m_tiles) * k_blocks * (TC_TILE_BYTES / 2);
-	for (size_t c = size_t(blockIdx.x) * blockDim.x + threadIdx.x; c < n_chunks; c += size_t(gridDim.x) * blockDim.x) {
-		int row, k8;
-		tc_chunk_to_row_k8(c, K / 8, row, k8);
-		float x[8];
-		if (row < M) {
-			const float4 a = *reinterpret_cast<const float4 *>(A + size_t(row) * K + 8 * k8);
-			const float4 b = *reinterpret_cast<const float4 *>(A + size_t(row) * K + 8 * k8 + 4);
-			x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-		} else {
-#pragma unroll
-			for (int i = 0; i < 8; i++) x[i] = 0.0f;
-		}
-		tc_pack8(out, term_stride, k_blocks, row, k8, x);
-	}
-}
-
 // ------------------------------------------------------------------ tcgen05 helpers
-// shared-memory matrix descriptor: K-major, no swizzle, LBO 128 B, SBO 512 B
-__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t smem_addr) {
-	uint64_t d = 0;
-	d |= uint64_t((smem_addr & 0x3FFFF) >> 4);   // start address, 16-byte units
-	d |= uint64_t(128 >> 4) << 16;               // leading-dimension byte offset (next 8 k)
-	d |= uint64_t(512 >> 4) << 32;               // stride-dimension byte offset (next 8 rows)
-	d |= uint64_t(1) << 46;                      // descriptor version of this architecture
-	return d;                                    // base offset 0, layout type 0 = no swizzle
-}
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
 	asm volatile(
 	    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"

@@ -1581,11 +1581,11 @@ struct AttnTcPlan {
 };
 AttnTcPlan attn_tc_plan(int S) {
 	AttnTcPlan p;
-	p.q_tiles = (4 * S + TC_BM - 1) / TC_BM;
-	p.k_tiles = (S + TC_BM - 1) / TC_BM;
-	p.v_blocks = 4 * ((S + AT_TC_KT - 1) / AT_TC_KT);  // 16 keys each
-	p.q_bytes = size_t(3) * p.q_tiles * 8 * TC_TILE_BYTES;
-	p.k_bytes = size_t(3) * p.k_tiles * 8 * TC_TILE_BYTES;
+	p.q_tiles = (4 * S + AT_TC_BM - 1) / AT_TC_BM;
+	p.k_tiles = (S + AT_TC_KT - 1) / AT_TC_KT;
+	p.v_blocks = (S + 15) / 16;
+	p.q_bytes = size_t(3) * p.q_tiles * 16 * AT_TC_QBYTES;
+	p.k_bytes = size_t(3) * p.k_tiles * 16 * AT_TC_QBYTES;
 	p.v_bytes = size_t(3) * p.v_blocks * AT_TC_VBYTES;
 	return p;
 }
@@ -2144,7 +2144,10 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		ra.sv = w.V.s;
 		ra.rows = S;
 		ra.cache_stride = size_t(slots) * AT_HD;
-		launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
+		if (attn_tc)  // (whole tiles of 32 queries)
+			launch_k(attn_qkv_pack_kernel, dim3(4 * atp.q_tiles, nb), dim3(192), 0, st, ra, at_q, at_k, at_v, atp.q_tiles, atp.k_tiles, atp.v_blocks);
+		else
+			launch_k(qk_norm_rope_prefill_kernel, dim3(S_seq, nb), dim3(192), 0, st, ra);
 		count_launch();
 		// Two queries per CTA: what the tensor cores do not take. The 960 decides between the CUDA-core kernels where the tensor cores are
 		// switched off (prefill of 1400 tokens, two queries per CTA / long-prompt kernel, 1B and 270m: 7.9 / 9.0 and 4.0 / 4.8 ms, 2000: 11.6 / 11.2 and 6.0 / 5.8).
@@ -2166,22 +2169,13 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 				TG_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_TC_SMEM));
 				at_configured[dev] = true;
 			}
-			auto pack_rows = [&](const float *src, __nv_bfloat16 *dst, int rows, int tiles) {
-				const size_t chunks = size_t(tiles) * TC_BM * (256 / 8);
-				launch_k(split_pack_kernel, dim3(unsigned(std::min<size_t>((chunks + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0, st, src, dst, rows,
-				         256, tiles);
-				count_launch();
-			};
-			pack_rows(q, at_q, 4 * S_seq, atp.q_tiles);  // rows = (query, head) pairs as they lie in q [S][4][256]
-			pack_rows(k, at_k, S_seq, atp.k_tiles);
-			launch_k(attn_pack_v_kernel, dim3(unsigned(std::min<size_t>((size_t(atp.v_blocks) * 512 + 255) / 256, size_t(g_num_sms) * 16)), nb), dim3(256), 0,
-			         st, (const float *)v, at_v, S_seq, atp.v_blocks);
-			count_launch();
 			AttnTcArgs aa{};
 			aa.qp = at_q;
 			aa.kp = at_k;
 			aa.vp = at_v;
-			aa.o = ao;
+			aa.x = tc.x;
+			aa.rowscale = i8_rowscale(tc, S, qd);
+			aa.groups = i8_groups(S);
 			aa.S = S_seq;
 			aa.q_tiles = atp.q_tiles;
 			aa.k_tiles = atp.k_tiles;
@@ -2206,7 +2200,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		if (use_tc) {
 			// the O, up|gate and down GEMMs leave raw K-split partial sums; the kernel that consumes them adds the splits
 			int ns = 0;
-			if (!attn_small) TG_TRY(pack_activations(ao, S, qd, tc, st));
+			if (!attn_small && !attn_tc) TG_TRY(pack_activations(ao, S, qd, tc, st));
 			{
 				const QW *ws[1] = {&w.O};
 				TG_TRY(gemm_raw(1, ws, &ns));
