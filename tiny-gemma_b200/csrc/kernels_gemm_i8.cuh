@@ -243,42 +243,43 @@ __global__ void __launch_bounds__(256) qgemm_wide_rows_kernel(float *C, const fl
 // t is the partial sums of the GEMM before: t[d] = tscale[d] * sum_sp t[(sp * M + row) * dim + d], added in split order.
 // A row belongs to NT threads, its values stay in their registers (dim <= 4 * NT * PER). A row is a chain of dependent
 // round trips (loads, two reductions), so everything that does not depend on the partial sums is requested before them.
-//   NT = 288 (one CTA per row): a few hundred rows, all resident at once, the chain's length counts
+//   NT = 160, 288 (one CTA per row, a quad of values per thread): a few hundred rows, all resident at once, the chain's length
+//   counts, and with it the instructions: rows of 1152 took 3.1 us with two quads per thread, half of them idle, and the column scales requested late
 //   NT = 32  (one warp per row, 8 rows per CTA): thousands of rows; no barriers, shuffles only, more rows in flight
 template <int NT, int PER>
 __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *h, const float *t, const float *w_post, const float *w_pre, uint8_t *out,
                                                                          float *rowscale, int M, int dim, int groups, int nsplit,
                                                                          const float *tscale) {
 	constexpr int NW = NT / 32;
-	__shared__ float2 red[NT == 32 ? 1 : NW];
+	__shared__ float2 red[2][NT == 32 ? 1 : NW];  // (one per reduction: a barrier each)
 	const int lt = NT == 32 ? int(threadIdx.x & 31) : int(threadIdx.x);
 	const int row = NT == 32 ? int(blockIdx.x * 8 + (threadIdx.x >> 5)) : int(blockIdx.x);
 	const int n4 = dim / 4;
-	// sum of a, maximum of the bit patterns b over the row's threads
-	auto reduce = [&](float a, uint32_t b) -> float2 {
+	// sum of a, maximum of the bit patterns b over the row's threads; i: the first or the second reduction
+	auto reduce = [&](float a, uint32_t b, int i) -> float2 {
 		a = warp_sum(a);
 		b = warp_umax(b);
 		if (NT == 32) return make_float2(a, __uint_as_float(b));
-		__syncthreads();
-		if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_float2(a, __uint_as_float(b));
+		if ((threadIdx.x & 31) == 0) red[i][threadIdx.x >> 5] = make_float2(a, __uint_as_float(b));
 		__syncthreads();
 		float s = 0.0f;
 		uint32_t m = 0;
 #pragma unroll
 		for (int w = 0; w < NW; w++) {
-			s += red[w].x;
-			m = max(m, __float_as_uint(red[w].y));
+			s += red[i][w].x;
+			m = max(m, __float_as_uint(red[i][w].y));
 		}
 		return make_float2(s, __uint_as_float(m));
 	};
 	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-	float4 wpost[PER], wpre[PER];  // the weights are nobody's output: requested before the wait for the predecessor
+	float4 wpost[PER], wpre[PER], scl[PER];  // the weights are nobody's output: requested before the wait for the predecessor
 #pragma unroll
 	for (int j = 0; j < PER; j++) {
 		const int k4 = lt + NT * j;
-		wpost[j] = wpre[j] = z4;
+		wpost[j] = wpre[j] = scl[j] = z4;
 		if (NT != 32 && k4 < n4) {
 			if (t) wpost[j] = __ldg(reinterpret_cast<const float4 *>(w_post) + k4);
+			if (t) scl[j] = __ldg(reinterpret_cast<const float4 *>(tscale) + k4);
 			if (w_pre) wpre[j] = __ldg(reinterpret_cast<const float4 *>(w_pre) + k4);
 		}
 	}
@@ -299,8 +300,8 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 		for (int j = 0; j < PER; j++) acc[j] = z4;
 		const float4 *base = reinterpret_cast<const float4 *>(t + size_t(row) * dim);
 		const size_t stride = size_t(M) * n4;
-		constexpr int QB = NT == 32 ? 1 : 8;  // splits requested together
-		for (int s0 = 0; s0 < nsplit; s0 += QB) {
+		auto splits = [&](auto qb, int s0) {  // qb splits requested together
+			constexpr int QB = decltype(qb)::value;
 			float4 q[QB][PER];
 #pragma unroll
 			for (int i = 0; i < QB; i++)
@@ -316,13 +317,22 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 				for (int j = 0; j < PER; j++) {
 					acc[j].x += q[i][j].x; acc[j].y += q[i][j].y; acc[j].z += q[i][j].z; acc[j].w += q[i][j].w;
 				}
+		};
+		if (NT == 32 || PER > 2) {
+			for (int s0 = 0; s0 < nsplit; s0++) splits(std::integral_constant<int, 1>(), s0);
+		} else if (nsplit <= 4) {
+			splits(std::integral_constant<int, 4>(), 0);
+		} else if (PER == 1 && nsplit > 8) {
+			for (int s0 = 0; s0 < nsplit; s0 += 16) splits(std::integral_constant<int, PER == 1 ? 16 : 8>(), s0);
+		} else {
+			for (int s0 = 0; s0 < nsplit; s0 += 8) splits(std::integral_constant<int, 8>(), s0);
 		}
 		float ss = 0.0f;
 #pragma unroll
 		for (int j = 0; j < PER; j++) {
 			const int k4 = lt + NT * j;
 			if (k4 < n4) {
-				const float4 s4 = __ldg(reinterpret_cast<const float4 *>(tscale) + k4);
+				const float4 s4 = NT == 32 ? __ldg(reinterpret_cast<const float4 *>(tscale) + k4) : scl[j];
 				acc[j].x *= s4.x; acc[j].y *= s4.y; acc[j].z *= s4.z; acc[j].w *= s4.w;
 				ss = fmaf(acc[j].x, acc[j].x, ss);
 				ss = fmaf(acc[j].y, acc[j].y, ss);
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 				ss = fmaf(acc[j].w, acc[j].w, ss);
 			}
 		}
-		const float r = inv_rms(reduce(ss, 0u).x, dim);
+		const float r = inv_rms(reduce(ss, 0u, 0).x, dim);
 #pragma unroll
 		for (int j = 0; j < PER; j++) {
 			const int k4 = lt + NT * j;
@@ -359,7 +369,7 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 		mx = max(mx, max(max(i8_abs_bits(hv[j].x * (wpre[j].x + 1.0f)), i8_abs_bits(hv[j].y * (wpre[j].y + 1.0f))),
 		                 max(i8_abs_bits(hv[j].z * (wpre[j].z + 1.0f)), i8_abs_bits(hv[j].w * (wpre[j].w + 1.0f)))));
 	}
-	const float2 sm = reduce(ss, mx);
+	const float2 sm = reduce(ss, mx, 1);
 	const float r = inv_rms(sm.x, dim);
 	const uint32_t mb = i8_abs_bits(sm.y * r);
 	const float mul = i8_row_mul(mb);
@@ -381,6 +391,28 @@ __global__ void __launch_bounds__(NT == 32 ? 256 : NT) resnorm_i8_kernel(float *
 // up to GE_LUT entries is looked up in shared memory (32 lanes, 32 banks); through the L1 a gather of 32 entries
 // touches ~20 of the table's 32 lines, one after the other, which alone took 0.25 ms of 0.58 for 16384 x 6912.
 constexpr int GE_LUT = 2048;
+// lut(g * gs) * (u * us) of four columns: GeluLut::index, the four look-ups together and selected instead of branched on (int(x) >= 0
+// is x > -1; a branch per look-up made 3.6 us of 178 rows of 6912)
+__device__ __forceinline__ float4 ge_quad(const GeluLut &lut, const float *values, const float4 &g, const float4 &gs, const float4 &u, const float4 &us) {
+	const float v[4] = {g.x * gs.x, g.y * gs.y, g.z * gs.z, g.w * gs.w};
+	float x[4], y[4];
+	if (lut.inv != 0.0f) {
+		const float base = -(lut.mn * lut.inv);
+#pragma unroll
+		for (int i = 0; i < 4; i++) x[i] = fmaf(v[i], lut.inv, base);
+	} else {
+#pragma unroll
+		for (int i = 0; i < 4; i++) x[i] = (v[i] - lut.mn) / lut.eps;
+	}
+#pragma unroll
+	for (int i = 0; i < 4; i++) y[i] = values[min(max(int(x[i]), 0), lut.size - 1)];
+#pragma unroll
+	for (int i = 0; i < 4; i++) {
+		const float in = int(x[i]) < lut.size ? y[i] : v[i];
+		y[i] = x[i] > -1.0f && x[i] < 2147483648.0f ? in : 0.0f;
+	}
+	return make_float4(y[0] * (u.x * us.x), y[1] * (u.y * us.y), y[2] * (u.z * us.z), y[3] * (u.w * us.w));
+}
 template <int NT, int PER>
 __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_t *out, float *rowscale, int M, int I, int groups, GeluLut lut,
                                                       int nsplit, const float *su, const float *sg) {
@@ -399,12 +431,7 @@ __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_
 	__syncthreads();
 	pdl_trigger();
 	pdl_wait();
-	auto gelu = [&](float v) -> float {
-		int idx;
-		if (!lut.index(v, idx)) return 0.0f;
-		if (idx >= lut.size) return v;
-		return in_smem ? table[idx] : __ldg(lut.table + idx);
-	};
+	const float *const values = in_smem ? table : lut.table;
 	const size_t stride = size_t(M) * 2 * n4;
 	for (int row = blockIdx.x; row < M; row += gridDim.x) {
 		const float4 *base = reinterpret_cast<const float4 *>(ug + size_t(row) * 2 * I);
@@ -441,10 +468,7 @@ __global__ void __launch_bounds__(NT, 2) geglu_i8_kernel(const float *ug, uint8_
 		for (int j = 0; j < PER; j++) {
 			const int k4 = min(tid + NT * j, n4 - 1);
 			const float4 fs = PER == 1 ? fs0 : __ldg(reinterpret_cast<const float4 *>(su) + k4), gs = PER == 1 ? gs0 : __ldg(reinterpret_cast<const float4 *>(sg) + k4);
-			u[j].x = gelu(g[j].x * gs.x) * (u[j].x * fs.x);
-			u[j].y = gelu(g[j].y * gs.y) * (u[j].y * fs.y);
-			u[j].z = gelu(g[j].z * gs.z) * (u[j].z * fs.z);
-			u[j].w = gelu(g[j].w * gs.w) * (u[j].w * fs.w);
+			u[j] = ge_quad(lut, values, g[j], gs, u[j], fs);
 			mx = max(mx, max(max(i8_abs_bits(u[j].x), i8_abs_bits(u[j].y)), max(i8_abs_bits(u[j].z), i8_abs_bits(u[j].w))));
 		}
 		mx = block_umax<NT / 32>(mx, red);
@@ -485,12 +509,7 @@ __global__ void __launch_bounds__(NT) geglu_i8_stream_kernel(const float *ug, ui
 	__syncthreads();
 	pdl_trigger();
 	pdl_wait();
-	auto gelu = [&](float v) -> float {
-		int idx;
-		if (!lut.index(v, idx)) return 0.0f;
-		if (idx >= lut.size) return v;
-		return in_smem ? table[idx] : __ldg(lut.table + idx);
-	};
+	const float *const values = in_smem ? table : lut.table;
 	auto issue = [&](int i, int st) {  // the CTA's i-th row; warp 0, converged
 		const int row = blockIdx.x + i * gridDim.x;
 		if (row < M && tc_elect()) {
@@ -512,10 +531,7 @@ __global__ void __launch_bounds__(NT) geglu_i8_stream_kernel(const float *ug, ui
 		for (int j = 0; j < PER; j++) {
 			const int k4 = min(tid + NT * j, n4 - 1);
 			const float4 u = u4[k4], g = g4[k4];
-			v[j].x = gelu(g.x * gs[j].x) * (u.x * fs[j].x);
-			v[j].y = gelu(g.y * gs[j].y) * (u.y * fs[j].y);
-			v[j].z = gelu(g.z * gs[j].z) * (u.z * fs[j].z);
-			v[j].w = gelu(g.w * gs[j].w) * (u.w * fs[j].w);
+			v[j] = ge_quad(lut, values, g, gs[j], u, fs[j]);
 			mx = max(mx, max(max(i8_abs_bits(v[j].x), i8_abs_bits(v[j].y)), max(i8_abs_bits(v[j].z), i8_abs_bits(v[j].w))));
 		}
 		mx = block_umax<NT / 32>(mx, red);  // (its barriers: every thread has read the row)

@@ -1618,7 +1618,12 @@ int launch_resnorm(float *h, const float *t, const float *w_post, const float *w
                    const TcScratch &sc, cudaStream_t st, int plan_rows = 0) {
 	const int groups = i8_groups(M);
 	float *rs = i8_rowscale(sc, M, dim);
-	if ((plan_rows ? plan_rows : M) < 1024)
+	const bool few = (plan_rows ? plan_rows : M) < 1024;
+	if (few && dim <= 640)
+		launch_k(resnorm_i8_kernel<160, 1>, dim3(M), dim3(160), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	else if (few && dim <= 1152)
+		launch_k(resnorm_i8_kernel<288, 1>, dim3(M), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
+	else if (few)
 		launch_k(resnorm_i8_kernel<288, 2>, dim3(M), dim3(288), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
 	else if (dim <= 640)
 		launch_k(resnorm_i8_kernel<32, 5>, dim3(groups), dim3(256), 0, st, h, t, w_post, w_pre, sc.x, rs, M, dim, groups, nsplit, tscale);
