@@ -17,10 +17,6 @@
 
 namespace tg {
 
-constexpr int AC_KEYS = 32;
-constexpr int AC_BUF = AC_KEYS * 1024;  // bytes of a K or V chunk
-constexpr int AC_SMEM = 2 * AC_BUF;
-
 // N partial sums per lane (N = 16): afterwards lane L holds the warp's total of value L >> 1
 __device__ __forceinline__ float ac_reduce16(float (&t)[16], int lane) {
 #pragma unroll
@@ -134,38 +130,18 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	pdl_wait();
 	int pos = a.step_pos[b];
 	const int base = a.is_local ? a.ring_base[b] : 0;
-	float4 lo = z4, hi = z4;
-	if (warp < AT_NH + 2) {  // (in flight together with the position)
-		const float4 *p = reinterpret_cast<const float4 *>(a.qkv + size_t(b) * NQ + warp * AT_HD);
-		if (a.qkv_nsplit > 0) {
-			const size_t sstride = size_t(a.qkv_B) * (NQ / 4);
-			for (int sp = 0; sp < a.qkv_nsplit; sp += 4) {
-				float4 u[4], v[4];
+	// the projections' K-splits, QB of them in flight together with the position; they are added behind the requests for the cache
+	constexpr int QB = 10;
+	const float4 *qkv = reinterpret_cast<const float4 *>(a.qkv + size_t(b) * NQ + warp * AT_HD) + lane;
+	const size_t sstride = size_t(a.qkv_B) * (NQ / 4);
+	const int nsp = warp < AT_NH + 2 ? max(a.qkv_nsplit, 1) : 0;
+	float4 u[QB], v[QB];
 #pragma unroll
-				for (int q = 0; q < 4; q++) {
-					u[q] = v[q] = z4;
-					if (sp + q < a.qkv_nsplit) {
-						u[q] = p[size_t(sp + q) * sstride + lane];
-						v[q] = p[size_t(sp + q) * sstride + 32 + lane];
-					}
-				}
-#pragma unroll
-				for (int q = 0; q < 4; q++) {
-					lo.x += u[q].x;
-					lo.y += u[q].y;
-					lo.z += u[q].z;
-					lo.w += u[q].w;
-					hi.x += v[q].x;
-					hi.y += v[q].y;
-					hi.z += v[q].z;
-					hi.w += v[q].w;
-				}
-			}
-			lo = make_float4(lo.x * s0.x, lo.y * s0.y, lo.z * s0.z, lo.w * s0.w);
-			hi = make_float4(hi.x * s1.x, hi.y * s1.y, hi.z * s1.z, hi.w * s1.w);
-		} else {
-			lo = p[lane];
-			hi = p[32 + lane];
+	for (int q = 0; q < QB; q++) {
+		u[q] = v[q] = z4;
+		if (q < nsp) {
+			u[q] = qkv[size_t(q) * sstride];
+			v[q] = qkv[size_t(q) * sstride + 32];
 		}
 	}
 	int slot, valid;
@@ -197,11 +173,36 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	};
 #pragma unroll
 	for (int i = 0; i < AD_STAGES; i++) issue(i);
+	float4 lo = z4, hi = z4, c0 = z4, c1 = z4, n0 = z4, n1 = z4;
+	if (warp <= AT_NH) {
+		const float4 *cr = reinterpret_cast<const float4 *>(a.cosT + size_t(pos) * AT_HD), *sr = reinterpret_cast<const float4 *>(a.sinT + size_t(pos) * AT_HD);
+		c0 = cr[lane];
+		c1 = cr[32 + lane];
+		n0 = sr[lane];
+		n1 = sr[32 + lane];
+	}
+	auto add = [](float4 &x, const float4 &y) {
+		x.x += y.x;
+		x.y += y.y;
+		x.z += y.z;
+		x.w += y.w;
+	};
+#pragma unroll
+	for (int q = 0; q < QB; q++) {
+		add(lo, u[q]);
+		add(hi, v[q]);
+	}
+	for (int q = QB; q < nsp; q++) {
+		add(lo, qkv[size_t(q) * sstride]);
+		add(hi, qkv[size_t(q) * sstride + 32]);
+	}
+	if (a.qkv_nsplit > 0) {
+		lo = make_float4(lo.x * s0.x, lo.y * s0.y, lo.z * s0.z, lo.w * s0.w);
+		hi = make_float4(hi.x * s1.x, hi.y * s1.y, hi.z * s1.z, hi.w * s1.w);
+	}
 	if (warp <= AT_NH) {  // per-head norm and RoPE; lane owns d = 4 lane .. and the partners 128 + d
 		// the reference scales q by 1/sqrt(256) = 2^-4 before the dot products (ops.hpp:262,283)
 		const float qs = warp < AT_NH ? 0.0625f : 1.0f;
-		const float4 *cr = reinterpret_cast<const float4 *>(a.cosT + size_t(pos) * AT_HD), *sr = reinterpret_cast<const float4 *>(a.sinT + size_t(pos) * AT_HD);
-		const float4 c0 = cr[lane], c1 = cr[32 + lane], n0 = sr[lane], n1 = sr[32 + lane];
 		const float lov[4] = {lo.x, lo.y, lo.z, lo.w}, hiv[4] = {hi.x, hi.y, hi.z, hi.w};
 		const float wlo[4] = {w0.x, w0.y, w0.z, w0.w}, whi[4] = {w1.x, w1.y, w1.z, w1.w};
 		const float clo[4] = {c0.x, c0.y, c0.z, c0.w}, chi[4] = {c1.x, c1.y, c1.z, c1.w};
@@ -346,15 +347,15 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		__syncthreads();
 		if (!s_last) return;
 		__threadfence();
+		constexpr int PB = 16;  // parts requested together (8: 300 positions of three sequences in 10 parts 0.6 us a layer slower)
 		float M = -INFINITY;
-		for (int sp = 0; sp < nact; sp++) M = fmaxf(M, __ldcg(pb + size_t(sp) * AT_PART + AT_NH * AT_HD + h));
 		r = make_float4(0.f, 0.f, 0.f, 0.f);
 		L = 0.0f;
-		for (int s0 = 0; s0 < nact; s0 += 4) {
-			float4 v[4];
-			float ms[4], ls[4];
+		for (int s0 = 0; s0 < nact; s0 += PB) {
+			float4 v[PB];
+			float ms[PB], ls[PB], mn = M;
 #pragma unroll
-			for (int q = 0; q < 4; q++) {
+			for (int q = 0; q < PB; q++) {
 				v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 				ms[q] = -INFINITY;
 				ls[q] = 0.0f;
@@ -366,7 +367,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 				}
 			}
 #pragma unroll
-			for (int q = 0; q < 4; q++) {
+			for (int q = 0; q < PB; q++) mn = fmaxf(mn, ms[q]);
+			const float c = expf(M - mn);  // (0 for the first parts)
+			M = mn;
+			L *= c;
+			r = make_float4(r.x * c, r.y * c, r.z * c, r.w * c);
+#pragma unroll
+			for (int q = 0; q < PB; q++) {
 				const float w = expf(ms[q] - M);
 				L = fmaf(ls[q], w, L);
 				ac_fma4(r, w, v[q]);
@@ -388,195 +395,221 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 }
 
 // ------------------------------------------------------------------ prefill of short prompts
-// Two queries (8 rows of 4 heads) per CTA of 16 warps; the FMAs and the score reductions bound it (~920 issue slots per 32
-// keys and step), so products are packed two to an instruction. q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
+// Two queries (8 rows of 4 heads) per CTA of 16 warps. As in the decode kernel a warp takes 4 keys at a time against the four heads of
+// one query, with a running maximum of its own; warps g and g + 8 share the keys of group g, which arrive through a ring of the group.
+// Nothing in the walk waits for another group. Shared memory and shuffles (~1500 clk per 32 keys and two queries), FMAs (1100) and copies (64 KB) bound it.
+// q [S][1024], k and v [off + S][256] per prompt; blockIdx.y is the
 // prompt. Query s is the token at key off + s (off > 0: a continuation, its context comes first). Causal; on local layers
 // a query sees at most `window` keys before itself (the reference's prefill rule, ops.hpp:439-443).
-// A cluster of ks CTAs shares two queries, each with a part of their keys (a chunk of 32 keys is a chain of three barriers, ~2 us): the
-// first one joins the parts, in key order. attn_small_split: how many.
-constexpr int APS_THREADS = 512;
-// CTAs per two queries of a prompt of S tokens behind `off` others. By the prompt alone: a prompt of a group gets the bits that it
-// gets by itself. Two chunks of keys per CTA at least, and not many more CTAs than are resident (one per SM): 178 tokens 2,
-// 61 behind 1500 cached ones 6. (prefill of 178 tokens 1862 -> 1804 us)
-inline int attn_small_split(int S, int off, int is_local, int window) {
-	const int keys = is_local ? std::min(off + S, window + 2) : off + S;
-	return std::max(1, std::min(std::min(8, (keys + AC_KEYS - 1) / AC_KEYS / 2), 192 / ((S + 1) / 2)));
+// The CTAs of a cluster share the keys of two queries, and hand their parts to the first one, which joins them in order; where two queries have
+// so few keys that one CTA takes no longer for them than a share of the longest walk, every CTA of a cluster takes two queries of its own.
+// 178 tokens, the longest walk of a launch: 10.2 us with 32 keys at a time for all 16 warps between three barriers, 8.0 now, and no
+// second wave of CTAs (all walks shared by two: 178 CTAs).
+constexpr int APS_GROUPS = 8, APS_THREADS = 2 * 32 * APS_GROUPS;
+constexpr int APS_KEYS = 4, APS_STAGES = 3;  // keys of a step; K and V of so many steps in a group's ring
+constexpr int APS_BUF = APS_KEYS * 1024;
+constexpr int APS_RING = APS_GROUPS * APS_STAGES * 2 * APS_BUF;
+constexpr int APS_PART = 2 * AT_NH * AT_HD + 2 * 2 * AT_NH;  // floats that a CTA hands over: 8 rows, their maxima and sums
+constexpr int APS_MAX_KS = 5;                                // CTAs of a cluster (their parts lie beside the ring)
+// ks: CTAs of a cluster. shared: the clusters that share two queries each, those with the most keys
+struct AttnSmallPlan {
+	int ks, shared, clusters;
+	int smem() const { return APS_RING + (ks - 1) * APS_PART * 4; }
+};
+// For a prompt of S tokens behind `off` others. By the prompt alone: a prompt of a group gets the bits that it gets by itself. The largest cluster
+// with two rounds of 32 keys per CTA at least whose CTAs are all resident at once (one per SM; the SMs of a GPC hold whole clusters): 178 tokens 2, 61 behind 1500 cached ones 4.
+inline AttnSmallPlan attn_small_plan(int S, int off, int is_local, int window) {
+	constexpr int ROUND = APS_GROUPS * APS_KEYS, resident[APS_MAX_KS + 1] = {0, 148, 148, 138, 128, 115};
+	const int pairs = (S + 1) / 2, most = is_local ? std::min(off + S, window + 2) : off + S;
+	for (int ks = std::min(APS_MAX_KS, (most + ROUND - 1) / ROUND / 2); ks > 1; ks--) {
+		const int share = (most + ks * ROUND - 1) / (ks * ROUND) * ROUND;                // keys of a CTA of the longest walk
+		const int alone = most <= share ? pairs : std::min(pairs, std::max(0, share - off) / 2);  // pair i has off + 2 i + 2 keys
+		const int clusters = pairs - alone + (alone + ks - 1) / ks;
+		if (clusters * ks <= resident[ks]) return AttnSmallPlan{ks, pairs - alone, clusters};
+	}
+	return AttnSmallPlan{1, 0, pairs};
 }
 __device__ __forceinline__ uint32_t ac_mapa(const void *p, int rank) {
 	uint32_t r;
 	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
 	return r;
 }
-__device__ __forceinline__ float ac_remote(const float *p, int rank) {
-	float v;
-	asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ac_mapa(p, rank)) : "memory");
-	return v;
-}
-__device__ __forceinline__ float4 ac_remote4(const float4 *p, int rank) {
-	float4 v;
-	asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ac_mapa(p, rank)) : "memory");
-	return v;
-}
 __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
                                                                             const float *k, const float *v, int S, int off, int is_local, int window,
-                                                                            int ks, int *err) {
+                                                                            int cluster, int shared, int *err) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
-	constexpr int R = 8;  // query rows
-	__shared__ __align__(16) float sc[AC_KEYS][R], pr[AC_KEYS][R];
-	__shared__ float corr_s[R], l_s[R], m_s[R];
-	__shared__ uint64_t kbar, vbar;
+	constexpr int R = 2 * AT_NH, H = AT_NH;  // query rows: query * 4 + head
+	__shared__ float m_s[APS_GROUPS][R], l_s[APS_GROUPS][R];
+	__shared__ uint64_t full[APS_GROUPS][APS_STAGES], done[APS_GROUPS][APS_STAGES];  // a step's keys and values landed; both warps have read them
 	__shared__ uint32_t red[APS_THREADS / 32];
-	float *K = reinterpret_cast<float *>(ac_smem), *V = reinterpret_cast<float *>(ac_smem + AC_BUF);
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	if (tid == 0) {
-		mbar_init(&kbar, 1);
-		mbar_init(&vbar, 1);
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = warp & (APS_GROUPS - 1), qi = warp / APS_GROUPS;  // this warp's query
+	uint8_t *ring = ac_smem + grp * (APS_STAGES * 2 * APS_BUF);
+	if (tid < APS_GROUPS * APS_STAGES) {
+		mbar_init(&full[0][0] + tid, 1);
+		mbar_init(&done[0][0] + tid, 2);
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	__syncthreads();
+	if (cluster > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");  // (waited for before anything is handed over)
 	pdl_trigger();
 	pdl_wait();
 	const size_t r0 = size_t(blockIdx.y) * S;
-	const int rank = ks > 1 ? int(blockIdx.x) % ks : 0;  // of the cluster's CTAs
-	const int s0 = (int(gridDim.x) / ks - 1 - int(blockIdx.x) / ks) * 2;  // (the longest walks start first)
+	// the cluster's queries (the longest walks start first), among how many CTAs they are shared, and which of them this one is
+	const int c = int(blockIdx.x) / cluster, last = (S + 1) / 2 - 1;
+	const int ks = c < shared ? cluster : 1, rank = ks > 1 ? int(blockIdx.x) % cluster : 0;
+	const int pair = last - (c < shared ? c : shared + (c - shared) * cluster + int(blockIdx.x) % cluster), s0 = 2 * max(pair, 0);
 	const int s_last = min(S - 1, s0 + 1);
 	const int j0 = (is_local && off + s0 >= window) ? off + s0 - window : 0, j1 = off + s_last + 1;
-	// this CTA's chunks: c_lo .. c_lo + nch - 1 of all
-	const int all = (j1 - j0 + AC_KEYS - 1) / AC_KEYS, c_lo = all * rank / ks, nch = all * (rank + 1) / ks - c_lo;
-	k += (r0 + j0) * 256;  // (a continuation is one sequence: r0 = 0)
-	v += (r0 + j0) * 256;
-	auto issue = [&](float *dst, const float *src, int c, uint64_t *bar) {
-		c += c_lo;
-		const uint32_t bytes = uint32_t(min(AC_KEYS, j1 - j0 - c * AC_KEYS)) * 1024u;
-		fence_proxy_async();
-		mbar_expect_tx(bar, bytes);
-		bulk_load(dst, src + size_t(c) * AC_KEYS * 256, bytes, bar);
+	// steps of four keys are dealt out to all groups of the cluster in turn: this group's first key, the distance to its next, how many steps
+	const int jw = j0 + APS_KEYS * (rank * APS_GROUPS + grp), jd = APS_KEYS * APS_GROUPS * ks, nit = pair < 0 ? 0 : max(0, (j1 - jw + jd - 1) / jd);
+	k += r0 * 256;  // (a continuation is one sequence: r0 = 0)
+	v += r0 * 256;
+	auto issue = [&](int i) {  // step i of the group; called by the whole warp
+		const int j = jw + i * jd, st = i % APS_STAGES;
+		if (i < nit && tc_elect()) {
+			const uint32_t bytes = uint32_t(min(APS_KEYS, j1 - j)) * 1024u;
+			mbar_expect_tx(&full[grp][st], 2 * bytes);
+			bulk_load(ring + st * 2 * APS_BUF, k + size_t(j) * 256, bytes, &full[grp][st]);
+			bulk_load(ring + st * 2 * APS_BUF + APS_BUF, v + size_t(j) * 256, bytes, &full[grp][st]);
+		}
 	};
-	if (tid == 0 && nch > 0) {
-		issue(K, k, 0, &kbar);
-		issue(V, v, 0, &vbar);
+	if (qi == 0) {
+#pragma unroll
+		for (int i = 0; i < APS_STAGES; i++) issue(i);
 	}
-	// row = query * 4 + head
-	float4 q0[R], q1[R];
+	// A lane keeps the heads, and the keys of a step, in an order of its own for the scores (slot ^ hperm, slot ^ kperm): every round of the
+	// reduce-scatter then keeps the lower and sends the upper slots, without selects.
+	const int hperm = (lane >> 1) & 3, kperm = lane >> 3;
+	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+	float4 q0[H], q1[H], o0[H], o1[H];  // lane: dimensions 4 lane .. and 128 + 4 lane ..
+	{
+		// (a query past the prompt's end repeats the last one; it is not stored)
+		const float4 *qr = reinterpret_cast<const float4 *>(q + (r0 + min(s0 + qi, S - 1)) * 1024) + lane;
 #pragma unroll
-	for (int r = 0; r < R; r++) {
-		const int s = s0 + (r >> 2);
-		q0[r] = q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-		if (s < S) {
-			const float4 *qr = reinterpret_cast<const float4 *>(q + (r0 + s) * 1024 + (r & 3) * 256);
-			q0[r] = qr[lane];
-			q1[r] = qr[32 + lane];
+		for (int h = 0; h < H; h++) {
+			q0[h] = qr[(h ^ hperm) * 64];
+			q1[h] = qr[(h ^ hperm) * 64 + 32];
+			o0[h] = o1[h] = z4;
 		}
-		// exact: the reference scales q by 1/sqrt(256) = 2^-4 before the dot products
-		q0[r].x *= 0.0625f; q0[r].y *= 0.0625f; q0[r].z *= 0.0625f; q0[r].w *= 0.0625f;
-		q1[r].x *= 0.0625f; q1[r].y *= 0.0625f; q1[r].z *= 0.0625f; q1[r].w *= 0.0625f;
 	}
-	const int d4 = tid & 63, kg = tid >> 6;  // 8 groups of 4 keys
-	float4 o[R];
 #pragma unroll
-	for (int r = 0; r < R; r++) o[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-	float m = -INFINITY, l = 0.0f;  // of row `warp` (warps 0..7)
-	for (int c = 0; c < nch; c++) {
-		const int base = j0 + (c_lo + c) * AC_KEYS, n = min(AC_KEYS, j1 - base);
-		tc_wait(&kbar, c & 1, err);
-		{
-			float t[16];
+	for (int h = 0; h < H; h++) {  // exact: the reference scales q by 1/sqrt(256) = 2^-4 before the dot products
+		q0[h].x *= 0.0625f; q0[h].y *= 0.0625f; q0[h].z *= 0.0625f; q0[h].w *= 0.0625f;
+		q1[h].x *= 0.0625f; q1[h].y *= 0.0625f; q1[h].z *= 0.0625f; q1[h].w *= 0.0625f;
+	}
+	float m = -INFINITY, l = 0.0f;  // of head hperm; this lane's score of a step is key kperm's
+	const int mine = off + s0 + qi, first = is_local ? mine - window : 0;  // the query's own key, the first one that it sees
+	int cap = TC_SPIN_CAP;
+	for (int it = 0; it < nit; it++) {
+		const int j = jw + it * jd, n = min(APS_KEYS, j1 - j), st = it % APS_STAGES, ph = it / APS_STAGES & 1;
+		const uint8_t *K = ring + st * 2 * APS_BUF, *V = K + APS_BUF;
+		tc_wait_cap(&full[grp][st], ph, cap);
+		float t[16];
 #pragma unroll
-			for (int kk = 0; kk < 2; kk++) {
-				const float4 k0 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 4 * lane);
-				const float4 k1 = *reinterpret_cast<const float4 *>(K + (2 * warp + kk) * 256 + 128 + 4 * lane);
+		for (int kk = 0; kk < APS_KEYS; kk++) {  // (rows past n hold an older step's keys, or nothing yet: their scores are not used)
+			const uint8_t *kr = K + (kk ^ kperm) * 1024 + 16 * lane;
+			const float4 k0 = *reinterpret_cast<const float4 *>(kr), k1 = *reinterpret_cast<const float4 *>(kr + 512);
 #pragma unroll
-				for (int r = 0; r < R; r++) t[kk * 8 + r] = ac_dot8x2(q0[r], q1[r], k0, k1);
-			}
-			const float z = ac_reduce16(t, lane);
-			if (!(lane & 1)) sc[2 * warp + (lane >> 4)][(lane >> 1) & 7] = z;
+			for (int h = 0; h < H; h++) t[kk * H + h] = ac_dot8x2(q0[h], q1[h], k0, k1);
 		}
-		__syncthreads();  // scores complete, K consumed
-		if (tid == 0 && c + 1 < nch) issue(K, k, c + 1, &kbar);
-		if (warp < R) {
-			const int s = off + s0 + (warp >> 2), j = base + lane;
-			const bool vis = lane < n && j <= s && !(is_local && j + window < s);
-			const float z = vis ? sc[lane][warp] : -INFINITY;
-			const float mn = fmaxf(m, warp_max(z));
-			// (a row may have no visible key in its first chunk: the second query's window starts one later)
-			const float p = vis ? expf(z - mn) : 0.0f, cr = m == -INFINITY ? 0.0f : expf(m - mn);
-			l = fmaf(l, cr, warp_sum(p));
-			m = mn;
-			pr[lane][warp] = p;
-			if (lane == 0) corr_s[warp] = cr;
-		}
-		tc_wait(&vbar, c & 1, err);
-		__syncthreads();  // probabilities complete
+		// the partner's lane differs in the bit that the round splits on: its upper slot is the key and head of this lane's lower one
 #pragma unroll
-		for (int r = 0; r < R; r++) {
-			const float cr = corr_s[r];
-			o[r].x *= cr;
-			o[r].y *= cr;
-			o[r].z *= cr;
-			o[r].w *= cr;
-		}
+		for (int o = 8; o >= 1; o >>= 1)
 #pragma unroll
-		for (int kk = 0; kk < AC_KEYS / 8; kk++) {
-			const int key = kg * (AC_KEYS / 8) + kk;
-			if (key < n) {
-				const float4 vv = *reinterpret_cast<const float4 *>(V + key * 256 + 4 * d4);
-				const float4 pa = *reinterpret_cast<const float4 *>(&pr[key][0]), pb = *reinterpret_cast<const float4 *>(&pr[key][4]);
-				ac_fma4x2(o[0], pa.x, vv);
-				ac_fma4x2(o[1], pa.y, vv);
-				ac_fma4x2(o[2], pa.z, vv);
-				ac_fma4x2(o[3], pa.w, vv);
-				ac_fma4x2(o[4], pb.x, vv);
-				ac_fma4x2(o[5], pb.y, vv);
-				ac_fma4x2(o[6], pb.z, vv);
-				ac_fma4x2(o[7], pb.w, vv);
+			for (int i = 0; i < o; i++) t[i] += __shfl_xor_sync(0xffffffffu, t[i + o], 2 * o);
+		t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
+		const int key = j + kperm;
+		const bool vis = kperm < n && key <= mine && key >= first;
+		const float z = vis ? t[0] : -INFINITY;
+		float mn = fmaxf(m, z);
+		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 8));
+		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 16));
+		// (no key may be visible yet: the window starts later, or the step lies behind the query)
+		const float p = vis ? expf(z - mn) : 0.0f, cr = m == mn ? 1.0f : expf(m - mn);
+		float ps = p + __shfl_xor_sync(0xffffffffu, p, 8);
+		ps += __shfl_xor_sync(0xffffffffu, ps, 16);
+		l = fmaf(l, cr, ps);
+		m = mn;
+		if (__any_sync(0xffffffffu, cr != 1.0f)) {
+#pragma unroll
+			for (int h = 0; h < H; h++) {
+				const float c = __shfl_sync(0xffffffffu, cr, 2 * h);
+				o0[h] = make_float4(o0[h].x * c, o0[h].y * c, o0[h].z * c, o0[h].w * c);
+				o1[h] = make_float4(o1[h].x * c, o1[h].y * c, o1[h].z * c, o1[h].w * c);
 			}
 		}
-		__syncthreads();  // V consumed
-		if (tid == 0 && c + 1 < nch) issue(V, v, c + 1, &vbar);
+#pragma unroll
+		for (int kk = 0; kk < APS_KEYS; kk++) {
+			if (kk < n) {
+				const float4 v0 = *reinterpret_cast<const float4 *>(V + kk * 1024 + 16 * lane), v1 = *reinterpret_cast<const float4 *>(V + kk * 1024 + 512 + 16 * lane);
+#pragma unroll
+				for (int h = 0; h < H; h++) {
+					const float w = __shfl_sync(0xffffffffu, p, 8 * kk + 2 * h);
+					ac_fma4x2(o0[h], w, v0);
+					ac_fma4x2(o1[h], w, v1);
+				}
+			}
+		}
+		__syncwarp();
+		if (it + APS_STAGES < nit) {
+			if (lane == 0) mbar_arrive(&done[grp][st]);
+			if (qi == 0) {  // (its other warp is about as far)
+				tc_wait_cap(&done[grp][st], ph, cap);
+				issue(it + APS_STAGES);
+			}
+		}
 	}
-	// ---- join the eight key groups (64 KB: both buffers); thread (query, k4) ends up with 4 of its query's 1024 outputs
+	if (cap == 0) *static_cast<volatile int *>(err) = 6;
+	// ---- join the groups: thread (query, k4) ends up with four of its query's 1024 outputs
+	__syncthreads();  // (every warp has read its ring)
 	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
 #pragma unroll
-	for (int r = 0; r < R; r++) jb[(kg * R + r) * 64 + d4] = o[r];
-	if (warp < R && lane == 0) {
-		l_s[warp] = l;
-		m_s[warp] = m;
+	for (int h = 0; h < H; h++) {
+		jb[(grp * R + qi * H + h) * 64 + lane] = o0[h];
+		jb[(grp * R + qi * H + h) * 64 + 32 + lane] = o1[h];
+	}
+	if (lane < 2 * H && !(lane & 1)) {
+		m_s[grp][qi * H + (lane >> 1)] = m;
+		l_s[grp][qi * H + (lane >> 1)] = l;
 	}
 	__syncthreads();
-	const int qi = tid >> 8, k4 = tid & 255, row = qi * 4 + (k4 >> 6);
-	float4 r = jb[row * 64 + (k4 & 63)];
+	const int k4 = tid & 255, row = tid >> 6;  // (query tid / 256 is the warp's own)
+	float M = -INFINITY, L = 0.0f;
 #pragma unroll
-	for (int g = 1; g < 8; g++) {
-		const float4 t = jb[(g * R + row) * 64 + (k4 & 63)];
-		r.x += t.x;
-		r.y += t.y;
-		r.z += t.z;
-		r.w += t.w;
+	for (int g = 0; g < APS_GROUPS; g++) M = fmaxf(M, m_s[g][row]);
+	float4 r = z4;
+#pragma unroll
+	for (int g = 0; g < APS_GROUPS; g++) {
+		const float mg = m_s[g][row], w = mg == -INFINITY ? 0.0f : expf(mg - M);
+		L = fmaf(l_s[g][row], w, L);
+		ac_fma4(r, w, jb[(g * R + row) * 64 + (k4 & 63)]);
 	}
-	float L = l_s[row];
-	if (ks > 1) {  // the other CTAs' parts, through the cluster's shared memory, in key order
-		float4 *mine = jb;
-		__syncthreads();  // (the key groups have been read)
-		mine[tid] = r;
-		i8_cluster_sync();
-		if (rank == 0) {
-			float M = m_s[row];
-#pragma unroll 1
-			for (int p = 1; p < ks; p++) {
-				const float pm = ac_remote(&m_s[row], p), pl = ac_remote(&l_s[row], p);
-				if (pm == -INFINITY) continue;  // (no key of its chunks is visible)
-				const float4 o4 = ac_remote4(&mine[tid], p);
-				const float mn = fmaxf(M, pm), ea = M == -INFINITY ? 0.0f : expf(M - mn), eb = expf(pm - mn);
-				L = fmaf(L, ea, pl * eb);
-				r.x = fmaf(r.x, ea, o4.x * eb);
-				r.y = fmaf(r.y, ea, o4.y * eb);
-				r.z = fmaf(r.z, ea, o4.z * eb);
-				r.w = fmaf(r.w, ea, o4.w * eb);
-				M = mn;
-			}
+	if (cluster > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+	if (pair < 0) return;
+	if (ks > 1) {  // the other CTAs' parts lie behind the first one's ring, rows and then maxima and sums
+		const float *in = reinterpret_cast<const float *>(ac_smem + APS_RING);
+		if (rank != 0) {
+			const uint32_t dst = ac_mapa(in + (rank - 1) * APS_PART, 0);
+			asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * tid), "f"(r.x), "f"(r.y), "f"(r.z), "f"(r.w) : "memory");
+			if ((k4 & 63) == 0)
+				asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + 4u * (R * AT_HD) + 8u * row), "f"(M), "f"(L) : "memory");
 		}
-		i8_cluster_sync();  // (nobody leaves while its memory is read)
+		asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 		if (rank != 0) return;
+#pragma unroll 1
+		for (int p = 0; p < ks - 1; p++, in += APS_PART) {
+			const float4 o4 = reinterpret_cast<const float4 *>(in)[tid];
+			const float2 ml = reinterpret_cast<const float2 *>(in + R * AT_HD)[row];
+			const float mn = fmaxf(M, ml.x);
+			if (mn == -INFINITY) continue;  // (no key of either is visible)
+			const float ea = expf(M - mn), eb = expf(ml.x - mn);
+			L = fmaf(L, ea, ml.y * eb);
+			r.x = fmaf(r.x, ea, o4.x * eb);
+			r.y = fmaf(r.y, ea, o4.y * eb);
+			r.z = fmaf(r.z, ea, o4.z * eb);
+			r.w = fmaf(r.w, ea, o4.w * eb);
+			M = mn;
+		}
 	}
 	r.x /= L;
 	r.y /= L;

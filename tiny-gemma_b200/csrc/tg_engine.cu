@@ -2161,12 +2161,12 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			static bool as_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
 			if (!as_configured[dev]) {
-				TG_CUDA(cudaFuncSetAttribute(attn_prefill_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM));
+				TG_CUDA(cudaFuncSetAttribute(attn_prefill_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmallPlan{APS_MAX_KS, 0, 0}.smem()));
 				as_configured[dev] = true;
 			}
-			const int ks = attn_small_split(S_seq, off, w.is_local ? 1 : 0, window);
-			launch_clusters(ks, attn_prefill_small_kernel, dim3((S_seq + 1) / 2 * ks, nb), dim3(APS_THREADS), AC_SMEM, st, ao, use_tc ? tc.x : nullptr,
-			                use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, ks, s->err_flag);
+			const AttnSmallPlan ap = attn_small_plan(S_seq, off, w.is_local ? 1 : 0, window);
+			launch_clusters(ap.ks, attn_prefill_small_kernel, dim3(ap.clusters * ap.ks, nb), dim3(APS_THREADS), ap.smem(), st, ao, use_tc ? tc.x : nullptr,
+			                use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, ap.ks, ap.shared, s->err_flag);
 		} else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
