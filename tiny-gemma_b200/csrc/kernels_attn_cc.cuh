@@ -59,6 +59,11 @@ __device__ __forceinline__ void ac_fma4(float4 &o, float p, const float4 &v) {
 	o.w = fmaf(p, v.w, o.w);
 }
 
+__device__ __forceinline__ uint32_t ac_mapa(const void *p, int rank) {
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+	return r;
+}
 // ------------------------------------------------------------------ decode: one query per sequence
 struct AttnArgs {
 	const float *qkv;   // [B][1536] = q(4x256) | k(256) | v(256)
@@ -82,7 +87,7 @@ struct AttnArgs {
 	uint8_t *x;         // the digits of the result (K = 1024) and their row scales
 	float *rowscale;
 	int groups;
-	int nsplit;
+	int nsplit, cluster;  // CTAs per sequence, and how many of them form a cluster (1: none)
 	int *err_flag;
 };
 constexpr int AT_THREADS = 256;
@@ -96,6 +101,12 @@ constexpr int AD_KEYS = 4, AD_ROUND = AD_KEYS * AT_THREADS / 32;
 constexpr int AD_BUF = AD_KEYS * 1024;
 constexpr int AD_STAGES = 3;
 constexpr int AD_SMEM = AT_THREADS / 32 * AD_STAGES * AD_BUF;
+// Few sequences: the splits of a sequence are clusters of CTAs, whose parts meet in the first one's shared memory; only where a cache takes more than
+// one cluster do parts go through memory and a ticket (a store, a fence, an atomic and a load, one behind the other: 1.5 us).
+// Steps of the 270m model in us, through memory against in clusters: 3 sequences of 61 positions 464 / 430, of 500 510 / 466, of 6000 540 / 483; 16 of 61
+// 501 / 487, but 16 of 500 539 / 589 (one CTA per SM): up to 8 sequences.
+constexpr int AD_CLUSTER = 8, AD_CLUSTER_SEQS = 8;
+inline int attn_decode_smem(int cluster) { return AD_SMEM + (cluster - 1) * AT_PART * 4; }
 
 __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
@@ -104,14 +115,18 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	__shared__ uint64_t full[AT_THREADS / 32][AD_STAGES];
 	__shared__ uint32_t red[AT_THREADS / 32];
 	__shared__ int s_last;
-	const int b = blockIdx.y, split = blockIdx.x;
+	__shared__ uint64_t joined;  // (of a cluster's first CTA) every warp of the others has handed over its part, or has none
+	const int b = blockIdx.y, split = blockIdx.x, rank = a.cluster > 1 ? split % AD_CLUSTER : 0;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	pdl_trigger();
 	uint8_t *ring = ac_smem + warp * (AD_STAGES * AD_BUF);
 	if (lane == 0) {
 		for (int i = 0; i < AD_STAGES; i++) mbar_init(&full[warp][i], 1);
+		if (warp == 0) mbar_init(&joined, (AD_CLUSTER - 1) * (AT_THREADS / 32));
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	__syncwarp();
+	if (a.cluster > 1) i8_cluster_sync();
 	// the weights are nobody's output: requested before the wait for the predecessor. Warps 0..3: a head of q, 4: k, 5: v
 	constexpr int NQ = AT_NH * AT_HD + 2 * AT_HD;
 	const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -126,7 +141,6 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		s0 = __ldg(scl + lane);
 		s1 = __ldg(scl + 32 + lane);
 	}
-	pdl_trigger();
 	pdl_wait();
 	int pos = a.step_pos[b];
 	const int base = a.is_local ? a.ring_base[b] : 0;
@@ -144,21 +158,25 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 			v[q] = qkv[size_t(q) * sstride + 32];
 		}
 	}
-	int slot, valid;
-	if (a.is_local) {
-		slot = (pos - base) % a.slots;
-		valid = min(pos + 1, a.slots);
-	} else {
-		if (pos >= a.slots) {  // cache full: refuse to write out of bounds
-			if (tid == 0) *a.err_flag = 2;
-			pos = a.slots - 1;
-		}
-		slot = pos;
-		valid = pos + 1;
+	int valid = min(pos + 1, a.slots);
+	if (!a.is_local && pos >= a.slots) {  // cache full: refuse to write out of bounds
+		if (tid == 0) *a.err_flag = 2;
+		pos = a.slots - 1;
 	}
 	// whole rounds of 32 keys are dealt out to the splits; splits without any leave at once
-	const int rounds = (valid + AD_ROUND - 1) / AD_ROUND, per = (rounds + a.nsplit - 1) / a.nsplit, nact = (rounds + per - 1) / per;
-	if (split >= nact) return;
+	const int rounds = (valid + AD_ROUND - 1) / AD_ROUND;
+	int per = 1, nact = rounds;
+	if (rounds > a.nsplit) {
+		per = (rounds + a.nsplit - 1) / a.nsplit;
+		nact = (rounds + per - 1) / per;
+	}
+	auto hand_over = [&](uint32_t count) {  // to the cluster's first CTA
+		asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(ac_mapa(&joined, 0)), "r"(count) : "memory");
+	};
+	if (split >= nact) {
+		if (a.cluster > 1 && split - rank < nact && tid == 0) hand_over(AT_THREADS / 32);
+		return;
+	}
 	const int j0 = split * per * AD_ROUND, j1 = min(valid, j0 + per * AD_ROUND);
 	const int jw = j0 + AD_KEYS * warp, nit = max(0, (j1 - jw + AD_ROUND - 1) / AD_ROUND);  // this warp's first key, its groups of keys
 	float *kc = a.kcache + size_t(b) * a.slots * AT_HD, *vc = a.vcache + size_t(b) * a.slots * AT_HD;
@@ -173,6 +191,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	};
 #pragma unroll
 	for (int i = 0; i < AD_STAGES; i++) issue(i);
+	const int slot = a.is_local ? (pos - base) % a.slots : pos;
 	float4 lo = z4, hi = z4, c0 = z4, c1 = z4, n0 = z4, n1 = z4;
 	if (warp <= AT_NH) {
 		const float4 *cr = reinterpret_cast<const float4 *>(a.cosT + size_t(pos) * AT_HD), *sr = reinterpret_cast<const float4 *>(a.sinT + size_t(pos) * AT_HD);
@@ -333,9 +352,39 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		L = fmaf(l_s[g][h], w, L);
 		ac_fma4(r, w, jb[(g * AT_NH + h) * 64 + d4]);
 	}
-	if (nact > 1) {
+	int nparts = nact, part = split;
+	if (a.cluster > 1) {
+		float *in = reinterpret_cast<float *>(ac_smem + AD_SMEM);  // the other CTAs' parts, laid out as in memory
+		if (rank != 0) {
+			const uint32_t dst = ac_mapa(in + (rank - 1) * AT_PART, 0);
+			asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * tid), "f"(r.x), "f"(r.y), "f"(r.z), "f"(r.w) : "memory");
+			if (d4 == 0)
+				asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + 4u * (AT_NH * AT_HD) + 8u * h), "f"(Ms), "f"(L) : "memory");
+			__syncwarp();
+			if (lane == 0) hand_over(1);
+			return;
+		}
+		uint32_t ok = 0;
+		for (int z = 0; !ok && z < TC_SPIN_CAP; z++)
+			asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(&joined)) : "memory");
+		if (!ok) *static_cast<volatile int *>(a.err_flag) = 6;
+		const int n = min(AD_CLUSTER, nact - split);
+#pragma unroll 1
+		for (int p = 1; p < n; p++, in += AT_PART) {  // (every part has a key)
+			const float4 o4 = reinterpret_cast<const float4 *>(in)[tid];
+			const float2 ml = reinterpret_cast<const float2 *>(in + AT_NH * AT_HD)[h];
+			const float mn = fmaxf(Ms, ml.x), ea = expf(Ms - mn), eb = expf(ml.x - mn);
+			L = fmaf(L, ea, ml.y * eb);
+			r = make_float4(r.x * ea, r.y * ea, r.z * ea, r.w * ea);
+			ac_fma4(r, eb, o4);
+			Ms = mn;
+		}
+		nparts = (nact + AD_CLUSTER - 1) / AD_CLUSTER;
+		part = split / AD_CLUSTER;
+	}
+	if (nparts > 1) {
 		float *pb = a.part + size_t(b) * a.nsplit * AT_PART;
-		float *prow = pb + size_t(split) * AT_PART;
+		float *prow = pb + size_t(part) * AT_PART;
 		__stcg(reinterpret_cast<float4 *>(prow) + tid, r);
 		if (d4 == 0) {
 			__stcg(prow + AT_NH * AT_HD + h, Ms);
@@ -343,7 +392,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		}
 		__threadfence();
 		__syncthreads();
-		if (tid == 0) s_last = atomicAdd(&a.tickets[b], 1u) == unsigned(nact - 1);
+		if (tid == 0) s_last = atomicAdd(&a.tickets[b], 1u) == unsigned(nparts - 1);
 		__syncthreads();
 		if (!s_last) return;
 		__threadfence();
@@ -351,7 +400,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		float M = -INFINITY;
 		r = make_float4(0.f, 0.f, 0.f, 0.f);
 		L = 0.0f;
-		for (int s0 = 0; s0 < nact; s0 += PB) {
+		for (int s0 = 0; s0 < nparts; s0 += PB) {
 			float4 v[PB];
 			float ms[PB], ls[PB], mn = M;
 #pragma unroll
@@ -359,7 +408,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 				v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 				ms[q] = -INFINITY;
 				ls[q] = 0.0f;
-				if (s0 + q < nact) {
+				if (s0 + q < nparts) {
 					const float *p = pb + size_t(s0 + q) * AT_PART;
 					v[q] = __ldcg(reinterpret_cast<const float4 *>(p) + tid);
 					ms[q] = __ldcg(p + AT_NH * AT_HD + h);
@@ -428,11 +477,6 @@ inline AttnSmallPlan attn_small_plan(int S, int off, int is_local, int window) {
 		if (clusters * ks <= resident[ks]) return AttnSmallPlan{ks, pairs - alone, clusters};
 	}
 	return AttnSmallPlan{1, 0, pairs};
-}
-__device__ __forceinline__ uint32_t ac_mapa(const void *p, int rank) {
-	uint32_t r;
-	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-	return r;
 }
 __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
                                                                             const float *k, const float *v, int S, int off, int is_local, int window,

@@ -556,13 +556,14 @@ int state_alloc(tg_state *s) {
 	TG_CUDA(cudaMemsetAsync(s->attn_tickets, 0, sizeof(unsigned) * B, s->stream));
 	// split-KV factor: as many CTAs (batch x splits) as are resident at once, two per SM. More would queue behind them, and
 	// every split repeats the q/k norm + RoPE and adds a partial to merge (step of 32 sequences of 600 tokens with 4, 8 and
-	// 16 splits: 1434, 1415, 1646 us; of 256 sequences of 178 with 1 and 2: 2427, 2721 us)
+	// 16 splits: 1434, 1415, 1646 us; of 256 sequences of 178 with 1 and 2: 2427, 2721 us). Few sequences: as many clusters as are resident, one for a ring.
 	auto pick_split = [&](int cap) {
+		if (B <= AD_CLUSTER_SEQS) return std::min(cap / AD_CLUSTER, std::max(1, 16 / B)) * AD_CLUSTER;
 		int ns = 1;
 		while (ns < cap && 2 * B * ns <= 2 * g_num_sms) ns *= 2;
 		return ns;
 	};
-	s->attn_nsplit_local = env_int("TG_ATTN_SPLIT_LOCAL", pick_split(16));
+	s->attn_nsplit_local = env_int("TG_ATTN_SPLIT_LOCAL", pick_split(B <= AD_CLUSTER_SEQS ? AD_CLUSTER : 16));
 	s->attn_nsplit_global = env_int("TG_ATTN_SPLIT_GLOBAL", pick_split(64));
 	int nsmax = std::max(s->attn_nsplit_local, s->attn_nsplit_global);
 	TG_TRY(allocf(&s->attn_part, size_t(B) * nsmax * (AT_NH * AT_HD + 8)));
@@ -604,14 +605,37 @@ int check_ready(const tg_model *m) {
 	return TG_OK;
 }
 
-int launch_attn_decode(const AttnArgs &a, int nb, cudaStream_t st) {
+// launch_k in clusters of `size` CTAs
+template <typename... KArgs, typename... Args>
+inline void launch_clusters(int size, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cudaLaunchAttribute at[2];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = size;
+	at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[1].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = use_pdl() ? 2 : 1;
+	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
+}
+
+int launch_attn_decode(AttnArgs a, int nb, cudaStream_t st) {
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AD_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_decode_smem(AD_CLUSTER)));
 		configured[dev] = true;
 	}
-	launch_k(attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), AD_SMEM, st, a);
+	a.cluster = nb <= AD_CLUSTER_SEQS && a.nsplit % AD_CLUSTER == 0 ? AD_CLUSTER : 1;
+	if (a.cluster > 1)
+		launch_clusters(AD_CLUSTER, attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), attn_decode_smem(AD_CLUSTER), st, a);
+	else
+		launch_k(attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), AD_SMEM, st, a);
 	count_launch();
 	return check_launch("attn_decode");
 }
@@ -1672,25 +1696,6 @@ int make_digit_map(CUtensorMap *out, const uint8_t *x, int K, int groups, int tg
 	if (r != CUDA_SUCCESS) return fail(TG_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(int(r)));
 	return TG_OK;
 }
-// launch_k in clusters of `size` CTAs
-template <typename... KArgs, typename... Args>
-inline void launch_clusters(int size, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = grid;
-	cfg.blockDim = block;
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = st;
-	cudaLaunchAttribute at[2];
-	at[0].id = cudaLaunchAttributeClusterDimension;
-	at[0].val.clusterDim.x = size;
-	at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-	at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	at[1].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = at;
-	cfg.numAttrs = use_pdl() ? 2 : 1;
-	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
-}
-
 int make_gemm_map(CUtensorMap *out, const QW &w) { return make_tmap(out, w.q, w.K, w.N, 128, I8_SK, w.ld, true); }
 
 // One launch for up to three weight matrices with the same K that multiply the same packed A
