@@ -42,6 +42,9 @@ inline I8Plan i8_plan(int M, int K, int ng, const int *N, int num_sms, size_t pa
 	for (int g = 0; g < ng; g++) ntot += N[g];
 	for (int cg = 1; cg <= 2; cg++) {
 		if (want_cg && cg != want_cg) continue;
+		// up to 64 tokens the digits that a pair would share are little beside the weights (vocabulary matrix of 1152 rows, pairs / single CTAs:
+		// 3 tokens 65.5 / 57.8 us, 64 74.8 / 71.0, but 256 200 / 227; of 640 rows 50 / 40)
+		if (!want_cg && cg == 2 && groups <= I8_TG) continue;
 		int col_tiles = 0;
 		for (int g = 0; g < ng; g++) col_tiles += (N[g] + 128 * cg - 1) / (128 * cg);
 		const int workers = num_sms / cg;

@@ -1709,10 +1709,10 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<1>::SMEM));
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		configured[dev] = true;
 	}
 	const int K = ws[0]->K;
@@ -1773,9 +1773,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	if (pl.cg == 2) {
 		CUtensorMap xmap;
 		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
-		launch_clusters(2, sc.top1 ? qgemm_i8_kernel<2, I8_TOP1> : qgemm_i8_kernel<2, I8_SUMS>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
+		launch_clusters(2, sc.top1 ? qgemm_i8_kernel<2, I8_TOP1> : qgemm_i8_kernel<2, I8_SUMS>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
 	} else {
-		launch_k(sc.top1 ? qgemm_i8_kernel<1, I8_TOP1> : qgemm_i8_kernel<1, I8_SUMS>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8Shape<1>::SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
+		launch_k(sc.top1 ? qgemm_i8_kernel<1, I8_TOP1> : qgemm_i8_kernel<1, I8_SUMS>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
 	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
@@ -1811,7 +1811,7 @@ int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
-		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8Shape<2>::SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		configured[dev] = true;
 	}
 	GemmI8GluArgs a{};
@@ -1835,7 +1835,7 @@ int launch_gemm_geglu(const QW &U, const QW &G, int M, const GeluLut &lut, const
 	a.raw = 1;
 	a.err = sc.err;
 	a.lut = lut;
-	launch_clusters(2, qgemm_i8_kernel<2, I8_GLU>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8Shape<2>::SMEM, st, wmap[0], wmap[1], wmap[1], xmap, a);
+	launch_clusters(2, qgemm_i8_kernel<2, I8_GLU>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[1], xmap, a);
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
 	return pack_activations(sc.partial, M, I, sc, st);
