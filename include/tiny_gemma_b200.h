@@ -182,6 +182,8 @@ int tg_qgemm(float *c_host, const float *a_host, const int8_t *w_host, const flo
  * (n = 262144 in the reference); minp mutates logits_host like the reference */
 int tg_argmax_logits(const float *logits_host, int n, int *tok);
 int tg_minp_logits(float *logits_host, int n, float minp, float temp, float randf, int *tok);
+/* the same with the probabilities written to probs_host (n floats apart from the logits, or the logits themselves) */
+int tg_minp_probabilities(const float *logits_host, float *probs_host, int n, float minp, float temp, float randf, int *tok);
 /* The last step of ops::minp_logits in isolation (ops.hpp:849-857, the inverse-CDF loop):
  * *idx = first i with fl(cum0 + p[0] + ... + p[i]) >= randf, the sum taken sequentially in fp32,
  * or -1 if it never gets there; *cum_out (may be null) = the running sum where the scan stopped.

@@ -62,6 +62,7 @@ SIGNATURES = {
     "tg_qgemm": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int]),
     "tg_argmax_logits": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
     "tg_minp_logits": (C.c_int, [_P, C.c_int, C.c_float, C.c_float, C.c_float, C.POINTER(C.c_int)]),
+    "tg_minp_probabilities": (C.c_int, [_P, _P, C.c_int, C.c_float, C.c_float, C.c_float, C.POINTER(C.c_int)]),
     "tg_inverse_cdf": (C.c_int, [_P, C.c_int, C.c_float, C.c_float, C.POINTER(C.c_int), C.POINTER(C.c_float)]),
     "tg_rmsnorm": (C.c_int, [_P, _P, C.c_int, C.c_int]),
     "tg_dev_qmatvec": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, _P]),
@@ -160,9 +161,12 @@ def argmax_logits(logits) -> int:
 
 def minp_logits(logits, minp: float, temp: float, randf: float):
     """returns (token, probabilities); the input array is left untouched"""
-    p = np.array(logits, np.float32, copy=True)
+    x = np.asarray(logits, np.float32)
+    if not (x.flags.c_contiguous or x.flags.f_contiguous):
+        x = x.copy(order="K")
+    p = np.empty_like(x, subok=False)  # (the library writes the whole of it: a copy of 1 MB less a call)
     t = C.c_int(0)
-    _ck(load().tg_minp_logits(_ptr(p), p.size, minp, temp, randf, C.byref(t)))
+    _ck(load().tg_minp_probabilities(_ptr(x), _ptr(p), p.size, minp, temp, randf, C.byref(t)))
     return t.value, p
 
 

@@ -3346,9 +3346,11 @@ int tg_argmax_logits(const float *logits, int n, int *tok) {
 	return sample_host_row(logits, nullptr, n, false, 2.0f, 1.0f, 0.0f, tok);
 }
 
-int tg_minp_logits(float *logits, int n, float minp, float temp, float randf, int *tok) {
-	if (!logits || !tok || n < SR_PART || n % SR_PART) return fail(TG_EINVAL, "bad argument (n must be a multiple of 8192)");
-	return sample_host_row(logits, logits, n, true, minp, temp, randf, tok);
+int tg_minp_logits(float *logits, int n, float minp, float temp, float randf, int *tok) { return tg_minp_probabilities(logits, logits, n, minp, temp, randf, tok); }
+
+int tg_minp_probabilities(const float *logits, float *probs, int n, float minp, float temp, float randf, int *tok) {
+	if (!logits || !probs || !tok || n < SR_PART || n % SR_PART) return fail(TG_EINVAL, "bad argument (n must be a multiple of 8192)");
+	return sample_host_row(logits, probs, n, true, minp, temp, randf, tok);
 }
 
 // The samplers' own kernels on a given vector: it is padded to whole parts with zeros, which add nothing, and its segment sums
