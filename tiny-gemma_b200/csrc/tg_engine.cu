@@ -2049,16 +2049,17 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 		tc.err = s->err_flag;
 		p += (tc.x_bytes + 3) / 4;
 	}
-	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 832 tokens, and for a group of
-	// equal prompts of 16 and more tokens each that has more than 400 + 55000 / S of them in all. Otherwise the CUDA-core kernel
-	// with two queries per CTA is faster: its CTAs are more, and a prompt fills no tiles of 32 queries and 64 keys, as which the
-	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill in ms, 1B and 270m: one prompt of 700 tokens
-	// 4.03 / 4.45 and 1.99 / 2.28, of 832 4.73 / 4.76 and 2.37 / 2.38, of 960 5.46 / 5.14 and 2.81 / 2.58; groups of 178 tokens: 712 rows 3.59 / 3.51
-	// and 1.69 / 1.64, 1424 6.09 / 5.00 and 2.65 / 1.96; of 61: 976 rows 3.70 / 3.83 and 1.59 / 1.70, 1464 4.86 / 4.79 and 1.80 / 1.79; of 30: 2100 rows
-	// 6.58 / 6.90 and 2.29 / 2.30, 3600 10.4 / 10.7 and 3.35 / 3.04; of 16: 2048 rows 6.17 / 6.37 and 2.23 / 2.32, 2880 9.01 / 9.81 and 2.79 / 2.97.
+	// Attention on the tensor cores, from packed copies of q, k and v: for one prompt of more than 940 tokens, and for a group of
+	// equal prompts of 24 and more tokens each that has more than 700 + 50000 / S of them in all. Otherwise the CUDA-core kernel
+	// with two queries per CTA is faster: its CTAs are more, and a prompt fills no tiles of 32 queries and 128 keys, as which the
+	// packing and the tensor-core kernel treat it. Measured, CUDA cores / tensor cores, prefill in ms, 1B and 270m: one prompt of 832 tokens
+	// 4.18 / 4.41 and 1.94 / 2.07, of 960 4.78 / 4.75 and 2.25 / 2.18, of 1100 5.67 / 5.24 and 2.59 / 2.30; groups of 300 tokens: 1200 rows 4.66 / 4.68
+	// and 1.94 / 1.92; of 178: 890 rows 3.73 / 3.81 and 1.58 / 1.55, 1068 4.50 / 4.43 and 1.81 / 1.68; of 120: 840 rows 3.59 / 3.78 and 1.48 / 1.47, 1200 4.58 / 4.40 and
+	// 1.88 / 1.67; of 61: 1159 rows 4.17 / 4.27 and 1.55 / 1.64, 1586 5.17 / 5.17 and 1.90 / 1.85; of 30: 2100 rows 6.49 / 6.73 and 2.24 / 2.11, 2880 8.68 / 9.16
+	// and 2.69 / 2.55; of 16: 3600 rows 10.4 / 11.5 and 3.28 / 3.38.
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
-	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", at_rows > S_seq ? 400 + 55000 / S_seq : 832);
-	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 16);
+	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", at_rows > S_seq ? 700 + 50000 / S_seq : 940);
+	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 24);
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
