@@ -47,12 +47,17 @@
 namespace tg {
 
 constexpr int I8_THREADS = 320;                // producer, MMA issuer, 8 epilogue warps
-// CG CTAs work on a tile of CG * 128 columns: each holds its own 128 columns of W and 1 / CG of the digits. The ring has as many stages as fit
-// beside each other: with the few tokens of a decode step a stage is 20 KB, and four of the 48 KB that 64 tokens take left 64 KB of weights in flight per
-// SM, too few for HBM's rate times its latency: three rows of 640 x 262144 43 us by single CTAs, with 9 stages 40 (1152 rows: 65 and 58).
-constexpr int I8_MAX_STAGES = 12;
-// (220 KB in place of 192 leave no room for a CTA of the next launch: a prompt of 61 tokens 1248 us instead of 1196)
+// CG CTAs work on a tile of CG * 128 columns: each holds its own 128 columns of W and 1 / CG of the digits. A stage of the ring holds the digits of SLOT token
+// groups. With the few tokens of a decode step four stages that 64 tokens would fit left 64 KB of weights in flight per SM, too few for HBM's rate times its
+// latency: three rows of 640 x 262144 43 us, with eight small stages 40 (1152 rows: 65 and 58). As constants, or each MMA takes longer to issue (a ring whose
+// numbers follow the launch: 77 x 1152 x 6912 18.3 -> 18.8 us). 220 KB in place of 192 leave no room for a CTA of the next launch: a prompt of 61 tokens 1196 -> 1248 us.
+constexpr int I8_FEW = 2;                // groups of a tile that takes the small stages
 constexpr int I8_ROOM = 192 * 1024, I8_SMEM = I8_ROOM + 1024;
+template <int CG, int SLOT> struct I8Shape {
+	static constexpr int X_KB = SLOT * I8_GROUP_BYTES / CG;  // digits of one K-block in a CTA
+	static constexpr int STAGE = I8_W_BYTES + (I8_SK / I8_BK) * X_KB;
+	static constexpr int NST = I8_ROOM / STAGE;
+};
 
 // ------------------------------------------------------------------ digits
 // exponent of a row from the bits of its largest |x| (NaN and infinity compare above every finite value)
@@ -633,21 +638,21 @@ __device__ __forceinline__ void i8_cluster_sync() {
 // epilogue bounds it: with a branch per look-up it took 215 us, and with the table index in a loop of its own as well (GeluLut::index) 250.
 // What the epilogue does is a parameter of the kernel, not of the launch: with the code of the others beside it
 // a prompt of 178 tokens took 1.79 ms instead of 1.76 (156 registers instead of 140, and more code to fetch).
-template <int CG, I8Epilogue EPI>
+template <int CG, I8Epilogue EPI, int SLOT = I8_TG>
 __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_constant__ CUtensorMap wmap0,
                                                                  const __grid_constant__ CUtensorMap wmap1,
                                                                  const __grid_constant__ CUtensorMap wmap2,
                                                                  const __grid_constant__ CUtensorMap xmap, I8KernelArgs<EPI> a) {
+	using SH = I8Shape<CG, SLOT>;
+	constexpr int NST = SH::NST;
 	constexpr bool GLU = EPI == I8_GLU, TOP1 = EPI == I8_TOP1;
 	GeluLut lut{};
 	if constexpr (GLU) lut = a.lut;
-	const int x_kb = a.tg * I8_GROUP_BYTES / CG, stage_bytes = I8_W_BYTES + (I8_SK / I8_BK) * x_kb;  // digits of one K-block in a stage; a stage
-	const int nst = min(I8_MAX_STAGES, int(unsigned(I8_ROOM) / unsigned(stage_bytes)));
 	pdl_trigger();
 	extern __shared__ uint8_t i8_smem_raw[];
 	uint8_t *smem = reinterpret_cast<uint8_t *>((uintptr_t(i8_smem_raw) + 1023) & ~uintptr_t(1023));
-	__shared__ uint64_t full_bar[I8_MAX_STAGES];  // W and digits of the stage landed
-	__shared__ uint64_t free_bar[I8_MAX_STAGES];  // the MMAs that read the stage have completed
+	__shared__ uint64_t full_bar[NST];  // W and digits of the stage landed
+	__shared__ uint64_t free_bar[NST];  // the MMAs that read the stage have completed
 	__shared__ uint64_t acc_full[2];        // the accumulator's MMAs have completed
 	__shared__ uint64_t acc_free[2];        // the 8 epilogue warps (of both CTAs) have read the accumulator
 	__shared__ uint64_t drain_bar;          // every MMA issued has completed
@@ -667,7 +672,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 	if (GLU && lut.size <= GE_LUT)
 		for (int i = tid; i < lut.size; i += I8_THREADS) table[i] = lut.table[i];
 	if (tid == 0) {
-		for (int s = 0; s < nst; s++) {
+		for (int s = 0; s < NST; s++) {
 			mbar_init(&full_bar[s], 1);
 			mbar_init(&free_bar[s], 1);
 		}
@@ -702,7 +707,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 		const uint64_t pol = l2_evict_first_policy();
 		auto load_w = [&](const I8Tile &t, int st, int s) {
 			const CUtensorMap *wmap = t.grp == 0 ? &wmap0 : (t.grp == 1 ? &wmap1 : &wmap2);
-			uint8_t *dst = smem + size_t(s) * stage_bytes;
+			uint8_t *dst = smem + size_t(s) * SH::STAGE;
 			const int y = (t.s0 + st) * I8_SK;
 			if constexpr (CG == 2) {
 				// (a pair's box is always a whole tile's: what lies past the last token or column is not used)
@@ -717,21 +722,21 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 			}
 		};
 		auto load_x = [&](const I8Tile &t, int st, int s) {
-			uint8_t *dst = smem + size_t(s) * stage_bytes + I8_W_BYTES;
+			uint8_t *dst = smem + size_t(s) * SH::STAGE + I8_W_BYTES;
 			const int kb = (t.s0 + st) * (I8_SK / I8_BK);
 #pragma unroll
 			for (int q = 0; q < I8_SK / I8_BK; q++) {
 				if constexpr (CG == 2)
-					i8_pair_load(dst + q * x_kb, &xmap, 0, ((kb + q) * a.groups + t.g0) * 4 + rank * 2 * t.ng, i8_leader(&full_bar[s]));
+					i8_pair_load(dst + q * SH::X_KB, &xmap, 0, ((kb + q) * a.groups + t.g0) * 4 + rank * 2 * t.ng, i8_leader(&full_bar[s]));
 				else
-					bulk_load(dst + q * x_kb, a.x + (size_t(kb + q) * a.groups + t.g0) * I8_GROUP_BYTES, uint32_t(t.ng) * I8_GROUP_BYTES, &full_bar[s]);
+					bulk_load(dst + q * SH::X_KB, a.x + (size_t(kb + q) * a.groups + t.g0) * I8_GROUP_BYTES, uint32_t(t.ng) * I8_GROUP_BYTES, &full_bar[s]);
 			}
 		};
 		int cap = TC_SPIN_CAP, c = 0, s = 0;  // stages issued so far, next slot
 		uint32_t ph = 1;                      // parity whose completion frees the slot (a fresh barrier passes parity 1)
 		I8Tile t = tile(0);
 		// The weights are nobody's output: the first tiles are requested before the wait for the predecessor.
-		const int pre = first < a.tiles ? min(nst, t.ns) : 0;
+		const int pre = first < a.tiles ? min(NST, t.ns) : 0;
 		for (int st = 0; st < pre; st++)
 			if (tc_elect()) load_w(t, st, st);
 		pdl_wait();
@@ -744,7 +749,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 					load_x(t, st, s);
 				}
 				c++;
-				if (++s == nst) {
+				if (++s == NST) {
 					s = 0;
 					ph ^= 1;
 				}
@@ -767,17 +772,17 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 				for (int st = 0; st < t.ns; st++) {
 					tc_wait_cap(&full_bar[s], ph, cap);
 					tc_fence_after();
-					const uint32_t w = smem_u32(smem) + uint32_t(s) * stage_bytes;
+					const uint32_t w = smem_u32(smem) + uint32_t(s) * SH::STAGE;
 					const uint64_t dw = i8_desc_w(w), dx = i8_desc_x(w + I8_W_BYTES);
 					if (tc_elect()) {
 #pragma unroll
 						for (int j = 0; j < I8_SK / 32; j++)
-							i8_mma<CG>(d, dw + uint64_t(j * 256), dx + uint64_t(((j >> 1) * x_kb + (j & 1) * 32) >> 4), id, (st > 0 || j > 0) ? 1u : 0u);
+							i8_mma<CG>(d, dw + uint64_t(j * 256), dx + uint64_t(((j >> 1) * SH::X_KB + (j & 1) * 32) >> 4), id, (st > 0 || j > 0) ? 1u : 0u);
 						i8_commit<CG>(&free_bar[s]);
 						if (st == t.ns - 1) i8_commit<CG>(&acc_full[it & 1]);
 					}
 					__syncwarp();
-					if (++s == nst) {
+					if (++s == NST) {
 						s = 0;
 						ph ^= 1;
 					}
@@ -929,9 +934,9 @@ __global__ void __launch_bounds__(I8_THREADS, 1) qgemm_i8_kernel(const __grid_co
 	if (warp == 0 && lane == 0 && rank == 0 && *(volatile int *)&s_fail) {
 		// a wait ran out: every load that was issued must land before the shared memory is given up
 		const int n = *(volatile int *)&s_issued;
-		for (int c = max(0, n - nst); c < n; c++) {
+		for (int c = max(0, n - NST); c < n; c++) {
 			int spins = 0;
-			while (!mbar_try_wait(&full_bar[c % nst], (c / nst) & 1) && ++spins < TC_SPIN_CAP) {
+			while (!mbar_try_wait(&full_bar[c % NST], (c / NST) & 1) && ++spins < TC_SPIN_CAP) {
 			}
 		}
 	}

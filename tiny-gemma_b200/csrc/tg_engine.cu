@@ -1710,6 +1710,8 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 	const int dev = current_device_slot();
 	if (!configured[dev]) {
 		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_SUMS, I8_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
+		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_TOP1, I8_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<1, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
 		TG_CUDA(cudaFuncSetAttribute(qgemm_i8_kernel<2, I8_TOP1>, cudaFuncAttributeMaxDynamicSharedMemorySize, I8_SMEM));
@@ -1775,7 +1777,9 @@ int launch_gemm_tc_group(int ng, float *const *Cs, const QW *const *ws, const in
 		TG_TRY(make_digit_map(&xmap, a.x, K, a.groups, a.tg));
 		launch_clusters(2, sc.top1 ? qgemm_i8_kernel<2, I8_TOP1> : qgemm_i8_kernel<2, I8_SUMS>, dim3(2 * std::min(a.tiles, g_num_sms / 2)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], xmap, a);
 	} else {
-		launch_k(sc.top1 ? qgemm_i8_kernel<1, I8_TOP1> : qgemm_i8_kernel<1, I8_SUMS>, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
+		const bool few = pl.tg <= I8_FEW;
+		auto *kernel = sc.top1 ? (few ? qgemm_i8_kernel<1, I8_TOP1, I8_FEW> : qgemm_i8_kernel<1, I8_TOP1>) : (few ? qgemm_i8_kernel<1, I8_SUMS, I8_FEW> : qgemm_i8_kernel<1, I8_SUMS>);
+		launch_k(kernel, dim3(std::min(a.tiles, g_num_sms)), dim3(I8_THREADS), I8_SMEM, st, wmap[0], wmap[1], wmap[2], wmap[2], a);
 	}
 	count_launch();
 	TG_TRY(check_launch("qgemm_i8"));
