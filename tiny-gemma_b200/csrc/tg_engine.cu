@@ -1678,6 +1678,8 @@ int launch_geglu(const float *ug, int M, int I, const GeluLut &lut, int nsplit, 
 	const unsigned grid = unsigned(std::min(M, 2 * g_num_sms));
 	if (I <= 2048)
 		launch_k(geglu_i8_kernel<512, 1>, dim3(grid), dim3(512), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
+	else if (M <= g_num_sms)
+		launch_k(geglu_i8_kernel<576, 3, 1>, dim3(grid), dim3(576), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
 	else
 		launch_k(geglu_i8_kernel<576, 3>, dim3(grid), dim3(576), 0, st, ug, sc.x, rs, M, I, groups, lut, nsplit, su, sg);
 	count_launch();
