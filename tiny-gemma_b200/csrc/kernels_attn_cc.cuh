@@ -476,11 +476,12 @@ struct AttnSmallPlan {
 	int smem() const { return APS_RING + (ks - 1) * APS_PART * 4; }
 };
 // For a prompt of S tokens behind `off` others. By the prompt alone: a prompt of a group gets the bits that it gets by itself. The largest cluster
-// with two rounds of 32 keys per CTA at least whose CTAs are all resident at once (one per SM; the SMs of a GPC hold whole clusters): 178 tokens 2, 61 behind 1500 cached ones 4.
+// with two rounds of 32 keys per CTA at least (one where there are three in all: 61 tokens of 1B 1139 -> 1125 us, but 128 1283 -> 1297) whose CTAs are all resident at once (one per SM; the SMs of a GPC hold whole clusters): 178 tokens 2, 61 behind 1500 cached ones 4.
 inline AttnSmallPlan attn_small_plan(int S, int off, int is_local, int window) {
 	constexpr int ROUND = APS_GROUPS * APS_KEYS, resident[APS_MAX_KS + 1] = {0, 148, 148, 138, 128, 115};
 	const int pairs = (S + 1) / 2, most = is_local ? std::min(off + S, window + 2) : off + S;
-	for (int ks = std::min(APS_MAX_KS, (most + ROUND - 1) / ROUND / 2); ks > 1; ks--) {
+	const int rounds = (most + ROUND - 1) / ROUND;
+	for (int ks = std::min(APS_MAX_KS, rounds <= 3 ? rounds : rounds / 2); ks > 1; ks--) {
 		const int share = (most + ks * ROUND - 1) / (ks * ROUND) * ROUND;                // keys of a CTA of the longest walk
 		const int alone = most <= share ? pairs : std::min(pairs, std::max(0, share - off) / 2);  // pair i has off + 2 i + 2 keys
 		const int clusters = pairs - alone + (alone + ks - 1) / ks;
