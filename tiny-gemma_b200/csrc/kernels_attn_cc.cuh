@@ -64,6 +64,14 @@ __device__ __forceinline__ uint32_t ac_mapa(const void *p, int rank) {
 	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
 	return r;
 }
+// a wait ran out: report it, and give the copies in flight time to land before the shared memory goes to another use
+__device__ __noinline__ void ac_give_up(int *err) {
+	*static_cast<volatile int *>(err) = 6;
+	const long long t0 = clock64();
+	while (clock64() - t0 < 2000000) {
+	}
+}
+
 // ------------------------------------------------------------------ decode: one query per sequence
 struct AttnArgs {
 	const float *qkv;   // [B][1536] = q(4x256) | k(256) | v(256)
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		__syncwarp();
 		issue(iv + AD_STAGES);
 	}
-	if (cap == 0) *static_cast<volatile int *>(a.err_flag) = 6;
+	if (cap == 0) ac_give_up(a.err_flag);
 	// ---- join the warps: thread (h, d4) ends up with four consecutive outputs
 	__syncthreads();  // (every warp has consumed its ring)
 	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
@@ -614,7 +622,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 			}
 		}
 	}
-	if (cap == 0) *static_cast<volatile int *>(err) = 6;
+	if (cap == 0) ac_give_up(err);
 	// ---- join the groups: thread (query, k4) ends up with four of its query's 1024 outputs
 	__syncthreads();  // (every warp has read its ring)
 	float4 *jb = reinterpret_cast<float4 *>(ac_smem);
