@@ -1,12 +1,10 @@
 // Attention over fp32 K / V rows on the CUDA cores, for the shapes whose time is latency and memory traffic, not
 // arithmetic: one decode step per sequence, and short prompts.
 //
-// The rows of a sequence's keys (values) follow each other in memory, so a chunk of 32 keys is ONE bulk copy of 32 KB
-// into shared memory: the whole traffic of a CTA is asynchronous and costs no registers. A buffer is filled again as soon
-// as its scores (K) or products (V) are done.
-// The prefill kernel's step over a chunk: scores (a warp takes a few keys against all query rows; a lane holds 8 of the 256 dimensions, and the
-// lanes' partial sums meet in a reduce-scatter, one shuffle per score), one softmax step per query row with lane = key,
-// then the products with V (a thread holds 4 dimensions of every row for a share of the keys).
+// The rows of a sequence's keys (values) follow each other in memory, so four of them are ONE bulk copy of 4 KB into a
+// warp's ring in shared memory: the whole traffic of a CTA is asynchronous and costs no registers. Both kernels take a step of
+// four keys against the heads of a query per warp: scores (a lane holds 8 of the 256 dimensions, and the lanes' partial sums meet in a
+// reduce-scatter), a softmax step with a running maximum of the warp's own, the products with V. The warps' parts are joined at the end.
 //
 // The result leaves as the digits of the O projection's operand (kernels_gemm_i8.cuh) where the caller wants them: the
 // CTA that finishes a row has all of it.
