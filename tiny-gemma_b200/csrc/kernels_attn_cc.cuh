@@ -94,6 +94,7 @@ struct AttnArgs {
 	float *rowscale;
 	int groups;
 	int nsplit, cluster;  // CTAs per sequence, and how many of them form a cluster (1: none)
+	int polls;            // limit of a wait for copies
 	int *err_flag;
 };
 constexpr int AT_THREADS = 256;
@@ -121,14 +122,12 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	__shared__ uint64_t full[AT_THREADS / 32][AD_STAGES];
 	__shared__ uint32_t red[AT_THREADS / 32];
 	__shared__ int s_last;
-	__shared__ uint64_t joined;  // (of a cluster's first CTA) every warp of the others has handed over its part, or has none
 	const int b = blockIdx.y, split = blockIdx.x, rank = a.cluster > 1 ? split % AD_CLUSTER : 0;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	pdl_trigger();
 	uint8_t *ring = ac_smem + warp * (AD_STAGES * AD_BUF);
 	if (lane == 0) {
 		for (int i = 0; i < AD_STAGES; i++) mbar_init(&full[warp][i], 1);
-		if (warp == 0) mbar_init(&joined, (AD_CLUSTER - 1) * (AT_THREADS / 32));
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	__syncwarp();
@@ -176,11 +175,14 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		per = (rounds + a.nsplit - 1) / a.nsplit;
 		nact = (rounds + per - 1) / per;
 	}
-	auto hand_over = [&](uint32_t count) {  // to the cluster's first CTA
-		asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(ac_mapa(&joined, 0)), "r"(count) : "memory");
+	// The cluster's first CTA stays until every other one has handed over its part, has none or has given up: it waits at the cluster's barrier, which the
+	// others reach because all waits in front of it are bounded. (A bounded wait of its own could run out first, and a part would arrive in a CTA that has left.)
+	auto hand_over = [] {
+		__syncwarp();
+		asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 	};
 	if (split >= nact) {
-		if (a.cluster > 1 && split - rank < nact && tid == 0) hand_over(AT_THREADS / 32);
+		if (a.cluster > 1) hand_over();
 		return;
 	}
 	const int j0 = split * per * AD_ROUND, j1 = min(valid, j0 + per * AD_ROUND);
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		fence_proxy_async();  // (the buffer's next content arrives by a bulk copy)
 		__syncwarp();
 	};
-	int cap = TC_SPIN_CAP;
+	int cap = a.polls;
 	for (int it = 0; it < nit; it++) {
 		const int j = jw + it * AD_ROUND, n = min(AD_KEYS, j1 - j);
 		const int ik = 2 * it, iv = 2 * it + 1;
@@ -376,14 +378,11 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 			asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + 16u * tid), "f"(r.x), "f"(r.y), "f"(r.z), "f"(r.w) : "memory");
 			if (d4 == 0)
 				asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + 4u * (AT_NH * AT_HD) + 8u * h), "f"(Ms), "f"(L) : "memory");
-			__syncwarp();
-			if (lane == 0) hand_over(1);
+			hand_over();
 			return;
 		}
-		uint32_t ok = 0;
-		for (int z = 0; !ok && z < TC_SPIN_CAP; z++)
-			asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(&joined)) : "memory");
-		if (!ok) *static_cast<volatile int *>(a.err_flag) = 6;
+		hand_over();
+		asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 		const int n = min(AD_CLUSTER, nact - split);
 #pragma unroll 1
 		for (int p = 1; p < n; p++, in += AT_PART) {  // (every part has a key)

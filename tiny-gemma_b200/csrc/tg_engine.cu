@@ -631,6 +631,7 @@ int launch_attn_decode(AttnArgs a, int nb, cudaStream_t st) {
 		TG_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_decode_smem(AD_CLUSTER)));
 		configured[dev] = true;
 	}
+	a.polls = env_int("TG_ATTN_POLLS", TC_SPIN_CAP);
 	a.cluster = nb <= AD_CLUSTER_SEQS && a.nsplit % AD_CLUSTER == 0 ? AD_CLUSTER : 1;
 	if (a.cluster > 1)
 		launch_clusters(AD_CLUSTER, attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), attn_decode_smem(AD_CLUSTER), st, a);
