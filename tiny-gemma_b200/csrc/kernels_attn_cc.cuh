@@ -193,10 +193,11 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 	const bool stream = long(gridDim.y) * valid > 16384;
 	const uint64_t policy = l2_evict_first_policy();
 	// item i of the warp's ring: the keys (i even) or the values (i odd) of group i / 2; called by the whole warp
+	int items = 2 * nit;  // (none any more behind a wait that ran out: the stage's barrier may still count an older copy)
 	auto issue = [&](int i) {
 		const int j = jw + (i >> 1) * AD_ROUND, st = i % AD_STAGES;
 		const uint32_t bytes = uint32_t(min(AD_KEYS, j1 - j)) * 1024u;
-		if (i < 2 * nit && tc_elect()) {
+		if (tc_elect() && i < items) {
 			mbar_expect_tx(&full[warp][st], bytes);
 			const float *src = (i & 1 ? vc : kc) + size_t(j) * AT_HD;
 			if (stream)
@@ -295,11 +296,15 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 		__syncwarp();
 	};
 	int cap = a.polls;
+	auto wait = [&](int i) {
+		tc_wait_cap(&full[warp][i % AD_STAGES], i / AD_STAGES & 1, cap);
+		if (cap == 0) items = 0;
+	};
 	for (int it = 0; it < nit; it++) {
 		const int j = jw + it * AD_ROUND, n = min(AD_KEYS, j1 - j);
 		const int ik = 2 * it, iv = 2 * it + 1;
 		uint8_t *K = ring + ik % AD_STAGES * AD_BUF, *V = ring + iv % AD_STAGES * AD_BUF;
-		tc_wait_cap(&full[warp][ik % AD_STAGES], ik / AD_STAGES & 1, cap);
+		wait(ik);
 		patch(K, slot - j, AT_NH);
 		float t[16];
 #pragma unroll
@@ -328,7 +333,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attn_decode_kernel(AttnArgs a) 
 				o1[h] = make_float4(o1[h].x * c, o1[h].y * c, o1[h].z * c, o1[h].w * c);
 			}
 		}
-		tc_wait_cap(&full[warp][iv % AD_STAGES], iv / AD_STAGES & 1, cap);
+		wait(iv);
 		patch(V, slot - j, AT_NH + 1);
 #pragma unroll
 		for (int kk = 0; kk < AD_KEYS; kk++) {
@@ -496,7 +501,7 @@ inline AttnSmallPlan attn_small_plan(int S, int off, int is_local, int window) {
 }
 __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(float *o_out, uint8_t *x, float *rowscale, int groups, const float *q,
                                                                             const float *k, const float *v, int S, int off, int is_local, int window,
-                                                                            int cluster, int shared, int *err) {
+                                                                            int cluster, int shared, int polls, int *err) {
 	extern __shared__ __align__(128) uint8_t ac_smem[];
 	constexpr int R = 2 * AT_NH, H = AT_NH;  // query rows: query * 4 + head
 	__shared__ float m_s[APS_GROUPS][R], l_s[APS_GROUPS][R];
@@ -524,9 +529,9 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	const int jw = j0 + APS_KEYS * (rank * APS_GROUPS + grp), jd = APS_KEYS * APS_GROUPS * ks, nit = pair < 0 ? 0 : max(0, (j1 - jw + jd - 1) / jd);
 	k += r0 * 256;  // (a continuation is one sequence: r0 = 0)
 	v += r0 * 256;
-	auto issue = [&](int i) {  // step i of the group; called by the whole warp
+	auto issue = [&](int i, int cap) {  // step i of the group; called by the whole warp (cap = 0: not behind a wait that ran out)
 		const int j = jw + i * jd, st = i % APS_STAGES;
-		if (i < nit && tc_elect()) {
+		if (i < nit && tc_elect() && cap > 0) {
 			const uint32_t bytes = uint32_t(min(APS_KEYS, j1 - j)) * 1024u;
 			mbar_expect_tx(&full[grp][st], 2 * bytes);
 			bulk_load(ring + st * 2 * APS_BUF, k + size_t(j) * 256, bytes, &full[grp][st]);
@@ -535,7 +540,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	};
 	if (qi == 0) {
 #pragma unroll
-		for (int i = 0; i < APS_STAGES; i++) issue(i);
+		for (int i = 0; i < APS_STAGES; i++) issue(i, 1);
 	}
 	// A lane keeps the heads, and the keys of a step, in an order of its own for the scores (slot ^ hperm, slot ^ kperm): every round of the
 	// reduce-scatter then keeps the lower and sends the upper slots, without selects.
@@ -559,7 +564,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 	}
 	float m = -INFINITY, l = 0.0f;  // of head hperm; this lane's score of a step is key kperm's
 	const int mine = off + s0 + qi, first = is_local ? mine - window : 0;  // the query's own key, the first one that it sees
-	int cap = TC_SPIN_CAP;
+	int cap = polls;
 	for (int it = 0; it < nit; it++) {
 		const int j = jw + it * jd, n = min(APS_KEYS, j1 - j), st = it % APS_STAGES, ph = it / APS_STAGES & 1;
 		const uint8_t *K = ring + st * 2 * APS_BUF, *V = K + APS_BUF;
@@ -615,7 +620,7 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 			if (lane == 0) mbar_arrive(&done[grp][st]);
 			if (qi == 0) {  // (its other warp is about as far)
 				tc_wait_cap(&done[grp][st], ph, cap);
-				issue(it + APS_STAGES);
+				issue(it + APS_STAGES, cap);
 			}
 		}
 	}

@@ -624,6 +624,8 @@ inline void launch_clusters(int size, void (*kernel)(KArgs...), dim3 grid, dim3 
 	cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
 }
 
+int attn_polls() { return env_int("TG_ATTN_POLLS", TC_SPIN_CAP); }
+
 int launch_attn_decode(AttnArgs a, int nb, cudaStream_t st) {
 	static bool configured[TG_MAX_DEVICES] = {false};
 	const int dev = current_device_slot();
@@ -631,7 +633,7 @@ int launch_attn_decode(AttnArgs a, int nb, cudaStream_t st) {
 		TG_CUDA(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_decode_smem(AD_CLUSTER)));
 		configured[dev] = true;
 	}
-	a.polls = env_int("TG_ATTN_POLLS", TC_SPIN_CAP);
+	a.polls = attn_polls();
 	a.cluster = nb <= AD_CLUSTER_SEQS && a.nsplit % AD_CLUSTER == 0 ? AD_CLUSTER : 1;
 	if (a.cluster > 1)
 		launch_clusters(AD_CLUSTER, attn_decode_kernel, dim3(a.nsplit, nb), dim3(AT_THREADS), attn_decode_smem(AD_CLUSTER), st, a);
@@ -2067,6 +2069,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 	const AttnTcPlan atp = attn_tc_plan(S_seq);
 	const int at_rows = plan_rows ? S_seq : S, at_line = env_int("TG_ATTN_SMALL_MAX", at_rows > S_seq ? 700 + 50000 / S_seq : 940);
 	const bool attn_tc = use_tc && pos0 < 0 && env_int("TG_ATTN_TC", 1) && at_rows > at_line && S_seq >= env_int("TG_ATTN_TC_MIN", 24);
+	const int polls = attn_polls();
 	__nv_bfloat16 *at_q = nullptr, *at_k = nullptr, *at_v = nullptr;
 	if (attn_tc) {
 		p = reinterpret_cast<float *>((uintptr_t(p) + 1023) & ~uintptr_t(1023));
@@ -2179,7 +2182,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			}
 			const AttnSmallPlan ap = attn_small_plan(S_seq, off, w.is_local ? 1 : 0, window);
 			launch_clusters(ap.ks, attn_prefill_small_kernel, dim3(ap.clusters * ap.ks, nb), dim3(APS_THREADS), ap.smem(), st, ao, use_tc ? tc.x : nullptr,
-			                use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, ap.ks, ap.shared, s->err_flag);
+			                use_tc ? i8_rowscale(tc, S, qd) : nullptr, i8_groups(S), q, kb, vb, S_seq, off, w.is_local ? 1 : 0, window, ap.ks, ap.shared, polls, s->err_flag);
 		} else if (attn_tc) {
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
