@@ -190,40 +190,40 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32])
 	    "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
 	    : "memory");
 }
-// bounded wait that also gives up when another role of the CTA already has
-__device__ __forceinline__ bool at_wait(uint64_t *bar, uint32_t parity, int *err, volatile int *s_fail) {
-	int spins = 0;
-	while (!mbar_try_wait(bar, parity)) {
-		if ((++spins & 1023) == 0 && *s_fail) return false;
+// Waits of the softmax warps: bounded, given up when another role of the CTA already has, and without an exit: a lane that gave up (ok) goes on with its
+// warp and waits no more, since the TMEM loads and stores behind a wait are instructions of the whole, converged warp.
+struct AtLimit {
+	int *err;
+	volatile int *s_fail;
+	bool ok = true;
+	__device__ __forceinline__ void spin(int &spins) {
+		if ((++spins & 1023) == 0 && *s_fail) ok = false;
 		if (spins > TC_SPIN_CAP) {
 			atomicExch(err, 6);
 			*s_fail = 1;
-			return false;
+			ok = false;
 		}
 	}
-	return true;
+};
+__device__ __forceinline__ void at_wait(uint64_t *bar, uint32_t parity, AtLimit &lim) {
+	int spins = 0;
+	while (lim.ok && !mbar_try_wait(bar, parity)) lim.spin(spins);
+	__syncwarp();
 }
 
 // The two threads of a row hand each other one float through shared memory: value, then tag; the reader
 // polls the partner's tag (bounded like every wait here).
-__device__ __forceinline__ bool at_exchange(float *val, int *tag, int me, float v, int t, float *other, int *err, volatile int *s_fail) {
+__device__ __forceinline__ float at_exchange(float *val, int *tag, int me, float v, int t, AtLimit &lim) {
 	volatile float *xv = val;
 	volatile int *xg = tag;
 	xv[me] = v;
 	__threadfence_block();
 	xg[me] = t;
 	int spins = 0;
-	while (xg[me ^ 1] != t) {
-		if ((++spins & 1023) == 0 && *s_fail) return false;
-		if (spins > TC_SPIN_CAP) {
-			atomicExch(err, 6);
-			*s_fail = 1;
-			return false;
-		}
-	}
+	while (lim.ok && xg[me ^ 1] != t) lim.spin(spins);
+	__syncwarp();
 	__threadfence_block();
-	*other = xv[me ^ 1];
-	return true;
+	return xv[me ^ 1];
 }
 
 struct AttnTcArgs {
@@ -416,9 +416,9 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		const int k_min = a.is_local ? max(0, qi - a.window) : 0;
 		const uint32_t lane_base = uint32_t(qd * 32) << 16;
 		float m = -INFINITY, l = 0.0f;             // max in use (the same in both threads of a row), sum over this thread's keys
-		bool ok = true;
-		for (int jt = 0; jt < ntiles && ok; jt++) {
-			if (!at_wait(&s_bar[jt & 1], (jt >> 1) & 1, a.err, fail)) { ok = false; break; }
+		AtLimit lim{a.err, fail};
+		for (int jt = 0; jt < ntiles; jt++) {
+			at_wait(&s_bar[jt & 1], (jt >> 1) & 1, lim);
 			tc_fence_after();
 			uint32_t sv[2][32];
 			tc_ld32(tmem_s + lane_base + uint32_t((jt & 1) * AT_TC_KT + HK * hf), sv[0]);
@@ -446,11 +446,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 				}
 			}
 			// the row's max over both halves
-			{
-				float other;
-				if (!at_exchange(xm[jt & 1][r], xt[jt & 1][r], hf, mt, jt + 1, &other, a.err, fail)) { ok = false; break; }
-				mt = fmaxf(mt, other);
-			}
+			mt = fmaxf(mt, at_exchange(xm[jt & 1][r], xt[jt & 1][r], hf, mt, jt + 1, lim));
 			// the max in use moves only when the new one exceeds it by more than 8 (or at the row's first visible key)
 			const float mn = (mt > m + 8.0f || m == -INFINITY) ? fmaxf(m, mt) : m;
 			const bool none = mn == -INFINITY;            // no visible key so far
@@ -465,7 +461,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			l = fmaf(l, corr, sum);
 			m = mn;
 			// the previous tile's P V reads P (and accumulates into O) until pv_bar: wait for it before touching either
-			if (jt > 0 && !at_wait(&pv_bar, (jt - 1) & 1, a.err, fail)) { ok = false; break; }
+			if (jt > 0) at_wait(&pv_bar, (jt - 1) & 1, lim);
 			tc_fence_after();
 			// the probabilities' three bf16 terms by truncation (p >= 0; hi + mid + lo = p exactly: 8 + 8 + 8 bits), eight keys of the row at a time
 #pragma unroll
@@ -513,48 +509,44 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		// ------------------------------------------------------------ epilogue: the digits of o = O / l
 		// A row of the O projection's operand is the four heads of a query: four neighbouring lanes, in both halves. Its largest value
 		// first, then O once more. (The partner is past its last read of a slot: it arrived at p_bar, which o_bar follows.)
-		if (ok && at_wait(&o_bar, 0, a.err, fail)) {
-			tc_fence_after();
-			float other = 0.0f;
-			bool got = at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, &other, a.err, fail);
-			const float inv = 1.0f / (l + other);  // (a visible key always exists: the query itself)
-			uint32_t mx = 0;
+		at_wait(&o_bar, 0, lim);
+		tc_fence_after();
+		const float inv = 1.0f / (l + at_exchange(xm[0][r], xt[0][r], hf, l, 0x40000000, lim));  // (a visible key always exists: the query itself)
+		uint32_t mx = 0;
 #pragma unroll 1
-			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
-				uint32_t ov[32];
-				tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
-				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+		for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
+			uint32_t ov[32];
+			tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
+			asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-				for (int i = 0; i < 32; i++) mx = max(mx, i8_abs_bits(__uint_as_float(ov[i]) * inv));
-			}
-			mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-			mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-			got = got && at_exchange(xm[1][r], xt[1][r], hf, __uint_as_float(mx), 0x40000001, &other, a.err, fail);
-			mx = max(mx, __float_as_uint(other));
-			const float mul = i8_row_mul(mx);
-			const int row = int(blockIdx.y) * a.S + qi, head = r & 3;
-			const bool store = row_ok && got;
-			if (store && hf == 0 && head == 0) a.rowscale[row] = i8_row_scale(mx);
+			for (int i = 0; i < 32; i++) mx = max(mx, i8_abs_bits(__uint_as_float(ov[i]) * inv));
+		}
+		mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+		mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+		mx = max(mx, __float_as_uint(at_exchange(xm[1][r], xt[1][r], hf, __uint_as_float(mx), 0x40000001, lim)));
+		const float mul = i8_row_mul(mx);
+		const int row = int(blockIdx.y) * a.S + qi, head = r & 3;
+		const bool store = row_ok && lim.ok;
+		if (store && hf == 0 && head == 0) a.rowscale[row] = i8_row_scale(mx);
 #pragma unroll 1
-			for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
-				uint32_t ov[32];
-				tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
-				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-				if (store) {
+		for (int c8 = 4 * hf; c8 < 4 * hf + 4; c8++) {
+			uint32_t ov[32];
+			tc_ld32(tmem_o + lane_base + uint32_t(32 * c8), ov);
+			asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+			if (store) {
 #pragma unroll
-					for (int h = 0; h < 2; h++) {  // 16 dimensions: one chunk of 16 bytes per digit
-						uint32_t d[4][4];
+				for (int h = 0; h < 2; h++) {  // 16 dimensions: one chunk of 16 bytes per digit
+					uint32_t d[4][4];
 #pragma unroll
-						for (int q = 0; q < 4; q++) {
-							uint32_t b[4];
+					for (int q = 0; q < 4; q++) {
+						uint32_t b[4];
 #pragma unroll
-							for (int i = 0; i < 4; i++) b[i] = i8_digits(__uint_as_float(ov[16 * h + 4 * q + i]) * inv, mul);
-							i8_transpose4(b, d[0][q], d[1][q], d[2][q], d[3][q]);
-						}
-						uint8_t *p = a.x + i8_offset(row, (head * 256 + 32 * c8 + 16 * h) >> 2, a.groups);
-#pragma unroll
-						for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(p + 512 * i) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
+						for (int i = 0; i < 4; i++) b[i] = i8_digits(__uint_as_float(ov[16 * h + 4 * q + i]) * inv, mul);
+						i8_transpose4(b, d[0][q], d[1][q], d[2][q], d[3][q]);
 					}
+					uint8_t *p = a.x + i8_offset(row, (head * 256 + 32 * c8 + 16 * h) >> 2, a.groups);
+#pragma unroll
+					for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(p + 512 * i) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
 				}
 			}
 		}
