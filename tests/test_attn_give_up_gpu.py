@@ -34,9 +34,9 @@ def test_batched_step(capi, synth, weights_270m, monkeypatch, n, S):
     m.close()
 
 
-# walks of one CTA, of a cluster, and more steps than the ring holds
-@pytest.mark.parametrize("S", [24, 61, 178, 500])
-def test_short_prompt(capi, synth, weights_270m, monkeypatch, S):
+# CUDA cores: walks of one CTA, of a cluster, and more steps than the ring holds; tensor cores: windows that begin in the first and in a later key tile
+@pytest.mark.parametrize("S", [24, 61, 178, 500, 941, 1500])
+def test_prompt(capi, synth, weights_270m, monkeypatch, S):
     m = capi.Model("270m").load_file(weights_270m).build_tables(1024)
     ids, st = synth.random_prompt(S, 3), m.state(1, S + 8)
     want = st.prefill(ids)

@@ -33,8 +33,9 @@
 // O rescaled, a TMEM round trip) when a row's new max exceeds the one in use by more than 8: the probabilities
 // are then at most e^8, far inside fp32, and the final division by the row sum removes the common factor.
 // The epilogue leaves the digits of the O projection's operand (a row of it is the four heads of a query).
-// All waits are bounded; a wait that runs out sets *err, and the CTA lets its copies land and frees its
-// TMEM before it returns.
+// All waits are bounded; behind one that runs out no copy is issued any more (its stage's barrier may still count an older one), *err is set, and the
+// CTA lets its copies land and frees its TMEM before it returns. POLLS, the limit, is 0 in a test (no MMA then
+// either); as an argument of the launch it cost 1.4 us a layer.
 #pragma once
 #include "kernels_gemm_i8.cuh"  // digits of the O projection's operand
 #include "kernels_prefill.cuh"  // RopeArgs
@@ -193,12 +194,12 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32])
 // Waits of the softmax warps: bounded, given up when another role of the CTA already has, and without an exit: a lane that gave up (ok) goes on with its
 // warp and waits no more, since the TMEM loads and stores behind a wait are instructions of the whole, converged warp.
 struct AtLimit {
-	int *err;
+	int polls, *err;
 	volatile int *s_fail;
 	bool ok = true;
 	__device__ __forceinline__ void spin(int &spins) {
 		if ((++spins & 1023) == 0 && *s_fail) ok = false;
-		if (spins > TC_SPIN_CAP) {
+		if (spins > polls) {
 			atomicExch(err, 6);
 			*s_fail = 1;
 			ok = false;
@@ -239,6 +240,7 @@ struct AttnTcArgs {
 	int *err;
 };
 
+template <int POLLS>
 __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnTcArgs a) {
 	pdl_trigger();
 	extern __shared__ uint8_t at_smem_raw[];
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		             v_term = size_t(a.v_blocks) * AT_TC_VBYTES;  // bytes
 		const uint8_t *qp = reinterpret_cast<const uint8_t *>(a.qp) + blockIdx.y * 3 * q_term + size_t(tile) * 16 * AT_TC_QBYTES,
 		              *kp = reinterpret_cast<const uint8_t *>(a.kp) + blockIdx.y * 3 * k_term, *vp = reinterpret_cast<const uint8_t *>(a.vp) + blockIdx.y * 3 * v_term;
-		int cap = TC_SPIN_CAP, st = 0;
+		int cap = POLLS, st = 0;
 		uint32_t ph = 1;  // (a fresh barrier passes parity 1)
 		auto next = [&] {
 			if (++st == AT_TC_NS) {
@@ -321,7 +323,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			    uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
 			    const uint8_t *q = qp + size_t(i) * AT_TC_QBYTES, *k = kp + (size_t(j_lo + t) * 16 + i) * AT_TC_QBYTES + lo;
 			    tc_wait_cap(&free_bar[st], ph, cap);
-			    if (tc_elect()) {
+			    if (tc_elect() && cap > 0) {
 				    mbar_expect_tx(&full_bar[st], 3u * (AT_TC_QBYTES + bytes));
 #pragma unroll
 				    for (int c = 0; c < 3; c++) {
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			    uint8_t *dst = smem + size_t(st) * AT_TC_STAGE;
 			    const uint8_t *v = vp + (size_t(j_lo + t) * (AT_TC_KT / 16) + u) * AT_TC_VBYTES;
 			    tc_wait_cap(&free_bar[st], ph, cap);
-			    if (tc_elect()) {
+			    if (tc_elect() && cap > 0) {
 				    mbar_expect_tx(&full_bar[st], 3u * AT_TC_VBYTES);
 #pragma unroll
 				    for (int c = 0; c < 3; c++) bulk_load(dst + c * AT_TC_VBYTES, v + c * v_term, AT_TC_VBYTES, &full_bar[st]);
@@ -351,7 +353,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		const uint32_t idesc_pv = at_idesc(256, 1);
 		// the six term products (A term, B term)
 		constexpr int ta[6] = {0, 0, 1, 1, 0, 2}, tb[6] = {0, 1, 0, 1, 2, 0};
-		int cap = TC_SPIN_CAP, st = 0;
+		int cap = POLLS, st = 0;
 		uint32_t ph = 0;
 		const uint32_t pb = smem_u32(pbuf);
 		bool ready = false;  // the next block has landed: asked before the MMAs of the one before it are issued (an answer takes 180 clk)
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			    const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE), lo = uint32_t(first_block(t)) * 16u, n = uint32_t(end_block(t)) * 16u - lo;
 			    const uint32_t d_s = tmem_s + uint32_t(t & 1) * AT_TC_KT + lo, idesc = at_idesc(int(n), 0);
 			    const uint64_t dq = at_qdesc(base), dk = at_qdesc(base + 3 * AT_TC_QBYTES);
-			    if (tc_elect()) {
+			    if (POLLS > 0 && tc_elect()) {
 #pragma unroll
 				    for (int c = 0; c < 6; c++)
 					    tc_mma(d_s, dq + uint64_t((ta[c] * AT_TC_QBYTES) >> 4), dk + uint64_t((tb[c] * AT_TC_QBYTES) >> 4), idesc, (i > 0 || c > 0) ? 1u : 0u);
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 			    landed();
 			    const uint32_t base = smem_u32(smem + size_t(st) * AT_TC_STAGE);
 			    const uint64_t dp = at_qdesc(pb + uint32_t(u) * AT_TC_QBYTES), dv = at_vdesc(base);
-			    if (tc_elect()) {
+			    if (POLLS > 0 && tc_elect()) {
 #pragma unroll
 				    for (int c = 0; c < 6; c++)
 					    tc_mma(tmem_o, dp + uint64_t((ta[c] * AT_TC_PTERM) >> 4), dv + uint64_t((tb[c] * AT_TC_VBYTES) >> 4), idesc_pv,
@@ -416,7 +418,7 @@ __global__ void __launch_bounds__(AT_TC_THREADS, 1) attn_prefill_tc_kernel(AttnT
 		const int k_min = a.is_local ? max(0, qi - a.window) : 0;
 		const uint32_t lane_base = uint32_t(qd * 32) << 16;
 		float m = -INFINITY, l = 0.0f;             // max in use (the same in both threads of a row), sum over this thread's keys
-		AtLimit lim{a.err, fail};
+		AtLimit lim{POLLS, a.err, fail};
 		for (int jt = 0; jt < ntiles; jt++) {
 			at_wait(&s_bar[jt & 1], (jt >> 1) & 1, lim);
 			tc_fence_after();

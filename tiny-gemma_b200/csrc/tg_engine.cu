@@ -2187,7 +2187,8 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			static bool at_configured[TG_MAX_DEVICES] = {false};
 			const int dev = current_device_slot();
 			if (!at_configured[dev]) {
-				TG_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_TC_SMEM));
+				TG_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<TC_SPIN_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_TC_SMEM));
+				TG_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_TC_SMEM));
 				at_configured[dev] = true;
 			}
 			AttnTcArgs aa{};
@@ -2204,7 +2205,7 @@ int enqueue_prefill_seq(tg_state *s, int b, int S_seq, int nb = 1, int pos0 = -1
 			aa.is_local = w.is_local ? 1 : 0;
 			aa.window = c.n_pos_local;
 			aa.err = s->err_flag;
-			launch_k(attn_prefill_tc_kernel, dim3(atp.q_tiles, nb), dim3(AT_TC_THREADS), size_t(AT_TC_SMEM), st, aa);
+			launch_k(polls ? attn_prefill_tc_kernel<TC_SPIN_CAP> : attn_prefill_tc_kernel<0>, dim3(atp.q_tiles, nb), dim3(AT_TC_THREADS), size_t(AT_TC_SMEM), st, aa);
 		} else
 			if (env_int("TG_ATTN_BLOCK4", 1)) {  // long prompts: four keys per step (TG_ATTN_BLOCK4=0: the per-key kernel)
 				static bool configured[TG_MAX_DEVICES] = {false};
