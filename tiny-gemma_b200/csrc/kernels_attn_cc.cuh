@@ -589,8 +589,8 @@ __global__ void __launch_bounds__(APS_THREADS, 1) attn_prefill_small_kernel(floa
 		float mn = fmaxf(m, z);
 		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 8));
 		mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 16));
-		// (no key may be visible yet: the window starts later, or the step lies behind the query)
-		const float p = vis ? expf(z - mn) : 0.0f, cr = m == mn ? 1.0f : expf(m - mn);
+		// (mn may still be -inf: no key is visible yet, since the window starts later or the step lies behind the query, or all four scores overflowed to it)
+		const float p = z != -INFINITY ? expf(z - mn) : 0.0f, cr = m == mn ? 1.0f : expf(m - mn);
 		float ps = p + __shfl_xor_sync(0xffffffffu, p, 8);
 		ps += __shfl_xor_sync(0xffffffffu, ps, 16);
 		l = fmaf(l, cr, ps);
