@@ -39,3 +39,16 @@ def test_kernel_of_a_prompt(capi, synth, weights_270m, monkeypatch, n, S, tensor
     assert np.array_equal(got, own) and not np.array_equal(got, other)
     for i in range(n):  # sums in another order, 18 layers: the bound of the other comparisons of attention kernels
         assert rel_l2(got[i], other[i]) <= 5e-5, i
+
+
+# the short-prompt kernel against the long-prompt kernel of the CUDA cores: one to three CTAs share a walk, with walks of their own beside them or none, odd
+# numbers of pairs, the last CTA of a cluster without work, walks that a window cuts
+@pytest.mark.parametrize("S", [2, 3, 24, 32, 33, 64, 65, 95, 97, 126, 150, 195, 212, 213, 221, 513, 515, 940])
+def test_short_prompt_kernel_against_the_long_prompt_kernel(capi, synth, weights_270m, monkeypatch, S):
+    m = capi.Model("270m").load_file(weights_270m).build_tables(1 << 20)
+    prompt = synth.random_prompt(S, 140)[None]
+    a = prefill(m, prompt, monkeypatch, {})
+    b = prefill(m, prompt, monkeypatch, {"TG_ATTN_TC": "0", "TG_ATTN_SMALL_MAX": "0"})
+    m.close()
+    assert not np.array_equal(a, b) or S < 4  # (another kernel; with a key or two its sums may be the same)
+    assert rel_l2(a, b) <= 5e-5 and np.all(np.isfinite(a))
