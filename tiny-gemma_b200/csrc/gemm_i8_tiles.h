@@ -42,8 +42,8 @@ inline I8Plan i8_plan(int M, int K, int ng, const int *N, int num_sms, size_t pa
 	for (int g = 0; g < ng; g++) ntot += N[g];
 	for (int cg = 1; cg <= 2; cg++) {
 		if (want_cg && cg != want_cg) continue;
-		// up to 64 tokens the digits that a pair would share are little beside the weights (vocabulary matrix of 1152 rows, pairs / single CTAs:
-		// 3 tokens 65.5 / 57.8 us, 64 74.8 / 71.0, but 256 200 / 227; of 640 rows 50 / 40)
+		// up to 64 tokens the digits that a pair would share are little beside the weights (vocabulary matrix, pairs / single CTAs with the same
+		// large stages, ncu: 640 rows, 3 tokens 44.2 / 36.0 us, 64 59.2 / 45.4; 1152 rows 58.0 / 58.8 and 72.0 / 71.0, but 256 tokens 200 / 227)
 		if (!want_cg && cg == 2 && groups <= I8_TG) continue;
 		int col_tiles = 0;
 		for (int g = 0; g < ng; g++) col_tiles += (N[g] + 128 * cg - 1) / (128 * cg);

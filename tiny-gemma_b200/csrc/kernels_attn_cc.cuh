@@ -110,8 +110,9 @@ constexpr int AD_STAGES = 3;
 constexpr int AD_SMEM = AT_THREADS / 32 * AD_STAGES * AD_BUF;
 // Few sequences: the splits of a sequence are clusters of CTAs, whose parts meet in the first one's shared memory; only where a cache takes more than
 // one cluster do parts go through memory and a ticket (a store, a fence, an atomic and a load, one behind the other: 1.5 us).
-// Steps of the 270m model in us, through memory against in clusters: 3 sequences of 61 positions 464 / 430, of 500 510 / 466, of 6000 540 / 483; 16 of 61
-// 501 / 487, but 16 of 500 539 / 589 (one CTA per SM): up to 8 sequences.
+// Steps in us, through memory / in clusters. 1B: 2 sequences of 61 positions 778 / 732, 8 837 / 752, 8 of 1500 910 / 868, 4 and 8 of 6000 900 / 896 and 975 / 953;
+// 270m: 451 / 411, 492 / 429, 531 / 501, 528 / 510 and 572 / 571; 16 of 61 501 / 487, but 16 of 500 539 / 589 (one CTA per SM): up to 8 sequences. (4 and 8 long
+// caches come to 16 clusters; a GPU holds 15 or 16 at once, by which of its SMs are in use.)
 constexpr int AD_CLUSTER = 8, AD_CLUSTER_SEQS = 8;
 inline int attn_decode_smem(int cluster) { return AD_SMEM + (cluster - 1) * AT_PART * 4; }
 
@@ -486,7 +487,8 @@ struct AttnSmallPlan {
 	int smem() const { return APS_RING + (ks - 1) * APS_PART * 4; }
 };
 // For a prompt of S tokens behind `off` others. By the prompt alone: a prompt of a group gets the bits that it gets by itself. The largest cluster
-// with two rounds of 32 keys per CTA at least (one where there are three in all: 61 tokens of 1B 1139 -> 1125 us, but 128 1283 -> 1297) whose CTAs are all resident at once (one per SM; the SMs of a GPC hold whole clusters): 178 tokens 2, 61 behind 1500 cached ones 4.
+// with two rounds of 32 keys per CTA at least (one where there are three in all: 61 tokens of 1B 1139 -> 1125 us, but 128 1283 -> 1297) whose CTAs are all resident at once (one per SM; the SMs of a GPC hold whole clusters): 178 tokens 2, 61 behind 1500 cached ones 4. How many
+// that are differs by GPU (clusters of 3, 4 and 5: 135 to 138, 128 to 132 and 115 to 130 CTAs seen); as constants, or a prompt's bits would differ with it.
 inline AttnSmallPlan attn_small_plan(int S, int off, int is_local, int window) {
 	constexpr int ROUND = APS_GROUPS * APS_KEYS, resident[APS_MAX_KS + 1] = {0, 148, 148, 138, 128, 115};
 	const int pairs = (S + 1) / 2, most = is_local ? std::min(off + S, window + 2) : off + S;

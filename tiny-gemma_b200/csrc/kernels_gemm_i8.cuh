@@ -49,7 +49,7 @@ namespace tg {
 constexpr int I8_THREADS = 320;                // producer, MMA issuer, 8 epilogue warps
 // CG CTAs work on a tile of CG * 128 columns: each holds its own 128 columns of W and 1 / CG of the digits. A stage of the ring holds the digits of SLOT token
 // groups. With the few tokens of a decode step four stages that 64 tokens would fit left 64 KB of weights in flight per SM, too few for HBM's rate times its
-// latency: three rows of 640 x 262144 43 us, with eight small stages 40 (1152 rows: 65 and 58). As constants, or each MMA takes longer to issue (a ring whose
+// latency: three rows of 640 x 262144 35.8 us, with eight small stages 31.4 (1152 rows: 58.6 and 52.9; ncu, single CTAs in both). As constants, or each MMA takes longer to issue (a ring whose
 // numbers follow the launch: 77 x 1152 x 6912 18.3 -> 18.8 us). 220 KB in place of 192 leave no room for a CTA of the next launch: a prompt of 61 tokens 1196 -> 1248 us.
 constexpr int I8_FEW = 2;                // groups of a tile that takes the small stages
 constexpr int I8_ROOM = 192 * 1024, I8_SMEM = I8_ROOM + 1024;
@@ -417,7 +417,7 @@ __device__ __forceinline__ float4 ge_quad(const GeluLut &lut, const float *value
 	}
 	return make_float4(y[0] * (u.x * us.x), y[1] * (u.y * us.y), y[2] * (u.z * us.z), y[3] * (u.w * us.w));
 }
-// CTAS: per SM. With one, the scales of a thread's columns are requested before the wait for the predecessor (48 rows of 6912, a layer 1.5 us less).
+// CTAS: per SM. With two, 80 bytes of a thread's registers spill (PER = 3). With one, the scales of a thread's columns are requested before the wait for the predecessor (48 rows of 6912, a layer 1.5 us less).
 template <int NT, int PER, int CTAS = 2>
 __global__ void __launch_bounds__(NT, CTAS) geglu_i8_kernel(const float *ug, uint8_t *out, float *rowscale, int M, int I, int groups, GeluLut lut,
                                                       int nsplit, const float *su, const float *sg) {
